@@ -131,6 +131,15 @@ int jt_gemm_tn(int tn);
 int jt_gemm_ext(const void* A, const void* EA, const void* B, const void* EB, void* Cm, void* CE, void* C32, void* Ce,
                 const void* Xm, const void* XE, void* Om2, void* OE2, const void* RA, const void* RB,
                 int M, int N, int K, int modo, int kid);
+/* jt_gemm_ext with a workspace (1024-byte aligned, at least jt_gemm_ws_bytes bytes, private to the call until its kernels are done): the
+ * half-precision tensor path, which needs one, takes the sizes where it is the faster one - jt_gemm_ws_bytes is 0 elsewhere - and with it
+ * every size jt_gemm_ext takes runs on the tensor cores.  Same bits either way. */
+long long jt_gemm_ws_bytes(int M, int N, int K, int modo);
+int jt_gemm_ws(const void* A, const void* EA, const void* B, const void* EB, void* Cm, void* CE, void* C32, void* Ce,
+               const void* Xm, const void* XE, void* Om2, void* OE2, const void* RA, const void* RB, void* ws,
+               int M, int N, int K, int modo, int kid);
+/* The stream set with jt_stream. */
+void* jt_stream_atual(void);
 /* R8[i] = max over the nb block exponents of row i of E (int8 [linhas, nb]): the RA / RB above. */
 int jt_max_linha(const void* E, void* R8, int linhas, int nb, int kid);
 

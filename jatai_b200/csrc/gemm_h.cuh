@@ -1,0 +1,461 @@
+// Block GEMM on the half-precision tensor pipe (tcgen05.mma kind::f16, fp32 accumulators in tensor memory) with the exponent alignment
+// folded into the operands.
+//
+//   C[M,N] = A[M,K] . B[N,K]^T, operands blocked along K (jatai_cuda/ops.py:95-108):
+//   acc_ij = sum over K-blocks b of rnd(p_ijb << 4, (RA_i - ea_ib) + (RB_j - eb_jb)),  p = exact int8 dot product of the block.
+//
+// What has to be rounded is r = p 2^(4 - sa - sb) with sa = RA_i - ea_ib, sb = RB_j - eb_jb.  A mantissa times a power of two is exact in
+// half precision over the range that matters, so a first kernel (k_prep_h) writes A' = a 2^(2 - sa) and B' = b 2^(2 - sb) as f16 and
+// the tensor core's fp32 sum over one block IS r, exactly: all products of a block are whole multiples of 2^(4 - sa - sb) below
+// 2^24 of them (|p| <= 32 * 127^2 < 2^19, block 128: < 2^21).  From sa = 27 on (or sb) |r| < 1/2 for every p, the rounded value is 0
+// and the operand is written as 0 (a 2^(2 - 26) is the smallest subnormal that occurs).
+//
+// That leaves the CUDA cores ONE packed addition per two element-steps - r + 1.5 * 2^23 rounds half to even at integer granularity -
+// and one three-input integer addition per two element-steps (two K-blocks at a time): no exponent table, no scaling, no int -> float
+// conversion.  The rounding is exact while |r| < 2^22, i.e. |p| 2^-(sa+sb) < 2^18.  Block 32: k_prep_h leaves, per 32 rows and K-block,
+// the largest squared norm of a block scaled by 4^-s; by Cauchy-Schwarz the bound holds for a warp's 32 x 64 outputs whenever the product
+// of its two norms is below 2^36, which a warp evaluates for 32 K-blocks at once; where it does not hold, and always with block 128 (a
+// quarter of the drains), the results' exponent fields are checked and a failing warp reads the accumulators again and converts.
+#pragma once
+#include "gemm_tc.cuh"
+
+namespace jt {
+namespace th {
+
+using namespace tc;
+
+constexpr int KH = 64;                                     // K elements per operand stage: 128 bytes of f16, one swizzle row
+constexpr float LIM_NORMA = 68719000000.0f;               // just below 2^36 (the product of two fp32 roundings included)
+
+// ------------------------------------------------------------------------------------------ operand preparation
+struct ArgsPrepH {
+    const int8_t* m[2]; const int8_t* E[2]; const int8_t* Rext[2];      // A and B: mantissas, exponents, external row maxima or nullptr
+    uint16_t* h[2]; int8_t* R[2]; float* nrm[2];                         // f16 operands, row maxima, norms [ceil(rows/32)][K/32] (block 32)
+    int linhas[2], ctas0;                                                // rows of each; CTAs of A (B's follow)
+    int K;
+};
+
+// 4 mantissas (bytes) -> 4 halves, scaled: with its sign bit flipped a byte b is b + 128; under the bits of 1024 it reads as the half
+// 1152 + b, and one fused multiply-add takes the 1152 off and scales, exactly (every result is representable)
+__device__ __forceinline__ void bytes_para_h(uint32_t w, uint32_t esc, uint32_t tira, uint32_t& lo, uint32_t& hi) {
+    const uint32_t u = w ^ 0x80808080u;
+    const uint32_t a = __byte_perm(u, 0x64646464u, 0x4140), b = __byte_perm(u, 0x64646464u, 0x4342);
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(lo) : "r"(a), "r"(esc), "r"(tira));
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(hi) : "r"(b), "r"(esc), "r"(tira));
+}
+__device__ __forceinline__ uint32_t dois_h(float v) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %1;" : "=r"(r) : "f"(v));
+    return r;
+}
+
+// One CTA of 256 threads: 32 rows x 512 columns of one operand; a warp takes 4 rows, a lane 16 consecutive elements of each.  Bound by
+// memory (1 byte in, 2 out per element); the exponents of the whole row are read by every CTA of the row (K / 32 bytes, from L2).
+template <int BLK>
+__global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
+    pdl_espera();
+    pdl_solta();
+    __shared__ float nrm_s[8][16];
+    const int q = (int)blockIdx.x >= P.ctas0, cta = (int)blockIdx.x - (q ? P.ctas0 : 0);
+    const int K = P.K, nb = K / BLK, nfx = (K + 511) / 512, c0 = (cta % nfx) * 512, g32 = cta / nfx;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, c = c0 + lane * 16;
+    const int8_t *m = q ? P.m[1] : P.m[0], *E = q ? P.E[1] : P.E[0], *Rx = q ? P.Rext[1] : P.Rext[0];
+    const int linhas = q ? P.linhas[1] : P.linhas[0], l0 = g32 * 32 + wid * 4;
+    uint16_t* h = q ? P.h[1] : P.h[0];
+    const bool dentro = c < K;
+    uint4 v[4];
+    int e[4], r[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int l = min(l0 + i, linhas - 1);
+        v[i] = dentro ? *reinterpret_cast<const uint4*>(m + (size_t)l * K + c) : make_uint4(0, 0, 0, 0);
+        e[i] = dentro ? (int)E[(size_t)l * nb + c / BLK] : E_ZERO;
+        r[i] = -128;
+    }
+    if (Rx) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) r[i] = Rx[min(l0 + i, linhas - 1)];
+    } else {
+        if ((nb & 3) == 0) {
+            for (int b = lane * 4; b < nb; b += 128)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const uint32_t w = *reinterpret_cast<const uint32_t*>(E + (size_t)min(l0 + i, linhas - 1) * nb + b);
+                    const unsigned m1 = __vmaxs4(w, w >> 16 | w << 16), m2 = __vmaxs4(m1, m1 >> 8 | m1 << 24);
+                    r[i] = max(r[i], (int)(int8_t)(m2 & 0xff));
+                }
+        } else {
+            for (int b = lane; b < nb; b += 32)
+#pragma unroll
+                for (int i = 0; i < 4; i++) r[i] = max(r[i], (int)E[(size_t)min(l0 + i, linhas - 1) * nb + b]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) r[i] = __reduce_max_sync(FULL, r[i]);
+    }
+    float nmax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int s = r[i] - e[i];
+        const float esc = s <= 26 ? pot2(2 - s) : 0.f;
+        const uint32_t e2 = dois_h(esc), t2 = dois_h(-1152.0f * esc);
+        uint32_t o[8];
+        bytes_para_h(v[i].x, e2, t2, o[0], o[1]);
+        bytes_para_h(v[i].y, e2, t2, o[2], o[3]);
+        bytes_para_h(v[i].z, e2, t2, o[4], o[5]);
+        bytes_para_h(v[i].w, e2, t2, o[6], o[7]);
+        if (dentro && l0 + i < linhas) {
+            uint4* d = reinterpret_cast<uint4*>(h + (size_t)(l0 + i) * K + c);
+            d[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            d[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+        if (BLK == 32) {
+            int n = __dp4a((int)v[i].x, (int)v[i].x, 0);
+            n = __dp4a((int)v[i].y, (int)v[i].y, n);
+            n = __dp4a((int)v[i].z, (int)v[i].z, n);
+            n = __dp4a((int)v[i].w, (int)v[i].w, n);
+            n += __shfl_xor_sync(FULL, n, 1);
+            nmax = fmaxf(nmax, (float)n * (s <= 26 ? pot2(-2 * s) : 0.f));
+        }
+    }
+    if (c0 == 0 && lane < 4 && l0 + lane < linhas) {
+        const int rr = lane == 0 ? r[0] : lane == 1 ? r[1] : lane == 2 ? r[2] : r[3];
+        (q ? P.R[1] : P.R[0])[l0 + lane] = (int8_t)rr;
+    }
+    if (BLK == 32) {
+        if ((lane & 1) == 0) nrm_s[wid][lane >> 1] = nmax;
+        __syncthreads();
+        if (threadIdx.x < 16 && c0 / 32 + (int)threadIdx.x < nb) {
+            float n = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; w++) n = fmaxf(n, nrm_s[w][threadIdx.x]);
+            (q ? P.nrm[1] : P.nrm[0])[(size_t)g32 * nb + c0 / 32 + threadIdx.x] = n;
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------ the product
+// A CTA works through 128 x TNv tiles of C (each optionally one K range of it); 4 x NCG drain warps, one warp that loads and one or two
+// that multiply.
+//   TNv 128, 16 drain warps, one CTA per SM, persistent: while the drain warps put a tile out, the next one's operands are already
+//           being loaded and multiplied
+//   TNv 64, 8 drain warps, two CTAs per SM, one tile each (block 32): where 128-wide tiles would leave SMs without work
+template <int TNv, int BLK>
+struct CfgH {
+    static constexpr bool PERSISTE = TNv == 128;
+    static constexpr int CTAS = PERSISTE ? 1 : 2, N_DW = PERSISTE ? 16 : 8, N_EPI = N_DW * 32;
+    static constexpr int COLS = TNv / (N_DW / 4);                           // accumulator columns of a drain thread: 32
+    static constexpr int G = BLK == 32 ? 2 : 1;                             // K-blocks handed over together
+    static constexpr int NS = 512 / CTAS / (G * TNv);                       // tensor-memory stages of G x TNv columns
+    static constexpr int N_MW = 2, N_THR = N_EPI + 32 + 32 * N_MW;          // multiplying warps: each takes every N_MW-th stage
+    static_assert(NS >= N_MW && COLS == 32, "");
+    static constexpr uint32_t B_BYTES = TNv * 128, STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int NST = 4;
+    // the staged accumulators: memory of their own where the loads of the next tile go on meanwhile, else the operand ring (when a
+    // drain thread stores them it has seen the commit of the last MMA)
+    static constexpr uint32_t ACC_BYTES = TM * (TNv + 4) * 4, OFF_ACC = PERSISTE ? NST * STAGE_BYTES : 0;
+    static_assert(PERSISTE || ACC_BYTES <= NST * STAGE_BYTES, "staged accumulators must fit in the operand ring");
+    static constexpr uint32_t OFF_RA = PERSISTE ? OFF_ACC + ACC_BYTES : NST * STAGE_BYTES, OFF_RB = OFF_RA + TM * 4, OFF_RBF = OFF_RB + TNv * 4,
+                              OFF_RBM = OFF_RBF + TNv * 4;
+    static constexpr uint32_t OFF_BAR = OFF_RBM + 32, OFF_MISC = OFF_BAR + (2 * NST + 2 * NS) * 8;
+    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;            // + slack to align the base to 1024 bytes
+    static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
+    // instruction descriptor kind::f16: D = f32, A = B = f16, both K-major, N = TNv, M = 128
+    static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+};
+// how the tiles are numbered: columns fastest, then rows, then K ranges
+struct Grade { int nx, ny, partes, ppp; };                                  // tiles per row and column, K ranges, 64-element chunks per range
+
+// one lane of a converged warp
+__device__ __forceinline__ bool elege() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acumula) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+                 ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(acumula) : "memory");
+}
+// 8, 16 or 32 consecutive columns of this lane, asynchronous: the registers may be used after tmem_pronto on them
+__device__ __forceinline__ void tmem_pede(uint32_t t, uint32_t (&d)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : JT_O4(d, 0), JT_O4(d, 4) : "r"(t) : "memory");
+}
+__device__ __forceinline__ void tmem_pede(uint32_t t, uint32_t (&d)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" : JT_O16(d, 0) : "r"(t) : "memory");
+}
+__device__ __forceinline__ void tmem_pede(uint32_t t, uint32_t (&d)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+                 "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];" : JT_O32(d, 0) : "r"(t) : "memory");
+}
+#define JT_IO4(a, i) "+r"(a[i]), "+r"(a[i + 1]), "+r"(a[i + 2]), "+r"(a[i + 3])
+#define JT_IO16(a, i) JT_IO4(a, i), JT_IO4(a, i + 4), JT_IO4(a, i + 8), JT_IO4(a, i + 12)
+__device__ __forceinline__ void tmem_pronto(uint32_t (&a)[8]) { asm volatile("tcgen05.wait::ld.sync.aligned;" : JT_IO4(a, 0), JT_IO4(a, 4)::"memory"); }
+__device__ __forceinline__ void tmem_pronto(uint32_t (&a)[16]) { asm volatile("tcgen05.wait::ld.sync.aligned;" : JT_IO16(a, 0)::"memory"); }
+__device__ __forceinline__ void tmem_pronto(uint32_t (&a)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : JT_IO16(a, 0)::"memory");
+    asm volatile("" : JT_IO16(a, 16)::"memory");                            // (an asm statement takes 30 operands: the rest is tied to the wait by order)
+}
+// two fp32 additions in one instruction: r + 1.5 * 2^23, the rounding of the specification
+__device__ __forceinline__ void soma_magia(uint32_t& a, uint32_t& b) {
+    asm volatile("{\n .reg .b64 t;\n mov.b64 t, {%0, %1};\n add.rn.f32x2 t, t, %2;\n mov.b64 {%0, %1}, t;\n}" : "+r"(a), "+r"(b) : "l"(par(MAGIA, MAGIA)));
+}
+// acc += a + b in one three-input addition of the integer pipe.  (volatile: left to itself the compiler turns such sums into pairs of
+// multiply-adds on the floating-point pipe, which the packed additions already fill)
+__device__ __forceinline__ void soma3(int& acc, uint32_t a, uint32_t b) {
+    asm volatile("add.s32 %0, %0, %1;\n add.s32 %0, %0, %2;" : "+r"(acc) : "r"(a), "r"(b));
+}
+// NV columns of two K-blocks onto the accumulators acc[o ...]
+template <int NV, int NA>
+__device__ __forceinline__ void junta_lote(uint32_t (&a)[NV], uint32_t (&b)[NV], int (&acc)[NA], int o) {
+#pragma unroll
+    for (int k = 0; k < NV; k += 2) {
+        soma_magia(a[k], a[k + 1]);
+        soma_magia(b[k], b[k + 1]);
+        soma3(acc[o + k], a[k], b[k]);
+        soma3(acc[o + k + 1], a[k + 1], b[k + 1]);
+    }
+}
+// the same by conversion, exact for every value (K-blocks whose norm product reaches 2^36)
+template <int NV, int NA>
+__device__ __forceinline__ void converte_lote(const uint32_t (&a)[NV], const uint32_t (&b)[NV], int (&acc)[NA], int o) {
+#pragma unroll
+    for (int k = 0; k < NV; k++)
+        acc[o + k] += __float2int_rn(__uint_as_float(a[k])) + __float2int_rn(__uint_as_float(b[k])) + (int)(2 * MAGIA);
+}
+
+template <int BLK, int MODO, int TNv>
+__global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k_gemm_h(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                                                       const int8_t* __restrict__ RA, const int8_t* __restrict__ RB, const float* __restrict__ nA,
+                                                       const float* __restrict__ nB, SaidaGemm S, int M, int N, int K, Grade Gr, int kid) {
+    using C_ = CfgH<TNv, BLK>;
+    constexpr int NST = C_::NST, NS = C_::NS, COLS = C_::COLS, LV = 16, N_EPI = C_::N_EPI, N_DW = C_::N_DW, N_MW = C_::N_MW;
+    constexpr int CB = BLK == 32 ? 1 : 2;                                   // chunks per tensor-memory stage: two K-blocks of 32, or one of 128
+    extern __shared__ unsigned char smem_bruto[];
+    unsigned char* smem = smem_bruto + ((1024u - (smem_u32(smem_bruto) & 1023u)) & 1023u);      // stays in the shared address space
+    const uint32_t sbase = smem_u32(smem);
+    int* acc_s = reinterpret_cast<int*>(smem + C_::OFF_ACC);
+    int* RAs = reinterpret_cast<int*>(smem + C_::OFF_RA);
+    int* RBs = reinterpret_cast<int*>(smem + C_::OFF_RB);
+    float* RBf = reinterpret_cast<float*>(smem + C_::OFF_RBF);
+    int* RBm = reinterpret_cast<int*>(smem + C_::OFF_RBM);
+    const uint32_t bar_full = sbase + C_::OFF_BAR, bar_empty = bar_full + NST * 8, bar_tfull = bar_empty + NST * 8, bar_tempty = bar_tfull + NS * 8;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C_::OFF_MISC);
+    volatile int* aborta = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 4);
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    const int ntiles = Gr.nx * Gr.ny * Gr.partes, npedT = (K + KH - 1) / KH;
+
+    if (tid == 0) {
+        for (int i = 0; i < NST; i++) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
+        for (int i = 0; i < NS; i++) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, N_DW); }
+        *aborta = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (wid == N_DW) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512 / C_::CTAS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_antes();
+    __syncthreads();
+    tc_fence_depois();
+    const uint32_t tmem = *tmem_slot;
+    pdl_espera();                                  // everything above touches no global memory: it overlaps the predecessor's tail
+    pdl_solta();
+
+    // The loading and the multiplying warps run their loops as whole warps, with one elected lane for the asynchronous instructions: the
+    // addresses and descriptors then live in uniform registers.  They share their schedulers with busy drain warps, so what counts
+    // is how few instructions a chunk takes them (with one lane in a divergent branch the multiplying warp took 680 cycles a chunk and
+    // bounded the kernel).
+    if (wid == N_DW) {
+        // ------------------------------------------------------------------ loads
+        if (*reinterpret_cast<volatile int*>(&g_sem_cargas) == 0) {
+            const bool eleito = elege();
+            int s = 0;
+            uint32_t fase = 1;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+                const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp;
+                const int xf = min(ped0 + Gr.ppp, npedT) * KH;
+                for (int x = ped0 * KH; x < xf; x += KH) {
+                    ok = __all_sync(FULL, espera(bar_empty + 8 * s, fase, aborta, kid, 1));
+                    if (!ok) break;
+                    if (eleito) {
+                        mbar_expect_tx(bar_full + 8 * s, C_::STAGE_BYTES);
+                        tma_2d(sbase + s * C_::STAGE_BYTES, &mapA, x, m0, bar_full + 8 * s);
+                        tma_2d(sbase + s * C_::STAGE_BYTES + A_BYTES, &mapB, x, n0, bar_full + 8 * s);
+                    }
+                    if (++s == NST) { s = 0; fase ^= 1; }
+                }
+            }
+        }
+    } else if (wid > N_DW) {
+        // ------------------------------------------------------------------ MMAs.  A chunk takes a warp ~500 cycles of waits and issue, its
+        // MMAs 256: two warps take the stages in turn (every stage starts a sum of its own).
+        const bool eleito = elege();
+        const uint64_t da0 = desc_sw128(sbase), db0 = desc_sw128(sbase + A_BYTES);
+        int s = 0, t = 0, vez = wid - N_DW - 1;
+        uint32_t fase = 0, fase_t = 1;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nped = min(Gr.ppp, npedT - ped0);
+            for (int i = 0; i < nped && ok; i += CB) {
+                const bool minha = vez == 0;
+                vez = minha ? N_MW - 1 : vez - 1;
+                if (minha) ok = __all_sync(FULL, espera(bar_tempty + 8 * t, fase_t, aborta, kid, 3));
+#pragma unroll
+                for (int j = 0; j < CB; j++) {
+                    if (minha && ok) {
+                        ok = __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
+                        tc_fence_depois();
+                        const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
+                        const uint32_t d = tmem + t * (C_::G * TNv);
+                        if (eleito && ok) {
+                            if (BLK == 32) {
+                                mma_f16(d, da, db, C_::IDESC, 0);                   // +32 bytes (16 elements of K) per instruction
+                                mma_f16(d, da + 2, db + 2, C_::IDESC, 1);
+                                mma_f16(d + TNv, da + 4, db + 4, C_::IDESC, 0);
+                                mma_f16(d + TNv, da + 6, db + 6, C_::IDESC, 1);
+                            } else {
+#pragma unroll
+                                for (int q = 0; q < 4; q++) mma_f16(d, da + 2 * q, db + 2 * q, C_::IDESC, j | q);
+                            }
+                            if (j == CB - 1) tc_commit(bar_tfull + 8 * t);
+                            tc_commit(bar_empty + 8 * s);
+                        }
+                    }
+                    if (++s == NST) { s = 0; fase ^= 1; }
+                }
+                if (++t == NS) { t = 0; fase_t ^= 1; }
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------ drain + output stage
+        const int quarto = wid & 3, cg = wid >> 2, lin = quarto * 32 + lane;
+        const uint32_t base = tmem + ((uint32_t)(quarto * 32) << 16) + cg * COLS;
+        int t = 0;
+        uint32_t fase_t = 0;
+        // waits for the next stage (a wait that gives up makes all later ones return at once) / hands it back, its contents in registers
+        auto recebe = [&]() {
+            espera(bar_tfull + 8 * t, fase_t, aborta, kid, 4);
+            __syncwarp();
+            tc_fence_depois();
+        };
+        auto devolve = [&]() {
+            tc_fence_antes();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
+            if (++t == NS) { t = 0; fase_t ^= 1; }
+        };
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, parte = tile / (Gr.nx * Gr.ny), ped0 = parte * Gr.ppp;
+            const int nped = min(Gr.ppp, npedT - ped0);
+            // the row maxima, wanted by the output stage: read now, stored to shared memory after the main loop
+            int ra = 0, rb = 0;
+            if (tid < TM) ra = m0 + tid < M ? (int)RA[m0 + tid] : 0;
+            if (tid < TNv) rb = RB[n0 + tid];
+            int acc[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; j++) acc[j] = 0;
+            if constexpr (BLK == 32) {
+                const int nb = K / 32;
+                unsigned suspeitos = 0;                                      // bit k: K-block (c & ~15) * 2 + k of this range may leave the exact window
+                for (int c = 0; c < nped; c++) {
+                    if ((c & 15) == 0) {
+                        // 32 K-blocks ahead: this warp's largest squared norms of A (32 rows) and B (32 columns)
+                        const int f = (ped0 + c) * 2 + lane;
+                        float pa = 0.f, pb = 0.f;
+                        if (f < nb) {
+                            pa = nA[(size_t)min(m0 / 32 + quarto, (M + 31) / 32 - 1) * nb + f];
+                            pb = nB[(size_t)((n0 + cg * COLS) / 32) * nb + f];
+                        }
+                        suspeitos = __ballot_sync(FULL, pa * pb >= LIM_NORMA);
+                    }
+                    const uint32_t ta = base + t * (2 * TNv);
+                    const bool certo = ((suspeitos >> (2 * (c & 15))) & 3u) == 0;
+                    recebe();
+                    if (certo) {
+#pragma unroll
+                        for (int o = 0; o < COLS; o += LV) {
+                            uint32_t a[LV], b[LV];
+                            tmem_pede(ta + o, a);
+                            tmem_pede(ta + TNv + o, b);
+                            tmem_pronto(a);
+                            tmem_pronto(b);
+                            if (o + LV == COLS) devolve();
+                            junta_lote(a, b, acc, o);
+                        }
+                    } else {
+#pragma unroll
+                        for (int o = 0; o < COLS; o += LV) {
+                            uint32_t a[LV], b[LV];
+                            tmem_pede(ta + o, a);
+                            tmem_pede(ta + TNv + o, b);
+                            tmem_pronto(a);
+                            tmem_pronto(b);
+                            converte_lote(a, b, acc, o);
+                        }
+                        devolve();
+                    }
+                }
+            } else {
+                for (int c = 0; c < nped / 2; c++) {
+                    const uint32_t ta = base + t * TNv;
+                    recebe();
+#pragma unroll
+                    for (int o = 0; o < COLS; o += LV) {
+                        uint32_t a[LV], x[LV], fora = 0;
+                        tmem_pede(ta + o, a);
+                        tmem_pronto(a);
+                        if (o + LV == COLS) devolve();
+                        // (the exponent field of every sum must be that of 1.5 * 2^23)
+#pragma unroll
+                        for (int k = 0; k < LV; k += 2) {
+                            x[k] = a[k]; x[k + 1] = a[k + 1];
+                            soma_magia(x[k], x[k + 1]);
+                            fora |= (x[k] ^ MAGIA) | (x[k + 1] ^ MAGIA);
+                        }
+                        if (__any_sync(FULL, (fora & 0xFF800000u) != 0)) {
+#pragma unroll
+                            for (int k = 0; k < LV; k++) x[k] = (uint32_t)__float2int_rn(__uint_as_float(a[k])) + MAGIA;
+                        }
+#pragma unroll
+                        for (int k = 0; k < LV; k++) acc[o + k] += (int)x[k];
+                    }
+                }
+            }
+            const uint32_t vies = (uint32_t)(BLK == 32 ? nped * 2 : nped / 2) * MAGIA;
+            constexpr int PITCHv = TNv + 4;
+            if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
+            if (tid < TM) RAs[tid] = ra;
+            if (tid < TNv) {
+                RBs[tid] = rb;
+                if (MODO != 1) {
+                    // what the fp32 path of the output stage needs: each block's extreme column exponents and the column scales
+                    int mn = __reduce_min_sync(FULL, rb), mx = __reduce_max_sync(FULL, rb);
+                    if (lane == 0) { RBm[wid] = mn; RBm[4 + wid] = mx; }
+                    if (BLK > 32) {                                          // one block over the four warps: place 0 gets its extremes
+                        asm volatile("bar.sync 3, %0;" ::"n"(TNv) : "memory");
+                        mn = min(min(RBm[0], RBm[1]), min(RBm[2], RBm[3]));
+                        mx = max(max(RBm[4], RBm[5]), max(RBm[6], RBm[7]));
+                        if (tid == 0) { RBm[0] = mn; RBm[4] = mx; }
+                    }
+                    RBf[tid] = pot2(min(rb - mn, 100));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < COLS; j += 4)
+                *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * COLS + j) =
+                    make_int4((int)((uint32_t)acc[j] - vies), (int)((uint32_t)acc[j + 1] - vies), (int)((uint32_t)acc[j + 2] - vies), (int)((uint32_t)acc[j + 3] - vies));
+            asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
+            epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s, RAs, RBs, min(TM, M - m0), m0, n0, N, S, Gr.partes > 1, parte == 0, kid, tid, RBf, RBm);
+        }
+    }
+    tc_fence_antes();
+    __syncthreads();
+    if (wid == N_DW) {
+        tc_fence_depois();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512 / C_::CTAS) : "memory");
+    }
+}
+
+}  // namespace th
+}  // namespace jt

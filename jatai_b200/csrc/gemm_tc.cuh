@@ -571,4 +571,16 @@ static bool faz_mapa(CUtensorMap* m, const void* p, int linhas, int K, int linha
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// the same for a matrix of halves [linhas, K]: box = linhas_caixa rows x 64 elements; rows and columns beyond the matrix read as zero
+static bool faz_mapa_h(CUtensorMap* m, const void* p, int linhas, int K, int linhas_caixa) {
+    PFN_tmap f = pega_tmap();
+    if (!f) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)linhas};
+    cuuint64_t passos[1] = {(cuuint64_t)K * 2};
+    cuuint32_t caixa[2] = {64, (cuuint32_t)linhas_caixa};
+    cuuint32_t um[2] = {1, 1};
+    return f(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(p), dims, passos, caixa, um, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace jt

@@ -18,6 +18,7 @@
 #include "gemm_comum.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
+#include "gemm_h.cuh"
 #include "atencao.cuh"
 #include "atencao_tc.cuh"
 #include "atencao_peq.cuh"
@@ -27,11 +28,12 @@ using namespace jt;
 // ---------------------------------------------------------------------------------------------- host state
 static cudaStream_t g_stream = 0;
 static int g_blk = 32;               // exponent block length: 32 (native) or 128 (the reference's format)
-static int g_via = 0;                // GEMM path: 0 automatic | 1 tensor core (forced) | 2 CUDA cores | 3 tensor core, rounding by conversion
+static int g_via = 0;                // GEMM path: 0 automatic | 1 tensor core (forced) | 2 CUDA cores | 3 tensor core, rounding by conversion | 4 half-precision tensor pipe (forced)
 static int g_alvo_ctas = 148;
 static int g_at_via = 0;             // attention path: 0 automatic (tensor cores at head dimension 64, one CTA per head for short sequences of small heads) | 1 the tiled CUDA-core kernels
 static int g_tn = 0;                 // tile width of the tensor-core GEMM: 0 automatic | 64 | 128        // split-K of raw GEMMs aims at this many CTAs
 
+constexpr int N_SM = 148;             // B200
 static int fim() { return (int)cudaGetLastError(); }
 static unsigned nblocos16(long long n16) { return (unsigned)((n16 + 255) / 256); }
 static unsigned nblocos16u(long long n16, int U) { return (unsigned)((n16 + 256LL * U - 1) / (256LL * U)); }      // U chunks per thread
@@ -116,6 +118,93 @@ static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const in
     return (int)cudaErrorInvalidValue;
 }
 
+// ---- the half-precision path (gemm_h.cuh): operands prepared in a workspace of the caller
+struct EspacoH { size_t A, B, RA, RB, nA, nB, total; };
+static EspacoH espaco_h(int M, int N, int K) {
+    auto ar = [](size_t x) { return (x + 1023) & ~(size_t)1023; };
+    EspacoH e;
+    e.A = 0;
+    e.B = e.A + ar((size_t)M * K * 2);
+    e.RA = e.B + ar((size_t)N * K * 2);
+    e.RB = e.RA + ar(M);
+    e.nA = e.RB + ar(N);
+    e.nB = e.nA + ar((size_t)((M + 31) / 32) * (K / 32) * 4);
+    e.total = e.nB + ar((size_t)(N / 32) * (K / 32) * 4);
+    return e;
+}
+static bool forma_gemm(int blk, int M, int N, int K, int modo) {
+    return M > 0 && N > 0 && K > 0 && M % 64 == 0 && N % TN == 0 && K % blk == 0 && K % 32 == 0 && modo >= 0 && modo <= 4;
+}
+// Estimated times of the GEMM kernels in microseconds (measured at 128..16384 rows, 128..4096 columns, K = 128..16384): waves of tiles
+// times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels.
+struct Custos { double i8, h64, h128; };
+static Custos custos_gemm(int blk, int M, int N, int K) {
+    const double n = (K + 63) / 64;
+    const long long t128 = (long long)(N / 128) * ((M + 127) / 128), t64 = 2 * t128;
+    auto ondas = [](long long t, int vagas) { return (double)((t + vagas - 1) / vagas); };
+    const double prep = 4.0 + (double)(M + N) * K * 3 / 4e6;                            // k_prep_h: a launch, and 3 bytes per element at 4 TB/s
+    Custos c;
+    c.h128 = prep + ondas(t128, N_SM) * (n * (blk == 32 ? 0.41 : 0.28) + 1.5);
+    c.h64 = blk == 32 ? prep + (t64 <= N_SM ? n * 0.31 + 2.5 : ondas(t64, 2 * N_SM) * (n * 0.45 + 2.0)) : 1e9;
+    if (M % tc::TM || K % tc::KC) c.i8 = 1e9;                                           // whole tiles only
+    else if (blk == 32) c.i8 = 2.5 + (t64 <= N_SM ? n * 0.75 : ondas(t64, 2 * N_SM) * n * 1.0);
+    else c.i8 = 2.5 + ondas(t128, N_SM) * (n * (t128 <= N_SM ? 0.58 : 0.43) + 1.0);
+    return c;
+}
+// whether a caller with a workspace takes the half-precision path
+static bool usa_h(int M, int N, int K) {
+    if (g_via != 0) return g_via == 4;
+    const Custos c = custos_gemm(g_blk, M, N, K);
+    return (c.h64 < c.h128 ? c.h64 : c.h128) < c.i8;
+}
+template <int BLK, int MODO, int TNv>
+static int lanca_h(const CUtensorMap& mA, const CUtensorMap& mB, const int8_t* RA, const int8_t* RB, const float* nA, const float* nB, const SaidaGemm& S,
+                   int M, int N, int K, const th::Grade& G, int kid) {
+    using C_ = th::CfgH<TNv, BLK>;
+    auto k = th::k_gemm_h<BLK, MODO, TNv>;
+    cudaError_t c = at_smem(k, C_::SMEM_BYTES);
+    if (c != cudaSuccess) return (int)c;
+    const int tiles = G.nx * G.ny * G.partes;
+    lanca_pdl(k, dim3(C_::PERSISTE && tiles > N_SM ? N_SM : tiles), dim3(C_::N_THR), C_::SMEM_BYTES, g_stream, mA, mB, RA, RB, nA, nB, S, M, N, K, G, kid);
+    return fim();
+}
+template <int BLK>
+static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8_t* EB, const int8_t* RA, const int8_t* RB, const SaidaGemm& S, int M, int N,
+                  int K, int modo, unsigned char* ws, int kid) {
+    const EspacoH e = espaco_h(M, N, K);
+    uint16_t *Ah = (uint16_t*)(ws + e.A), *Bh = (uint16_t*)(ws + e.B);
+    int8_t *RAw = (int8_t*)(ws + e.RA), *RBw = (int8_t*)(ws + e.RB);
+    float *nA = (float*)(ws + e.nA), *nB = (float*)(ws + e.nB);
+    const int nfx = (K + 511) / 512, ctasA = (M + 31) / 32 * nfx, ctasB = N / 32 * nfx;
+    th::ArgsPrepH P = {{A, B}, {EA, EB}, {RA, RB}, {Ah, Bh}, {RAw, RBw}, {nA, nB}, {M, N}, ctasA, K};
+    lanca_pdl(th::k_prep_h<BLK>, dim3(ctasA + ctasB), dim3(256), 0, g_stream, P);
+    const Custos c = custos_gemm(BLK, M, N, K);
+    const bool estreito = BLK == 32 && g_tn != 128 && (g_tn == 64 || c.h64 < c.h128);
+    const int tn = estreito ? 64 : TN;
+    CUtensorMap mA, mB;
+    if (!(faz_mapa_h(&mA, Ah, M, K, tc::TM) && faz_mapa_h(&mB, Bh, N, K, tn))) return (int)cudaErrorInvalidValue;
+    const int nped = (K + th::KH - 1) / th::KH, uni = BLK / 64 > 1 ? BLK / 64 : 1;
+    const long long tiles = (long long)(N / tn) * ((M + 127) / 128);
+    int partes = 1;
+    if (modo == 1)
+        while (tiles * partes * 2 <= (estreito ? 2 : 1) * g_alvo_ctas && nped >= partes * 2 * 32) partes *= 2;
+    const int ppp = ((nped + partes - 1) / partes + uni - 1) / uni * uni;
+    partes = (nped + ppp - 1) / ppp;
+    const th::Grade G = {N / tn, (M + 127) / 128, partes, ppp};
+    if (partes > 1) {
+        cudaError_t c = cudaMemsetAsync(S.C32, 0, (size_t)M * N * sizeof(int), g_stream);
+        if (c != cudaSuccess) return (int)c;
+    }
+#define JT_H(MD)                                                                                                                            \
+    case MD:                                                                                                                                \
+        if constexpr (BLK == 32)                                                                                                            \
+            if (estreito) return lanca_h<32, MD, 64>(mA, mB, RAw, RBw, nA, nB, S, M, N, K, G, kid);                                      \
+        return lanca_h<BLK, MD, 128>(mA, mB, RAw, RBw, nA, nB, S, M, N, K, G, kid);
+    switch (modo) { JT_H(0) JT_H(1) JT_H(2) JT_H(3) JT_H(4) }
+#undef JT_H
+    return (int)cudaErrorInvalidValue;
+}
+
 #define JT_POR_BLK(EXPR32, EXPR128) (g_blk == 32 ? (EXPR32) : (EXPR128))
 
 extern "C" {
@@ -154,6 +243,7 @@ int jt_erro_limpa() {
 }
 int jt_sincroniza() { return (int)cudaDeviceSynchronize(); }
 void jt_stream(void* st) { g_stream = (cudaStream_t)st; }
+void* jt_stream_atual() { return (void*)g_stream; }
 void jt_gemm_split(int alvo) { g_alvo_ctas = alvo > 0 ? alvo : 148; }
 void jt_gemm_bm(int) {}
 void jt_atencao_linhas(int) {}
@@ -170,7 +260,7 @@ int jt_gemm_tn(int tn) {
     return 0;
 }
 int jt_gemm_via(int via) {
-    if (via < 0 || via > 3) return (int)cudaErrorInvalidValue;
+    if (via < 0 || via > 4) return (int)cudaErrorInvalidValue;
     g_via = via;
     return 0;
 }
@@ -192,6 +282,24 @@ int jt_gemm_f(const void* A, const void* EA, const void* B, const void* EB, void
 int jt_gemm(const void* A, const void* EA, const void* B, const void* EB, void* Cm, void* CE, void* C32, void* Ce, int M, int N, int K,
             int modo, int kid) {
     return jt_gemm_ext(A, EA, B, EB, Cm, CE, C32, Ce, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, M, N, K, modo, kid);
+}
+// Workspace of jt_gemm_ws for these sizes, in bytes; 0: the call would not use one (jt_gemm_ext is the same).
+long long jt_gemm_ws_bytes(int M, int N, int K, int modo) {
+    if (!forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K)) return 0;
+    return (long long)espaco_h(M, N, K).total;
+}
+// jt_gemm_ext with a workspace of at least jt_gemm_ws_bytes bytes (1024-byte aligned, private to this call until its kernels are done)
+int jt_gemm_ws(const void* A, const void* EA, const void* B, const void* EB, void* Cm, void* CE, void* C32, void* Ce, const void* Xm, const void* XE,
+               void* Om2, void* OE2, const void* RA, const void* RB, void* ws, int M, int N, int K, int modo, int kid) {
+    const bool alinhado = (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
+    if (!ws || ((uintptr_t)ws & 1023) || !alinhado || !forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K))
+        return jt_gemm_ext(A, EA, B, EB, Cm, CE, C32, Ce, Xm, XE, Om2, OE2, RA, RB, M, N, K, modo, kid);
+    SaidaGemm S = {(int8_t*)Cm, (int8_t*)CE, (int*)C32, (int16_t*)Ce, (const int8_t*)Xm, (const int8_t*)XE, (int8_t*)Om2, (int8_t*)OE2};
+    if (modo == 1 ? (!C32 || !Ce) : (!Cm || !CE)) return (int)cudaErrorInvalidValue;
+    if ((modo == 2 || modo == 4) && (!Xm || !XE)) return (int)cudaErrorInvalidValue;
+    if (modo == 3 && (!Om2 || !OE2)) return (int)cudaErrorInvalidValue;
+    return JT_POR_BLK(gemm_h<32>((const int8_t*)A, (const int8_t*)EA, (const int8_t*)B, (const int8_t*)EB, (const int8_t*)RA, (const int8_t*)RB, S, M, N, K, modo, (unsigned char*)ws, kid),
+                      gemm_h<128>((const int8_t*)A, (const int8_t*)EA, (const int8_t*)B, (const int8_t*)EB, (const int8_t*)RA, (const int8_t*)RB, S, M, N, K, modo, (unsigned char*)ws, kid));
 }
 // row-maximum exponents of a block tensor [R, C] (int8 per row): what a data-parallel rank exchanges before a
 // weight-gradient GEMM so that all ranks align their partial sums to the same exponents

@@ -32,7 +32,7 @@ _INT_FUNCS = ("jt_gemm", "jt_gemm_f", "jt_gemm_ext", "jt_max_linha", "jt_quant",
               "jt_momento", "jt_peso", "jt_momento_peso", "jt_transpoe", "jt_transpoe2", "jt_embed", "jt_um_quente", "jt_rms", "jt_rms_back", "jt_rms_back_soma", "jt_atencao",
               "jt_atencao_back", "jt_softmax_ce", "jt_erro_le", "jt_erro_limpa", "jt_sincroniza", "jt_para16", "jt_para8",
               "jt_soma16", "jt_res_estocastico", "jt_blk", "jt_blk_atual", "jt_gemm_via", "jt_gemm_tn", "jt_atencao_back_fixo", "jt_atencao_via", "jt_atencao_quant", "jt_atencao_back_quant",
-              "jt_espera_limite", "jt_teste_espera", "jt_transpoe2_max", "jt_pdl", "jt_gemm_sem_cargas")
+              "jt_espera_limite", "jt_teste_espera", "jt_transpoe2_max", "jt_pdl", "jt_gemm_sem_cargas", "jt_gemm_ws")
 
 
 def g_rms(D):
@@ -53,6 +53,9 @@ def carrega_biblioteca(caminho=None):
     for f in _INT_FUNCS:
         if hasattr(lib, f):
             getattr(lib, f).restype = ctypes.c_int
+    if hasattr(lib, "jt_gemm_ws_bytes"):
+        lib.jt_gemm_ws_bytes.restype = ctypes.c_longlong
+        lib.jt_stream_atual.restype = ctypes.c_void_p
     return lib
 
 
@@ -150,7 +153,12 @@ class OpsCuda:
         if duas:
             C2 = self._bloco_vazio(M, N, dev)
         x = X if X is not None else (None, None)
-        if hasattr(self.lib, "jt_gemm_ext"):
+        n_ws = self._ws_gemm(M, N, K, modo)
+        if n_ws:
+            ws = torch.empty(n_ws, dtype=torch.uint8, device=dev)
+            self._lanca(op, "jt_gemm_ws", (a, ea, b, eb, Cb[0], Cb[1], Cr[0], Cr[1], x[0], x[1], C2[0], C2[1], RA, RB, ws),
+                        (M, N, K, modo), ent, (M, N))
+        elif hasattr(self.lib, "jt_gemm_ext"):
             self._lanca(op, "jt_gemm_ext", (a, ea, b, eb, Cb[0], Cb[1], Cr[0], Cr[1], x[0], x[1], C2[0], C2[1], RA, RB),
                         (M, N, K, modo), ent, (M, N))
         else:       # a library with only the reference's entry points (no external row maxima)
@@ -160,6 +168,14 @@ class OpsCuda:
         if modo == 1:
             return Cr
         return (Cb, C2) if duas else Cb
+
+    def _ws_gemm(self, M, N, K, modo):
+        """Bytes of workspace the library wants for this product (0: none).  The workspace goes back to PyTorch's allocator right after the
+        launch, which is safe only where the library launches on the stream the allocator orders it by."""
+        lib = self.lib
+        if not hasattr(lib, "jt_gemm_ws_bytes") or (lib.jt_stream_atual() or 0) != torch.cuda.current_stream().cuda_stream:
+            return 0
+        return lib.jt_gemm_ws_bytes(M, N, K, modo)
 
     def gemm(self, A, B, cru=False, RA=None, RB=None):
         """C = A . B^T, operands blocked along K.  cru=True: raw int32 accumulators + int16 exponents.

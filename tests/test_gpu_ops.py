@@ -142,6 +142,35 @@ def test_gemm_formas(amb, blk, M, N, K, cru):
     compara(f"gemm {M}x{N}x{K}", casos.plano(out), casos.plano(spec.Spec(blk).gemm(A, B, cru=cru)))
 
 
+@pytest.mark.parametrize("tn", [64, 128])
+@pytest.mark.parametrize("blk,M,N,K", [(32, 64, 128, 32), (32, 128, 128, 96), (32, 192, 256, 2080), (32, 320, 384, 512), (32, 2432, 1408, 160), (32, 128, 128, 8192),
+                                       (128, 64, 128, 128), (128, 192, 384, 640), (128, 2432, 1408, 256)])
+def test_gemm_meia_precisao(amb, blk, M, N, K, tn):
+    """The half-precision tensor path, forced, in every mode against the oracle: rows that fill no tile, a K of half a chunk, more tiles
+    than SMs, K ranges added with atomics, exponents spread beyond what f16 holds, zero blocks; and saturated rows, whose norms
+    exclude the fast rounding."""
+    ops, oc, reg = amb
+    ops.define_blk(blk)
+    assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(tn) == 0
+    try:
+        reg.novo_passo(0)
+        G = casos.Gen(31 + M + N + K + blk, blk)
+        A, B, X = para_gpu(G.bloco(M, K, espalha=15, zera=0.1)), para_gpu(G.bloco(N, K, espalha=5)), para_gpu(G.bloco(M, N, espalha=4))
+        A[0][5::64, :2048] = 127                      # (more saturated K-blocks than this would overflow the accumulator)
+        A[1][5::64] = -8
+        B[0][7::32, :2048] = -127
+        B[1][7::32] = -8
+        s = spec.Spec(blk)
+        for op, args, kw in (("gemm", (A, B), {}), ("gemm", (A, B), dict(cru=True)), ("gemm_soma", (A, B, X), {}), ("gemm_relu2", (A, B), {}), ("gemm_relu2_back", (A, B, X), {})):
+            outs = casos.roda(oc, op, args, kw)
+            torch.cuda.synchronize()
+            compara(f"{op} {kw} {M}x{N}x{K} blk {blk} tn {tn}", outs, casos.roda(s, op, args, kw))
+    finally:
+        oc.lib.jt_gemm_via(0)
+        oc.lib.jt_gemm_tn(0)
+        ops.define_blk(32)
+
+
 def test_gemm_maximos_externos(amb):
     """Row maxima supplied by the caller (the data-parallel path): two K halves with the global maxima add up to
     the full GEMM, bit for bit."""
