@@ -95,7 +95,9 @@ int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, in
 int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge,
                     int Bt, int T, int H, int D, int GA, int limite, int kid);
 int jt_softmax_ce(const void* acc, const void* e, const void* alvo, void* gm, void* gE, void* d_alvo, void* soma,
-                  int M, int V, int log2M, int kid);                                                            /* jatai_cuda.cu:1195 */
+                  int M, int V, int log2M, int kid);
+/* loss of every row of jt_softmax_ce's outputs (report only): perda[i] = d_alvo[i] / 256 + log(soma[i] / 4096), double precision */
+int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid);                                                            /* jatai_cuda.cu:1195 */
 
 /* The reference's 16-bit residual stream (opt-in ablation, no int64 specification).  Exported so that a launcher
  * that looks the symbols up keeps working; each returns cudaErrorNotSupported.  jatai_cuda.cu:1074-1086 */

@@ -782,4 +782,12 @@ __global__ void __launch_bounds__(256) k_softmax_ce(const int* __restrict__ acc,
     if (lane == 0 && linha_ok) { d_alvo[lin] = umax - ut; soma[lin] = s; }
 }
 
+// loss of every row of softmax_ce's outputs, d / 256 + log(s / 4096) in double precision (report only)
+__global__ void __launch_bounds__(256) k_perda(const int* __restrict__ d, const int* __restrict__ s, double* __restrict__ saida, int M) {
+    pdl_espera();
+    pdl_solta();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < M) saida[i] = (double)d[i] / 256 + log((double)s[i] / 4096);
+}
+
 }  // namespace jt

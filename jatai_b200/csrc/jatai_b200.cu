@@ -236,10 +236,15 @@ int jt_teste_espera(int* saiu, int kid) {
 }
 // Programmatic dependent launch of the kernels that support it (0 = plain stream order).
 int jt_pdl(int ligado) { pdl_ligado() = ligado ? 1 : 0; return 0; }
+// Clears the error record, in the order of the launches (on the stream set with jt_stream): a step that begins does not wait for the GPU.
 int jt_erro_limpa() {
-    Erro e;
-    memset(&e, 0, sizeof(e));
-    return (int)cudaMemcpyToSymbol(g_erro, &e, sizeof(Erro));
+    static void* onde[64];                 // address of the record, per device
+    int dev = 0;
+    cudaError_t c = cudaGetDevice(&dev);
+    if (c != cudaSuccess) return (int)c;
+    if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+    if (!onde[dev] && (c = cudaGetSymbolAddress(&onde[dev], g_erro)) != cudaSuccess) return (int)c;
+    return (int)cudaMemsetAsync(onde[dev], 0, sizeof(Erro), g_stream);
 }
 int jt_sincroniza() { return (int)cudaDeviceSynchronize(); }
 void jt_stream(void* st) { g_stream = (cudaStream_t)st; }
@@ -468,6 +473,13 @@ int jt_softmax_ce(const void* acc, const void* e, const void* alvo, void* gm, vo
     if (M <= 0 || V <= 0 || V % g_blk || V > 2048) return (int)cudaErrorInvalidValue;
     JT_LINHA(k_softmax_ce, V, (const int*)acc, (const int16_t*)e, (const int*)alvo, (int8_t*)gm, (int8_t*)gE, (int*)d_alvo, (int*)soma, M, V,
              log2M, kid);
+    return fim();
+}
+
+int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid) {
+    (void)kid;
+    if (M <= 0) return (int)cudaErrorInvalidValue;
+    lanca_pdl(k_perda, dim3((M + 255) / 256), dim3(256), 0, g_stream, (const int*)d_alvo, (const int*)soma, (double*)perda, M);
     return fim();
 }
 

@@ -1,0 +1,209 @@
+// Host half of the operator launcher in native code (a CPython extension): the format checks of the arguments, the allocation of the
+// outputs and the call of a C-ABI entry point, which in Python cost three to five times the launch itself.  What is wrong with an
+// argument is found and told by the Python checks of registro.py: these functions only say that something is.
+#include <Python.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+namespace {
+
+inline const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// (mantissas, exponents) of a block tensor with block length `blk`: int8, on a GPU, contiguous, exponents [R, C / blk]
+bool bloco_valido(PyObject* par, int64_t blk, int64_t* R, int64_t* C) {
+    if (!PyTuple_Check(par) || PyTuple_GET_SIZE(par) != 2) return false;
+    const at::Tensor *m = tensor(PyTuple_GET_ITEM(par, 0)), *e = tensor(PyTuple_GET_ITEM(par, 1));
+    if (!m || !e || m->scalar_type() != at::kChar || e->scalar_type() != at::kChar || !m->is_cuda() || !e->is_cuda()) return false;
+    if (m->dim() != 2 || e->dim() != 2 || !m->is_contiguous() || !e->is_contiguous()) return false;
+    *R = m->size(0);
+    *C = m->size(1);
+    return *C % blk == 0 && e->size(0) == *R && e->size(1) == *C / blk;
+}
+
+// blocos(blk, t1, t2, ...) -> (R1, C1, R2, C2, ...), or None when one of them is no block tensor
+PyObject* blocos(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n < 2) { PyErr_SetString(PyExc_TypeError, "blocos(blk, tensor pair, ...)"); return nullptr; }
+    const int64_t blk = PyLong_AsLongLong(args[0]);
+    if (blk <= 0) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "block length"); return nullptr; }
+    PyObject* r = PyTuple_New(2 * (n - 1));
+    for (Py_ssize_t i = 1; r && i < n; i++) {
+        int64_t R, C;
+        if (!bloco_valido(args[i], blk, &R, &C)) { Py_DECREF(r); Py_RETURN_NONE; }
+        PyTuple_SET_ITEM(r, 2 * (i - 1), PyLong_FromLongLong(R));
+        PyTuple_SET_ITEM(r, 2 * (i - 1) + 1, PyLong_FromLongLong(C));
+    }
+    return r;
+}
+
+// cru((acc, e)) -> (R, C), or None: int32 accumulators and int16 exponents of one shape, on a GPU, contiguous, two dimensions
+PyObject* cru(PyObject*, PyObject* par) {
+    if (!PyTuple_Check(par) || PyTuple_GET_SIZE(par) != 2) Py_RETURN_NONE;
+    const at::Tensor *a = tensor(PyTuple_GET_ITEM(par, 0)), *e = tensor(PyTuple_GET_ITEM(par, 1));
+    if (!a || !e || a->scalar_type() != at::kInt || e->scalar_type() != at::kShort || !a->is_cuda() || !e->is_cuda()) Py_RETURN_NONE;
+    if (a->dim() != 2 || a->sizes() != e->sizes() || !a->is_contiguous() || !e->is_contiguous()) Py_RETURN_NONE;
+    PyObject* r = PyTuple_New(2);
+    if (!r) return nullptr;
+    PyTuple_SET_ITEM(r, 0, PyLong_FromLongLong(a->size(0)));
+    PyTuple_SET_ITEM(r, 1, PyLong_FromLongLong(a->size(1)));
+    return r;
+}
+
+at::Tensor vazio(at::IntArrayRef forma, at::ScalarType tipo, const at::Device& dev) { return at::empty(forma, at::TensorOptions().dtype(tipo).device(dev)); }
+
+PyObject* par_de(at::Tensor a, at::Tensor b) {
+    PyObject* r = PyTuple_New(2);
+    if (!r) return nullptr;
+    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(a)));
+    PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(std::move(b)));
+    return r;
+}
+
+// novo_bloco(like, R, C, blk) / novo_cru(like, R, C): uninitialised outputs on the device of the tensor `like`
+PyObject* novo_bloco(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    const at::Tensor* como = n == 4 ? tensor(args[0]) : nullptr;
+    if (!como) { PyErr_SetString(PyExc_TypeError, "novo_bloco(tensor, R, C, blk)"); return nullptr; }
+    const int64_t R = PyLong_AsLongLong(args[1]), C = PyLong_AsLongLong(args[2]), blk = PyLong_AsLongLong(args[3]);
+    if (PyErr_Occurred()) return nullptr;
+    try {
+        return par_de(vazio({R, C}, at::kChar, como->device()), vazio({R, C / blk}, at::kChar, como->device()));
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+PyObject* novo_cru(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    const at::Tensor* como = n == 3 ? tensor(args[0]) : nullptr;
+    if (!como) { PyErr_SetString(PyExc_TypeError, "novo_cru(tensor, R, C)"); return nullptr; }
+    const int64_t R = PyLong_AsLongLong(args[1]), C = PyLong_AsLongLong(args[2]);
+    if (PyErr_Occurred()) return nullptr;
+    try {
+        return par_de(vazio({R, C}, at::kInt, como->device()), vazio({R, C}, at::kShort, como->device()));
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+// novo(like, type, d0, d1, ...): "u1" uint8, "i4" int32
+PyObject* novo(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    const at::Tensor* como = n >= 3 && n <= 6 ? tensor(args[0]) : nullptr;
+    const char* t = como ? PyUnicode_AsUTF8(args[1]) : nullptr;
+    if (!t) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "novo(tensor, type, d0, ...)"); return nullptr; }
+    int64_t d[4];
+    for (Py_ssize_t i = 2; i < n; i++) d[i - 2] = PyLong_AsLongLong(args[i]);
+    if (PyErr_Occurred()) return nullptr;
+    try {
+        return THPVariable_Wrap(vazio(at::IntArrayRef(d, n - 2), t[0] == 'u' ? at::kByte : at::kInt, como->device()));
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+
+// espaco_gemm(address of jt_gemm_ws_bytes, address of jt_stream_atual, like, M, N, K, mode) -> workspace tensor, or None where the product
+// wants none.  The workspace goes back to PyTorch's allocator right after the launch, which is safe only where the library launches on the
+// stream the allocator orders it by: on any other stream there is none, and the library takes the kernel that needs none.
+PyObject* espaco_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    const at::Tensor* como = n == 7 ? tensor(args[2]) : nullptr;
+    if (!como) { PyErr_SetString(PyExc_TypeError, "espaco_gemm(function, function, tensor, M, N, K, mode)"); return nullptr; }
+    void *fb = PyLong_AsVoidPtr(args[0]), *fs = PyLong_AsVoidPtr(args[1]);
+    int d[4];
+    for (int i = 0; i < 4; i++) d[i] = (int)PyLong_AsLong(args[3 + i]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!fb || !fs) Py_RETURN_NONE;
+    if (reinterpret_cast<void* (*)()>(fs)() != (void*)c10::cuda::getCurrentCUDAStream(como->device().index()).stream()) Py_RETURN_NONE;
+    const long long bytes = reinterpret_cast<long long (*)(int, int, int, int)>(fb)(d[0], d[1], d[2], d[3]);
+    if (bytes <= 0) Py_RETURN_NONE;
+    try {
+        return THPVariable_Wrap(vazio({bytes}, at::kByte, como->device()));
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+
+// Entry points of the library take pointers and ints (long long for element counts) and return an int: every one of them is an integer
+// argument of the x86-64 calling convention, passed in a 64-bit register or stack slot of which the callee reads what it declares, so one
+// call through a pointer type with N 64-bit arguments serves every signature with N arguments.
+typedef long long A_;
+int chama(void* f, const A_* a, int n) {
+#define C_(...) return reinterpret_cast<int (*)(__VA_ARGS__)>(f)
+    switch (n) {
+        case 1: C_(A_)(a[0]);
+        case 2: C_(A_, A_)(a[0], a[1]);
+        case 3: C_(A_, A_, A_)(a[0], a[1], a[2]);
+        case 4: C_(A_, A_, A_, A_)(a[0], a[1], a[2], a[3]);
+        case 5: C_(A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4]);
+        case 6: C_(A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5]);
+        case 7: C_(A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6]);
+        case 8: C_(A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+        case 9: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8]);
+        case 10: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9]);
+        case 11: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10]);
+        case 12: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11]);
+        case 13: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12]);
+        case 14: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13]);
+        case 15: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13], a[14]);
+        case 16: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13], a[14], a[15]);
+        case 17: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13], a[14], a[15], a[16]);
+        case 18: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13], a[14], a[15], a[16], a[17]);
+        case 19: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13], a[14], a[15], a[16], a[17], a[18]);
+        case 20: C_(A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_, A_)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13], a[14], a[15], a[16], a[17], a[18], a[19]);
+    }
+#undef C_
+    return -1;
+}
+
+PyObject *S_op, *S_trecho, *S_entradas, *S_forma;
+
+// lanca(function address, launch list, op, section, names, tensors, ints, output shape) -> (launch id, return code)
+// Records the launch ({op, trecho, entradas, forma}; `names` name the first tensors, None skips one) and calls function(pointers..., ints...,
+// launch id).  A None tensor is a null pointer.
+PyObject* lanca(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 8 || !PyList_Check(args[1]) || !PyTuple_Check(args[4]) || !PyTuple_Check(args[5]) || !PyTuple_Check(args[6])) {
+        PyErr_SetString(PyExc_TypeError, "lanca(function, launches, op, section, names, tensors, ints, shape)");
+        return nullptr;
+    }
+    PyObject *lista = args[1], *nomes = args[4], *ts = args[5], *ints = args[6];
+    const Py_ssize_t np = PyTuple_GET_SIZE(ts), ni = PyTuple_GET_SIZE(ints), nn = PyTuple_GET_SIZE(nomes);
+    if (np + ni + 1 > 20 || nn > np) { PyErr_SetString(PyExc_ValueError, "too many arguments"); return nullptr; }
+    A_ a[20];
+    for (Py_ssize_t i = 0; i < np; i++) {
+        PyObject* o = PyTuple_GET_ITEM(ts, i);
+        if (o == Py_None) { a[i] = 0; continue; }
+        const at::Tensor* t = tensor(o);
+        if (!t) { PyErr_Format(PyExc_TypeError, "argument %zd is no tensor", i); return nullptr; }
+        a[i] = (A_)(t->numel() ? t->data_ptr() : nullptr);
+    }
+    for (Py_ssize_t i = 0; i < ni; i++) a[np + i] = PyLong_AsLongLong(PyTuple_GET_ITEM(ints, i));
+    void* f = PyLong_AsVoidPtr(args[0]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!f) { PyErr_SetString(PyExc_ValueError, "null function"); return nullptr; }
+    PyObject *ent = PyDict_New(), *d = PyDict_New();
+    if (!ent || !d) { Py_XDECREF(ent); Py_XDECREF(d); return nullptr; }
+    for (Py_ssize_t i = 0; i < nn; i++)
+        if (PyTuple_GET_ITEM(nomes, i) != Py_None) PyDict_SetItem(ent, PyTuple_GET_ITEM(nomes, i), PyTuple_GET_ITEM(ts, i));
+    PyDict_SetItem(d, S_op, args[2]);
+    PyDict_SetItem(d, S_trecho, args[3]);
+    PyDict_SetItem(d, S_entradas, ent);
+    PyDict_SetItem(d, S_forma, args[7]);
+    Py_DECREF(ent);
+    const Py_ssize_t kid = PyList_GET_SIZE(lista);
+    const int falhou = PyList_Append(lista, d);
+    Py_DECREF(d);
+    if (falhou) return nullptr;
+    a[np + ni] = (A_)kid;
+    const int rc = chama(f, a, (int)(np + ni + 1));
+    if (rc == 0) Py_RETURN_NONE;
+    return Py_BuildValue("(ni)", kid, rc);
+}
+
+PyMethodDef metodos[] = {
+    {"blocos", (PyCFunction)(void (*)(void))blocos, METH_FASTCALL, "shapes of block tensors, or None"},
+    {"cru", cru, METH_O, "shape of a raw tensor, or None"},
+    {"novo_bloco", (PyCFunction)(void (*)(void))novo_bloco, METH_FASTCALL, "uninitialised block tensor"},
+    {"novo_cru", (PyCFunction)(void (*)(void))novo_cru, METH_FASTCALL, "uninitialised raw tensor"},
+    {"novo", (PyCFunction)(void (*)(void))novo, METH_FASTCALL, "uninitialised tensor"},
+    {"espaco_gemm", (PyCFunction)(void (*)(void))espaco_gemm, METH_FASTCALL, "workspace of a product, or None"},
+    {"lanca", (PyCFunction)(void (*)(void))lanca, METH_FASTCALL, "records and performs a launch; None, or (launch id, error code)"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef modulo = {PyModuleDef_HEAD_INIT, "_nativo", "host half of the operator launcher", -1, metodos, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__nativo(void) {
+    S_op = PyUnicode_InternFromString("op");
+    S_trecho = PyUnicode_InternFromString("trecho");
+    S_entradas = PyUnicode_InternFromString("entradas");
+    S_forma = PyUnicode_InternFromString("forma");
+    return PyModule_Create(&modulo);
+}

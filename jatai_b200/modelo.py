@@ -17,6 +17,7 @@ nothing but the optimiser, so all weight-gradient GEMMs are deferred to the end 
 is forward + backward with no communication, ONE MAX collective, the deferred GEMMs, ONE SUM collective, the
 optimiser.  Integer addition is associative, so the result is bit-identical to one GPU running the concatenated batch.
 """
+import contextlib
 import math
 
 import os
@@ -59,6 +60,8 @@ class Modelo:
         usa_lado = hasattr(ops, "lib") and torch.device(dev).type == "cuda"
         self._lado = torch.cuda.Stream(device=dev) if usa_lado else None
         self._pendente, self._feitos, self._k_lr_lado = None, set(), None
+        self._ev = (torch.cuda.Event(), torch.cuda.Event()) if usa_lado else None         # main -> side and side -> main, used again and again
+        self._ramo, self._presos = None, []          # the second stream in this step (or None), and what it reads until the streams join
         na_gpu = redutor is not None and hasattr(ops, "lib") and torch.device(dev).type == "cuda"
         self._ramos = [torch.cuda.Stream(device=dev) for _ in range(3)] if na_gpu else []
 
@@ -119,7 +122,7 @@ class Modelo:
         maxima are kept - because a weight gradient feeds nothing but the optimiser; all of them run after the
         backward, between the two collectives of the step (see `_gemms_adiados`)."""
         ops = self.ops
-        if self._lado is None:
+        if self._ramo is None:
             if self.redutor is None:
                 a, b = self._transpoe_par(gy, x)
                 self._grads[nome] = ops.gemm(a, b, cru=True)
@@ -129,44 +132,55 @@ class Modelo:
         # A weight gradient is a leaf of the backward graph: its two transpositions and its GEMM run on a second
         # stream, next to the dX chain, and fill SMs the small GEMMs of that chain leave idle.  Under capture the
         # second stream becomes a parallel branch of the CUDA graph.
+        with self._no_lado(gy, x):
+            self._otimiza_pendente()
+            if self.redutor is None:
+                a, b = self._transpoe_par(gy, x)
+                self._grads[nome] = ops.gemm(a, b, cru=True)
+                self._pendente = nome
+            else:       # data parallel: only the transpositions and the row maxima now, the GEMM after the exchange
+                self._adiados.append((nome, *self._transpoe_par_max(gy, x)))
+
+    @contextlib.contextmanager
+    def _no_lado(self, *lidos):
+        """The launches of the block go to the second stream, ordered after everything queued on the main one so far.  `lidos` (what they
+        read of the main stream's tensors) stays referenced until the streams join: cheaper than telling the allocator of
+        every tensor's second stream."""
+        self._presos.append(lidos)
         principal = torch.cuda.current_stream()
-        self._lado.wait_stream(principal)
-        for t in (*gy, *x):
-            t.record_stream(self._lado)
-        with torch.cuda.stream(self._lado):
-            ops.lib.jt_stream(self._lado.cuda_stream)
+        self._ev[0].record(principal)
+        self._ramo.wait_event(self._ev[0])
+        with torch.cuda.stream(self._ramo):
+            self.ops.lib.jt_stream(self._ramo.cuda_stream)
             try:
-                self._otimiza_pendente()
-                if self.redutor is None:
-                    a, b = self._transpoe_par(gy, x)
-                    self._grads[nome] = ops.gemm(a, b, cru=True)
-                    self._pendente = nome
-                else:       # data parallel: only the transpositions and the row maxima now, the GEMM after the exchange
-                    self._adiados.append((nome, *self._transpoe_par_max(gy, x)))
+                yield
             finally:
-                ops.lib.jt_stream(principal.cuda_stream)
+                self.ops.lib.jt_stream(principal.cuda_stream)
+
+    def _junta_lado(self):
+        """The main stream waits for the second one."""
+        self._ev[1].record(self._ramo)
+        torch.cuda.current_stream().wait_event(self._ev[1])
+
+    # Tokens x columns from which a step that is not being recorded uses the second stream: below it a step is bound by its launches,
+    # which another stream only adds to (512 tokens x 256 columns: 2.6 ms of launches, 1.8 ms of kernels).
+    RAMO_MINIMO = 1 << 19
+
+    def _usa_ramo(self, tokens):
+        if self._lado is None:
+            return None
+        return self._lado if tokens * self.D >= self.RAMO_MINIMO or torch.cuda.is_current_stream_capturing() else None
 
     def _pesos_transpostos(self):
         """The backward multiplies by every weight transposed (and re-quantised along the new rows).  The weights do not change
         between the start of a step and their own update, so on the CUDA launcher all those transpositions are issued at the
         start of the step on the second stream, beside the forward pass, instead of inside the backward's dependency chain.
         Returns {id of the weight's mantissa tensor: transposed block tensor} (empty where there is no second stream)."""
-        if self._lado is None:
+        if self._ramo is None:
             return {}
-        ops, principal = self.ops, torch.cuda.current_stream()
-        self._lado.wait_stream(principal)
-        wt = {}
-        with torch.cuda.stream(self._lado):
-            ops.lib.jt_stream(self._lado.cuda_stream)
-            try:
-                with self.reg.trecho("pesos transpostos"):
-                    for n, w in self.p.items():
-                        if n != "emb":
-                            wt[id(w[0])] = t = ops.transpoe(w)
-                            for x in t:
-                                x.record_stream(principal)
-            finally:
-                ops.lib.jt_stream(principal.cuda_stream)
+        with self._no_lado(), self.reg.trecho("pesos transpostos"):
+            wt = {id(w[0]): self.ops.transpoe(w) for n, w in self.p.items() if n != "emb"}
+        self._presos.append(wt)                        # the main stream reads them; they go back only after it has joined
         return wt
 
     def _otimiza_pendente(self):
@@ -264,7 +278,8 @@ class Modelo:
         alvo = alvo.reshape(-1).to(torch.int32).contiguous()
         self._grads, self._adiados = {}, []
         self._pendente, self._feitos = None, set()
-        self._k_lr_lado = k_lr if (self.redutor is None and self._lado is not None) else None
+        self._ramo, self._presos = self._usa_ramo(tok.numel()), []
+        self._k_lr_lado = k_lr if (self.redutor is None and self._ramo is not None) else None
         inicio = getattr(self.redutor, "inicio_passo", None) if treina else None
         if inicio is not None:
             inicio()                                               # data parallel: the buffer of row maxima starts the step at -128
@@ -295,11 +310,12 @@ class Modelo:
                 else:
                     g, d_alvo, soma = ops.softmax_ce(logits, alvo, log2M=self.redutor.log2_tokens(tok.numel()))
         # loss report: stays on the device; the caller converts after the step without stalling the queue
-        self._perda = perda = (d_alvo.double() / 256 + torch.log(soma.double() / 4096)).mean()
+        perda = getattr(ops, "perda", None)
+        self._perda = perda(d_alvo, soma) if perda is not None else (d_alvo.double() / 256 + torch.log(soma.double() / 4096)).mean()
         if not treina:
             return
-        if self._lado is not None and wt:
-            torch.cuda.current_stream().wait_stream(self._lado)         # the transposed weights are ready (they were, long ago)
+        if wt:
+            self._junta_lado()                                     # the transposed weights are ready (they were, long ago)
         T_ = lambda w: wt[id(w[0])] if id(w[0]) in wt else ops.transpoe(w)
         with reg.trecho("backward"):
             with reg.trecho("saida"):
@@ -325,22 +341,17 @@ class Modelo:
                         gx = self._soma_rms_back(gx, gn, n1, c1)
                         self._st(f"c{l}.grad_qkv", gq); self._st(f"c{l}.grad_residuo", gx)
                 if l in cortes:
-                    if self._lado is not None:
-                        torch.cuda.current_stream().wait_stream(self._lado)
+                    if self._ramo is not None:
+                        self._junta_lado()
                     yield l
             with reg.trecho("embedding"):
                 self._grad_peso("emb", ops.um_quente(tok, self.V), gx)
-        if self._lado is not None:
+        if self._ramo is not None:
             if self._pendente is not None and self._k_lr_lado is not None:
-                principal = torch.cuda.current_stream()
-                self._lado.wait_stream(principal)
-                with torch.cuda.stream(self._lado):
-                    ops.lib.jt_stream(self._lado.cuda_stream)
-                    try:
-                        self._otimiza_pendente()
-                    finally:
-                        ops.lib.jt_stream(principal.cuda_stream)
-            torch.cuda.current_stream().wait_stream(self._lado)          # join the weight-gradient branch
+                with self._no_lado():
+                    self._otimiza_pendente()
+            self._junta_lado()                                     # join the weight-gradient branch
+        self._presos = []
 
 
 class PassoGravado:

@@ -16,6 +16,7 @@ is the compatibility format), and optional arguments for the data-parallel step 
 CPU tensors, raises.
 """
 import ctypes
+import functools
 import math
 import os
 
@@ -32,12 +33,17 @@ _INT_FUNCS = ("jt_gemm", "jt_gemm_f", "jt_gemm_ext", "jt_max_linha", "jt_quant",
               "jt_momento", "jt_peso", "jt_momento_peso", "jt_transpoe", "jt_transpoe2", "jt_embed", "jt_um_quente", "jt_rms", "jt_rms_back", "jt_rms_back_soma", "jt_atencao",
               "jt_atencao_back", "jt_softmax_ce", "jt_erro_le", "jt_erro_limpa", "jt_sincroniza", "jt_para16", "jt_para8",
               "jt_soma16", "jt_res_estocastico", "jt_blk", "jt_blk_atual", "jt_gemm_via", "jt_gemm_tn", "jt_atencao_back_fixo", "jt_atencao_via", "jt_atencao_quant", "jt_atencao_back_quant",
-              "jt_espera_limite", "jt_teste_espera", "jt_transpoe2_max", "jt_pdl", "jt_gemm_sem_cargas", "jt_gemm_ws")
+              "jt_espera_limite", "jt_teste_espera", "jt_transpoe2_max", "jt_pdl", "jt_gemm_sem_cargas", "jt_gemm_ws", "jt_perda")
 
 
 def g_rms(D):
     """(guard bits of RMSNorm forward, of its backward) for D columns; reference ops.py:28-30."""
-    nb = D // BLK
+    return _g_rms(D, BLK)
+
+
+@functools.lru_cache(maxsize=64)
+def _g_rms(D, blk):
+    nb = D // blk
     return 2 * ((8 - int(math.log2(nb))) // 2), 14 - int(math.log2(D))
 
 
@@ -73,14 +79,6 @@ def define_blk(blk, lib=None):
         raise RuntimeError("this library has a fixed block length of 128")
 
 
-def _ptr(x):
-    if x is None:
-        return ctypes.c_void_p(0)
-    if torch.is_tensor(x):
-        return ctypes.c_void_p(x.data_ptr() if x.numel() else 0)
-    raise TypeError(type(x))
-
-
 class OpsCuda:
     """Launcher of the CUDA kernels; interface of the reference's OpsCuda (ops.py:294-515)."""
     nome = "cuda"
@@ -101,81 +99,91 @@ class OpsCuda:
             raise RuntimeError("this library has a fixed block length of 128; call ops.define_blk(128) first")
         if hasattr(self.lib, "jt_pdl"):                           # programmatic dependent launches: JT_PDL=0 switches them off
             self.lib.jt_pdl(0 if os.environ.get("JT_PDL", "1") == "0" else 1)
+        from . import _nativo
+        self._nat = _nativo
+        self._fn = {}                                             # address of every entry point used so far
+        self._ws = self._endereco("jt_gemm_ws_bytes"), self._endereco("jt_stream_atual")
         # a library with only the reference's entry points: the fused extras read as absent, callers fall back to the separate operations
         for metodo, fn in (("transpoe2", "jt_transpoe2"), ("momento_peso", "jt_momento_peso"), ("rms_back_soma", "jt_rms_back_soma"),
-                           ("max_linha", "jt_max_linha"), ("atencao_quant", "jt_atencao_quant"), ("atencao_back_quant", "jt_atencao_back_quant")):
+                           ("max_linha", "jt_max_linha"), ("atencao_quant", "jt_atencao_quant"), ("atencao_back_quant", "jt_atencao_back_quant"),
+                           ("perda", "jt_perda")):
             if not hasattr(self.lib, fn):
                 setattr(self, metodo, None)
 
     # ------------------------------------------------------------------ plumbing
-    def _lanca(self, op, fn, ponteiros, inteiros, entradas, forma, longos=()):
-        """ponteiros: tensors / None; inteiros: C ints (indices in `longos` are long long); kid goes last."""
-        kid = self.reg.registra(op, entradas, forma)
-        args = [_ptr(p) for p in ponteiros]
-        args += [ctypes.c_longlong(v) if i in longos else ctypes.c_int(v) for i, v in enumerate(inteiros)]
-        rc = getattr(self.lib, fn)(*args, ctypes.c_int(kid))
-        self.reg.depois(kid, rc)
+    # Checks, output allocation and the call itself run in the native module (csrc/nativo.cpp); what is wrong with an argument it leaves to
+    # the Python checks of the registry, which name it.
+    def _endereco(self, fn):
+        e = self._fn.get(fn)
+        if e is None:
+            e = self._fn[fn] = ctypes.cast(getattr(self.lib, fn), ctypes.c_void_p).value if hasattr(self.lib, fn) else 0
+        return e
 
-    @staticmethod
-    def _bloco_vazio(R, C, dev):
-        return torch.empty(R, C, dtype=torch.int8, device=dev), torch.empty(R, C // BLK, dtype=torch.int8, device=dev)
+    def _lanca(self, op, fn, tensores, inteiros, nomes, forma):
+        """Registers the launch and calls the entry point: pointers of `tensores` (None = null), then `inteiros`, then the launch id.
+        `nomes` name the first tensors in the launch record (None leaves one out)."""
+        reg = self.reg
+        if reg.perfil:
+            reg.cronometra(op)
+        r = self._nat.lanca(self._endereco(fn), reg.lancamentos, op, reg.onde(), nomes, tensores, inteiros, forma)
+        if r is not None:
+            reg.depois(*r)
+        elif reg.perfil or reg.vigiar:
+            reg.depois(len(reg.lancamentos) - 1, 0)
 
-    @staticmethod
-    def _cru_vazio(R, C, dev):
-        return torch.empty(R, C, dtype=torch.int32, device=dev), torch.empty(R, C, dtype=torch.int16, device=dev)
+    def _blocos(self, nomes, *tensores):
+        """(R1, C1, R2, C2, ...) of valid block tensors; raises, naming the argument, otherwise."""
+        d = self._nat.blocos(BLK, *tensores)
+        if d is None:
+            for n, t in zip(nomes, tensores):
+                self.reg.confere_bloco(n, t)
+            self.reg.falha(f"{nomes}: not block tensors (mantissa and exponent tensors on the GPU, in a tuple)")
+        return d
+
+    def _cru(self, nome, t):
+        d = self._nat.cru(t)
+        if d is None:
+            self.reg.confere_cru(nome, t)
+            self.reg.falha(f"argument '{nome}' is not a raw tensor of two dimensions")
+        return d
 
     # ------------------------------------------------------------------ GEMM family
     def _gemm(self, op, modo, A, B, X=None, duas=False, RA=None, RB=None):
-        reg = self.reg
-        reg.confere_bloco("A", A)
-        reg.confere_bloco("B", B)
+        reg, nat = self.reg, self._nat
+        if X is None:
+            M, K, N, Kb = self._blocos(("A", "B"), A, B)
+        else:
+            M, K, N, Kb, Mx, Nx = self._blocos(("A", "B", "X"), A, B, X)
         (a, ea), (b, eb) = A, B
-        M, K = a.shape
-        N = b.shape[0]
-        reg.exige(b.shape[1] == K, f"{op}: K differs, A {tuple(a.shape)} x B {tuple(b.shape)}")
-        reg.exige(M % 64 == 0 and N % 128 == 0 and K % BLK == 0,
-                  f"{op}: M must be a multiple of 64, N of 128, K of {BLK} (M={M}, N={N}, K={K})")
-        ent = dict(A=a, EA=ea, B=b, EB=eb)
-        if X is not None:
-            reg.confere_bloco("X", X)
-            reg.exige(tuple(X[0].shape) == (M, N), f"{op}: X has shape {tuple(X[0].shape)}, expected {(M, N)}")
-            ent.update(X=X[0], XE=X[1])
+        if Kb != K:
+            reg.falha(f"{op}: K differs, A {tuple(a.shape)} x B {tuple(b.shape)}")
+        if M % 64 or N % 128 or K % BLK:
+            reg.falha(f"{op}: M must be a multiple of 64, N of 128, K of {BLK} (M={M}, N={N}, K={K})")
+        if X is None:
+            x, nomes = (None, None), ("A", "EA", "B", "EB")
+        else:
+            if Mx != M or Nx != N:
+                reg.falha(f"{op}: X has shape {(Mx, Nx)}, expected {(M, N)}")
+            x, nomes = X, ("A", "EA", "B", "EB", None, None, None, None, "X", "XE")
         for nome, r, n in (("RA", RA, M), ("RB", RB, N)):
             if r is not None:
                 reg.exige(r.dtype == torch.int8 and r.is_cuda and r.is_contiguous() and r.numel() == n,
                           f"{op}: {nome} must be a contiguous int8 CUDA tensor with {n} elements")
-        dev = a.device
-        Cb = Cr = C2 = (None, None)
-        if modo == 1:
-            Cr = self._cru_vazio(M, N, dev)
-        else:
-            Cb = self._bloco_vazio(M, N, dev)
-        if duas:
-            C2 = self._bloco_vazio(M, N, dev)
-        x = X if X is not None else (None, None)
-        n_ws = self._ws_gemm(M, N, K, modo)
-        if n_ws:
-            ws = torch.empty(n_ws, dtype=torch.uint8, device=dev)
-            self._lanca(op, "jt_gemm_ws", (a, ea, b, eb, Cb[0], Cb[1], Cr[0], Cr[1], x[0], x[1], C2[0], C2[1], RA, RB, ws),
-                        (M, N, K, modo), ent, (M, N))
-        elif hasattr(self.lib, "jt_gemm_ext"):
-            self._lanca(op, "jt_gemm_ext", (a, ea, b, eb, Cb[0], Cb[1], Cr[0], Cr[1], x[0], x[1], C2[0], C2[1], RA, RB),
-                        (M, N, K, modo), ent, (M, N))
+        nada = (None, None)
+        Cb, Cr = (nada, nat.novo_cru(a, M, N)) if modo == 1 else (nat.novo_bloco(a, M, N, BLK), nada)
+        C2 = nat.novo_bloco(a, M, N, BLK) if duas else nada
+        t = (a, ea, b, eb, *Cb, *Cr, *x, *C2)
+        ws = nat.espaco_gemm(*self._ws, a, M, N, K, modo)
+        if ws is not None:
+            self._lanca(op, "jt_gemm_ws", (*t, RA, RB, ws), (M, N, K, modo), nomes, (M, N))
+        elif self._endereco("jt_gemm_ext"):
+            self._lanca(op, "jt_gemm_ext", (*t, RA, RB), (M, N, K, modo), nomes, (M, N))
         else:       # a library with only the reference's entry points (no external row maxima)
             reg.exige(RA is None and RB is None, f"{op}: this library has no jt_gemm_ext (RA / RB unsupported)")
-            self._lanca(op, "jt_gemm_f", (a, ea, b, eb, Cb[0], Cb[1], Cr[0], Cr[1], x[0], x[1], C2[0], C2[1]),
-                        (M, N, K, modo), ent, (M, N))
+            self._lanca(op, "jt_gemm_f", t, (M, N, K, modo), nomes, (M, N))
         if modo == 1:
             return Cr
         return (Cb, C2) if duas else Cb
-
-    def _ws_gemm(self, M, N, K, modo):
-        """Bytes of workspace the library wants for this product (0: none).  The workspace goes back to PyTorch's allocator right after the
-        launch, which is safe only where the library launches on the stream the allocator orders it by."""
-        lib = self.lib
-        if not hasattr(lib, "jt_gemm_ws_bytes") or (lib.jt_stream_atual() or 0) != torch.cuda.current_stream().cuda_stream:
-            return 0
-        return lib.jt_gemm_ws_bytes(M, N, K, modo)
 
     def gemm(self, A, B, cru=False, RA=None, RB=None):
         """C = A . B^T, operands blocked along K.  cru=True: raw int32 accumulators + int16 exponents.
@@ -194,159 +202,138 @@ class OpsCuda:
 
     def max_linha(self, X):
         """Row-maximum exponents (int8 [R]) of a block tensor: the RA / RB a GEMM derives from its operand."""
-        self.reg.confere_bloco("X", X)
+        self._blocos(("X",), X)
         E = X[1]
         R = torch.empty(E.shape[0], dtype=torch.int8, device=E.device)
-        self._lanca("max_linha", "jt_max_linha", (E, R), (E.shape[0], E.shape[1]), dict(E=E), (E.shape[0], 1))
+        self._lanca("max_linha", "jt_max_linha", (E, R), (E.shape[0], E.shape[1]), ("E",), (E.shape[0], 1))
         return R
 
     def transpoe(self, X):
-        self.reg.confere_bloco("X", X)
+        R, C = self._blocos(("X",), X)
         m, E = X
-        R, C = m.shape
-        self.reg.exige(R % 128 == 0 and C % 64 == 0, f"transpoe: rows {R} must be a multiple of 128 and columns {C} of 64")
-        Y = self._bloco_vazio(C, R, m.device)
-        self._lanca("transpoe", "jt_transpoe", (m, E, Y[0], Y[1]), (R, C), dict(X=m, EX=E), (C, R))
+        if R % 128 or C % 64:
+            self.reg.falha(f"transpoe: rows {R} must be a multiple of 128 and columns {C} of 64")
+        Y = self._nat.novo_bloco(m, C, R, BLK)
+        self._lanca("transpoe", "jt_transpoe", (m, E, *Y), (R, C), ("X", "EX"), (C, R))
         return Y
 
     def transpoe2(self, X1, X2):
         """(transpoe(X1), transpoe(X2)) for two block tensors with the same number of rows, in one launch (an addition of
         this library; the two operands of a weight-gradient GEMM)."""
-        self.reg.confere_bloco("X1", X1)
-        self.reg.confere_bloco("X2", X2)
-        (m1, E1), (m2, E2) = X1, X2
-        R, C1 = m1.shape
-        C2 = m2.shape[1]
-        self.reg.exige(m2.shape[0] == R, f"transpoe2: row counts differ ({R} and {m2.shape[0]})")
-        self.reg.exige(R % 128 == 0 and C1 % 64 == 0 and C2 % 64 == 0, f"transpoe2: rows {R} must be a multiple of 128 and columns {C1}, {C2} of 64")
-        Y1, Y2 = self._bloco_vazio(C1, R, m1.device), self._bloco_vazio(C2, R, m1.device)
-        self._lanca("transpoe2", "jt_transpoe2", (m1, E1, Y1[0], Y1[1], m2, E2, Y2[0], Y2[1]), (C1, C2, R), dict(X1=m1, EX1=E1, X2=m2, EX2=E2),
-                    (C1 + C2, R))
+        R, C1, R2, C2 = self._blocos(("X1", "X2"), X1, X2)
+        if R2 != R:
+            self.reg.falha(f"transpoe2: row counts differ ({R} and {R2})")
+        if R % 128 or C1 % 64 or C2 % 64:
+            self.reg.falha(f"transpoe2: rows {R} must be a multiple of 128 and columns {C1}, {C2} of 64")
+        m = X1[0]
+        Y1, Y2 = self._nat.novo_bloco(m, C1, R, BLK), self._nat.novo_bloco(m, C2, R, BLK)
+        self._lanca("transpoe2", "jt_transpoe2", (*X1, *Y1, *X2, *Y2), (C1, C2, R), ("X1", "EX1", None, None, "X2", "EX2"), (C1 + C2, R))
         return Y1, Y2
 
     def transpoe2_max(self, X1, X2, R1, R2):
         """transpoe2, and the row maxima of both results (max_linha) written into R1 [C1] / R2 [C2] - int8 views the caller has
         pre-set to -128 (data parallel: slices of the buffer of its MAX collective).  None where this library or these
         shapes do not offer it (the caller then uses transpoe2 and max_linha)."""
-        (m1, E1), (m2, E2) = X1, X2
-        R, C1 = m1.shape
-        C2 = m2.shape[1]
-        if BLK != 32 or C1 % 256 or C2 % 256 or R % 128 or m2.shape[0] != R or not hasattr(self.lib, "jt_transpoe2_max"):
+        R, C1 = X1[0].shape
+        C2 = X2[0].shape[1]
+        if BLK != 32 or C1 % 256 or C2 % 256 or R % 128 or X2[0].shape[0] != R or not hasattr(self.lib, "jt_transpoe2_max"):
             return None
-        self.reg.confere_bloco("X1", X1)
-        self.reg.confere_bloco("X2", X2)
+        self._blocos(("X1", "X2"), X1, X2)
         self.reg.exige(R1.numel() == C1 and R2.numel() == C2 and R1.dtype == torch.int8 and R2.dtype == torch.int8 and
                        R1.data_ptr() % 4 == 0 and R2.data_ptr() % 4 == 0, "transpoe2_max: row-maximum views of the wrong size, type or alignment")
-        Y1, Y2 = self._bloco_vazio(C1, R, m1.device), self._bloco_vazio(C2, R, m1.device)
-        self._lanca("transpoe2", "jt_transpoe2_max", (m1, E1, Y1[0], Y1[1], m2, E2, Y2[0], Y2[1], R1, R2), (C1, C2, R),
-                    dict(X1=m1, EX1=E1, X2=m2, EX2=E2), (C1 + C2, R))
+        m = X1[0]
+        Y1, Y2 = self._nat.novo_bloco(m, C1, R, BLK), self._nat.novo_bloco(m, C2, R, BLK)
+        self._lanca("transpoe2", "jt_transpoe2_max", (*X1, *Y1, *X2, *Y2, R1, R2), (C1, C2, R), ("X1", "EX1", None, None, "X2", "EX2"), (C1 + C2, R))
         return Y1, Y2
 
     # ------------------------------------------------------------------ block elementwise
     def quant(self, Cc):
-        self.reg.confere_cru("C", Cc)
-        acc, e = Cc
-        R, C = acc.shape
-        self.reg.exige(C % BLK == 0, f"quant: {C} columns is not a multiple of {BLK}")
-        Y = self._bloco_vazio(R, C, acc.device)
-        self._lanca("quant", "jt_quant", (acc, e, Y[0], Y[1]), (R * C // BLK,), dict(acc=acc, e=e), (R, C), longos=(0,))
+        R, C = self._cru("C", Cc)
+        if C % BLK:
+            self.reg.falha(f"quant: {C} columns is not a multiple of {BLK}")
+        Y = self._nat.novo_bloco(Cc[0], R, C, BLK)
+        self._lanca("quant", "jt_quant", (*Cc, *Y), (R * C // BLK,), ("acc", "e"), (R, C))
         return Y
 
-    def _elemento(self, op, fn, tensores, nomes):
-        for n, t in zip(nomes, tensores):
-            self.reg.confere_bloco(n, t)
-        forma = tuple(tensores[0][0].shape)
-        for n, t in zip(nomes[1:], tensores[1:]):
-            self.reg.exige(tuple(t[0].shape) == forma, f"{op}: '{n}' has shape {tuple(t[0].shape)}, expected {forma}")
-        Y = self._bloco_vazio(*forma, tensores[0][0].device)
-        ptrs = [x for t in tensores for x in t] + [Y[0], Y[1]]
-        ent = {f"{n}{s}": x for n, t in zip(nomes, tensores) for s, x in zip(("", "E"), t)}
-        self._lanca(op, fn, ptrs, (tensores[0][0].numel() // BLK,), ent, forma, longos=(0,))
-        return Y
+    def _elemento(self, op, fn, X, nomes):
+        R, C = self._blocos(nomes[:1], X)
+        Z = self._nat.novo_bloco(X[0], R, C, BLK)
+        self._lanca(op, fn, (*X, *Z), (R * C // BLK,), nomes, (R, C))
+        return Z
+
+    def _elemento2(self, op, fn, X, Y, nomes):
+        R, C, R2, C2 = self._blocos(nomes[::2], X, Y)
+        if R2 != R or C2 != C:
+            self.reg.falha(f"{op}: '{nomes[2]}' has shape {(R2, C2)}, expected {(R, C)}")
+        Z = self._nat.novo_bloco(X[0], R, C, BLK)
+        self._lanca(op, fn, (*X, *Y, *Z), (R * C // BLK,), nomes, (R, C))
+        return Z
 
     def soma(self, X, Y):
-        return self._elemento("soma", "jt_soma", (X, Y), ("x", "y"))
+        return self._elemento2("soma", "jt_soma", X, Y, ("x", "xE", "y", "yE"))
 
     def relu2(self, Hh):
-        return self._elemento("relu2", "jt_relu2", (Hh,), ("h",))
+        return self._elemento("relu2", "jt_relu2", Hh, ("h", "hE"))
 
     def relu2_back(self, Gg, Hh):
-        return self._elemento("relu2_back", "jt_relu2_back", (Gg, Hh), ("g", "h"))
+        return self._elemento2("relu2_back", "jt_relu2_back", Gg, Hh, ("g", "gE", "h", "hE"))
 
     def embed(self, W, tok):
-        self.reg.confere_bloco("W", W)
-        m, E = W
-        V, D = m.shape
+        V, D = self._blocos(("W",), W)
         M = tok.numel()
-        X = self._bloco_vazio(M, D, m.device)
-        self._lanca("embed", "jt_embed", (m, E, tok, X[0], X[1]), (M, D, V), dict(W=m, tok=tok), (M, D))
+        X = self._nat.novo_bloco(W[0], M, D, BLK)
+        self._lanca("embed", "jt_embed", (*W, tok, *X), (M, D, V), ("W", None, "tok"), (M, D))
         return X
 
     def um_quente(self, tok, V):
         M = tok.numel()
-        U = self._bloco_vazio(M, V, tok.device)
-        self._lanca("um_quente", "jt_um_quente", (tok, U[0], U[1]), (M, V), dict(tok=tok), (M, V))
+        U = self._nat.novo_bloco(tok, M, V, BLK)
+        self._lanca("um_quente", "jt_um_quente", (tok, *U), (M, V), ("tok",), (M, V))
         return U
 
     # ------------------------------------------------------------------ RMSNorm
     def rms(self, X):
-        self.reg.confere_bloco("x", X)
-        m, E = X
-        M, D = m.shape
-        self.reg.exige(D <= 2048 and D & (D - 1) == 0, f"rms: D={D} must be a power of two <= 2048")
-        G, _ = g_rms(D)
-        Y = self._bloco_vazio(M, D, m.device)
-        r = torch.empty(M, dtype=torch.int32, device=m.device)
-        emax = torch.empty(M, dtype=torch.int32, device=m.device)
-        self._lanca("rms", "jt_rms", (m, E, Y[0], Y[1], r, emax), (M, D, int(math.log2(D)), G), dict(x=m, xE=E), (M, D))
+        M, D = self._blocos(("x",), X)
+        if D > 2048 or D & (D - 1):
+            self.reg.falha(f"rms: D={D} must be a power of two <= 2048")
+        nat, m = self._nat, X[0]
+        Y, r, emax = nat.novo_bloco(m, M, D, BLK), nat.novo(m, "i4", M), nat.novo(m, "i4", M)
+        self._lanca("rms", "jt_rms", (*X, *Y, r, emax), (M, D, D.bit_length() - 1, g_rms(D)[0]), ("x", "xE"), (M, D))
         return Y, (r, emax)
 
     def rms_back(self, Gg, Y, cache):
-        self.reg.confere_bloco("g", Gg)
-        self.reg.confere_bloco("y", Y)
-        (g, gE), (y, yE) = Gg, Y
-        M, D = g.shape
-        G, GB = g_rms(D)
-        O = self._bloco_vazio(M, D, g.device)
-        self._lanca("rms_back", "jt_rms_back", (g, gE, y, yE, cache[0], cache[1], O[0], O[1]), (M, D, int(math.log2(D)), G, GB),
-                    dict(g=g, gE=gE, y=y, yE=yE, r=cache[0], emax=cache[1]), (M, D))
+        M, D, _, _ = self._blocos(("g", "y"), Gg, Y)
+        O = self._nat.novo_bloco(Gg[0], M, D, BLK)
+        self._lanca("rms_back", "jt_rms_back", (*Gg, *Y, *cache, *O), (M, D, D.bit_length() - 1, *g_rms(D)), ("g", "gE", "y", "yE", "r", "emax"), (M, D))
         return O
 
     def rms_back_soma(self, X, Gg, Y, cache):
         """soma(X, rms_back(Gg, Y, cache)) in one launch (an addition of this library; same results)."""
-        for n, t in (("x", X), ("g", Gg), ("y", Y)):
-            self.reg.confere_bloco(n, t)
-        (g, gE), (y, yE) = Gg, Y
-        M, D = g.shape
-        self.reg.exige(tuple(X[0].shape) == (M, D), f"rms_back_soma: x has shape {tuple(X[0].shape)}, expected {(M, D)}")
-        G, GB = g_rms(D)
-        O = self._bloco_vazio(M, D, g.device)
-        self._lanca("rms_back_soma", "jt_rms_back_soma", (g, gE, y, yE, cache[0], cache[1], X[0], X[1], O[0], O[1]),
-                    (M, D, int(math.log2(D)), G, GB), dict(g=g, gE=gE, y=y, yE=yE, r=cache[0], emax=cache[1], x=X[0], xE=X[1]), (M, D))
+        Mx, Dx, M, D, _, _ = self._blocos(("x", "g", "y"), X, Gg, Y)
+        if Mx != M or Dx != D:
+            self.reg.falha(f"rms_back_soma: x has shape {(Mx, Dx)}, expected {(M, D)}")
+        O = self._nat.novo_bloco(Gg[0], M, D, BLK)
+        self._lanca("rms_back_soma", "jt_rms_back_soma", (*Gg, *Y, *cache, *X, *O), (M, D, D.bit_length() - 1, *g_rms(D)),
+                    ("g", "gE", "y", "yE", "r", "emax", "x", "xE"), (M, D))
         return O
 
     # ------------------------------------------------------------------ attention
     def atencao(self, QKV, Bt, T, H):
-        self.reg.confere_bloco("qkv", QKV)
-        m, E = QKV
-        D = m.shape[1] // 3
+        M, D3 = self._blocos(("qkv",), QKV)
+        D = D3 // 3
         hd = D // H
-        self.reg.exige(m.shape[0] == Bt * T and H * hd == D and hd in (4, 16, 64) and T % 32 == 0 and T <= 1024,
-                       f"atencao: rows {m.shape[0]} (= Bt*T = {Bt * T}), head dim {hd} (4, 16 or 64), T={T} (multiple of 32, <= 1024)")
-        oacc, oe = self._cru_vazio(Bt * T, D, m.device)
-        P = torch.empty(Bt * H, T, T, dtype=torch.uint8, device=m.device)
-        self._lanca("atencao", "jt_atencao", (m, E, oacc, oe, P), (Bt, T, H, D, GA), dict(qkv=m, qkvE=E), (Bt * T, D))
-        return (oacc, oe), P
+        if M != Bt * T or H * hd != D or hd not in (4, 16, 64) or T % 32 or T > 1024:
+            self.reg.falha(f"atencao: rows {M} (= Bt*T = {Bt * T}), head dim {hd} (4, 16 or 64), T={T} (multiple of 32, <= 1024)")
+        o, P = self._nat.novo_cru(QKV[0], M, D), self._nat.novo(QKV[0], "u1", Bt * H, T, T)
+        self._lanca("atencao", "jt_atencao", (*QKV, *o, P), (Bt, T, H, D, GA), ("qkv", "qkvE"), (M, D))
+        return o, P
 
     def atencao_back(self, GO, QKV, P, Bt, T, H):
-        self.reg.confere_bloco("go", GO)
-        self.reg.confere_bloco("qkv", QKV)
-        (gm, gE), (m, E) = GO, QKV
-        D = gm.shape[1]
-        acc, e = self._cru_vazio(Bt * T, 3 * D, m.device)
-        self._lanca("atencao_back", "jt_atencao_back", (gm, gE, m, E, P, acc, e), (Bt, T, H, D, GA, int(ATENCAO_LIMITE)),
-                    dict(go=gm, goE=gE, qkv=m, qkvE=E, P=P), (Bt * T, 3 * D))
-        return acc, e
+        M, D, _, _ = self._blocos(("go", "qkv"), GO, QKV)
+        g = self._nat.novo_cru(QKV[0], Bt * T, 3 * D)
+        self._lanca("atencao_back", "jt_atencao_back", (*GO, *QKV, P, *g), (Bt, T, H, D, GA, int(ATENCAO_LIMITE)), ("go", "goE", "qkv", "qkvE", "P"),
+                    (Bt * T, 3 * D))
+        return g
 
     def _atencao_fundida(self, T, H, D):
         """Whether the library quantises the attention outputs in its own output stage for this shape (else: two launches)."""
@@ -358,12 +345,11 @@ class OpsCuda:
         if not self._atencao_fundida(T, H, D):
             oc, P = self.atencao(QKV, Bt, T, H)
             return self.quant(oc), P
-        self.reg.confere_bloco("qkv", QKV)
-        m, E = QKV
-        self.reg.exige(m.shape[0] == Bt * T, f"atencao_quant: rows {m.shape[0]} (= Bt*T = {Bt * T})")
-        O = self._bloco_vazio(Bt * T, D, m.device)
-        P = torch.empty(Bt * H, T, T, dtype=torch.uint8, device=m.device)
-        self._lanca("atencao_quant", "jt_atencao_quant", (m, E, O[0], O[1], P), (Bt, T, H, D, GA), dict(qkv=m, qkvE=E), (Bt * T, D))
+        M, _ = self._blocos(("qkv",), QKV)
+        if M != Bt * T:
+            self.reg.falha(f"atencao_quant: rows {M} (= Bt*T = {Bt * T})")
+        O, P = self._nat.novo_bloco(QKV[0], M, D, BLK), self._nat.novo(QKV[0], "u1", Bt * H, T, T)
+        self._lanca("atencao_quant", "jt_atencao_quant", (*QKV, *O, P), (Bt, T, H, D, GA), ("qkv", "qkvE"), (M, D))
         return O, P
 
     def atencao_back_quant(self, GO, QKV, P, Bt, T, H):
@@ -371,53 +357,54 @@ class OpsCuda:
         D = GO[0].shape[1]
         if not self._atencao_fundida(T, H, D):
             return self.quant(self.atencao_back(GO, QKV, P, Bt, T, H))
-        self.reg.confere_bloco("go", GO)
-        self.reg.confere_bloco("qkv", QKV)
-        (gm, gE), (m, E) = GO, QKV
-        G = self._bloco_vazio(Bt * T, 3 * D, m.device)
-        self._lanca("atencao_back_quant", "jt_atencao_back_quant", (gm, gE, m, E, P, G[0], G[1]), (Bt, T, H, D, GA, int(ATENCAO_LIMITE)),
-                    dict(go=gm, goE=gE, qkv=m, qkvE=E, P=P), (Bt * T, 3 * D))
+        self._blocos(("go", "qkv"), GO, QKV)
+        G = self._nat.novo_bloco(QKV[0], Bt * T, 3 * D, BLK)
+        self._lanca("atencao_back_quant", "jt_atencao_back_quant", (*GO, *QKV, P, *G), (Bt, T, H, D, GA, int(ATENCAO_LIMITE)),
+                    ("go", "goE", "qkv", "qkvE", "P"), (Bt * T, 3 * D))
         return G
 
     # ------------------------------------------------------------------ loss and optimiser
     def softmax_ce(self, L, alvo, log2M=None):
         """log2M: log2 of the token count the gradient is averaged over (default: rows of L; a data-parallel
         rank passes the global count)."""
-        self.reg.confere_cru("logits", L)
-        acc, e = L
-        M, V = acc.shape
+        M, V = self._cru("logits", L)
         if log2M is None:
-            self.reg.exige(M & (M - 1) == 0, f"softmax_ce: {M} rows is not a power of two")
-            log2M = int(math.log2(M))
-        self.reg.exige(V <= 2048 and V % BLK == 0, f"softmax_ce: V={V}")
-        g = self._bloco_vazio(M, V, acc.device)
-        d = torch.empty(M, dtype=torch.int32, device=acc.device)
-        s = torch.empty(M, dtype=torch.int32, device=acc.device)
-        self._lanca("softmax_ce", "jt_softmax_ce", (acc, e, alvo, g[0], g[1], d, s), (M, V, log2M), dict(acc=acc, e=e, alvo=alvo), (M, V))
+            if M & (M - 1):
+                self.reg.falha(f"softmax_ce: {M} rows is not a power of two")
+            log2M = M.bit_length() - 1
+        if V > 2048 or V % BLK:
+            self.reg.falha(f"softmax_ce: V={V}")
+        nat, acc = self._nat, L[0]
+        g, d, s = nat.novo_bloco(acc, M, V, BLK), nat.novo(acc, "i4", M), nat.novo(acc, "i4", M)
+        self._lanca("softmax_ce", "jt_softmax_ce", (*L, alvo, *g, d, s), (M, V, log2M), ("acc", "e", "alvo"), (M, V))
         return g, d, s
 
+    def perda(self, d_alvo, soma):
+        """The loss report of softmax_ce's outputs, mean over the tokens of d_alvo / 256 + log(soma / 4096) in double precision (an addition of
+        this library: the terms in one launch, then the mean)."""
+        p = torch.empty(d_alvo.numel(), dtype=torch.float64, device=d_alvo.device)
+        self._lanca("perda", "jt_perda", (d_alvo, soma, p), (d_alvo.numel(),), ("d_alvo", "soma"), (d_alvo.numel(), 1))
+        return p.mean()
+
     def momento(self, Gc, Mom):
-        self.reg.confere_cru("grad", Gc)
-        self.reg.confere_bloco("momento", Mom)
-        self.reg.exige(tuple(Gc[0].shape) == tuple(Mom[0].shape), "momento: gradient and momentum shapes differ")
-        self._lanca("momento", "jt_momento", (Gc[0], Gc[1], Mom[0], Mom[1]), (Mom[0].numel() // BLK,), dict(g=Gc[0], ge=Gc[1]),
-                    tuple(Mom[0].shape), longos=(0,))
+        d = self._cru("grad", Gc)
+        R, C = self._blocos(("momento",), Mom)
+        if d != (R, C):
+            self.reg.falha("momento: gradient and momentum shapes differ")
+        self._lanca("momento", "jt_momento", (*Gc, *Mom), (R * C // BLK,), ("g", "ge"), (R, C))
         return Mom
 
     def momento_peso(self, Gc, Mom, W, R, k, ef):
         """momento(Gc, Mom) followed by peso(W, Mom, R, k, ef) in one launch (an addition of this library; same results).
         Returns (Mom, W, R), all updated in place."""
-        self.reg.confere_cru("grad", Gc)
-        for n, t in (("W", W), ("momento", Mom), ("residuo", R)):
-            self.reg.confere_bloco(n, t)
-        self.reg.exige(tuple(Gc[0].shape) == tuple(Mom[0].shape) == tuple(W[0].shape), "momento_peso: gradient, momentum and weight shapes differ")
-        self._lanca("momento_peso", "jt_momento_peso", (Gc[0], Gc[1], Mom[0], Mom[1], W[0], W[1], R[0], R[1]),
-                    (k, int(ef), W[0].numel() // BLK), dict(g=Gc[0], ge=Gc[1]), tuple(W[0].shape), longos=(2,))
+        d = self._cru("grad", Gc)
+        Rw, Cw, Rm, Cm, _, _ = self._blocos(("W", "momento", "residuo"), W, Mom, R)
+        if not d == (Rw, Cw) == (Rm, Cm):
+            self.reg.falha("momento_peso: gradient, momentum and weight shapes differ")
+        self._lanca("momento_peso", "jt_momento_peso", (*Gc, *Mom, *W, *R), (k, int(ef), Rw * Cw // BLK), ("g", "ge"), (Rw, Cw))
         return Mom, W, R
 
     def peso(self, W, Mom, R, k, ef):
-        for n, t in (("W", W), ("momento", Mom), ("residuo", R)):
-            self.reg.confere_bloco(n, t)
-        self._lanca("peso", "jt_peso", (W[0], W[1], Mom[0], Mom[1], R[0], R[1]), (k, int(ef), W[0].numel() // BLK), dict(),
-                    tuple(W[0].shape), longos=(2,))
+        Rw, Cw, _, _, _, _ = self._blocos(("W", "momento", "residuo"), W, Mom, R)
+        self._lanca("peso", "jt_peso", (*W, *Mom, *R), (k, int(ef), Rw * Cw // BLK), (), (Rw, Cw))
         return W, R
