@@ -99,6 +99,16 @@ __device__ __forceinline__ int exp_int(int d) {
 }
 // exp(-(mx - u)/256) with the difference clamped before subtracting (mx - u may not fit in int32)
 __device__ __forceinline__ int exp_dif(int mx, int u) { return exp_int(u <= mx - 6000 ? 6000 : mx - u); }
+// exp_dif(mx, u) >> 3, the form the softmaxes use, with the cubic on p * 2^16 (|p| < 2^15 at every step): (p f) >> 15 = mulhi(p << 16, 2 f), and
+// p >> (n + 3) is 0 from n = 12 on (0 <= p < 2^15), as is the shift clamped to 31
+__device__ __forceinline__ int exp3_dif(int mx, int u) {
+    const int t = (u <= mx - 6000 ? 6000 : mx - u) * 23637, f2 = (t >> 6) & 0xFFFE;
+    int p = -1295 * 65536;
+    p = __mulhi(p, f2) * 65536 + 7556 * 65536;
+    p = __mulhi(p, f2) * 65536 - 22645 * 65536;
+    p = __mulhi(p, f2) * 65536 + 32765 * 65536;
+    return p >> min(19 + (t >> 22), 31);
+}
 
 // integer square root (ops.py:84-89: 10 Newton steps from a power of two above the root, each min(x, (x + n/x) >> 1); from
 // above they converge to floor(sqrt(n)) well inside 10 steps for every n < 2^31, and the result is clamped to >= 1).
@@ -264,6 +274,16 @@ __device__ __forceinline__ void bytes_para_float(const uint4& r, float (&f)[16])
     }
 }
 
+// low bytes of 16 words
+__device__ __forceinline__ uint4 junta16(const uint32_t (&r)[16]) {
+    uint4 p;
+    p.x = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+    p.y = __byte_perm(__byte_perm(r[4], r[5], 0x0040), __byte_perm(r[6], r[7], 0x0040), 0x5410);
+    p.z = __byte_perm(__byte_perm(r[8], r[9], 0x0040), __byte_perm(r[10], r[11], 0x0040), 0x5410);
+    p.w = __byte_perm(__byte_perm(r[12], r[13], 0x0040), __byte_perm(r[14], r[15], 0x0040), 0x5410);
+    return p;
+}
+
 // Block quantiser in fp32 for integer-valued floats below 2^24 that share the exponent e (exact: ops.py:58-72).
 // The largest magnitude gives bitlen through its exponent field; one FFMA against 1.5*2^23 rounds v * 2^-sh half
 // to even (the low byte of the result's bit pattern is the mantissa); the "one more bit" retry is decided on the
@@ -285,11 +305,19 @@ __device__ __forceinline__ int quant_f32(const float (&f)[16], int e, uint4& pac
     uint32_t r[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) r[i] = (uint32_t)__float_as_int(fmaf(f[i], sc, 12582912.0f));
-    pac.x = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
-    pac.y = __byte_perm(__byte_perm(r[4], r[5], 0x0040), __byte_perm(r[6], r[7], 0x0040), 0x5410);
-    pac.z = __byte_perm(__byte_perm(r[8], r[9], 0x0040), __byte_perm(r[10], r[11], 0x0040), 0x5410);
-    pac.w = __byte_perm(__byte_perm(r[12], r[13], 0x0040), __byte_perm(r[14], r[15], 0x0040), 0x5410);
+    pac = junta16(r);
     return E;
 }
 
+// ---------------------------------------------------------------------------------------- exact arithmetic in double precision
+// The FP64 pipe of an SM takes 64 lanes a clock, half the rate of FP32 and four times that of clz and of the conversions, and 53 bits hold
+// every intermediate of the specification (at most 30 bits) exactly.  There a rounding shift by any amount, either way, is ONE fused
+// multiply-add against 1.5 * 2^52 - half to even at integer granularity, the low word of the result being the integer - and a bit
+// length is the exponent field.
+constexpr double MAGIA_D = 6755399441055744.0;                    // 1.5 * 2^52
+__device__ __forceinline__ double int_para_d(int v) { return __hiloint2double(0x43300000, v ^ (int)0x80000000) - 4503601774854144.0; }      // (2^52 + 2^31 + v) - both
+__device__ __forceinline__ double pot2_d(int e) { return __hiloint2double((1023 + max(e, -1000)) << 20, 0); }      // 2^e, e <= 1023; below 2^-1000: 2^-1000 (rounds everything here to 0)
+__device__ __forceinline__ int bitlen_d(double x) { return max(((__double2hiint(x) >> 20) & 0x7ff) - 1022, 0); }   // of an integer-valued x; 0 for 0
+// byte k of a word, sign-extended
+__device__ __forceinline__ int byte_s(uint32_t w, int k) { return (int)(int8_t)(w >> (8 * k)); }
 }  // namespace jt
