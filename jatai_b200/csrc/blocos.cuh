@@ -242,12 +242,11 @@ __global__ void __launch_bounds__(256) k_relu2_back(const int8_t* __restrict__ g
 // per element ec = max(em + 10, eg + bitlen(g)) - 28.  ops.py:273-278.  The 16 elements of a lane, in double precision: the two roundings are
 // fused multiply-adds (the second sum leaves v + 1.5 * 2^52), the bit lengths exponent fields, the quantiser's rounding a third one.
 // Returns the block exponent; `pac` receives the mantissas.  (All int before: 72 instructions per element, a third of them at the
-// quarter rate of clz: 65 us at 16384 x 1024, now 40; the traffic's floor is 21.)
+// quarter rate of clz: 65 us at 16384 x 1024, now 36; the traffic's floor is 21.)
 template <int GL>
 __device__ __forceinline__ int momento16(const uint4& m4, int em, const int (&g)[16], const int (&eg)[16], uint4& pac, int kid, long long o) {
     const uint32_t mw[4] = {m4.x, m4.y, m4.z, m4.w};
-    double v[16];
-    int ec[16], topo = SEM_TOPO, blmax = 0;
+    int v[16], ec[16], topo = SEM_TOPO, blmax = 0;
 #pragma unroll
     for (int i = 0; i < 16; i++) {
         const double gd = int_para_d(g[i]);
@@ -255,8 +254,9 @@ __device__ __forceinline__ int momento16(const uint4& m4, int em, const int (&g)
         blmax = max(blmax, bl);
         ec[i] = max(em + 10, eg[i] + bl) - 28;
         const double a = fma(gd, pot2_d(eg[i] - ec[i]), MAGIA_D), b = fma(int_para_d(byte_s(mw[i >> 2], i & 3) * 7), pot2_d(em - ec[i]), MAGIA_D);
-        v[i] = ((a - MAGIA_D) + b) - MAGIA_D;
-        const int bv = (__double2hiint(v[i]) >> 20) & 0x7ff;
+        const double t = (a - MAGIA_D) + b;
+        v[i] = __double2loint(t);
+        const int bv = (__double2hiint(t - MAGIA_D) >> 20) & 0x7ff;
         topo = max(topo, bv == 0 ? SEM_TOPO : bv - 1022 + ec[i]);
     }
     if (blmax > 30) {                                              // (cold) a gradient at or beyond 2^30
@@ -272,13 +272,13 @@ __device__ __forceinline__ int momento16(const uint4& m4, int em, const int (&g)
     int qm = 0;
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-        q[i] = (uint32_t)__double2loint(fma(v[i], pot2_d(ec[i] - E), MAGIA_D));
+        q[i] = (uint32_t)__double2loint(fma(int_para_d(v[i]), pot2_d(ec[i] - E), MAGIA_D));
         qm = max(qm, abs((int)q[i]));
     }
     if (grupo_max<GL>(qm) > 127) {
         E += 1;
 #pragma unroll
-        for (int i = 0; i < 16; i++) q[i] = (uint32_t)__double2loint(fma(v[i], pot2_d(ec[i] - E), MAGIA_D));
+        for (int i = 0; i < 16; i++) q[i] = (uint32_t)__double2loint(fma(int_para_d(v[i]), pot2_d(ec[i] - E), MAGIA_D));
     }
     if (E < -126) return E_ZERO;
     if (E > 126) reporta(E_EXP, kid, o, E, topo);
@@ -289,7 +289,7 @@ __device__ __forceinline__ int momento16(const uint4& m4, int em, const int (&g)
 // weight step with error feedback: W <- quant(W - M 2^-k + R), R <- quant(what that rounding lost).  ops.py:280-290.  The exponents are
 // those of the blocks, so the three alignments are multiplications by one power of two each (an operand 2^20 below the
 // largest or less is rounded first: cold), and the residual, below 2^23, goes through the fp32 quantiser.
-// (57 us at 16384 x 1024 with integer shifts throughout, now 28.)
+// (57 us at 16384 x 1024 with integer shifts throughout, now 25.)
 template <int GL>
 __device__ __forceinline__ void peso16(const uint4& w4, int ew, const uint4& m4, int em, const uint4& r4, int er, bool ef, uint4& pw, int& Ew, uint4& pr, int& Er,
                                        int kid, long long o) {
@@ -355,7 +355,7 @@ __device__ __forceinline__ void peso16(const uint4& w4, int ew, const uint4& m4,
 }
 
 template <int BLK>
-__global__ void __launch_bounds__(256) k_momento(const int* __restrict__ gacc, const int16_t* __restrict__ ge, int8_t* __restrict__ Mm,
+__global__ void __launch_bounds__(128, 5) k_momento(const int* __restrict__ gacc, const int16_t* __restrict__ ge, int8_t* __restrict__ Mm,
                                                  int8_t* __restrict__ ME, long long n16, int kid) {
     JT_FIO16
     int g[16], eg[16];
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(256) k_peso(int8_t* __restrict__ Wm, int8_t* _
 // momentum and weight step of the same 16 elements in one launch (the optimiser of a weight is always this pair):
 // k_momento followed by k_peso on the momentum just written, which stays in registers.
 template <int BLK>
-__global__ void __launch_bounds__(256) k_momento_peso(const int* __restrict__ gacc, const int16_t* __restrict__ ge, int8_t* __restrict__ Mm,
+__global__ void __launch_bounds__(128, 5) k_momento_peso(const int* __restrict__ gacc, const int16_t* __restrict__ ge, int8_t* __restrict__ Mm,
                                                       int8_t* __restrict__ ME, int8_t* __restrict__ Wm, int8_t* __restrict__ WE,
                                                       int8_t* __restrict__ Rm, int8_t* __restrict__ RE, int k_lr, int ef, long long n16, int kid) {
     pdl_espera();
@@ -451,72 +451,6 @@ __global__ void __launch_bounds__(256) k_um_quente(const int* __restrict__ tok, 
     if (c % BLK == 0) UE[(size_t)lin * (V / BLK) + c / BLK] = 0;
 }
 
-// [R,C] blocked along C -> [C,R] blocked along R; the new blocks span BLK rows of one column, so every
-// element brings its own exponent and the block is quantised again.  ops.py:121-123
-// Tile: 128 rows x 64 columns through shared memory; a thread then owns 16 consecutive rows of one column.
-template <int BLK>
-__global__ void __launch_bounds__(256) k_transpoe(const int8_t* __restrict__ X, const int8_t* __restrict__ EX, int8_t* __restrict__ Y,
-                                                  int8_t* __restrict__ EY, int R, int C, int kid) {
-    constexpr int TR = 128, TC = 64, NE = (TC + BLK - 1) / BLK;     // exponent columns a tile touches
-    __shared__ int8_t tile[TC][TR + 16];                            // stored transposed: [column][row]
-    __shared__ int8_t et[TR][NE];
-    const int r0 = blockIdx.y * TR, c0 = blockIdx.x * TC;
-    const int tid = threadIdx.x;
-    // load: 128 rows x 64 B = 512 x 16 B, two per thread, scattered transposed into shared memory
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const int idx = tid + it * 256, lr = idx / 4, lc = (idx % 4) * 16;
-        const uint4 v = *reinterpret_cast<const uint4*>(X + (size_t)(r0 + lr) * C + c0 + lc);
-        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 16; k++) tile[lc + k][lr] = (int8_t)(u[k >> 2] >> (8 * (k & 3)));
-    }
-    for (int i = tid; i < TR * NE; i += 256) et[i / NE][i % NE] = EX[(size_t)(r0 + i / NE) * (C / BLK) + c0 / BLK + i % NE];
-    __syncthreads();
-    // 64 columns x 8 row-groups of 16 = 512 tasks; consecutive lanes take consecutive row-groups of a column
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const int idx = tid + it * 256, col = idx / 8, rg = idx % 8;
-        int v[16], e[16], q[16];
-        const uint4 w4 = *reinterpret_cast<const uint4*>(&tile[col][rg * 16]);
-        const uint32_t u[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            v[k] = (int)(int8_t)(u[k >> 2] >> (8 * (k & 3)));
-            e[k] = et[rg * 16 + k][(c0 % BLK + col) / BLK];
-        }
-        const long long o = (long long)(c0 + col) * R + r0 + rg * 16;
-        const int Eo = quant_geral<16, BLK / 16>(v, e, q, kid, o);
-        grava16(Y + o, q);
-        if (rg % (BLK / 16) == 0) EY[(size_t)(c0 + col) * (R / BLK) + (r0 + rg * 16) / BLK] = (int8_t)Eo;
-    }
-}
-
-// Transposition for block 32, wide tiles: TR (32, 64 or 128) rows x 256 columns per CTA of 2 TR threads; the launcher
-// takes the tallest tile that still gives every SM a CTA (and, for the smallest matrices, a thread per column instead
-// of per word: CPT = 1).  A thread owns a 32-row block of 4
-// adjacent columns (one 32-bit word per row) and quantises the 4 new blocks without leaving its registers.
-// The quantiser runs in fp32, exactly: a mantissa times 2^(e - eref) is exact in fp32, the largest magnitude gives
-// top = max(e + bitlen(v)) through its exponent field, and one FFMA against 1.5*2^23 rounds v * 2^(e - E) half to
-// even (|result| <= 127, inside the window).  A transposed block can never need the "one more bit" retry
-// (|m| <= 127 going in).  Blocks whose exponents are more than 100 apart take an integer path.
-constexpr int T32_PW = 256 / 4 + 1;
-// integer path of k_transpoe32 for one column of a block whose exponents are too far apart for fp32 (cold)
-__device__ __noinline__ int transpoe32_lento(const uint32_t (*tile)[T32_PW], const int8_t (*et)[8], int rb, int cw, int k, int8_t* dst,
-                                              int8_t* Edst, int kid, long long idx0) {
-    int v[32], e[32], q[32];
-#pragma unroll
-    for (int i = 0; i < 32; i++) {
-        v[i] = (int)(int8_t)(tile[rb * 32 + i][cw] >> (8 * k));
-        e[i] = et[rb * 32 + i][cw >> 3];
-    }
-    const int Eo = quant_geral<32, 1>(v, e, q, kid, idx0);
-#pragma unroll
-    for (int i4 = 0; i4 < 8; i4++) reinterpret_cast<uint32_t*>(dst)[i4] = junta4(q[4 * i4], q[4 * i4 + 1], q[4 * i4 + 2], q[4 * i4 + 3]);
-    *Edst = (int8_t)Eo;
-    return Eo;
-}
-
 // per-byte signed maximum into a 4-byte-aligned word of an int8 array
 __device__ __forceinline__ void max4_atomico(int8_t* p, uint32_t meu) {
     unsigned* w = reinterpret_cast<unsigned*>(p);
@@ -530,104 +464,149 @@ __device__ __forceinline__ void max4_atomico(int8_t* p, uint32_t meu) {
     }
 }
 
-template <int TR, int CPT>
-__device__ __forceinline__ void transpoe32_corpo(const int8_t* __restrict__ X, const int8_t* __restrict__ EX, int8_t* __restrict__ Y,
-                                                 int8_t* __restrict__ EY, int R, int C, int kid, int8_t* __restrict__ RM = nullptr) {
+// [R,C] blocked along C -> [C,R] blocked along R; the new blocks span BLK rows of one column, so every element brings its own exponent and the
+// block is quantised again.  ops.py:121-123
+//
+// A warp takes 32 rows x 128 columns straight from global memory: a lane loads the word of its 4 columns in every row (32 coalesced 128-byte
+// loads in flight per warp, no shared memory, no barrier), which is four 32-element columns; the exponents, a row per lane, travel by
+// shuffles.  The quantiser runs in fp32, exactly: a mantissa times 2^(e - eref) is exact, the largest magnitude gives
+// top = max(e + bitlen(v)) through its exponent field, and one FFMA against 1.5*2^23 rounds v * 2^(e - E) half to even
+// (|result| <= 127, inside the window).  A transposed block can never need the "one more bit" retry (|m| <= 127 going in).  Rows whose
+// exponents are more than 100 apart take integers.  Block 128: the four warps of a CTA (128 rows) exchange their columns' tops first.
+// CPT = 4: a lane does its 4 columns; CPT = 1, for matrices that would leave SMs idle: four warps share the 32 x 128 piece, a column each.
+// (Tiles staged in shared memory before, two shared loads per element: 16384 x (4096 + 1024) 95 -> 66 us, block 128 154 -> 50 us; 128 x 128
+// 6.4 -> 2.1 us.)
+struct ArgsTransp { const int8_t* X; const int8_t* EX; int8_t* Y; int8_t* EY; int C; int8_t* RM; };
+
+// (cold) the 32 rows of one column in integers, read again: e + bitlen of the largest / the mantissas for the exponent Eo
+__device__ __noinline__ int transpoe_topo_lento(const int8_t* X, const int8_t* E, int C, int nbx) {
+    int topo = SEM_TOPO;
+    for (int i = 0; i < 32; i++)
+        if (X[(size_t)i * C] != 0) topo = max(topo, (int)E[(size_t)i * nbx] + bitlen(X[(size_t)i * C]));
+    return topo;
+}
+__device__ __noinline__ void transpoe_grava_lento(const int8_t* X, const int8_t* E, int C, int nbx, int Eo, int8_t* dst) {
+    for (int i = 0; i < 32; i++) {
+        const int v = X[(size_t)i * C];
+        dst[i] = (int8_t)(Eo == E_ZERO || v == 0 ? 0 : desloca(v, Eo - (int)E[(size_t)i * nbx]));
+    }
+}
+
+template <int BLK, int CPT>
+__device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int c0, int R, int kid) {
     pdl_espera();
     pdl_solta();
-    static_assert(CPT == 4 || CPT == 1, "a thread owns the 4 columns of a word or one of them");
-    constexpr int TC = 256, PW = T32_PW, NT = 8 * TR / CPT, NPAR = (TR / 32) * 8;
-    __shared__ uint32_t tile[TR][PW];
-    __shared__ __align__(4) int8_t et[TR][8];
-    __shared__ float fA[TR][8];                   // 2^(e - largest exponent of the row's 32-row block), per 32-column block
-    __shared__ int eref_s[NPAR];                  // that largest exponent; bit 30 set: exponents too far apart for fp32
-    const int r0 = blockIdx.y * TR, c0 = blockIdx.x * TC;
-    const int tid = threadIdx.x;
-    const int nbx = C / 32, nby = R / 32;
+    __shared__ int topos[BLK == 128 ? 4 : 1][BLK == 128 ? 128 : 1];
+    // block 32: a CTA is 32 rows (CPT = 1) or 128; block 128 always 128, its four 32-row groups belong together
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rg = CPT == 1 && BLK == 32 ? 0 : wid & 3, k0 = CPT == 1 ? (BLK == 32 ? wid : wid >> 2) : 0;
+    const int C = A.C, nbx = C / BLK, nby = R / BLK, col0 = c0 + 4 * lane, lin0 = r0 + rg * 32;
+    const bool dentro = col0 < C;
+    // lane r: the exponents of row r, one byte per 32-column block of the piece (block 128: the same byte four times)
+    uint32_t ew;
+    {
+        const int8_t* pe = A.EX + (size_t)(lin0 + lane) * nbx + c0 / BLK;
+        if (BLK == 128) ew = (uint32_t)(uint8_t)pe[0] * 0x01010101u;
+        else if ((nbx & 3) == 0 && ((uintptr_t)A.EX & 3) == 0) ew = *reinterpret_cast<const uint32_t*>(pe);
+        else {
+            ew = 0;
 #pragma unroll
-    for (int k = 0; k < TR * 16 / NT; k++) {
-        const int idx = tid + NT * k, lr = idx >> 4, c16 = idx & 15;
-        const uint4 v = *reinterpret_cast<const uint4*>(X + (size_t)(r0 + lr) * C + c0 + c16 * 16);
-        tile[lr][c16 * 4] = v.x; tile[lr][c16 * 4 + 1] = v.y; tile[lr][c16 * 4 + 2] = v.z; tile[lr][c16 * 4 + 3] = v.w;
-    }
-    if (tid < 2 * TR) {
-        const int lr = tid >> 1, k4 = (tid & 1) * 4;
-        *reinterpret_cast<uint32_t*>(&et[lr][k4]) = *reinterpret_cast<const uint32_t*>(EX + (size_t)(r0 + lr) * nbx + c0 / 32 + k4);
-    }
-    __syncthreads();
-    // scales of the rows: a warp per (32-row block, 32-column block), a lane per row.  Rows of all-zero blocks do not count
-    // for the spread (their mantissas are zero whatever the scale).
-    for (int p = tid >> 5; p < NPAR; p += NT / 32) {
-        const int rb = p >> 3, cb = p & 7, i = tid & 31;
-        const int e = et[rb * 32 + i][cb];
-        const int eref = __reduce_max_sync(0xffffffffu, e);
-        const int emin = __reduce_min_sync(0xffffffffu, e == E_ZERO ? 127 : e);
-        fA[rb * 32 + i][cb] = __int_as_float(max(127 + e - eref, 0) << 23);
-        if (i == 0) eref_s[p] = (eref & 0xffff) | (eref - emin > 100 ? 1 << 30 : 0);
-    }
-    __syncthreads();
-    // word column, 32-row block and (CPT = 1: small matrices, four times the threads) the byte of the word
-    const int cw = tid & 63, rb = CPT == 4 ? tid >> 6 : tid >> 8, k_meu = (tid >> 6) & 3;
-    const int er = eref_s[rb * 8 + (cw >> 3)];
-    const int eref = (int)(int16_t)(er & 0xffff);
-    const bool largo = (er >> 30) & 1;                              // spread too wide for the fp32 path
-    const float* fa = &fA[rb * 32][cw >> 3];
-    uint32_t emax4 = 0x80808080u;                                   // the new exponents of this thread's columns, -128 where it has none
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        if (CPT == 1 && k != k_meu) continue;
-        const size_t col = (size_t)(c0 + 4 * cw + k);
-        int8_t* dst = Y + col * R + r0 + rb * 32;
-        int8_t* Edst = EY + col * nby + (r0 + rb * 32) / 32;
-        if (largo) {
-            const int Eo = transpoe32_lento(tile, et, rb, cw, k, dst, Edst, kid, (long long)col * R + r0 + rb * 32);
-            emax4 = (emax4 & ~(0xffu << (8 * k))) | ((uint32_t)(uint8_t)(int8_t)Eo << (8 * k));
-            continue;
+            for (int b = 0; b < 4; b++) ew |= (uint32_t)(uint8_t)(c0 / 32 + b < nbx ? pe[b] : (int8_t)E_ZERO) << (8 * b);
         }
-        float t[32], mx = 0.f;
+    }
+    uint32_t w[32];                                                // sign bits flipped: byte b stands for b + 128
+    {
+        const int8_t* px = A.X + (size_t)lin0 * C + (dentro ? col0 : 0);
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
-            t[i] = (float)(int)(int8_t)(tile[rb * 32 + i][cw] >> (8 * k)) * fa[8 * i];     // the words stay in shared memory: registers hold t
-            mx = fmaxf(mx, fabsf(t[i]));
+        for (int i = 0; i < 32; i++, px += C) w[i] = *reinterpret_cast<const uint32_t*>(px) ^ 0x80808080u;
+    }
+    uint32_t mx4;
+    if (BLK == 128) mx4 = (uint32_t)(uint8_t)(int8_t)__reduce_max_sync(FULL, (int)(int8_t)ew) * 0x01010101u;
+    else {
+        mx4 = 0;
+#pragma unroll
+        for (int b = 0; b < 4; b++) mx4 |= (uint32_t)(uint8_t)(int8_t)__reduce_max_sync(FULL, (int)(int8_t)(ew >> (8 * b))) << (8 * b);
+    }
+    // how far below the largest exponent of its block this row's are (0..254); beyond 100, all-zero blocks (-127) apart, fp32 does not reach
+    uint32_t d4 = __vsub4(mx4, ew);
+    const uint32_t longe = __reduce_or_sync(FULL, __vcmpgtu4(d4, 0x64646464u) & ~__vcmpeq4(ew, 0x81818181u));
+    const int bl = lane >> 3, eref = (int)(int8_t)(mx4 >> (8 * bl));
+    const bool largo = (longe >> (8 * bl)) & 1;
+    d4 = __vminu4(d4, 0x7f7f7f7fu);
+    float fa[32];                                                  // 2^(e - eref)
+#pragma unroll
+    for (int i = 0; i < 32; i++) fa[i] = __int_as_float(0x3f800000 - (int)((__shfl_sync(FULL, d4, i) >> (8 * bl)) & 0xff) * 0x800000);
+    auto valor = [&](int i, int k) {                               // element (row i, column k) times 2^(e - eref), exact
+        return (__uint_as_float(__byte_perm(w[i], 0x4B400000u, 0x7650 + k)) - 12583040.0f) * fa[i];
+    };
+    auto topo_de = [&](float mx) { return mx == 0.f ? SEM_TOPO : eref + (__float_as_int(mx) >> 23) - 126; };       // e + bitlen of the largest
+    const int8_t *px0 = A.X + (size_t)lin0 * C + (dentro ? col0 : 0), *pe0 = A.EX + (size_t)lin0 * nbx + (dentro ? col0 : 0) / BLK;      // (cold path)
+    uint32_t emax4 = 0x80808080u;                                  // the new exponents of this lane's columns, -128 where it has none
+    if (BLK == 128) {
+        float mx[CPT];
+#pragma unroll
+        for (int kk = 0; kk < CPT; kk++) mx[kk] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+#pragma unroll
+            for (int kk = 0; kk < CPT; kk++) mx[kk] = fmaxf(mx[kk], fabsf(valor(i, k0 + kk)));
+#pragma unroll
+        for (int kk = 0; kk < CPT; kk++) topos[rg][4 * lane + k0 + kk] = largo ? transpoe_topo_lento(px0 + k0 + kk, pe0, C, nbx) : topo_de(mx[kk]);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 32; i++) asm volatile("" : "+r"(w[i]));          // the values are computed again below rather than kept: 128 registers
+    }
+#pragma unroll
+    for (int kk = 0; kk < CPT; kk++) {
+        const int k = k0 + kk;
+        float t[32];
+        int topo;
+        if (BLK == 128) {
+            topo = max(max(topos[0][4 * lane + k], topos[1][4 * lane + k]), max(topos[2][4 * lane + k], topos[3][4 * lane + k]));
+#pragma unroll
+            for (int i = 0; i < 32; i++) t[i] = valor(i, k);
+        } else {
+            float mx = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; i++) { t[i] = valor(i, k); mx = fmaxf(mx, fabsf(t[i])); }
+            topo = topo_de(mx);
+            if (largo) topo = transpoe_topo_lento(px0 + k, pe0, C, nbx);
         }
-        const int expo = (__float_as_int(mx) >> 23) - 127;          // floor(log2 mx); mx is a normal number or 0 here
-        int Eo = eref + expo + 1 - 7;
-        const bool morto = mx == 0.f || Eo < -126;
-        if (!morto && Eo > 126) reporta(E_EXP, kid, (long long)col * R + r0 + rb * 32, Eo, eref);
-        const float B = morto ? 0.f : __int_as_float((127 + 6 - expo) << 23);
+        const size_t col = (size_t)col0 + k;
+        int Eo = topo - 7;
+        const bool morto = Eo < -126;
+        if (dentro && Eo > 126) reporta(E_EXP, kid, (long long)col * R + lin0, Eo, eref);
+        const float B = morto ? 0.f : __int_as_float((127 + max(min(eref - Eo, 127), -120)) << 23);
         if (morto) Eo = E_ZERO;
-        uint32_t saida[8];
+        if (dentro) {
+            int8_t* dst = A.Y + col * R + lin0;
+            if (largo) transpoe_grava_lento(px0 + k, pe0, C, nbx, Eo, dst);
+            else {
+                uint32_t a[16], b[16];
 #pragma unroll
-        for (int i4 = 0; i4 < 8; i4++) {
-            uint32_t r[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) r[j] = (uint32_t)__float_as_int(fmaf(t[4 * i4 + j], B, 12582912.0f));
-            saida[i4] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+                for (int i = 0; i < 16; i++) {
+                    a[i] = (uint32_t)__float_as_int(fmaf(t[i], B, 12582912.0f));
+                    b[i] = (uint32_t)__float_as_int(fmaf(t[16 + i], B, 12582912.0f));
+                }
+                reinterpret_cast<uint4*>(dst)[0] = junta16(a);
+                reinterpret_cast<uint4*>(dst)[1] = junta16(b);
+            }
+            if (BLK == 32 || rg == 0) A.EY[col * nby + lin0 / BLK] = (int8_t)Eo;
         }
-        reinterpret_cast<uint4*>(dst)[0] = make_uint4(saida[0], saida[1], saida[2], saida[3]);
-        reinterpret_cast<uint4*>(dst)[1] = make_uint4(saida[4], saida[5], saida[6], saida[7]);
-        *Edst = (int8_t)Eo;
         emax4 = (emax4 & ~(0xffu << (8 * k))) | ((uint32_t)(uint8_t)(int8_t)Eo << (8 * k));
     }
     // row maxima of the transposed tensor (what a GEMM aligns its rows to): the caller pre-set RM to -128
-    if (RM != nullptr) max4_atomico(RM + c0 + 4 * cw, emax4);
+    if (A.RM != nullptr && dentro) max4_atomico(A.RM + col0, emax4);
 }
 
-template <int TR, int CPT = 4>
-__global__ void __launch_bounds__(8 * TR / CPT, 768 / (8 * TR / CPT)) k_transpoe32(const int8_t* __restrict__ X, const int8_t* __restrict__ EX,
-                                                                                   int8_t* __restrict__ Y, int8_t* __restrict__ EY, int R, int C,
-                                                                                   int kid) {
-    transpoe32_corpo<TR, CPT>(X, EX, Y, EY, R, C, kid);
-}
-
-// Two transpositions of matrices with the same number of rows in one launch (the two operands of a weight-gradient
-// GEMM): blockIdx.z picks the matrix, the grid is as wide as the wider one.
-struct ArgsTransp { const int8_t* X; const int8_t* EX; int8_t* Y; int8_t* EY; int C; int8_t* RM; };
-template <int TR, int CPT = 4>
-__global__ void __launch_bounds__(8 * TR / CPT, 768 / (8 * TR / CPT)) k_transpoe32_par(ArgsTransp a0, ArgsTransp a1, int R, int kid) {
-    const ArgsTransp a = blockIdx.z ? a1 : a0;
-    if ((int)blockIdx.x * 256 >= a.C) return;
-    transpoe32_corpo<TR, CPT>(a.X, a.EX, a.Y, a.EY, R, a.C, kid, a.RM);
+// one or two matrices with the same number of rows (the operands of a weight-gradient GEMM) in one launch: CTAs 0 .. n0-1 take the first
+template <int BLK, int CPT>
+__global__ void __launch_bounds__(CPT == 1 && BLK == 128 ? 512 : 128, CPT == 1 && BLK == 128 ? 1 : 4) k_transpoe(const ArgsTransp a0, const ArgsTransp a1, int n0, int R, int kid) {
+    constexpr int TR = CPT == 1 && BLK == 32 ? 32 : 128;           // rows of a CTA
+    const bool segunda = (int)blockIdx.x >= n0;
+    const ArgsTransp A = segunda ? a1 : a0;
+    const int t = (int)blockIdx.x - (segunda ? n0 : 0), nx = (A.C + 127) / 128;
+    transpoe_corpo<BLK, CPT>(A, t / nx * TR, t % nx * 128, R, kid);
 }
 
 // RMSNorm without gain, one warp per row, NP*512 >= D columns held in registers.  ops.py:153-165

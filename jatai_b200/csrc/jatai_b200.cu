@@ -36,6 +36,7 @@ static int g_tn = 0;                 // tile width of the tensor-core GEMM: 0 au
 constexpr int N_SM = 148;             // B200
 static int fim() { return (int)cudaGetLastError(); }
 static unsigned nblocos16(long long n16) { return (unsigned)((n16 + 255) / 256); }
+static unsigned nblocos_128(long long n16) { return (unsigned)((n16 + 127) / 128); }
 static unsigned nblocos16u(long long n16, int U) { return (unsigned)((n16 + 256LL * U - 1) / (256LL * U)); }      // U chunks per thread
 
 template <int BLK, int MODO, int VIA, int TNv>
@@ -347,8 +348,8 @@ int jt_relu2_back(const void* gm, const void* gE, const void* hm, const void* hE
 }
 int jt_momento(const void* gacc, const void* ge, void* Mm, void* ME, long long nblocos, int kid) {
     const long long n16 = JT_N16;
-    if (g_blk == 32) k_momento<32><<<nblocos16(n16), 256, 0, g_stream>>>((const int*)gacc, (const int16_t*)ge, (int8_t*)Mm, (int8_t*)ME, n16, kid);
-    else k_momento<128><<<nblocos16(n16), 256, 0, g_stream>>>((const int*)gacc, (const int16_t*)ge, (int8_t*)Mm, (int8_t*)ME, n16, kid);
+    if (g_blk == 32) k_momento<32><<<nblocos_128(n16), 128, 0, g_stream>>>((const int*)gacc, (const int16_t*)ge, (int8_t*)Mm, (int8_t*)ME, n16, kid);
+    else k_momento<128><<<nblocos_128(n16), 128, 0, g_stream>>>((const int*)gacc, (const int16_t*)ge, (int8_t*)Mm, (int8_t*)ME, n16, kid);
     return fim();
 }
 int jt_peso(void* Wm, void* WE, const void* Mm, const void* ME, void* Rm, void* RE, int k_lr, int ef, long long nblocos, int kid) {
@@ -363,49 +364,41 @@ int jt_momento_peso(const void* gacc, const void* ge, void* Mm, void* ME, void* 
                     long long nblocos, int kid) {
     const long long n16 = JT_N16;
 #define ARGS (const int*)gacc, (const int16_t*)ge, (int8_t*)Mm, (int8_t*)ME, (int8_t*)Wm, (int8_t*)WE, (int8_t*)Rm, (int8_t*)RE, k_lr, ef, n16, kid
-    if (g_blk == 32) lanca_pdl(k_momento_peso<32>, dim3(nblocos16(n16)), dim3(256), 0, g_stream, ARGS);
-    else lanca_pdl(k_momento_peso<128>, dim3(nblocos16(n16)), dim3(256), 0, g_stream, ARGS);
+    if (g_blk == 32) lanca_pdl(k_momento_peso<32>, dim3(nblocos_128(n16)), dim3(128), 0, g_stream, ARGS);
+    else lanca_pdl(k_momento_peso<128>, dim3(nblocos_128(n16)), dim3(128), 0, g_stream, ARGS);
 #undef ARGS
     return fim();
 }
+}  // extern "C"
+static int transpoe_impl(const ArgsTransp& a0, const ArgsTransp& a1, int R, int kid) {
+    auto pecas = [&](const ArgsTransp& a) { return a.X ? (a.C + 127) / 128 * (R / 128) : 0; };
+    const int n0 = pecas(a0), n = n0 + pecas(a1);              // 128 x 128 pieces
+    // fewer than three (block 128: two) per SM: four warps share the columns of every 32 rows
+    const bool poucas = n < (g_blk == 32 ? 3 : 2) * N_SM;
+    if (g_blk == 32) {
+        if (poucas) lanca_pdl(k_transpoe<32, 1>, dim3(4 * n), dim3(128), 0, g_stream, a0, a1, 4 * n0, R, kid);
+        else lanca_pdl(k_transpoe<32, 4>, dim3(n), dim3(128), 0, g_stream, a0, a1, n0, R, kid);
+    } else {
+        if (poucas) lanca_pdl(k_transpoe<128, 1>, dim3(n), dim3(512), 0, g_stream, a0, a1, n0, R, kid);
+        else lanca_pdl(k_transpoe<128, 4>, dim3(n), dim3(128), 0, g_stream, a0, a1, n0, R, kid);
+    }
+    return fim();
+}
+extern "C" {
 int jt_transpoe(const void* X, const void* EX, void* Y, void* EY, int R, int C, int kid) {
     if (R <= 0 || C <= 0 || R % 128 || C % 64 || C % g_blk) return (int)cudaErrorInvalidValue;
-    if (g_blk == 32 && C % 256 == 0 && ((uintptr_t)EX & 3) == 0) {
-        const long long t128 = (long long)(C / 256) * (R / 128);
-#define ARGS (const int8_t*)X, (const int8_t*)EX, (int8_t*)Y, (int8_t*)EY, R, C, kid
-        if (t128 >= 148) lanca_pdl(k_transpoe32<128>, dim3(dim3(C / 256, R / 128)), dim3(256), 0, g_stream, ARGS);
-        else if (2 * t128 >= 148) lanca_pdl(k_transpoe32<64>, dim3(dim3(C / 256, R / 64)), dim3(128), 0, g_stream, ARGS);
-        else if (4 * t128 >= 296) lanca_pdl(k_transpoe32<32>, dim3(dim3(C / 256, R / 32)), dim3(64), 0, g_stream, ARGS);
-        else lanca_pdl(k_transpoe32<32, 1>, dim3(dim3(C / 256, R / 32)), dim3(256), 0, g_stream, ARGS);
-#undef ARGS
-        return fim();
-    }
-    const dim3 grade(C / 64, R / 128);
-    if (g_blk == 32) k_transpoe<32><<<grade, 256, 0, g_stream>>>((const int8_t*)X, (const int8_t*)EX, (int8_t*)Y, (int8_t*)EY, R, C, kid);
-    else k_transpoe<128><<<grade, 256, 0, g_stream>>>((const int8_t*)X, (const int8_t*)EX, (int8_t*)Y, (int8_t*)EY, R, C, kid);
-    return fim();
+    return transpoe_impl({(const int8_t*)X, (const int8_t*)EX, (int8_t*)Y, (int8_t*)EY, C, nullptr}, {}, R, kid);
 }
 // the pair of transpositions; RM1 / RM2 (optional, both or none): int8 [C1] / [C2], pre-set to -128 by the caller, receive the
 // row maxima of the exponents of Y1 / Y2 (what jt_max_linha would compute from EY1 / EY2)
 static int transpoe2_impl(const void* X1, const void* EX1, void* Y1, void* EY1, const void* X2, const void* EX2, void* Y2, void* EY2, int C1, int C2,
                           int R, void* RM1, void* RM2, int kid) {
-    if (R <= 0 || C1 <= 0 || C2 <= 0 || R % 128) return (int)cudaErrorInvalidValue;
+    if (R <= 0 || C1 <= 0 || C2 <= 0 || R % 128 || C1 % 64 || C2 % 64 || C1 % g_blk || C2 % g_blk) return (int)cudaErrorInvalidValue;
     const bool com_max = RM1 != nullptr || RM2 != nullptr;
     if (com_max && (RM1 == nullptr || RM2 == nullptr || (((uintptr_t)RM1 | (uintptr_t)RM2) & 3) != 0)) return (int)cudaErrorInvalidValue;
-    if (g_blk == 32 && C1 % 256 == 0 && C2 % 256 == 0 && (((uintptr_t)EX1 | (uintptr_t)EX2) & 3) == 0) {
-        const ArgsTransp a0 = {(const int8_t*)X1, (const int8_t*)EX1, (int8_t*)Y1, (int8_t*)EY1, C1, (int8_t*)RM1};
-        const ArgsTransp a1 = {(const int8_t*)X2, (const int8_t*)EX2, (int8_t*)Y2, (int8_t*)EY2, C2, (int8_t*)RM2};
-        const int cx = (C1 > C2 ? C1 : C2) / 256;
-        const long long t128 = (long long)((C1 + C2) / 256) * (R / 128);
-        if (t128 >= 148) lanca_pdl(k_transpoe32_par<128>, dim3(dim3(cx, R / 128, 2)), dim3(256), 0, g_stream, a0, a1, R, kid);
-        else if (2 * t128 >= 148) lanca_pdl(k_transpoe32_par<64>, dim3(dim3(cx, R / 64, 2)), dim3(128), 0, g_stream, a0, a1, R, kid);
-        else if (4 * t128 >= 296) lanca_pdl(k_transpoe32_par<32>, dim3(dim3(cx, R / 32, 2)), dim3(64), 0, g_stream, a0, a1, R, kid);
-        else lanca_pdl(k_transpoe32_par<32, 1>, dim3(dim3(cx, R / 32, 2)), dim3(256), 0, g_stream, a0, a1, R, kid);
-        return fim();
-    }
-    if (com_max) return (int)cudaErrorNotSupported;            // the maxima are written by the wide block-32 kernel only
-    const int c = jt_transpoe(X1, EX1, Y1, EY1, R, C1, kid);
-    return c ? c : jt_transpoe(X2, EX2, Y2, EY2, R, C2, kid);
+    if (com_max && (g_blk != 32 || C1 % 256 || C2 % 256)) return (int)cudaErrorNotSupported;
+    return transpoe_impl({(const int8_t*)X1, (const int8_t*)EX1, (int8_t*)Y1, (int8_t*)EY1, C1, (int8_t*)RM1},
+                         {(const int8_t*)X2, (const int8_t*)EX2, (int8_t*)Y2, (int8_t*)EY2, C2, (int8_t*)RM2}, R, kid);
 }
 int jt_transpoe2(const void* X1, const void* EX1, void* Y1, void* EY1, const void* X2, const void* EX2, void* Y2, void* EY2, int C1, int C2,
                  int R, int kid) {
