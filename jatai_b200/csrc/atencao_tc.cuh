@@ -1,36 +1,37 @@
-// Integer causal attention with ALiBi on the tensor cores (tcgen05.mma kind::i8, accumulators in tensor memory), head dimension 64.
+// Integer causal attention with ALiBi on the tensor cores, head dimension 64 or 16, every T that is a multiple of 32.
 //
-// Same specification and layouts as atencao.cuh (jatai_cuda/ops.py:186-258 generalised; jatai_cuda/jatai_cuda.cu:822-1006).  What
-// changes is where the six contractions run.  Every one of them - q.k^T, P.V, dO.v^T, dS'.k, dS'^T.q, P^T.dO - is an exact integer
-// sum followed by ONE rounding, so (unlike the block GEMM) a whole contraction can accumulate in tensor memory.  The aligned
-// operands have 12 bits (|m << 4| <= 2032) and dS' has 13; kind::i8 takes 8, so each value is split into two signed digits,
-//     v = 128 hi + lo,   lo in [-64, 63],   hi in [-32, 32],
-// and a product of two split operands is three accumulators: hi.hi, hi.lo + lo.hi, lo.lo, recombined with shifts after the drain
-// (all sums stay far below 2^31; the final int32 wraps exactly like the specification's int64 -> int32 truncation).  P is uint8
-// and enters as it is (kind::i8 takes u8 x s8).
+// Same specification and layouts as atencao.cuh (jatai_cuda/ops.py:186-258 generalised; jatai_cuda/jatai_cuda.cu:822-1006).  Every one of
+// the six contractions - q.k^T, P.V, dO.v^T, dS'.k, dS'^T.q, P^T.dO - is an exact integer sum followed by ONE rounding, so (unlike the
+// block GEMM) a whole contraction can accumulate in tensor memory.
+//   * Scores and gP = dO.v^T: aligned operands have |a| <= 2032, which f16 holds exactly; the other side is split in two signed 6-bit
+//     digits, b = 64 hi + lo, so that each of the two fp32 accumulators (kind::f16) is an exact integer below 2^22 (64 x 2032 x 32).
+//   * The others take the token axis as K and reach further than 24 bits: two signed 8-bit digits v = 128 hi + lo (lo in [-64, 63]) on
+//     kind::i8, hi.hi / hi.lo + lo.hi / lo.lo recombined with shifts (the final int32 wraps exactly like the specification's
+//     int64 -> int32 truncation); P is uint8 and enters as it is.
 //
-// A preparation kernel aligns q, k, v (and dO) of every head to the head's maximum exponent once, splits them and writes the
-// digits to a workspace in the two layouts the MMAs need (both K-major):
-//     row layout     [BH*T][128]   token row = [hi digits of the 64 columns | lo digits]     (operand whose K is the head dimension)
-//     transposed     [BH*128][T]   row = one digit of one column, over the tokens            (operand whose K is the token axis)
-// The attention kernels fetch their tiles from there by TMA (128-byte swizzle) and never touch q, k, v again.
+// A preparation kernel aligns q, k, v (and dO) of every head to the head's maximum exponent once and writes what the MMAs read (all
+// K-major, rows of 128 bytes, TMA with the 128-byte swizzle; a head of 16 columns is padded with zeros to 64):
+//     plain          [BH*T][64] f16                      token rows
+//     digits         [2][BH*T][64] f16                   token rows of the hi digits, then of the lo digits
+//     transposed     [BH*128][T] int8                    row = one digit of one column, over the tokens
 //
-// Orientation of every score-like product: tensor-memory lane = key j (M = 128 keys of a chunk), column = query i (N = 32 queries of
-// the CTA's row tile); a thread of the drain owns one key and 16 queries.  Stored P is key-major, so that thread reads or writes 16
-// contiguous bytes of P.  Products whose output is [token, 64] are computed transposed: lane = digit row of the 64 columns
-// (hi rows 0..63, lo rows 64..127), column = token, and recombined through shared memory.
+// A query tile of 64 rows takes its keys in windows of 128 that end with the tile's last query and go back from there.  With the
+// reference's slopes P is exactly zero a few dozen keys behind the diagonal, so one window is nearly always all there is: the forward
+// works out after the first window how many it needs, the backward reads a map of the non-zero parts of P.  The one-window case keeps
+// everything in registers between the passes (scores, exponentials, P); with more windows each pass computes the scores again.
+// Between load, MMA and drain a block has little to overlap, so the overlap comes from two blocks per SM.
 //
-// What an MMA costs here: a kind::i8 instruction (M = 128, K = 32) takes ~190 cycles of the SM's tensor pipe whatever its N
-// (measured for N = 32 ... 256), so the kernels are built to issue FEW instructions: the B operand is widened instead.  The three
-// digit products of a score tile come out of ONE sequence of four instructions (K = 128 bytes of a row [hi | lo]) by stacking
-// three arrangements of the query tile as B rows - [qh | 0], [ql | qh], [0 | ql] - so that columns 0..63 of the result are
-// hi.hi, 64..127 the cross term and 128..191 lo.lo; likewise the two digits of dS' are stacked as B rows of one tile.
+// Orientation of every score-like product of a query tile: tensor-memory lane = key (M = 128 keys of a window), column = query; a
+// thread of the drain owns one key and 32 queries.  Stored P is key-major, so that thread reads or writes 32 contiguous bytes of P.
+// Products whose output is [token, column] are computed transposed: lane = digit row of the columns (hi rows 0..63, lo rows
+// 64..127), column = token, and recombined through shared memory.
 //
 // Every mbarrier wait is bounded (sentinel 7, abort flag, normal exit with tensor memory freed), as in the block GEMM.
 #pragma once
 #include <type_traits>
 #include "comum.cuh"
 #include "gemm_tc.cuh"
+#include "gemm_h.cuh"
 #include "atencao.cuh"
 
 namespace jt {
@@ -38,14 +39,15 @@ namespace atc {
 
 using namespace tc;
 
-constexpr int HD = 64, NI = 64, TJ = 128, NJ = 64;
-constexpr int NTL = 512;                 // threads of the row-tile kernels: 4 lane quarters x 4 groups of 16 query columns
-constexpr int SB = 3 * NI;               // columns of one score buffer in tensor memory: hi.hi | cross | lo.lo
+constexpr int NI = 64, TJ = 128;         // queries (or keys) of a tile, keys (or queries) of a window
+constexpr int NTA = 256;                 // threads: 4 lane quarters x 2 halves of 32 columns
+constexpr int SB = 2 * NI;               // columns of a score buffer in tensor memory: hi | lo
 constexpr uint32_t idesc(int n, bool b_sem_sinal) {       // kind::i8, D = s32, A = s8, B = s8 or u8, both K-major, M = 128
     return (2u << 4) | (1u << 7) | ((b_sem_sinal ? 0u : 1u) << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
-constexpr uint32_t ID_S3 = idesc(SB, false), ID_S2 = idesc(2 * NI, false), ID_PU = idesc(NI, true), ID_C2 = idesc(2 * NJ, false), ID_CU = idesc(NJ, true);
-constexpr uint32_t TILE_A = 128 * 128, TILE_NI = NI * 128, TILE_NJ = NJ * 128, TILE_Q3 = 3 * TILE_NI;
+constexpr uint32_t ID_S = idesc(SB, false), ID_PU = idesc(NI, true);
+constexpr uint32_t ID_F16 = (1u << 4) | ((uint32_t)(SB >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);      // kind::f16, D = f32, N = 128, M = 128
+constexpr uint32_t TILE_A = 128 * 128, TILE_N = NI * 128;
 
 __device__ __forceinline__ void digitos(int v, int& hi, int& lo) {
     hi = (v + 64) >> 7;
@@ -57,25 +59,6 @@ __device__ __forceinline__ uint32_t sw128(int linha, int byte) {
 }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// 16 columns of this thread's lane from three accumulators `passo` columns apart (hi.hi, cross, lo.lo)
-__device__ __forceinline__ void tmem_le16x3(uint32_t t, uint32_t (&a)[16], uint32_t (&b)[16], uint32_t (&c)[16], uint32_t passo = NI) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%48];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%49];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%50];\n"
-        "tcgen05.wait::ld.sync.aligned;\n"
-        : JT_O16(a, 0), JT_O16(b, 0), JT_O16(c, 0)
-        : "r"(t), "r"(t + passo), "r"(t + 2 * passo)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_le16(uint32_t t, uint32_t (&a)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        "tcgen05.wait::ld.sync.aligned;\n"
-        : JT_O16(a, 0)
-        : "r"(t)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_aloca(uint32_t* slot, int colunas) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(colunas) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -83,35 +66,40 @@ __device__ __forceinline__ void tmem_aloca(uint32_t* slot, int colunas) {
 __device__ __forceinline__ void tmem_libera(uint32_t tmem, int colunas) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(colunas) : "memory");
 }
-// the four MMAs of one score-like product: A = 128 rows of [hi | lo], B = the stacked query tile (3 NI rows) -> hi.hi | cross | lo.lo
-__device__ __forceinline__ void mma_digitos(uint32_t tm, uint64_t da, uint64_t db3) {
+// the four MMAs of one score-like product: A = 128 token rows (plain), B = the 64 token rows of the hi digits and the 64 of the lo digits
+__device__ __forceinline__ void mma_escores(uint32_t tm, uint64_t da, uint64_t db) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) tc_mma_i8(tm, da + 2 * q, db3 + 2 * q, ID_S3, q != 0);
+    for (int q = 0; q < 4; q++) th::mma_f16(tm, da + 2 * q, db + 2 * q, ID_F16, q != 0);
 }
-// the stacked B operand from a tile of NI rows of [hi | lo] (128-byte swizzle on both sides): rows 0..NI-1 = [hi | 0],
-// NI..2NI-1 = [lo | hi], 2NI..3NI-1 = [0 | lo].  Called by all NTL threads; 16-byte pieces.
-__device__ __forceinline__ void empilha3(const unsigned char* orig, unsigned char* dest, int tid) {
-    for (int t = tid; t < 3 * NI * 8; t += NTL) {
-        const int R = t >> 3, c = t & 7, bloco = R / NI, r = R % NI;
-        int co = -1;                                               // source piece, -1 = zeros
-        if (bloco == 0) co = c < 4 ? c : -1;
-        else if (bloco == 1) co = c < 4 ? c + 4 : c - 4;
-        else co = c < 4 ? -1 : c;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (co >= 0) v = *reinterpret_cast<const uint4*>(orig + (r >> 3) * 1024 + (r & 7) * 128 + ((co ^ (r & 7)) << 4));
-        *reinterpret_cast<uint4*>(dest + (R >> 3) * 1024 + (R & 7) * 128 + ((c ^ (R & 7)) << 4)) = v;
+// 16 scores of this lane from the two accumulators (hi at t, lo 64 columns on): 64 hi + lo, through the bit patterns of hi + 1.5 * 2^23 and
+// lo + 1.5 * 2^23
+__device__ __forceinline__ void escores16(uint32_t t, int (&x)[16]) {
+    uint32_t h[16], l[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : JT_O16(h, 0), JT_O16(l, 0)
+        : "r"(t), "r"(t + NI)
+        : "memory");
+#pragma unroll
+    for (int k = 0; k < 16; k += 2) {
+        th::soma_magia(h[k], h[k + 1]);
+        th::soma_magia(l[k], l[k + 1]);
+        x[k] = (int)((h[k] << 6) + (l[k] - 65u * MAGIA));
+        x[k + 1] = (int)((h[k + 1] << 6) + (l[k + 1] - 65u * MAGIA));
     }
 }
-// CTA-wide maximum of a non-negative per-thread value (NTL threads) -> one atomicMax
-__device__ __forceinline__ void max_cta16(int v, int* destino, int* red, int tid) {
-    v = warp_max(v);
+// CTA-wide maximum of a non-negative per-thread value -> one atomicMax
+__device__ __forceinline__ void max_cta(int v, int* destino, int* red, int tid) {
+    v = __reduce_max_sync(FULL, v);
     __syncthreads();
     if ((tid & 31) == 0) red[tid >> 5] = v;
     __syncthreads();
     if (tid == 0) {
         int r = red[0];
 #pragma unroll
-        for (int i = 1; i < NTL / 32; i++) r = max(r, red[i]);
+        for (int i = 1; i < NTA / 32; i++) r = max(r, red[i]);
         if (r > 0) atomicMax(destino, r);
     }
 }
@@ -139,844 +127,893 @@ __device__ __forceinline__ void grava8(int* acc, int16_t* ex, int8_t* qm, int8_t
 }
 
 // -------------------------------------------------------------------------------------------------- preparation
-// z = 0 q, 1 k, 2 v (columns of QKV), 3 dO.  Per tensor: destination in row layout and / or transposed layout (nullptr = not needed).
+// z = 0 q, 1 k, 2 v (columns of QKV), 3 dO.  Per tensor: the layouts wanted (nullptr = not).
 struct ArgsPrep {
     const int8_t* qm; const int8_t* qE; const int8_t* gm; const int8_t* gE;
-    int8_t* lin[4]; int8_t* tra[4];
+    uint16_t* plano[4]; uint16_t* dig[4]; int8_t* tra[4];
     int* em;                    // [BH][4] head-maximum exponents, indexed by z
     int* est;                   // backward: the statistics slots [BH][N_EST] to clear (nullptr in the forward)
-    int* nrm;                   // forward: [BH][2][ceil(T/128)] largest sum of squares of an aligned row of q (0) / k (1) per 128 tokens, or nullptr
-    int T, H, D, GA, blk;
+    int* nrm;                   // forward: [BH][2][ceil(T/128)] largest sum of squares of an aligned row of q (0) / k (1) per 128 tokens
+    int BH, T, H, D, hd, GA, blk, por_cta;       // por_cta: 128-token pieces of a CTA
 };
+__device__ __forceinline__ uint32_t par_h(int a, int b) {           // two integers of at most 2048 as halves
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"((float)b), "f"((float)a));
+    return r;
+}
 
-// grid (ceil(T / 128), BH, 4), 256 threads: 128 tokens of one head of one tensor
+// grid (CTAs per head, BH, 3 or 4), 256 threads: `por_cta` pieces of 128 tokens of one head of one tensor; a thread has half a token's row.
+// The head's maximum exponent takes a look at every token, so a CTA does as many pieces as leave the GPU full.
 __global__ void __launch_bounds__(256) k_at_prep(const ArgsPrep A) {
     pdl_espera();
     pdl_solta();
     __shared__ int red[8];
     __shared__ __align__(16) uint8_t tr[128 * 144];
-    const int tid = threadIdx.x, z = blockIdx.z, bh = blockIdx.y, b = bh / A.H, h = bh % A.H, t0 = blockIdx.x * 128;
-    int8_t* dl = z == 0 ? A.lin[0] : z == 1 ? A.lin[1] : z == 2 ? A.lin[2] : A.lin[3];
+    const int tid = threadIdx.x, z = blockIdx.z, bh = blockIdx.y, b = bh / A.H, h = bh % A.H;
+    uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
+    uint16_t* dg = z == 0 ? A.dig[0] : z == 1 ? A.dig[1] : z == 2 ? A.dig[2] : A.dig[3];
     int8_t* dt = z == 0 ? A.tra[0] : z == 1 ? A.tra[1] : z == 2 ? A.tra[2] : A.tra[3];
-    if (!dl && !dt) return;
-    const int T = A.T, D = A.D, blk = A.blk, linha0 = b * T;
+    const int T = A.T, D = A.D, blk = A.blk, hd = A.hd, linha0 = b * T;
     const int8_t* m = z == 3 ? A.gm : A.qm;
     const int8_t* E = z == 3 ? A.gE : A.qE;
-    const int ld = z == 3 ? D : 3 * D, col0 = z == 3 ? h * HD : z * D + h * HD, ldb = ld / blk;
-    const int em = at::max_cabeca<HD>(E, ldb, blk, linha0, T, col0, red, tid);
+    const int ld = z == 3 ? D : 3 * D, col0 = z == 3 ? h * hd : z * D + h * hd, ldb = ld / blk;
+    int em = -128;
+    {
+        const int nbh = hd > blk ? hd / blk : 1;
+        const int8_t* pe = E + (size_t)linha0 * ldb + col0 / blk;
+        for (int t = tid; t < T; t += 256)
+            for (int k = 0; k < nbh; k++) em = max(em, (int)pe[(size_t)t * ldb + k]);
+        em = __reduce_max_sync(FULL, em);
+        if ((tid & 31) == 0) red[tid >> 5] = em;
+        __syncthreads();
+        em = red[0];
+#pragma unroll
+        for (int i = 1; i < 8; i++) em = max(em, red[i]);
+        __syncthreads();                                           // red[] is used again below
+    }
     if (blockIdx.x == 0 && tid == 0) A.em[bh * 4 + z] = em;
     if (A.est && blockIdx.x == 0 && z == 3 && tid < at::N_EST) A.est[bh * at::N_EST + tid] = 0;
-    const int r = tid >> 1, meio = tid & 1, t = t0 + r;
-    int norma = 0;
-    if (t < T) {
-        const size_t lin = (size_t)(linha0 + t);
+    const int r = tid >> 1, meio = tid & 1;
+    const size_t BHT = (size_t)A.BH * T;
+    for (int p = 0; p < A.por_cta; p++) {
+        const int peca = blockIdx.x * A.por_cta + p, t0 = peca * 128, t = t0 + r;
+        if (t0 >= T) break;
+        int norma = 0;
+        if (t < T) {
+            const size_t lin = (size_t)(linha0 + t), o = ((size_t)bh * T + t) * 64;
 #pragma unroll
-        for (int parte = 0; parte < 2; parte++) {
-            const int c = meio * 32 + parte * 16;
-            int v[16], hi[16], lo[16];
-            le16(m + lin * ld + col0 + c, v);
-            const int s = em - (int)E[lin * ldb + (col0 + c) / blk];
+            for (int parte = 0; parte < 2; parte++) {
+                const int c = meio * 32 + parte * 16;
+                int v[16];
+                if (c < hd) {
+                    le16(m + lin * ld + col0 + c, v);
+                    const int s = em - (int)E[lin * ldb + (col0 + c) / blk];
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int a = rnd_d(v[k] << A.GA, s);
-                norma += a * a;                                    // 12-bit values, 64 of them: below 2^28
-                digitos(a, hi[k], lo[k]);
-            }
-            if (dl) {
-                int8_t* p = dl + ((size_t)bh * T + t) * 128 + c;
-                grava16(p, hi);
-                grava16(p + 64, lo);
-            }
-            if (dt) {
+                    for (int k = 0; k < 16; k++) {
+                        v[k] = rnd_d(v[k] << A.GA, s);
+                        norma += v[k] * v[k];                      // 12-bit values, 64 of them: below 2^28
+                    }
+                } else {
 #pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    tr[(c + k) * 144 + r] = (uint8_t)hi[k];
-                    tr[(64 + c + k) * 144 + r] = (uint8_t)lo[k];
+                    for (int k = 0; k < 16; k++) v[k] = 0;
+                }
+                auto grava = [&](uint16_t* d, auto f) {
+                    uint4* q = reinterpret_cast<uint4*>(d + o + c);
+                    q[0] = make_uint4(par_h(f(v[0]), f(v[1])), par_h(f(v[2]), f(v[3])), par_h(f(v[4]), f(v[5])), par_h(f(v[6]), f(v[7])));
+                    q[1] = make_uint4(par_h(f(v[8]), f(v[9])), par_h(f(v[10]), f(v[11])), par_h(f(v[12]), f(v[13])), par_h(f(v[14]), f(v[15])));
+                };
+                if (dp) grava(dp, [](int x) { return x; });
+                if (dg) {
+                    grava(dg, [](int x) { return (x + 32) >> 6; });
+                    grava(dg + BHT * 64, [](int x) { return x - (((x + 32) >> 6) << 6); });
+                }
+                if (dt) {
+#pragma unroll
+                    for (int k = 0; k < 16; k++) {
+                        int hi, lo;
+                        digitos(v[k], hi, lo);
+                        tr[(c + k) * 144 + r] = (uint8_t)hi;
+                        tr[(64 + c + k) * 144 + r] = (uint8_t)lo;
+                    }
                 }
             }
         }
-    }
-    if (A.nrm && z < 2) {
-        // the largest squared norm of an aligned row among this CTA's 128 tokens (the two halves of a row sit in neighbouring lanes)
-        norma += __shfl_xor_sync(0xffffffffu, norma, 1);
-        norma = __reduce_max_sync(0xffffffffu, norma);
-        __syncthreads();                                           // red[] is free again (max_cabeca used it)
-        if ((tid & 31) == 0) red[tid >> 5] = norma;
-        __syncthreads();
-        if (tid == 0) {
-            int mx = 0;
-            for (int w = 0; w < 8; w++) mx = max(mx, red[w]);
-            A.nrm[((size_t)bh * 2 + z) * gridDim.x + blockIdx.x] = mx;
+        if (A.nrm && z < 2) {
+            // the largest squared norm of an aligned row among the 128 tokens (the two halves of a row sit in neighbouring lanes)
+            norma += __shfl_xor_sync(FULL, norma, 1);
+            norma = __reduce_max_sync(FULL, norma);
+            if ((tid & 31) == 0) red[tid >> 5] = norma;
+            __syncthreads();
+            if (tid == 0) {
+                int mx = 0;
+                for (int w = 0; w < 8; w++) mx = max(mx, red[w]);
+                A.nrm[((size_t)bh * 2 + z) * ((T + 127) / 128) + peca] = mx;
+            }
         }
-    }
-    if (dt) {
-        __syncthreads();
-        const int dd = tid >> 1;
+        if (dt) {
+            __syncthreads();
+            const int dd = tid >> 1;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int off = meio * 64 + q * 16;
-            if (t0 + off < T)
-                *reinterpret_cast<uint4*>(dt + ((size_t)bh * 128 + dd) * T + t0 + off) = *reinterpret_cast<const uint4*>(tr + dd * 144 + off);
+            for (int q = 0; q < 4; q++) {
+                const int off = meio * 64 + q * 16;
+                if (t0 + off < T)
+                    *reinterpret_cast<uint4*>(dt + ((size_t)bh * 128 + dd) * T + t0 + off) = *reinterpret_cast<const uint4*>(tr + dd * 144 + off);
+            }
         }
+        __syncthreads();                                           // red[] and tr[] go to the next piece
     }
 }
 
-// shared-memory carve-up helpers: every operand tile starts on a 1024-byte boundary
 struct Barras {
     uint32_t base;
     __device__ uint32_t operator[](int i) const { return base + 8 * i; }
 };
-
-// -------------------------------------------------------------------------------------------------- forward
-// ops.py:198-219.  grid (T / 64, BH), 512 threads; a drain thread owns one key of the chunk and 16 of the 64 query rows.
-//   sweep 1 over the key chunks: scores u (tensor core + drain), row maxima;
-//   sweep 2: the scores again (recomputing costs 13 instructions per score, keeping them 128 KB of shared memory), the
-//            exponentials ex = exp(-(m - u)/256) >> 3 (12 bits, kept as uint16 [64][T+8]) and their row sums;
-//   pass 3 : P = min((ex * inv + 2^19) >> 20, 255); the thread's 16 rows of its key are 16 contiguous bytes of the stored,
-//            key-major P; the same bytes go to a small MMA-layout tile and O^T += V^T . P^T runs chunk by chunk behind it.
-// Shared: 2 operand stages (K chunks, then V^T chunks), the query tile as loaded and stacked, 2 P tiles, ex.  Tensor memory:
-// two score buffers of 3 x 64 columns, one output accumulator of 64 columns (512 allocated, one CTA per SM).
-__global__ void __launch_bounds__(NTL) k_atencao_tc(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
-                                                    const __grid_constant__ CUtensorMap mVt, const int* __restrict__ em, int* __restrict__ Oacc,
-                                                    int16_t* __restrict__ Oe, int8_t* __restrict__ Qm, int8_t* __restrict__ QE, uint8_t* __restrict__ P,
-                                                    int T, int H, int D, int GA, int kid) {
-    extern __shared__ unsigned char bruto[];
+// What every kernel below starts with: barriers, the abort flag, tensor memory.  The carve-up behind the operands (OFF): barriers, the
+// tensor-memory address, the abort flag, then 128 bytes in, `n` words of the kernel's own.
+struct Base {
+    unsigned char* smem; uint32_t s, tmem; volatile int* aborta; Barras bar;
+};
+__device__ __forceinline__ Base comeca(unsigned char* bruto, uint32_t off, int barras, int colunas) {
+    Base b;
     // (pointer arithmetic on the array keeps the shared address space: a round trip through an integer makes every access generic)
-    unsigned char* smem = bruto + ((1024u - (smem_u32(bruto) & 1023u)) & 1023u);
-    const uint32_t sbase = smem_u32(smem);
-    const int nchT = (T + TJ - 1) / TJ, TPX = T + 8;
-    // 3 operand stages (a TMA load takes longer than one step of a sweep: loads run three steps ahead) | stacked query tile |
-    // 2 P tiles (the query tile as loaded sits there until it has been stacked) | barriers, row statistics | ex
-    constexpr int NSTF = 3;
-    constexpr uint32_t OFF_Q3 = NSTF * TILE_A, OFF_PB = OFF_Q3 + TILE_Q3, OFF_Q = OFF_PB, OFF_BAR = OFF_PB + 2 * TILE_NI, OFF_EX = OFF_BAR + 640;
-    uint8_t* pB = smem + OFF_PB;                                   // [2][64 x 128]
-    uint16_t* ex_s = reinterpret_cast<uint16_t*>(smem + OFF_EX);   // [64][T + 8]
-    const Barras bar = {sbase + OFF_BAR};                          // 0 q | 1..3 k | 4,5 s | 6..8 v | 9,10 pv done | 11 o
-    constexpr int B_K = 1, B_S = 4, B_V = 6, B_PV = 9, B_O = 11;
-    uint32_t* slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 112);
-    volatile int* aborta = reinterpret_cast<volatile int*>(smem + OFF_BAR + 116);
-    int* m_s = reinterpret_cast<int*>(smem + OFF_BAR + 128);       // [64] row maxima, then 2^28 / row sum
-    int* s_acc = m_s + NI;                                         // [64] row sums
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int ordem = blockIdx.y * gridDim.x + blockIdx.x;         // heaviest (last) row tiles of all heads first
-    const int bh = ordem % gridDim.y, b = bh / H, h = bh % H, i0 = (gridDim.x - 1 - ordem / gridDim.y) * NI, linha0 = b * T;
-    const int nproc = i0 + NI, nch = (nproc + TJ - 1) / TJ;
-    const uint32_t sA[NSTF] = {sbase, sbase + TILE_A, sbase + 2 * TILE_A}, sQ = sbase + OFF_Q, sQ3 = sbase + OFF_Q3, sPB = sbase + OFF_PB;
-    // a CTA lives a few microseconds, so what it waits for first is asked for first: the operand loads go out as soon as their
-    // barriers exist, the small global reads follow, and tensor memory is allocated while all of that is in flight
-    if (tid == 0) {
-        for (int i = 0; i < 12; i++) mbar_init(bar[i], 1);
-        *aborta = 0;
+    b.smem = bruto + ((1024u - (smem_u32(bruto) & 1023u)) & 1023u);
+    b.s = smem_u32(b.smem);
+    b.bar.base = b.s + off;
+    uint32_t* slot = reinterpret_cast<uint32_t*>(b.smem + off + 112);
+    b.aborta = reinterpret_cast<volatile int*>(b.smem + off + 116);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < barras; i++) mbar_init(b.bar[i], 1);
+        *b.aborta = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    pdl_espera();                                                  // the operands below are the previous kernel's outputs
-    pdl_solta();
-    const bool pode_pular = T > 2 * TJ;                            // up to two key chunks nearly every chunk is next to the diagonal
-    if (tid == 0) {
-        mbar_expect_tx(bar[0], TILE_NI);
-        tma_2d(sQ, &mQ, 0, bh * T + i0, bar[0]);
-        if (!pode_pular)                                           // every chunk stays: its loads need not wait for the bound
-            for (int c = 0; c < NSTF && c < 2 * nch; c++) {
-                mbar_expect_tx(bar[B_K + c], TILE_A);
-                tma_2d(sA[c], &mK, 0, bh * T + (c % nch) * TJ, bar[B_K + c]);
-            }
-    }
-    const int emq = em[bh * 4], emk = em[bh * 4 + 1], emv = em[bh * 4 + 2];
-    const int s_u = -((emq - GA) + (emk - GA) - 3 + 8), incl = at::incl_alibi(h);
-    // Key chunks that cannot matter.  |q_i . k_j| <= sqrt(|q_i|^2 |k_j|^2) (the preparation left the largest squared norms per 128
-    // tokens), so with B >= (|x| >> s_u) + 1 every score is u_ij <= B - (i - j) 2^incl and every row maximum is m_i >= u_ii >= -B.
-    // The exponential (>> 3) is exactly 0 from m - u = 2130 on (p < 2^15 shifted by n + 3 >= 15), so a key at distance
-    // (i - j) 2^incl >= 2132 + 2 B adds nothing to the row sum, cannot be the maximum and has P = 0: chunks wholly at that distance
-    // from the tile's first query are left out of all three passes (P = 0 is still written).  Only on the right-shift path.
-    int c0 = 0;
-    if (pode_pular && s_u > 0 && s_u < 31) {
-        const int* nrm = em + 4 * gridDim.y;
-        const int nq = nrm[((size_t)bh * 2) * nchT + i0 / TJ];
-        int nk = 0;
-        for (int c = 0; c < nch; c++) nk = max(nk, nrm[((size_t)bh * 2 + 1) * nchT + c]);
-        const long long B = ((long long)sqrt((double)nq * (double)nk) + 2) >> s_u;
-        const long long lim = 2132 + 2 * (B + 2), D0 = (lim + (1 << incl) - 1) >> incl;
-        if (i0 - D0 + 1 > 0) c0 = (int)((i0 - D0 + 1) / TJ);
-    }
-    const int nviv = nch - c0, nvoltas = 2 * nviv;                  // live chunks c0 .. nch - 1, swept twice
-    if (tid == 0 && pode_pular) {
-        for (int c = 0; c < NSTF && c < nvoltas; c++) {
-            mbar_expect_tx(bar[B_K + c], TILE_A);
-            tma_2d(sA[c], &mK, 0, bh * T + (c0 + c % nviv) * TJ, bar[B_K + c]);
-        }
-    }
-    if (tid < NI) { m_s[tid] = U_MIN; s_acc[tid] = 0; }
-    if (wid == 0) tmem_aloca(slot, 512);
+    if (threadIdx.x < 32) tmem_aloca(slot, colunas);
     tc_fence_antes();
     __syncthreads();
     tc_fence_depois();
-    const uint32_t tmem = *slot;
-    const int jl = 32 * (wid & 3) + lane, g = wid >> 2;            // this thread's key within a chunk, its quarter of the query rows
-    const uint32_t t_lane = tmem + ((uint32_t)(32 * (wid & 3)) << 16);
-
-    auto emite = [&](int cc) -> bool {                             // one thread: the score MMAs of step cc (key chunk cc % nch)
-        if (!espera(bar[B_K + cc % NSTF], (cc / NSTF) & 1, aborta, kid, 21)) return false;
-        tc_fence_depois();
-        mma_digitos(tmem + (cc & 1) * SB, desc_sw128(sA[cc % NSTF]), desc_sw128(sQ3));
-        tc_commit(bar[B_S + (cc & 1)]);
-        return true;
-    };
-    int v16[16], mi[16];                                           // running maxima, then running sums | this thread's row maxima, then 2^28 / sum
-#pragma unroll
-    for (int k = 0; k < 16; k++) { v16[k] = U_MIN; mi[k] = 0; }
-    bool ok = __all_sync(FULL, espera(bar[0], 0, aborta, kid, 20));     // the query tile has landed: stack its three arrangements
-    if (ok) empilha3(smem + OFF_Q, smem + OFF_Q3, tid);
-    fence_async();
+    b.tmem = *slot;
+    return b;
+}
+__device__ __forceinline__ void termina(const Base& b, int colunas) {
+    tc_fence_antes();
     __syncthreads();
-    if (tid == 0 && ok) ok = emite(0);
-    for (int cc = 0; cc < nvoltas; cc++) {
-        const int c = c0 + cc % nviv, st = cc & 1;
-        if (tid == 0 && ok && cc + 1 < nvoltas) ok = emite(cc + 1);
-        __syncwarp();
-        ok = __all_sync(FULL, ok && espera(bar[B_S + st], (cc >> 1) & 1, aborta, kid, 22));
+    if (threadIdx.x < 32) {
         tc_fence_depois();
-        if (tid == 0 && ok && cc + NSTF < nvoltas) {               // this step's MMAs are done: its stage takes the chunk of step cc + 3
-            mbar_expect_tx(bar[B_K + cc % NSTF], TILE_A);
-            tma_2d(sA[cc % NSTF], &mK, 0, bh * T + (c0 + (cc + NSTF) % nviv) * TJ, bar[B_K + cc % NSTF]);
-        }
-        if (cc == nviv) {
-            // between the sweeps: the row maxima from the per-thread maxima
+        tmem_libera(b.tmem, colunas);
+    }
+}
+// one thread: window rows of a token-major or transposed operand -> shared memory
+__device__ __forceinline__ void carrega(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bytes, uint32_t bar) {
+    mbar_expect_tx(bar, bytes);
+    tma_2d(dst, m, x, y, bar);
+}
+// the 64 hi and the 64 lo digit rows of a tile, token rows `lin` on (BHT rows to the lo digits)
+__device__ __forceinline__ void carrega_dig(uint32_t dst, const CUtensorMap* m, int lin, int BHT, uint32_t bar) {
+    mbar_expect_tx(bar, 2 * TILE_N);
+    tma_2d(dst, m, 0, lin, bar);
+    tma_2d(dst + TILE_N, m, 0, BHT + lin, bar);
+}
+// 32 bytes as numbers
+__device__ __forceinline__ int byte_u(const uint32_t (&w)[8], int k) { return (int)__byte_perm(w[k >> 2], 0, 0x4440 + (k & 3)); }
+
+// -------------------------------------------------------------------------------------------------- forward
+// ops.py:198-219.  A CTA owns 64 queries of one head.  Three passes over the windows: row maxima; exponentials ex = exp(-(m - u)/256) >> 3
+// and their row sums; P = min((ex * inv + 2^19) >> 20, 255), stored, put into an MMA tile, and O^T += V^T . P^T.  With one window the
+// scores are computed once and stay in registers.
+//
+// How many windows.  |q_i . k_j| <= sqrt(|q_i|^2 |k_j|^2) (the preparation left the largest squared norms per 128 tokens), so with
+// B >= (|x| >> s_u) + 1 every score is u_ij <= B - (i - j) 2^incl.  The exponential (>> 3) is exactly 0 from m - u = 2130 on (p < 2^15
+// shifted by n + 3 >= 15), so with the maximum m_i of the first window (which holds the diagonal; the true maximum is no smaller) a key
+// at distance (i - j) 2^incl >= 2130 + B - m_i adds nothing to the row sum, cannot be the maximum and has P = 0.  This holds on the
+// right-shift path, the only one that occurs in earnest; any other shift takes every window and the general roundings.
+//
+// Shared: Q digits 16 KB | K window 16 KB | V^T window 16 KB | P tile 8 KB; the output staging goes over the first three.
+// Tensor memory: scores 128 columns, O 64 (256 allocated: two blocks per SM).
+struct ArgsFrente {
+    const int* em; const int* nrm;
+    int* Oacc; int16_t* Oe; int8_t* Qm; int8_t* QE; uint8_t* P;   // Qm / QE: block output (head dimension 64, block length 32) instead of the raw one
+    int BH, T, H, D, hd, GA, kid;
+};
+constexpr uint32_t FR_K = 2 * TILE_N, FR_V = FR_K + TILE_A, FR_P = FR_V + TILE_A, FR_BAR = FR_P + TILE_N;
+constexpr size_t SM_FRENTE = 1024 + FR_BAR + 128 + (6 * NI + 2) * 4;
+
+__global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
+                                                      const __grid_constant__ CUtensorMap mVt, const ArgsFrente A) {
+    extern __shared__ unsigned char bruto[];
+    enum { B_Q = 0, B_K = 1, B_V = 2, B_S = 3, B_O = 4 };
+    const Base S = comeca(bruto, FR_BAR, 5, 256);
+    int* r_s = reinterpret_cast<int*>(S.smem + FR_BAR + 128);      // [4 lane quarters][64] partial maxima, partial sums
+    int* m_s = r_s + 4 * NI;                                       // [64] row maxima
+    int* i_s = m_s + NI;                                           // [64] 2^28 / row sum
+    int* n_s = i_s + NI;                                           // [2] windows needed, per 32 queries
+    const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane;
+    const int tile = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y, b = bh / H, h = bh % H, i0 = tile * NI, linha0 = b * T;
+    const int j00 = i0 + NI - TJ;                                  // first key of the first window (may lie before the sequence: such rows are masked)
+    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
+    pdl_espera();
+    pdl_solta();
+    if (tid == 0) {
+        carrega_dig(S.s, &mQ, bh * T + i0, A.BH * T, S.bar[B_Q]);
+        carrega(S.s + FR_K, &mK, 0, bh * T + j00, TILE_A, S.bar[B_K]);
+        carrega(S.s + FR_V, &mVt, j00, bh * 128, TILE_A, S.bar[B_V]);
+    }
+    const int emq = A.em[bh * 4], emk = A.em[bh * 4 + 1], emv = A.em[bh * 4 + 2];
+    const int s_u = -((emq - GA) + (emk - GA) - (hd == 64 ? 3 : 2) + 8), incl = at::incl_alibi(h);
+    const bool direita = s_u > 0 && s_u < 31;
+    const int nmax = (i0 + NI - 1) / TJ + 1;
+    int B = 0;                                                     // bound of the products in the units of the scores
+    if (direita && nmax > 1) {
+        const int nch = (T + TJ - 1) / TJ;
+        const int nq = A.nrm[(size_t)bh * 2 * nch + i0 / TJ];
+        int nk = lane <= min(i0 + NI - 1, T - 1) / TJ ? A.nrm[((size_t)bh * 2 + 1) * nch + lane] : 0;
+        nk = __reduce_max_sync(FULL, nk);
+        B = (int)(((long long)sqrt((double)nq * (double)nk) + 2) >> s_u) + 1;
+    }
+    // zeros of P outside the first window, while the loads are on their way (further windows overwrite their part)
+    for (int t = tid; t < T * 4; t += NTA) {
+        const int j = t >> 2, i = i0 + 16 * (t & 3);
+        if ((j < j00 || j >= i0 + NI) && i < T) *reinterpret_cast<uint4*>(A.P + ((size_t)bh * T + j) * T + i) = make_uint4(0, 0, 0, 0);
+    }
+    int v[32];                                                     // this thread's 32 scores of the window at hand, then their exponentials
+    int minha = U_MIN;                                             // query q0 + lane: maximum, then sum, over this warp's keys
+    int n = 1, passo = 0;                                          // windows; score computations so far
+    bool ok = true, tem_ex = false;
+#pragma unroll 1
+    for (int fase = 0; fase < 3; fase++) {
+        if (fase == 1) minha = 0;
+#pragma unroll 1
+        for (int s = 0; s < n; s++) {
+            const int j = j00 - s * TJ + jl, dj = i0 + q0 - j;     // dj + k = distance of query k to this key
+            const bool ha = j >= 0 && j < T && i0 + q0 < T;
+            const int kmin = ha ? -dj : 32;                        // the key counts for query k >= kmin
+            if (fase == 0 || n > 1) {
+                if (passo) { tc_fence_antes(); __syncthreads(); }   // everyone has read the previous scores
+                if (tid == 0 && ok) {
+                    if (passo) carrega(S.s + FR_K, &mK, 0, bh * T + j00 - s * TJ, TILE_A, S.bar[B_K]);
+                    else ok = espera(S.bar[B_Q], 0, S.aborta, kid, 20);
+                    ok = ok && espera(S.bar[B_K], passo & 1, S.aborta, kid, 21);
+                    if (ok) {
+                        tc_fence_depois();
+                        mma_escores(S.tmem, desc_sw128(S.s + FR_K), desc_sw128(S.s));
+                        tc_commit(S.bar[B_S]);
+                    }
+                }
+                __syncwarp();
+                ok = __all_sync(FULL, ok && espera(S.bar[B_S], passo & 1, S.aborta, kid, 22));
+                tc_fence_depois();
+                passo++;
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int m = warp_max(v16[k]);
-                if (lane == 0) atomicMax(&m_s[16 * g + k], m);
+                for (int g = 0; g < 2; g++) {
+                    int x[16];
+                    escores16(t_lane + q0 + 16 * g, x);
+                    if (direita) {
+                        // rnd_d(x, s) = (x + 2^(s-1) - 1 + ((x >> s) & 1)) >> s
+                        const int meio = (1 << (s_u - 1)) - 1;
+#pragma unroll
+                        for (int k = 0; k < 16; k++) {
+                            const int u = ((x[k] + meio + ((x[k] >> s_u) & 1)) >> s_u) - ((dj + 16 * g + k) << incl);
+                            v[16 * g + k] = 16 * g + k >= kmin ? u : U_MIN;
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 16; k++) {
+                            const int kk = 16 * g + k;
+                            v[kk] = U_MIN;
+                            if (kk >= kmin) v[kk] = rnd(x[k], s_u, kid, (long long)(linha0 + i0 + q0 + kk) * D + h * hd) - ((dj + kk) << incl);
+                        }
+                    }
+                }
+            }
+            if (fase == 0) {
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    const int r = __reduce_max_sync(FULL, v[k]);
+                    minha = lane == k ? max(minha, r) : minha;
+                }
+                if (s == 0 || s == n - 1) {
+                    r_s[quarto * NI + q0 + lane] = minha;
+                    __syncthreads();
+                    if (tid < NI) {
+                        const int m = max(max(r_s[tid], r_s[NI + tid]), max(r_s[2 * NI + tid], r_s[3 * NI + tid]));
+                        m_s[tid] = m;
+                        int ni = nmax;
+                        if (direita) {
+                            // keys from distance `longe` on do not count; n windows leave out the distances tid + 65 + 128 (n - 1) and more
+                            const int longe = max((2130 + B - m + (1 << incl) - 1) >> incl, 0);
+                            ni = i0 + tid < T ? 1 + max((longe - (tid + 65) + TJ - 1) / TJ, 0) : 1;
+                        }
+                        ni = __reduce_max_sync(FULL, ni);
+                        if (lane == 0) n_s[wid] = min(ni, nmax);
+                    }
+                    __syncthreads();
+                    if (s == 0) n = max(n_s[0], n_s[1]);
+                }
+                continue;
+            }
+            if (!tem_ex) {
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    const int m = m_s[q0 + k], t = (k < kmin || v[k] <= m - 6000 ? 6000 : m - v[k]) * 23637, f2 = (t >> 6) & 0xFFFE;
+                    int p = -1295 * 65536;                         // exp3_dif, a key beyond the diagonal being infinitely far below
+                    p = __mulhi(p, f2) * 65536 + 7556 * 65536;
+                    p = __mulhi(p, f2) * 65536 - 22645 * 65536;
+                    p = __mulhi(p, f2) * 65536 + 32765 * 65536;
+                    v[k] = p >> min(19 + (t >> 22), 31);
+                }
+                tem_ex = n == 1;
+            }
+            if (fase == 1) {
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    const int r = __reduce_add_sync(FULL, v[k]);
+                    minha += lane == k ? r : 0;
+                }
+                continue;
+            }
+            if (s) ok = __all_sync(FULL, ok && espera(S.bar[B_O], (s - 1) & 1, S.aborta, kid, 23));      // the P tile and the V stage are free again
+            uint32_t w[8];
+#pragma unroll
+            for (int k = 0; k < 32; k++) {
+                const int p = min((v[k] * i_s[q0 + k] + (1 << 19)) >> 20, 255);
+                w[k >> 2] = (k & 3) == 0 ? (uint32_t)p : w[k >> 2] | (uint32_t)p << (8 * (k & 3));
+                S.smem[FR_P + sw128(q0 + k, jl)] = (uint8_t)p;
+            }
+            if (ha) {
+                uint4* d = reinterpret_cast<uint4*>(A.P + ((size_t)bh * T + j) * T + i0 + q0);
+                d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                d[1] = make_uint4(w[4], w[5], w[6], w[7]);
+            }
+            fence_async();                                         // the tile is read by the tensor core (async proxy)
+            __syncthreads();
+            if (tid == 0 && ok) {
+                if (s) carrega(S.s + FR_V, &mVt, j00 - s * TJ, bh * 128, TILE_A, S.bar[B_V]);
+                ok = espera(S.bar[B_V], s & 1, S.aborta, kid, 24);
+                if (ok) {
+                    tc_fence_depois();
+                    const uint64_t da = desc_sw128(S.s + FR_V), db = desc_sw128(S.s + FR_P);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) tc_mma_i8(S.tmem + SB, da + 2 * q, db + 2 * q, ID_PU, (s | q) != 0);
+                    tc_commit(S.bar[B_O]);
+                }
+            }
+            __syncwarp();
+        }
+        if (fase == 1) {
+            r_s[quarto * NI + q0 + lane] = minha;
+            __syncthreads();
+            if (tid < NI) {
+                int soma = r_s[tid] + r_s[NI + tid] + r_s[2 * NI + tid] + r_s[3 * NI + tid];
+                if (soma <= 0 && i0 + tid < T) reporta(E_DIV, kid, (long long)(linha0 + i0 + tid) * D + h * hd, soma, 0);
+                i_s[tid] = (1 << 28) / max(soma, 1);               // ops.py:215
             }
             __syncthreads();
-#pragma unroll
-            for (int k = 0; k < 16; k++) { mi[k] = m_s[16 * g + k]; v16[k] = 0; }
-        }
-        if (ok) {
-            const int j = c * TJ + jl;
-            uint32_t hh[16], cr[16], ll[16];
-            tmem_le16x3(t_lane + st * SB + 16 * g, hh, cr, ll);
-            if (j < nproc && s_u > 0 && s_u < 31) {
-                // the usual case, a right shift: rounding, slope and exponential written out with their invariants hoisted.
-                //   rnd_d(x, s)              = (x + 2^(s-1) - 1 + ((x >> s) & 1)) >> s
-                //   exp_int(d) >> 3, d>=0    : t = min(d, 6000) * 23637, n = t >> 22, f = bits 7..21 of t; the cubic in f runs on
-                //                              p * 2^16 (|p| < 2^15 at every step): (p f) >> 15 = mulhi(p << 16, 2 f); the result
-                //                              p >> (n + 3) is 0 from n = 12 on (0 <= p < 2^15), as is the shift clamped to 31
-                const int meio = (1 << (s_u - 1)) - 1, dj = i0 + 16 * g - j, menos = -(1 << incl);
-                const bool diagonal = c == nch - 1;                    // the only chunk with keys beyond some query of the tile
-#pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int x = junta3(hh[k], cr[k], ll[k]);
-                    int u = (x + meio + ((x >> s_u) & 1)) >> s_u;
-                    u += (dj + k) * menos;
-                    const bool dentro = !diagonal || dj + k >= 0;
-                    if (cc < nviv) v16[k] = max(v16[k], dentro ? u : U_MIN);
-                    else {
-                        // a key beyond the diagonal counts as infinitely far below the maximum; mi >= u otherwise, and
-                        // |u| < 2^30 + 2^18: the difference cannot overflow
-                        const int t = min(dentro ? mi[k] - u : 6000, 6000) * 23637;
-                        const int f2 = (t >> 6) & 0xFFFE;
-                        int pp = -1295 * 65536;
-                        pp = __mulhi(pp, f2) * 65536 + 7556 * 65536;
-                        pp = __mulhi(pp, f2) * 65536 - 22645 * 65536;
-                        pp = __mulhi(pp, f2) * 65536 + 32765 * 65536;
-                        const int ex = pp >> min(19 + (t >> 22), 31);
-                        v16[k] += ex;
-                        ex_s[(16 * g + k) * TPX + j] = (uint16_t)ex;
-                    }
-                }
-            } else if (j < nproc) {
-#pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int i = i0 + 16 * g + k;
-                    const bool dentro = j <= i;
-                    int u = U_MIN;
-                    if (dentro) u = rnd(junta3(hh[k], cr[k], ll[k]), s_u, kid, (long long)(linha0 + i) * D + h * HD) - ((i - j) << incl);
-                    if (cc < nviv) v16[k] = max(v16[k], u);
-                    else {
-                        const int ex = dentro ? exp_dif(mi[k], u) >> 3 : 0;
-                        v16[k] += ex;
-                        ex_s[(16 * g + k) * TPX + j] = (uint16_t)ex;
-                    }
-                }
-            }
-        }
-        tc_fence_antes();
-        __syncthreads();
-    }
-    // row sums -> 2^28 / sum (ops.py:215)
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const int sm = warp_sum(v16[k]);
-        if (lane == 0) atomicAdd(&s_acc[16 * g + k], sm);
-    }
-    __syncthreads();
-    if (tid < NI) {
-        int soma = s_acc[tid];
-        if (soma <= 0) { reporta(E_DIV, kid, (long long)(linha0 + i0 + tid) * D + h * HD, soma, 0); soma = 1; }
-        m_s[tid] = (1 << 28) / soma;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 16; k++) mi[k] = m_s[16 * g + k];
-    // pass 3: P of every key (explicit zeros before the first live chunk and beyond the diagonal, to the end of the sequence) and
-    // O^T += V^T . P^T behind it, over the live chunks (m = c - c0 counts them: stages and parities go by m)
-    if (tid == 0 && ok) {
-        for (int m = 0; m < NSTF && m < nviv; m++) {
-            mbar_expect_tx(bar[B_V + m], TILE_A);
-            tma_2d(sA[m], &mVt, (c0 + m) * TJ, bh * 128, bar[B_V + m]);
         }
     }
-    for (int c = 0; c < nchT; c++) {
-        const int m = c - c0, st = m & 1, j = c * TJ + jl;
-        const bool com_mma = c >= c0 && c < nch;
-        if (com_mma && m >= 2) ok = __all_sync(FULL, ok && espera(bar[B_PV + st], ((m - 2) >> 1) & 1, aborta, kid, 26));      // tile st is free again
-        if (com_mma && m >= 2 && m + 1 >= NSTF && m + 1 < nviv && tid == 0 && ok) {      // and so is the operand stage of chunk m - 2: it takes chunk m + 1
-            mbar_expect_tx(bar[B_V + (m + 1) % NSTF], TILE_A);
-            tma_2d(sA[(m + 1) % NSTF], &mVt, (c + 1) * TJ, bh * 128, bar[B_V + (m + 1) % NSTF]);
-        }
-        uint32_t w[4] = {0, 0, 0, 0};
-        if (com_mma && j < nproc) {
-#pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int p = min(((int)ex_s[(16 * g + k) * TPX + j] * mi[k] + (1 << 19)) >> 20, 255);
-                w[k >> 2] |= (uint32_t)p << (8 * (k & 3));
-            }
-        }
-        if (j < T) *reinterpret_cast<uint4*>(P + ((size_t)bh * T + j) * T + i0 + 16 * g) = make_uint4(w[0], w[1], w[2], w[3]);
-        if (!com_mma) continue;
-#pragma unroll
-        for (int k = 0; k < 16; k++) pB[st * TILE_NI + sw128(16 * g + k, jl)] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
-        fence_async();                                             // the tile is read by the tensor core (async proxy)
-        __syncthreads();
-        if (tid == 0 && ok) {
-            ok = espera(bar[B_V + m % NSTF], (m / NSTF) & 1, aborta, kid, 23);
-            if (ok) {
-                tc_fence_depois();
-                const uint64_t da = desc_sw128(sA[m % NSTF]), db = desc_sw128(sPB + st * TILE_NI);
-#pragma unroll
-                for (int q = 0; q < 4; q++) tc_mma_i8(tmem + 2 * SB, da + 2 * q, db + 2 * q, ID_PU, (m | q) != 0);
-                tc_commit(bar[B_PV + st]);
-                if (c == nch - 1) tc_commit(bar[B_O]);
-            }
-        }
-    }
-    __syncwarp();
-    ok = __all_sync(FULL, ok && espera(bar[B_O], 0, aborta, kid, 25));
+    ok = __all_sync(FULL, ok && espera(S.bar[B_O], (n - 1) & 1, S.aborta, kid, 25));
     tc_fence_depois();
-    __syncthreads();                                               // every thread is done with ex_s: it becomes the staging area
-    int* o_s = reinterpret_cast<int*>(smem + OFF_EX);              // [128 digit rows][65]
+    int* o_s = reinterpret_cast<int*>(S.smem);                     // [128 digit rows][65] over the operands
     if (ok) {
-        uint32_t d[16];
-        tmem_le16(t_lane + 2 * SB + 16 * g, d);
+        uint32_t d[32];
+        tmem_le32(t_lane + SB + q0, d);
 #pragma unroll
-        for (int k = 0; k < 16; k++) o_s[jl * 65 + 16 * g + k] = (int)d[k];
+        for (int k = 0; k < 32; k++) o_s[jl * 65 + q0 + k] = (int)d[k];
     }
-    tc_fence_antes();
     __syncthreads();
-    {
-        const int i = tid >> 3, d0 = (tid & 7) * 8;
+    for (int t = tid; t < NI * hd / 8; t += NTA) {                 // (whole warps: 64 or 16 columns of 64 rows)
+        const int i = t / (hd / 8), d0 = t % (hd / 8) * 8;
         int o[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) o[k] = (int)(((uint32_t)o_s[(d0 + k) * 65 + i] << 7) + (uint32_t)o_s[(64 + d0 + k) * 65 + i]);
-        const size_t lin = (size_t)(linha0 + i0 + i);
-        grava8(Oacc, Oe, Qm, QE, lin * D + h * HD + d0, lin * (D / 32) + (h * HD + d0) / 32, o, (emv - GA) - 8, kid, tid);
+        const size_t lin = (size_t)(linha0 + min(i0 + i, T - 1));
+        grava8(A.Oacc, A.Oe, A.Qm, A.QE, lin * D + h * hd + d0, lin * (D / 32) + (h * hd + d0) / 32, o, (emv - GA) - 8, kid, t, i0 + i < T);
     }
-    if (wid == 0) {
-        tc_fence_depois();
-        tmem_libera(tmem, 512);
-    }
-}
-// ex needs 64 * (T + 8) * 2 bytes, the output staging that reuses it 128 * 65 * 4
-inline size_t smem_frente_tc(int T) {
-    const size_t ex = (size_t)NI * (T + 8) * 2, os = 128 * 65 * 4;
-    return 1024 + 3 * TILE_A + TILE_Q3 + 2 * TILE_NI + 640 + (ex > os ? ex : os);
+    termina(S, 256);
 }
 
-// -------------------------------------------------------------------------------------------------- where stored P is zero
-// zm[bh][kt] = bit qt set when P (key-major, [BH*T][T]) has a non-zero among keys 64 kt .. 64 kt + 63 and queries 64 qt .. 64 qt + 63.
-// grid (ceil(T / 64), BH), 256 threads: 4 threads per key row, from the diagonal on (P is zero above it by construction).
-__global__ void __launch_bounds__(256) k_p_mapa(const uint8_t* __restrict__ P, int* __restrict__ zm, int T) {
+// -------------------------------------------------------------------------------------------------- backward
+// ops.py:222-258.  Two matrix-wide maxima of a head lie between its phases (ops.py:235,244), hence three kernels:
+//   k_ab_max     max |gP| over j <= i, and the map of the non-zero parts of P (blocks of their own in the same launch)
+//   k_ab_soma    gP' = rnd(gP, sh); s_lin; max |dS|
+//   k_ab_saida   dS' = rnd(P (gP' - s_lin), sh2); gq = dS' . k (query tiles), gk = dS'^T . q and gv = P^T . dO (key tiles)
+// Each computes gP = dO . v^T again on the tensor core; nothing T x T is kept anywhere.
+struct ArgsTras {
+    const uint8_t* P; int* Gacc; int16_t* Ge; int* est; int* sl; const int* em;      // em: [BH][4] = q, k, v, dO
+    int* zm;                                                                          // [BH][16]: per 64 keys, bit qt = P may have a non-zero among queries 64 qt .. 64 qt + 63
+    int8_t* Gm; int8_t* GE;                                                           // block output [M, 3D] instead of the raw one, or nullptr
+    int BH, T, H, D, hd, GA, limite, kid, blocos_mapa;
+};
+// The windows of a query tile / of a key tile in which stored P may be non-zero: everywhere else dS and P contribute nothing.  The first
+// window always counts; the bounded variant takes maxima over everything and keeps them all.
+__device__ __forceinline__ unsigned janelas_consulta(const ArgsTras& A, int bh, int qt) {
+    const int n = (qt * NI + NI - 1) / TJ + 1;
+    unsigned vivas = 1u;
+    for (int s = 1; s < n; s++) {                                  // keys of the tiles qt - 2 s - 1 and qt - 2 s
+        const int kt = qt - 2 * s;
+        int m = A.limite ? -1 : A.zm[bh * 16 + kt];
+        if (kt > 0 && !A.limite) m |= A.zm[bh * 16 + kt - 1];
+        if (m >> qt & 1) vivas |= 1u << s;
+    }
+    return vivas;
+}
+__device__ __forceinline__ unsigned janelas_chave(const ArgsTras& A, int bh, int kt) {
+    const int n = (A.T - kt * NI + TJ - 1) / TJ;
+    unsigned vivas = 1u;
+    if (n > 1) {
+        const int m = A.limite ? -1 : A.zm[bh * 16 + kt];
+        for (int s = 1; s < n; s++)
+            if (m >> (kt + 2 * s) & 3) vivas |= 1u << s;
+    }
+    return vivas;
+}
+
+// zm[bh][kt]: P (key-major, [BH*T][T]) from the query tile kt + 2 on; the two before it belong to the first window and count anyway.
+// One block per (head, key tile); a warp reads 8 key rows, 512 bytes at a time.
+__device__ void mapa_p(const ArgsTras& A, int bh, int kt, unsigned* ou) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, T = A.T;
+    unsigned m = 3u << kt;
+    if (tid == 0) *ou = 0;
+    __syncthreads();
+    for (int p = 4 * (kt + 2) + lane; p < T / 16; p += 32) {       // 16-byte pieces; piece p belongs to query tile p / 4
+        uint4 x[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int j = kt * NI + wid * 8 + r;                   // (a piece at or beyond the tile kt + 2 exists only if the whole key tile does)
+            x[r] = *reinterpret_cast<const uint4*>(A.P + ((size_t)bh * T + j) * T + 16 * p);
+        }
+        uint32_t o = 0;
+#pragma unroll
+        for (int r = 0; r < 8; r++) o |= x[r].x | x[r].y | x[r].z | x[r].w;
+        if (o) m |= 1u << (p >> 2);
+    }
+    m = __reduce_or_sync(FULL, m);
+    if (lane == 0) atomicOr(ou, m);
+    __syncthreads();
+    if (tid == 0) A.zm[bh * 16 + kt] = (int)*ou;
+}
+
+// Shared: dO digits 16 KB | two V windows 16 KB each; tensor memory: two score buffers.  The load of the window after next and the
+// product of the next one run behind the drain.
+constexpr uint32_t MX_V = 2 * TILE_N, MX_BAR = MX_V + 2 * TILE_A;
+constexpr size_t SM_MAX = 1024 + MX_BAR + 128;
+__global__ void __launch_bounds__(NTA, 2) k_ab_max(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
+    extern __shared__ unsigned char bruto[];
+    __shared__ int red[NTA / 32];
+    __shared__ unsigned ou;
+    const int T = A.T, nt = (T + NI - 1) / NI;
+    if ((int)blockIdx.x < A.blocos_mapa) {
+        pdl_espera();
+        pdl_solta();
+        mapa_p(A, blockIdx.x / nt, blockIdx.x % nt, &ou);
+        return;
+    }
+    enum { B_G = 0, B_V = 1, B_S = 3 };
+    const Base S = comeca(bruto, MX_BAR, 5, 256);
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane, kid = A.kid;
+    const int item = blockIdx.x - A.blocos_mapa, bh = item % A.BH, i0 = (nt - 1 - item / A.BH) * NI, j00 = i0 + NI - TJ, n = (i0 + NI - 1) / TJ + 1;
+    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
     pdl_espera();
     pdl_solta();
-    __shared__ unsigned ou;
-    const int tid = threadIdx.x, kt = blockIdx.x, bh = blockIdx.y, r = tid >> 2, parte = tid & 3, j = kt * NJ + r;
-    if (tid == 0) ou = 0;
-    __syncthreads();
-    unsigned m = 0;
-    if (j < T) {
-        const uint4* linha = reinterpret_cast<const uint4*>(P + ((size_t)bh * T + j) * T);
-        for (int p = 4 * kt + parte; p < T / 16; p += 4) {          // 16-byte pieces; piece p belongs to query tile p / 4
-            const uint4 v = linha[p];
-            if (v.x | v.y | v.z | v.w) m |= 1u << (p >> 2);
-        }
-    }
-    m = __reduce_or_sync(0xffffffffu, m);
-    if ((tid & 31) == 0 && m) atomicOr(&ou, m);
-    __syncthreads();
-    if (tid == 0) zm[bh * gridDim.x + kt] = (int)ou;
-}
-
-// -------------------------------------------------------------------------------------------------- backward, row tiles
-struct ArgsTrasTC {
-    const uint8_t* P; int* Gacc; int16_t* Ge; int* est; int* sl; const int* em;      // em: [BH][4] = q, k, v, dO
-    const int* zm;                                                                    // [BH][ceil(T/64)]: per 64 keys, bit qt = P has a non-zero among queries 64 qt .. 64 qt + 63
-    int8_t* DSh; int8_t* DSl;                                                         // [BH*T][T] digits of dS', key-major (transposed)
-    int8_t* Gm; int8_t* GE;                                                           // block output [M, 3D] instead of the raw one, or nullptr
-    int T, H, D, GA, limite, kid;
-};
-
-// FASE 1: max |gP| over j <= i.   FASE 2: s_lin and the maxima of dS (two sweeps over the keys).   FASE 3: dS' (digits to the
-// workspace, key-major, for the key-tile kernel) and gq = dS' . k.     grid (T / 64, BH), 512 threads.
-// Every sweep recomputes gP = dO . v^T on the tensor core; nothing T x T is kept in shared memory.
-// Tensor memory: two score buffers (3 x 64 columns each) + in phase 3 two output accumulators of 64 columns (512 allocated).
-template <int FASE>
-__global__ void __launch_bounds__(NTL) k_ab_linhas_tc(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG,
-                                                      const __grid_constant__ CUtensorMap mKt, const ArgsTrasTC A) {
-    extern __shared__ unsigned char bruto[];
-    // (pointer arithmetic on the array keeps the shared address space: a round trip through an integer makes every access generic)
-    unsigned char* smem = bruto + ((1024u - (smem_u32(bruto) & 1023u)) & 1023u);
-    const uint32_t sbase = smem_u32(smem);
-    // stages: V chunks [4] (a TMA load takes longer than a step of a sweep: loads run four steps ahead) | dO tile as loaded |
-    // dO tile stacked | (phase 3) K^T chunks [4] | dS' digit tiles [2][hi rows, lo rows]
-    constexpr int NSTV = 4;
-    constexpr uint32_t OFF_G = NSTV * TILE_A, OFF_G3 = OFF_G + TILE_NI, OFF_KT = OFF_G3 + TILE_Q3, OFF_DS = OFF_KT + (FASE == 3 ? NSTV * TILE_A : 0);
-    constexpr uint32_t OFF_BAR = OFF_DS + (FASE == 3 ? 4 * TILE_NI : 0);
-    const Barras bar = {sbase + OFF_BAR};                          // 0 dO | 1..4 v | 5,6 s | 7..10 kt | 11,12 gq done | 13 o
-    constexpr int B_V = 1, B_S = 5, B_KT = 7, B_G = 11, B_O = 13;
-    uint32_t* slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 112);
-    volatile int* aborta = reinterpret_cast<volatile int*>(smem + OFF_BAR + 116);
-    int* sl_s = reinterpret_cast<int*>(smem + OFF_BAR + 128);      // [64]
-    int* s_acc = sl_s + NI;                                        // [64]
-    __shared__ int red[NTL / 32];
-    const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid;
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int ordem = blockIdx.y * gridDim.x + blockIdx.x;
-    const int bh = ordem % gridDim.y, b = bh / H, h = bh % H, i0 = (gridDim.x - 1 - ordem / gridDim.y) * NI, linha0 = b * T;
-    int* est = A.est + bh * at::N_EST;
-    const int nproc = i0 + NI, nch = (nproc + TJ - 1) / TJ;
-    const uint32_t sG = sbase + OFF_G, sG3 = sbase + OFF_G3, sKt0 = sbase + OFF_KT;          // V stage s at sbase + s * TILE_A, K^T stage s at sKt0 + s * TILE_A
-    uint8_t* ds_b = smem + OFF_DS;                                 // [2 stages][hi rows | lo rows][64 x 128]
-    // first the operand loads (as soon as their barriers exist), then the small global reads, then tensor memory
-    if (tid == 0) {
-        for (int i = 0; i < 14; i++) mbar_init(bar[i], 1);
-        *aborta = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    pdl_espera();                                                  // the operands below are the previous kernel's outputs
-    pdl_solta();
-    if (tid == 0) {
-        mbar_expect_tx(bar[0], TILE_NI);
-        tma_2d(sG, &mG, 0, bh * T + i0, bar[0]);
-    }
-    // Key chunks in which stored P is zero for this query tile and its two neighbours (A.zm: per 64 keys, the 64-query tiles
-    // with a non-zero P) add nothing to s_lin, dS' and gq, and the key-tile kernel does not read their dS': phases 2 and 3 leave
-    // them out.  The diagonal chunk always stays; phase 1 (a maximum over every position) and the bounded variant keep them all.
-    unsigned vivos = (1u << nch) - 1u;
-    if (FASE != 1 && !A.limite && A.zm) {
-        const int qt = i0 / NI, nkt = (T + NJ - 1) / NJ;
-        const unsigned vizinhos = (7u << qt) >> 1;                 // query tiles qt - 1, qt, qt + 1
-        vivos = 1u << (nch - 1);
-        if (qt >= 1) vivos |= 1u << ((qt - 1) / 2);               // the chunk of key tile qt - 1: the key-tile kernel's first step reads it
-        for (int c = 0; c < nch - 1; c++) {
-            unsigned m = (unsigned)A.zm[bh * nkt + 2 * c];
-            if (2 * c + 1 < nkt) m |= (unsigned)A.zm[bh * nkt + 2 * c + 1];
-            if (m & vizinhos) vivos |= 1u << c;
-        }
-    }
-    const int nviv = __popc(vivos);
-    const int nvoltas = FASE == 2 ? 2 * nviv : nviv;               // phase 2 sweeps the keys twice
-    auto pedaco = [&](int cc) -> int { return (int)__fns(vivos, 0, cc % nviv + 1); };      // the live chunk of step cc
-    if (tid == 0) {
-        for (int c = 0; c < NSTV && c < nvoltas; c++) {
-            mbar_expect_tx(bar[B_V + c], TILE_A);
-            tma_2d(sbase + c * TILE_A, &mV, 0, bh * T + pedaco(c) * TJ, bar[B_V + c]);
-        }
-        if (FASE == 3)
-            for (int c = 0; c < 2 && c < nviv; c++) {
-                mbar_expect_tx(bar[B_KT + c], TILE_A);
-                tma_2d(sKt0 + c * TILE_A, &mKt, pedaco(c) * TJ, bh * 128, bar[B_KT + c]);
-            }
-    }
-    const int emk = A.em[bh * 4 + 1], emv = A.em[bh * 4 + 2], emg = A.em[bh * 4 + 3];
-    const int sh = FASE == 1 ? 0 : at::desl1(est, A.limite);
-    const int sh2 = FASE == 3 ? at::desl2(est, A.limite) : 0;
-    if (tid < NI) { s_acc[tid] = 0; sl_s[tid] = FASE == 3 ? A.sl[(size_t)bh * T + i0 + tid] : 0; }
-    if (wid == 0) tmem_aloca(slot, 512);
-    tc_fence_antes();
-    __syncthreads();
-    tc_fence_depois();
-    const uint32_t tmem = *slot;
-    const int nzero = min((nproc + NJ - 1) / NJ * NJ, T);          // phase 3 writes explicit zeros of dS' up to the key tile's end
-    auto emite = [&](int cc) -> bool {
-        if (!espera(bar[B_V + cc % NSTV], (cc / NSTV) & 1, aborta, kid, 31)) return false;
+    auto emite = [&](int s) -> bool {                              // one thread
+        if (!espera(S.bar[B_V + (s & 1)], (s >> 1) & 1, S.aborta, kid, 31)) return false;
         tc_fence_depois();
-        mma_digitos(tmem + (cc & 1) * SB, desc_sw128(sbase + (cc % NSTV) * TILE_A), desc_sw128(sG3));
-        tc_commit(bar[B_S + (cc & 1)]);
+        mma_escores(S.tmem + (s & 1) * SB, desc_sw128(S.s + MX_V + (s & 1) * TILE_A), desc_sw128(S.s));
+        tc_commit(S.bar[B_S + (s & 1)]);
         return true;
     };
-    int mgp = 0, mds = 0, mp = 0;
-    int s_part[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) s_part[k] = 0;
-    bool ok = __all_sync(FULL, espera(bar[0], 0, aborta, kid, 30));     // the dO tile has landed: stack its three arrangements
-    if (ok) empilha3(smem + OFF_G, smem + OFF_G3, tid);
-    fence_async();
-    __syncthreads();
-    if (tid == 0 && ok) ok = emite(0);
-    for (int cc = 0; cc < nvoltas; cc++) {
-        const int c = pedaco(cc), st = cc & 1;
-        if (tid == 0 && ok && cc + 1 < nvoltas) ok = emite(cc + 1);
+    bool ok = true;
+    if (tid == 0) {
+        carrega_dig(S.s, &mG, bh * T + i0, A.BH * T, S.bar[B_G]);
+        for (int s = 0; s < 2 && s < n; s++) carrega(S.s + MX_V + s * TILE_A, &mV, 0, bh * T + j00 - s * TJ, TILE_A, S.bar[B_V + s]);
+        ok = espera(S.bar[B_G], 0, S.aborta, kid, 30) && emite(0);
+    }
+    int mx = 0;
+    for (int s = 0; s < n; s++) {
         __syncwarp();
-        ok = __all_sync(FULL, ok && espera(bar[B_S + st], (cc >> 1) & 1, aborta, kid, 32));
+        ok = __all_sync(FULL, ok && espera(S.bar[B_S + (s & 1)], (s >> 1) & 1, S.aborta, kid, 32));
         tc_fence_depois();
-        if (tid == 0 && ok && cc + NSTV < nvoltas) {               // this step's MMAs are done: its stage takes the chunk of step cc + 4
-            mbar_expect_tx(bar[B_V + cc % NSTV], TILE_A);
-            tma_2d(sbase + (cc % NSTV) * TILE_A, &mV, 0, bh * T + pedaco(cc + NSTV) * TJ, bar[B_V + cc % NSTV]);
+        if (tid == 0 && ok) {                                      // this product is done: its V stage takes the window after next
+            if (s + 2 < n) carrega(S.s + MX_V + (s & 1) * TILE_A, &mV, 0, bh * T + j00 - (s + 2) * TJ, TILE_A, S.bar[B_V + (s & 1)]);
+            if (s + 1 < n) ok = emite(s + 1);
         }
-        if (FASE == 3) {
-            // the digit tiles of this parity and the K^T stage of chunk cc - 2 are free once that chunk's output MMAs are done;
-            // the stage takes chunk cc + 2 (the first two steps fill the stages nobody has used yet)
-            if (cc >= 2) ok = __all_sync(FULL, ok && espera(bar[B_G + st], ((cc - 2) >> 1) & 1, aborta, kid, 33));
-            if (tid == 0 && ok && cc + 2 < nviv) {
-                mbar_expect_tx(bar[B_KT + (cc + 2) % NSTV], TILE_A);
-                tma_2d(sKt0 + ((cc + 2) % NSTV) * TILE_A, &mKt, pedaco(cc + 2) * TJ, bh * 128, bar[B_KT + (cc + 2) % NSTV]);
-            }
-        }
-        if (FASE == 2 && cc == nviv) {
-            // between the sweeps: s_lin of the 32 rows from the per-thread partial sums
+        __syncwarp();
+        const int j = j00 - s * TJ + jl, kmin = j >= 0 && i0 + q0 < T ? j - i0 - q0 : 32;
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int s = warp_sum(s_part[k]);
-                if (lane == 0) atomicAdd(&s_acc[16 * (wid >> 2) + k], s);
-            }
-            __syncthreads();
-            if (tid < NI) {
-                const int sl = rnd_d(s_acc[tid], 8);
-                sl_s[tid] = sl;
-                A.sl[(size_t)bh * T + i0 + tid] = sl;
-            }
-            __syncthreads();
-        }
-        if (ok) {
-            const int jl = 32 * (wid & 3) + lane, g = wid >> 2, j = c * TJ + jl;
-            uint32_t hh[16], cr[16], ll[16];
-            tmem_le16x3(tmem + ((uint32_t)(32 * (wid & 3)) << 16) + st * SB + 16 * g, hh, cr, ll);
-            uint32_t pw[4] = {0, 0, 0, 0};
-            if (FASE != 1 && j < nproc) {
-                const uint4 w = *reinterpret_cast<const uint4*>(A.P + ((size_t)bh * T + j) * T + i0 + 16 * g);
-                pw[0] = w.x; pw[1] = w.y; pw[2] = w.z; pw[3] = w.w;
-            }
-            int dh[16], dl[16];
-            // A key counts for query i0 + 16 g + k when it exists for this tile (j < nproc) and is not beyond the diagonal, which only
-            // the last chunk can be: one comparison of k against a per-thread bound.  With both shifts in 1..30 the roundings are
-            // written out with their constants hoisted: rnd_d(x, s) = (x + 2^(s-1) - 1 + ((x >> s) & 1)) >> s.
-            const int kmin = j >= nproc ? 16 : (c == nch - 1 ? j - (i0 + 16 * g) : 0);      // dentro <=> k >= kmin
-            auto corpo = [&](auto rapido_t) {
-                constexpr bool RAP = decltype(rapido_t)::value;
-                const int meio1 = RAP && FASE != 1 ? (1 << max(sh - 1, 0)) - 1 : 0, meio2 = RAP && FASE == 3 ? (1 << max(sh2 - 1, 0)) - 1 : 0;
+        for (int g = 0; g < 2; g++) {
+            int x[16];
+            escores16(t_lane + (s & 1) * SB + q0 + 16 * g, x);
 #pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const bool dentro = k >= kmin;
-                    const int x = junta3(hh[k], cr[k], ll[k]);
-                    int gp;
-                    if (FASE == 1) gp = x;
-                    else if (RAP) gp = (x + meio1 + ((x >> sh) & 1)) >> sh;
-                    else gp = rnd_d(x, sh);
-                    gp = dentro ? gp : 0;
-                    if (FASE == 1 || (FASE == 2 && cc < nviv)) mgp = max(mgp, gp < 0 ? -gp : gp);
-                    if (FASE == 1) continue;
-                    const int p = (int)((pw[k >> 2] >> (8 * (k & 3))) & 0xff);
-                    if (FASE == 2) {
-                        if (cc < nviv) s_part[k] += p * gp;
-                        else {
-                            const int ds = p * (gp - sl_s[16 * g + k]);
-                            mds = max(mds, ds < 0 ? -ds : ds);
-                            mp = max(mp, p);
-                        }
-                    } else {
-                        const int y = p * (gp - sl_s[16 * g + k]);
-                        int ds;
-                        if (RAP) ds = (y + meio2 + ((y >> sh2) & 1)) >> sh2;
-                        else ds = rnd_d(y, sh2);
-                        ds = dentro ? ds : 0;
-                        digitos(ds, dh[k], dl[k]);
-                        ds_b[(2 * st) * TILE_NI + sw128(16 * g + k, jl)] = (uint8_t)dh[k];              // rows 0..63 of the stage's stacked tile
-                        ds_b[(2 * st + 1) * TILE_NI + sw128(16 * g + k, jl)] = (uint8_t)dl[k];          // rows 64..127
+            for (int k = 0; k < 16; k++) mx = max(mx, 16 * g + k >= kmin ? abs(x[k]) : 0);
+        }
+        tc_fence_antes();
+        __syncthreads();                                           // everyone has read this buffer: the product after next may write it
+    }
+    max_cta(mx, A.est + bh * at::N_EST + at::S_GP, red, tid);
+    termina(S, 256);
+}
+
+// rnd_d(x, s) for 0 <= s <= 30 with the constants of s hoisted: (x + 2^(s-1) - 1 + ((x >> s) & 1)) >> s, and x itself at s = 0.  The
+// shifts of the backward are bitlen(int) - 15 and bitlen(int) - 12, at most 20.
+struct Arred {
+    int s, meio, um;
+    __device__ explicit Arred(int s_) : s(s_), meio(s_ ? (1 << (s_ - 1)) - 1 : 0), um(s_ ? 1 : 0) {}
+    __device__ int operator()(int x) const { return (x + meio + ((x >> s) & um)) >> s; }
+};
+
+// Query tiles: s_lin and the maxima of dS.  With one live window gP' and P stay in registers between the two passes.
+// Shared: dO digits 16 KB | V window 16 KB; tensor memory: the scores.
+constexpr uint32_t SO_V = 2 * TILE_N, SO_BAR = SO_V + TILE_A;
+constexpr size_t SM_SOMA = 1024 + SO_BAR + 128 + 5 * NI * 4;
+__global__ void __launch_bounds__(NTA, 2) k_ab_soma(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
+    extern __shared__ unsigned char bruto[];
+    __shared__ int red[NTA / 32];
+    enum { B_G = 0, B_V = 1, B_S = 2 };
+    const Base S = comeca(bruto, SO_BAR, 3, SB);
+    int* r_s = reinterpret_cast<int*>(S.smem + SO_BAR + 128);      // [4 lane quarters][64] partial sums
+    int* sl_s = r_s + 4 * NI;                                      // [64]
+    const int T = A.T, kid = A.kid, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane;
+    const int qt = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y, i0 = qt * NI, j00 = i0 + NI - TJ;
+    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
+    int* est = A.est + bh * at::N_EST;
+    pdl_espera();
+    pdl_solta();
+    if (tid == 0) {
+        carrega_dig(S.s, &mG, bh * T + i0, A.BH * T, S.bar[B_G]);
+        carrega(S.s + SO_V, &mV, 0, bh * T + j00, TILE_A, S.bar[B_V]);
+    }
+    const unsigned vivas = janelas_consulta(A, bh, qt);
+    const bool uma = vivas == 1u;
+    const Arred arred(at::desl1(est, A.limite));
+    int v[32], minha = 0, mgp = 0, mds = 0, mp = 0, passo = 0;
+    uint32_t w[8];
+    bool ok = true;
+#pragma unroll 1
+    for (int fase = 0; fase < 2; fase++) {
+#pragma unroll 1
+        for (unsigned m = vivas; m; m &= m - 1) {
+            const int s = __ffs(m) - 1, j = j00 - s * TJ + jl;
+            if (fase == 0 || !uma) {
+                const bool ha = j >= 0 && j < T && i0 + q0 < T;
+                const int kmin = ha ? j - i0 - q0 : 32;            // the key counts for query k >= kmin
+#pragma unroll
+                for (int k = 0; k < 8; k++) w[k] = 0;
+                if (ha) {
+                    const uint4* p = reinterpret_cast<const uint4*>(A.P + ((size_t)bh * T + j) * T + i0 + q0);
+                    const uint4 a = p[0], c = p[1];
+                    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y; w[6] = c.z; w[7] = c.w;
+                }
+                if (passo) { tc_fence_antes(); __syncthreads(); }   // everyone has read the previous scores
+                if (tid == 0 && ok) {
+                    if (passo) carrega(S.s + SO_V, &mV, 0, bh * T + j00 - s * TJ, TILE_A, S.bar[B_V]);
+                    else ok = espera(S.bar[B_G], 0, S.aborta, kid, 33);
+                    ok = ok && espera(S.bar[B_V], passo & 1, S.aborta, kid, 34);
+                    if (ok) {
+                        tc_fence_depois();
+                        mma_escores(S.tmem, desc_sw128(S.s + SO_V), desc_sw128(S.s));
+                        tc_commit(S.bar[B_S]);
                     }
                 }
-            };
-            const bool rapido = FASE == 1 || (sh >= 1 && sh <= 30 && (FASE != 3 || (sh2 >= 1 && sh2 <= 30)));
-            if (rapido) corpo(std::true_type{});
-            else corpo(std::false_type{});
-            if (FASE == 3 && j < nzero) {
-                const size_t o = ((size_t)bh * T + j) * T + i0 + 16 * g;
-                grava16(A.DSh + o, dh);
-                grava16(A.DSl + o, dl);
+                __syncwarp();
+                ok = __all_sync(FULL, ok && espera(S.bar[B_S], passo & 1, S.aborta, kid, 35));
+                tc_fence_depois();
+                passo++;
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    int x[16];
+                    escores16(t_lane + q0 + 16 * g, x);
+#pragma unroll
+                    for (int k = 0; k < 16; k++) v[16 * g + k] = 16 * g + k >= kmin ? arred(x[k]) : 0;
+                }
+            }
+            if (fase == 0) {
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    if (A.limite) mgp = max(mgp, abs(v[k]));
+                    const int r = __reduce_add_sync(FULL, byte_u(w, k) * v[k]);
+                    minha += lane == k ? r : 0;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    const int p = byte_u(w, k);
+                    mds = max(mds, abs(p * (v[k] - sl_s[q0 + k])));
+                    if (A.limite) mp = max(mp, p);
+                }
             }
         }
-        if (FASE == 3) fence_async();
-        tc_fence_antes();
-        __syncthreads();
-        if (FASE == 3 && tid == 0 && ok) {
-            // gq^T[digit row of k][query] += K^T chunk . (dS' digits)^T: hi digits -> columns 0..63, lo digits -> 64..127
-            ok = espera(bar[B_KT + cc % NSTV], (cc / NSTV) & 1, aborta, kid, 34);
-            if (ok) {
-                tc_fence_depois();
-                const uint64_t da = desc_sw128(sKt0 + (cc % NSTV) * TILE_A), db = desc_sw128(sbase + OFF_DS + (2 * st) * TILE_NI);
-#pragma unroll
-                for (int q = 0; q < 4; q++) tc_mma_i8(tmem + 2 * SB, da + 2 * q, db + 2 * q, ID_S2, (cc | q) != 0);
-                tc_commit(bar[B_G + st]);
-                if (cc == nvoltas - 1) tc_commit(bar[B_O]);
+        if (fase == 0) {
+            r_s[quarto * NI + q0 + lane] = minha;
+            __syncthreads();
+            if (tid < NI) {
+                const int sl = rnd_d(r_s[tid] + r_s[NI + tid] + r_s[2 * NI + tid] + r_s[3 * NI + tid], 8);
+                sl_s[tid] = sl;
+                if (i0 + tid < T) A.sl[(size_t)bh * T + i0 + tid] = sl;
             }
+            __syncthreads();
         }
     }
-    if (FASE == 1) {
-        max_cta16(mgp, est + at::S_GP, red, tid);
-    } else if (FASE == 2) {
-        int msl = 0;
-        if (tid < NI) msl = sl_s[tid] < 0 ? -sl_s[tid] : sl_s[tid];
-        max_cta16(mds, est + at::S_DS, red, tid);
-        if (A.limite) {
-            max_cta16(mp, est + at::S_P, red, tid);
-            max_cta16(mgp, est + at::S_GPQ, red, tid);
-            max_cta16(msl, est + at::S_SL, red, tid);
-        }
-    } else {
-        __syncwarp();
-        ok = __all_sync(FULL, ok && espera(bar[B_O], 0, aborta, kid, 35));
-        tc_fence_depois();
-        int* o_s = reinterpret_cast<int*>(smem);                   // [2][128][65] over the dead operand stages
-        if (ok) {
-            uint32_t d1[16], d2[16];
-            const int dd = 32 * (wid & 3) + lane, g = wid >> 2;
-            const uint32_t t = tmem + ((uint32_t)(32 * (wid & 3)) << 16) + 2 * SB + 16 * g;
-            tmem_le16(t, d1);
-            tmem_le16(t + NI, d2);
-#pragma unroll
-            for (int k = 0; k < 16; k++) {
-                o_s[dd * 65 + 16 * g + k] = (int)d1[k];
-                o_s[128 * 65 + dd * 65 + 16 * g + k] = (int)d2[k];
+    max_cta(mds, est + at::S_DS, red, tid);
+    if (A.limite) {
+        max_cta(mp, est + at::S_P, red, tid);
+        max_cta(mgp, est + at::S_GPQ, red, tid);
+        max_cta(tid < NI && i0 + tid < T ? abs(sl_s[tid]) : 0, est + at::S_SL, red, tid);
+    }
+    termina(S, SB);
+}
+
+// The output kernel.  Three roles (blockIdx.z): 0 key tiles, gk; 1 query tiles, gq; 2 key tiles, gv.
+//   gq, gk: scores (lane = the other side's token in the window, column = the tile's token), dS' as digits into an MMA tile
+//           (hi rows 0..63, lo rows 64..127, 128 bytes of window), then D[digit row of k or q][hi | lo column] += X^T . dS'.
+//   gv:     dO^T . P only, both operands straight from memory.
+// Shared: tile digits 16 KB | window 16 KB | transposed window 16 KB | dS' 16 KB | P tile 8 KB (key tiles); the output staging goes
+// over the first four.  Tensor memory: scores 128 columns, output 128 (256 allocated: two blocks per SM).
+constexpr uint32_t SA_A = 2 * TILE_N, SA_X = SA_A + TILE_A, SA_D = SA_X + TILE_A, SA_P = SA_D + 2 * TILE_N, SA_BAR = SA_P + TILE_N;
+constexpr size_t SM_SAIDA = 1024 + SA_BAR + 128 + NI * 4;
+static_assert(2 * 128 * 65 * 4 <= SA_BAR, "the staging lies below the barriers");
+
+template <bool CHAVE>
+__device__ __forceinline__ void ab_saida(const Base& S, const CUtensorMap& mB, const CUtensorMap& mA, const CUtensorMap& mX, const CUtensorMap& mP,
+                                         const ArgsTras& A, int bh, int tile) {
+    enum { B_B = 0, B_A = 1, B_X = 2, B_S = 3, B_O = 4 };
+    int* sl_s = reinterpret_cast<int*>(S.smem + SA_BAR + 128);     // [64], query tiles
+    const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane;
+    const int b = bh / H, h = bh % H, t0 = tile * NI, w0 = CHAVE ? t0 : t0 + NI - TJ, wp = CHAVE ? TJ : -TJ;      // window s starts at token w0 + s wp
+    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
+    const int* est = A.est + bh * at::N_EST;
+    auto janela = [&](int s) {                                     // one thread: the operands of window s
+        const int t = w0 + s * wp;
+        carrega(S.s + SA_A, &mA, 0, bh * T + t, TILE_A, S.bar[B_A]);
+        mbar_expect_tx(S.bar[B_X], TILE_A + (CHAVE ? TILE_N : 0));
+        tma_2d(S.s + SA_X, &mX, t, bh * 128, S.bar[B_X]);
+        if (CHAVE) tma_2d(S.s + SA_P, &mP, t, bh * T + t0, S.bar[B_X]);
+    };
+    if (tid == 0) {
+        carrega_dig(S.s, &mB, bh * T + t0, A.BH * T, S.bar[B_B]);
+        janela(0);
+    }
+    const int sh = at::desl1(est, A.limite), sh2 = at::desl2(est, A.limite);
+    const Arred arred(sh), arred2(sh2);
+    const unsigned vivas = CHAVE ? janelas_chave(A, bh, tile) : janelas_consulta(A, bh, tile);
+    if (!CHAVE && tid < NI) sl_s[tid] = A.sl[(size_t)bh * T + min(t0 + tid, T - 1)];
+    if (!CHAVE) __syncthreads();
+    int passo = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (unsigned m = vivas; m; m &= m - 1, passo++) {
+        const int s = __ffs(m) - 1, t = w0 + s * wp + jl;          // this thread's token of the window
+        if (passo) ok = __all_sync(FULL, ok && espera(S.bar[B_O], (passo - 1) & 1, S.aborta, kid, 36));      // every operand is free again
+        if (tid == 0 && ok) {
+            if (passo) janela(s);
+            else ok = espera(S.bar[B_B], 0, S.aborta, kid, 37);
+            ok = ok && espera(S.bar[B_A], passo & 1, S.aborta, kid, 38);
+            if (ok) {
+                tc_fence_depois();
+                mma_escores(S.tmem, desc_sw128(S.s + SA_A), desc_sw128(S.s));
+                tc_commit(S.bar[B_S]);
             }
         }
+        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        int sl = 0;
+        if (CHAVE) sl = A.sl[(size_t)bh * T + min(t, T - 1)];      // (a query beyond T has P = 0, the fill value)
+        else if (t >= 0 && t < T && t0 + q0 < T) {
+            const uint4* p = reinterpret_cast<const uint4*>(A.P + ((size_t)bh * T + t) * T + t0 + q0);
+            const uint4 a = p[0], c = p[1];
+            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y; w[6] = c.z; w[7] = c.w;
+        }
+        __syncwarp();
+        ok = __all_sync(FULL, ok && (!CHAVE || espera(S.bar[B_X], passo & 1, S.aborta, kid, 39)) && espera(S.bar[B_S], passo & 1, S.aborta, kid, 40));
+        tc_fence_depois();
+        const int dist = CHAVE ? t - t0 - q0 : t0 + q0 - t;        // query minus key at column q0
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+            int x[16];
+            escores16(t_lane + q0 + 16 * g, x);
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const int kk = 16 * g + k;
+                const int p = CHAVE ? S.smem[SA_P + sw128(q0 + kk, jl)] : byte_u(w, kk);
+                const int y = p * (arred(x[k]) - (CHAVE ? sl : sl_s[q0 + kk]));
+                const int ds = (CHAVE ? kk <= dist : kk >= -dist) ? arred2(y) : 0;
+                int hi, lo;
+                digitos(ds, hi, lo);
+                S.smem[SA_D + sw128(q0 + kk, jl)] = (uint8_t)hi;
+                S.smem[SA_D + TILE_N + sw128(q0 + kk, jl)] = (uint8_t)lo;
+            }
+        }
+        fence_async();
         tc_fence_antes();
         __syncthreads();
-        const int i = tid >> 3, d0 = (tid & 7) * 8;
-        const int eds = (emg - GA) + (emv - GA) + sh - 9 + sh2, e = eds + (emk - GA);
+        if (tid == 0 && ok) {
+            ok = CHAVE || espera(S.bar[B_X], passo & 1, S.aborta, kid, 41);
+            if (ok) {
+                tc_fence_depois();
+                const uint64_t da = desc_sw128(S.s + SA_X), db = desc_sw128(S.s + SA_D);
+#pragma unroll
+                for (int q = 0; q < 4; q++) tc_mma_i8(S.tmem + SB, da + 2 * q, db + 2 * q, ID_S, (passo | q) != 0);
+                tc_commit(S.bar[B_O]);
+            }
+        }
+        __syncwarp();
+    }
+    ok = __all_sync(FULL, ok && espera(S.bar[B_O], (passo - 1) & 1, S.aborta, kid, 42));
+    tc_fence_depois();
+    int* o_s = reinterpret_cast<int*>(S.smem);                     // [2: columns of the hi digits, of the lo digits][128 digit rows][65]
+    if (ok) {
+#pragma unroll
+        for (int a = 0; a < 2; a++) {
+            uint32_t d[32];
+            tmem_le32(t_lane + SB + NI * a + q0, d);
+#pragma unroll
+            for (int k = 0; k < 32; k++) o_s[(a * 128 + jl) * 65 + q0 + k] = (int)d[k];
+        }
+    }
+    __syncthreads();
+    const int emz = A.em[bh * 4 + (CHAVE ? 0 : 1)], emv = A.em[bh * 4 + 2], emg = A.em[bh * 4 + 3];
+    const int e = (emg - GA) + (emv - GA) + sh - 9 + sh2 + (emz - GA), col = (CHAVE ? D : 0) + h * hd;
+    for (int n = tid; n < NI * hd / 8; n += NTA) {                 // (whole warps)
+        const int r = n / (hd / 8), d0 = n % (hd / 8) * 8;
         int o[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const int d = d0 + k;
-            const uint32_t hhv = (uint32_t)o_s[d * 65 + i], crv = (uint32_t)o_s[(64 + d) * 65 + i] + (uint32_t)o_s[128 * 65 + d * 65 + i],
-                           llv = (uint32_t)o_s[128 * 65 + (64 + d) * 65 + i];
-            o[k] = junta3(hhv, crv, llv);
+            const int* p = o_s + (d0 + k) * 65 + r;
+            o[k] = junta3((uint32_t)p[0], (uint32_t)p[64 * 65] + (uint32_t)p[128 * 65], (uint32_t)p[192 * 65]);
         }
-        const size_t lin = (size_t)(linha0 + i0 + i);
-        grava8(A.Gacc, A.Ge, A.Gm, A.GE, lin * 3 * D + h * HD + d0, lin * (3 * D / 32) + (h * HD + d0) / 32, o, e, kid, tid);
-    }
-    tc_fence_antes();
-    __syncthreads();
-    if (wid == 0) {
-        tc_fence_depois();
-        tmem_libera(tmem, 512);
+        const size_t lin = (size_t)(b * T + min(t0 + r, T - 1));
+        grava8(A.Gacc, A.Ge, A.Gm, A.GE, lin * 3 * D + col + d0, lin * (3 * D / 32) + (col + d0) / 32, o, e, kid, n, t0 + r < T);
     }
 }
-inline size_t smem_linhas_tc(int fase) { return 1024 + 4 * TILE_A + TILE_NI + TILE_Q3 + (fase == 3 ? 4 * TILE_A + 4 * TILE_NI : 0) + 640; }
-
-// -------------------------------------------------------------------------------------------------- backward, key tiles
-// gk[j] = sum_i dS'[i][j] q[i], gv[j] = sum_i P[i][j] dO[i] for the 64 keys of the tile, over the query chunks from the tile's first
-// key on (everything before is causally zero).  All five operands come by TMA: q^T and dO^T digit rows (A), the tile's rows of the
-// dS' digits and of P (B).  grid (ceil(T / 64), BH), 256 threads; tensor memory: three accumulators of 64 columns (256 allocated).
-__global__ void __launch_bounds__(256) k_ab_colunas_tc(const __grid_constant__ CUtensorMap mQt, const __grid_constant__ CUtensorMap mGt,
-                                                       const __grid_constant__ CUtensorMap mDh, const __grid_constant__ CUtensorMap mDl,
-                                                       const __grid_constant__ CUtensorMap mP, const ArgsTrasTC A) {
-    extern __shared__ unsigned char bruto[];
-    // (pointer arithmetic on the array keeps the shared address space: a round trip through an integer makes every access generic)
-    unsigned char* smem = bruto + ((1024u - (smem_u32(bruto) & 1023u)) & 1023u);
-    const uint32_t sbase = smem_u32(smem);
-    constexpr int NSTC = 3;                                        // a TMA load takes longer than a step: loads run two steps ahead
-    constexpr uint32_t STAGE = 2 * TILE_A + 3 * TILE_NJ, OFF_BAR = NSTC * STAGE;
-    const Barras bar = {sbase + OFF_BAR};                          // 0..2 full | 3..5 free | 6 o
-    uint32_t* slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 64);
-    volatile int* aborta = reinterpret_cast<volatile int*>(smem + OFF_BAR + 68);
-    const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid;
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int ordem = blockIdx.y * gridDim.x + blockIdx.x;         // heaviest (first) key tiles of all heads first
-    const int bh = ordem % gridDim.y, b = bh / H, h = bh % H, j0 = (ordem / gridDim.y) * NJ, linha0 = b * T;
-    const int* est = A.est + bh * at::N_EST;
-    const int nq = (T - j0 + TJ - 1) / TJ;
-    auto carrega = [&](int n, int c) {                             // one thread: the five operand tiles of query chunk c, step n
-        const uint32_t s = sbase + (n % NSTC) * STAGE, f = bar[n % NSTC];
-        const int ic = j0 + c * TJ;
-        mbar_expect_tx(f, STAGE);
-        tma_2d(s, &mQt, ic, bh * 128, f);
-        tma_2d(s + TILE_A, &mGt, ic, bh * 128, f);
-        tma_2d(s + 2 * TILE_A, &mDh, ic, bh * T + j0, f);
-        tma_2d(s + 2 * TILE_A + TILE_NJ, &mDl, ic, bh * T + j0, f);
-        tma_2d(s + 2 * TILE_A + 2 * TILE_NJ, &mP, ic, bh * T + j0, f);
-    };
+__device__ __forceinline__ void ab_valor(const Base& S, const CUtensorMap& mX, const CUtensorMap& mP, const ArgsTras& A, int bh, int tile) {
+    enum { B_X = 0, B_O = 2 };                                     // two stages
+    constexpr uint32_t EST = TILE_A + TILE_N;
+    const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane;
+    const int b = bh / H, h = bh % H, t0 = tile * NI;
+    const unsigned vivas = janelas_chave(A, bh, tile);
+    const int n = __popc(vivas);
+    bool ok = true;
     if (tid == 0) {
-        for (int i = 0; i < 7; i++) mbar_init(bar[i], 1);
-        *aborta = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    pdl_espera();                                                  // the operands are the previous kernels' outputs
-    pdl_solta();
-    // query chunks (128 queries from j0 + 128 c) in which stored P is zero for this key tile add nothing to gk and gv, and phase 3
-    // wrote no dS' there: they are left out.  The first step (the diagonal) always stays.
-    unsigned vivos = (1u << nq) - 1u;
-    if (!A.limite && A.zm) {
-        const unsigned m = (unsigned)A.zm[bh * ((T + NJ - 1) / NJ) + j0 / NJ];
-        vivos = 1u;
-        for (int c = 1; c < nq; c++)
-            if (m & (3u << ((j0 + c * TJ) / NI))) vivos |= 1u << c;
-    }
-    const int nviv = __popc(vivos);
-    auto passo = [&](int n) -> int { return (int)__fns(vivos, 0, n + 1); };      // the query chunk of live step n
-    if (tid == 0)                                                  // the loads go out before anything else
-        for (int n = 0; n < NSTC && n < nviv; n++) carrega(n, passo(n));
-    if (wid == 0) tmem_aloca(slot, 256);
-    tc_fence_antes();
-    __syncthreads();
-    tc_fence_depois();
-    const uint32_t tmem = *slot;
-    if (tid == 0) {
-        bool ok = true;
-        for (int c = 0; c < nviv && ok; c++) {                      // c counts the live steps
-            ok = espera(bar[c % NSTC], (c / NSTC) & 1, aborta, kid, 40);
+        auto janela = [&](int passo) {
+            const int t = t0 + ((int)__fns(vivas, 0, passo + 1)) * TJ;
+            const uint32_t d = S.s + (passo & 1) * EST, f = S.bar[B_X + (passo & 1)];
+            mbar_expect_tx(f, EST);
+            tma_2d(d, &mX, t, bh * 128, f);
+            tma_2d(d + TILE_A, &mP, t, bh * T + t0, f);
+        };
+        janela(0);
+        if (n > 1) janela(1);
+        for (int c = 0; c < n && ok; c++) {
+            ok = espera(S.bar[B_X + (c & 1)], (c >> 1) & 1, S.aborta, kid, 43);
             if (!ok) break;
             tc_fence_depois();
-            const uint32_t s = sbase + (c % NSTC) * STAGE;
-            // the hi and lo digit tiles of dS' lie one after the other: one B operand of 128 rows -> columns 0..63 | 64..127
-            const uint64_t dq = desc_sw128(s), dg = desc_sw128(s + TILE_A), dhl = desc_sw128(s + 2 * TILE_A), dp = desc_sw128(s + 2 * TILE_A + 2 * TILE_NJ);
+            const uint64_t da = desc_sw128(S.s + (c & 1) * EST), db = desc_sw128(S.s + (c & 1) * EST + TILE_A);
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                tc_mma_i8(tmem, dq + 2 * q, dhl + 2 * q, ID_C2, (c | q) != 0);
-                tc_mma_i8(tmem + 128, dg + 2 * q, dp + 2 * q, ID_CU, (c | q) != 0);
-            }
-            tc_commit(bar[NSTC + c % NSTC]);
-            if (c >= 1 && c + 2 < nviv) {                          // step c - 1's MMAs done: its stage takes step c + 2
-                ok = espera(bar[NSTC + (c - 1) % NSTC], ((c - 1) / NSTC) & 1, aborta, kid, 41);
-                if (ok) carrega(c + 2, passo(c + 2));
-            }
+            for (int q = 0; q < 4; q++) tc_mma_i8(S.tmem, da + 2 * q, db + 2 * q, ID_PU, (c | q) != 0);
+            tc_commit(S.bar[B_O]);
+            if (c + 1 < n) ok = espera(S.bar[B_O], c & 1, S.aborta, kid, 44);
+            if (c + 2 < n && ok) janela(c + 2);
         }
-        tc_commit(bar[2 * NSTC]);
     }
     __syncwarp();
-    const bool ok = __all_sync(FULL, espera(bar[2 * NSTC], 0, aborta, kid, 42));
+    ok = __all_sync(FULL, ok);
+    ok = __syncthreads_and(ok) && __all_sync(FULL, espera(S.bar[B_O], (n - 1) & 1, S.aborta, kid, 45));
     tc_fence_depois();
-    int* o_s = reinterpret_cast<int*>(smem);                       // [3][128][65] over the dead stages
+    int* o_s = reinterpret_cast<int*>(S.smem);                     // [128 digit rows][65]
     if (ok) {
-        const int dd = 32 * (wid & 3) + lane, g = wid >> 2;        // 32 of the 64 columns per thread
+        uint32_t d[32];
+        tmem_le32(S.tmem + ((uint32_t)(32 * quarto) << 16) + q0, d);
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            uint32_t d[32];
-            tmem_le32(tmem + ((uint32_t)(32 * (wid & 3)) << 16) + 64 * a + 32 * g, d);
-#pragma unroll
-            for (int k = 0; k < 32; k++) o_s[(a * 128 + dd) * 65 + 32 * g + k] = (int)d[k];
-        }
+        for (int k = 0; k < 32; k++) o_s[jl * 65 + q0 + k] = (int)d[k];
     }
-    tc_fence_antes();
     __syncthreads();
-    {
-        const int sh = at::desl1(est, A.limite), sh2 = at::desl2(est, A.limite);
-        const int emq = A.em[bh * 4], emv = A.em[bh * 4 + 2], emg = A.em[bh * 4 + 3];
-        const int ego = emg - GA, eds = ego + (emv - GA) + sh - 9 + sh2, e_k = eds + (emq - GA), e_v = ego - 8;
-        for (int t = tid; t < NJ * 8; t += 256) {
-            const int jl = t >> 3, d0 = (t & 7) * 8, j = min(j0 + jl, T - 1);      // rows beyond T (whole groups of 8 lanes) compute and store nothing
-            const bool grava = j0 + jl < T;
-            int gk[8], gv[8];
+    const int e = A.em[bh * 4 + 3] - GA - 8, col = 2 * D + h * hd;
+    for (int t = tid; t < NI * hd / 8; t += NTA) {                 // (whole warps)
+        const int r = t / (hd / 8), d0 = t % (hd / 8) * 8;
+        int o[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int d = d0 + k;
-                const uint32_t hhv = (uint32_t)o_s[d * 65 + jl], crv = (uint32_t)o_s[(64 + d) * 65 + jl] + (uint32_t)o_s[(128 + d) * 65 + jl],
-                               llv = (uint32_t)o_s[(128 + 64 + d) * 65 + jl];
-                gk[k] = junta3(hhv, crv, llv);
-                gv[k] = (int)(((uint32_t)o_s[(256 + d) * 65 + jl] << 7) + (uint32_t)o_s[(256 + 64 + d) * 65 + jl]);
-            }
-            const size_t lin = (size_t)(linha0 + j), p = lin * 3 * D + D + h * HD + d0, pe = lin * (3 * D / 32) + (D + h * HD + d0) / 32;
-            grava8(A.Gacc, A.Ge, A.Gm, A.GE, p, pe, gk, e_k, kid, t, grava);
-            grava8(A.Gacc, A.Ge, A.Gm, A.GE, p + D, pe + D / 32, gv, e_v, kid, t, grava);
-        }
-    }
-    if (wid == 0) {
-        tc_fence_depois();
-        tmem_libera(tmem, 256);
+        for (int k = 0; k < 8; k++) o[k] = (int)(((uint32_t)o_s[(d0 + k) * 65 + r] << 7) + (uint32_t)o_s[(64 + d0 + k) * 65 + r]);
+        const size_t lin = (size_t)(b * T + min(t0 + r, T - 1));
+        grava8(A.Gacc, A.Ge, A.Gm, A.GE, lin * 3 * D + col + d0, lin * (3 * D / 32) + (col + d0) / 32, o, e, kid, t, t0 + r < T);
     }
 }
-inline size_t smem_colunas_tc() { return 1024 + 3 * (2 * TILE_A + 3 * TILE_NJ) + 128; }
+__global__ void __launch_bounds__(NTA, 2) k_ab_saida(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG,
+                                                     const __grid_constant__ CUtensorMap mVd, const __grid_constant__ CUtensorMap mGd,
+                                                     const __grid_constant__ CUtensorMap mKt, const __grid_constant__ CUtensorMap mQt,
+                                                     const __grid_constant__ CUtensorMap mGt, const __grid_constant__ CUtensorMap mP, const ArgsTras A) {
+    extern __shared__ unsigned char bruto[];
+    const Base S = comeca(bruto, SA_BAR, 5, 256);
+    pdl_espera();
+    pdl_solta();
+    const int bh = blockIdx.y;
+    if (blockIdx.z == 0) ab_saida<true>(S, mVd, mG, mQt, mP, A, bh, blockIdx.x);
+    else if (blockIdx.z == 1) ab_saida<false>(S, mGd, mV, mKt, mP, A, bh, gridDim.x - 1 - blockIdx.x);
+    else ab_valor(S, mGt, mP, A, bh, blockIdx.x);
+    termina(S, 256);
+}
 
 }  // namespace atc
 
 // -------------------------------------------------------------------------------------------------- host side
 static size_t atc_arredonda(size_t x) { return (x + 1023) & ~(size_t)1023; }
 
-// head dimension 64, whole row tiles of 64 queries and at least one full key chunk (the TMA boxes are 128 tokens wide)
-static bool atc_serve(int blk, int T, int H, int D) { return D == H * atc::HD && T % atc::NI == 0 && T >= 128 && T <= 1024 && D % blk == 0 && (blk == 32 || blk == 128); }
+// head dimension 64 or 16; the aligned operands fit f16 exactly up to 4 guard bits (127 << 4 = 2032)
+static bool atc_serve(int blk, int T, int H, int D, int GA) {
+    return (D == H * 64 || D == H * 16) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 && (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
+}
+// pieces of 128 tokens per preparation block: as many as leave two blocks per SM
+static int atc_por_cta(int T, int BH, int z) {
+    const int np = (T + 127) / 128;
+    int por = 1;
+    while (por < np && (long long)((np + 2 * por - 1) / (2 * por)) * BH * z >= 4 * N_SM) por *= 2;
+    return por;
+}
 
-// forward: preparation (q, k row layout; v transposed) + the tensor-core kernel
-// Qm / QE: block output (jt_quant of the raw output) instead of Oacc / Oe, block length 32 only; nullptr = raw output
+// forward: preparation (q digits, k plain, v transposed), then the kernel
+// Qm / QE: block output (jt_quant of the raw output) instead of Oacc / Oe, block length 32 and head dimension 64 only; nullptr = raw output
 static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* Oacc, int16_t* Oe, int8_t* Qm, int8_t* QE, uint8_t* P, int Bt, int T, int H,
                              int D, int GA, int kid, cudaStream_t st) {
-    if (Qm && (blk != 32 || !QE)) return (int)cudaErrorInvalidValue;
-    const int BH = Bt * H;
+    if (Qm && (blk != 32 || !QE || D != H * 64)) return (int)cudaErrorInvalidValue;
+    const int BH = Bt * H, hd = D / H;
     // head-maximum exponents [BH][4], then the largest squared row norms of q and k per 128 tokens [BH][2][ceil(T/128)]
     const size_t b_em = atc_arredonda((size_t)BH * 16 + (size_t)BH * 2 * ((T + 127) / 128) * 4), b_lin = atc_arredonda((size_t)BH * T * 128);
     unsigned char* ws = nullptr;
-    if (int r = at_ws(b_em + 3 * b_lin, st, reinterpret_cast<void**>(&ws))) return r;
+    if (int r = at_ws(b_em + 4 * b_lin, st, reinterpret_cast<void**>(&ws))) return r;
     int* em = reinterpret_cast<int*>(ws);
-    int8_t *Q2 = reinterpret_cast<int8_t*>(ws + b_em), *K2 = Q2 + b_lin, *Vt2 = K2 + b_lin;
-    atc::ArgsPrep Pp = {qm, qE, nullptr, nullptr, {Q2, K2, nullptr, nullptr}, {nullptr, nullptr, Vt2, nullptr}, em, nullptr, T > 2 * atc::TJ ? em + 4 * BH : nullptr, T, H, D, GA, blk};
-    lanca_pdl(atc::k_at_prep, dim3(dim3((T + 127) / 128, BH, 3)), dim3(256), 0, st, Pp);
+    int* nrm = em + 4 * BH;
+    uint16_t *Qd = reinterpret_cast<uint16_t*>(ws + b_em), *K = reinterpret_cast<uint16_t*>(ws + b_em + 2 * b_lin);
+    int8_t* Vt = reinterpret_cast<int8_t*>(ws + b_em + 3 * b_lin);
+    const int por = atc_por_cta(T, BH, 3);
+    atc::ArgsPrep Pp = {qm, qE, nullptr, nullptr, {nullptr, K, nullptr, nullptr}, {Qd, nullptr, nullptr, nullptr}, {nullptr, nullptr, Vt, nullptr},
+                        em, nullptr, nrm, BH, T, H, D, hd, GA, blk, por};
+    lanca_pdl(atc::k_at_prep, dim3(((T + 127) / 128 + por - 1) / por, BH, 3), dim3(256), 0, st, Pp);
     CUtensorMap mQ, mK, mVt;
-    if (!(faz_mapa(&mQ, Q2, BH * T, 128, atc::NI) && faz_mapa(&mK, K2, BH * T, 128, 128) && faz_mapa(&mVt, Vt2, BH * 128, T, 128)))
+    if (!(faz_mapa_h(&mQ, Qd, 2 * BH * T, 64, atc::NI) && faz_mapa_h(&mK, K, BH * T, 64, 128) && faz_mapa(&mVt, Vt, BH * 128, T, 128)))
         return (int)cudaErrorInvalidValue;
-    const size_t sm = atc::smem_frente_tc(T);
-    cudaError_t c = at_smem(atc::k_atencao_tc, sm);
+    cudaError_t c = at_smem(atc::k_at_frente, atc::SM_FRENTE);
     if (c != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_atencao_tc, dim3(dim3(T / atc::NI, BH)), dim3(atc::NTL), sm, st, mQ, mK, mVt, em, Oacc, Oe, Qm, QE, P, T, H, D, GA, kid);
+    const atc::ArgsFrente A = {em, nrm, Oacc, Oe, Qm, QE, P, BH, T, H, D, hd, GA, kid};
+    lanca_pdl(atc::k_at_frente, dim3((T + atc::NI - 1) / atc::NI, BH), dim3(atc::NTA), atc::SM_FRENTE, st, mQ, mK, mVt, A);
     return (int)cudaGetLastError();
 }
 
-// backward: preparation (v, dO row layout; q, k, dO transposed), the three row-tile phases, the key-tile kernel
+// backward: preparation (v, dO plain and digits; q, k, dO transposed), the maxima, the sums, the outputs
 static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const int8_t* qm, const int8_t* qE, const uint8_t* P, int* Gacc, int16_t* Ge,
                            int8_t* Gm, int8_t* GE, int Bt, int T, int H, int D, int GA, int limite, int kid, cudaStream_t st) {
-    if (Gm && (blk != 32 || !GE)) return (int)cudaErrorInvalidValue;
-    const int BH = Bt * H;
-    const size_t b_est = atc_arredonda((size_t)BH * (at::N_EST + T + 4 + 16) * sizeof(int)), b_lin = atc_arredonda((size_t)BH * T * 128),
-                 b_ds = atc_arredonda((size_t)BH * T * T);
+    if (Gm && (blk != 32 || !GE || D != H * 64)) return (int)cudaErrorInvalidValue;
+    const int BH = Bt * H, hd = D / H, nt = (T + atc::NI - 1) / atc::NI;
+    const size_t b_est = atc_arredonda((size_t)BH * (at::N_EST + T + 4 + 16) * sizeof(int)), b_lin = atc_arredonda((size_t)BH * T * 128);
     unsigned char* ws = nullptr;
-    if (int r = at_ws(b_est + 5 * b_lin + 2 * b_ds, st, reinterpret_cast<void**>(&ws))) return r;
+    if (int r = at_ws(b_est + 9 * b_lin, st, reinterpret_cast<void**>(&ws))) return r;
     int* est = reinterpret_cast<int*>(ws);
     int* sl = est + (size_t)BH * at::N_EST;
     int* em = sl + (size_t)BH * T;
-    int* zm = em + (size_t)BH * 4;                               // [BH][ceil(T/64)] (T <= 1024: at most 16 per head)
-    int8_t *V2 = reinterpret_cast<int8_t*>(ws + b_est), *G2 = V2 + b_lin, *Qt2 = G2 + b_lin, *Kt2 = Qt2 + b_lin, *Gt2 = Kt2 + b_lin;
-    int8_t *DSh = Gt2 + b_lin, *DSl = DSh + b_ds;
-    cudaError_t c;
-    atc::ArgsPrep Pp = {qm, qE, gom, goE, {nullptr, nullptr, V2, G2}, {Qt2, Kt2, nullptr, Gt2}, em, est, nullptr, T, H, D, GA, blk};
-    lanca_pdl(atc::k_at_prep, dim3(dim3((T + 127) / 128, BH, 4)), dim3(256), 0, st, Pp);
-    CUtensorMap mV, mG, mKt, mQt, mGt, mDh, mDl, mP;
-    if (!(faz_mapa(&mV, V2, BH * T, 128, 128) && faz_mapa(&mG, G2, BH * T, 128, atc::NI) && faz_mapa(&mKt, Kt2, BH * 128, T, 128) &&
-          faz_mapa(&mQt, Qt2, BH * 128, T, 128) && faz_mapa(&mGt, Gt2, BH * 128, T, 128) && faz_mapa(&mDh, DSh, BH * T, T, atc::NJ) &&
-          faz_mapa(&mDl, DSl, BH * T, T, atc::NJ) && faz_mapa(&mP, P, BH * T, T, atc::NJ)))
+    int* zm = em + (size_t)BH * 4;
+    auto parte = [&](int n) { return ws + b_est + n * b_lin; };
+    uint16_t *V = (uint16_t*)parte(0), *G = (uint16_t*)parte(1), *Vd = (uint16_t*)parte(2), *Gd = (uint16_t*)parte(4);
+    int8_t *Qt = (int8_t*)parte(6), *Kt = (int8_t*)parte(7), *Gt = (int8_t*)parte(8);
+    const int por = atc_por_cta(T, BH, 4);
+    atc::ArgsPrep Pp = {qm, qE, gom, goE, {nullptr, nullptr, V, G}, {nullptr, nullptr, Vd, Gd}, {Qt, Kt, nullptr, Gt},
+                        em, est, nullptr, BH, T, H, D, hd, GA, blk, por};
+    lanca_pdl(atc::k_at_prep, dim3(((T + 127) / 128 + por - 1) / por, BH, 4), dim3(256), 0, st, Pp);
+    CUtensorMap mV, mG, mVd, mGd, mKt, mQt, mGt, mP;
+    if (!(faz_mapa_h(&mV, V, BH * T, 64, 128) && faz_mapa_h(&mG, G, BH * T, 64, 128) && faz_mapa_h(&mVd, Vd, 2 * BH * T, 64, atc::NI) &&
+          faz_mapa_h(&mGd, Gd, 2 * BH * T, 64, atc::NI) && faz_mapa(&mKt, Kt, BH * 128, T, 128) && faz_mapa(&mQt, Qt, BH * 128, T, 128) &&
+          faz_mapa(&mGt, Gt, BH * 128, T, 128) && faz_mapa(&mP, P, BH * T, T, atc::NI)))
         return (int)cudaErrorInvalidValue;
-    // the map of zero tiles of P pays from three key chunks on (T > 256): below that nearly every chunk is next to the diagonal
-    const bool com_mapa = !limite && T > 256;
-    atc::ArgsTrasTC A = {P, Gacc, Ge, est, sl, em, com_mapa ? zm : nullptr, DSh, DSl, Gm, GE, T, H, D, GA, limite, kid};
-    if (com_mapa) lanca_pdl(atc::k_p_mapa, dim3((T + atc::NJ - 1) / atc::NJ, BH), dim3(256), 0, st, P, zm, T);
-    const dim3 grade(T / atc::NI, BH);
+    // up to two key tiles the first window is all there is: no map
+    const atc::ArgsTras A = {P, Gacc, Ge, est, sl, em, zm, Gm, GE, BH, T, H, D, hd, GA, limite, kid, nt > 2 ? BH * nt : 0};
+    cudaError_t c;
     if (limite) {
         at::ArgsTras L = {gom, goE, qm, qE, P, Gacc, Ge, est, sl, nullptr, T, H, D, GA, blk, limite, kid};
-        at::k_lim<atc::HD><<<BH, 256, 0, st>>>(L);
+        if (hd == 64) at::k_lim<64><<<BH, 256, 0, st>>>(L);
+        else at::k_lim<16><<<BH, 256, 0, st>>>(L);
     } else {
-        if ((c = at_smem(atc::k_ab_linhas_tc<1>, atc::smem_linhas_tc(1))) != cudaSuccess) return (int)c;
-        lanca_pdl(atc::k_ab_linhas_tc<1>, dim3(grade), dim3(atc::NTL), atc::smem_linhas_tc(1), st, mV, mG, mKt, A);
+        if ((c = at_smem(atc::k_ab_max, atc::SM_MAX)) != cudaSuccess) return (int)c;
+        lanca_pdl(atc::k_ab_max, dim3(A.blocos_mapa + BH * nt), dim3(atc::NTA), atc::SM_MAX, st, mV, mGd, A);
     }
-    if ((c = at_smem(atc::k_ab_linhas_tc<2>, atc::smem_linhas_tc(2))) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_linhas_tc<2>, dim3(grade), dim3(atc::NTL), atc::smem_linhas_tc(2), st, mV, mG, mKt, A);
-    if ((c = at_smem(atc::k_ab_linhas_tc<3>, atc::smem_linhas_tc(3))) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_linhas_tc<3>, dim3(grade), dim3(atc::NTL), atc::smem_linhas_tc(3), st, mV, mG, mKt, A);
-    if ((c = at_smem(atc::k_ab_colunas_tc, atc::smem_colunas_tc())) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_colunas_tc, dim3(dim3((T + atc::NJ - 1) / atc::NJ, BH)), dim3(256), atc::smem_colunas_tc(), st, mQt, mGt, mDh, mDl, mP, A);
+    if ((c = at_smem(atc::k_ab_soma, atc::SM_SOMA)) != cudaSuccess) return (int)c;
+    lanca_pdl(atc::k_ab_soma, dim3(nt, BH), dim3(atc::NTA), atc::SM_SOMA, st, mV, mGd, A);
+    if ((c = at_smem(atc::k_ab_saida, atc::SM_SAIDA)) != cudaSuccess) return (int)c;
+    lanca_pdl(atc::k_ab_saida, dim3(nt, BH, 3), dim3(atc::NTA), atc::SM_SAIDA, st, mV, mG, mVd, mGd, mKt, mQt, mGt, mP, A);
     return (int)cudaGetLastError();
 }
 

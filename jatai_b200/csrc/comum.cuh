@@ -15,6 +15,7 @@ namespace jt {
 constexpr int E_ZERO = -127;          // exponent of an all-zero block
 constexpr int LIM = 1 << 30;          // register invariant |v| < 2^30
 constexpr int SEM_TOPO = -100000;     // "block has no non-zero element"
+constexpr int N_SM = 148;             // B200
 constexpr int U_MIN = -2147483647;    // "-infinity" of scores / logits
 constexpr unsigned FULL = 0xffffffffu;
 

@@ -337,7 +337,7 @@ class OpsCuda:
 
     def _atencao_fundida(self, T, H, D):
         """Whether the library quantises the attention outputs in its own output stage for this shape (else: two launches)."""
-        return BLK == 32 and D == 64 * H and T % 64 == 0 and 128 <= T <= 1024
+        return BLK == 32 and D == 64 * H and T % 32 == 0 and T <= 1024 and GA <= 4
 
     def atencao_quant(self, QKV, Bt, T, H):
         """(quant(O), P) of atencao(QKV, Bt, T, H): one launch where the library offers it (an addition of this library; same results)."""

@@ -626,6 +626,36 @@ def test_atencao_pedacos_de_chaves_sem_efeito(amb, mmax, esp, T):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("blk,Bt,T,H,D,e0,longe", [(32, 2, 32, 2, 128, -8, 0), (32, 1, 96, 4, 64, -8, 1), (128, 1, 160, 8, 128, -8, 2), (32, 1, 288, 26, 416, -5, 3),
+                                                   (32, 1, 416, 2, 128, -8, 4), (32, 1, 1024, 34, 544, -4, 0), (32, 1, 1024, 2, 128, -8, 5)])
+def test_atencao_janelas(amb, blk, Bt, T, H, D, e0, longe):
+    """The tensor-core attention walks the keys in windows of 128 that end with a tile of 64 queries: sequence lengths from one
+    half tile to 16 tiles, odd numbers of half tiles, both head dimensions, scores and slopes (heads 16 and on) that need several
+    windows, and a backward on a P with non-zeros put far from the diagonal, against the oracle."""
+    ops, oc, reg = amb
+    ops.define_blk(blk)
+    reg.novo_passo(0)
+    G = casos.Gen(911 + T + H + D, blk)
+    qkv, go = G.bloco(Bt * T, 3 * D, e0=e0, espalha=4, zera=0.02), G.bloco(Bt * T, D, e0=-20, espalha=4)
+    s = spec.Spec(blk)
+    o_r, P = s.atencao(qkv, Bt, T, H)
+    try:
+        o_c, P_c = oc.atencao(para_gpu(qkv), Bt, T, H)
+        P = P.clone()
+        for n in range(longe):                       # [Bt*H, T (keys), T (queries)]
+            j = (37 * n) % (T // 4)
+            P[n % (Bt * H), j, T - 1 - 29 * n] = 200
+            P[(n + 1) % (Bt * H), j + 3, (T // 2 + 64 * n) % T:] = 3 if j + 3 < (T // 2 + 64 * n) % T else 0
+        g_r = s.atencao_back(go, qkv, P, Bt, T, H)
+        g_c = oc.atencao_back(para_gpu(go), para_gpu(qkv), para_gpu(P), Bt, T, H)
+        torch.cuda.synchronize()
+    finally:
+        ops.define_blk(32)
+    compara(f"atencao T {T} H {H} D {D}", list(o_c), list(o_r))
+    compara(f"atencao_back T {T} H {H} D {D}", list(g_c), list(g_r))
+
+
+@pytest.mark.gpu
 def test_atencao_back_com_P_alterado(amb):
     """The backward works from the P it is given: with whole tiles of P zeroed by hand (tiles its zero map then leaves out, tiles
     next to the diagonal, a whole key range) it still equals the oracle's backward on that same P."""
