@@ -631,14 +631,6 @@ __global__ void __launch_bounds__(NTA, 2) k_ab_max(const __grid_constant__ CUten
     termina(S, 256);
 }
 
-// rnd_d(x, s) for 0 <= s <= 30 with the constants of s hoisted: (x + 2^(s-1) - 1 + ((x >> s) & 1)) >> s, and x itself at s = 0.  The
-// shifts of the backward are bitlen(int) - 15 and bitlen(int) - 12, at most 20.
-struct Arred {
-    int s, meio, um;
-    __device__ explicit Arred(int s_) : s(s_), meio(s_ ? (1 << (s_ - 1)) - 1 : 0), um(s_ ? 1 : 0) {}
-    __device__ int operator()(int x) const { return (x + meio + ((x >> s) & um)) >> s; }
-};
-
 // Query tiles: s_lin and the maxima of dS.  With one live window gP' and P stay in registers between the two passes.
 // Shared: dO digits 16 KB | V window 16 KB; tensor memory: the scores.
 constexpr uint32_t SO_V = 2 * TILE_N, SO_BAR = SO_V + TILE_A;

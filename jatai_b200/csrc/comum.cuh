@@ -76,6 +76,14 @@ __device__ __forceinline__ int rnd_d(int x, int s) {
     return (x + ((1 << (s - 1)) - 1) + ((x >> s) & 1)) >> s;
 }
 
+// rnd_d(x, s) for 0 <= s <= 30 with the constants of s hoisted: (x + 2^(s-1) - 1 + ((x >> s) & 1)) >> s, and x itself at s = 0.  The
+// shifts of the backward are bitlen(int) - 15 and bitlen(int) - 12, at most 20.
+struct Arred {
+    int s, meio, um;
+    __device__ explicit Arred(int s_) : s(s_), meio(s_ ? (1 << (s_ - 1)) - 1 : 0), um(s_ ? 1 : 0) {}
+    __device__ int operator()(int x) const { return (x + meio + ((x >> s) & um)) >> s; }
+};
+
 // x * 2^-s for any sign of s; the left shift is reported (E_SHL) if it would leave the 2^30 range.
 __device__ __forceinline__ int rnd(int x, int s, int kid, long long idx) {
     if (s > 0) return rnd_d(x, s);

@@ -479,7 +479,7 @@ int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid) 
 int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, int Bt, int T, int H, int D, int GA, int kid) {
     if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA))
         return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, nullptr, nullptr, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
-    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D))
+    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA))
         return atencao_frente_peq(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
     return atencao_frente(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
 }
@@ -488,7 +488,7 @@ int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void
     if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA))
         return atencao_tras_tc(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
                                (int16_t*)Ge, nullptr, nullptr, Bt, T, H, D, GA, limite, kid, g_stream);
-    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D))
+    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA))
         return atencao_tras_peq(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
                                 (int16_t*)Ge, Bt, T, H, D, GA, limite, kid, g_stream);
     return atencao_tras(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,

@@ -656,6 +656,37 @@ def test_atencao_janelas(amb, blk, Bt, T, H, D, e0, longe):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("limite", [False, True])
+@pytest.mark.parametrize("blk,Bt,T,H,e0,esp", [(32, 1, 32, 8, -8, 4), (128, 1, 64, 32, -4, 3), (32, 1, 128, 64, -8, 4), (32, 1, 96, 8, -1, 0), (32, 2, 128, 8, 0, 0),
+                                               (32, 1, 64, 8, 1, 0)])
+def test_atencao_cabecas_de_4(amb, blk, Bt, T, H, e0, esp, limite):
+    """Heads of 4 at T <= 128: every slope (64 heads), score shifts on both sides of the float rounding's range (shift 3; 1 and a
+    left shift take the general way), and a backward on a P with entries put far from the diagonal, against the oracle."""
+    ops, oc, reg = amb
+    ops.define_blk(blk)
+    reg.novo_passo(0)
+    D = 4 * H
+    G = casos.Gen(3 * T + H + e0, blk)
+    qkv, go = G.bloco(Bt * T, 3 * D, e0=e0, espalha=esp, zera=0.02 if esp else 0.0), G.bloco(Bt * T, D, e0=-20, espalha=4)
+    s = spec.Spec(blk, limite=limite)
+    o_r, P = s.atencao(qkv, Bt, T, H)
+    ops.ATENCAO_LIMITE = limite
+    try:
+        o_c, P_c = oc.atencao(para_gpu(qkv), Bt, T, H)
+        P2 = P.clone()                               # [Bt*H, T (keys), T (queries)]
+        P2[0, 1, T - 1] = 255
+        P2[1, 5:9, T - 20:] = 7
+        g_r = s.atencao_back(go, qkv, P2, Bt, T, H)
+        g_c = oc.atencao_back(para_gpu(go), para_gpu(qkv), para_gpu(P2), Bt, T, H)
+        torch.cuda.synchronize()
+    finally:
+        ops.ATENCAO_LIMITE = False
+        ops.define_blk(32)
+    compara(f"atencao T {T} H {H} e0 {e0}", [*o_c, P_c], [*o_r, P])
+    compara(f"atencao_back T {T} H {H} e0 {e0} limite {limite}", list(g_c), list(g_r))
+
+
+@pytest.mark.gpu
 def test_atencao_back_com_P_alterado(amb):
     """The backward works from the P it is given: with whole tiles of P zeroed by hand (tiles its zero map then leaves out, tiles
     next to the diagonal, a whole key range) it still equals the oracle's backward on that same P."""
