@@ -12,7 +12,7 @@
 //     warp's 32 rows at a time are skipped when none of them counts (exponentials, P.V and, from the bytes of P, everything in the backward
 //     but the first maximum);
 //   * the exponentials of the row sum are kept (16 bits, shared memory) for P.
-// 16 sequences of 128 tokens, 64 heads: forward 62 -> XX us, backward 68 -> XX us.
+// 16 sequences of 128 tokens, 64 heads: forward 62 -> 31 us, backward 68 -> 51 us (both at 60 % of the issue slots).
 //
 // Specification and layouts as in atencao.cuh (jatai_cuda/ops.py:186-258; jatai_cuda/jatai_cuda.cu:822-1006): QKV [Bt*T, 3D]
 // block tensor, P uint8 [Bt*H][j][i] with explicit zeros for j > i, raw outputs.
@@ -85,8 +85,7 @@ __device__ __forceinline__ void grava_cru(int* acc, int16_t* e, size_t p, const 
 //
 // A shift of the scores below 2 (or left, or above 31) leaves the range of the float rounding: such a head, which no trained model has, goes
 // the general way, key by key.
-__device__ __noinline__ void frente_geral(int* k_s, const int* v_s, int4 q, int s_u, int incl, int kid, long long idx, uint8_t* Pc, int T, int (&o)[4]) {
-    const int i = threadIdx.x;
+__device__ __noinline__ void frente_geral(int i, int* k_s, const int* v_s, int4 q, int s_u, int incl, int kid, long long idx, uint8_t* Pc, int T, int (&o)[4]) {
     auto score = [&](int j) {
         const int4 k = reinterpret_cast<const int4*>(k_s)[j];
         return rnd(q.x * k.x + q.y * k.y + q.z * k.z + q.w * k.w, s_u, kid, idx) - ((i - j) << incl);
@@ -113,7 +112,9 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_peq(const int8_t* __restric
     float* k_s = reinterpret_cast<float*>(sm);
     int* v_s = reinterpret_cast<int*>(sm + T * 16);
     __shared__ int red[12];
-    const int i = threadIdx.x, lane = i & 31, w = i >> 5, bh = blockIdx.x, b = bh / H, h = bh % H, ld = 3 * D, ldb = ld / blk;
+    // the warp of the last rows has the most to do and warp n of a block sits on the SM's scheduler n & 3: the rows turn with the block
+    const int lane = threadIdx.x & 31, w = ((threadIdx.x >> 5) + blockIdx.x) % (T >> 5), i = 32 * w + lane;
+    const int bh = blockIdx.x, b = bh / H, h = bh % H, ld = 3 * D, ldb = ld / blk;
     uint2* ex_s = reinterpret_cast<uint2*>(sm + T * 32 + 1024 * w * (w + 1)) + lane;
     const size_t lin = (size_t)b * T + i;
     pdl_espera();
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_peq(const int8_t* __restric
     const uint32_t mq = *reinterpret_cast<const uint32_t*>(qm + lin * ld + h * HD), mk = *reinterpret_cast<const uint32_t*>(qm + lin * ld + D + h * HD),
                    mv = *reinterpret_cast<const uint32_t*>(qm + lin * ld + 2 * D + h * HD);
     int em[3] = {eq, ek, ev};
-    max_cta<3>(em, red, i);
+    max_cta<3>(em, red, threadIdx.x);
     const int4 q = alinha(mq, em[0] - eq, GA), kk = alinha(mk, em[1] - ek, GA);
     const int s_u = -((em[0] - GA) + (em[1] - GA) - 1 + 8), incl = at::incl_alibi(h);
     const bool rapido = s_u >= 2 && s_u <= 31;                     // the same for the whole CTA
@@ -172,14 +173,8 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_peq(const int8_t* __restric
             vivos |= 1u << g;
             uint32_t e[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) {                          // exp3_dif
-                const uint32_t t = __float_as_uint(fminf(d[k], DOIS23 + 6000.0f)) * 23637u - 0x4B000000u * 23637u;
-                const int f2 = (int)((t >> 6) & 0xFFFE);
-                int p = -1295 * 65536;
-                p = __mulhi(p, f2) * 65536 + 7556 * 65536;
-                p = __mulhi(p, f2) * 65536 - 22645 * 65536;
-                p = __mulhi(p, f2) * 65536 + 32765 * 65536;
-                e[k] = (uint32_t)(p >> min(19 + (int)(t >> 22), 31));
+            for (int k = 0; k < 4; k++) {
+                e[k] = (uint32_t)exp3_t(__float_as_uint(fminf(d[k], DOIS23 + 6000.0f)) * 23637u + ((13u << 22) - 0x4B000000u * 23637u));
                 soma += (int)e[k];
             }
             ex_s[g * 32] = make_uint2(e[0] | e[1] << 16, e[2] | e[3] << 16);
@@ -204,7 +199,7 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_peq(const int8_t* __restric
             }
         }
     } else
-        frente_geral(reinterpret_cast<int*>(k_s), v_s, q, s_u, incl, kid, idx, Ph + i, T, o);
+        frente_geral(i, reinterpret_cast<int*>(k_s), v_s, q, s_u, incl, kid, idx, Ph + i, T, o);
     grava_cru(Oacc, Oe, lin * D + h * HD, o, (em[2] - GA) - 8);
 }
 inline size_t smem_frente_peq(int T) { return (size_t)T * 32 + 1024 * (T / 32) * (T / 32 + 1); }
@@ -214,7 +209,7 @@ inline size_t smem_frente_peq(int T) { return (size_t)T * 32 + 1024 * (T / 32) *
 // norms); s_lin; max |dS|; dS' and gq; then thread = key column: gk and gv.  P of the head sits in shared memory from the diagonal on:
 // block b of 32 key rows holds the queries from 32 b, row pitch T - 32 b + 4 bytes (an odd number of words).  What a hand-made P has
 // beyond the diagonal is dropped while it is loaded.
-// Dynamic shared memory: v pairs [T][4] | k | q | g [T][4] | s_lin [T] | P.
+// Dynamic shared memory: v pairs [T][4] | k | q | g [T][4] | g pairs [T][4] | s_lin + 1.5 * 2^23's bits [T] | P.
 __device__ __forceinline__ int pk_passo(int T, int bl) { return T - 32 * bl + 4; }
 __device__ __forceinline__ int pk_base(int T, int bl) { return 32 * bl * (T + 4) - 512 * bl * (bl - 1); }      // sum of 32 (T + 4 - 32 b') over b' < bl
 
@@ -226,10 +221,13 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_back_peq(const int8_t* __re
     int4* k_s = reinterpret_cast<int4*>(sm + T * 16);
     int4* q_s = k_s + T;
     int4* g_s = q_s + T;
-    int* sl_s = reinterpret_cast<int*>(g_s + T);
+    float* gf_s = reinterpret_cast<float*>(g_s + T);
+    int* sl_s = reinterpret_cast<int*>(gf_s + 4 * T);
     uint8_t* P_s = reinterpret_cast<uint8_t*>(sl_s + T);
     __shared__ int red[16];
-    const int i = threadIdx.x, lane = i & 31, w = i >> 5, bh = blockIdx.x, b = bh / H, h = bh % H, ld = 3 * D, ldb = ld / blk;
+    // the warp of the last rows has the most to do and warp n of a block sits on the SM's scheduler n & 3: the rows turn with the block
+    const int lane = threadIdx.x & 31, w = ((threadIdx.x >> 5) + blockIdx.x) % (T >> 5), i = 32 * w + lane;
+    const int bh = blockIdx.x, b = bh / H, h = bh % H, ld = 3 * D, ldb = ld / blk;
     const size_t lin = (size_t)b * T + i;
     pdl_espera();
     pdl_solta();
@@ -258,20 +256,21 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_back_peq(const int8_t* __re
         }
     }
     int em[4] = {eg, eq, ek, ev};
-    max_cta<4>(em, red, i);
+    max_cta<4>(em, red, threadIdx.x);
     const int emg = em[0], emq = em[1], emk = em[2], emv = em[3];
     const int4 g = alinha(mg, emg - eg, GA), v = alinha(mv, emv - ev, GA);
     guarda_par(v_s, i, v);
     k_s[i] = alinha(mk, emk - ek, GA);
     q_s[i] = alinha(mq, emq - eq, GA);
     g_s[i] = g;
+    guarda_par(gf_s, i, g);
     __syncthreads();
     const uint64_t gp[4] = {par_f((float)g.x, (float)g.x), par_f((float)g.y, (float)g.y), par_f((float)g.z, (float)g.z), par_f((float)g.w, (float)g.w)};
     // shift of gP (to 15 bits): from its exact maximum over j <= i, or from the bounds of the upper-bound variant (ops.py:231-235)
     int sh;
     if (limite) {
         int mx[2] = {max(max(abs(g.x), abs(g.y)), max(abs(g.z), abs(g.w))), abs(v.x) + abs(v.y) + abs(v.z) + abs(v.w)};
-        max_cta<2>(mx, red, i);
+        max_cta<2>(mx, red, threadIdx.x);
         sh = max(bitlen(mx[0] * mx[1]) - 15, 0);
     } else {
         float mx = 0.0f;
@@ -286,40 +285,51 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_back_peq(const int8_t* __re
             mx = fmaxf(mx, fmaxf(2 * n <= lane ? fabsf(f_lo(x)) : 0.0f, 2 * n < lane ? fabsf(f_hi(x)) : 0.0f));
         }
         int m1[1] = {(int)mx};
-        max_cta<1>(m1, red, i);
+        max_cta<1>(m1, red, threadIdx.x);
         sh = max(bitlen(m1[0]) - 15, 0);
     }
     const uint64_t esc = par_f(pot2_f(-sh), pot2_f(-sh)), mag = par_f(MAGIA_F, MAGIA_F);
     // bit patterns of gP' + 1.5 * 2^23 for 4 keys (|gP'| <= 2^15; the sums below wrap like the specification's, so the bias comes off at the end)
-    auto gpl = [&](int n, uint32_t (&x)[4]) {
-        const uint64_t a = ffma2(ponto2(gp, v_s, 2 * n), esc, mag), c = ffma2(ponto2(gp, v_s, 2 * n + 1), esc, mag);
+    auto gpl4 = [&](const uint64_t (&um)[4], const float* outro, int n, uint32_t (&x)[4]) {
+        const uint64_t a = ffma2(ponto2(um, outro, 2 * n), esc, mag), c = ffma2(ponto2(um, outro, 2 * n + 1), esc, mag);
         x[0] = (uint32_t)a; x[1] = (uint32_t)(a >> 32); x[2] = (uint32_t)c; x[3] = (uint32_t)(c >> 32);
     };
-    // f(first key of the group, the four P of this row, the four gP') over the groups of 4 keys in which this warp has a non-zero P
-    auto anda = [&](auto f) {
-#pragma unroll 1
-        for (int bl = 0; bl <= w; bl++) {
-            const int pp = pk_passo(T, bl);
-            const uint8_t* p = P_s + pk_base(T, bl) + i - 32 * bl;
-#pragma unroll 2
-            for (int n = 0; n < 8; n++, p += 4 * pp) {
-                const uint32_t pv[4] = {p[0], p[pp], p[2 * pp], p[3 * pp]};
-                if (!__any_sync(FULL, (pv[0] | pv[1] | pv[2] | pv[3]) != 0)) continue;
-                uint32_t x[4];
-                gpl(8 * bl + n, x);
-                f(32 * bl + 4 * n, pv, x);
-            }
-        }
-    };
+    auto gpl = [&](int n, uint32_t (&x)[4]) { gpl4(gp, v_s, n, x); };
     // s_lin of this row, then the maxima that give the shift of dS (to 12 bits) (ops.py:236-244)
     uint32_t s = 0, sp = 0;
+    unsigned vivos = 0;                                            // groups of 4 keys in which this warp has a non-zero P
+#pragma unroll 1
+    for (int bl = 0; bl <= w; bl++) {
+        const int pp = pk_passo(T, bl);
+        const uint8_t* p = P_s + pk_base(T, bl) + i - 32 * bl;
+        uint32_t soma[8];
+#pragma unroll
+        for (int n = 0; n < 8; n++) {
+            soma[n] = (uint32_t)p[(4 * n) * pp] + p[(4 * n + 1) * pp] + p[(4 * n + 2) * pp] + p[(4 * n + 3) * pp];
+            sp += soma[n];
+        }
+#pragma unroll
+        for (int n = 0; n < 8; n++) vivos |= (__any_sync(FULL, soma[n] != 0) ? 1u : 0u) << (8 * bl + n);
+    }
+    // f(first key of the group, the four P of this row, the four gP') over those groups
+    auto anda = [&](auto f) {
+#pragma unroll 2
+        for (unsigned m = vivos; m; m &= m - 1) {
+            const int n = __ffs(m) - 1, bl = n >> 3, pp = pk_passo(T, bl);
+            const uint8_t* p = P_s + pk_base(T, bl) + i - 32 * bl + 4 * (n & 7) * pp;
+            const uint32_t pv[4] = {p[0], p[pp], p[2 * pp], p[3 * pp]};
+            uint32_t x[4];
+            gpl(n, x);
+            f(4 * n, pv, x);
+        }
+    };
     anda([&](int, const uint32_t (&p)[4], const uint32_t (&x)[4]) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) { s += p[k] * x[k]; sp += p[k]; }
+        for (int k = 0; k < 4; k++) s += p[k] * x[k];
     });
     const int sl = rnd_d((int)(s - MAGIA * sp), 8);
-    sl_s[i] = sl;
     const uint32_t tira = MAGIA + (uint32_t)sl;
+    sl_s[i] = (int)tira;
     int sh2;
     {
         int mds = 0;
@@ -337,16 +347,16 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_back_peq(const int8_t* __re
                     if (4 * n + k <= i) mgq = max(mgq, abs((int)(x[k] - MAGIA)));
             }
             int mx[3] = {mp, mgq, abs(sl)};
-            max_cta<3>(mx, red, i);
+            max_cta<3>(mx, red, threadIdx.x);
             sh2 = max(bitlen(mx[0] * (mx[1] + mx[2])) - 12, 0);
         } else {
             int mx[1] = {mds};
-            max_cta<1>(mx, red, i);
+            max_cta<1>(mx, red, threadIdx.x);
             sh2 = max(bitlen(mx[0]) - 12, 0);
         }
     }
     const int eds = (emg - GA) + (emv - GA) + sh - 9 + sh2;
-    const Arred arred(sh), arred2(sh2);
+    const Arred arred2(sh2);
     // gq of this row
     int o[4] = {0, 0, 0, 0};
     anda([&](int j, const uint32_t (&p)[4], const uint32_t (&x)[4]) {
@@ -362,15 +372,23 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_back_peq(const int8_t* __re
     // thread = key j = i: gk[j] = sum_{r >= j} dS'[r][j] q[r], gv[j] = sum_{r >= j} P[r][j] dO[r]
     int gk[4] = {0, 0, 0, 0}, gv[4] = {0, 0, 0, 0};
     const uint32_t* pk = reinterpret_cast<const uint32_t*>(P_s + pk_base(T, w) + lane * pk_passo(T, w));
-#pragma unroll 1
-    for (int r0 = 32 * w; r0 < T; r0 += 4) {
-        const uint32_t p4 = pk[(r0 - 32 * w) >> 2];
-        if (!__any_sync(FULL, p4 != 0)) continue;
+    unsigned vivas = 0;                                            // groups of 4 queries in which this warp's keys have a non-zero P
+#pragma unroll 8
+    for (int n = 8 * w; n < T / 4; n++) vivas |= (__any_sync(FULL, pk[n - 8 * w] != 0) ? 1u : 0u) << n;
+    const uint64_t vp[4] = {par_f((float)v.x, (float)v.x), par_f((float)v.y, (float)v.y), par_f((float)v.z, (float)v.z), par_f((float)v.w, (float)v.w)};
+#pragma unroll 2
+    for (unsigned m = vivas; m; m &= m - 1) {
+        const int n = __ffs(m) - 1;
+        const uint32_t p4 = pk[n - 8 * w];
+        uint32_t x[4];
+        gpl4(vp, gf_s, n, x);
+        const int4 sl4 = reinterpret_cast<const int4*>(sl_s)[n];
+        const int tl[4] = {sl4.x, sl4.y, sl4.z, sl4.w};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const int p = (int)(p4 >> (8 * k) & 0xff);
-            const int4 y = g_s[r0 + k], z = q_s[r0 + k];
-            const int ds = arred2(p * (arred(y.x * v.x + y.y * v.y + y.z * v.z + y.w * v.w) - sl_s[r0 + k]));
+            const int p = (int)__byte_perm(p4, 0, 0x4440 + k);
+            const int4 y = g_s[4 * n + k], z = q_s[4 * n + k];
+            const int ds = arred2(p * ((int)x[k] - tl[k]));
             gv[0] += p * y.x; gv[1] += p * y.y; gv[2] += p * y.z; gv[3] += p * y.w;
             gk[0] += ds * z.x; gk[1] += ds * z.y; gk[2] += ds * z.z; gk[3] += ds * z.w;
         }
@@ -380,7 +398,7 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_back_peq(const int8_t* __re
 }
 inline size_t smem_back_peq(int T) {
     const int nb = T / 32;
-    return (size_t)T * 68 + 32 * nb * (T + 4) - 512 * nb * (nb - 1);
+    return (size_t)T * 84 + 32 * nb * (T + 4) - 512 * nb * (nb - 1);
 }
 
 }  // namespace atp

@@ -433,12 +433,8 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
             if (!tem_ex) {
 #pragma unroll
                 for (int k = 0; k < 32; k++) {
-                    const int m = m_s[q0 + k], t = (k < kmin || v[k] <= m - 6000 ? 6000 : m - v[k]) * 23637, f2 = (t >> 6) & 0xFFFE;
-                    int p = -1295 * 65536;                         // exp3_dif, a key beyond the diagonal being infinitely far below
-                    p = __mulhi(p, f2) * 65536 + 7556 * 65536;
-                    p = __mulhi(p, f2) * 65536 - 22645 * 65536;
-                    p = __mulhi(p, f2) * 65536 + 32765 * 65536;
-                    v[k] = p >> min(19 + (t >> 22), 31);
+                    const int m = m_s[q0 + k];                     // a key beyond the diagonal is infinitely far below
+                    v[k] = exp3_t((uint32_t)(k < kmin || v[k] <= m - 6000 ? 6000 : m - v[k]) * 23637u + (13u << 22));
                 }
                 tem_ex = n == 1;
             }

@@ -108,16 +108,20 @@ __device__ __forceinline__ int exp_int(int d) {
 }
 // exp(-(mx - u)/256) with the difference clamped before subtracting (mx - u may not fit in int32)
 __device__ __forceinline__ int exp_dif(int mx, int u) { return exp_int(u <= mx - 6000 ? 6000 : mx - u); }
-// exp_dif(mx, u) >> 3, the form the softmaxes use, with the cubic on p * 2^16 (|p| < 2^15 at every step): (p f) >> 15 = mulhi(p << 16, 2 f), and
-// p >> (n + 3) is 0 from n = 12 on (0 <= p < 2^15), as is the shift clamped to 31
-__device__ __forceinline__ int exp3_dif(int mx, int u) {
-    const int t = (u <= mx - 6000 ? 6000 : mx - u) * 23637, f2 = (t >> 6) & 0xFFFE;
-    int p = -1295 * 65536;
-    p = __mulhi(p, f2) * 65536 + 7556 * 65536;
-    p = __mulhi(p, f2) * 65536 - 22645 * 65536;
-    p = __mulhi(p, f2) * 65536 + 32765 * 65536;
-    return p >> min(19 + (t >> 22), 31);
+// exp_int(d) >> 3 from t = d * 23637 + (13 << 22) for 0 <= d <= 6000, the form the softmaxes use: the cubic on p * 2^10 (|p| < 2^15 at every
+// step) and f in place, (p f) >> 15 = mulhi(p << 10, f << 7), and the integer part of t is the shift n + 3 + 10 as it stands (a shift of
+// 32 and more gives 0 here as p >= 0; from n = 12 on the result is 0 anyway)
+__device__ __forceinline__ int exp3_t(uint32_t t) {
+    const int f7 = (int)(t & 0x3FFF80u);
+    int p = -1295 * 1024, r;
+    p = __mulhi(p, f7) * 1024 + 7556 * 1024;
+    p = __mulhi(p, f7) * 1024 - 22645 * 1024;
+    p = __mulhi(p, f7) * 1024 + 32765 * 1024;
+    asm("shr.s32 %0, %1, %2;" : "=r"(r) : "r"(p), "r"(t >> 22));
+    return r;
 }
+// exp_dif(mx, u) >> 3
+__device__ __forceinline__ int exp3_dif(int mx, int u) { return exp3_t((uint32_t)(u <= mx - 6000 ? 6000 : mx - u) * 23637u + (13u << 22)); }
 
 // integer square root (ops.py:84-89: 10 Newton steps from a power of two above the root, each min(x, (x + n/x) >> 1); from
 // above they converge to floor(sqrt(n)) well inside 10 steps for every n < 2^31, and the result is clamped to >= 1).
