@@ -18,29 +18,13 @@
 // block tensor, P uint8 [Bt*H][j][i] with explicit zeros for j > i, raw outputs.
 #pragma once
 #include "comum.cuh"
-#include "gemm_tc.cuh"
 #include "atencao.cuh"
 
 namespace jt {
 namespace atp {
 
-using tc::MAGIA; using tc::par_f; using tc::ffma2;
 constexpr int TMAX = 128, HD = 4;
-constexpr float MAGIA_F = 12582912.0f, DOIS23 = 8388608.0f;
-
-__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float f_lo(uint64_t a) { return __uint_as_float((uint32_t)a); }
-__device__ __forceinline__ float f_hi(uint64_t a) { return __uint_as_float((uint32_t)(a >> 32)); }
-__device__ __forceinline__ float pot2_f(int e) { return __int_as_float((e + 127) << 23); }
+constexpr float DOIS23 = 8388608.0f;
 
 // N per-thread values -> their CTA-wide maxima (blockDim.x a multiple of 32, <= 128; red is [N][4])
 template <int N>
@@ -136,7 +120,7 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_peq(const int8_t* __restric
     int o[4] = {0, 0, 0, 0};
     if (rapido) {
         const uint64_t qp[4] = {par_f((float)q.x, (float)q.x), par_f((float)q.y, (float)q.y), par_f((float)q.z, (float)q.z), par_f((float)q.w, (float)q.w)};
-        const uint64_t esc = par_f(pot2_f(-s_u), pot2_f(-s_u)), mag = par_f(MAGIA_F, MAGIA_F);
+        const uint64_t esc = par_f(pot2(-s_u), pot2(-s_u)), mag = par_f(MAGIA_F, MAGIA_F);
         const float I = (float)(1 << incl);
         // scores of the pair n: rounded product (biased by 1.5 * 2^23) minus bias and slope; the sums stay below 2^24
         const uint64_t n0 = par_f(-MAGIA_F - (float)i * I, -MAGIA_F - (float)(i - 1) * I), passo = par_f(2 * I, 2 * I), passo2 = par_f(4 * I, 4 * I);
@@ -288,7 +272,7 @@ __global__ void __launch_bounds__(TMAX, 7) k_atencao_back_peq(const int8_t* __re
         max_cta<1>(m1, red, threadIdx.x);
         sh = max(bitlen(m1[0]) - 15, 0);
     }
-    const uint64_t esc = par_f(pot2_f(-sh), pot2_f(-sh)), mag = par_f(MAGIA_F, MAGIA_F);
+    const uint64_t esc = par_f(pot2(-sh), pot2(-sh)), mag = par_f(MAGIA_F, MAGIA_F);
     // bit patterns of gP' + 1.5 * 2^23 for 4 keys (|gP'| <= 2^15; the sums below wrap like the specification's, so the bias comes off at the end)
     auto gpl4 = [&](const uint64_t (&um)[4], const float* outro, int n, uint32_t (&x)[4]) {
         const uint64_t a = ffma2(ponto2(um, outro, 2 * n), esc, mag), c = ffma2(ponto2(um, outro, 2 * n + 1), esc, mag);

@@ -10,10 +10,11 @@
 //     int64 -> int32 truncation); P is uint8 and enters as it is.
 //
 // A preparation kernel aligns q, k, v (and dO) of every head to the head's maximum exponent once and writes what the MMAs read (all
-// K-major, rows of 128 bytes, TMA with the 128-byte swizzle; a head of 16 columns is padded with zeros to 64):
+// K-major, rows of 128 bytes, TMA with the 128-byte swizzle):
 //     plain          [BH*T][64] f16                      token rows
 //     digits         [2][BH*T][64] f16                   token rows of the hi digits, then of the lo digits
-//     transposed     [BH*128][T] int8                    row = one digit of one column, over the tokens
+//     transposed     [BH*128][T] int8                    row = one digit of one column (hi rows 0..63, lo rows 64..127), over the tokens
+// A head of 16 columns fills 16 of the 64 (and of each 64 digit rows); the rest is neither written nor multiplied into a result.
 //
 // A query tile of 64 rows takes its keys in windows of 128 that end with the tile's last query and go back from there.  With the
 // reference's slopes P is exactly zero a few dozen keys behind the diagonal, so one window is nearly always all there is: the forward
@@ -47,6 +48,7 @@ constexpr uint32_t idesc(int n, bool b_sem_sinal) {       // kind::i8, D = s32, 
 }
 constexpr uint32_t ID_S = idesc(SB, false), ID_PU = idesc(NI, true);
 constexpr uint32_t ID_F16 = (1u << 4) | ((uint32_t)(SB >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);      // kind::f16, D = f32, N = 128, M = 128
+constexpr uint32_t ID_F16N = (1u << 4) | ((uint32_t)(NI >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);     // the same with N = 64
 constexpr uint32_t TILE_A = 128 * 128, TILE_N = NI * 128;
 
 __device__ __forceinline__ void digitos(int v, int& hi, int& lo) {
@@ -66,15 +68,20 @@ __device__ __forceinline__ void tmem_aloca(uint32_t* slot, int colunas) {
 __device__ __forceinline__ void tmem_libera(uint32_t tmem, int colunas) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(colunas) : "memory");
 }
-// the four MMAs of one score-like product: A = 128 token rows (plain), B = the 64 token rows of the hi digits and the 64 of the lo digits
-__device__ __forceinline__ void mma_escores(uint32_t tm, uint64_t da, uint64_t db) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) th::mma_f16(tm, da + 2 * q, db + 2 * q, ID_F16, q != 0);
+// The MMAs of one score-like product, hd columns.  A = 128 token rows (plain), B = the 64 token rows of the hi digits and the 64 of the lo
+// digits; or, digits on the A side, two products with the 64 token rows of B (plain).
+__device__ __forceinline__ void mma_escores(uint32_t tm, uint64_t da, uint64_t db, int hd) {
+    for (int q = 0; q < hd / 16; q++) th::mma_f16(tm, da + 2 * q, db + 2 * q, ID_F16, q != 0);
+}
+__device__ __forceinline__ void mma_escores_a(uint32_t tm, uint64_t dah, uint64_t dal, uint64_t db, int hd) {
+    for (int q = 0; q < hd / 16; q++) {
+        th::mma_f16(tm, dah + 2 * q, db + 2 * q, ID_F16N, q != 0);
+        th::mma_f16(tm + NI, dal + 2 * q, db + 2 * q, ID_F16N, q != 0);
+    }
 }
 // 16 scores of this lane from the two accumulators (hi at t, lo 64 columns on): 64 hi + lo, through the bit patterns of hi + 1.5 * 2^23 and
 // lo + 1.5 * 2^23
-__device__ __forceinline__ void escores16(uint32_t t, int (&x)[16]) {
-    uint32_t h[16], l[16];
+__device__ __forceinline__ void escores16_cru(uint32_t t, uint32_t (&h)[16], uint32_t (&l)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n"
@@ -82,6 +89,10 @@ __device__ __forceinline__ void escores16(uint32_t t, int (&x)[16]) {
         : JT_O16(h, 0), JT_O16(l, 0)
         : "r"(t), "r"(t + NI)
         : "memory");
+}
+__device__ __forceinline__ void escores16(uint32_t t, int (&x)[16]) {
+    uint32_t h[16], l[16];
+    escores16_cru(t, h, l);
 #pragma unroll
     for (int k = 0; k < 16; k += 2) {
         th::soma_magia(h[k], h[k + 1]);
@@ -136,19 +147,21 @@ struct ArgsPrep {
     int* nrm;                   // forward: [BH][2][ceil(T/128)] largest sum of squares of an aligned row of q (0) / k (1) per 128 tokens
     int BH, T, H, D, hd, GA, blk, por_cta;       // por_cta: 128-token pieces of a CTA
 };
-__device__ __forceinline__ uint32_t par_h(int a, int b) {           // two integers of at most 2048 as halves
+__device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats that halves hold exactly
     uint32_t r;
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"((float)b), "f"((float)a));
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(f_hi(x)), "f"(f_lo(x)));
     return r;
 }
 
-// grid (CTAs per head, BH, 3 or 4), 256 threads: `por_cta` pieces of 128 tokens of one head of one tensor; a thread has half a token's row.
-// The head's maximum exponent takes a look at every token, so a CTA does as many pieces as leave the GPU full.
-__global__ void __launch_bounds__(256) k_at_prep(const ArgsPrep A) {
-    pdl_espera();
-    pdl_solta();
+// grid (CTAs per head, BH, 3 or 4), 256 threads: `por_cta` pieces of 128 tokens of one head of one tensor.  The bound of a plain version (one
+// element at a time in integers, digit bytes stored one by one) was instruction issue, three times the memory time.  So: a thread takes 4
+// tokens x 8 columns; pairs of elements in f32x2 (a byte becomes a float by its place in 2^23's mantissa; v 2^(GA - s) rounds to even in one
+// FMA against 1.5 * 2^23, exactly rnd_d; the 6-bit digits are hi = round(r / 64), lo = r - 64 hi); the transposed digits of 4 tokens are
+// packed into a word and cross shared memory in 16-byte pieces swapped by the column group, without bank conflicts.
+// 16 x 1024 tokens, 16 heads of 64, forward + backward: 218 -> XX us.
+__global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
     __shared__ int red[8];
-    __shared__ __align__(16) uint8_t tr[128 * 144];
+    __shared__ __align__(16) uint32_t tr[128 * 32];
     const int tid = threadIdx.x, z = blockIdx.z, bh = blockIdx.y, b = bh / A.H, h = bh % A.H;
     uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
     uint16_t* dg = z == 0 ? A.dig[0] : z == 1 ? A.dig[1] : z == 2 ? A.dig[2] : A.dig[3];
@@ -157,6 +170,11 @@ __global__ void __launch_bounds__(256) k_at_prep(const ArgsPrep A) {
     const int8_t* m = z == 3 ? A.gm : A.qm;
     const int8_t* E = z == 3 ? A.gE : A.qE;
     const int ld = z == 3 ? D : 3 * D, col0 = z == 3 ? h * hd : z * D + h * hd, ldb = ld / blk;
+    const int cg = tid & 7, tg = tid >> 3;                         // columns 8 cg .. + 7, tokens 4 tg .. + 3 of a piece
+    const bool ha = 8 * cg < hd;
+    const size_t BHT = (size_t)A.BH * T;
+    pdl_espera();
+    pdl_solta();
     int em = -128;
     {
         const int nbh = hd > blk ? hd / blk : 1;
@@ -173,71 +191,87 @@ __global__ void __launch_bounds__(256) k_at_prep(const ArgsPrep A) {
     }
     if (blockIdx.x == 0 && tid == 0) A.em[bh * 4 + z] = em;
     if (A.est && blockIdx.x == 0 && z == 3 && tid < at::N_EST) A.est[bh * at::N_EST + tid] = 0;
-    const int r = tid >> 1, meio = tid & 1;
-    const size_t BHT = (size_t)A.BH * T;
+    const uint64_t mag = par_f(MAGIA_F, MAGIA_F), menos_mag = par_f(-MAGIA_F, -MAGIA_F), vies = par_f(-8388736.0f, -8388736.0f);      // 2^23 + 128
+    const uint64_t um64 = par_f(0.015625f, 0.015625f), m64 = par_f(-64.0f, -64.0f);
     for (int p = 0; p < A.por_cta; p++) {
-        const int peca = blockIdx.x * A.por_cta + p, t0 = peca * 128, t = t0 + r;
+        const int peca = blockIdx.x * A.por_cta + p, t0 = peca * 128;
         if (t0 >= T) break;
-        int norma = 0;
-        if (t < T) {
-            const size_t lin = (size_t)(linha0 + t), o = ((size_t)bh * T + t) * 64;
+        float norma = 0.0f;
+        uint32_t u[4][8];                                          // 2 r + 128: hi digit in byte 1, 2 (lo + 64) in byte 0
+        const bool dentro = t0 + 4 * tg < T;                       // (T is a multiple of 32)
+        uint2 w[4];
+        int s[4];
 #pragma unroll
-            for (int parte = 0; parte < 2; parte++) {
-                const int c = meio * 32 + parte * 16;
-                int v[16];
-                if (c < hd) {
-                    le16(m + lin * ld + col0 + c, v);
-                    const int s = em - (int)E[lin * ldb + (col0 + c) / blk];
+        for (int k = 0; k < 4; k++) {
+            const size_t lin = (size_t)(linha0 + t0 + 4 * tg + k);
+            w[k] = make_uint2(0, 0);
+            s[k] = 0;
+            if (dentro && ha) {
+                w[k] = *reinterpret_cast<const uint2*>(m + lin * ld + col0 + 8 * cg);
+                s[k] = min(em - (int)E[lin * ldb + (col0 + 8 * cg) / blk], 40);      // |v 2^GA| < 2^11: 0 from a shift of 13 on
+            }
+        }
 #pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        v[k] = rnd_d(v[k] << A.GA, s);
-                        norma += v[k] * v[k];                      // 12-bit values, 64 of them: below 2^28
-                    }
-                } else {
+        for (int k = 0; k < 4; k++) {
+            const uint64_t f = par_f(pot2(A.GA - s[k]), pot2(A.GA - s[k]));
+            uint32_t pl[4], dh[4], dl[4];
+            float nk = 0.0f;
 #pragma unroll
-                    for (int k = 0; k < 16; k++) v[k] = 0;
-                }
-                auto grava = [&](uint16_t* d, auto f) {
-                    uint4* q = reinterpret_cast<uint4*>(d + o + c);
-                    q[0] = make_uint4(par_h(f(v[0]), f(v[1])), par_h(f(v[2]), f(v[3])), par_h(f(v[4]), f(v[5])), par_h(f(v[6]), f(v[7])));
-                    q[1] = make_uint4(par_h(f(v[8]), f(v[9])), par_h(f(v[10]), f(v[11])), par_h(f(v[12]), f(v[13])), par_h(f(v[14]), f(v[15])));
-                };
-                if (dp) grava(dp, [](int x) { return x; });
+            for (int c = 0; c < 4; c++) {                          // two columns at a time
+                const uint32_t x = (c < 2 ? w[k].x : w[k].y) ^ 0x80808080u;
+                const uint64_t v = fadd2(par(__byte_perm(x, 0x4B000000u, 0x7540 + 2 * (c & 1)), __byte_perm(x, 0x4B000000u, 0x7540 + 2 * (c & 1) + 1)), vies);
+                const uint64_t r = ffma2(v, f, mag), rf = fadd2(r, menos_mag);
+                u[k][2 * c] = 2 * (uint32_t)r + (128u - 2 * MAGIA);
+                u[k][2 * c + 1] = 2 * (uint32_t)(r >> 32) + (128u - 2 * MAGIA);
+                if (dp) pl[c] = par_h(rf);
                 if (dg) {
-                    grava(dg, [](int x) { return (x + 32) >> 6; });
-                    grava(dg + BHT * 64, [](int x) { return x - (((x + 32) >> 6) << 6); });
+                    const uint64_t hi = fadd2(ffma2(rf, um64, mag), menos_mag);
+                    dh[c] = par_h(hi);
+                    dl[c] = par_h(ffma2(hi, m64, rf));
                 }
-                if (dt) {
-#pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        int hi, lo;
-                        digitos(v[k], hi, lo);
-                        tr[(c + k) * 144 + r] = (uint8_t)hi;
-                        tr[(64 + c + k) * 144 + r] = (uint8_t)lo;
-                    }
+                if (A.nrm) nk = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk));
+            }
+            if (dentro && ha) {
+                const size_t o = ((size_t)bh * T + t0 + 4 * tg + k) * 64 + 8 * cg;
+                if (dp) *reinterpret_cast<uint4*>(dp + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+                if (dg) {
+                    *reinterpret_cast<uint4*>(dg + o) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
+                    *reinterpret_cast<uint4*>(dg + BHT * 64 + o) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
                 }
+            }
+            if (A.nrm && z < 2) {                                  // squared norm of the token's row: its 8 lanes are neighbours
+                nk += __shfl_xor_sync(FULL, nk, 1);
+                nk += __shfl_xor_sync(FULL, nk, 2);
+                nk += __shfl_xor_sync(FULL, nk, 4);
+                norma = fmaxf(norma, nk);
             }
         }
         if (A.nrm && z < 2) {
-            // the largest squared norm of an aligned row among the 128 tokens (the two halves of a row sit in neighbouring lanes)
-            norma += __shfl_xor_sync(FULL, norma, 1);
-            norma = __reduce_max_sync(FULL, norma);
-            if ((tid & 31) == 0) red[tid >> 5] = norma;
+            // the largest of the 128 tokens, rounded up by more than the error of 64 fp32 additions (it only bounds products)
+            const int n = __reduce_max_sync(FULL, __float2int_ru(norma * 1.00002f));
+            if ((tid & 31) == 0) red[tid >> 5] = n;
             __syncthreads();
             if (tid == 0) {
                 int mx = 0;
-                for (int w = 0; w < 8; w++) mx = max(mx, red[w]);
+                for (int k = 0; k < 8; k++) mx = max(mx, red[k]);
                 A.nrm[((size_t)bh * 2 + z) * ((T + 127) / 128) + peca] = mx;
             }
         }
         if (dt) {
+            if (ha)
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const uint32_t lo = __byte_perm(__byte_perm(u[0][c], u[1][c], 0x0040), __byte_perm(u[2][c], u[3][c], 0x0040), 0x5410) >> 1 ^ 0x40404040u;
+                    const int q = (8 * cg + c) * 32 + (tg ^ 4 * cg);
+                    tr[q] = __byte_perm(__byte_perm(u[0][c], u[1][c], 0x0051), __byte_perm(u[2][c], u[3][c], 0x0051), 0x5410);
+                    tr[64 * 32 + q] = lo | (lo & 0x40404040u) << 1;      // 7 bits to a signed byte
+                }
             __syncthreads();
-            const int dd = tid >> 1;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const int off = meio * 64 + q * 16;
-                if (t0 + off < T)
-                    *reinterpret_cast<uint4*>(dt + ((size_t)bh * 128 + dd) * T + t0 + off) = *reinterpret_cast<const uint4*>(tr + dd * 144 + off);
+                const int linha = (tid >> 3) + 32 * q, c = tid & 7;
+                if ((linha & 63) < hd && t0 + 16 * c < T)
+                    *reinterpret_cast<uint4*>(dt + ((size_t)bh * 128 + linha) * T + t0 + 16 * c) = *reinterpret_cast<const uint4*>(tr + linha * 32 + 4 * (c ^ (linha >> 3 & 7)));
             }
         }
         __syncthreads();                                           // red[] and tr[] go to the next piece
@@ -251,27 +285,31 @@ struct Barras {
 // What every kernel below starts with: barriers, the abort flag, tensor memory.  The carve-up behind the operands (OFF): barriers, the
 // tensor-memory address, the abort flag, then 128 bytes in, `n` words of the kernel's own.
 struct Base {
-    unsigned char* smem; uint32_t s, tmem; volatile int* aborta; Barras bar;
+    unsigned char* smem; uint32_t s, tmem; uint32_t* slot; volatile int* aborta; Barras bar;
 };
-__device__ __forceinline__ Base comeca(unsigned char* bruto, uint32_t off, int barras, int colunas) {
+__device__ __forceinline__ Base comeca(unsigned char* bruto, uint32_t off, int barras) {
     Base b;
     // (pointer arithmetic on the array keeps the shared address space: a round trip through an integer makes every access generic)
     b.smem = bruto + ((1024u - (smem_u32(bruto) & 1023u)) & 1023u);
     b.s = smem_u32(b.smem);
     b.bar.base = b.s + off;
-    uint32_t* slot = reinterpret_cast<uint32_t*>(b.smem + off + 112);
+    b.slot = reinterpret_cast<uint32_t*>(b.smem + off + 112);
     b.aborta = reinterpret_cast<volatile int*>(b.smem + off + 116);
     if (threadIdx.x == 0) {
         for (int i = 0; i < barras; i++) mbar_init(b.bar[i], 1);
         *b.aborta = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x < 32) tmem_aloca(slot, colunas);
+    return b;
+}
+// Tensor memory, once per block (it waits until the blocks beside it leave enough: 512 columns per SM).  The blocks that need one window take
+// only the columns of the scores, so that three fit an SM; the output then goes over the scores, which everyone has read by then.
+__device__ __forceinline__ void aloca(Base& b, int colunas) {
+    if (threadIdx.x < 32) tmem_aloca(b.slot, colunas);
     tc_fence_antes();
     __syncthreads();
     tc_fence_depois();
-    b.tmem = *slot;
-    return b;
+    b.tmem = *b.slot;
 }
 __device__ __forceinline__ void termina(const Base& b, int colunas) {
     tc_fence_antes();
@@ -281,16 +319,31 @@ __device__ __forceinline__ void termina(const Base& b, int colunas) {
         tmem_libera(b.tmem, colunas);
     }
 }
-// one thread: window rows of a token-major or transposed operand -> shared memory
+// One thread: 32 n token rows of a token-major operand (the maps' boxes are 32 rows high).  With `gira`, the 32-row groups of a window are
+// turned: group p of the tile, which the MMA puts into tensor-memory lanes 32 p .. 32 p + 31 and which the warps p and p + 4 drain, is
+// group (p + gira) & 3 of the window.  Warp w sits on scheduler w & 3 of its SM and the groups near the diagonal have nearly all the
+// work, so without the turn (by the block's number) the blocks of an SM would all lean on the same two schedulers.
+__device__ __forceinline__ void linhas32(uint32_t dst, const CUtensorMap* m, int y, int n, int gira, uint32_t bar) {
+    for (int p = 0; p < n; p++) tma_2d(dst + p * 4096, m, 0, y + 32 * (n == 4 ? (p + gira) & 3 : p), bar);
+}
 __device__ __forceinline__ void carrega(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bytes, uint32_t bar) {
     mbar_expect_tx(bar, bytes);
     tma_2d(dst, m, x, y, bar);
 }
+__device__ __forceinline__ void carrega_janela(uint32_t dst, const CUtensorMap* m, int y, int gira, uint32_t bar) {
+    mbar_expect_tx(bar, TILE_A);
+    linhas32(dst, m, y, 4, gira, bar);
+}
 // the 64 hi and the 64 lo digit rows of a tile, token rows `lin` on (BHT rows to the lo digits)
 __device__ __forceinline__ void carrega_dig(uint32_t dst, const CUtensorMap* m, int lin, int BHT, uint32_t bar) {
     mbar_expect_tx(bar, 2 * TILE_N);
-    tma_2d(dst, m, 0, lin, bar);
-    tma_2d(dst + TILE_N, m, 0, BHT + lin, bar);
+    linhas32(dst, m, lin, 2, 0, bar);
+    linhas32(dst + TILE_N, m, BHT + lin, 2, 0, bar);
+}
+// a warp writes zeros to rows q0 .. q0 + 31, bytes 32 kq .. 32 kq + 31 of a swizzled tile
+__device__ __forceinline__ void zera_bloco(unsigned char* tile, int q0, int kq, int lane) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) *reinterpret_cast<uint4*>(tile + sw128(q0 + (lane >> 1) + 16 * k, 32 * kq + 16 * (lane & 1))) = make_uint4(0, 0, 0, 0);
 }
 // 32 bytes as numbers
 __device__ __forceinline__ int byte_u(const uint32_t (&w)[8], int k) { return (int)__byte_perm(w[k >> 2], 0, 0x4440 + (k & 3)); }
@@ -307,7 +360,7 @@ __device__ __forceinline__ int byte_u(const uint32_t (&w)[8], int k) { return (i
 // right-shift path, the only one that occurs in earnest; any other shift takes every window and the general roundings.
 //
 // Shared: Q digits 16 KB | K window 16 KB | V^T window 16 KB | P tile 8 KB; the output staging goes over the first three.
-// Tensor memory: scores 128 columns, O 64 (256 allocated: two blocks per SM).
+// Tensor memory: scores 128 columns, O 64.
 struct ArgsFrente {
     const int* em; const int* nrm;
     int* Oacc; int16_t* Oe; int8_t* Qm; int8_t* QE; uint8_t* P;   // Qm / QE: block output (head dimension 64, block length 32) instead of the raw one
@@ -316,25 +369,25 @@ struct ArgsFrente {
 constexpr uint32_t FR_K = 2 * TILE_N, FR_V = FR_K + TILE_A, FR_P = FR_V + TILE_A, FR_BAR = FR_P + TILE_N;
 constexpr size_t SM_FRENTE = 1024 + FR_BAR + 128 + (6 * NI + 2) * 4;
 
-__global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
+__global__ void __launch_bounds__(NTA, 3) k_at_frente(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
                                                       const __grid_constant__ CUtensorMap mVt, const ArgsFrente A) {
     extern __shared__ unsigned char bruto[];
     enum { B_Q = 0, B_K = 1, B_V = 2, B_S = 3, B_O = 4 };
-    const Base S = comeca(bruto, FR_BAR, 5, 256);
+    Base S = comeca(bruto, FR_BAR, 5);
     int* r_s = reinterpret_cast<int*>(S.smem + FR_BAR + 128);      // [4 lane quarters][64] partial maxima, partial sums
     int* m_s = r_s + 4 * NI;                                       // [64] row maxima
     int* i_s = m_s + NI;                                           // [64] 2^28 / row sum
     int* n_s = i_s + NI;                                           // [2] windows needed, per 32 queries
     const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), lt = 32 * quarto + lane;
     const int tile = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y, b = bh / H, h = bh % H, i0 = tile * NI, linha0 = b * T;
+    const int gira = (tile + bh) & 3, kq = (quarto + gira) & 3, jl = 32 * kq + lane;      // this warp's keys of a window, this thread's key
     const int j00 = i0 + NI - TJ;                                  // first key of the first window (may lie before the sequence: such rows are masked)
-    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
     pdl_espera();
     pdl_solta();
     if (tid == 0) {
         carrega_dig(S.s, &mQ, bh * T + i0, A.BH * T, S.bar[B_Q]);
-        carrega(S.s + FR_K, &mK, 0, bh * T + j00, TILE_A, S.bar[B_K]);
+        carrega_janela(S.s + FR_K, &mK, bh * T + j00, gira, S.bar[B_K]);
         carrega(S.s + FR_V, &mVt, j00, bh * 128, TILE_A, S.bar[B_V]);
     }
     const int emq = A.em[bh * 4], emk = A.em[bh * 4 + 1], emv = A.em[bh * 4 + 2];
@@ -342,13 +395,18 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
     const bool direita = s_u > 0 && s_u < 31;
     const int nmax = (i0 + NI - 1) / TJ + 1;
     int B = 0;                                                     // bound of the products in the units of the scores
-    if (direita && nmax > 1) {
+    if (direita) {
         const int nch = (T + TJ - 1) / TJ;
         const int nq = A.nrm[(size_t)bh * 2 * nch + i0 / TJ];
         int nk = lane <= min(i0 + NI - 1, T - 1) / TJ ? A.nrm[((size_t)bh * 2 + 1) * nch + lane] : 0;
         nk = __reduce_max_sync(FULL, nk);
-        B = (int)(((long long)sqrt((double)nq * (double)nk) + 2) >> s_u) + 1;
+        B = (__float2int_ru(__fsqrt_ru(__fmul_ru(__int2float_ru(nq), __int2float_ru(nk)))) >> s_u) + 2;
     }
+    // (from the norms alone, u_ii >= -B: usually this already says one window)
+    const bool talvez_mais = nmax > 1 && (!direita || 65 << incl < 2130 + 2 * B);
+    const int colunas = talvez_mais ? 256 : SB;
+    aloca(S, colunas);
+    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16), t_o = talvez_mais ? SB : 0;
     // zeros of P outside the first window, while the loads are on their way (further windows overwrite their part)
     for (int t = tid; t < T * 4; t += NTA) {
         const int j = t >> 2, i = i0 + 16 * (t & 3);
@@ -357,7 +415,7 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
     int v[32];                                                     // this thread's 32 scores of the window at hand, then their exponentials
     int minha = U_MIN;                                             // query q0 + lane: maximum, then sum, over this warp's keys
     int n = 1, passo = 0;                                          // windows; score computations so far
-    bool ok = true, tem_ex = false;
+    bool ok = true, tem_ex = false, sem_efeito = false;            // v holds exponentials; they are all zero
 #pragma unroll 1
     for (int fase = 0; fase < 3; fase++) {
         if (fase == 1) minha = 0;
@@ -366,15 +424,19 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
             const int j = j00 - s * TJ + jl, dj = i0 + q0 - j;     // dj + k = distance of query k to this key
             const bool ha = j >= 0 && j < T && i0 + q0 < T;
             const int kmin = ha ? -dj : 32;                        // the key counts for query k >= kmin
+            // Nothing of this warp's 32 keys x 32 queries counts: all beyond the diagonal or outside the sequence, or all so far behind it
+            // that u_ij <= B - d 2^incl stays 2130 below u_ii >= -B.
+            const int perto = i0 + q0 - (j00 - s * TJ + 32 * kq + 31);      // the smallest distance (query minus key), 62 below the largest
+            bool morto = j - lane + 31 < 0 || perto < -62 || i0 + q0 >= T || (direita && perto > 0 && perto << incl >= 2130 + 2 * B);
             if (fase == 0 || n > 1) {
                 if (passo) { tc_fence_antes(); __syncthreads(); }   // everyone has read the previous scores
                 if (tid == 0 && ok) {
-                    if (passo) carrega(S.s + FR_K, &mK, 0, bh * T + j00 - s * TJ, TILE_A, S.bar[B_K]);
+                    if (passo) carrega_janela(S.s + FR_K, &mK, bh * T + j00 - s * TJ, gira, S.bar[B_K]);
                     else ok = espera(S.bar[B_Q], 0, S.aborta, kid, 20);
                     ok = ok && espera(S.bar[B_K], passo & 1, S.aborta, kid, 21);
                     if (ok) {
                         tc_fence_depois();
-                        mma_escores(S.tmem, desc_sw128(S.s + FR_K), desc_sw128(S.s));
+                        mma_escores(S.tmem, desc_sw128(S.s + FR_K), desc_sw128(S.s), hd);
                         tc_commit(S.bar[B_S]);
                     }
                 }
@@ -382,6 +444,7 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
                 ok = __all_sync(FULL, ok && espera(S.bar[B_S], passo & 1, S.aborta, kid, 22));
                 tc_fence_depois();
                 passo++;
+                if (!morto)
 #pragma unroll
                 for (int g = 0; g < 2; g++) {
                     int x[16];
@@ -405,6 +468,7 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
                 }
             }
             if (fase == 0) {
+                if (!morto)
 #pragma unroll
                 for (int k = 0; k < 32; k++) {
                     const int r = __reduce_max_sync(FULL, v[k]);
@@ -416,8 +480,8 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
                     if (tid < NI) {
                         const int m = max(max(r_s[tid], r_s[NI + tid]), max(r_s[2 * NI + tid], r_s[3 * NI + tid]));
                         m_s[tid] = m;
-                        int ni = nmax;
-                        if (direita) {
+                        int ni = talvez_mais ? nmax : 1;
+                        if (direita && talvez_mais) {
                             // keys from distance `longe` on do not count; n windows leave out the distances tid + 65 + 128 (n - 1) and more
                             const int longe = max((2130 + B - m + (1 << incl) - 1) >> incl, 0);
                             ni = i0 + tid < T ? 1 + max((longe - (tid + 65) + TJ - 1) / TJ, 0) : 1;
@@ -430,15 +494,25 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
                 }
                 continue;
             }
-            if (!tem_ex) {
+            if (!morto && !tem_ex) {
+                int dmin = 6000;
 #pragma unroll
                 for (int k = 0; k < 32; k++) {
                     const int m = m_s[q0 + k];                     // a key beyond the diagonal is infinitely far below
-                    v[k] = exp3_t((uint32_t)(k < kmin || v[k] <= m - 6000 ? 6000 : m - v[k]) * 23637u + (13u << 22));
+                    v[k] = k < kmin || v[k] <= m - 6000 ? 6000 : m - v[k];
+                    dmin = min(dmin, v[k]);
                 }
+                if (__any_sync(FULL, dmin < 2130)) {
+#pragma unroll
+                    for (int k = 0; k < 32; k++) v[k] = exp3_t((uint32_t)v[k] * 23637u + (13u << 22));
+                } else
+                    sem_efeito = true;
                 tem_ex = n == 1;
             }
+            morto = morto || sem_efeito;
+            if (n > 1) sem_efeito = false;
             if (fase == 1) {
+                if (!morto)
 #pragma unroll
                 for (int k = 0; k < 32; k++) {
                     const int r = __reduce_add_sync(FULL, v[k]);
@@ -447,19 +521,22 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
                 continue;
             }
             if (s) ok = __all_sync(FULL, ok && espera(S.bar[B_O], (s - 1) & 1, S.aborta, kid, 23));      // the P tile and the V stage are free again
-            uint32_t w[8];
+            uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            if (morto) zera_bloco(S.smem + FR_P, q0, kq, lane);
+            else
 #pragma unroll
-            for (int k = 0; k < 32; k++) {
-                const int p = min((v[k] * i_s[q0 + k] + (1 << 19)) >> 20, 255);
-                w[k >> 2] = (k & 3) == 0 ? (uint32_t)p : w[k >> 2] | (uint32_t)p << (8 * (k & 3));
-                S.smem[FR_P + sw128(q0 + k, jl)] = (uint8_t)p;
-            }
+                for (int k = 0; k < 32; k++) {
+                    const int p = min((v[k] * i_s[q0 + k] + (1 << 19)) >> 20, 255);
+                    w[k >> 2] = (k & 3) == 0 ? (uint32_t)p : w[k >> 2] | (uint32_t)p << (8 * (k & 3));
+                    S.smem[FR_P + sw128(q0 + k, jl)] = (uint8_t)p;
+                }
             if (ha) {
                 uint4* d = reinterpret_cast<uint4*>(A.P + ((size_t)bh * T + j) * T + i0 + q0);
                 d[0] = make_uint4(w[0], w[1], w[2], w[3]);
                 d[1] = make_uint4(w[4], w[5], w[6], w[7]);
             }
             fence_async();                                         // the tile is read by the tensor core (async proxy)
+            tc_fence_antes();
             __syncthreads();
             if (tid == 0 && ok) {
                 if (s) carrega(S.s + FR_V, &mVt, j00 - s * TJ, bh * 128, TILE_A, S.bar[B_V]);
@@ -468,7 +545,7 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
                     tc_fence_depois();
                     const uint64_t da = desc_sw128(S.s + FR_V), db = desc_sw128(S.s + FR_P);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) tc_mma_i8(S.tmem + SB, da + 2 * q, db + 2 * q, ID_PU, (s | q) != 0);
+                    for (int q = 0; q < 4; q++) tc_mma_i8(S.tmem + t_o, da + 2 * q, db + 2 * q, ID_PU, (s | q) != 0);
                     tc_commit(S.bar[B_O]);
                 }
             }
@@ -490,9 +567,9 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
     int* o_s = reinterpret_cast<int*>(S.smem);                     // [128 digit rows][65] over the operands
     if (ok) {
         uint32_t d[32];
-        tmem_le32(t_lane + SB + q0, d);
+        tmem_le32(t_lane + t_o + q0, d);
 #pragma unroll
-        for (int k = 0; k < 32; k++) o_s[jl * 65 + q0 + k] = (int)d[k];
+        for (int k = 0; k < 32; k++) o_s[lt * 65 + q0 + k] = (int)d[k];
     }
     __syncthreads();
     for (int t = tid; t < NI * hd / 8; t += NTA) {                 // (whole warps: 64 or 16 columns of 64 rows)
@@ -503,7 +580,7 @@ __global__ void __launch_bounds__(NTA, 2) k_at_frente(const __grid_constant__ CU
         const size_t lin = (size_t)(linha0 + min(i0 + i, T - 1));
         grava8(A.Oacc, A.Oe, A.Qm, A.QE, lin * D + h * hd + d0, lin * (D / 32) + (h * hd + d0) / 32, o, (emv - GA) - 8, kid, t, i0 + i < T);
     }
-    termina(S, 256);
+    termina(S, colunas);
 }
 
 // -------------------------------------------------------------------------------------------------- backward
@@ -567,11 +644,12 @@ __device__ void mapa_p(const ArgsTras& A, int bh, int kt, unsigned* ou) {
     if (tid == 0) A.zm[bh * 16 + kt] = (int)*ou;
 }
 
-// Shared: dO digits 16 KB | two V windows 16 KB each; tensor memory: two score buffers.  The load of the window after next and the
-// product of the next one run behind the drain.
+// Shared: dO digits 16 KB | two V windows 16 KB each; tensor memory: the scores.  The load of the next window runs behind the drain, the rest
+// overlaps among the four blocks of an SM.  Only the bit length of the maximum is used (ops.py:235), and 64 hi + lo rounded towards
+// zero to fp32 has the bit length of the exact value: two instructions an element instead of seven.
 constexpr uint32_t MX_V = 2 * TILE_N, MX_BAR = MX_V + 2 * TILE_A;
 constexpr size_t SM_MAX = 1024 + MX_BAR + 128;
-__global__ void __launch_bounds__(NTA, 2) k_ab_max(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
+__global__ void __launch_bounds__(NTA, 4) k_ab_max(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
     extern __shared__ unsigned char bruto[];
     __shared__ int red[NTA / 32];
     __shared__ unsigned ou;
@@ -583,77 +661,88 @@ __global__ void __launch_bounds__(NTA, 2) k_ab_max(const __grid_constant__ CUten
         return;
     }
     enum { B_G = 0, B_V = 1, B_S = 3 };
-    const Base S = comeca(bruto, MX_BAR, 5, 256);
+    Base S = comeca(bruto, MX_BAR, 4);
+    aloca(S, SB);
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane, kid = A.kid;
     const int item = blockIdx.x - A.blocos_mapa, bh = item % A.BH, i0 = (nt - 1 - item / A.BH) * NI, j00 = i0 + NI - TJ, n = (i0 + NI - 1) / TJ + 1;
     const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
     pdl_espera();
     pdl_solta();
-    auto emite = [&](int s) -> bool {                              // one thread
-        if (!espera(S.bar[B_V + (s & 1)], (s >> 1) & 1, S.aborta, kid, 31)) return false;
-        tc_fence_depois();
-        mma_escores(S.tmem + (s & 1) * SB, desc_sw128(S.s + MX_V + (s & 1) * TILE_A), desc_sw128(S.s));
-        tc_commit(S.bar[B_S + (s & 1)]);
-        return true;
-    };
     bool ok = true;
     if (tid == 0) {
         carrega_dig(S.s, &mG, bh * T + i0, A.BH * T, S.bar[B_G]);
         for (int s = 0; s < 2 && s < n; s++) carrega(S.s + MX_V + s * TILE_A, &mV, 0, bh * T + j00 - s * TJ, TILE_A, S.bar[B_V + s]);
-        ok = espera(S.bar[B_G], 0, S.aborta, kid, 30) && emite(0);
+        ok = espera(S.bar[B_G], 0, S.aborta, kid, 30);
     }
-    int mx = 0;
+    float mx = 0.0f;
     for (int s = 0; s < n; s++) {
-        __syncwarp();
-        ok = __all_sync(FULL, ok && espera(S.bar[B_S + (s & 1)], (s >> 1) & 1, S.aborta, kid, 32));
-        tc_fence_depois();
-        if (tid == 0 && ok) {                                      // this product is done: its V stage takes the window after next
-            if (s + 2 < n) carrega(S.s + MX_V + (s & 1) * TILE_A, &mV, 0, bh * T + j00 - (s + 2) * TJ, TILE_A, S.bar[B_V + (s & 1)]);
-            if (s + 1 < n) ok = emite(s + 1);
+        if (tid == 0 && ok) {
+            ok = espera(S.bar[B_V + (s & 1)], (s >> 1) & 1, S.aborta, kid, 31);
+            if (ok) {
+                tc_fence_depois();
+                mma_escores(S.tmem, desc_sw128(S.s + MX_V + (s & 1) * TILE_A), desc_sw128(S.s), A.hd);
+                tc_commit(S.bar[B_S]);
+            }
         }
+        __syncwarp();
+        ok = __all_sync(FULL, ok && espera(S.bar[B_S], s & 1, S.aborta, kid, 32));
+        tc_fence_depois();
+        if (tid == 0 && ok && s + 2 < n)                           // this product is done: its V stage takes the window after next
+            carrega(S.s + MX_V + (s & 1) * TILE_A, &mV, 0, bh * T + j00 - (s + 2) * TJ, TILE_A, S.bar[B_V + (s & 1)]);
         __syncwarp();
         const int j = j00 - s * TJ + jl, kmin = j >= 0 && i0 + q0 < T ? j - i0 - q0 : 32;
+        if (kmin < 32 || s == 0)                                   // (s == 0: a mixed warp reads together)
 #pragma unroll
         for (int g = 0; g < 2; g++) {
-            int x[16];
-            escores16(t_lane + (s & 1) * SB + q0 + 16 * g, x);
+            uint32_t hi[16], lo[16];
+            escores16_cru(t_lane + q0 + 16 * g, hi, lo);
+            if (s) {
 #pragma unroll
-            for (int k = 0; k < 16; k++) mx = max(mx, 16 * g + k >= kmin ? abs(x[k]) : 0);
+                for (int k = 0; k < 16; k++) mx = fmaxf(mx, fabsf(__fmaf_rz(__uint_as_float(hi[k]), 64.0f, __uint_as_float(lo[k]))));
+            } else {
+#pragma unroll
+                for (int k = 0; k < 16; k++) {
+                    const float x = fabsf(__fmaf_rz(__uint_as_float(hi[k]), 64.0f, __uint_as_float(lo[k])));
+                    mx = fmaxf(mx, 16 * g + k >= kmin ? x : 0.0f);
+                }
+            }
         }
         tc_fence_antes();
-        __syncthreads();                                           // everyone has read this buffer: the product after next may write it
+        __syncthreads();                                           // everyone has read the scores: the next product may write them
     }
-    max_cta(mx, A.est + bh * at::N_EST + at::S_GP, red, tid);
-    termina(S, 256);
+    max_cta((int)mx, A.est + bh * at::N_EST + at::S_GP, red, tid);
+    termina(S, SB);
 }
 
 // Query tiles: s_lin and the maxima of dS.  With one live window gP' and P stay in registers between the two passes.
 // Shared: dO digits 16 KB | V window 16 KB; tensor memory: the scores.
 constexpr uint32_t SO_V = 2 * TILE_N, SO_BAR = SO_V + TILE_A;
 constexpr size_t SM_SOMA = 1024 + SO_BAR + 128 + 5 * NI * 4;
-__global__ void __launch_bounds__(NTA, 2) k_ab_soma(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
+__global__ void __launch_bounds__(NTA, 3) k_ab_soma(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
     extern __shared__ unsigned char bruto[];
     __shared__ int red[NTA / 32];
     enum { B_G = 0, B_V = 1, B_S = 2 };
-    const Base S = comeca(bruto, SO_BAR, 3, SB);
+    Base S = comeca(bruto, SO_BAR, 3);
+    aloca(S, SB);
     int* r_s = reinterpret_cast<int*>(S.smem + SO_BAR + 128);      // [4 lane quarters][64] partial sums
     int* sl_s = r_s + 4 * NI;                                      // [64]
-    const int T = A.T, kid = A.kid, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane;
+    const int T = A.T, kid = A.kid, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2);
     const int qt = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y, i0 = qt * NI, j00 = i0 + NI - TJ;
+    const int gira = (qt + bh) & 3, jl = 32 * ((quarto + gira) & 3) + lane;
     const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
     int* est = A.est + bh * at::N_EST;
     pdl_espera();
     pdl_solta();
     if (tid == 0) {
         carrega_dig(S.s, &mG, bh * T + i0, A.BH * T, S.bar[B_G]);
-        carrega(S.s + SO_V, &mV, 0, bh * T + j00, TILE_A, S.bar[B_V]);
+        carrega_janela(S.s + SO_V, &mV, bh * T + j00, gira, S.bar[B_V]);
     }
     const unsigned vivas = janelas_consulta(A, bh, qt);
     const bool uma = vivas == 1u;
     const Arred arred(at::desl1(est, A.limite));
     int v[32], minha = 0, mgp = 0, mds = 0, mp = 0, passo = 0;
     uint32_t w[8];
-    bool ok = true;
+    bool ok = true, morto = false;                                 // P is zero in this warp's 32 x 32 part of the window
 #pragma unroll 1
     for (int fase = 0; fase < 2; fase++) {
 #pragma unroll 1
@@ -669,14 +758,15 @@ __global__ void __launch_bounds__(NTA, 2) k_ab_soma(const __grid_constant__ CUte
                     const uint4 a = p[0], c = p[1];
                     w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y; w[6] = c.z; w[7] = c.w;
                 }
+                morto = !A.limite && !__any_sync(FULL, (w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0);
                 if (passo) { tc_fence_antes(); __syncthreads(); }   // everyone has read the previous scores
                 if (tid == 0 && ok) {
-                    if (passo) carrega(S.s + SO_V, &mV, 0, bh * T + j00 - s * TJ, TILE_A, S.bar[B_V]);
+                    if (passo) carrega_janela(S.s + SO_V, &mV, bh * T + j00 - s * TJ, gira, S.bar[B_V]);
                     else ok = espera(S.bar[B_G], 0, S.aborta, kid, 33);
                     ok = ok && espera(S.bar[B_V], passo & 1, S.aborta, kid, 34);
                     if (ok) {
                         tc_fence_depois();
-                        mma_escores(S.tmem, desc_sw128(S.s + SO_V), desc_sw128(S.s));
+                        mma_escores(S.tmem, desc_sw128(S.s + SO_V), desc_sw128(S.s), A.hd);
                         tc_commit(S.bar[B_S]);
                     }
                 }
@@ -684,6 +774,7 @@ __global__ void __launch_bounds__(NTA, 2) k_ab_soma(const __grid_constant__ CUte
                 ok = __all_sync(FULL, ok && espera(S.bar[B_S], passo & 1, S.aborta, kid, 35));
                 tc_fence_depois();
                 passo++;
+                if (!morto)
 #pragma unroll
                 for (int g = 0; g < 2; g++) {
                     int x[16];
@@ -692,6 +783,7 @@ __global__ void __launch_bounds__(NTA, 2) k_ab_soma(const __grid_constant__ CUte
                     for (int k = 0; k < 16; k++) v[16 * g + k] = 16 * g + k >= kmin ? arred(x[k]) : 0;
                 }
             }
+            if (morto) continue;
             if (fase == 0) {
 #pragma unroll
                 for (int k = 0; k < 32; k++) {
@@ -732,38 +824,51 @@ __global__ void __launch_bounds__(NTA, 2) k_ab_soma(const __grid_constant__ CUte
 //   gq, gk: scores (lane = the other side's token in the window, column = the tile's token), dS' as digits into an MMA tile
 //           (hi rows 0..63, lo rows 64..127, 128 bytes of window), then D[digit row of k or q][hi | lo column] += X^T . dS'.
 //   gv:     dO^T . P only, both operands straight from memory.
-// Shared: tile digits 16 KB | window 16 KB | transposed window 16 KB | dS' 16 KB | P tile 8 KB (key tiles); the output staging goes
-// over the first four.  Tensor memory: scores 128 columns, output 128 (256 allocated: two blocks per SM).
-constexpr uint32_t SA_A = 2 * TILE_N, SA_X = SA_A + TILE_A, SA_D = SA_X + TILE_A, SA_P = SA_D + 2 * TILE_N, SA_BAR = SA_P + TILE_N;
+// A warp whose 32 x 32 part of P is zero (half of them or more near the diagonal) only writes zeros of dS'.
+// Shared, query tiles: dO digits 16 KB | v window 16 KB | transposed window 16 KB; key tiles: v 8 KB, P tile 8 KB | dO digits of the window
+// 32 KB | transposed window 16 KB.  The dS' digits (16 KB) go over the window, which the scores have used up by then, and the output
+// staging over everything.  Tensor memory: scores 128 columns, output 128 over them or, with several windows, beside them.
+constexpr uint32_t SA_P = TILE_N, SA_A = 2 * TILE_N, SA_D = SA_A, SA_X = SA_A + 2 * TILE_A, SA_BAR = 2 * 128 * 65 * 4;
+static_assert(SA_X + TILE_A <= SA_BAR, "the barriers lie behind the operands and the staging");
 constexpr size_t SM_SAIDA = 1024 + SA_BAR + 128 + NI * 4;
-static_assert(2 * 128 * 65 * 4 <= SA_BAR, "the staging lies below the barriers");
 
 template <bool CHAVE>
-__device__ __forceinline__ void ab_saida(const Base& S, const CUtensorMap& mB, const CUtensorMap& mA, const CUtensorMap& mX, const CUtensorMap& mP,
+__device__ __forceinline__ int ab_saida(Base& S, const CUtensorMap& mB, const CUtensorMap& mA, const CUtensorMap& mX, const CUtensorMap& mP,
                                          const ArgsTras& A, int bh, int tile) {
     enum { B_B = 0, B_A = 1, B_X = 2, B_S = 3, B_O = 4 };
     int* sl_s = reinterpret_cast<int*>(S.smem + SA_BAR + 128);     // [64], query tiles
     const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), jl = 32 * quarto + lane;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), lt = 32 * quarto + lane;
+    const int gira = (tile + bh) & 3, kq = (quarto + gira) & 3, jl = 32 * kq + lane;      // this thread's token of a window
     const int b = bh / H, h = bh % H, t0 = tile * NI, w0 = CHAVE ? t0 : t0 + NI - TJ, wp = CHAVE ? TJ : -TJ;      // window s starts at token w0 + s wp
-    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
     const int* est = A.est + bh * at::N_EST;
     auto janela = [&](int s) {                                     // one thread: the operands of window s
         const int t = w0 + s * wp;
-        carrega(S.s + SA_A, &mA, 0, bh * T + t, TILE_A, S.bar[B_A]);
+        if (CHAVE) {
+            mbar_expect_tx(S.bar[B_A], 2 * TILE_A);
+            linhas32(S.s + SA_A, &mA, bh * T + t, 4, gira, S.bar[B_A]);
+            linhas32(S.s + SA_A + TILE_A, &mA, (A.BH + bh) * T + t, 4, gira, S.bar[B_A]);
+        } else
+            carrega_janela(S.s + SA_A, &mA, bh * T + t, gira, S.bar[B_A]);
         mbar_expect_tx(S.bar[B_X], TILE_A + (CHAVE ? TILE_N : 0));
         tma_2d(S.s + SA_X, &mX, t, bh * 128, S.bar[B_X]);
         if (CHAVE) tma_2d(S.s + SA_P, &mP, t, bh * T + t0, S.bar[B_X]);
     };
     if (tid == 0) {
-        carrega_dig(S.s, &mB, bh * T + t0, A.BH * T, S.bar[B_B]);
+        if (CHAVE) {
+            mbar_expect_tx(S.bar[B_B], TILE_N);
+            linhas32(S.s, &mB, bh * T + t0, 2, 0, S.bar[B_B]);
+        } else
+            carrega_dig(S.s, &mB, bh * T + t0, A.BH * T, S.bar[B_B]);
         janela(0);
     }
     const int sh = at::desl1(est, A.limite), sh2 = at::desl2(est, A.limite);
     const Arred arred(sh), arred2(sh2);
     const unsigned vivas = CHAVE ? janelas_chave(A, bh, tile) : janelas_consulta(A, bh, tile);
+    const int colunas = vivas == 1u ? SB : 2 * SB;
     if (!CHAVE && tid < NI) sl_s[tid] = A.sl[(size_t)bh * T + min(t0 + tid, T - 1)];
-    if (!CHAVE) __syncthreads();
+    aloca(S, colunas);
+    const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16), t_o = colunas - SB;
     int passo = 0;
     bool ok = true;
 #pragma unroll 1
@@ -776,7 +881,8 @@ __device__ __forceinline__ void ab_saida(const Base& S, const CUtensorMap& mB, c
             ok = ok && espera(S.bar[B_A], passo & 1, S.aborta, kid, 38);
             if (ok) {
                 tc_fence_depois();
-                mma_escores(S.tmem, desc_sw128(S.s + SA_A), desc_sw128(S.s));
+                if (CHAVE) mma_escores_a(S.tmem, desc_sw128(S.s + SA_A), desc_sw128(S.s + SA_A + TILE_A), desc_sw128(S.s), hd);
+                else mma_escores(S.tmem, desc_sw128(S.s + SA_A), desc_sw128(S.s), hd);
                 tc_commit(S.bar[B_S]);
             }
         }
@@ -789,9 +895,21 @@ __device__ __forceinline__ void ab_saida(const Base& S, const CUtensorMap& mB, c
             w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y; w[6] = c.z; w[7] = c.w;
         }
         __syncwarp();
-        ok = __all_sync(FULL, ok && (!CHAVE || espera(S.bar[B_X], passo & 1, S.aborta, kid, 39)) && espera(S.bar[B_S], passo & 1, S.aborta, kid, 40));
+        ok = __all_sync(FULL, ok && (!CHAVE || espera(S.bar[B_X], passo & 1, S.aborta, kid, 39)));
+        if (CHAVE) {                                               // only to see whether anything is there
+            const uint4 a = *reinterpret_cast<const uint4*>(S.smem + SA_P + sw128(q0 + (lane >> 1), 32 * kq + 16 * (lane & 1))),
+                        c = *reinterpret_cast<const uint4*>(S.smem + SA_P + sw128(q0 + 16 + (lane >> 1), 32 * kq + 16 * (lane & 1)));
+            w[0] = a.x | a.y | a.z | a.w | c.x | c.y | c.z | c.w;
+        }
+        const bool morto = !__any_sync(FULL, (w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0);
+        ok = __all_sync(FULL, ok && espera(S.bar[B_S], passo & 1, S.aborta, kid, 40));
         tc_fence_depois();
+        if (morto) {
+            zera_bloco(S.smem + SA_D, q0, kq, lane);
+            zera_bloco(S.smem + SA_D + TILE_N, q0, kq, lane);
+        }
         const int dist = CHAVE ? t - t0 - q0 : t0 + q0 - t;        // query minus key at column q0
+        if (!morto)
 #pragma unroll
         for (int g = 0; g < 2; g++) {
             int x[16];
@@ -817,7 +935,7 @@ __device__ __forceinline__ void ab_saida(const Base& S, const CUtensorMap& mB, c
                 tc_fence_depois();
                 const uint64_t da = desc_sw128(S.s + SA_X), db = desc_sw128(S.s + SA_D);
 #pragma unroll
-                for (int q = 0; q < 4; q++) tc_mma_i8(S.tmem + SB, da + 2 * q, db + 2 * q, ID_S, (passo | q) != 0);
+                for (int q = 0; q < 4; q++) tc_mma_i8(S.tmem + t_o, da + 2 * q, db + 2 * q, ID_S, (passo | q) != 0);
                 tc_commit(S.bar[B_O]);
             }
         }
@@ -830,9 +948,9 @@ __device__ __forceinline__ void ab_saida(const Base& S, const CUtensorMap& mB, c
 #pragma unroll
         for (int a = 0; a < 2; a++) {
             uint32_t d[32];
-            tmem_le32(t_lane + SB + NI * a + q0, d);
+            tmem_le32(t_lane + t_o + NI * a + q0, d);
 #pragma unroll
-            for (int k = 0; k < 32; k++) o_s[(a * 128 + jl) * 65 + q0 + k] = (int)d[k];
+            for (int k = 0; k < 32; k++) o_s[(a * 128 + lt) * 65 + q0 + k] = (int)d[k];
         }
     }
     __syncthreads();
@@ -849,8 +967,9 @@ __device__ __forceinline__ void ab_saida(const Base& S, const CUtensorMap& mB, c
         const size_t lin = (size_t)(b * T + min(t0 + r, T - 1));
         grava8(A.Gacc, A.Ge, A.Gm, A.GE, lin * 3 * D + col + d0, lin * (3 * D / 32) + (col + d0) / 32, o, e, kid, n, t0 + r < T);
     }
+    return colunas;
 }
-__device__ __forceinline__ void ab_valor(const Base& S, const CUtensorMap& mX, const CUtensorMap& mP, const ArgsTras& A, int bh, int tile) {
+__device__ __forceinline__ void ab_valor(Base& S, const CUtensorMap& mX, const CUtensorMap& mP, const ArgsTras& A, int bh, int tile) {
     enum { B_X = 0, B_O = 2 };                                     // two stages
     constexpr uint32_t EST = TILE_A + TILE_N;
     const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
@@ -859,6 +978,7 @@ __device__ __forceinline__ void ab_valor(const Base& S, const CUtensorMap& mX, c
     const unsigned vivas = janelas_chave(A, bh, tile);
     const int n = __popc(vivas);
     bool ok = true;
+    aloca(S, NI);
     if (tid == 0) {
         auto janela = [&](int passo) {
             const int t = t0 + ((int)__fns(vivas, 0, passo + 1)) * TJ;
@@ -903,19 +1023,19 @@ __device__ __forceinline__ void ab_valor(const Base& S, const CUtensorMap& mX, c
         grava8(A.Gacc, A.Ge, A.Gm, A.GE, lin * 3 * D + col + d0, lin * (3 * D / 32) + (col + d0) / 32, o, e, kid, t, t0 + r < T);
     }
 }
-__global__ void __launch_bounds__(NTA, 2) k_ab_saida(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG,
-                                                     const __grid_constant__ CUtensorMap mVd, const __grid_constant__ CUtensorMap mGd,
+__global__ void __launch_bounds__(NTA, 3) k_ab_saida(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mGd,
                                                      const __grid_constant__ CUtensorMap mKt, const __grid_constant__ CUtensorMap mQt,
                                                      const __grid_constant__ CUtensorMap mGt, const __grid_constant__ CUtensorMap mP, const ArgsTras A) {
     extern __shared__ unsigned char bruto[];
-    const Base S = comeca(bruto, SA_BAR, 5, 256);
+    Base S = comeca(bruto, SA_BAR, 5);
     pdl_espera();
     pdl_solta();
     const int bh = blockIdx.y;
-    if (blockIdx.z == 0) ab_saida<true>(S, mVd, mG, mQt, mP, A, bh, blockIdx.x);
-    else if (blockIdx.z == 1) ab_saida<false>(S, mGd, mV, mKt, mP, A, bh, gridDim.x - 1 - blockIdx.x);
+    int colunas = NI;
+    if (blockIdx.z == 0) colunas = ab_saida<true>(S, mV, mGd, mQt, mP, A, bh, blockIdx.x);
+    else if (blockIdx.z == 1) colunas = ab_saida<false>(S, mGd, mV, mKt, mP, A, bh, gridDim.x - 1 - blockIdx.x);
     else ab_valor(S, mGt, mP, A, bh, blockIdx.x);
-    termina(S, 256);
+    termina(S, colunas);
 }
 
 }  // namespace atc
@@ -927,11 +1047,11 @@ static size_t atc_arredonda(size_t x) { return (x + 1023) & ~(size_t)1023; }
 static bool atc_serve(int blk, int T, int H, int D, int GA) {
     return (D == H * 64 || D == H * 16) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 && (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
 }
-// pieces of 128 tokens per preparation block: as many as leave two blocks per SM
+// pieces of 128 tokens per preparation block (each looks at the exponents of the whole sequence first): as many as leave 16 blocks per SM
 static int atc_por_cta(int T, int BH, int z) {
     const int np = (T + 127) / 128;
     int por = 1;
-    while (por < np && (long long)((np + 2 * por - 1) / (2 * por)) * BH * z >= 4 * N_SM) por *= 2;
+    while (por < np && (long long)((np + 2 * por - 1) / (2 * por)) * BH * z >= 16 * N_SM) por *= 2;
     return por;
 }
 
@@ -954,7 +1074,7 @@ static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* O
                         em, nullptr, nrm, BH, T, H, D, hd, GA, blk, por};
     lanca_pdl(atc::k_at_prep, dim3(((T + 127) / 128 + por - 1) / por, BH, 3), dim3(256), 0, st, Pp);
     CUtensorMap mQ, mK, mVt;
-    if (!(faz_mapa_h(&mQ, Qd, 2 * BH * T, 64, atc::NI) && faz_mapa_h(&mK, K, BH * T, 64, 128) && faz_mapa(&mVt, Vt, BH * 128, T, 128)))
+    if (!(faz_mapa_h(&mQ, Qd, 2 * BH * T, 64, 32) && faz_mapa_h(&mK, K, BH * T, 64, 32) && faz_mapa(&mVt, Vt, BH * 128, T, 128)))
         return (int)cudaErrorInvalidValue;
     cudaError_t c = at_smem(atc::k_at_frente, atc::SM_FRENTE);
     if (c != cudaSuccess) return (int)c;
@@ -963,29 +1083,29 @@ static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* O
     return (int)cudaGetLastError();
 }
 
-// backward: preparation (v, dO plain and digits; q, k, dO transposed), the maxima, the sums, the outputs
+// backward: preparation (v plain, dO digits; q, k, dO transposed), the maxima, the sums, the outputs
 static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const int8_t* qm, const int8_t* qE, const uint8_t* P, int* Gacc, int16_t* Ge,
                            int8_t* Gm, int8_t* GE, int Bt, int T, int H, int D, int GA, int limite, int kid, cudaStream_t st) {
     if (Gm && (blk != 32 || !GE || D != H * 64)) return (int)cudaErrorInvalidValue;
     const int BH = Bt * H, hd = D / H, nt = (T + atc::NI - 1) / atc::NI;
     const size_t b_est = atc_arredonda((size_t)BH * (at::N_EST + T + 4 + 16) * sizeof(int)), b_lin = atc_arredonda((size_t)BH * T * 128);
     unsigned char* ws = nullptr;
-    if (int r = at_ws(b_est + 9 * b_lin, st, reinterpret_cast<void**>(&ws))) return r;
+    if (int r = at_ws(b_est + 6 * b_lin, st, reinterpret_cast<void**>(&ws))) return r;
     int* est = reinterpret_cast<int*>(ws);
     int* sl = est + (size_t)BH * at::N_EST;
     int* em = sl + (size_t)BH * T;
     int* zm = em + (size_t)BH * 4;
     auto parte = [&](int n) { return ws + b_est + n * b_lin; };
-    uint16_t *V = (uint16_t*)parte(0), *G = (uint16_t*)parte(1), *Vd = (uint16_t*)parte(2), *Gd = (uint16_t*)parte(4);
-    int8_t *Qt = (int8_t*)parte(6), *Kt = (int8_t*)parte(7), *Gt = (int8_t*)parte(8);
+    uint16_t *V = (uint16_t*)parte(0), *Gd = (uint16_t*)parte(1);
+    int8_t *Qt = (int8_t*)parte(3), *Kt = (int8_t*)parte(4), *Gt = (int8_t*)parte(5);
     const int por = atc_por_cta(T, BH, 4);
-    atc::ArgsPrep Pp = {qm, qE, gom, goE, {nullptr, nullptr, V, G}, {nullptr, nullptr, Vd, Gd}, {Qt, Kt, nullptr, Gt},
+    atc::ArgsPrep Pp = {qm, qE, gom, goE, {nullptr, nullptr, V, nullptr}, {nullptr, nullptr, nullptr, Gd}, {Qt, Kt, nullptr, Gt},
                         em, est, nullptr, BH, T, H, D, hd, GA, blk, por};
     lanca_pdl(atc::k_at_prep, dim3(((T + 127) / 128 + por - 1) / por, BH, 4), dim3(256), 0, st, Pp);
-    CUtensorMap mV, mG, mVd, mGd, mKt, mQt, mGt, mP;
-    if (!(faz_mapa_h(&mV, V, BH * T, 64, 128) && faz_mapa_h(&mG, G, BH * T, 64, 128) && faz_mapa_h(&mVd, Vd, 2 * BH * T, 64, atc::NI) &&
-          faz_mapa_h(&mGd, Gd, 2 * BH * T, 64, atc::NI) && faz_mapa(&mKt, Kt, BH * 128, T, 128) && faz_mapa(&mQt, Qt, BH * 128, T, 128) &&
-          faz_mapa(&mGt, Gt, BH * 128, T, 128) && faz_mapa(&mP, P, BH * T, T, atc::NI)))
+    CUtensorMap mV, mV128, mGd, mKt, mQt, mGt, mP;
+    if (!(faz_mapa_h(&mV, V, BH * T, 64, 32) && faz_mapa_h(&mV128, V, BH * T, 64, 128) && faz_mapa_h(&mGd, Gd, 2 * BH * T, 64, 32) &&
+          faz_mapa(&mKt, Kt, BH * 128, T, 128) && faz_mapa(&mQt, Qt, BH * 128, T, 128) && faz_mapa(&mGt, Gt, BH * 128, T, 128) &&
+          faz_mapa(&mP, P, BH * T, T, atc::NI)))
         return (int)cudaErrorInvalidValue;
     // up to two key tiles the first window is all there is: no map
     const atc::ArgsTras A = {P, Gacc, Ge, est, sl, em, zm, Gm, GE, BH, T, H, D, hd, GA, limite, kid, nt > 2 ? BH * nt : 0};
@@ -996,12 +1116,12 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
         else at::k_lim<16><<<BH, 256, 0, st>>>(L);
     } else {
         if ((c = at_smem(atc::k_ab_max, atc::SM_MAX)) != cudaSuccess) return (int)c;
-        lanca_pdl(atc::k_ab_max, dim3(A.blocos_mapa + BH * nt), dim3(atc::NTA), atc::SM_MAX, st, mV, mGd, A);
+        lanca_pdl(atc::k_ab_max, dim3(A.blocos_mapa + BH * nt), dim3(atc::NTA), atc::SM_MAX, st, mV128, mGd, A);
     }
     if ((c = at_smem(atc::k_ab_soma, atc::SM_SOMA)) != cudaSuccess) return (int)c;
     lanca_pdl(atc::k_ab_soma, dim3(nt, BH), dim3(atc::NTA), atc::SM_SOMA, st, mV, mGd, A);
     if ((c = at_smem(atc::k_ab_saida, atc::SM_SAIDA)) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_saida, dim3(nt, BH, 3), dim3(atc::NTA), atc::SM_SAIDA, st, mV, mG, mVd, mGd, mKt, mQt, mGt, mP, A);
+    lanca_pdl(atc::k_ab_saida, dim3(nt, BH, 3), dim3(atc::NTA), atc::SM_SAIDA, st, mV, mGd, mKt, mQt, mGt, mP, A);
     return (int)cudaGetLastError();
 }
 

@@ -66,6 +66,36 @@ static inline void lanca_pdl(void (*k)(KP...), dim3 grade, dim3 bloco, size_t sm
     (void)cudaLaunchKernelEx(&c, k, a...);                         // errors surface through cudaGetLastError like those of <<< >>>
 }
 
+// ---------------------------------------------------------------------------------------- fp32 pairs
+constexpr uint32_t MAGIA = 0x4B400000u;                        // bit pattern of 1.5 * 2^23
+constexpr float MAGIA_F = 12582912.0f;
+// two fp32 lanes per instruction
+__device__ __forceinline__ uint64_t par(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t par_f(float lo, float hi) { return par(__float_as_uint(lo), __float_as_uint(hi)); }
+__device__ __forceinline__ void separa(uint64_t v, uint32_t& lo, uint32_t& hi) { asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v)); }
+__device__ __forceinline__ float f_lo(uint64_t a) { return __uint_as_float((uint32_t)a); }
+__device__ __forceinline__ float f_hi(uint64_t a) { return __uint_as_float((uint32_t)(a >> 32)); }
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float pot2(int e) { return __int_as_float((e + 127) << 23); }      // 2^e, -126 <= e <= 127
+
 // ---------------------------------------------------------------------------------------- arithmetic
 __device__ __forceinline__ int bitlen(int x) { return 32 - __clz(x < 0 ? -x : x); }
 

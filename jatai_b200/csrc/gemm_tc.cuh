@@ -57,8 +57,6 @@ constexpr long long LIMITE_CICLOS = 4000000000LL;              // ~2 s at B200 c
 __device__ long long g_limite_espera = LIMITE_CICLOS;          // the limit in force (jt_espera_limite); read on the slow path of a wait only
 __device__ int g_sem_cargas = 0;                               // test switch (jt_gemm_sem_cargas): the producer issues no operand load, so the
                                                                // first wait of the MMA warp runs out with nothing asynchronous in flight
-constexpr uint32_t MAGIA = 0x4B400000u;                        // bit pattern of 1.5 * 2^23
-constexpr float MAGIA_F = 12582912.0f;
 constexpr int DESLOC = 32 * 127 * 127;                         // the largest |partial product| of 32 int8 pairs
 
 // ------------------------------------------------------------------------------------------ PTX wrappers
@@ -164,21 +162,6 @@ __device__ __forceinline__ void tmem_le8x2(uint32_t ta, uint32_t tb, uint32_t (&
         : "r"(ta), "r"(tb)
         : "memory");
 }
-// two fp32 lanes per instruction (fma.rn.f32x2): the align/round loop is bound by instruction issue, not by the FMA pipe
-__device__ __forceinline__ uint64_t par(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t par_f(float lo, float hi) { return par(__float_as_uint(lo), __float_as_uint(hi)); }
-__device__ __forceinline__ void separa(uint64_t v, uint32_t& lo, uint32_t& hi) { asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
-__device__ __forceinline__ float pot2(int e) { return __int_as_float((127 + e) << 23); }      // 2^e, -126 <= e <= 127
 
 // How a K-block's partial product p (exact int32 from tensor memory, |p| <= 32 * 127^2 < 2^19) becomes rnd(p << 4, sa + sb):
 // VIA 1 (block 32): every slice gets a second MMA of two constant operands (all bytes 127) onto the same accumulator, so what
