@@ -145,7 +145,7 @@ struct ArgsPrep {
     int* em;                    // [BH][4] head-maximum exponents, indexed by z
     int* est;                   // backward: the statistics slots [BH][N_EST] to clear (nullptr in the forward)
     int* nrm;                   // forward: [BH][2][ceil(T/128)] largest sum of squares of an aligned row of q (0) / k (1) per 128 tokens
-    int BH, T, H, D, hd, GA, blk, por_cta;       // por_cta: 128-token pieces of a CTA
+    int BH, T, H, D, GA, blk, por_cta;           // por_cta: 128-token pieces of a CTA
 };
 __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats that halves hold exactly
     uint32_t r;
@@ -153,44 +153,54 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
     return r;
 }
 
-// grid (CTAs per head, BH, 3 or 4), 256 threads: `por_cta` pieces of 128 tokens of one head of one tensor.  The bound of a plain version (one
-// element at a time in integers, digit bytes stored one by one) was instruction issue, three times the memory time.  So: a thread takes 4
-// tokens x 8 columns; pairs of elements in f32x2 (a byte becomes a float by its place in 2^23's mantissa; v 2^(GA - s) rounds to even in one
-// FMA against 1.5 * 2^23, exactly rnd_d; the 6-bit digits are hi = round(r / 64), lo = r - 64 hi); the transposed digits of 4 tokens are
-// packed into a word and cross shared memory in 16-byte pieces swapped by the column group, without bank conflicts.
-// 16 x 1024 tokens, 16 heads of 64, forward + backward: 218 -> XX us.
+// grid (CTAs per 64 columns, sequences x groups of 64 / hd heads, 3 or 4), 256 threads: `por_cta` pieces of 128 tokens of 64 columns - one
+// head of 64 or four of 16 - of one tensor.  The bound of a plain version (one element at a time in integers, digit bytes stored one by
+// one) was instruction issue, three times the memory time.  So: a thread takes 4 tokens x 8 columns; pairs of elements in f32x2 (a byte
+// becomes a float by its place in 2^23's mantissa; v 2^(GA - s) rounds to even in one FMA against 1.5 * 2^23, exactly rnd_d; the 6-bit
+// digits are hi = round(r / 64), lo = r - 64 hi); the transposed digits of 4 tokens are packed into a word and cross shared memory in
+// 16-byte pieces swapped by the column group, without bank conflicts.
+// 16 x 1024 tokens, forward + backward: 16 heads of 64 218 -> 181 us, 16 heads of 16 196 -> 63 us.
+template <int hd>
 __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
-    __shared__ int red[8];
+    __shared__ int red[8 * 8];
     __shared__ __align__(16) uint32_t tr[128 * 32];
-    const int tid = threadIdx.x, z = blockIdx.z, bh = blockIdx.y, b = bh / A.H, h = bh % A.H;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, z = blockIdx.z, hpc = 64 / hd, gh = (A.H + hpc - 1) / hpc;
+    const int b = blockIdx.y / gh, h0 = blockIdx.y % gh * hpc;     // first head of the group
     uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
     uint16_t* dg = z == 0 ? A.dig[0] : z == 1 ? A.dig[1] : z == 2 ? A.dig[2] : A.dig[3];
     int8_t* dt = z == 0 ? A.tra[0] : z == 1 ? A.tra[1] : z == 2 ? A.tra[2] : A.tra[3];
-    const int T = A.T, D = A.D, blk = A.blk, hd = A.hd, linha0 = b * T;
+    const int T = A.T, D = A.D, blk = A.blk, linha0 = b * T;
     const int8_t* m = z == 3 ? A.gm : A.qm;
     const int8_t* E = z == 3 ? A.gE : A.qE;
-    const int ld = z == 3 ? D : 3 * D, col0 = z == 3 ? h * hd : z * D + h * hd, ldb = ld / blk;
+    const int ld = z == 3 ? D : 3 * D, col0 = (z == 3 ? 0 : z * D) + h0 * hd, ldb = ld / blk;
     const int cg = tid & 7, tg = tid >> 3;                         // columns 8 cg .. + 7, tokens 4 tg .. + 3 of a piece
-    const bool ha = 8 * cg < hd;
+    const int h = h0 + 8 * cg / hd, ch = 8 * cg % hd, bh = b * A.H + h;
+    const bool ha = h < A.H;
     const size_t BHT = (size_t)A.BH * T;
     pdl_espera();
     pdl_solta();
-    int em = -128;
+    int em;
     {
-        const int nbh = hd > blk ? hd / blk : 1;
-        const int8_t* pe = E + (size_t)linha0 * ldb + col0 / blk;
-        for (int t = tid; t < T; t += 256)
-            for (int k = 0; k < nbh; k++) em = max(em, (int)pe[(size_t)t * ldb + k]);
-        em = __reduce_max_sync(FULL, em);
-        if ((tid & 31) == 0) red[tid >> 5] = em;
+        // maximum exponents of the two halves of 32 columns (a head of 16 lies in one of them, a head of 64 in both)
+        const int8_t* pe = E + (size_t)linha0 * ldb;
+        const bool segunda = h0 * hd + 32 < D;
+        int e0 = -128, e1 = -128;
+        for (int t = tid; t < T; t += 256) {
+            e0 = max(e0, (int)pe[(size_t)t * ldb + col0 / blk]);
+            if (segunda) e1 = max(e1, (int)pe[(size_t)t * ldb + (col0 + 32) / blk]);
+        }
+        e0 = __reduce_max_sync(FULL, e0);
+        e1 = __reduce_max_sync(FULL, e1);
+        if (lane == 0) { red[wid] = e0; red[8 + wid] = e1; }
         __syncthreads();
-        em = red[0];
 #pragma unroll
-        for (int i = 1; i < 8; i++) em = max(em, red[i]);
+        for (int i = 0; i < 8; i++) { e0 = max(e0, red[i]); e1 = max(e1, red[8 + i]); }
+        if (hd == 64) e0 = e1 = max(e0, e1);
+        em = cg < 4 ? e0 : e1;
         __syncthreads();                                           // red[] is used again below
     }
-    if (blockIdx.x == 0 && tid == 0) A.em[bh * 4 + z] = em;
-    if (A.est && blockIdx.x == 0 && z == 3 && tid < at::N_EST) A.est[bh * at::N_EST + tid] = 0;
+    if (blockIdx.x == 0 && tid < 8 && ch == 0 && ha) A.em[bh * 4 + z] = em;
+    if (A.est && blockIdx.x == 0 && z == 3 && tg < at::N_EST && ch == 0 && ha) A.est[bh * at::N_EST + tg] = 0;
     const uint64_t mag = par_f(MAGIA_F, MAGIA_F), menos_mag = par_f(-MAGIA_F, -MAGIA_F), vies = par_f(-8388736.0f, -8388736.0f);      // 2^23 + 128
     const uint64_t um64 = par_f(0.015625f, 0.015625f), m64 = par_f(-64.0f, -64.0f);
     for (int p = 0; p < A.por_cta; p++) {
@@ -232,28 +242,31 @@ __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
                 if (A.nrm) nk = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk));
             }
             if (dentro && ha) {
-                const size_t o = ((size_t)bh * T + t0 + 4 * tg + k) * 64 + 8 * cg;
+                const size_t o = ((size_t)bh * T + t0 + 4 * tg + k) * 64 + ch;
                 if (dp) *reinterpret_cast<uint4*>(dp + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
                 if (dg) {
                     *reinterpret_cast<uint4*>(dg + o) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
                     *reinterpret_cast<uint4*>(dg + BHT * 64 + o) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
                 }
             }
-            if (A.nrm && z < 2) {                                  // squared norm of the token's row: its 8 lanes are neighbours
+            if (A.nrm && z < 2) {                                  // squared norm of a head's row: its 8 or 2 lanes are neighbours
                 nk += __shfl_xor_sync(FULL, nk, 1);
-                nk += __shfl_xor_sync(FULL, nk, 2);
-                nk += __shfl_xor_sync(FULL, nk, 4);
+                if (hd == 64) {
+                    nk += __shfl_xor_sync(FULL, nk, 2);
+                    nk += __shfl_xor_sync(FULL, nk, 4);
+                }
                 norma = fmaxf(norma, nk);
             }
         }
         if (A.nrm && z < 2) {
             // the largest of the 128 tokens, rounded up by more than the error of 64 fp32 additions (it only bounds products)
-            const int n = __reduce_max_sync(FULL, __float2int_ru(norma * 1.00002f));
-            if ((tid & 31) == 0) red[tid >> 5] = n;
+            norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 8));
+            norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 16));
+            if (lane < 8) red[8 * wid + lane] = __float2int_ru(norma * 1.00002f);
             __syncthreads();
-            if (tid == 0) {
+            if (tid < 8 && ch == 0 && ha) {
                 int mx = 0;
-                for (int k = 0; k < 8; k++) mx = max(mx, red[k]);
+                for (int k = 0; k < 8; k++) mx = max(mx, red[8 * k + cg]);
                 A.nrm[((size_t)bh * 2 + z) * ((T + 127) / 128) + peca] = mx;
             }
         }
@@ -269,9 +282,10 @@ __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
             __syncthreads();
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const int linha = (tid >> 3) + 32 * q, c = tid & 7;
-                if ((linha & 63) < hd && t0 + 16 * c < T)
-                    *reinterpret_cast<uint4*>(dt + ((size_t)bh * 128 + linha) * T + t0 + 16 * c) = *reinterpret_cast<const uint4*>(tr + linha * 32 + 4 * (c ^ (linha >> 3 & 7)));
+                const int linha = (tid >> 3) + 32 * q, c = tid & 7, cv = linha & 63, hh = h0 + cv / hd;      // digit row, virtual column, its head
+                if (hh < A.H && t0 + 16 * c < T)
+                    *reinterpret_cast<uint4*>(dt + ((size_t)(b * A.H + hh) * 128 + (linha & 64) + cv % hd) * T + t0 + 16 * c) =
+                        *reinterpret_cast<const uint4*>(tr + linha * 32 + 4 * (c ^ (linha >> 3 & 7)));
             }
         }
         __syncthreads();                                           // red[] and tr[] go to the next piece
@@ -1048,7 +1062,7 @@ static bool atc_serve(int blk, int T, int H, int D, int GA) {
     return (D == H * 64 || D == H * 16) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 && (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
 }
 // pieces of 128 tokens per preparation block (each looks at the exponents of the whole sequence first): as many as leave 16 blocks per SM
-static int atc_por_cta(int T, int BH, int z) {
+static int atc_por_cta(int T, int BH, int z) {                      // BH: groups of 64 columns
     const int np = (T + 127) / 128;
     int por = 1;
     while (por < np && (long long)((np + 2 * por - 1) / (2 * por)) * BH * z >= 16 * N_SM) por *= 2;
@@ -1069,10 +1083,10 @@ static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* O
     int* nrm = em + 4 * BH;
     uint16_t *Qd = reinterpret_cast<uint16_t*>(ws + b_em), *K = reinterpret_cast<uint16_t*>(ws + b_em + 2 * b_lin);
     int8_t* Vt = reinterpret_cast<int8_t*>(ws + b_em + 3 * b_lin);
-    const int por = atc_por_cta(T, BH, 3);
+    const int grupos = Bt * ((H + 64 / hd - 1) / (64 / hd)), por = atc_por_cta(T, grupos, 3);
     atc::ArgsPrep Pp = {qm, qE, nullptr, nullptr, {nullptr, K, nullptr, nullptr}, {Qd, nullptr, nullptr, nullptr}, {nullptr, nullptr, Vt, nullptr},
-                        em, nullptr, nrm, BH, T, H, D, hd, GA, blk, por};
-    lanca_pdl(atc::k_at_prep, dim3(((T + 127) / 128 + por - 1) / por, BH, 3), dim3(256), 0, st, Pp);
+                        em, nullptr, nrm, BH, T, H, D, GA, blk, por};
+    lanca_pdl(hd == 64 ? atc::k_at_prep<64> : atc::k_at_prep<16>, dim3(((T + 127) / 128 + por - 1) / por, grupos, 3), dim3(256), 0, st, Pp);
     CUtensorMap mQ, mK, mVt;
     if (!(faz_mapa_h(&mQ, Qd, 2 * BH * T, 64, 32) && faz_mapa_h(&mK, K, BH * T, 64, 32) && faz_mapa(&mVt, Vt, BH * 128, T, 128)))
         return (int)cudaErrorInvalidValue;
@@ -1098,10 +1112,10 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
     auto parte = [&](int n) { return ws + b_est + n * b_lin; };
     uint16_t *V = (uint16_t*)parte(0), *Gd = (uint16_t*)parte(1);
     int8_t *Qt = (int8_t*)parte(3), *Kt = (int8_t*)parte(4), *Gt = (int8_t*)parte(5);
-    const int por = atc_por_cta(T, BH, 4);
+    const int grupos = Bt * ((H + 64 / hd - 1) / (64 / hd)), por = atc_por_cta(T, grupos, 4);
     atc::ArgsPrep Pp = {qm, qE, gom, goE, {nullptr, nullptr, V, nullptr}, {nullptr, nullptr, nullptr, Gd}, {Qt, Kt, nullptr, Gt},
-                        em, est, nullptr, BH, T, H, D, hd, GA, blk, por};
-    lanca_pdl(atc::k_at_prep, dim3(((T + 127) / 128 + por - 1) / por, BH, 4), dim3(256), 0, st, Pp);
+                        em, est, nullptr, BH, T, H, D, GA, blk, por};
+    lanca_pdl(hd == 64 ? atc::k_at_prep<64> : atc::k_at_prep<16>, dim3(((T + 127) / 128 + por - 1) / por, grupos, 4), dim3(256), 0, st, Pp);
     CUtensorMap mV, mV128, mGd, mKt, mQt, mGt, mP;
     if (!(faz_mapa_h(&mV, V, BH * T, 64, 32) && faz_mapa_h(&mV128, V, BH * T, 64, 128) && faz_mapa_h(&mGd, Gd, 2 * BH * T, 64, 32) &&
           faz_mapa(&mKt, Kt, BH * 128, T, 128) && faz_mapa(&mQt, Qt, BH * 128, T, 128) && faz_mapa(&mGt, Gt, BH * 128, T, 128) &&
