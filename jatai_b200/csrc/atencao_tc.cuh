@@ -138,7 +138,7 @@ __device__ __forceinline__ void grava8(int* acc, int16_t* ex, int8_t* qm, int8_t
 }
 
 // -------------------------------------------------------------------------------------------------- preparation
-// z = 0 q, 1 k, 2 v (columns of QKV), 3 dO.  Per tensor: the layouts wanted (nullptr = not).
+// z = 0 q, 1 k, 2 v (columns of QKV), 3 dO.  Per tensor: the layouts wanted (nullptr = not), of the combinations that k_at_prep lists.
 struct ArgsPrep {
     const int8_t* qm; const int8_t* qE; const int8_t* gm; const int8_t* gE;
     uint16_t* plano[4]; uint16_t* dig[4]; int8_t* tra[4];
@@ -160,15 +160,10 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
 // digits are hi = round(r / 64), lo = r - 64 hi); the transposed digits of 4 tokens are packed into a word and cross shared memory in
 // 16-byte pieces swapped by the column group, without bank conflicts.
 // 16 x 1024 tokens, forward + backward: 16 heads of 64 218 -> 181 us, 16 heads of 16 196 -> 63 us.
-template <int hd>
-__global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
-    __shared__ int red[8 * 8];
-    __shared__ __align__(16) uint32_t tr[128 * 32];
+template <int hd, bool PLANO, bool DIG, bool TRA, bool NRM>
+__device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint16_t* dg, int8_t* dt, int* red, uint32_t* tr) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, z = blockIdx.z, hpc = 64 / hd, gh = (A.H + hpc - 1) / hpc;
     const int b = blockIdx.y / gh, h0 = blockIdx.y % gh * hpc;     // first head of the group
-    uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
-    uint16_t* dg = z == 0 ? A.dig[0] : z == 1 ? A.dig[1] : z == 2 ? A.dig[2] : A.dig[3];
-    int8_t* dt = z == 0 ? A.tra[0] : z == 1 ? A.tra[1] : z == 2 ? A.tra[2] : A.tra[3];
     const int T = A.T, D = A.D, blk = A.blk, linha0 = b * T;
     const int8_t* m = z == 3 ? A.gm : A.qm;
     const int8_t* E = z == 3 ? A.gE : A.qE;
@@ -177,8 +172,6 @@ __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
     const int h = h0 + 8 * cg / hd, ch = 8 * cg % hd, bh = b * A.H + h;
     const bool ha = h < A.H;
     const size_t BHT = (size_t)A.BH * T;
-    pdl_espera();
-    pdl_solta();
     int em;
     {
         // maximum exponents of the two halves of 32 columns (a head of 16 lies in one of them, a head of 64 in both)
@@ -233,23 +226,23 @@ __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
                 const uint64_t r = ffma2(v, f, mag), rf = fadd2(r, menos_mag);
                 u[k][2 * c] = 2 * (uint32_t)r + (128u - 2 * MAGIA);
                 u[k][2 * c + 1] = 2 * (uint32_t)(r >> 32) + (128u - 2 * MAGIA);
-                if (dp) pl[c] = par_h(rf);
-                if (dg) {
+                if (PLANO) pl[c] = par_h(rf);
+                if (DIG) {
                     const uint64_t hi = fadd2(ffma2(rf, um64, mag), menos_mag);
                     dh[c] = par_h(hi);
                     dl[c] = par_h(ffma2(hi, m64, rf));
                 }
-                if (A.nrm) nk = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk));
+                if (NRM) nk = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk));
             }
             if (dentro && ha) {
                 const size_t o = ((size_t)bh * T + t0 + 4 * tg + k) * 64 + ch;
-                if (dp) *reinterpret_cast<uint4*>(dp + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-                if (dg) {
+                if (PLANO) *reinterpret_cast<uint4*>(dp + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+                if (DIG) {
                     *reinterpret_cast<uint4*>(dg + o) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
                     *reinterpret_cast<uint4*>(dg + BHT * 64 + o) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
                 }
             }
-            if (A.nrm && z < 2) {                                  // squared norm of a head's row: its 8 or 2 lanes are neighbours
+            if (NRM) {                                  // squared norm of a head's row: its 8 or 2 lanes are neighbours
                 nk += __shfl_xor_sync(FULL, nk, 1);
                 if (hd == 64) {
                     nk += __shfl_xor_sync(FULL, nk, 2);
@@ -258,7 +251,7 @@ __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
                 norma = fmaxf(norma, nk);
             }
         }
-        if (A.nrm && z < 2) {
+        if (NRM) {
             // the largest of the 128 tokens, rounded up by more than the error of 64 fp32 additions (it only bounds products)
             norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 8));
             norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 16));
@@ -270,7 +263,7 @@ __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
                 A.nrm[((size_t)bh * 2 + z) * ((T + 127) / 128) + peca] = mx;
             }
         }
-        if (dt) {
+        if (TRA) {
             if (ha)
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
@@ -289,6 +282,26 @@ __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
             }
         }
         __syncthreads();                                           // red[] and tr[] go to the next piece
+    }
+}
+template <int hd>
+__global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
+    __shared__ int red[8 * 8];
+    __shared__ __align__(16) uint32_t tr[128 * 32];
+    const int z = blockIdx.z;
+    uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
+    uint16_t* dg = z == 0 ? A.dig[0] : z == 1 ? A.dig[1] : z == 2 ? A.dig[2] : A.dig[3];
+    int8_t* dt = z == 0 ? A.tra[0] : z == 1 ? A.tra[1] : z == 2 ? A.tra[2] : A.tra[3];
+    pdl_espera();
+    pdl_solta();
+    if (A.nrm) {                                                   // forward: q digits, k plain, v transposed
+        if (dg) prep_corpo<hd, false, true, false, true>(A, dp, dg, dt, red, tr);
+        else if (dp) prep_corpo<hd, true, false, false, true>(A, dp, dg, dt, red, tr);
+        else prep_corpo<hd, false, false, true, false>(A, dp, dg, dt, red, tr);
+    } else {                                                       // backward: q, k transposed, v plain, dO digits and transposed
+        if (dg) prep_corpo<hd, false, true, true, false>(A, dp, dg, dt, red, tr);
+        else if (dp) prep_corpo<hd, true, false, false, false>(A, dp, dg, dt, red, tr);
+        else prep_corpo<hd, false, false, true, false>(A, dp, dg, dt, red, tr);
     }
 }
 
