@@ -29,7 +29,7 @@
 //
 // Every mbarrier wait is bounded (sentinel 7, abort flag, normal exit with tensor memory freed), as in the block GEMM.
 #pragma once
-#include <type_traits>
+#include <cooperative_groups.h>
 #include "comum.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_h.cuh"
@@ -145,7 +145,7 @@ struct ArgsPrep {
     int* em;                    // [BH][4] head-maximum exponents, indexed by z
     int* est;                   // backward: the statistics slots [BH][N_EST] to clear (nullptr in the forward)
     int* nrm;                   // forward: [BH][2][ceil(T/128)] largest sum of squares of an aligned row of q (0) / k (1) per 128 tokens
-    int BH, T, H, D, GA, blk, por_cta;           // por_cta: 128-token pieces of a CTA
+    int BH, T, H, D, GA, blk;
 };
 __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats that halves hold exactly
     uint32_t r;
@@ -153,13 +153,14 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
     return r;
 }
 
-// grid (CTAs per 64 columns, sequences x groups of 64 / hd heads, 3 or 4), 256 threads: `por_cta` pieces of 128 tokens of 64 columns - one
-// head of 64 or four of 16 - of one tensor.  The bound of a plain version (one element at a time in integers, digit bytes stored one by
+// grid (pieces of 128 tokens, sequences x groups of 64 / hd heads, 3 or 4), 256 threads: 128 tokens of 64 columns - one head of 64 or four
+// of 16 - of one tensor.  The pieces of a sequence are a cluster (at most 8), which exchanges the maximum exponents: reading a
+// sequence's exponents in every block was half of the traffic to the cache.  The bound of a plain version (one element at a time in integers, digit bytes stored one by
 // one) was instruction issue, three times the memory time.  So: a thread takes 4 tokens x 8 columns; pairs of elements in f32x2 (a byte
 // becomes a float by its place in 2^23's mantissa; v 2^(GA - s) rounds to even in one FMA against 1.5 * 2^23, exactly rnd_d; the 6-bit
 // digits are hi = round(r / 64), lo = r - 64 hi); the transposed digits of 4 tokens are packed into a word and cross shared memory in
 // 16-byte pieces swapped by the column group, without bank conflicts.
-// 16 x 1024 tokens, forward + backward: 16 heads of 64 218 -> 181 us, 16 heads of 16 196 -> 63 us.
+// 16 x 1024 tokens, forward + backward: 16 heads of 64 218 -> 175 us, 16 heads of 16 196 -> 57 us.
 template <int hd, bool PLANO, bool DIG, bool TRA, bool NRM>
 __device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint16_t* dg, int8_t* dt, int* red, uint32_t* tr) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, z = blockIdx.z, hpc = 64 / hd, gh = (A.H + hpc - 1) / hpc;
@@ -172,121 +173,126 @@ __device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint
     const int h = h0 + 8 * cg / hd, ch = 8 * cg % hd, bh = b * A.H + h;
     const bool ha = h < A.H;
     const size_t BHT = (size_t)A.BH * T;
-    int em;
-    {
-        // maximum exponents of the two halves of 32 columns (a head of 16 lies in one of them, a head of 64 in both)
-        const int8_t* pe = E + (size_t)linha0 * ldb;
-        const bool segunda = h0 * hd + 32 < D;
-        int e0 = -128, e1 = -128;
-        for (int t = tid; t < T; t += 256) {
-            e0 = max(e0, (int)pe[(size_t)t * ldb + col0 / blk]);
-            if (segunda) e1 = max(e1, (int)pe[(size_t)t * ldb + (col0 + 32) / blk]);
+    const int peca = blockIdx.x, t0 = peca * 128;
+    const bool dentro = t0 + 4 * tg < T;                           // (T is a multiple of 32)
+    uint2 w[4];
+    int ex[4], em;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const size_t lin = (size_t)(linha0 + t0 + 4 * tg + k);
+        w[k] = make_uint2(0, 0);
+        ex[k] = -128;
+        if (dentro && ha) {
+            w[k] = *reinterpret_cast<const uint2*>(m + lin * ld + col0 + 8 * cg);
+            ex[k] = E[lin * ldb + (col0 + 8 * cg) / blk];
         }
-        e0 = __reduce_max_sync(FULL, e0);
-        e1 = __reduce_max_sync(FULL, e1);
+    }
+    {
+        // maximum exponents of the two halves of 32 columns (a head of 16 lies in one of them, a head of 64 in both), over the sequence:
+        // the blocks of the cluster have the other tokens
+        const int meu = max(max(ex[0], ex[1]), max(ex[2], ex[3]));
+        int e0 = __reduce_max_sync(FULL, cg < 4 ? meu : -128), e1 = __reduce_max_sync(FULL, cg < 4 ? -128 : meu);
         if (lane == 0) { red[wid] = e0; red[8 + wid] = e1; }
         __syncthreads();
+        if (tid < 2) {
+            int e = red[8 * tid];
 #pragma unroll
-        for (int i = 0; i < 8; i++) { e0 = max(e0, red[i]); e1 = max(e1, red[8 + i]); }
-        if (hd == 64) e0 = e1 = max(e0, e1);
-        em = cg < 4 ? e0 : e1;
-        __syncthreads();                                           // red[] is used again below
+            for (int i = 1; i < 8; i++) e = max(e, red[8 * tid + i]);
+            red[16 + tid] = e;
+        }
+        const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        cl.sync();
+        if (tid < 32) {
+            const int* r = cl.map_shared_rank(red, lane < (int)gridDim.x ? lane : 0);
+            e0 = __reduce_max_sync(FULL, r[16]);
+            e1 = __reduce_max_sync(FULL, r[17]);
+            if (lane == 0) { red[18] = e0; red[19] = e1; }
+        }
+        __syncthreads();
+        // (nobody leaves before everyone has read: the second half of this barrier is at the end)
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+        e0 = red[18]; e1 = red[19];
+        em = hd == 64 ? max(e0, e1) : cg < 4 ? e0 : e1;
     }
     if (blockIdx.x == 0 && tid < 8 && ch == 0 && ha) A.em[bh * 4 + z] = em;
     if (A.est && blockIdx.x == 0 && z == 3 && tg < at::N_EST && ch == 0 && ha) A.est[bh * at::N_EST + tg] = 0;
     const uint64_t mag = par_f(MAGIA_F, MAGIA_F), menos_mag = par_f(-MAGIA_F, -MAGIA_F), vies = par_f(-8388736.0f, -8388736.0f);      // 2^23 + 128
     const uint64_t um64 = par_f(0.015625f, 0.015625f), m64 = par_f(-64.0f, -64.0f);
-    for (int p = 0; p < A.por_cta; p++) {
-        const int peca = blockIdx.x * A.por_cta + p, t0 = peca * 128;
-        if (t0 >= T) break;
-        float norma = 0.0f;
-        uint32_t u[4][8];                                          // 2 r + 128: hi digit in byte 1, 2 (lo + 64) in byte 0
-        const bool dentro = t0 + 4 * tg < T;                       // (T is a multiple of 32)
-        uint2 w[4];
-        int s[4];
+    float norma = 0.0f;
+    uint32_t u[4][8];                                          // 2 r + 128: hi digit in byte 1, 2 (lo + 64) in byte 0
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const size_t lin = (size_t)(linha0 + t0 + 4 * tg + k);
-            w[k] = make_uint2(0, 0);
-            s[k] = 0;
-            if (dentro && ha) {
-                w[k] = *reinterpret_cast<const uint2*>(m + lin * ld + col0 + 8 * cg);
-                s[k] = min(em - (int)E[lin * ldb + (col0 + 8 * cg) / blk], 40);      // |v 2^GA| < 2^11: 0 from a shift of 13 on
+    for (int k = 0; k < 4; k++) {
+        const float f1 = pot2(A.GA - min(em - ex[k], 40));     // |v 2^GA| < 2^11: 0 from a shift of 13 on
+        const uint64_t f = par_f(f1, f1);
+        uint32_t pl[4], dh[4], dl[4];
+        float nk = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {                          // two columns at a time
+            const uint32_t x = (c < 2 ? w[k].x : w[k].y) ^ 0x80808080u;
+            const uint64_t v = fadd2(par(__byte_perm(x, 0x4B000000u, 0x7540 + 2 * (c & 1)), __byte_perm(x, 0x4B000000u, 0x7540 + 2 * (c & 1) + 1)), vies);
+            const uint64_t r = ffma2(v, f, mag), rf = fadd2(r, menos_mag);
+            u[k][2 * c] = 2 * (uint32_t)r + (128u - 2 * MAGIA);
+            u[k][2 * c + 1] = 2 * (uint32_t)(r >> 32) + (128u - 2 * MAGIA);
+            if (PLANO) pl[c] = par_h(rf);
+            if (DIG) {
+                const uint64_t hi = fadd2(ffma2(rf, um64, mag), menos_mag);
+                dh[c] = par_h(hi);
+                dl[c] = par_h(ffma2(hi, m64, rf));
+            }
+            if (NRM) nk = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk));
+        }
+        if (dentro && ha) {
+            const size_t o = ((size_t)bh * T + t0 + 4 * tg + k) * 64 + ch;
+            if (PLANO) *reinterpret_cast<uint4*>(dp + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+            if (DIG) {
+                *reinterpret_cast<uint4*>(dg + o) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
+                *reinterpret_cast<uint4*>(dg + BHT * 64 + o) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
             }
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const uint64_t f = par_f(pot2(A.GA - s[k]), pot2(A.GA - s[k]));
-            uint32_t pl[4], dh[4], dl[4];
-            float nk = 0.0f;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {                          // two columns at a time
-                const uint32_t x = (c < 2 ? w[k].x : w[k].y) ^ 0x80808080u;
-                const uint64_t v = fadd2(par(__byte_perm(x, 0x4B000000u, 0x7540 + 2 * (c & 1)), __byte_perm(x, 0x4B000000u, 0x7540 + 2 * (c & 1) + 1)), vies);
-                const uint64_t r = ffma2(v, f, mag), rf = fadd2(r, menos_mag);
-                u[k][2 * c] = 2 * (uint32_t)r + (128u - 2 * MAGIA);
-                u[k][2 * c + 1] = 2 * (uint32_t)(r >> 32) + (128u - 2 * MAGIA);
-                if (PLANO) pl[c] = par_h(rf);
-                if (DIG) {
-                    const uint64_t hi = fadd2(ffma2(rf, um64, mag), menos_mag);
-                    dh[c] = par_h(hi);
-                    dl[c] = par_h(ffma2(hi, m64, rf));
-                }
-                if (NRM) nk = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk));
+        if (NRM) {                                  // squared norm of a head's row: its 8 or 2 lanes are neighbours
+            nk += __shfl_xor_sync(FULL, nk, 1);
+            if (hd == 64) {
+                nk += __shfl_xor_sync(FULL, nk, 2);
+                nk += __shfl_xor_sync(FULL, nk, 4);
             }
-            if (dentro && ha) {
-                const size_t o = ((size_t)bh * T + t0 + 4 * tg + k) * 64 + ch;
-                if (PLANO) *reinterpret_cast<uint4*>(dp + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-                if (DIG) {
-                    *reinterpret_cast<uint4*>(dg + o) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
-                    *reinterpret_cast<uint4*>(dg + BHT * 64 + o) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
-                }
-            }
-            if (NRM) {                                  // squared norm of a head's row: its 8 or 2 lanes are neighbours
-                nk += __shfl_xor_sync(FULL, nk, 1);
-                if (hd == 64) {
-                    nk += __shfl_xor_sync(FULL, nk, 2);
-                    nk += __shfl_xor_sync(FULL, nk, 4);
-                }
-                norma = fmaxf(norma, nk);
-            }
+            norma = fmaxf(norma, nk);
         }
-        if (NRM) {
-            // the largest of the 128 tokens, rounded up by more than the error of 64 fp32 additions (it only bounds products)
-            norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 8));
-            norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 16));
-            if (lane < 8) red[8 * wid + lane] = __float2int_ru(norma * 1.00002f);
-            __syncthreads();
-            if (tid < 8 && ch == 0 && ha) {
-                int mx = 0;
-                for (int k = 0; k < 8; k++) mx = max(mx, red[8 * k + cg]);
-                A.nrm[((size_t)bh * 2 + z) * ((T + 127) / 128) + peca] = mx;
-            }
-        }
-        if (TRA) {
-            if (ha)
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const uint32_t lo = __byte_perm(__byte_perm(u[0][c], u[1][c], 0x0040), __byte_perm(u[2][c], u[3][c], 0x0040), 0x5410) >> 1 ^ 0x40404040u;
-                    const int q = (8 * cg + c) * 32 + (tg ^ 4 * cg);
-                    tr[q] = __byte_perm(__byte_perm(u[0][c], u[1][c], 0x0051), __byte_perm(u[2][c], u[3][c], 0x0051), 0x5410);
-                    tr[64 * 32 + q] = lo | (lo & 0x40404040u) << 1;      // 7 bits to a signed byte
-                }
-            __syncthreads();
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int linha = (tid >> 3) + 32 * q, c = tid & 7, cv = linha & 63, hh = h0 + cv / hd;      // digit row, virtual column, its head
-                if (hh < A.H && t0 + 16 * c < T)
-                    *reinterpret_cast<uint4*>(dt + ((size_t)(b * A.H + hh) * 128 + (linha & 64) + cv % hd) * T + t0 + 16 * c) =
-                        *reinterpret_cast<const uint4*>(tr + linha * 32 + 4 * (c ^ (linha >> 3 & 7)));
-            }
-        }
-        __syncthreads();                                           // red[] and tr[] go to the next piece
     }
+    if (NRM) {
+        // the largest of the 128 tokens, rounded up by more than the error of 64 fp32 additions (it only bounds products)
+        norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 8));
+        norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 16));
+        if (lane < 8) red[32 + 8 * wid + lane] = __float2int_ru(norma * 1.00002f);
+        __syncthreads();
+        if (tid < 8 && ch == 0 && ha) {
+            int mx = 0;
+            for (int k = 0; k < 8; k++) mx = max(mx, red[32 + 8 * k + cg]);
+            A.nrm[((size_t)bh * 2 + z) * ((T + 127) / 128) + peca] = mx;
+        }
+    }
+    if (TRA) {
+        if (ha)
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const uint32_t lo = __byte_perm(__byte_perm(u[0][c], u[1][c], 0x0040), __byte_perm(u[2][c], u[3][c], 0x0040), 0x5410) >> 1 ^ 0x40404040u;
+                const int q = (8 * cg + c) * 32 + (tg ^ 4 * cg);
+                tr[q] = __byte_perm(__byte_perm(u[0][c], u[1][c], 0x0051), __byte_perm(u[2][c], u[3][c], 0x0051), 0x5410);
+                tr[64 * 32 + q] = lo | (lo & 0x40404040u) << 1;      // 7 bits to a signed byte
+            }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int linha = (tid >> 3) + 32 * q, c = tid & 7, cv = linha & 63, hh = h0 + cv / hd;      // digit row, virtual column, its head
+            if (hh < A.H && t0 + 16 * c < T)
+                *reinterpret_cast<uint4*>(dt + ((size_t)(b * A.H + hh) * 128 + (linha & 64) + cv % hd) * T + t0 + 16 * c) =
+                    *reinterpret_cast<const uint4*>(tr + linha * 32 + 4 * (c ^ (linha >> 3 & 7)));
+        }
+    }
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 template <int hd>
 __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
-    __shared__ int red[8 * 8];
+    __shared__ int red[32 + 8 * 8];
     __shared__ __align__(16) uint32_t tr[128 * 32];
     const int z = blockIdx.z;
     uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
@@ -1074,12 +1080,9 @@ static size_t atc_arredonda(size_t x) { return (x + 1023) & ~(size_t)1023; }
 static bool atc_serve(int blk, int T, int H, int D, int GA) {
     return (D == H * 64 || D == H * 16) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 && (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
 }
-// pieces of 128 tokens per preparation block (each looks at the exponents of the whole sequence first): as many as leave 16 blocks per SM
-static int atc_por_cta(int T, int BH, int z) {                      // BH: groups of 64 columns
-    const int np = (T + 127) / 128;
-    int por = 1;
-    while (por < np && (long long)((np + 2 * por - 1) / (2 * por)) * BH * z >= 16 * N_SM) por *= 2;
-    return por;
+static void atc_prep(const atc::ArgsPrep& A, int Bt, int hd, int z, cudaStream_t st) {
+    const int np = (A.T + 127) / 128, hpc = 64 / hd;
+    lanca_cluster(hd == 64 ? atc::k_at_prep<64> : atc::k_at_prep<16>, dim3(np, Bt * ((A.H + hpc - 1) / hpc), z), dim3(256), 0, st, np, A);
 }
 
 // forward: preparation (q digits, k plain, v transposed), then the kernel
@@ -1096,10 +1099,9 @@ static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* O
     int* nrm = em + 4 * BH;
     uint16_t *Qd = reinterpret_cast<uint16_t*>(ws + b_em), *K = reinterpret_cast<uint16_t*>(ws + b_em + 2 * b_lin);
     int8_t* Vt = reinterpret_cast<int8_t*>(ws + b_em + 3 * b_lin);
-    const int grupos = Bt * ((H + 64 / hd - 1) / (64 / hd)), por = atc_por_cta(T, grupos, 3);
     atc::ArgsPrep Pp = {qm, qE, nullptr, nullptr, {nullptr, K, nullptr, nullptr}, {Qd, nullptr, nullptr, nullptr}, {nullptr, nullptr, Vt, nullptr},
-                        em, nullptr, nrm, BH, T, H, D, GA, blk, por};
-    lanca_pdl(hd == 64 ? atc::k_at_prep<64> : atc::k_at_prep<16>, dim3(((T + 127) / 128 + por - 1) / por, grupos, 3), dim3(256), 0, st, Pp);
+                        em, nullptr, nrm, BH, T, H, D, GA, blk};
+    atc_prep(Pp, Bt, hd, 3, st);
     CUtensorMap mQ, mK, mVt;
     if (!(faz_mapa_h(&mQ, Qd, 2 * BH * T, 64, 32) && faz_mapa_h(&mK, K, BH * T, 64, 32) && faz_mapa(&mVt, Vt, BH * 128, T, 128)))
         return (int)cudaErrorInvalidValue;
@@ -1125,10 +1127,9 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
     auto parte = [&](int n) { return ws + b_est + n * b_lin; };
     uint16_t *V = (uint16_t*)parte(0), *Gd = (uint16_t*)parte(1);
     int8_t *Qt = (int8_t*)parte(3), *Kt = (int8_t*)parte(4), *Gt = (int8_t*)parte(5);
-    const int grupos = Bt * ((H + 64 / hd - 1) / (64 / hd)), por = atc_por_cta(T, grupos, 4);
     atc::ArgsPrep Pp = {qm, qE, gom, goE, {nullptr, nullptr, V, nullptr}, {nullptr, nullptr, nullptr, Gd}, {Qt, Kt, nullptr, Gt},
-                        em, est, nullptr, BH, T, H, D, GA, blk, por};
-    lanca_pdl(hd == 64 ? atc::k_at_prep<64> : atc::k_at_prep<16>, dim3(((T + 127) / 128 + por - 1) / por, grupos, 4), dim3(256), 0, st, Pp);
+                        em, est, nullptr, BH, T, H, D, GA, blk};
+    atc_prep(Pp, Bt, hd, 4, st);
     CUtensorMap mV, mV128, mGd, mKt, mQt, mGt, mP;
     if (!(faz_mapa_h(&mV, V, BH * T, 64, 32) && faz_mapa_h(&mV128, V, BH * T, 64, 128) && faz_mapa_h(&mGd, Gd, 2 * BH * T, 64, 32) &&
           faz_mapa(&mKt, Kt, BH * 128, T, 128) && faz_mapa(&mQt, Qt, BH * 128, T, 128) && faz_mapa(&mGt, Gt, BH * 128, T, 128) &&

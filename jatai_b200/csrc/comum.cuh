@@ -66,6 +66,20 @@ static inline void lanca_pdl(void (*k)(KP...), dim3 grade, dim3 bloco, size_t sm
     (void)cudaLaunchKernelEx(&c, k, a...);                         // errors surface through cudaGetLastError like those of <<< >>>
 }
 
+// the same with clusters of `cl` blocks along x
+template <typename... KP, typename... A>
+static inline void lanca_cluster(void (*k)(KP...), dim3 grade, dim3 bloco, size_t smem, cudaStream_t st, int cl, A... a) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grade; c.blockDim = bloco; c.dynamicSmemBytes = smem; c.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cl; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at; c.numAttrs = pdl_ligado() ? 2 : 1;
+    (void)cudaLaunchKernelEx(&c, k, a...);
+}
+
 // ---------------------------------------------------------------------------------------- fp32 pairs
 constexpr uint32_t MAGIA = 0x4B400000u;                        // bit pattern of 1.5 * 2^23
 constexpr float MAGIA_F = 12582912.0f;
