@@ -58,10 +58,12 @@ class Modelo:
         self.estatisticas = False
         # second stream for the weight-gradient GEMMs (single GPU, CUDA launcher only)
         usa_lado = hasattr(ops, "lib") and torch.device(dev).type == "cuda"
-        self._lado = torch.cuda.Stream(device=dev) if usa_lado else None
-        self._pendente, self._feitos, self._k_lr_lado = None, set(), None
-        self._ev = (torch.cuda.Event(), torch.cuda.Event()) if usa_lado else None         # main -> side and side -> main, used again and again
-        self._ramo, self._presos = None, []          # the second stream in this step (or None), and what it reads until the streams join
+        # Side streams.  The chains of the weight gradients (transposition, product, optimiser step) are independent of each other and
+        # each is a row of small kernels, so they go round several streams; what else runs beside the main stream takes the first.
+        self._lados = [torch.cuda.Stream(device=dev) for _ in range(self.N_LADOS)] if usa_lado else []
+        self._pendente, self._vez, self._feitos, self._k_lr_lado = [None] * self.N_LADOS, 0, set(), None
+        self._ev = [torch.cuda.Event() for _ in range(1 + self.N_LADOS)] if usa_lado else None         # main -> side and sides -> main, used again and again
+        self._ramo, self._presos = None, []          # the side streams in this step (or None), and what they read until the streams join
         na_gpu = redutor is not None and hasattr(ops, "lib") and torch.device(dev).type == "cuda"
         self._ramos = [torch.cuda.Stream(device=dev) for _ in range(3)] if na_gpu else []
 
@@ -129,47 +131,61 @@ class Modelo:
             else:
                 self._adiados.append((nome, *self._transpoe_par_max(gy, x)))
             return
-        # A weight gradient is a leaf of the backward graph: its two transpositions and its GEMM run on a second
+        # A weight gradient is a leaf of the backward graph: its two transpositions and its GEMM run on a side
         # stream, next to the dX chain, and fill SMs the small GEMMs of that chain leave idle.  Under capture the
-        # second stream becomes a parallel branch of the CUDA graph.
-        with self._no_lado(gy, x):
-            self._otimiza_pendente()
-            if self.redutor is None:
-                a, b = self._transpoe_par(gy, x)
-                self._grads[nome] = ops.gemm(a, b, cru=True)
-                self._pendente = nome
-            else:       # data parallel: only the transpositions and the row maxima now, the GEMM after the exchange
+        # side streams become parallel branches of the CUDA graph.
+        if self.redutor is not None:       # data parallel: only the transpositions and the row maxima now, the GEMM after the exchange
+            with self._no_lado(gy, x):
                 self._adiados.append((nome, *self._transpoe_par_max(gy, x)))
+            return
+        f = self._vez
+        self._vez = (f + 1) % len(self._ramo)
+        with self._no_lado(gy, x, faixa=f):
+            self._otimiza_pendente(f)
+            a, b = self._transpoe_par(gy, x)
+            self._grads[nome] = ops.gemm(a, b, cru=True)
+            self._pendente[f] = nome
 
     @contextlib.contextmanager
-    def _no_lado(self, *lidos):
-        """The launches of the block go to the second stream, ordered after everything queued on the main one so far.  `lidos` (what they
+    def _no_lado(self, *lidos, faixa=0):
+        """The launches of the block go to a side stream, ordered after everything queued on the main one so far.  `lidos` (what they
         read of the main stream's tensors) stays referenced until the streams join: cheaper than telling the allocator of
         every tensor's second stream."""
         self._presos.append(lidos)
         principal = torch.cuda.current_stream()
         self._ev[0].record(principal)
-        self._ramo.wait_event(self._ev[0])
-        with torch.cuda.stream(self._ramo):
-            self.ops.lib.jt_stream(self._ramo.cuda_stream)
+        ramo = self._ramo[faixa]
+        self._usadas.add(faixa)
+        ramo.wait_event(self._ev[0])
+        with torch.cuda.stream(ramo):
+            self.ops.lib.jt_stream(ramo.cuda_stream)
             try:
                 yield
             finally:
                 self.ops.lib.jt_stream(principal.cuda_stream)
 
     def _junta_lado(self):
-        """The main stream waits for the second one."""
-        self._ev[1].record(self._ramo)
-        torch.cuda.current_stream().wait_event(self._ev[1])
+        """The main stream waits for the side streams that have had work since they last joined."""
+        principal = torch.cuda.current_stream()
+        for f in sorted(self._usadas):
+            self._ev[1 + f].record(self._ramo[f])
+            principal.wait_event(self._ev[1 + f])
+        self._usadas.clear()
 
     # Tokens x columns from which a step that is not being recorded uses the second stream: below it a step is bound by its launches,
     # which another stream only adds to (512 tokens x 256 columns: 2.6 ms of launches, 1.8 ms of kernels).
     RAMO_MINIMO = 1 << 19
+    # Side streams, and tokens x columns from which a step uses all of them: below, a chain is a few microseconds long and what another
+    # branch costs at its ends eats what it gives (128 tokens x 128 columns: 1 stream 264 us, 3 streams 273; 2048 x 256: 2.87 and 2.55 ms;
+    # 2048 x 512: 3.65 and 3.36 ms; a fourth gives nothing).
+    N_LADOS, VARIOS_MINIMO = 3, 1 << 17
 
     def _usa_ramo(self, tokens):
-        if self._lado is None:
+        if not self._lados:
             return None
-        return self._lado if tokens * self.D >= self.RAMO_MINIMO or torch.cuda.is_current_stream_capturing() else None
+        if tokens * self.D < self.RAMO_MINIMO and not torch.cuda.is_current_stream_capturing():
+            return None
+        return self._lados if tokens * self.D >= self.VARIOS_MINIMO else self._lados[:1]
 
     def _pesos_transpostos(self):
         """The backward multiplies by every weight transposed (and re-quantised along the new rows).  The weights do not change
@@ -183,18 +199,18 @@ class Modelo:
         self._presos.append(wt)                        # the main stream reads them; they go back only after it has joined
         return wt
 
-    def _otimiza_pendente(self):
-        """Single GPU, on the second stream: the optimiser step of the weight whose gradient was computed by the
-        previous call.  Safe because the second stream has just waited for the main stream, and by then the main
+    def _otimiza_pendente(self, f):
+        """Single GPU, on side stream f: the optimiser step of the weight whose gradient was computed there by the
+        previous call.  Safe because that stream has just waited for the main stream, and by then the main
         stream has queued its last read of that weight in this step (each weight is read once in the forward and
         once, transposed, in the backward, right after its own `_grad_peso` call)."""
-        n = self._pendente
+        n = self._pendente[f]
         if n is None or self._k_lr_lado is None:
             return
         with self.reg.trecho("otimizador"), self.reg.trecho(n):
             self._otimiza({n: self._grads[n]}, self._k_lr_lado)
         self._feitos.add(n)
-        self._pendente = None
+        self._pendente[f] = None
 
     def _gemms_adiados(self, maximos, inicio=0, fim=None):
         """Data parallel, after the MAX collective: the weight-gradient GEMMs [inicio, fim) of the deferred list (all of
@@ -277,7 +293,7 @@ class Modelo:
         tok = tok.reshape(-1).to(torch.int32).contiguous()
         alvo = alvo.reshape(-1).to(torch.int32).contiguous()
         self._grads, self._adiados = {}, []
-        self._pendente, self._feitos = None, set()
+        self._pendente, self._vez, self._feitos, self._usadas = [None] * self.N_LADOS, 0, set(), set()
         self._ramo, self._presos = self._usa_ramo(tok.numel()), []
         self._k_lr_lado = k_lr if (self.redutor is None and self._ramo is not None) else None
         inicio = getattr(self.redutor, "inicio_passo", None) if treina else None
@@ -347,9 +363,10 @@ class Modelo:
             with reg.trecho("embedding"):
                 self._grad_peso("emb", ops.um_quente(tok, self.V), gx)
         if self._ramo is not None:
-            if self._pendente is not None and self._k_lr_lado is not None:
-                with self._no_lado():
-                    self._otimiza_pendente()
+            for f, n in enumerate(self._pendente):
+                if n is not None and self._k_lr_lado is not None:
+                    with self._no_lado(faixa=f):
+                        self._otimiza_pendente(f)
             self._junta_lado()                                     # join the weight-gradient branch
         self._presos = []
 
