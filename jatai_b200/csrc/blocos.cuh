@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) k_quant(const int* __restrict__ acc, cons
 
 // One 16-element chunk of z = x + y (see k_soma below for the arithmetic); the GL lanes of a block call together.
 // Returns the block exponent, `pac` receives the 16 mantissas.
-template <int GL>
+template <int GL, int ST = 1>
 __device__ __forceinline__ int soma16(const int (&xv)[16], int ex, const int (&yv)[16], int ey, uint4& pac, int kid, long long o) {
     const bool x_maior = ex >= ey;
     const int eH = x_maior ? ex : ey, d = x_maior ? ex - ey : ey - ex;
@@ -95,7 +95,7 @@ __device__ __forceinline__ int soma16(const int (&xv)[16], int ex, const int (&y
         wv[i] = (hi[i] << dl) + rnd_d(lo[i], s2);
         mx = max(mx, wv[i] < 0 ? -wv[i] : wv[i]);
     }
-    mx = grupo_max<GL>(mx);
+    mx = grupo_max<GL, ST>(mx);
     int s = bitlen(mx) - 7;
     if (desloca(mx, s) > 127) s += 1;
     const int E = eH - dl + s;
@@ -122,7 +122,7 @@ __device__ __forceinline__ int soma16(const int (&xv)[16], int ex, const int (&y
 }
 
 // One lane's 16 elements of the sum of two block tensors, in fp32 where the exponents are at most 16 apart (k_soma has the reasons)
-template <int GL>
+template <int GL, int ST = 1>
 __device__ __forceinline__ int soma16_misto(const uint4& rx, int ex, const uint4& ry, int ey, uint4& pac, int kid, long long o) {
     const bool x_maior = ex >= ey;
     const int eH = x_maior ? ex : ey, eL = x_maior ? ey : ex;
@@ -135,12 +135,12 @@ __device__ __forceinline__ int soma16_misto(const uint4& rx, int ex, const uint4
         const float a = x_maior ? __int_as_float((127 + d) << 23) : 1.f, b = x_maior ? 1.f : __int_as_float((127 + d) << 23);
 #pragma unroll
         for (int i = 0; i < 16; i++) fx[i] = fmaf(fx[i], a, fy[i] * b);
-        return quant_f32<GL>(fx, eH - d, pac, kid, o);
+        return quant_f32<GL, ST>(fx, eH - d, pac, kid, o);
     }
     int xv[16], yv[16];
     desempacota16(rx, xv);
     desempacota16(ry, yv);
-    return soma16<GL>(xv, ex, yv, ey, pac, kid, o);
+    return soma16<GL, ST>(xv, ex, yv, ey, pac, kid, o);
 }
 
 // z = x + y.  ops.py:128-132: ec = max(xE, yE) - 21; v = rnd(x, ec - xE) + rnd(y, ec - yE); quant(v, ec).

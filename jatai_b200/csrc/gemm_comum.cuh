@@ -43,6 +43,13 @@ __device__ __forceinline__ void epilogo_tile(const int* acc_s, const int* RAs, c
         const int r = g4 * RPW + (lane & (RPW - 1)), ch = lane / RPW;
         const int gi = m0 + r, gj = n0 + ch * 16;
         const long long o = (long long)gi * N + gj;
+        const long long oe = (long long)gi * (N / BLK) + gj / BLK;
+        uint4 X = make_uint4(0, 0, 0, 0);          // on its way while the accumulators are quantised
+        int eX = 0;
+        if (MODO == 2 || MODO == 4) {
+            X = *reinterpret_cast<const uint4*>(S.Xm + o);
+            eX = S.XE[oe];
+        }
         int v[16];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -71,7 +78,6 @@ __device__ __forceinline__ void epilogo_tile(const int* acc_s, const int* RAs, c
             continue;
         }
         const bool lider = (ch % GL) == 0;
-        const long long oe = (long long)gi * (N / BLK) + gj / BLK;
         int q[16], E;
         bool rapido = false;
         if (RBf) {
@@ -107,15 +113,20 @@ __device__ __forceinline__ void epilogo_tile(const int* acc_s, const int* RAs, c
                 if (MODO == 4) {                   // relu2_back (ops.py:139-141): |g h 2| <= 32258
                     float h[16];
                     bytes_para_float(pac, f);
-                    bytes_para_float(*reinterpret_cast<const uint4*>(S.Xm + o), h);
+                    bytes_para_float(X, h);
 #pragma unroll
                     for (int k = 0; k < 16; k++) f[k] = f[k] * fmaxf(h[k], 0.f) * 2.f;
-                    const int E2 = quant_f32<GL, RPW>(f, E + (int)S.XE[oe], pac, kid, o);
+                    const int E2 = quant_f32<GL, RPW>(f, E + eX, pac, kid, o);
                     *reinterpret_cast<uint4*>(S.Cm + o) = pac;
                     if (lider) S.CE[oe] = (int8_t)E2;
                     continue;
                 }
-                desempacota16(pac, q);             // MODO 2 goes on in integers: its sums reach 2^28
+                if (MODO == 2) {                   // soma(X, gemm): ops.py:128-132
+                    E = soma16_misto<GL, RPW>(X, eX, pac, (int)(int8_t)E, pac, kid, o);
+                    *reinterpret_cast<uint4*>(S.Cm + o) = pac;
+                    if (lider) S.CE[oe] = (int8_t)E;
+                    continue;
+                }
             }
         }
         if (!rapido) {
@@ -129,10 +140,10 @@ __device__ __forceinline__ void epilogo_tile(const int* acc_s, const int* RAs, c
             if (lider) S.CE[oe] = (int8_t)E;
         } else if (MODO == 2) {            // soma(X, gemm): ops.py:128-132
             int x[16], z[16];
-            le16(S.Xm + o, x);
-            const int ex = S.XE[oe], ec = max(ex, E) - 21;
+            desempacota16(X, x);
+            const int ec = max(eX, E) - 21;
 #pragma unroll
-            for (int k = 0; k < 16; k++) x[k] = desloca(x[k], ec - ex) + desloca(q[k], ec - E);
+            for (int k = 0; k < 16; k++) x[k] = desloca(x[k], ec - eX) + desloca(q[k], ec - E);
             const int E2 = quant_uniforme<16, GL, RPW>(x, ec, z, kid, o);
             grava16(S.Cm + o, z);
             if (lider) S.CE[oe] = (int8_t)E2;
@@ -147,11 +158,10 @@ __device__ __forceinline__ void epilogo_tile(const int* acc_s, const int* RAs, c
             if (lider) S.OE2[oe] = (int8_t)E2;
         } else {                            // relu2_back(gemm, h): ops.py:139-141
             int h[16], z[16];
-            le16(S.Xm + o, h);
-            const int eh = S.XE[oe];
+            desempacota16(X, h);
 #pragma unroll
             for (int k = 0; k < 16; k++) h[k] = q[k] * max(h[k], 0) * 2;
-            const int E2 = quant_uniforme<16, GL, RPW>(h, E + eh, z, kid, o);
+            const int E2 = quant_uniforme<16, GL, RPW>(h, E + eX, z, kid, o);
             grava16(S.Cm + o, z);
             if (lider) S.CE[oe] = (int8_t)E2;
         }
