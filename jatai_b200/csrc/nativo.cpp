@@ -3,6 +3,7 @@
 // argument is found and told by the Python checks of registro.py: these functions only say that something is.
 #include <Python.h>
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -50,7 +51,7 @@ PyObject* cru(PyObject*, PyObject* par) {
     return r;
 }
 
-at::Tensor vazio(at::IntArrayRef forma, at::ScalarType tipo, const at::Device& dev) { return at::empty(forma, at::TensorOptions().dtype(tipo).device(dev)); }
+at::Tensor vazio(at::IntArrayRef forma, at::ScalarType tipo, const at::Device& dev) { return at::detail::empty_cuda(forma, tipo, dev, c10::nullopt); }      // at::empty without the dispatcher
 
 PyObject* par_de(at::Tensor a, at::Tensor b) {
     PyObject* r = PyTuple_New(2);
@@ -143,7 +144,21 @@ int chama(void* f, const A_* a, int n) {
     return -1;
 }
 
-PyObject *S_op, *S_trecho, *S_entradas, *S_forma;
+PyObject *S_op, *S_trecho, *S_entradas, *S_forma, *S_A[2], *S_B[2], *S_X[2];
+
+// The launch record {op, trecho, entradas, forma} appended to `lista`; its index, or -1 with a Python error set.
+Py_ssize_t anota(PyObject* lista, PyObject* op, PyObject* trecho, PyObject* entradas, PyObject* forma) {
+    PyObject* d = PyDict_New();
+    if (!d) return -1;
+    PyDict_SetItem(d, S_op, op);
+    PyDict_SetItem(d, S_trecho, trecho);
+    PyDict_SetItem(d, S_entradas, entradas);
+    PyDict_SetItem(d, S_forma, forma);
+    const Py_ssize_t kid = PyList_GET_SIZE(lista);
+    const int falhou = PyList_Append(lista, d);
+    Py_DECREF(d);
+    return falhou ? -1 : kid;
+}
 
 // lanca(function address, launch list, op, section, names, tensors, ints, output shape) -> (launch id, return code)
 // Records the launch ({op, trecho, entradas, forma}; `names` name the first tensors, None skips one) and calls function(pointers..., ints...,
@@ -168,23 +183,78 @@ PyObject* lanca(PyObject*, PyObject* const* args, Py_ssize_t n) {
     void* f = PyLong_AsVoidPtr(args[0]);
     if (PyErr_Occurred()) return nullptr;
     if (!f) { PyErr_SetString(PyExc_ValueError, "null function"); return nullptr; }
-    PyObject *ent = PyDict_New(), *d = PyDict_New();
-    if (!ent || !d) { Py_XDECREF(ent); Py_XDECREF(d); return nullptr; }
+    PyObject* ent = PyDict_New();
+    if (!ent) return nullptr;
     for (Py_ssize_t i = 0; i < nn; i++)
         if (PyTuple_GET_ITEM(nomes, i) != Py_None) PyDict_SetItem(ent, PyTuple_GET_ITEM(nomes, i), PyTuple_GET_ITEM(ts, i));
-    PyDict_SetItem(d, S_op, args[2]);
-    PyDict_SetItem(d, S_trecho, args[3]);
-    PyDict_SetItem(d, S_entradas, ent);
-    PyDict_SetItem(d, S_forma, args[7]);
+    const Py_ssize_t kid = anota(lista, args[2], args[3], ent, args[7]);
     Py_DECREF(ent);
-    const Py_ssize_t kid = PyList_GET_SIZE(lista);
-    const int falhou = PyList_Append(lista, d);
-    Py_DECREF(d);
-    if (falhou) return nullptr;
+    if (kid < 0) return nullptr;
     a[np + ni] = (A_)kid;
     const int rc = chama(f, a, (int)(np + ni + 1));
     if (rc == 0) Py_RETURN_NONE;
     return Py_BuildValue("(ni)", kid, rc);
+}
+
+// gemm(address of jt_gemm_ws_bytes, of jt_stream_atual, of jt_gemm_ws, of jt_gemm_ext, blk, launch list, op, section, mode, A, B, X or None, two
+// outputs) -> the output (pair), or both; None where an argument is not as it should be (nothing was done), the return code where the launch
+// failed.  The whole of a product in one call: checks, outputs, workspace, record, launch.
+PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 13 || !PyList_Check(args[5])) { PyErr_SetString(PyExc_TypeError, "gemm(4 functions, blk, launches, op, section, mode, A, B, X, two)"); return nullptr; }
+    void *fb = PyLong_AsVoidPtr(args[0]), *fs = PyLong_AsVoidPtr(args[1]), *fw = PyLong_AsVoidPtr(args[2]), *fe = PyLong_AsVoidPtr(args[3]);
+    const int64_t blk = PyLong_AsLongLong(args[4]);
+    const int modo = (int)PyLong_AsLong(args[8]), duas = PyObject_IsTrue(args[12]);
+    if (PyErr_Occurred()) return nullptr;
+    int64_t M, K, N, Kb, Mx, Nx;
+    if (!fb || !fs || !fw || !fe || blk <= 0 || !bloco_valido(args[9], blk, &M, &K) || !bloco_valido(args[10], blk, &N, &Kb)) Py_RETURN_NONE;
+    const bool tem_x = args[11] != Py_None;
+    if (Kb != K || M % 64 || N % 128 || K % blk || (tem_x && (!bloco_valido(args[11], blk, &Mx, &Nx) || Mx != M || Nx != N))) Py_RETURN_NONE;
+    try {
+        const at::Tensor& a = *tensor(PyTuple_GET_ITEM(args[9], 0));
+        const at::Device dev = a.device();
+        A_ p[20] = {0};
+        auto poe = [&](int i, PyObject* par) { for (int k = 0; k < 2; k++) p[i + k] = (A_)tensor(PyTuple_GET_ITEM(par, k))->data_ptr(); };
+        poe(0, args[9]);
+        poe(2, args[10]);
+        at::Tensor m1, e1, m2, e2, ws;
+        if (modo == 1) { m1 = vazio({M, N}, at::kInt, dev); e1 = vazio({M, N}, at::kShort, dev); }
+        else { m1 = vazio({M, N}, at::kChar, dev); e1 = vazio({M, N / blk}, at::kChar, dev); }
+        p[modo == 1 ? 6 : 4] = (A_)m1.data_ptr();
+        p[modo == 1 ? 7 : 5] = (A_)e1.data_ptr();
+        if (tem_x) poe(8, args[11]);
+        if (duas) {
+            m2 = vazio({M, N}, at::kChar, dev); e2 = vazio({M, N / blk}, at::kChar, dev);
+            p[10] = (A_)m2.data_ptr(); p[11] = (A_)e2.data_ptr();
+        }
+        long long bytes = 0;
+        if (reinterpret_cast<void* (*)()>(fs)() == (void*)c10::cuda::getCurrentCUDAStream(dev.index()).stream())
+            bytes = reinterpret_cast<long long (*)(int, int, int, int)>(fb)((int)M, (int)N, (int)K, modo);
+        int i = 14;                                                // (12, 13: no external row maxima)
+        if (bytes > 0) { ws = vazio({(int64_t)bytes}, at::kByte, dev); p[i++] = (A_)ws.data_ptr(); }
+        p[i++] = M; p[i++] = N; p[i++] = K; p[i++] = modo;
+        PyObject *ent = PyDict_New(), *forma = Py_BuildValue("(LL)", (long long)M, (long long)N);
+        if (!ent || !forma) { Py_XDECREF(ent); Py_XDECREF(forma); return nullptr; }
+        for (int k = 0; k < 2; k++) {
+            PyDict_SetItem(ent, S_A[k], PyTuple_GET_ITEM(args[9], k));
+            PyDict_SetItem(ent, S_B[k], PyTuple_GET_ITEM(args[10], k));
+            if (tem_x) PyDict_SetItem(ent, S_X[k], PyTuple_GET_ITEM(args[11], k));
+        }
+        const Py_ssize_t kid = anota(args[5], args[6], args[7], ent, forma);
+        Py_DECREF(ent);
+        Py_DECREF(forma);
+        if (kid < 0) return nullptr;
+        p[i++] = (A_)kid;
+        const int rc = chama(bytes > 0 ? fw : fe, p, i);
+        if (rc) return PyLong_FromLong(rc);
+        PyObject* r = par_de(std::move(m1), std::move(e1));
+        if (!r || !duas) return r;
+        PyObject* r2 = par_de(std::move(m2), std::move(e2));
+        if (!r2) { Py_DECREF(r); return nullptr; }
+        PyObject* dois = PyTuple_Pack(2, r, r2);
+        Py_DECREF(r);
+        Py_DECREF(r2);
+        return dois;
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
 }
 
 PyMethodDef metodos[] = {
@@ -194,6 +264,7 @@ PyMethodDef metodos[] = {
     {"novo_cru", (PyCFunction)(void (*)(void))novo_cru, METH_FASTCALL, "uninitialised raw tensor"},
     {"novo", (PyCFunction)(void (*)(void))novo, METH_FASTCALL, "uninitialised tensor"},
     {"espaco_gemm", (PyCFunction)(void (*)(void))espaco_gemm, METH_FASTCALL, "workspace of a product, or None"},
+    {"gemm", (PyCFunction)(void (*)(void))gemm, METH_FASTCALL, "a product: checks, outputs, workspace, record, launch"},
     {"lanca", (PyCFunction)(void (*)(void))lanca, METH_FASTCALL, "records and performs a launch; None, or (launch id, error code)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef modulo = {PyModuleDef_HEAD_INIT, "_nativo", "host half of the operator launcher", -1, metodos, nullptr, nullptr, nullptr, nullptr};
@@ -205,5 +276,10 @@ PyMODINIT_FUNC PyInit__nativo(void) {
     S_trecho = PyUnicode_InternFromString("trecho");
     S_entradas = PyUnicode_InternFromString("entradas");
     S_forma = PyUnicode_InternFromString("forma");
+    for (int k = 0; k < 2; k++) {
+        S_A[k] = PyUnicode_InternFromString(k ? "EA" : "A");
+        S_B[k] = PyUnicode_InternFromString(k ? "EB" : "B");
+        S_X[k] = PyUnicode_InternFromString(k ? "XE" : "X");
+    }
     return PyModule_Create(&modulo);
 }

@@ -103,6 +103,7 @@ class OpsCuda:
         self._nat = _nativo
         self._fn = {}                                             # address of every entry point used so far
         self._ws = self._endereco("jt_gemm_ws_bytes"), self._endereco("jt_stream_atual")
+        self._ws_gemm = self._endereco("jt_gemm_ws"), self._endereco("jt_gemm_ext")
         # a library with only the reference's entry points: the fused extras read as absent, callers fall back to the separate operations
         for metodo, fn in (("transpoe2", "jt_transpoe2"), ("momento_peso", "jt_momento_peso"), ("rms_back_soma", "jt_rms_back_soma"),
                            ("max_linha", "jt_max_linha"), ("atencao_quant", "jt_atencao_quant"), ("atencao_back_quant", "jt_atencao_back_quant"),
@@ -150,6 +151,15 @@ class OpsCuda:
     # ------------------------------------------------------------------ GEMM family
     def _gemm(self, op, modo, A, B, X=None, duas=False, RA=None, RB=None):
         reg, nat = self.reg, self._nat
+        if RA is None and RB is None and not reg.perfil:
+            r = nat.gemm(*self._ws, *self._ws_gemm, BLK, reg.lancamentos, op, reg.onde(), modo, A, B, X, duas)
+            if r.__class__ is tuple:
+                if reg.vigiar:
+                    reg.depois(len(reg.lancamentos) - 1, 0)
+                return r
+            if r is not None:
+                reg.depois(len(reg.lancamentos) - 1, r)
+        # with external row maxima, timed, for a library with only the reference's entry points - and what is wrong with an argument
         if X is None:
             M, K, N, Kb = self._blocos(("A", "B"), A, B)
         else:
