@@ -86,12 +86,14 @@ static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const in
     // a shape the tensor-core kernel takes never falls back silently: a tensor map that can not be encoded is an error
     if (usa_tc && !(faz_mapa(&mA, A, M, K) && faz_mapa(&mB, B, N, K, tn))) return (int)cudaErrorInvalidValue;
     if (!usa_tc && g_via != 0 && g_via != 2) return (int)cudaErrorInvalidValue;     // nor does a forced tensor-core path on a shape it can not take
-    // split-K (raw output only): powers of two while the grid stays below the target and the K range divides evenly
+    // split-K (raw output only): powers of two while the grid stays below the target and the K range divides evenly.  Clearing the output and
+    // adding atomically cost 6 to 9 us, a unit of the tensor-core kernel takes 1.2: a part keeps at least 8 (512 x 256 x 256: 13.8 us in
+    // two parts, 6.8 in one).
     const int unidades = usa_tc ? K / tc::KC : K / BLK;            // indivisible K units of the chosen kernel
     const long long tiles = usa_tc ? (long long)(N / tn) * (M / tc::TM) : (long long)(N / TN) * (M / 64);
     int partes = 1;
     if (modo == 1)
-        while (partes * 2 <= unidades && tiles * partes * 2 <= g_alvo_ctas && unidades % (partes * 2) == 0) partes *= 2;
+        while (partes * (usa_tc ? 16 : 2) <= unidades && tiles * partes * 2 <= g_alvo_ctas && unidades % (partes * 2) == 0) partes *= 2;
     if (partes > 1) {
         cudaError_t c = cudaMemsetAsync(S.C32, 0, (size_t)M * N * sizeof(int), g_stream);
         if (c != cudaSuccess) return (int)c;
