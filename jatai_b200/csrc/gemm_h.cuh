@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
 // that multiply.
 //   TNv 128, 16 drain warps, one CTA per SM, persistent: while the drain warps put a tile out, the next one's operands are already
 //           being loaded and multiplied
-//   TNv 64, 8 drain warps, two CTAs per SM, one tile each (block 32): where 128-wide tiles would leave SMs without work
+//   TNv 64, 8 drain warps, two CTAs per SM, one tile each (block 32): where 128-wide tiles would leave SMs without work; where even these
+//           do, the K ranges of a tile go to a cluster of 2 to 8 CTAs (512 x 512 x 2048: 17.6 -> 12.2 us)
 template <int TNv, int BLK>
 struct CfgH {
     static constexpr bool PERSISTE = TNv == 128;
@@ -163,6 +164,8 @@ struct CfgH {
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 };
 // how the tiles are numbered: columns fastest, then rows, then K ranges
+// With GRUPO the K ranges of a tile are the blocks of a cluster (one tile per block): each leaves its accumulators in shared memory, and each
+// puts out 1 / partes of the rows, summed over the cluster.
 struct Grade { int nx, ny, partes, ppp; };                                  // tiles per row and column, K ranges, 64-element chunks per range
 
 // one lane of a converged warp
@@ -223,7 +226,18 @@ __device__ __forceinline__ void converte_lote(const uint32_t (&a)[NV], const uin
         acc[o + k] += __float2int_rn(__uint_as_float(a[k])) + __float2int_rn(__uint_as_float(b[k])) + (int)(2 * MAGIA);
 }
 
-template <int BLK, int MODO, int TNv>
+__device__ __forceinline__ void grupo_barreira() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes at the same place of another block of the cluster
+__device__ __forceinline__ int4 le_vizinho(uint32_t end, int bloco) {
+    int4 v;
+    asm volatile("{\n .reg .b32 t;\n mapa.shared::cluster.u32 t, %4, %5;\n ld.shared::cluster.v4.s32 {%0, %1, %2, %3}, [t];\n}"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(end), "r"(bloco) : "memory");
+    return v;
+}
+
+template <int BLK, int MODO, int TNv, bool GRUPO>
 __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k_gemm_h(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                                                        const int8_t* __restrict__ RA, const int8_t* __restrict__ RB, const float* __restrict__ nA,
                                                        const float* __restrict__ nB, SaidaGemm S, int M, int N, int K, Grade Gr, int kid) {
@@ -243,6 +257,9 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     volatile int* aborta = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 4);
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int ntiles = Gr.nx * Gr.ny * Gr.partes, npedT = (K + KH - 1) / KH;
+    static_assert(!GRUPO || !C_::PERSISTE, "");
+    // the first tile of this block: in a cluster the K ranges lie next to each other
+    const int tile0 = GRUPO ? (int)blockIdx.x / Gr.partes + (int)blockIdx.x % Gr.partes * (Gr.nx * Gr.ny) : (int)blockIdx.x;
 
     if (tid == 0) {
         for (int i = 0; i < NST; i++) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
@@ -272,7 +289,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             int s = 0;
             uint32_t fase = 1;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+            for (int tile = tile0; tile < ntiles && ok; tile += C_::PERSISTE ? (int)gridDim.x : ntiles) {
                 const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp;
                 const int xf = min(ped0 + Gr.ppp, npedT) * KH;
                 for (int x = ped0 * KH; x < xf; x += KH) {
@@ -295,8 +312,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         int s = 0, t = 0, vez = wid - N_DW - 1;
         uint32_t fase = 0, fase_t = 1;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nped = min(Gr.ppp, npedT - ped0);
+        for (int tile = tile0; tile < ntiles && ok; tile += C_::PERSISTE ? (int)gridDim.x : ntiles) {
+            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nped = max(min(Gr.ppp, npedT - ped0), 0);
             for (int i = 0; i < nped && ok; i += CB) {
                 const bool minha = vez == 0;
                 vez = minha ? N_MW - 1 : vez - 1;
@@ -345,9 +362,9 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
             if (++t == NS) { t = 0; fase_t ^= 1; }
         };
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        for (int tile = tile0; tile < ntiles; tile += C_::PERSISTE ? (int)gridDim.x : ntiles) {
             const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, parte = tile / (Gr.nx * Gr.ny), ped0 = parte * Gr.ppp;
-            const int nped = min(Gr.ppp, npedT - ped0);
+            const int nped = max(min(Gr.ppp, npedT - ped0), 0);
             // the row maxima, wanted by the output stage: read now, stored to shared memory after the main loop
             int ra = 0, rb = 0;
             if (tid < TM) ra = m0 + tid < M ? (int)RA[m0 + tid] : 0;
@@ -424,7 +441,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             }
             const uint32_t vies = (uint32_t)(BLK == 32 ? nped * 2 : nped / 2) * MAGIA;
             constexpr int PITCHv = TNv + 4;
-            if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
+            if (C_::PERSISTE && tile != tile0) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
             if (tid < TM) RAs[tid] = ra;
             if (tid < TNv) {
                 RBs[tid] = rb;
@@ -446,8 +463,28 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                 *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * COLS + j) =
                     make_int4((int)((uint32_t)acc[j] - vies), (int)((uint32_t)acc[j + 1] - vies), (int)((uint32_t)acc[j + 2] - vies), (int)((uint32_t)acc[j + 3] - vies));
             asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
-            epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s, RAs, RBs, min(TM, M - m0), m0, n0, N, S, Gr.partes > 1, parte == 0, kid, tid, RBf, RBm);
+            if constexpr (!GRUPO) epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s, RAs, RBs, min(TM, M - m0), m0, n0, N, S, Gr.partes > 1, parte == 0, kid, tid, RBf, RBm);
+            else {
+                grupo_barreira();                                            // every block's accumulators are there
+                const int lr = TM / Gr.partes, r0 = parte * lr;              // the rows this block puts out
+                for (int t = tid; t < lr * (TNv / 4); t += N_EPI) {
+                    const int o = (r0 + t / (TNv / 4)) * PITCHv + t % (TNv / 4) * 4;
+                    int4 v = *reinterpret_cast<const int4*>(acc_s + o);
+                    for (int k = 1; k < Gr.partes; k++) {
+                        const int4 x = le_vizinho(smem_u32(acc_s + o), (parte + k) % Gr.partes);
+                        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+                    }
+                    *reinterpret_cast<int4*>(acc_s + o) = v;                 // (only this block reads these rows of its own)
+                }
+                asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
+                epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s + r0 * PITCHv, RAs + r0, RBs, min(lr, max(M - m0 - r0, 0)), m0 + r0, n0, N, S, false, true, kid, tid, RBf, RBm);
+            }
         }
+    }
+    if constexpr (GRUPO) {
+        __syncwarp();
+        if (wid >= N_DW) grupo_barreira();
+        grupo_barreira();                                                    // nobody leaves while another reads its accumulators
     }
     tc_fence_antes();
     __syncthreads();

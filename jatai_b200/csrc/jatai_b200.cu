@@ -139,7 +139,7 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
 }
 // Estimated times of the GEMM kernels in microseconds (measured at 128..16384 rows, 128..4096 columns, K = 128..16384): waves of tiles
 // times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels.
-struct Custos { double i8, h64, h128; };
+struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
 static Custos custos_gemm(int blk, int M, int N, int K) {
     const double n = (K + 63) / 64;
     const long long t128 = (long long)(N / 128) * ((M + 127) / 128), t64 = 2 * t128;
@@ -148,6 +148,13 @@ static Custos custos_gemm(int blk, int M, int N, int K) {
     Custos c;
     c.h128 = prep + ondas(t128, N_SM) * (n * (blk == 32 ? 0.41 : 0.28) + 1.5);
     c.h64 = blk == 32 ? prep + (t64 <= N_SM ? n * 0.31 + 2.5 : ondas(t64, 2 * N_SM) * (n * 0.45 + 2.0)) : 1e9;
+    c.grupo = 1;
+    // K ranges over a cluster while every block still has an SM for itself and keeps 4 chunks.  (Two to an SM, the blocks of 128 tiles in
+    // two ranges take longer than 128 blocks: 2048 x 512 x 2048 20.8 us against 19.3.)
+    for (int g = 2; blk == 32 && g <= 8 && t64 * g <= N_SM && n >= 4 * g; g *= 2) {
+        const double t = prep + (n / g) * 0.31 + 3.5;
+        if (t < c.h64) { c.h64 = t; c.grupo = g; }
+    }
     if (M % tc::TM || K % tc::KC) c.i8 = 1e9;                                           // whole tiles only
     else if (blk == 32) c.i8 = 2.5 + (t64 <= N_SM ? n * 0.75 : ondas(t64, 2 * N_SM) * n * 1.0);
     else c.i8 = 2.5 + ondas(t128, N_SM) * (n * (t128 <= N_SM ? 0.58 : 0.43) + 1.0);
@@ -159,15 +166,16 @@ static bool usa_h(int M, int N, int K) {
     const Custos c = custos_gemm(g_blk, M, N, K);
     return (c.h64 < c.h128 ? c.h64 : c.h128) < c.i8;
 }
-template <int BLK, int MODO, int TNv>
+template <int BLK, int MODO, int TNv, bool GRUPO>
 static int lanca_h(const CUtensorMap& mA, const CUtensorMap& mB, const int8_t* RA, const int8_t* RB, const float* nA, const float* nB, const SaidaGemm& S,
                    int M, int N, int K, const th::Grade& G, int kid) {
     using C_ = th::CfgH<TNv, BLK>;
-    auto k = th::k_gemm_h<BLK, MODO, TNv>;
+    auto k = th::k_gemm_h<BLK, MODO, TNv, GRUPO>;
     cudaError_t c = at_smem(k, C_::SMEM_BYTES);
     if (c != cudaSuccess) return (int)c;
     const int tiles = G.nx * G.ny * G.partes;
-    lanca_pdl(k, dim3(C_::PERSISTE && tiles > N_SM ? N_SM : tiles), dim3(C_::N_THR), C_::SMEM_BYTES, g_stream, mA, mB, RA, RB, nA, nB, S, M, N, K, G, kid);
+    if (GRUPO) lanca_cluster(k, dim3(tiles), dim3(C_::N_THR), C_::SMEM_BYTES, g_stream, G.partes, mA, mB, RA, RB, nA, nB, S, M, N, K, G, kid);
+    else lanca_pdl(k, dim3(C_::PERSISTE && tiles > N_SM ? N_SM : tiles), dim3(C_::N_THR), C_::SMEM_BYTES, g_stream, mA, mB, RA, RB, nA, nB, S, M, N, K, G, kid);
     return fim();
 }
 template <int BLK>
@@ -187,21 +195,24 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     if (!(faz_mapa_h(&mA, Ah, M, K, tc::TM) && faz_mapa_h(&mB, Bh, N, K, tn))) return (int)cudaErrorInvalidValue;
     const int nped = (K + th::KH - 1) / th::KH, uni = BLK / 64 > 1 ? BLK / 64 : 1;
     const long long tiles = (long long)(N / tn) * ((M + 127) / 128);
-    int partes = 1;
-    if (modo == 1)
+    const bool grupo = estreito && c.grupo > 1;
+    int partes = grupo ? c.grupo : 1;
+    if (modo == 1 && !grupo)
         while (tiles * partes * 2 <= (estreito ? 2 : 1) * g_alvo_ctas && nped >= partes * 2 * 32) partes *= 2;
     const int ppp = ((nped + partes - 1) / partes + uni - 1) / uni * uni;
-    partes = (nped + ppp - 1) / ppp;
+    if (!grupo) partes = (nped + ppp - 1) / ppp;                   // (in a cluster a block without chunks adds zeros)
     const th::Grade G = {N / tn, (M + 127) / 128, partes, ppp};
-    if (partes > 1) {
+    if (partes > 1 && !grupo) {
         cudaError_t c = cudaMemsetAsync(S.C32, 0, (size_t)M * N * sizeof(int), g_stream);
         if (c != cudaSuccess) return (int)c;
     }
 #define JT_H(MD)                                                                                                                            \
     case MD:                                                                                                                                \
         if constexpr (BLK == 32)                                                                                                            \
-            if (estreito) return lanca_h<32, MD, 64>(mA, mB, RAw, RBw, nA, nB, S, M, N, K, G, kid);                                      \
-        return lanca_h<BLK, MD, 128>(mA, mB, RAw, RBw, nA, nB, S, M, N, K, G, kid);
+            if (estreito)                                                                                                                   \
+                return grupo ? lanca_h<32, MD, 64, true>(mA, mB, RAw, RBw, nA, nB, S, M, N, K, G, kid)                                      \
+                             : lanca_h<32, MD, 64, false>(mA, mB, RAw, RBw, nA, nB, S, M, N, K, G, kid);                                    \
+        return lanca_h<BLK, MD, 128, false>(mA, mB, RAw, RBw, nA, nB, S, M, N, K, G, kid);
     switch (modo) { JT_H(0) JT_H(1) JT_H(2) JT_H(3) JT_H(4) }
 #undef JT_H
     return (int)cudaErrorInvalidValue;

@@ -144,10 +144,11 @@ def test_gemm_formas(amb, blk, M, N, K, cru):
 
 @pytest.mark.parametrize("tn", [64, 128])
 @pytest.mark.parametrize("blk,M,N,K", [(32, 64, 128, 32), (32, 128, 128, 96), (32, 192, 256, 2080), (32, 320, 384, 512), (32, 2432, 1408, 160), (32, 128, 128, 8192),
+                                       (32, 320, 128, 544), (32, 192, 256, 1056),
                                        (128, 64, 128, 128), (128, 192, 384, 640), (128, 2432, 1408, 256)])
 def test_gemm_meia_precisao(amb, blk, M, N, K, tn):
     """The half-precision tensor path, forced, in every mode against the oracle: rows that fill no tile, a K of half a chunk, more tiles
-    than SMs, K ranges added with atomics, exponents spread beyond what f16 holds, zero blocks; and saturated rows, whose norms
+    than SMs, K ranges added with atomics or over clusters of 2, 4 and 8 blocks (one of them without chunks), exponents spread beyond what f16 holds, zero blocks; and saturated rows, whose norms
     exclude the fast rounding."""
     ops, oc, reg = amb
     ops.define_blk(blk)
