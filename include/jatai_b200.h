@@ -121,8 +121,8 @@ int jt_gemm_via(int via);
 int jt_atencao_quant(const void* qm, const void* qE, void* Om, void* OE, void* P, int Bt, int T, int H, int D, int GA, int kid);
 int jt_atencao_back_quant(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gm, void* GE,
                           int Bt, int T, int H, int D, int GA, int limite, int kid);
-/* Attention path: 0 automatic (tensor cores when the head dimension is 64 or 16; one CTA per head when T <= 128 and the head dimension
- * is 4) | 1 the tiled CUDA-core kernels.  Same bits either way. */
+/* Attention path: 0 automatic (tensor cores when the head dimension is 64 or 16, and for heads of 4 on longer sequences; one CTA per head
+ * when T <= 128 and the head dimension is 4) | 1 the tiled CUDA-core kernels.  Same bits either way. */
 int jt_atencao_via(int via);
 /* Tile width of the tensor-core GEMM: 0 automatic (64 columns when 128-column tiles would leave most SMs idle, block
  * 32 only) | 64 | 128. */

@@ -1,4 +1,4 @@
-// Integer causal attention with ALiBi on the tensor cores, head dimension 64 or 16, every T that is a multiple of 32.
+// Integer causal attention with ALiBi on the tensor cores, head dimension 64, 16 or 4, every T that is a multiple of 32.
 //
 // Same specification and layouts as atencao.cuh (jatai_cuda/ops.py:186-258 generalised; jatai_cuda/jatai_cuda.cu:822-1006).  Every one of
 // the six contractions - q.k^T, P.V, dO.v^T, dS'.k, dS'^T.q, P^T.dO - is an exact integer sum followed by ONE rounding, so (unlike the
@@ -14,7 +14,8 @@
 //     plain          [BH*T][64] f16                      token rows
 //     digits         [2][BH*T][64] f16                   token rows of the hi digits, then of the lo digits
 //     transposed     [BH*128][T] int8                    row = one digit of one column (hi rows 0..63, lo rows 64..127), over the tokens
-// A head of 16 columns fills 16 of the 64 (and of each 64 digit rows); the rest is neither written nor multiplied into a result.
+// A head of 16 columns fills 16 of the 64 (and of each 64 digit rows); the rest is neither written nor multiplied into a result.  A head of 4
+// has zeros behind it in the token rows, up to the 16 columns of one MMA.
 //
 // A query tile of 64 rows takes its keys in windows of 128 that end with the tile's last query and go back from there.  With the
 // reference's slopes P is exactly zero a few dozen keys behind the diagonal, so one window is nearly always all there is: the forward
@@ -71,10 +72,10 @@ __device__ __forceinline__ void tmem_libera(uint32_t tmem, int colunas) {
 // The MMAs of one score-like product, hd columns.  A = 128 token rows (plain), B = the 64 token rows of the hi digits and the 64 of the lo
 // digits; or, digits on the A side, two products with the 64 token rows of B (plain).
 __device__ __forceinline__ void mma_escores(uint32_t tm, uint64_t da, uint64_t db, int hd) {
-    for (int q = 0; q < hd / 16; q++) th::mma_f16(tm, da + 2 * q, db + 2 * q, ID_F16, q != 0);
+    for (int q = 0; q < (hd + 15) / 16; q++) th::mma_f16(tm, da + 2 * q, db + 2 * q, ID_F16, q != 0);
 }
 __device__ __forceinline__ void mma_escores_a(uint32_t tm, uint64_t dah, uint64_t dal, uint64_t db, int hd) {
-    for (int q = 0; q < hd / 16; q++) {
+    for (int q = 0; q < (hd + 15) / 16; q++) {
         th::mma_f16(tm, dah + 2 * q, db + 2 * q, ID_F16N, q != 0);
         th::mma_f16(tm + NI, dal + 2 * q, db + 2 * q, ID_F16N, q != 0);
     }
@@ -153,8 +154,8 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
     return r;
 }
 
-// grid (pieces of 128 tokens, sequences x groups of 64 / hd heads, 3 or 4), 256 threads: 128 tokens of 64 columns - one head of 64 or four
-// of 16 - of one tensor.  The pieces of a sequence are a cluster (at most 8), which exchanges the maximum exponents: reading a
+// grid (pieces of 128 tokens, sequences x groups of 64 / hd heads, 3 or 4), 256 threads: 128 tokens of 64 columns - one head of 64, four
+// of 16 or sixteen of 4 - of one tensor.  The pieces of a sequence are a cluster (at most 8), which exchanges the maximum exponents: reading a
 // sequence's exponents in every block was half of the traffic to the cache.  The bound of a plain version (one element at a time in integers, digit bytes stored one by
 // one) was instruction issue, three times the memory time.  So: a thread takes 4 tokens x 8 columns; pairs of elements in f32x2 (a byte
 // becomes a float by its place in 2^23's mantissa; v 2^(GA - s) rounds to even in one FMA against 1.5 * 2^23, exactly rnd_d; the 6-bit
@@ -170,8 +171,9 @@ __device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint
     const int8_t* E = z == 3 ? A.gE : A.qE;
     const int ld = z == 3 ? D : 3 * D, col0 = (z == 3 ? 0 : z * D) + h0 * hd, ldb = ld / blk;
     const int cg = tid & 7, tg = tid >> 3;                         // columns 8 cg .. + 7, tokens 4 tg .. + 3 of a piece
+    constexpr int NH = hd < 8 ? 8 / hd : 1;                        // heads of this thread
     const int h = h0 + 8 * cg / hd, ch = 8 * cg % hd, bh = b * A.H + h;
-    const bool ha = h < A.H;
+    const bool ha = h < A.H;                                       // (H is a multiple of 2 where a thread has two heads: D is one of 32)
     const size_t BHT = (size_t)A.BH * T;
     const int peca = blockIdx.x, t0 = peca * 128;
     const bool dentro = t0 + 4 * tg < T;                           // (T is a multiple of 32)
@@ -214,18 +216,22 @@ __device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint
         e0 = red[18]; e1 = red[19];
         em = hd == 64 ? max(e0, e1) : cg < 4 ? e0 : e1;
     }
-    if (blockIdx.x == 0 && tid < 8 && ch == 0 && ha) A.em[bh * 4 + z] = em;
-    if (A.est && blockIdx.x == 0 && z == 3 && tg < at::N_EST && ch == 0 && ha) A.est[bh * at::N_EST + tg] = 0;
+    if (blockIdx.x == 0 && ch == 0 && ha)
+#pragma unroll
+        for (int k = 0; k < NH; k++) {
+            if (tid < 8) A.em[(bh + k) * 4 + z] = em;
+            if (A.est && z == 3 && tg < at::N_EST) A.est[(bh + k) * at::N_EST + tg] = 0;
+        }
     const uint64_t mag = par_f(MAGIA_F, MAGIA_F), menos_mag = par_f(-MAGIA_F, -MAGIA_F), vies = par_f(-8388736.0f, -8388736.0f);      // 2^23 + 128
     const uint64_t um64 = par_f(0.015625f, 0.015625f), m64 = par_f(-64.0f, -64.0f);
-    float norma = 0.0f;
+    float norma[NH] = {};
     uint32_t u[4][8];                                          // 2 r + 128: hi digit in byte 1, 2 (lo + 64) in byte 0
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const float f1 = pot2(A.GA - min(em - ex[k], 40));     // |v 2^GA| < 2^11: 0 from a shift of 13 on
         const uint64_t f = par_f(f1, f1);
         uint32_t pl[4], dh[4], dl[4];
-        float nk = 0.0f;
+        float nk[NH] = {};
 #pragma unroll
         for (int c = 0; c < 4; c++) {                          // two columns at a time
             const uint32_t x = (c < 2 ? w[k].x : w[k].y) ^ 0x80808080u;
@@ -239,36 +245,52 @@ __device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint
                 dh[c] = par_h(hi);
                 dl[c] = par_h(ffma2(hi, m64, rf));
             }
-            if (NRM) nk = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk));
+            if (NRM) nk[c * NH / 4] = fmaf(f_lo(rf), f_lo(rf), fmaf(f_hi(rf), f_hi(rf), nk[c * NH / 4]));
         }
         if (dentro && ha) {
-            const size_t o = ((size_t)bh * T + t0 + 4 * tg + k) * 64 + ch;
-            if (PLANO) *reinterpret_cast<uint4*>(dp + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+            // a head's 8 columns or, of heads of 4, two times 4 columns and 12 zeros
+            auto poe = [&](uint16_t* d, const uint32_t (&x)[4]) {
+#pragma unroll
+                for (int n = 0; n < NH; n++) {
+                    uint4* q = reinterpret_cast<uint4*>(d + ((size_t)(bh + n) * T + t0 + 4 * tg + k) * 64 + ch);
+                    q[0] = NH == 1 ? make_uint4(x[0], x[1], x[2], x[3]) : make_uint4(x[2 * n], x[2 * n + 1], 0, 0);
+                    if (NH > 1) q[1] = make_uint4(0, 0, 0, 0);
+                }
+            };
+            if (PLANO) poe(dp, pl);
             if (DIG) {
-                *reinterpret_cast<uint4*>(dg + o) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
-                *reinterpret_cast<uint4*>(dg + BHT * 64 + o) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
+                poe(dg, dh);
+                poe(dg + BHT * 64, dl);
             }
         }
-        if (NRM) {                                  // squared norm of a head's row: its 8 or 2 lanes are neighbours
-            nk += __shfl_xor_sync(FULL, nk, 1);
-            if (hd == 64) {
-                nk += __shfl_xor_sync(FULL, nk, 2);
-                nk += __shfl_xor_sync(FULL, nk, 4);
+        if (NRM) {                                                 // squared norm of a head's row: its 8 or 2 lanes are neighbours
+#pragma unroll
+            for (int n = 0; n < NH; n++) {
+                if (hd > 8) nk[n] += __shfl_xor_sync(FULL, nk[n], 1);
+                if (hd == 64) {
+                    nk[n] += __shfl_xor_sync(FULL, nk[n], 2);
+                    nk[n] += __shfl_xor_sync(FULL, nk[n], 4);
+                }
+                norma[n] = fmaxf(norma[n], nk[n]);
             }
-            norma = fmaxf(norma, nk);
         }
     }
     if (NRM) {
         // the largest of the 128 tokens, rounded up by more than the error of 64 fp32 additions (it only bounds products)
-        norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 8));
-        norma = fmaxf(norma, __shfl_xor_sync(FULL, norma, 16));
-        if (lane < 8) red[32 + 8 * wid + lane] = __float2int_ru(norma * 1.00002f);
-        __syncthreads();
-        if (tid < 8 && ch == 0 && ha) {
-            int mx = 0;
-            for (int k = 0; k < 8; k++) mx = max(mx, red[32 + 8 * k + cg]);
-            A.nrm[((size_t)bh * 2 + z) * ((T + 127) / 128) + peca] = mx;
+#pragma unroll
+        for (int n = 0; n < NH; n++) {
+            norma[n] = fmaxf(norma[n], __shfl_xor_sync(FULL, norma[n], 8));
+            norma[n] = fmaxf(norma[n], __shfl_xor_sync(FULL, norma[n], 16));
+            if (lane < 8) red[32 + (8 * n + wid) * 8 + lane] = __float2int_ru(norma[n] * 1.00002f);
         }
+        __syncthreads();
+        if (tid < 8 && ch == 0 && ha)
+#pragma unroll
+            for (int n = 0; n < NH; n++) {
+                int mx = 0;
+                for (int k = 0; k < 8; k++) mx = max(mx, red[32 + (8 * n + k) * 8 + cg]);
+                A.nrm[((size_t)(bh + n) * 2 + z) * ((T + 127) / 128) + peca] = mx;
+            }
     }
     if (TRA) {
         if (ha)
@@ -292,7 +314,7 @@ __device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint
 }
 template <int hd>
 __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
-    __shared__ int red[32 + 8 * 8];
+    __shared__ int red[32 + 2 * 8 * 8];
     __shared__ __align__(16) uint32_t tr[128 * 32];
     const int z = blockIdx.z;
     uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
@@ -381,6 +403,29 @@ __device__ __forceinline__ void zera_bloco(unsigned char* tile, int q0, int kq, 
 // 32 bytes as numbers
 __device__ __forceinline__ int byte_u(const uint32_t (&w)[8], int k) { return (int)__byte_perm(w[k >> 2], 0, 0x4440 + (k & 3)); }
 
+// Output of the columns of a tile's 64 rows (all threads of the block): valor(row, column) gives the integer, `lin` the token row of row 0,
+// the rows from `fim` on are not stored; `col` of `ld` columns.
+template <typename F>
+__device__ __forceinline__ void grava_tile(F valor, int* acc, int16_t* ex, int8_t* qm, int8_t* qE, size_t lin, int fim, int ld, int col, int hd, int e, int kid, int tid) {
+    if (hd == 4) {                                                 // (raw only)
+        if (tid < fim) {
+            const uint32_t e2 = (uint32_t)(e & 0xffff) | ((uint32_t)e << 16);
+            const size_t p = (lin + tid) * ld + col;
+            *reinterpret_cast<int4*>(acc + p) = make_int4(valor(tid, 0), valor(tid, 1), valor(tid, 2), valor(tid, 3));
+            *reinterpret_cast<uint2*>(ex + p) = make_uint2(e2, e2);
+        }
+        return;
+    }
+    for (int t = tid; t < NI * hd / 8; t += NTA) {                 // (whole warps)
+        const int r = t / (hd / 8), d0 = t % (hd / 8) * 8;
+        int o[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) o[k] = valor(r, d0 + k);
+        const size_t l = lin + min(r, fim - 1);
+        grava8(acc, ex, qm, qE, l * ld + col + d0, l * (ld / 32) + (col + d0) / 32, o, e, kid, t, r < fim);
+    }
+}
+
 // -------------------------------------------------------------------------------------------------- forward
 // ops.py:198-219.  A CTA owns 64 queries of one head.  Three passes over the windows: row maxima; exponentials ex = exp(-(m - u)/256) >> 3
 // and their row sums; P = min((ex * inv + 2^19) >> 20, 255), stored, put into an MMA tile, and O^T += V^T . P^T.  With one window the
@@ -424,7 +469,7 @@ __global__ void __launch_bounds__(NTA, 3) k_at_frente(const __grid_constant__ CU
         carrega(S.s + FR_V, &mVt, j00, bh * 128, TILE_A, S.bar[B_V]);
     }
     const int emq = A.em[bh * 4], emk = A.em[bh * 4 + 1], emv = A.em[bh * 4 + 2];
-    const int s_u = -((emq - GA) + (emk - GA) - (hd == 64 ? 3 : 2) + 8), incl = at::incl_alibi(h);
+    const int s_u = -((emq - GA) + (emk - GA) - (hd == 64 ? 3 : hd == 16 ? 2 : 1) + 8), incl = at::incl_alibi(h);
     const bool direita = s_u > 0 && s_u < 31;
     const int nmax = (i0 + NI - 1) / TJ + 1;
     int B = 0;                                                     // bound of the products in the units of the scores
@@ -605,14 +650,8 @@ __global__ void __launch_bounds__(NTA, 3) k_at_frente(const __grid_constant__ CU
         for (int k = 0; k < 32; k++) o_s[lt * 65 + q0 + k] = (int)d[k];
     }
     __syncthreads();
-    for (int t = tid; t < NI * hd / 8; t += NTA) {                 // (whole warps: 64 or 16 columns of 64 rows)
-        const int i = t / (hd / 8), d0 = t % (hd / 8) * 8;
-        int o[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) o[k] = (int)(((uint32_t)o_s[(d0 + k) * 65 + i] << 7) + (uint32_t)o_s[(64 + d0 + k) * 65 + i]);
-        const size_t lin = (size_t)(linha0 + min(i0 + i, T - 1));
-        grava8(A.Oacc, A.Oe, A.Qm, A.QE, lin * D + h * hd + d0, lin * (D / 32) + (h * hd + d0) / 32, o, (emv - GA) - 8, kid, t, i0 + i < T);
-    }
+    grava_tile([&](int i, int d) { return (int)(((uint32_t)o_s[d * 65 + i] << 7) + (uint32_t)o_s[(64 + d) * 65 + i]); }, A.Oacc, A.Oe, A.Qm, A.QE,
+               (size_t)linha0 + i0, min(NI, T - i0), D, h * hd, hd, (emv - GA) - 8, kid, tid);
     termina(S, colunas);
 }
 
@@ -989,17 +1028,10 @@ __device__ __forceinline__ int ab_saida(Base& S, const CUtensorMap& mB, const CU
     __syncthreads();
     const int emz = A.em[bh * 4 + (CHAVE ? 0 : 1)], emv = A.em[bh * 4 + 2], emg = A.em[bh * 4 + 3];
     const int e = (emg - GA) + (emv - GA) + sh - 9 + sh2 + (emz - GA), col = (CHAVE ? D : 0) + h * hd;
-    for (int n = tid; n < NI * hd / 8; n += NTA) {                 // (whole warps)
-        const int r = n / (hd / 8), d0 = n % (hd / 8) * 8;
-        int o[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int* p = o_s + (d0 + k) * 65 + r;
-            o[k] = junta3((uint32_t)p[0], (uint32_t)p[64 * 65] + (uint32_t)p[128 * 65], (uint32_t)p[192 * 65]);
-        }
-        const size_t lin = (size_t)(b * T + min(t0 + r, T - 1));
-        grava8(A.Gacc, A.Ge, A.Gm, A.GE, lin * 3 * D + col + d0, lin * (3 * D / 32) + (col + d0) / 32, o, e, kid, n, t0 + r < T);
-    }
+    grava_tile([&](int r, int d) {
+        const int* p = o_s + d * 65 + r;
+        return junta3((uint32_t)p[0], (uint32_t)p[64 * 65] + (uint32_t)p[128 * 65], (uint32_t)p[192 * 65]);
+    }, A.Gacc, A.Ge, A.Gm, A.GE, (size_t)b * T + t0, min(NI, T - t0), 3 * D, col, hd, e, kid, tid);
     return colunas;
 }
 __device__ __forceinline__ void ab_valor(Base& S, const CUtensorMap& mX, const CUtensorMap& mP, const ArgsTras& A, int bh, int tile) {
@@ -1047,14 +1079,8 @@ __device__ __forceinline__ void ab_valor(Base& S, const CUtensorMap& mX, const C
     }
     __syncthreads();
     const int e = A.em[bh * 4 + 3] - GA - 8, col = 2 * D + h * hd;
-    for (int t = tid; t < NI * hd / 8; t += NTA) {                 // (whole warps)
-        const int r = t / (hd / 8), d0 = t % (hd / 8) * 8;
-        int o[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) o[k] = (int)(((uint32_t)o_s[(d0 + k) * 65 + r] << 7) + (uint32_t)o_s[(64 + d0 + k) * 65 + r]);
-        const size_t lin = (size_t)(b * T + min(t0 + r, T - 1));
-        grava8(A.Gacc, A.Ge, A.Gm, A.GE, lin * 3 * D + col + d0, lin * (3 * D / 32) + (col + d0) / 32, o, e, kid, t, t0 + r < T);
-    }
+    grava_tile([&](int r, int d) { return (int)(((uint32_t)o_s[d * 65 + r] << 7) + (uint32_t)o_s[(64 + d) * 65 + r]); }, A.Gacc, A.Ge, A.Gm, A.GE,
+               (size_t)b * T + t0, min(NI, T - t0), 3 * D, col, hd, e, kid, tid);
 }
 __global__ void __launch_bounds__(NTA, 3) k_ab_saida(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mGd,
                                                      const __grid_constant__ CUtensorMap mKt, const __grid_constant__ CUtensorMap mQt,
@@ -1076,13 +1102,17 @@ __global__ void __launch_bounds__(NTA, 3) k_ab_saida(const __grid_constant__ CUt
 // -------------------------------------------------------------------------------------------------- host side
 static size_t atc_arredonda(size_t x) { return (x + 1023) & ~(size_t)1023; }
 
-// head dimension 64 or 16; the aligned operands fit f16 exactly up to 4 guard bits (127 << 4 = 2032)
-static bool atc_serve(int blk, int T, int H, int D, int GA) {
-    return (D == H * 64 || D == H * 16) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 && (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
+// Head dimension 64, 16 or, on long sequences, 4; the aligned operands fit f16 exactly up to 4 guard bits (127 << 4 = 2032).  A head of 4 is
+// cheap to multiply on the CUDA cores, so the forward of atencao.cuh stays ahead up to T = 256 (2 x 256 tokens, 32 heads: 24 us against
+// 40; 2 x 512, 64 heads: 150 against 135; 1 x 1024: 408 against 199); its backward does not (2 x 256: 66 us against 40), and up to
+// T = 128 the kernels of one CTA per head take both.
+static bool atc_serve(int blk, int T, int H, int D, int GA, bool tras) {
+    return (D == H * 64 || D == H * 16 || (D == H * 4 && T > (tras ? 128 : 256))) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 &&
+           (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
 }
 static void atc_prep(const atc::ArgsPrep& A, int Bt, int hd, int z, cudaStream_t st) {
     const int np = (A.T + 127) / 128, hpc = 64 / hd;
-    lanca_cluster(hd == 64 ? atc::k_at_prep<64> : atc::k_at_prep<16>, dim3(np, Bt * ((A.H + hpc - 1) / hpc), z), dim3(256), 0, st, np, A);
+    lanca_cluster(hd == 64 ? atc::k_at_prep<64> : hd == 16 ? atc::k_at_prep<16> : atc::k_at_prep<4>, dim3(np, Bt * ((A.H + hpc - 1) / hpc), z), dim3(256), 0, st, np, A);
 }
 
 // forward: preparation (q digits, k plain, v transposed), then the kernel
@@ -1141,7 +1171,8 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
     if (limite) {
         at::ArgsTras L = {gom, goE, qm, qE, P, Gacc, Ge, est, sl, nullptr, T, H, D, GA, blk, limite, kid};
         if (hd == 64) at::k_lim<64><<<BH, 256, 0, st>>>(L);
-        else at::k_lim<16><<<BH, 256, 0, st>>>(L);
+        else if (hd == 16) at::k_lim<16><<<BH, 256, 0, st>>>(L);
+        else at::k_lim<4><<<BH, 256, 0, st>>>(L);
     } else {
         if ((c = at_smem(atc::k_ab_max, atc::SM_MAX)) != cudaSuccess) return (int)c;
         lanca_pdl(atc::k_ab_max, dim3(A.blocos_mapa + BH * nt), dim3(atc::NTA), atc::SM_MAX, st, mV128, mGd, A);

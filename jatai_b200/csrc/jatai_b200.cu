@@ -30,7 +30,7 @@ static cudaStream_t g_stream = 0;
 static int g_blk = 32;               // exponent block length: 32 (native) or 128 (the reference's format)
 static int g_via = 0;                // GEMM path: 0 automatic | 1 tensor core (forced) | 2 CUDA cores | 3 tensor core, rounding by conversion | 4 half-precision tensor pipe (forced)
 static int g_alvo_ctas = 148;
-static int g_at_via = 0;             // attention path: 0 automatic (tensor cores at head dimensions 64 and 16, one CTA per head for short sequences of small heads) | 1 the tiled CUDA-core kernels
+static int g_at_via = 0;             // attention path: 0 automatic (tensor cores; one CTA per head for short sequences of heads of 4) | 1 the tiled CUDA-core kernels
 static int g_tn = 0;                 // tile width of the tensor-core GEMM: 0 automatic | 64 | 128        // split-K of raw GEMMs aims at this many CTAs
 
 static int fim() { return (int)cudaGetLastError(); }
@@ -490,7 +490,7 @@ int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid) 
 
 // ---------------------------------------------------------------------------------------------- attention
 int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, int Bt, int T, int H, int D, int GA, int kid) {
-    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA))
+    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, false))
         return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, nullptr, nullptr, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
     if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA))
         return atencao_frente_peq(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
@@ -498,7 +498,7 @@ int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, in
 }
 int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge, int Bt, int T,
                     int H, int D, int GA, int limite, int kid) {
-    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA))
+    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, true))
         return atencao_tras_tc(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
                                (int16_t*)Ge, nullptr, nullptr, Bt, T, H, D, GA, limite, kid, g_stream);
     if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA))
@@ -511,12 +511,12 @@ int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void
 // [Bt*T, 3D] come out directly.  Served by the tensor-core path at head dimension 64 and block length 32; elsewhere
 // cudaErrorNotSupported, and the caller composes the two operations.
 int jt_atencao_quant(const void* qm, const void* qE, void* Om, void* OE, void* P, int Bt, int T, int H, int D, int GA, int kid) {
-    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA)) return (int)cudaErrorNotSupported;
+    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, false)) return (int)cudaErrorNotSupported;
     return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, nullptr, nullptr, (int8_t*)Om, (int8_t*)OE, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
 }
 int jt_atencao_back_quant(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gm, void* GE, int Bt, int T, int H,
                           int D, int GA, int limite, int kid) {
-    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA)) return (int)cudaErrorNotSupported;
+    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, true)) return (int)cudaErrorNotSupported;
     return atencao_tras_tc(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, nullptr, nullptr,
                            (int8_t*)Gm, (int8_t*)GE, Bt, T, H, D, GA, limite, kid, g_stream);
 }

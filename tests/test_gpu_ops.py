@@ -628,10 +628,11 @@ def test_atencao_pedacos_de_chaves_sem_efeito(amb, mmax, esp, T):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("blk,Bt,T,H,D,e0,longe", [(32, 2, 32, 2, 128, -8, 0), (32, 1, 96, 4, 64, -8, 1), (128, 1, 160, 8, 128, -8, 2), (32, 1, 288, 26, 416, -5, 3),
-                                                   (32, 1, 416, 2, 128, -8, 4), (32, 1, 1024, 34, 544, -4, 0), (32, 1, 1024, 2, 128, -8, 5)])
+                                                   (32, 1, 416, 2, 128, -8, 4), (32, 1, 1024, 34, 544, -4, 0), (32, 1, 1024, 2, 128, -8, 5),
+                                                   (32, 1, 160, 8, 32, -8, 2), (128, 1, 288, 32, 128, -5, 3), (32, 1, 1024, 72, 288, -6, 0), (32, 2, 416, 8, 32, -8, 4)])
 def test_atencao_janelas(amb, blk, Bt, T, H, D, e0, longe):
     """The tensor-core attention walks the keys in windows of 128 that end with a tile of 64 queries: sequence lengths from one
-    half tile to 16 tiles, odd numbers of half tiles, both head dimensions, scores and slopes (heads 16 and on) that need several
+    half tile to 16 tiles, odd numbers of half tiles, the head dimensions, scores and slopes (heads 16 and on) that need several
     windows, and a backward on a P with non-zeros put far from the diagonal, against the oracle."""
     ops, oc, reg = amb
     ops.define_blk(blk)
