@@ -799,10 +799,11 @@ __global__ void __launch_bounds__(256) k_rms_back_soma(const int8_t* __restrict_
     rms_back_corpo<BLK, NP, true>(gm, gE, ym, yE, cr, cemax, xm, xE, om, oE, M, D, log2D, G, GB, kid);
 }
 
-// integer softmax + cross-entropy gradient, one warp per row of raw logits.  ops.py:260-271
+// integer softmax + cross-entropy gradient, LL lanes (a warp; half a warp for V <= 256: 16384 x 256 21.4 -> 12.7 us) per row of raw logits.
+// ops.py:260-271
 //   u = rnd(acc, -(e + 8)); ex = exp(-(umax - u)/256) >> 3; s = sum ex; v = (ex * (2^28 / s) + 2^15) >> 16;
 //   v[target] -= 4096; g = quant(v, -12 - log2M); also d_alvo = umax - u[target] and s for the loss report.
-template <int BLK, int NP>
+template <int BLK, int NP, int LL = 32>
 __global__ void __launch_bounds__(256) k_softmax_ce(const int* __restrict__ acc, const int16_t* __restrict__ e, const int* __restrict__ alvo,
                                                     int8_t* __restrict__ gm, int8_t* __restrict__ gE, int* __restrict__ d_alvo, int* __restrict__ soma,
                                                     int M, int V, int log2M, int kid) {
@@ -810,17 +811,18 @@ __global__ void __launch_bounds__(256) k_softmax_ce(const int* __restrict__ acc,
     pdl_solta();
     constexpr int GL = BLK / 16;
     const int lane = threadIdx.x & 31;
-    const long long lin_ = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int ll = lane & (LL - 1);                                 // lane within the row
+    const long long lin_ = (long long)blockIdx.x * (256 / LL) + threadIdx.x / LL;
     const bool linha_ok = lin_ < M;
     const long long lin = linha_ok ? lin_ : 0;
     int u[NP][16];
     bool tem[NP];
     int umax = U_MIN;
     const int tk = alvo[lin];
-    if (lane == 0 && linha_ok && (tk < 0 || tk >= V)) reporta(E_ARG, kid, lin * V, tk, V);
+    if (ll == 0 && linha_ok && (tk < 0 || tk >= V)) reporta(E_ARG, kid, lin * V, tk, V);
 #pragma unroll
     for (int p = 0; p < NP; p++) {
-        const int c = (p * 32 + lane) * 16;
+        const int c = (p * 32 + ll) * 16;
         tem[p] = c < V;
         int a[16], ee[16], emx = -100000;
         if (tem[p]) {
@@ -845,11 +847,11 @@ __global__ void __launch_bounds__(256) k_softmax_ce(const int* __restrict__ acc,
             umax = max(umax, u[p][i]);
         }
     }
-    umax = warp_max(umax);
+    umax = grupo_max<LL>(umax);
     int s = 0, ut = U_MIN;
 #pragma unroll
     for (int p = 0; p < NP; p++) {
-        const int c = (p * 32 + lane) * 16;
+        const int c = (p * 32 + ll) * 16;
 #pragma unroll
         for (int i = 0; i < 16; i++) {
             if (c + i == tk) ut = u[p][i];
@@ -857,13 +859,14 @@ __global__ void __launch_bounds__(256) k_softmax_ce(const int* __restrict__ acc,
             s += u[p][i];
         }
     }
-    s = warp_sum(s);
-    ut = warp_max(ut);
-    if (s <= 0) { if (lane == 0 && linha_ok) reporta(E_DIV, kid, lin * V, s, 0); s = 1; }
+#pragma unroll
+    for (int d = LL / 2; d; d >>= 1) s += __shfl_xor_sync(FULL, s, d);
+    ut = grupo_max<LL>(ut);
+    if (s <= 0) { if (ll == 0 && linha_ok) reporta(E_DIV, kid, lin * V, s, 0); s = 1; }
     const int inv = (1 << 28) / s;
 #pragma unroll
     for (int p = 0; p < NP; p++) {
-        const int c = (p * 32 + lane) * 16;
+        const int c = (p * 32 + ll) * 16;
         float f[16];                                                       // |v| <= 2^12 + 2^15: exact in fp32
 #pragma unroll
         for (int i = 0; i < 16; i++) f[i] = (float)(((u[p][i] * inv + (1 << 15)) >> 16) - (c + i == tk ? 4096 : 0));
@@ -874,7 +877,7 @@ __global__ void __launch_bounds__(256) k_softmax_ce(const int* __restrict__ acc,
             if ((lane % GL) == 0) gE[lin * (V / BLK) + c / BLK] = (int8_t)Eo;
         }
     }
-    if (lane == 0 && linha_ok) { d_alvo[lin] = umax - ut; soma[lin] = s; }
+    if (ll == 0 && linha_ok) { d_alvo[lin] = umax - ut; soma[lin] = s; }
 }
 
 // loss of every row of softmax_ce's outputs, d / 256 + log(s / 4096) in double precision (report only)

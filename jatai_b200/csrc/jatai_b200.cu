@@ -476,6 +476,11 @@ int jt_rms_back_soma(const void* gm, const void* gE, const void* ym, const void*
 int jt_softmax_ce(const void* acc, const void* e, const void* alvo, void* gm, void* gE, void* d_alvo, void* soma, int M, int V, int log2M,
                   int kid) {
     if (M <= 0 || V <= 0 || V % g_blk || V > 2048) return (int)cudaErrorInvalidValue;
+    if (V <= 256) {                        // 16 lanes take a row: with 32 half of a warp would have nothing
+        lanca_pdl(g_blk == 32 ? k_softmax_ce<32, 1, 16> : k_softmax_ce<128, 1, 16>, dim3((M + 15) / 16), dim3(256), 0, g_stream, (const int*)acc,
+                  (const int16_t*)e, (const int*)alvo, (int8_t*)gm, (int8_t*)gE, (int*)d_alvo, (int*)soma, M, V, log2M, kid);
+        return fim();
+    }
     JT_LINHA(k_softmax_ce, V, (const int*)acc, (const int16_t*)e, (const int*)alvo, (int8_t*)gm, (int8_t*)gE, (int*)d_alvo, (int*)soma, M, V,
              log2M, kid);
     return fim();
