@@ -19,7 +19,7 @@ namespace jt {
 
 // raw (acc int32, e int16 per element) -> block.  ops.py:125-126
 template <int BLK>
-__global__ void __launch_bounds__(256) k_quant(const int* __restrict__ acc, const int16_t* __restrict__ e, int8_t* __restrict__ m,
+__global__ void __launch_bounds__(256, 4) k_quant(const int* __restrict__ acc, const int16_t* __restrict__ e, int8_t* __restrict__ m,
                                                int8_t* __restrict__ E, long long n16, int kid) {
     JT_FIO16
     int v[16], ee[16], q[16];
@@ -149,7 +149,7 @@ __device__ __forceinline__ int soma16_misto(const uint4& rx, int ex, const uint4
 // The quantiser is invariant under the common power of two, so the block is quant(w, e_hi - dl): the same bits with
 // 28-bit instead of 30-bit intermediates, one code path for every d, and rounding shifts shared by the block.
 template <int BLK, int U = 4>
-__global__ void __launch_bounds__(256) k_soma(const int8_t* __restrict__ xm, const int8_t* __restrict__ xE, const int8_t* __restrict__ ym,
+__global__ void __launch_bounds__(256, 3) k_soma(const int8_t* __restrict__ xm, const int8_t* __restrict__ xE, const int8_t* __restrict__ ym,
                                               const int8_t* __restrict__ yE, int8_t* __restrict__ zm, int8_t* __restrict__ zE,
                                               long long n16, int kid) {
     constexpr int GL = BLK / 16;
