@@ -43,13 +43,6 @@ __device__ __forceinline__ void epilogo_tile(const int* acc_s, const int* RAs, c
         const int r = g4 * RPW + (lane & (RPW - 1)), ch = lane / RPW;
         const int gi = m0 + r, gj = n0 + ch * 16;
         const long long o = (long long)gi * N + gj;
-        const long long oe = (long long)gi * (N / BLK) + gj / BLK;
-        uint4 X = make_uint4(0, 0, 0, 0);          // on its way while the accumulators are quantised
-        int eX = 0;
-        if (MODO == 2 || MODO == 4) {
-            X = *reinterpret_cast<const uint4*>(S.Xm + o);
-            eX = S.XE[oe];
-        }
         int v[16];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -78,6 +71,13 @@ __device__ __forceinline__ void epilogo_tile(const int* acc_s, const int* RAs, c
             continue;
         }
         const bool lider = (ch % GL) == 0;
+        const long long oe = (long long)gi * (N / BLK) + gj / BLK;
+        uint4 X = make_uint4(0, 0, 0, 0);          // on its way while the accumulators are quantised
+        int eX = 0;
+        if (MODO == 2 || MODO == 4) {
+            X = *reinterpret_cast<const uint4*>(S.Xm + o);
+            eX = S.XE[oe];
+        }
         int q[16], E;
         bool rapido = false;
         if (RBf) {

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     const int ntiles = Gr.nx * Gr.ny * Gr.partes, npedT = (K + KH - 1) / KH;
     static_assert(!GRUPO || !C_::PERSISTE, "");
     // the first tile of this block: in a cluster the K ranges lie next to each other
-    const int tile0 = GRUPO ? (int)blockIdx.x / Gr.partes + (int)blockIdx.x % Gr.partes * (Gr.nx * Gr.ny) : (int)blockIdx.x;
+    auto tile0 = [&]() -> int { return GRUPO ? (int)blockIdx.x / Gr.partes + (int)blockIdx.x % Gr.partes * (Gr.nx * Gr.ny) : (int)blockIdx.x; };
 
     if (tid == 0) {
         for (int i = 0; i < NST; i++) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             int s = 0;
             uint32_t fase = 1;
             bool ok = true;
-            for (int tile = tile0; tile < ntiles && ok; tile += C_::PERSISTE ? (int)gridDim.x : ntiles) {
+            for (int tile = tile0(); tile < ntiles && ok; tile += GRUPO ? ntiles : gridDim.x) {
                 const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp;
                 const int xf = min(ped0 + Gr.ppp, npedT) * KH;
                 for (int x = ped0 * KH; x < xf; x += KH) {
@@ -312,8 +312,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         int s = 0, t = 0, vez = wid - N_DW - 1;
         uint32_t fase = 0, fase_t = 1;
         bool ok = true;
-        for (int tile = tile0; tile < ntiles && ok; tile += C_::PERSISTE ? (int)gridDim.x : ntiles) {
-            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nped = max(min(Gr.ppp, npedT - ped0), 0);
+        for (int tile = tile0(); tile < ntiles && ok; tile += GRUPO ? ntiles : gridDim.x) {
+            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
             for (int i = 0; i < nped && ok; i += CB) {
                 const bool minha = vez == 0;
                 vez = minha ? N_MW - 1 : vez - 1;
@@ -362,9 +362,9 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
             if (++t == NS) { t = 0; fase_t ^= 1; }
         };
-        for (int tile = tile0; tile < ntiles; tile += C_::PERSISTE ? (int)gridDim.x : ntiles) {
+        for (int tile = tile0(); tile < ntiles; tile += GRUPO ? ntiles : gridDim.x) {
             const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, parte = tile / (Gr.nx * Gr.ny), ped0 = parte * Gr.ppp;
-            const int nped = max(min(Gr.ppp, npedT - ped0), 0);
+            const int nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
             // the row maxima, wanted by the output stage: read now, stored to shared memory after the main loop
             int ra = 0, rb = 0;
             if (tid < TM) ra = m0 + tid < M ? (int)RA[m0 + tid] : 0;
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             }
             const uint32_t vies = (uint32_t)(BLK == 32 ? nped * 2 : nped / 2) * MAGIA;
             constexpr int PITCHv = TNv + 4;
-            if (C_::PERSISTE && tile != tile0) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
+            if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
             if (tid < TM) RAs[tid] = ra;
             if (tid < TNv) {
                 RBs[tid] = rb;
