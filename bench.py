@@ -53,7 +53,7 @@ CONFIGS = {
 SWEEP = [(16384, 4096, 4096), (16384, 4096, 16384), (16384, 16384, 4096)]        # benchmark configuration 2
 # DRAM bytes read + written per launch of the tensor-core GEMM, from one ncu capture (1 launch, --clock-control none,
 # cold L2) of the 4096 x 4096 x 4096 block GEMM; other shapes scale by their algorithmic bytes (traffic grows with them)
-TRAFEGO_NCU = dict(bytes=35.2e6, forma=(4096, 4096, 4096), fonte="ncu dram__bytes_read.sum + dram__bytes_write.sum, k_gemm_tc 4096x4096x4096, 1 launch")
+TRAFEGO_NCU = dict(bytes=118.7e6, forma=(4096, 4096, 4096), fonte="ncu dram__bytes_read.sum + dram__bytes_write.sum, k_prep_h + k_gemm_h 4096x4096x4096, 1 launch each")
 
 
 # ------------------------------------------------------------------------------------------------ helpers
@@ -413,12 +413,12 @@ def braco_gemm(args):
                      "frac_of_2x_bf16_sustained": ach / (2.0 * pk["bf16_sust"]),
                      "traffic": TRAFEGO_NCU["bytes"] * alg / bytes_gemm(*TRAFEGO_NCU["forma"], BLK, False), "traffic_source": TRAFEGO_NCU["fonte"] + ", scaled by algorithmic bytes",
                      "algorithmic_bytes": alg,
-                     "kernel": "k_gemm_tc<32,0> forward GEMM", "peak_source": f"2 x cuBLAS bf16 burst ({pk['origem']}): kind::i8 issues at twice the bf16 rate",
+                     "kernel": "k_prep_h<32> + k_gemm_h<32,0> forward GEMM", "peak_source": f"2 x cuBLAS bf16 burst ({pk['origem']}): kind::i8 issues at twice the bf16 rate",
                      "alu_bound_note": "every 32-wide K slice is drained from tensor memory and rounded on the CUDA cores: M*N*K/32 element-steps"},
         "clocks": clocks,
         "e2e": {"value": tops_e2e, "unit": "TOPS", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "ms_per_step": ms_e2e,
                 "includes": "H2D of X, W, dY from pinned memory, 3 transposes, 3 GEMMs, D2H of Y, dX, dW"},
-        "gpu_launches": 3 * args.steps,
+        "gpu_launches": 6 * args.steps,                      # a preparation and a product each
     }
     if mundo == 1 and not args.sem_cpu:
         try:
@@ -475,17 +475,23 @@ def mede_sweep(oc, reg, dev, reps=3):
 
 # ------------------------------------------------------------------------------------------------ training step
 def nucleos_por_passo(reg, c):
-    """Kernels of this library launched per step: one per recorded operation, except the attention on the tensor-core
-    path (head dimension 64, T >= 128), whose forward is 2 launches (operand preparation + the kernel) and whose backward is
-    5 (preparation, three row phases, the key-tile kernel), 6 with the map of zero tiles of P from T = 512 on.  The split-K memsets are not counted."""
+    """Kernels of this library launched per step: one per recorded operation, and beyond that
+    a product that takes the half-precision tensor path (the library wants a workspace for it): one more, the preparation;
+    the attention on the tensor cores: one more forward (the preparation), three more backward (preparation, maxima, sums, outputs);
+    the backward of the CUDA-core attention: three more.  The split-K memsets are not counted."""
     from jatai_b200 import ops
-    n = len(reg.lancamentos)
-    if ops.BLK == 32 and c["D"] == 64 * c["H"] and c["T"] % 64 == 0 and 128 <= c["T"] <= 1024:
-        for lanc in reg.lancamentos:
-            if lanc["op"].startswith("atencao_back"):
-                n += 4 if (ops.ATENCAO_LIMITE or c["T"] <= 256) else 5
-            elif lanc["op"].startswith("atencao"):
-                n += 1
+    n, hd, T = len(reg.lancamentos), c["D"] // c["H"], c["T"]
+    ws = getattr(reg.lib, "jt_gemm_ws_bytes", None)
+    if ws is not None:
+        ws.restype = ctypes.c_longlong
+    for lanc in reg.lancamentos:
+        if lanc["op"].startswith("gemm") and ws is not None:
+            A, B = lanc["entradas"]["A"], lanc["entradas"]["B"]
+            n += ws(A.shape[0], B.shape[0], A.shape[1], 0) > 0
+        elif lanc["op"].startswith("atencao_back"):
+            n += 0 if hd == 4 and T <= 128 else 3
+        elif lanc["op"].startswith("atencao"):
+            n += hd != 4 or T > 256
     return n
 
 
@@ -667,7 +673,7 @@ def braco_passo(args):
                      "traffic": TRAFEGO_NCU["bytes"] * pf["gemm_bytes"] / bytes_gemm(*TRAFEGO_NCU["forma"], BLK, False) if mundo == 1 else None,
                      "traffic_source": TRAFEGO_NCU["fonte"] + "; scaled to the step's GEMM launches by their algorithmic bytes (cold-L2 figure: inside the step most operands are still in L2)",
                      "algorithmic_bytes": pf["gemm_bytes"],
-                     "kernel": f"all {r.get('n_gemms')} block GEMMs of one step (k_gemm_tc), issued back to back from one CUDA graph with the step's own operands",
+                     "kernel": f"all {r.get('n_gemms')} block GEMMs of one step (k_gemm_h with k_prep_h, k_gemm_tc), issued back to back from one CUDA graph with the step's own operands",
                      "peak_source": f"2 x cuBLAS bf16 sustained ({pk['origem']}); frac_of_2x_bf16_burst uses the burst figure", "gemm_ms_per_step": r.get("gemm_ms")},
         "clocks": r["clocks"],
         "e2e": {"value": r["tps_e2e"], "unit": "tokens/s", "h2d_bytes_per_step": r["h2d"], "d2h_bytes_per_step": r["d2h"],
