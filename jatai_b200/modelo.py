@@ -175,17 +175,18 @@ class Modelo:
     # Tokens x columns from which a step that is not being recorded uses the second stream: below it a step is bound by its launches,
     # which another stream only adds to (512 tokens x 256 columns: 2.6 ms of launches, 1.8 ms of kernels).
     RAMO_MINIMO = 1 << 19
-    # Side streams, and tokens x columns from which a step uses all of them: below, a chain is a few microseconds long and what another
-    # branch costs at its ends eats what it gives (128 tokens x 128 columns: 1 stream 264 us, 3 streams 273; 2048 x 256: 2.87 and 2.55 ms;
-    # 2048 x 512: 3.65 and 3.36 ms; a fourth gives nothing).
+    # Side streams, and tokens x columns from which a step that is being recorded uses all of them: below, a chain is a few microseconds
+    # long and what another branch costs at its ends eats what it gives (128 tokens x 128 columns: 1 stream 264 us, 3 streams 273; 2048 x
+    # 256: 2.87 and 2.55 ms; 2048 x 512: 3.65 and 3.36 ms; a fourth gives nothing).  A step that is launched operator by operator has its
+    # launches to pay for each (4096 x 512, 6 layers: 1 stream 3.1 to 3.3 ms, 3 streams 3.2 to 3.9) and takes one.
     N_LADOS, VARIOS_MINIMO = 3, 1 << 17
 
     def _usa_ramo(self, tokens):
         if not self._lados:
             return None
-        if tokens * self.D < self.RAMO_MINIMO and not torch.cuda.is_current_stream_capturing():
-            return None
-        return self._lados if tokens * self.D >= self.VARIOS_MINIMO else self._lados[:1]
+        if torch.cuda.is_current_stream_capturing():
+            return self._lados if tokens * self.D >= self.VARIOS_MINIMO else self._lados[:1]
+        return self._lados[:1] if tokens * self.D >= self.RAMO_MINIMO else None
 
     def _pesos_transpostos(self):
         """The backward multiplies by every weight transposed (and re-quantised along the new rows).  The weights do not change
