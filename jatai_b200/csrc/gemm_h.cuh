@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
 #pragma unroll
         for (int i = 0; i < 4; i++) r[i] = Rx[min(l0 + i, linhas - 1)];
     } else {
-        if ((nb & 3) == 0) {
+        if ((nb & 3) == 0 && ((uintptr_t)E & 3) == 0) {          // (an exponent tensor may start at any byte of a larger buffer)
             for (int b = lane * 4; b < nb; b += 128)
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
