@@ -113,6 +113,21 @@ __device__ __forceinline__ void prod4x4(const int* a_s, const int* b_s, int ty, 
     else prod4xn<HD, 1>(a_s, b_s, ty, lane, acc);
 }
 
+// 16 bytes of stored P; `alinhado`: P starts at a multiple of 16 (the caller's tensor may start anywhere in a larger buffer)
+__device__ __forceinline__ uint4 le_p16(const uint8_t* p, bool alinhado) {
+    if (alinhado) return *reinterpret_cast<const uint4*>(p);
+    uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 16; k++) w[k >> 2] |= (uint32_t)p[k] << (8 * (k & 3));
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void grava_p16(uint8_t* p, const uint4& v, bool alinhado) {
+    if (alinhado) { *reinterpret_cast<uint4*>(p) = v; return; }
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 16; k++) p[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
+}
+
 // Row products: out[r][d] = sum_j w_s[4 ty + r][j0 + j] * v_s[j][d] for the 4 rows of warp ty (P.V, dS'.k, dS'^T.q, P^T.dO).
 // A lane owns 4 adjacent columns d (d4 = lane % (HD/4)) and one of NJ = 32 / (HD/4) interleaved groups of 4 keys, so
 // both operands come in 128-bit shared-memory loads (4 rows x 4 keys of w, 4 keys x 4 columns of v -> 64 MACs per 8
@@ -234,7 +249,7 @@ __global__ void __launch_bounds__(256) k_atencao(const int8_t* __restrict__ qm, 
         const int j = k >> 1, hf = k & 1;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (j < nproc) v = *reinterpret_cast<const uint4*>(pT + j * TI + hf * 16);
-        *reinterpret_cast<uint4*>(P + ((size_t)bh * T + j) * T + i0 + hf * 16) = v;
+        grava_p16(P + ((size_t)bh * T + j) * T + i0 + hf * 16, v, ((uintptr_t)P & 15) == 0);
     }
     // O = P . V
     int o[4][4];
@@ -369,7 +384,7 @@ __global__ void __launch_bounds__(256) k_ab_linhas(ArgsTras A) {
     // stored P of this tile: key-major, 32 bytes per key
     for (int k = tid; k < nproc * 2; k += 256) {
         const int j = k >> 1, hf = k & 1;
-        *reinterpret_cast<uint4*>(pT + j * TI + hf * 16) = *reinterpret_cast<const uint4*>(A.P + ((size_t)bh * T + j) * T + i0 + hf * 16);
+        *reinterpret_cast<uint4*>(pT + j * TI + hf * 16) = le_p16(A.P + ((size_t)bh * T + j) * T + i0 + hf * 16, ((uintptr_t)A.P & 15) == 0);
     }
     __syncthreads();
     if (FASE == 2) {

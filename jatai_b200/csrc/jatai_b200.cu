@@ -494,19 +494,26 @@ int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid) 
 }
 
 // ---------------------------------------------------------------------------------------------- attention
+}  // extern "C"
+// What the accesses of the kernels ask of the addresses: the tensor-core path reads mantissas 8 bytes and P 16 bytes (and by TMA) at a time, the
+// one-CTA-per-head kernels mantissas 4 and P 16 bytes.  A tensor that starts elsewhere in a larger buffer goes to the general
+// kernels, which take heads of 4 at any multiple of 4 and P anywhere.
+static bool p_alinhado(const void* P) { return ((uintptr_t)P & 15) == 0; }
+static bool atc_alinhado(const void* qm, const void* gom, const void* P) { return (((uintptr_t)qm | (uintptr_t)gom) & 7) == 0 && p_alinhado(P); }
+extern "C" {
 int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, int Bt, int T, int H, int D, int GA, int kid) {
-    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, false))
+    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, false) && atc_alinhado(qm, nullptr, P))
         return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, nullptr, nullptr, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
-    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA))
+    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA) && p_alinhado(P))
         return atencao_frente_peq(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
     return atencao_frente(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
 }
 int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge, int Bt, int T,
                     int H, int D, int GA, int limite, int kid) {
-    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, true))
+    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, true) && atc_alinhado(qm, gom, P))
         return atencao_tras_tc(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
                                (int16_t*)Ge, nullptr, nullptr, Bt, T, H, D, GA, limite, kid, g_stream);
-    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA))
+    if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA) && p_alinhado(P))
         return atencao_tras_peq(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
                                 (int16_t*)Ge, Bt, T, H, D, GA, limite, kid, g_stream);
     return atencao_tras(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
@@ -516,12 +523,14 @@ int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void
 // [Bt*T, 3D] come out directly.  Served by the tensor-core path at head dimension 64 and block length 32; elsewhere
 // cudaErrorNotSupported, and the caller composes the two operations.
 int jt_atencao_quant(const void* qm, const void* qE, void* Om, void* OE, void* P, int Bt, int T, int H, int D, int GA, int kid) {
-    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, false)) return (int)cudaErrorNotSupported;
+    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, false) || !atc_alinhado(qm, nullptr, P))
+        return (int)cudaErrorNotSupported;
     return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, nullptr, nullptr, (int8_t*)Om, (int8_t*)OE, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
 }
 int jt_atencao_back_quant(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gm, void* GE, int Bt, int T, int H,
                           int D, int GA, int limite, int kid) {
-    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, true)) return (int)cudaErrorNotSupported;
+    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, true) || !atc_alinhado(qm, gom, P))
+        return (int)cudaErrorNotSupported;
     return atencao_tras_tc(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, nullptr, nullptr,
                            (int8_t*)Gm, (int8_t*)GE, Bt, T, H, D, GA, limite, kid, g_stream);
 }

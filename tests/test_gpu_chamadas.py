@@ -51,3 +51,27 @@ def test_produto_com_expoentes_em_qualquer_endereco(amb, blk, M, N, K):
             assert A1[1].data_ptr() % 4 and B1[1].data_ptr() % 4
             for cru in (False, True):
                 compara(f"gemm, exponents at offset {n}, via {via}, cru {cru}", oc.gemm(A1, B1, cru=cru), ref[cru])
+
+
+@pytest.mark.parametrize("blk,Bt,T,H,hd", [(32, 2, 64, 8, 4), (32, 1, 160, 8, 4), (128, 1, 288, 32, 4), (32, 2, 96, 4, 16), (32, 1, 160, 2, 64)])
+def test_atencao_em_qualquer_endereco(amb, blk, Bt, T, H, hd):
+    """P at addresses that are no multiple of 16 (or of 4), and for heads of 4 mantissas at a multiple of 4 that is none of 8: what the
+    kernels with wider accesses cannot take goes to the general ones."""
+    ops, oc, reg = amb
+    ops.define_blk(blk)
+    D, M = H * hd, Bt * T
+    G = casos.Gen(17 + T + H, blk)
+    qkv, go = para_gpu(G.bloco(M, 3 * D, espalha=4, zera=0.02)), para_gpu(G.bloco(M, D, e0=-20, espalha=4))
+    o, P = oc.atencao(qkv, Bt, T, H)
+    ref = oc.atencao_back(go, qkv, P, Bt, T, H)
+    s = spec.Spec(blk)
+    compara("atencao", [*o, P], [*casos.plano(s.atencao(qkv, Bt, T, H))])
+    compara("atencao_back", ref, s.atencao_back(go, qkv, P, Bt, T, H))
+    for n in (1, 4, 8):
+        compara(f"atencao_back, P at offset {n}", oc.atencao_back(go, qkv, deslocado(P, n), Bt, T, H), ref)
+    for n in (4, 8, 12) if hd == 4 else ():
+        q2, g2 = (deslocado(qkv[0], n), deslocado(qkv[1], 1)), (deslocado(go[0], n), deslocado(go[1], 3))
+        o2, P2 = oc.atencao(q2, Bt, T, H)
+        compara(f"atencao, mantissas at offset {n}", [*o2, P2], [*o, P])
+        compara(f"atencao_back, mantissas at offset {n}", oc.atencao_back(g2, q2, P, Bt, T, H), ref)
+        compara(f"atencao_back, everything at offset {n}", oc.atencao_back(g2, q2, deslocado(P, n), Bt, T, H), ref)
