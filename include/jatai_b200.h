@@ -12,13 +12,13 @@
  *     cudaErrorInvalidValue (1) and launch nothing;
  *   - all launches go to the stream given to jt_stream (NULL = legacy default stream); nothing synchronises
  *     except jt_erro_le and jt_sincroniza, so a whole step can be captured in a CUDA graph;
- *   - every input and output is owned by the caller; the only device memory the library allocates is the attention
- *     workspace, one per device: cudaMalloc the first time a size is seen, reused afterwards, replaced by a larger one when
- *     needed (never freed: a recorded CUDA graph may hold the old address; growth inside a stream capture is refused with
- *     cudaErrorStreamCaptureUnsupported, so run one step eagerly before capturing).  Head dimension 64: the split operands
- *     (384 bytes per token and head in the forward, 640 in the backward) and, in the backward, 2*Bt*H*T*T bytes of dS' digits;
- *     other head dimensions: Bt*H*(8+T+T*T) ints (the T*T part only below 1 GiB).  Calls that overlap on the GPU share it;
- *   - host state (stream, block length, paths) is per process; the workspace and kernel attributes are kept per device;
+ *   - every input and output is owned by the caller; the only device memory the library takes is the attention workspace of a call that
+ *     brings none (jt_atencao_ws brings one): allocated in stream order before the call's first kernel and given back behind its last, so calls
+ *     on several streams or threads share nothing; inside a stream capture the allocation becomes part of the graph.  The library's pool
+ *     keeps at most 1 GiB per device between calls (jt_espaco_libera returns it).  Tensor-core path: 512 bytes per token and head in the
+ *     forward, 768 in the backward; where they are not to be had jt_atencao and jt_atencao_back take the CUDA-core kernels: no
+ *     workspace in the forward, Bt*H*(8+T+T*T) ints in the backward (the T*T part only below 1 GiB and where it is to be had);
+ *   - host state (stream, block length, paths) is per process; the pool and kernel attributes are kept per device;
  *   - kernels never trap: a broken invariant is recorded in the device error record and the kernel goes on.
  *
  * Tensor formats (jatai_cuda.cu:3-9):
@@ -121,6 +121,19 @@ int jt_gemm_via(int via);
 int jt_atencao_quant(const void* qm, const void* qE, void* Om, void* OE, void* P, int Bt, int T, int H, int D, int GA, int kid);
 int jt_atencao_back_quant(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gm, void* GE,
                           int Bt, int T, int H, int D, int GA, int limite, int kid);
+/* jt_atencao / jt_atencao_quant and jt_atencao_back / jt_atencao_back_quant with a workspace of the caller (128-byte aligned, at least
+ * jt_atencao_ws_bytes bytes - tras = 0 forward, 1 backward; 0 bytes: the call uses none - private to the call until its kernels are done).  The
+ * raw outputs (Oacc, Oe / Gacc, Ge) or the block outputs (Om, OE / Gm, GE), the others NULL.  Without a workspace that serves (or with
+ * mantissas at no multiple of 8 bytes or P at none of 16) the raw forms run on the kernels that need none, and the block forms are
+ * refused with cudaErrorNotSupported.  Same bits every way. */
+long long jt_atencao_ws_bytes(int Bt, int T, int H, int D, int GA, int tras);
+int jt_atencao_ws(const void* qm, const void* qE, void* Oacc, void* Oe, void* Om, void* OE, void* P, void* ws, int Bt, int T, int H, int D, int GA,
+                  int kid);
+int jt_atencao_back_ws(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge, void* Gm, void* GE,
+                       void* ws, int Bt, int T, int H, int D, int GA, int limite, int kid);
+/* The largest workspace the library takes for a call, in bytes (0, the default: no limit) / return what its pool keeps between calls. */
+int jt_espaco_limite(long long bytes);
+int jt_espaco_libera(void);
 /* Attention path: 0 automatic (tensor cores when the head dimension is 64 or 16, and for heads of 4 on longer sequences; one CTA per head
  * when T <= 128 and the head dimension is 4) | 1 the tiled CUDA-core kernels.  Same bits either way. */
 int jt_atencao_via(int via);
@@ -168,8 +181,8 @@ int jt_transpoe2_max(const void* X1, const void* EX1, void* Y1, void* EY1, const
                      void* RM2, int C1, int C2, int R, int kid);
 
 /* jt_atencao_back for callers that may not allocate device memory (fixed memory budgets, code running where
- * cudaMalloc is forbidden): same arguments and results, but the workspace lives in a fixed 4 MiB device array
- * inside the library instead of a cudaMalloc'd buffer, and no allocating routine is called.  Refuses
+ * allocation is forbidden): same arguments and results, but the workspace lives in a fixed 4 MiB device array
+ * inside the library instead of an allocated buffer, and no allocating routine is called.  Refuses
  * Bt*H*(8+T) > 2^20 with cudaErrorInvalidValue; when Bt*H*(8+T+T*T) does not fit either, its kernels recompute the
  * intermediate matrices instead of handing them on (same bits, slower).  The first call on a device resolves the array's address: make it
  * outside stream capture.  All calls share the array; calls that overlap on the GPU race.

@@ -23,6 +23,7 @@
 // computed once and handed on: k_ab1 stores gP, k_ab2 turns it into gP', k_ab3q into dS', k_ab3k reads dS'.  Without
 // it every phase recomputes dO . v^T from the operands.
 #pragma once
+#include <mutex>
 #include "comum.cuh"
 
 namespace jt {
@@ -549,32 +550,50 @@ inline size_t smem_colunas(int HD) { return 4 * ((size_t)TI * (HD + 4) + 2 * TJ 
 
 }  // namespace at
 
-// Workspace of the attention backward (statistics, s_lin, the T x T matrices), one per device, grown on demand.
-// A superseded buffer is never freed: a CUDA graph recorded earlier may still hold its address.  Growth needs
-// cudaMalloc, which a stream capture does not allow: a call that would have to grow while its stream is capturing is
-// refused (cudaErrorStreamCaptureUnsupported); run one step eagerly before capturing, as the reference's loop does.
+// Device memory of one call, in the order of its stream: taken before its first kernel, given back behind its last, so that calls on several
+// streams or threads never share any.  It comes from a pool per device that keeps at most 1 GiB between calls (jt_espaco_libera returns
+// that too).  While the stream is being captured the allocation becomes part of the graph and belongs to it.
 constexpr int AT_MAX_DEV = 64;
-static void* g_at_ws[AT_MAX_DEV];
-static size_t g_at_ws_bytes[AT_MAX_DEV];
+constexpr unsigned long long AT_GUARDA = 1ull << 30;
+static std::mutex g_pool_trava;
+static cudaMemPool_t g_pool[AT_MAX_DEV];
+static long long g_espaco_limite = 0;     // largest workspace the library takes for a call, in bytes; 0 = no limit
 
-// the current device's workspace, at least `bytes` long (0 = ok, else a cudaError_t)
-static int at_ws(size_t bytes, cudaStream_t st, void** p) {
-    int dev = 0;
-    cudaError_t c = cudaGetDevice(&dev);
-    if (c != cudaSuccess) return (int)c;
-    if (dev < 0 || dev >= AT_MAX_DEV) return (int)cudaErrorInvalidDevice;
-    if (bytes > g_at_ws_bytes[dev]) {
+struct Espaco {
+    void* p = nullptr;
+    cudaStream_t st;
+    explicit Espaco(cudaStream_t s) : st(s) {}
+    Espaco(const Espaco&) = delete;
+    ~Espaco() { if (p) (void)cudaFreeAsync(p, st); }
+    // false: not to be had (no error is left behind; the caller takes kernels that need less)
+    bool toma(size_t bytes) {
+        if (g_espaco_limite > 0 && bytes > (size_t)g_espaco_limite) return false;
+        int dev = 0;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return (int)cudaErrorStreamCaptureUnsupported;
-        void* novo = nullptr;
-        c = cudaMalloc(&novo, bytes);
-        if (c != cudaSuccess) return (int)c;
-        g_at_ws[dev] = novo;              // the old buffer stays allocated until the process exits
-        g_at_ws_bytes[dev] = bytes;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= AT_MAX_DEV || cudaStreamIsCapturing(st, &cap) != cudaSuccess) return falhou();
+        if (cap != cudaStreamCaptureStatusNone) return cudaMallocAsync(&p, bytes, st) == cudaSuccess || falhou();
+        {
+            std::lock_guard<std::mutex> l(g_pool_trava);
+            if (!g_pool[dev]) {
+                cudaMemPoolProps pr = {};
+                pr.allocType = cudaMemAllocationTypePinned;
+                pr.location.type = cudaMemLocationTypeDevice;
+                pr.location.id = dev;
+                unsigned long long guarda = AT_GUARDA;
+                if (cudaMemPoolCreate(&g_pool[dev], &pr) != cudaSuccess) { g_pool[dev] = nullptr; return falhou(); }
+                (void)cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &guarda);
+            }
+        }
+        return cudaMallocFromPoolAsync(&p, bytes, g_pool[dev], st) == cudaSuccess || falhou();
     }
-    *p = g_at_ws[dev];
-    return 0;
-}
+
+private:
+    bool falhou() {
+        p = nullptr;
+        (void)cudaGetLastError();
+        return false;
+    }
+};
 
 static int at_log2(int x) { int k = 0; while ((1 << k) < x) k++; return (1 << k) == x ? k : -1; }
 
@@ -657,13 +676,12 @@ static int atencao_tras(int blk, const int8_t* gom, const int8_t* goE, const int
                         int16_t* Ge, int Bt, int T, int H, int D, int GA, int limite, int kid, cudaStream_t st) {
     if (Bt <= 0 || T <= 0 || H <= 0) return (int)cudaErrorInvalidValue;
     // statistics and s_lin, plus the T x T matrix per (sequence, head) that carries gP / gP' / dS' between the phases
-    // (1 GiB at most; beyond that the phases recompute instead)
+    // (1 GiB at most; beyond that, or where it is not to be had, the phases recompute instead)
     const size_t base = (size_t)Bt * H * (at::N_EST + T), matriz = (size_t)Bt * H * T * T;
-    const bool com_matriz = matriz <= ((size_t)1 << 28);
-    const size_t precisa = base + (com_matriz ? matriz : 0);
-    int* ws = nullptr;
-    if (int r = at_ws(precisa * sizeof(int), st, reinterpret_cast<void**>(&ws))) return r;
-    return atencao_tras_ws(blk, gom, goE, qm, qE, P, Gacc, Ge, Bt, T, H, D, GA, limite, kid, st, ws, com_matriz);
+    Espaco ws(st);
+    const bool com_matriz = matriz <= ((size_t)1 << 28) && ws.toma((base + matriz) * sizeof(int));
+    if (!com_matriz && !ws.toma(base * sizeof(int))) return (int)cudaErrorMemoryAllocation;
+    return atencao_tras_ws(blk, gom, goE, qm, qE, P, Gacc, Ge, Bt, T, H, D, GA, limite, kid, st, static_cast<int*>(ws.p), com_matriz);
 }
 
 }  // namespace jt

@@ -1115,16 +1115,24 @@ static void atc_prep(const atc::ArgsPrep& A, int Bt, int hd, int z, cudaStream_t
     lanca_cluster(hd == 64 ? atc::k_at_prep<64> : hd == 16 ? atc::k_at_prep<16> : atc::k_at_prep<4>, dim3(np, Bt * ((A.H + hpc - 1) / hpc), z), dim3(256), 0, st, np, A);
 }
 
-// forward: preparation (q digits, k plain, v transposed), then the kernel
+// Workspace: what the preparation writes.  Forward: head-maximum exponents [BH][4] and the largest squared row norms of q and k per 128 tokens
+// [BH][2][ceil(T/128)]; q digits, k plain, v transposed.  Backward: statistics, s_lin, exponents, map of P; v plain, dO digits, q, k, dO transposed.
+static size_t atc_ws_em(size_t BH, int T, bool tras) {
+    return atc_arredonda(tras ? BH * (at::N_EST + T + 4 + 16) * sizeof(int) : BH * 16 + BH * 2 * ((T + 127) / 128) * 4);
+}
+static size_t atc_ws_lin(size_t BH, int T) { return atc_arredonda(BH * T * 128); }
+static size_t atc_ws_bytes(int Bt, int H, int T, bool tras) {
+    const size_t BH = (size_t)Bt * H;
+    return atc_ws_em(BH, T, tras) + (tras ? 6 : 4) * atc_ws_lin(BH, T);
+}
+
+// forward: preparation (q digits, k plain, v transposed), then the kernel; ws: atc_ws_bytes bytes
 // Qm / QE: block output (jt_quant of the raw output) instead of Oacc / Oe, block length 32 and head dimension 64 only; nullptr = raw output
 static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* Oacc, int16_t* Oe, int8_t* Qm, int8_t* QE, uint8_t* P, int Bt, int T, int H,
-                             int D, int GA, int kid, cudaStream_t st) {
+                             int D, int GA, int kid, cudaStream_t st, unsigned char* ws) {
     if (Qm && (blk != 32 || !QE || D != H * 64)) return (int)cudaErrorInvalidValue;
     const int BH = Bt * H, hd = D / H;
-    // head-maximum exponents [BH][4], then the largest squared row norms of q and k per 128 tokens [BH][2][ceil(T/128)]
-    const size_t b_em = atc_arredonda((size_t)BH * 16 + (size_t)BH * 2 * ((T + 127) / 128) * 4), b_lin = atc_arredonda((size_t)BH * T * 128);
-    unsigned char* ws = nullptr;
-    if (int r = at_ws(b_em + 4 * b_lin, st, reinterpret_cast<void**>(&ws))) return r;
+    const size_t b_em = atc_ws_em(BH, T, false), b_lin = atc_ws_lin(BH, T);
     int* em = reinterpret_cast<int*>(ws);
     int* nrm = em + 4 * BH;
     uint16_t *Qd = reinterpret_cast<uint16_t*>(ws + b_em), *K = reinterpret_cast<uint16_t*>(ws + b_em + 2 * b_lin);
@@ -1144,12 +1152,10 @@ static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* O
 
 // backward: preparation (v plain, dO digits; q, k, dO transposed), the maxima, the sums, the outputs
 static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const int8_t* qm, const int8_t* qE, const uint8_t* P, int* Gacc, int16_t* Ge,
-                           int8_t* Gm, int8_t* GE, int Bt, int T, int H, int D, int GA, int limite, int kid, cudaStream_t st) {
+                           int8_t* Gm, int8_t* GE, int Bt, int T, int H, int D, int GA, int limite, int kid, cudaStream_t st, unsigned char* ws) {
     if (Gm && (blk != 32 || !GE || D != H * 64)) return (int)cudaErrorInvalidValue;
     const int BH = Bt * H, hd = D / H, nt = (T + atc::NI - 1) / atc::NI;
-    const size_t b_est = atc_arredonda((size_t)BH * (at::N_EST + T + 4 + 16) * sizeof(int)), b_lin = atc_arredonda((size_t)BH * T * 128);
-    unsigned char* ws = nullptr;
-    if (int r = at_ws(b_est + 6 * b_lin, st, reinterpret_cast<void**>(&ws))) return r;
+    const size_t b_est = atc_ws_em(BH, T, true), b_lin = atc_ws_lin(BH, T);
     int* est = reinterpret_cast<int*>(ws);
     int* sl = est + (size_t)BH * at::N_EST;
     int* em = sl + (size_t)BH * T;

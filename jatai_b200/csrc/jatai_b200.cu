@@ -499,40 +499,82 @@ int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid) 
 // one-CTA-per-head kernels mantissas 4 and P 16 bytes.  A tensor that starts elsewhere in a larger buffer goes to the general
 // kernels, which take heads of 4 at any multiple of 4 and P anywhere.
 static bool p_alinhado(const void* P) { return ((uintptr_t)P & 15) == 0; }
-static bool atc_alinhado(const void* qm, const void* gom, const void* P) { return (((uintptr_t)qm | (uintptr_t)gom) & 7) == 0 && p_alinhado(P); }
+static bool usa_atc(int Bt, int T, int H, int D, int GA, bool tras) { return g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, tras); }
+static bool usa_atc(const void* qm, const void* gom, const void* P, int Bt, int T, int H, int D, int GA, bool tras) {
+    return (((uintptr_t)qm | (uintptr_t)gom) & 7) == 0 && p_alinhado(P) && usa_atc(Bt, T, H, D, GA, tras);
+}
+static bool ws_serve(const void* ws) { return ws && ((uintptr_t)ws & 127) == 0; }
 extern "C" {
-int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, int Bt, int T, int H, int D, int GA, int kid) {
-    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, false) && atc_alinhado(qm, nullptr, P))
-        return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, nullptr, nullptr, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
+// Workspace of jt_atencao_ws (tras = 0) / jt_atencao_back_ws (1) for these sizes, in bytes; 0: the call would not use one.
+long long jt_atencao_ws_bytes(int Bt, int T, int H, int D, int GA, int tras) {
+    return usa_atc(Bt, T, H, D, GA, tras != 0) ? (long long)atc_ws_bytes(Bt, H, T, tras != 0) : 0;
+}
+// jt_atencao, or (Om, OE instead of Oacc, Oe) jt_atencao_quant, with a workspace of the caller: at least jt_atencao_ws_bytes bytes, 128-byte
+// aligned, private to this call until its kernels are done.  Without one that serves, the raw form is jt_atencao, the other is not supported.
+int jt_atencao_ws(const void* qm, const void* qE, void* Oacc, void* Oe, void* Om, void* OE, void* P, void* ws, int Bt, int T, int H, int D, int GA, int kid) {
+    const bool tc = ws_serve(ws) && usa_atc(qm, nullptr, P, Bt, T, H, D, GA, false);
+    if (Om ? !tc || g_blk != 32 || D != 64 * H : !Oacc || !Oe) return (int)(Om ? cudaErrorNotSupported : cudaErrorInvalidValue);
+    if (tc)
+        return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (int8_t*)Om, (int8_t*)OE, (uint8_t*)P, Bt, T, H, D, GA,
+                                 kid, g_stream, (unsigned char*)ws);
     if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA) && p_alinhado(P))
         return atencao_frente_peq(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
     return atencao_frente(g_blk, (const int8_t*)qm, (const int8_t*)qE, (int*)Oacc, (int16_t*)Oe, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
 }
-int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge, int Bt, int T,
-                    int H, int D, int GA, int limite, int kid) {
-    if (g_at_via == 0 && Bt > 0 && H > 0 && atc_serve(g_blk, T, H, D, GA, true) && atc_alinhado(qm, gom, P))
+int jt_atencao_back_ws(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge, void* Gm, void* GE, void* ws,
+                       int Bt, int T, int H, int D, int GA, int limite, int kid) {
+    const bool tc = ws_serve(ws) && usa_atc(qm, gom, P, Bt, T, H, D, GA, true);
+    if (Gm ? !tc || g_blk != 32 || D != 64 * H : !Gacc || !Ge) return (int)(Gm ? cudaErrorNotSupported : cudaErrorInvalidValue);
+    if (tc)
         return atencao_tras_tc(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
-                               (int16_t*)Ge, nullptr, nullptr, Bt, T, H, D, GA, limite, kid, g_stream);
+                               (int16_t*)Ge, (int8_t*)Gm, (int8_t*)GE, Bt, T, H, D, GA, limite, kid, g_stream, (unsigned char*)ws);
     if (g_at_via == 0 && Bt > 0 && atp_serve(g_blk, T, H, D, GA) && p_alinhado(P))
         return atencao_tras_peq(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
                                 (int16_t*)Ge, Bt, T, H, D, GA, limite, kid, g_stream);
     return atencao_tras(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, (int*)Gacc,
                         (int16_t*)Ge, Bt, T, H, D, GA, limite, kid, g_stream);
 }
+// Without a workspace of the caller the library takes one for the length of the call; where there is none to be had, the raw forms go to the
+// general kernels, which need none (forward) or little (backward).
+int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, int Bt, int T, int H, int D, int GA, int kid) {
+    Espaco ws(g_stream);
+    if (usa_atc(qm, nullptr, P, Bt, T, H, D, GA, false)) (void)ws.toma(atc_ws_bytes(Bt, H, T, false));
+    return jt_atencao_ws(qm, qE, Oacc, Oe, nullptr, nullptr, P, ws.p, Bt, T, H, D, GA, kid);
+}
+int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge, int Bt, int T,
+                    int H, int D, int GA, int limite, int kid) {
+    Espaco ws(g_stream);
+    if (usa_atc(qm, gom, P, Bt, T, H, D, GA, true)) (void)ws.toma(atc_ws_bytes(Bt, H, T, true));
+    return jt_atencao_back_ws(gom, goE, qm, qE, P, Gacc, Ge, nullptr, nullptr, ws.p, Bt, T, H, D, GA, limite, kid);
+}
 // jt_quant(jt_atencao(...)) and jt_quant(jt_atencao_back(...)) in the attention kernels' own output stage: block tensors [Bt*T, D] and
 // [Bt*T, 3D] come out directly.  Served by the tensor-core path at head dimension 64 and block length 32; elsewhere
 // cudaErrorNotSupported, and the caller composes the two operations.
 int jt_atencao_quant(const void* qm, const void* qE, void* Om, void* OE, void* P, int Bt, int T, int H, int D, int GA, int kid) {
-    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, false) || !atc_alinhado(qm, nullptr, P))
-        return (int)cudaErrorNotSupported;
-    return atencao_frente_tc(g_blk, (const int8_t*)qm, (const int8_t*)qE, nullptr, nullptr, (int8_t*)Om, (int8_t*)OE, (uint8_t*)P, Bt, T, H, D, GA, kid, g_stream);
+    if (!Om || g_blk != 32 || D != 64 * H || !usa_atc(qm, nullptr, P, Bt, T, H, D, GA, false)) return (int)cudaErrorNotSupported;
+    Espaco ws(g_stream);
+    if (!ws.toma(atc_ws_bytes(Bt, H, T, false))) return (int)cudaErrorMemoryAllocation;
+    return jt_atencao_ws(qm, qE, nullptr, nullptr, Om, OE, P, ws.p, Bt, T, H, D, GA, kid);
 }
 int jt_atencao_back_quant(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gm, void* GE, int Bt, int T, int H,
                           int D, int GA, int limite, int kid) {
-    if (g_at_via != 0 || g_blk != 32 || Bt <= 0 || H <= 0 || D != 64 * H || !atc_serve(g_blk, T, H, D, GA, true) || !atc_alinhado(qm, gom, P))
-        return (int)cudaErrorNotSupported;
-    return atencao_tras_tc(g_blk, (const int8_t*)gom, (const int8_t*)goE, (const int8_t*)qm, (const int8_t*)qE, (const uint8_t*)P, nullptr, nullptr,
-                           (int8_t*)Gm, (int8_t*)GE, Bt, T, H, D, GA, limite, kid, g_stream);
+    if (!Gm || g_blk != 32 || D != 64 * H || !usa_atc(qm, gom, P, Bt, T, H, D, GA, true)) return (int)cudaErrorNotSupported;
+    Espaco ws(g_stream);
+    if (!ws.toma(atc_ws_bytes(Bt, H, T, true))) return (int)cudaErrorMemoryAllocation;
+    return jt_atencao_back_ws(gom, goE, qm, qE, P, nullptr, nullptr, Gm, GE, ws.p, Bt, T, H, D, GA, limite, kid);
+}
+// The largest workspace the library takes for a call, in bytes (0: no limit) / returns what its pool of the current device keeps between calls.
+int jt_espaco_limite(long long bytes) {
+    if (bytes < 0) return (int)cudaErrorInvalidValue;
+    g_espaco_limite = bytes;
+    return 0;
+}
+int jt_espaco_libera() {
+    int dev = 0;
+    cudaError_t c = cudaGetDevice(&dev);
+    if (c != cudaSuccess) return (int)c;
+    std::lock_guard<std::mutex> l(g_pool_trava);
+    return dev < 0 || dev >= AT_MAX_DEV || !g_pool[dev] ? 0 : (int)cudaMemPoolTrimTo(g_pool[dev], 0);
 }
 int jt_atencao_via(int via) {
     if (via < 0 || via > 1) return (int)cudaErrorInvalidValue;
@@ -541,9 +583,9 @@ int jt_atencao_via(int via) {
 }
 
 // Attention backward for callers that must not allocate device memory: a process that runs under a fixed memory
-// budget carved up before start-up, a host thread inside a stream capture or a callback where cudaMalloc is not
+// budget carved up before start-up, a host thread inside a callback where allocation is not
 // permitted, or an embedding runtime that forbids the library to touch the allocator at all.  jt_atencao_back
-// sizes its workspace with cudaMalloc on first use; this variant keeps the workspace (statistics + one s_lin per
+// takes a workspace for the length of the call; this variant keeps the workspace (statistics + one s_lin per
 // query row = Bt*H*(8+T) ints) in the fixed array below instead, and calls no allocating routine.
 //   * limit: Bt*H*(8+T) <= JT_FIXO_INTS (2^20 ints = 4 MiB, resident on every GPU that loads the library until
 //     the process exits); larger problems are refused with cudaErrorInvalidValue and a message on stderr;

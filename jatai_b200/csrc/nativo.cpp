@@ -10,7 +10,12 @@
 
 namespace {
 
+typedef long long A_;
+
 inline const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// the two members of a pair that bloco_valido has passed
+inline PyObject* const* par_de_args(PyObject* par) { return &PyTuple_GET_ITEM(par, 0); }
 
 // (mantissas, exponents) of a block tensor with block length `blk`: int8, on a GPU, contiguous, exponents [R, C / blk]
 bool bloco_valido(PyObject* par, int64_t blk, int64_t* R, int64_t* C) {
@@ -115,7 +120,6 @@ PyObject* espaco_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // Entry points of the library take pointers and ints (long long for element counts) and return an int: every one of them is an integer
 // argument of the x86-64 calling convention, passed in a 64-bit register or stack slot of which the callee reads what it declares, so one
 // call through a pointer type with N 64-bit arguments serves every signature with N arguments.
-typedef long long A_;
 int chama(void* f, const A_* a, int n) {
 #define C_(...) return reinterpret_cast<int (*)(__VA_ARGS__)>(f)
     switch (n) {
@@ -144,7 +148,7 @@ int chama(void* f, const A_* a, int n) {
     return -1;
 }
 
-PyObject *S_op, *S_trecho, *S_entradas, *S_forma, *S_A[2], *S_B[2], *S_X[2];
+PyObject *S_op, *S_trecho, *S_entradas, *S_forma, *S_A[2], *S_B[2], *S_X[2], *S_qkv[2], *S_go[2], *S_P;
 
 // The launch record {op, trecho, entradas, forma} appended to `lista`; its index, or -1 with a Python error set.
 Py_ssize_t anota(PyObject* lista, PyObject* op, PyObject* trecho, PyObject* entradas, PyObject* forma) {
@@ -257,6 +261,85 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
 }
 
+// atencao(address of jt_atencao_ws_bytes, of jt_stream_atual, of the entry point with a workspace, of the raw one without, blk, launch list, op,
+// section, QKV, dO or None, P or None, Bt, T, H, GA, limit, block outputs) -> forward: (output pair, P), backward (dO and P given): the output
+// pair; None where an argument is not as it should be or there is no workspace for block outputs (nothing was done), the return code
+// where the launch failed.  The whole of an attention call: checks, outputs, workspace, record, launch.
+PyObject* atencao(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 17 || !PyList_Check(args[5])) { PyErr_SetString(PyExc_TypeError, "atencao(4 functions, blk, launches, op, section, QKV, dO, P, Bt, T, H, GA, limit, blocks)"); return nullptr; }
+    void *fb = PyLong_AsVoidPtr(args[0]), *fs = PyLong_AsVoidPtr(args[1]), *fw = PyLong_AsVoidPtr(args[2]), *fp = PyLong_AsVoidPtr(args[3]);
+    const int64_t blk = PyLong_AsLongLong(args[4]), Bt = PyLong_AsLongLong(args[11]), T = PyLong_AsLongLong(args[12]), H = PyLong_AsLongLong(args[13]);
+    const int GA = (int)PyLong_AsLong(args[14]), limite = (int)PyLong_AsLong(args[15]), blocos_ = PyObject_IsTrue(args[16]);
+    if (PyErr_Occurred()) return nullptr;
+    const bool tras = args[9] != Py_None;
+    int64_t M, D3, Mg = 0, Dg = 0;
+    if (!fb || !fs || !fw || !fp || blk <= 0 || Bt <= 0 || T <= 0 || H <= 0 || !bloco_valido(args[8], blk, &M, &D3)) Py_RETURN_NONE;
+    const at::Tensor* P0 = tras ? tensor(args[10]) : nullptr;
+    if (tras && (!P0 || !bloco_valido(args[9], blk, &Mg, &Dg))) Py_RETURN_NONE;
+    const int64_t D = tras ? Dg : D3 / 3, hd = D / H;
+    if (M != Bt * T || D3 != 3 * D || D != H * hd || (tras && Mg != M) || (hd != 4 && hd != 16 && hd != 64) || T % 32 || T > 1024 || Bt * H > INT32_MAX) Py_RETURN_NONE;
+    try {
+        PyObject* const* qkv = par_de_args(args[8]);
+        PyObject* const* go = tras ? par_de_args(args[9]) : nullptr;
+        const at::Tensor &q0 = *tensor(qkv[0]), &q1 = *tensor(qkv[1]);
+        const at::Device dev = q0.device();
+        const A_ pg = tras ? (A_)tensor(go[0])->data_ptr() : 0, pP = tras ? (A_)P0->data_ptr() : 0;
+        at::Tensor ws, m, e, P;
+        long long bytes = 0;
+        if ((((A_)q0.data_ptr() | pg) & 7) == 0 && (pP & 15) == 0 &&
+            reinterpret_cast<void* (*)()>(fs)() == (void*)c10::cuda::getCurrentCUDAStream(dev.index()).stream())
+            bytes = reinterpret_cast<long long (*)(int, int, int, int, int, int)>(fb)((int)Bt, (int)T, (int)H, (int)D, GA, tras);
+        if (bytes <= 0 && blocos_) Py_RETURN_NONE;
+        const int64_t C = tras ? 3 * D : D;
+        m = vazio({M, C}, blocos_ ? at::kChar : at::kInt, dev);
+        e = vazio({M, blocos_ ? C / blk : C}, blocos_ ? at::kChar : at::kShort, dev);
+        if (!tras) P = vazio({Bt * H, T, T}, at::kByte, dev);
+        if (bytes > 0) {
+            try {
+                ws = vazio({(int64_t)bytes}, at::kByte, dev);
+            } catch (const c10::OutOfMemoryError&) {
+                if (blocos_) Py_RETURN_NONE;
+                bytes = 0;                                         // the library sees to it
+            }
+        }
+        A_ p[20];
+        int i = 0;
+        if (tras) { p[i++] = pg; p[i++] = (A_)tensor(go[1])->data_ptr(); }
+        p[i++] = (A_)q0.data_ptr();
+        p[i++] = (A_)q1.data_ptr();
+        if (tras) p[i++] = pP;
+        if (bytes > 0 && blocos_) { p[i++] = 0; p[i++] = 0; }
+        p[i++] = (A_)m.data_ptr();
+        p[i++] = (A_)e.data_ptr();
+        if (bytes > 0 && !blocos_) { p[i++] = 0; p[i++] = 0; }
+        if (!tras) p[i++] = (A_)P.data_ptr();
+        if (bytes > 0) p[i++] = (A_)ws.data_ptr();
+        p[i++] = Bt; p[i++] = T; p[i++] = H; p[i++] = D; p[i++] = GA;
+        if (tras) p[i++] = limite;
+        PyObject *ent = PyDict_New(), *forma = Py_BuildValue("(LL)", (long long)M, (long long)C);
+        bool certo = ent && forma;
+        for (int k = 0; k < 2 && certo; k++) {
+            certo = PyDict_SetItem(ent, S_qkv[k], qkv[k]) == 0;
+            if (tras) certo = certo && PyDict_SetItem(ent, S_go[k], go[k]) == 0;
+        }
+        if (tras) certo = certo && PyDict_SetItem(ent, S_P, args[10]) == 0;
+        const Py_ssize_t kid = certo ? anota(args[5], args[6], args[7], ent, forma) : -1;
+        Py_XDECREF(ent);
+        Py_XDECREF(forma);
+        if (kid < 0) return nullptr;
+        p[i++] = (A_)kid;
+        const int rc = chama(bytes > 0 ? fw : fp, p, i);
+        if (rc) return PyLong_FromLong(rc);
+        PyObject* r = par_de(std::move(m), std::move(e));
+        if (!r || tras) return r;
+        PyObject* Po = THPVariable_Wrap(std::move(P));
+        PyObject* dois = Po ? PyTuple_Pack(2, r, Po) : nullptr;
+        Py_DECREF(r);
+        Py_XDECREF(Po);
+        return dois;
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+
 PyMethodDef metodos[] = {
     {"blocos", (PyCFunction)(void (*)(void))blocos, METH_FASTCALL, "shapes of block tensors, or None"},
     {"cru", cru, METH_O, "shape of a raw tensor, or None"},
@@ -265,6 +348,7 @@ PyMethodDef metodos[] = {
     {"novo", (PyCFunction)(void (*)(void))novo, METH_FASTCALL, "uninitialised tensor"},
     {"espaco_gemm", (PyCFunction)(void (*)(void))espaco_gemm, METH_FASTCALL, "workspace of a product, or None"},
     {"gemm", (PyCFunction)(void (*)(void))gemm, METH_FASTCALL, "a product: checks, outputs, workspace, record, launch"},
+    {"atencao", (PyCFunction)(void (*)(void))atencao, METH_FASTCALL, "an attention call: checks, outputs, workspace, record, launch"},
     {"lanca", (PyCFunction)(void (*)(void))lanca, METH_FASTCALL, "records and performs a launch; None, or (launch id, error code)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef modulo = {PyModuleDef_HEAD_INIT, "_nativo", "host half of the operator launcher", -1, metodos, nullptr, nullptr, nullptr, nullptr};
@@ -280,6 +364,9 @@ PyMODINIT_FUNC PyInit__nativo(void) {
         S_A[k] = PyUnicode_InternFromString(k ? "EA" : "A");
         S_B[k] = PyUnicode_InternFromString(k ? "EB" : "B");
         S_X[k] = PyUnicode_InternFromString(k ? "XE" : "X");
+        S_qkv[k] = PyUnicode_InternFromString(k ? "qkvE" : "qkv");
+        S_go[k] = PyUnicode_InternFromString(k ? "goE" : "go");
     }
+    S_P = PyUnicode_InternFromString("P");
     return PyModule_Create(&modulo);
 }

@@ -379,8 +379,8 @@ class PassoGravado:
     the graph's pool at fixed addresses; weights, momentum and residual are updated in place by the kernels, so
     the graph stays valid.  Inputs go to fixed buffers (copy_) before each replay.  The launch list of the
     recording is kept: the launch ids are baked into the kernel arguments, so a sentinel raised during a replay
-    names the same operation and section as it would in eager mode.  Run one eager step before recording (the
-    attention sizes its workspace on first use, which a capture does not allow).
+    names the same operation and section as it would in eager mode.  Run one eager step before recording: it loads the
+    kernels (and, data parallel, sizes the reducer's buffers).
 
     Data parallel: no collective is ever part of a captured graph; the step is cut into GRUPOS pieces of consecutive layers
     and recorded as 3 graphs per piece, with the collectives issued eagerly between the replays:

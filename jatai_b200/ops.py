@@ -33,7 +33,7 @@ _INT_FUNCS = ("jt_gemm", "jt_gemm_f", "jt_gemm_ext", "jt_max_linha", "jt_quant",
               "jt_momento", "jt_peso", "jt_momento_peso", "jt_transpoe", "jt_transpoe2", "jt_embed", "jt_um_quente", "jt_rms", "jt_rms_back", "jt_rms_back_soma", "jt_atencao",
               "jt_atencao_back", "jt_softmax_ce", "jt_erro_le", "jt_erro_limpa", "jt_sincroniza", "jt_para16", "jt_para8",
               "jt_soma16", "jt_res_estocastico", "jt_blk", "jt_blk_atual", "jt_gemm_via", "jt_gemm_tn", "jt_atencao_back_fixo", "jt_atencao_via", "jt_atencao_quant", "jt_atencao_back_quant",
-              "jt_espera_limite", "jt_teste_espera", "jt_transpoe2_max", "jt_pdl", "jt_gemm_sem_cargas", "jt_gemm_ws", "jt_perda")
+              "jt_espera_limite", "jt_teste_espera", "jt_transpoe2_max", "jt_pdl", "jt_gemm_sem_cargas", "jt_gemm_ws", "jt_perda", "jt_atencao_ws", "jt_atencao_back_ws", "jt_espaco_limite", "jt_espaco_libera")
 
 
 def g_rms(D):
@@ -61,6 +61,8 @@ def carrega_biblioteca(caminho=None):
             getattr(lib, f).restype = ctypes.c_int
     if hasattr(lib, "jt_gemm_ws_bytes"):
         lib.jt_gemm_ws_bytes.restype = ctypes.c_longlong
+        lib.jt_atencao_ws_bytes.restype = ctypes.c_longlong
+        lib.jt_espaco_limite.argtypes = [ctypes.c_longlong]
         lib.jt_stream_atual.restype = ctypes.c_void_p
     return lib
 
@@ -104,6 +106,9 @@ class OpsCuda:
         self._fn = {}                                             # address of every entry point used so far
         self._ws = self._endereco("jt_gemm_ws_bytes"), self._endereco("jt_stream_atual")
         self._ws_gemm = self._endereco("jt_gemm_ws"), self._endereco("jt_gemm_ext")
+        self._ws_at = self._endereco("jt_atencao_ws_bytes"), self._endereco("jt_stream_atual")
+        self._at_frente = self._endereco("jt_atencao_ws"), self._endereco("jt_atencao")
+        self._at_tras = self._endereco("jt_atencao_back_ws"), self._endereco("jt_atencao_back")
         # a library with only the reference's entry points: the fused extras read as absent, callers fall back to the separate operations
         for metodo, fn in (("transpoe2", "jt_transpoe2"), ("momento_peso", "jt_momento_peso"), ("rms_back_soma", "jt_rms_back_soma"),
                            ("max_linha", "jt_max_linha"), ("atencao_quant", "jt_atencao_quant"), ("atencao_back_quant", "jt_atencao_back_quant"),
@@ -328,7 +333,26 @@ class OpsCuda:
         return O
 
     # ------------------------------------------------------------------ attention
+    def _atencao_nativa(self, op, entradas, blocos, QKV, GO, P, Bt, T, H):
+        """The call in one piece, workspace included (`entradas`: the entry points with one and, raw outputs only, without), or None: block
+        outputs without a workspace, a library with only the reference's entry points - and what is wrong with an argument."""
+        reg = self.reg
+        if reg.perfil:
+            reg.cronometra(op)
+        r = self._nat.atencao(*self._ws_at, *entradas, BLK, reg.lancamentos, op, reg.onde(), QKV, GO, P, Bt, T, H, GA, int(ATENCAO_LIMITE), blocos)
+        if r is None:
+            if reg.perfil:
+                reg.eventos.pop()
+        elif r.__class__ is int:
+            reg.depois(len(reg.lancamentos) - 1, r)
+        elif reg.perfil or reg.vigiar:
+            reg.depois(len(reg.lancamentos) - 1, 0)
+        return r
+
     def atencao(self, QKV, Bt, T, H):
+        r = self._atencao_nativa("atencao", self._at_frente, False, QKV, None, None, Bt, T, H)
+        if r is not None:
+            return r
         M, D3 = self._blocos(("qkv",), QKV)
         D = D3 // 3
         hd = D // H
@@ -339,6 +363,9 @@ class OpsCuda:
         return o, P
 
     def atencao_back(self, GO, QKV, P, Bt, T, H):
+        r = self._atencao_nativa("atencao_back", self._at_tras, False, QKV, GO, P, Bt, T, H)
+        if r is not None:
+            return r
         M, D, _, _ = self._blocos(("go", "qkv"), GO, QKV)
         g = self._nat.novo_cru(QKV[0], Bt * T, 3 * D)
         self._lanca("atencao_back", "jt_atencao_back", (*GO, *QKV, P, *g), (Bt, T, H, D, GA, int(ATENCAO_LIMITE)), ("go", "goE", "qkv", "qkvE", "P"),
@@ -350,28 +377,24 @@ class OpsCuda:
         return BLK == 32 and D == 64 * H and T % 32 == 0 and T <= 1024 and GA <= 4
 
     def atencao_quant(self, QKV, Bt, T, H):
-        """(quant(O), P) of atencao(QKV, Bt, T, H): one launch where the library offers it (an addition of this library; same results)."""
+        """(quant(O), P) of atencao(QKV, Bt, T, H): one launch where the library offers it and its workspace is to be had (an addition of
+        this library; same results)."""
         D = QKV[0].shape[1] // 3
-        if not self._atencao_fundida(T, H, D):
-            oc, P = self.atencao(QKV, Bt, T, H)
-            return self.quant(oc), P
-        M, _ = self._blocos(("qkv",), QKV)
-        if M != Bt * T:
-            self.reg.falha(f"atencao_quant: rows {M} (= Bt*T = {Bt * T})")
-        O, P = self._nat.novo_bloco(QKV[0], M, D, BLK), self._nat.novo(QKV[0], "u1", Bt * H, T, T)
-        self._lanca("atencao_quant", "jt_atencao_quant", (*QKV, *O, P), (Bt, T, H, D, GA), ("qkv", "qkvE"), (M, D))
-        return O, P
+        if self._atencao_fundida(T, H, D):
+            r = self._atencao_nativa("atencao_quant", self._at_frente, True, QKV, None, None, Bt, T, H)
+            if r is not None:
+                return r
+        oc, P = self.atencao(QKV, Bt, T, H)
+        return self.quant(oc), P
 
     def atencao_back_quant(self, GO, QKV, P, Bt, T, H):
-        """quant(atencao_back(GO, QKV, P, Bt, T, H)): one launch sequence without the raw intermediate where the library offers it."""
-        D = GO[0].shape[1]
-        if not self._atencao_fundida(T, H, D):
-            return self.quant(self.atencao_back(GO, QKV, P, Bt, T, H))
-        self._blocos(("go", "qkv"), GO, QKV)
-        G = self._nat.novo_bloco(QKV[0], Bt * T, 3 * D, BLK)
-        self._lanca("atencao_back_quant", "jt_atencao_back_quant", (*GO, *QKV, P, *G), (Bt, T, H, D, GA, int(ATENCAO_LIMITE)),
-                    ("go", "goE", "qkv", "qkvE", "P"), (Bt * T, 3 * D))
-        return G
+        """quant(atencao_back(GO, QKV, P, Bt, T, H)): one launch sequence without the raw intermediate where the library offers it and its
+        workspace is to be had."""
+        if self._atencao_fundida(T, H, GO[0].shape[1]):
+            r = self._atencao_nativa("atencao_back_quant", self._at_tras, True, QKV, GO, P, Bt, T, H)
+            if r is not None:
+                return r
+        return self.quant(self.atencao_back(GO, QKV, P, Bt, T, H))
 
     # ------------------------------------------------------------------ loss and optimiser
     def softmax_ce(self, L, alvo, log2M=None):

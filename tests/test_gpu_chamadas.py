@@ -75,3 +75,140 @@ def test_atencao_em_qualquer_endereco(amb, blk, Bt, T, H, hd):
         compara(f"atencao, mantissas at offset {n}", [*o2, P2], [*o, P])
         compara(f"atencao_back, mantissas at offset {n}", oc.atencao_back(g2, q2, P, Bt, T, H), ref)
         compara(f"atencao_back, everything at offset {n}", oc.atencao_back(g2, q2, deslocado(P, n), Bt, T, H), ref)
+
+
+def _limita_torch(folga):
+    """PyTorch's allocator gets `folga` bytes beyond what it holds."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + folga) / torch.cuda.mem_get_info()[1])
+
+
+@pytest.fixture
+def memoria(amb):
+    yield _limita_torch
+    torch.cuda.set_per_process_memory_fraction(1.0)
+    amb[1].lib.jt_espaco_limite(0)
+
+
+def _problema(blk, Bt, T, H, hd, semente=23):
+    G = casos.Gen(semente + T + H, blk)
+    D, M = H * hd, Bt * T
+    return para_gpu(G.bloco(M, 3 * D, espalha=4, zera=0.02)), para_gpu(G.bloco(M, D, e0=-20, espalha=4)), (Bt, T, H)
+
+
+def _tudo(oc, qkv, go, forma):
+    """Raw and quantised attention, both ways."""
+    o, P = oc.atencao(qkv, *forma)
+    g = oc.atencao_back(go, qkv, P, *forma)
+    oq, Pq = oc.atencao_quant(qkv, *forma)
+    return [*o, P, *g, *oq, Pq, *oc.atencao_back_quant(go, qkv, P, *forma)]
+
+
+ESPACOS = [(32, 2, 96, 2, 64), (32, 2, 128, 2, 64), (32, 3, 64, 16, 16), (32, 1, 288, 8, 4), (128, 1, 160, 8, 16)]
+
+
+@pytest.mark.parametrize("blk,Bt,T,H,hd", ESPACOS)
+def test_atencao_sem_memoria_para_o_espaco(amb, memoria, blk, Bt, T, H, hd):
+    """Same bits with the workspace of the caller's allocator, of the library's own pool (the launches are on another stream than the
+    allocator's) and with none: too little memory for either."""
+    ops, oc, reg = amb
+    ops.define_blk(blk)
+    qkv, go, forma = _problema(blk, Bt, T, H, hd)
+    ref = _tudo(oc, qkv, go, forma)
+    s = spec.Spec(blk)
+    compara("atencao", ref[:3], casos.plano(s.atencao(qkv, *forma)))
+    compara("atencao_back", ref[3:5], s.atencao_back(go, qkv, ref[2], *forma))
+    outro = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for limite in (0, 4096 + 4 * Bt * H * (8 + T), 1024):
+        oc.lib.jt_espaco_limite(limite)
+        with torch.cuda.stream(outro):                 # the library goes on launching on the default stream, which waits for nobody here
+            if limite != 1024:
+                out = _tudo(oc, qkv, go, forma)
+                torch.cuda.synchronize()
+                compara(f"own workspace, at most {limite} bytes", out, ref)
+            else:
+                with pytest.raises(Exception, match="refused the launch of 'atencao_back'"):      # not even the sums of the rows
+                    oc.atencao_back(go, qkv, ref[2], *forma)
+    oc.lib.jt_espaco_limite(0)
+    assert oc.lib.jt_espaco_libera() == 0
+
+
+def test_atencao_com_o_alocador_cheio(amb, memoria):
+    """PyTorch's allocator has room for the outputs and none for the workspace: the library's pool serves, then the general kernels."""
+    ops, oc, reg = amb
+    qkv, go, forma = _problema(32, 8, 128, 64, 16)
+    o, P = oc.atencao(qkv, *forma)
+    ref = [*o, P, *oc.atencao_back(go, qkv, P, *forma)]
+    del o, P
+    for limite in (0, 1 << 20):
+        oc.lib.jt_espaco_limite(limite)
+        memoria(50 << 20)                              # outputs 15 and 19 MB (in segments of 20 and 34), workspaces 33 and 50
+        o, P = oc.atencao(qkv, *forma)
+        compara("forward", [*o, P], ref[:3])
+        del o, P
+        memoria(45 << 20)
+        g = oc.atencao_back(go, qkv, ref[2], *forma)
+        compara("backward", g, ref[3:])
+        del g
+
+
+def test_atencao_em_duas_correntes(amb):
+    """Two problems at the same time on two streams: neither sees the other's workspace, with the allocator's and with the library's."""
+    ops, oc, reg = amb
+    reg.vigiar = False
+    ps = [_problema(32, 64, 128, 32, 16, semente=n) for n in (1, 2)]
+    refs = [_tudo(oc, *p) for p in ps]
+    torch.cuda.synchronize()
+    st = [torch.cuda.Stream() for _ in ps]
+    try:
+        for volta in range(12):
+            outs = [[], []]
+            for n in (0, 1):
+                with torch.cuda.stream(st[n]):
+                    torch.cuda._sleep(2_000_000)       # the second one's launches are queued before the first one starts
+            for rep in range(2):
+                for n in (0, 1):
+                    with torch.cuda.stream(st[n]):
+                        oc.lib.jt_stream(st[n].cuda_stream)
+                        outs[n].append(_tudo(oc, *ps[n]))
+            torch.cuda.synchronize()
+            for n in (0, 1):
+                for out in outs[n]:
+                    compara(f"stream {n}, time {volta}", out, refs[n])
+    finally:
+        oc.lib.jt_stream(None)
+
+
+@pytest.mark.parametrize("proprio", [False, True])
+def test_atencao_primeira_chamada_numa_gravacao(amb, proprio):
+    """The first call at a size, both ways, inside a CUDA graph: with the allocator's workspace and with the library's (the graph's own); two
+    graphs recorded on one stream are replayed at the same time on two."""
+    ops, oc, reg = amb
+    reg.vigiar = False
+    ps = [_problema(32, 64, 96, 32, 16, semente=n) for n in (1, 2)]
+    refs = [_tudo(oc, *p) for p in ps]
+    torch.cuda.synchronize()
+    if proprio:
+        oc._ws_at = (0, 0)                             # the launcher brings none
+    grafos, saidas = [], []
+    try:
+        for p in ps:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                oc.lib.jt_stream(torch.cuda.current_stream().cuda_stream)
+                saidas.append(_tudo(oc, *p))
+            grafos.append(g)
+    finally:
+        oc.lib.jt_stream(None)
+    st = [torch.cuda.Stream() for _ in ps]
+    for volta in range(4):
+        for g, s in zip(grafos, st):
+            with torch.cuda.stream(s):
+                g.replay()
+                g.replay()
+        torch.cuda.synchronize()
+        for n in (0, 1):
+            compara(f"replay {volta} of graph {n}", saidas[n], refs[n])
+    del grafos
