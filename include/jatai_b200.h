@@ -146,7 +146,7 @@ int jt_gemm_tn(int tn);
 int jt_gemm_ext(const void* A, const void* EA, const void* B, const void* EB, void* Cm, void* CE, void* C32, void* Ce,
                 const void* Xm, const void* XE, void* Om2, void* OE2, const void* RA, const void* RB,
                 int M, int N, int K, int modo, int kid);
-/* jt_gemm_ext with a workspace (1024-byte aligned, at least jt_gemm_ws_bytes bytes, private to the call until its kernels are done): the
+/* jt_gemm_ext with a workspace (128-byte aligned, at least jt_gemm_ws_bytes bytes, private to the call until its kernels are done): the
  * half-precision tensor path, which needs one, takes the sizes where it is the faster one - jt_gemm_ws_bytes is 0 elsewhere - and with it
  * every size jt_gemm_ext takes runs on the tensor cores.  Same bits either way. */
 long long jt_gemm_ws_bytes(int M, int N, int K, int modo);

@@ -218,6 +218,9 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     return (int)cudaErrorInvalidValue;
 }
 
+// a workspace of the caller: the kernels' widest access to one is a TMA box of 128-byte rows (PyTorch's allocator gives multiples of 512)
+static bool ws_serve(const void* ws) { return ws && ((uintptr_t)ws & 127) == 0; }
+
 #define JT_POR_BLK(EXPR32, EXPR128) (g_blk == 32 ? (EXPR32) : (EXPR128))
 
 extern "C" {
@@ -306,11 +309,11 @@ long long jt_gemm_ws_bytes(int M, int N, int K, int modo) {
     if (!forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K)) return 0;
     return (long long)espaco_h(M, N, K).total;
 }
-// jt_gemm_ext with a workspace of at least jt_gemm_ws_bytes bytes (1024-byte aligned, private to this call until its kernels are done)
+// jt_gemm_ext with a workspace of at least jt_gemm_ws_bytes bytes (128-byte aligned, private to this call until its kernels are done)
 int jt_gemm_ws(const void* A, const void* EA, const void* B, const void* EB, void* Cm, void* CE, void* C32, void* Ce, const void* Xm, const void* XE,
                void* Om2, void* OE2, const void* RA, const void* RB, void* ws, int M, int N, int K, int modo, int kid) {
     const bool alinhado = (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
-    if (!ws || ((uintptr_t)ws & 1023) || !alinhado || !forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K))
+    if (!ws_serve(ws) || !alinhado || !forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K))
         return jt_gemm_ext(A, EA, B, EB, Cm, CE, C32, Ce, Xm, XE, Om2, OE2, RA, RB, M, N, K, modo, kid);
     SaidaGemm S = {(int8_t*)Cm, (int8_t*)CE, (int*)C32, (int16_t*)Ce, (const int8_t*)Xm, (const int8_t*)XE, (int8_t*)Om2, (int8_t*)OE2};
     if (modo == 1 ? (!C32 || !Ce) : (!Cm || !CE)) return (int)cudaErrorInvalidValue;
@@ -503,7 +506,6 @@ static bool usa_atc(int Bt, int T, int H, int D, int GA, bool tras) { return g_a
 static bool usa_atc(const void* qm, const void* gom, const void* P, int Bt, int T, int H, int D, int GA, bool tras) {
     return (((uintptr_t)qm | (uintptr_t)gom) & 7) == 0 && p_alinhado(P) && usa_atc(Bt, T, H, D, GA, tras);
 }
-static bool ws_serve(const void* ws) { return ws && ((uintptr_t)ws & 127) == 0; }
 extern "C" {
 // Workspace of jt_atencao_ws (tras = 0) / jt_atencao_back_ws (1) for these sizes, in bytes; 0: the call would not use one.
 long long jt_atencao_ws_bytes(int Bt, int T, int H, int D, int GA, int tras) {

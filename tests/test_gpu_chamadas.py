@@ -212,3 +212,27 @@ def test_atencao_primeira_chamada_numa_gravacao(amb, proprio):
         for n in (0, 1):
             compara(f"replay {volta} of graph {n}", saidas[n], refs[n])
     del grafos
+
+
+@pytest.mark.parametrize("blk", [32, 128])
+def test_produto_com_espaco_de_128_em_128_bytes(amb, blk):
+    """The workspace of a product may start at any multiple of 128 bytes (small blocks of PyTorch's allocator start at multiples of 512): on
+    64 rows, which only the half-precision path of the forced ones takes, the call must serve."""
+    import ctypes
+    ops, oc, reg = amb
+    ops.define_blk(blk)
+    M, N, K = 64, 128, 256
+    G = casos.Gen(12, blk)
+    A, B = para_gpu(G.bloco(M, K, espalha=4)), para_gpu(G.bloco(N, K, espalha=4))
+    ref = spec.Spec(blk).gemm(A, B)
+    oc.lib.jt_gemm_via(4)
+    n = oc.lib.jt_gemm_ws_bytes(M, N, K, 0)
+    assert n > 0
+    buf = torch.empty(n + 2048, dtype=torch.uint8, device="cuda")
+    for desl in (128, 512, 896):
+        ws = buf[(-buf.data_ptr()) % 1024 + desl:]
+        C = torch.zeros(M, N, dtype=torch.int8, device="cuda"), torch.zeros(M, N // blk, dtype=torch.int8, device="cuda")
+        p = [ctypes.c_void_p(t.data_ptr()) if t is not None else None for t in (*A, *B, *C, *[None] * 8, ws)]
+        assert oc.lib.jt_gemm_ws(*p, *(ctypes.c_int(v) for v in (M, N, K, 0, 0))) == 0
+        torch.cuda.synchronize()
+        compara(f"workspace at {desl}", C, ref)
