@@ -179,7 +179,7 @@ __device__ __forceinline__ void max_cta_atomico(int v, int* destino, int* red, i
 }
 
 // -------------------------------------------------------------------------------------------------- forward
-// ops.py:198-219.  grid (T/32, Bt*H), 256 threads.  Shared: u[32][T+4] int32, kv[128][hd+4], q[32][hd+4], pT[T][32] bytes.
+// ops.py:198-219.  grid (Bt*H, T/32), 256 threads.  Shared: u[32][T+4] int32, kv[128][hd+4], q[32][hd+4], pT[T][32] bytes.
 template <int HD>
 __global__ void __launch_bounds__(256) k_atencao(const int8_t* __restrict__ qm, const int8_t* __restrict__ qE, int* __restrict__ Oacc,
                                                  int16_t* __restrict__ Oe, uint8_t* __restrict__ P, int T, int H, int D, int GA, int blk, int lg2,
@@ -194,8 +194,7 @@ __global__ void __launch_bounds__(256) k_atencao(const int8_t* __restrict__ qm, 
     __shared__ int red[8];
     const int tid = threadIdx.x, ty = tid >> 5, lane = tid & 31;
     // causal work grows with the row tile: CTAs are dispatched in linear order, so the heaviest tiles of all heads go first
-    const int ordem = blockIdx.y * gridDim.x + blockIdx.x;
-    const int bh = ordem % gridDim.y, b = bh / H, h = bh % H, i0 = (gridDim.x - 1 - ordem / gridDim.y) * TI;
+    const int bh = blockIdx.x, b = bh / H, h = bh % H, i0 = (gridDim.y - 1 - blockIdx.y) * TI;
     const int ld = 3 * D, ldb = ld / blk, linha0 = b * T;
     const int emq = max_cabeca<HD>(qE, ldb, blk, linha0, T, h * HD, red, tid);
     const int emk = max_cabeca<HD>(qE, ldb, blk, linha0, T, D + h * HD, red, tid);
@@ -319,7 +318,7 @@ __global__ void __launch_bounds__(256) k_lim(ArgsTras A) {
     max_cta_atomico(mv, A.est + bh * N_EST + S_V1, red, tid);
 }
 
-// FASE 1: max |gP| over j <= i.   FASE 2: gP', s_lin, maxima.   FASE 3: dS', gq.     grid (T/32, Bt*H)
+// FASE 1: max |gP| over j <= i.   FASE 2: gP', s_lin, maxima.   FASE 3: dS', gq.     grid (Bt*H, T/32)
 template <int HD, int FASE>
 __global__ void __launch_bounds__(256) k_ab_linhas(ArgsTras A) {
     constexpr int PK = HD + 4, ND4 = HD / 4;
@@ -332,8 +331,7 @@ __global__ void __launch_bounds__(256) k_ab_linhas(ArgsTras A) {
     __shared__ int red[8];
     __shared__ int sl_s[TI];
     const int tid = threadIdx.x, ty = tid >> 5, lane = tid & 31;
-    const int ordem = blockIdx.y * gridDim.x + blockIdx.x;          // heaviest (last) row tiles of all heads first
-    const int bh = ordem % gridDim.y, b = bh / H, h = bh % H, i0 = (gridDim.x - 1 - ordem / gridDim.y) * TI, linha0 = b * T;
+    const int bh = blockIdx.x, b = bh / H, h = bh % H, i0 = (gridDim.y - 1 - blockIdx.y) * TI, linha0 = b * T;      // heaviest (last) row tiles of all heads first
     int* est = A.est + bh * N_EST;
     const int emg = max_cabeca<HD>(A.goE, D / blk, blk, linha0, T, h * HD, red, tid);
     const int emv = max_cabeca<HD>(A.qE, 3 * D / blk, blk, linha0, T, 2 * D + h * HD, red, tid);
@@ -457,7 +455,7 @@ __global__ void __launch_bounds__(256) k_ab_linhas(ArgsTras A) {
     }
 }
 
-// key tiles: gk[j] = sum_i dS'[i][j] q[i], gv[j] = sum_i P[i][j] dO[i].   grid (T/32, Bt*H)
+// key tiles: gk[j] = sum_i dS'[i][j] q[i], gv[j] = sum_i P[i][j] dO[i].   grid (Bt*H, T/32)
 template <int HD>
 __global__ void __launch_bounds__(256, 2) k_ab_colunas(ArgsTras A) {
     constexpr int PK = HD + 4, ND4 = HD / 4, CP = TJ + 4;
@@ -470,8 +468,7 @@ __global__ void __launch_bounds__(256, 2) k_ab_colunas(ArgsTras A) {
     int* p_c = ds_c + TI * CP;        // [32][132] P of the chunk
     __shared__ int red[8];
     const int tid = threadIdx.x, ty = tid >> 5, lane = tid & 31;
-    const int ordem = blockIdx.y * gridDim.x + blockIdx.x;          // heaviest (first) key tiles of all heads first
-    const int bh = ordem % gridDim.y, b = bh / H, h = bh % H, j0 = (ordem / gridDim.y) * TI, linha0 = b * T;
+    const int bh = blockIdx.x, b = bh / H, h = bh % H, j0 = blockIdx.y * TI, linha0 = b * T;      // heaviest (first) key tiles of all heads first
     const int* est = A.est + bh * N_EST;
     const int emg = max_cabeca<HD>(A.goE, D / blk, blk, linha0, T, h * HD, red, tid);
     const int emq = max_cabeca<HD>(A.qE, 3 * D / blk, blk, linha0, T, h * HD, red, tid);
@@ -632,7 +629,7 @@ static int atencao_frente(int blk, const int8_t* qm, const int8_t* qE, int* Oacc
                           int kid, cudaStream_t st) {
     int hd, lg2;
     if (!at_valido(blk, Bt, T, H, D, &hd, &lg2)) return (int)cudaErrorInvalidValue;
-    const dim3 grade(T / at::TI, Bt * H);
+    const dim3 grade(Bt * H, T / at::TI);
     const size_t sm = at::smem_frente(hd, T);
     cudaError_t c;
 #define JT_F(HD)                                                                                              \
@@ -652,7 +649,7 @@ static int atencao_tras_ws(int blk, const int8_t* gom, const int8_t* goE, const 
                       T, H, D, GA, blk, limite, kid};
     cudaError_t c = cudaMemsetAsync(ws, 0, (size_t)BH * at::N_EST * sizeof(int), st);
     if (c != cudaSuccess) return (int)c;
-    const dim3 grade(T / at::TI, BH);
+    const dim3 grade(BH, T / at::TI);
 #define JT_B(HD)                                                                                                          \
     {                                                                                                                     \
         if (limite) at::k_lim<HD><<<BH, 256, 0, st>>>(A);                                                                 \

@@ -44,6 +44,7 @@ using namespace tc;
 constexpr int NI = 64, TJ = 128;         // queries (or keys) of a tile, keys (or queries) of a window
 constexpr int NTA = 256;                 // threads: 4 lane quarters x 2 halves of 32 columns
 constexpr int SB = 2 * NI;               // columns of a score buffer in tensor memory: hi | lo
+constexpr int GY = 65535;                // limit of a grid's y: heads beyond go to further layers of z
 constexpr uint32_t idesc(int n, bool b_sem_sinal) {       // kind::i8, D = s32, A = s8, B = s8 or u8, both K-major, M = 128
     return (2u << 4) | (1u << 7) | ((b_sem_sinal ? 0u : 1u) << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
@@ -154,7 +155,7 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
     return r;
 }
 
-// grid (pieces of 128 tokens, sequences x groups of 64 / hd heads, 3 or 4), 256 threads: 128 tokens of 64 columns - one head of 64, four
+// grid (pieces of 128 tokens, sequences x groups of 64 / hd heads (GY to a layer), layers x 3 or 4 tensors), 256 threads: 128 tokens of 64 columns - one head of 64, four
 // of 16 or sixteen of 4 - of one tensor.  The pieces of a sequence are a cluster (at most 8), which exchanges the maximum exponents: reading a
 // sequence's exponents in every block was half of the traffic to the cache.  The bound of a plain version (one element at a time in integers, digit bytes stored one by
 // one) was instruction issue, three times the memory time.  So: a thread takes 4 tokens x 8 columns; pairs of elements in f32x2 (a byte
@@ -163,9 +164,9 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
 // 16-byte pieces swapped by the column group, without bank conflicts.
 // 16 x 1024 tokens, forward + backward: 16 heads of 64 218 -> 175 us, 16 heads of 16 196 -> 57 us.
 template <int hd, bool PLANO, bool DIG, bool TRA, bool NRM>
-__device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint16_t* dg, int8_t* dt, int* red, uint32_t* tr) {
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, z = blockIdx.z, hpc = 64 / hd, gh = (A.H + hpc - 1) / hpc;
-    const int b = blockIdx.y / gh, h0 = blockIdx.y % gh * hpc;     // first head of the group
+__device__ __forceinline__ void prep_corpo(const ArgsPrep& A, int z, int grupo, uint16_t* dp, uint16_t* dg, int8_t* dt, int* red, uint32_t* tr) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, hpc = 64 / hd, gh = (A.H + hpc - 1) / hpc;
+    const int b = grupo / gh, h0 = grupo % gh * hpc;               // first head of the group
     const int T = A.T, D = A.D, blk = A.blk, linha0 = b * T;
     const int8_t* m = z == 3 ? A.gm : A.qm;
     const int8_t* E = z == 3 ? A.gE : A.qE;
@@ -316,20 +317,21 @@ template <int hd>
 __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
     __shared__ int red[32 + 2 * 8 * 8];
     __shared__ __align__(16) uint32_t tr[128 * 32];
-    const int z = blockIdx.z;
+    const int nz = A.nrm ? 3 : 4, z = blockIdx.z % nz, grupo = blockIdx.y + blockIdx.z / nz * GY, hpc = 64 / hd;
+    if (grupo >= A.BH / A.H * ((A.H + hpc - 1) / hpc)) return;     // (all pieces of a sequence: the whole cluster)
     uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
     uint16_t* dg = z == 0 ? A.dig[0] : z == 1 ? A.dig[1] : z == 2 ? A.dig[2] : A.dig[3];
     int8_t* dt = z == 0 ? A.tra[0] : z == 1 ? A.tra[1] : z == 2 ? A.tra[2] : A.tra[3];
     pdl_espera();
     pdl_solta();
     if (A.nrm) {                                                   // forward: q digits, k plain, v transposed
-        if (dg) prep_corpo<hd, false, true, false, true>(A, dp, dg, dt, red, tr);
-        else if (dp) prep_corpo<hd, true, false, false, true>(A, dp, dg, dt, red, tr);
-        else prep_corpo<hd, false, false, true, false>(A, dp, dg, dt, red, tr);
+        if (dg) prep_corpo<hd, false, true, false, true>(A, z, grupo, dp, dg, dt, red, tr);
+        else if (dp) prep_corpo<hd, true, false, false, true>(A, z, grupo, dp, dg, dt, red, tr);
+        else prep_corpo<hd, false, false, true, false>(A, z, grupo, dp, dg, dt, red, tr);
     } else {                                                       // backward: q, k transposed, v plain, dO digits and transposed
-        if (dg) prep_corpo<hd, false, true, true, false>(A, dp, dg, dt, red, tr);
-        else if (dp) prep_corpo<hd, true, false, false, false>(A, dp, dg, dt, red, tr);
-        else prep_corpo<hd, false, false, true, false>(A, dp, dg, dt, red, tr);
+        if (dg) prep_corpo<hd, false, true, true, false>(A, z, grupo, dp, dg, dt, red, tr);
+        else if (dp) prep_corpo<hd, true, false, false, false>(A, z, grupo, dp, dg, dt, red, tr);
+        else prep_corpo<hd, false, false, true, false>(A, z, grupo, dp, dg, dt, red, tr);
     }
 }
 
@@ -449,6 +451,8 @@ constexpr size_t SM_FRENTE = 1024 + FR_BAR + 128 + (6 * NI + 2) * 4;
 
 __global__ void __launch_bounds__(NTA, 3) k_at_frente(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
                                                       const __grid_constant__ CUtensorMap mVt, const ArgsFrente A) {
+    const int bh = blockIdx.y + blockIdx.z * GY;
+    if (bh >= A.BH) return;
     extern __shared__ unsigned char bruto[];
     enum { B_Q = 0, B_K = 1, B_V = 2, B_S = 3, B_O = 4 };
     Base S = comeca(bruto, FR_BAR, 5);
@@ -458,7 +462,7 @@ __global__ void __launch_bounds__(NTA, 3) k_at_frente(const __grid_constant__ CU
     int* n_s = i_s + NI;                                           // [2] windows needed, per 32 queries
     const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), lt = 32 * quarto + lane;
-    const int tile = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y, b = bh / H, h = bh % H, i0 = tile * NI, linha0 = b * T;
+    const int tile = gridDim.x - 1 - blockIdx.x, b = bh / H, h = bh % H, i0 = tile * NI, linha0 = b * T;
     const int gira = (tile + bh) & 3, kq = (quarto + gira) & 3, jl = 32 * kq + lane;      // this warp's keys of a window, this thread's key
     const int j00 = i0 + NI - TJ;                                  // first key of the first window (may lie before the sequence: such rows are masked)
     pdl_espera();
@@ -791,6 +795,8 @@ __global__ void __launch_bounds__(NTA, 4) k_ab_max(const __grid_constant__ CUten
 constexpr uint32_t SO_V = 2 * TILE_N, SO_BAR = SO_V + TILE_A;
 constexpr size_t SM_SOMA = 1024 + SO_BAR + 128 + 5 * NI * 4;
 __global__ void __launch_bounds__(NTA, 3) k_ab_soma(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
+    const int bh = blockIdx.y + blockIdx.z * GY;
+    if (bh >= A.BH) return;
     extern __shared__ unsigned char bruto[];
     __shared__ int red[NTA / 32];
     enum { B_G = 0, B_V = 1, B_S = 2 };
@@ -799,7 +805,7 @@ __global__ void __launch_bounds__(NTA, 3) k_ab_soma(const __grid_constant__ CUte
     int* r_s = reinterpret_cast<int*>(S.smem + SO_BAR + 128);      // [4 lane quarters][64] partial sums
     int* sl_s = r_s + 4 * NI;                                      // [64]
     const int T = A.T, kid = A.kid, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2);
-    const int qt = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y, i0 = qt * NI, j00 = i0 + NI - TJ;
+    const int qt = gridDim.x - 1 - blockIdx.x, i0 = qt * NI, j00 = i0 + NI - TJ;
     const int gira = (qt + bh) & 3, jl = 32 * ((quarto + gira) & 3) + lane;
     const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
     int* est = A.est + bh * at::N_EST;
@@ -892,7 +898,7 @@ __global__ void __launch_bounds__(NTA, 3) k_ab_soma(const __grid_constant__ CUte
     termina(S, SB);
 }
 
-// The output kernel.  Three roles (blockIdx.z): 0 key tiles, gk; 1 query tiles, gq; 2 key tiles, gv.
+// The output kernel.  Three roles (blockIdx.z % 3): 0 key tiles, gk; 1 query tiles, gq; 2 key tiles, gv.
 //   gq, gk: scores (lane = the other side's token in the window, column = the tile's token), dS' as digits into an MMA tile
 //           (hi rows 0..63, lo rows 64..127, 128 bytes of window), then D[digit row of k or q][hi | lo column] += X^T . dS'.
 //   gv:     dO^T . P only, both operands straight from memory.
@@ -1085,14 +1091,15 @@ __device__ __forceinline__ void ab_valor(Base& S, const CUtensorMap& mX, const C
 __global__ void __launch_bounds__(NTA, 3) k_ab_saida(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mGd,
                                                      const __grid_constant__ CUtensorMap mKt, const __grid_constant__ CUtensorMap mQt,
                                                      const __grid_constant__ CUtensorMap mGt, const __grid_constant__ CUtensorMap mP, const ArgsTras A) {
+    const int papel = blockIdx.z % 3, bh = blockIdx.y + blockIdx.z / 3 * GY;
+    if (bh >= A.BH) return;
     extern __shared__ unsigned char bruto[];
     Base S = comeca(bruto, SA_BAR, 5);
     pdl_espera();
     pdl_solta();
-    const int bh = blockIdx.y;
     int colunas = NI;
-    if (blockIdx.z == 0) colunas = ab_saida<true>(S, mV, mGd, mQt, mP, A, bh, blockIdx.x);
-    else if (blockIdx.z == 1) colunas = ab_saida<false>(S, mGd, mV, mKt, mP, A, bh, gridDim.x - 1 - blockIdx.x);
+    if (papel == 0) colunas = ab_saida<true>(S, mV, mGd, mQt, mP, A, bh, blockIdx.x);
+    else if (papel == 1) colunas = ab_saida<false>(S, mGd, mV, mKt, mP, A, bh, gridDim.x - 1 - blockIdx.x);
     else ab_valor(S, mGt, mP, A, bh, blockIdx.x);
     termina(S, colunas);
 }
@@ -1110,9 +1117,12 @@ static bool atc_serve(int blk, int T, int H, int D, int GA, bool tras) {
     return (D == H * 64 || D == H * 16 || (D == H * 4 && T > (tras ? 128 : 256))) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 &&
            (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
 }
+// n (sequences x) heads or groups of heads along y, GY to a layer of z
+static dim3 atc_grade(int x, int n, int papeis) { return dim3(x, n < atc::GY ? n : atc::GY, (n + atc::GY - 1) / atc::GY * papeis); }
 static void atc_prep(const atc::ArgsPrep& A, int Bt, int hd, int z, cudaStream_t st) {
     const int np = (A.T + 127) / 128, hpc = 64 / hd;
-    lanca_cluster(hd == 64 ? atc::k_at_prep<64> : hd == 16 ? atc::k_at_prep<16> : atc::k_at_prep<4>, dim3(np, Bt * ((A.H + hpc - 1) / hpc), z), dim3(256), 0, st, np, A);
+    const dim3 g = atc_grade(np, Bt * ((A.H + hpc - 1) / hpc), z);
+    lanca_cluster(hd == 64 ? atc::k_at_prep<64> : hd == 16 ? atc::k_at_prep<16> : atc::k_at_prep<4>, g, dim3(256), 0, st, np, A);
 }
 
 // Workspace: what the preparation writes.  Forward: head-maximum exponents [BH][4] and the largest squared row norms of q and k per 128 tokens
@@ -1146,7 +1156,7 @@ static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* O
     cudaError_t c = at_smem(atc::k_at_frente, atc::SM_FRENTE);
     if (c != cudaSuccess) return (int)c;
     const atc::ArgsFrente A = {em, nrm, Oacc, Oe, Qm, QE, P, BH, T, H, D, hd, GA, kid};
-    lanca_pdl(atc::k_at_frente, dim3((T + atc::NI - 1) / atc::NI, BH), dim3(atc::NTA), atc::SM_FRENTE, st, mQ, mK, mVt, A);
+    lanca_pdl(atc::k_at_frente, atc_grade((T + atc::NI - 1) / atc::NI, BH, 1), dim3(atc::NTA), atc::SM_FRENTE, st, mQ, mK, mVt, A);
     return (int)cudaGetLastError();
 }
 
@@ -1184,9 +1194,9 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
         lanca_pdl(atc::k_ab_max, dim3(A.blocos_mapa + BH * nt), dim3(atc::NTA), atc::SM_MAX, st, mV128, mGd, A);
     }
     if ((c = at_smem(atc::k_ab_soma, atc::SM_SOMA)) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_soma, dim3(nt, BH), dim3(atc::NTA), atc::SM_SOMA, st, mV, mGd, A);
+    lanca_pdl(atc::k_ab_soma, atc_grade(nt, BH, 1), dim3(atc::NTA), atc::SM_SOMA, st, mV, mGd, A);
     if ((c = at_smem(atc::k_ab_saida, atc::SM_SAIDA)) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_saida, dim3(nt, BH, 3), dim3(atc::NTA), atc::SM_SAIDA, st, mV, mGd, mKt, mQt, mGt, mP, A);
+    lanca_pdl(atc::k_ab_saida, atc_grade(nt, BH, 3), dim3(atc::NTA), atc::SM_SAIDA, st, mV, mGd, mKt, mQt, mGt, mP, A);
     return (int)cudaGetLastError();
 }
 

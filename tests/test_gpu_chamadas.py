@@ -236,3 +236,24 @@ def test_produto_com_espaco_de_128_em_128_bytes(amb, blk):
         assert oc.lib.jt_gemm_ws(*p, *(ctypes.c_int(v) for v in (M, N, K, 0, 0))) == 0
         torch.cuda.synchronize()
         compara(f"workspace at {desl}", C, ref)
+
+
+@pytest.mark.parametrize("via,hd,H", [(0, 16, 16), (1, 16, 16), (0, 64, 16)])
+def test_atencao_com_mais_de_65535_cabecas(amb, via, hd, H):
+    """(Sequences x heads) beyond the limit of a grid's y: 17 sequences repeated 241 times give 241 times what they give alone."""
+    ops, oc, reg = amb
+    reg.vigiar = False
+    n, T = 241, 32
+    qkv, go, _ = _problema(32, 17, T, H, hd)
+    o, P = oc.atencao(qkv, 17, T, H)
+    ref = [*o, P, *oc.atencao_back(go, qkv, P, 17, T, H)]
+    assert 17 * n * H > 65535
+    oc.lib.jt_atencao_via(via)
+    try:
+        big, gobig = tuple(t.repeat(n, 1) for t in qkv), tuple(t.repeat(n, 1) for t in go)
+        o, P = oc.atencao(big, 17 * n, T, H)
+        out = [*o, P, *oc.atencao_back(gobig, big, P, 17 * n, T, H)]
+    finally:
+        oc.lib.jt_atencao_via(0)
+    for i, (a, b) in enumerate(zip(out, ref)):
+        assert bool((a.view(n, *b.shape) == b).all()), f"output {i}"
