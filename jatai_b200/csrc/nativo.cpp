@@ -6,6 +6,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 namespace {
@@ -13,6 +14,20 @@ namespace {
 typedef long long A_;
 
 inline const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// in a catch block: the exception in flight as a Python error of the type that PyTorch's own functions raise for it
+PyObject* erro_python() {
+    try {
+        throw;
+    } catch (const c10::OutOfMemoryError& e) {
+        PyErr_SetString(THPException_OutOfMemoryError, e.what_without_backtrace());
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) {
+        PyErr_SetString(PyExc_RuntimeError, "unknown exception");
+    }
+    return nullptr;
+}
 
 // the two members of a pair that bloco_valido has passed
 inline PyObject* const* par_de_args(PyObject* par) { return &PyTuple_GET_ITEM(par, 0); }
@@ -74,7 +89,7 @@ PyObject* novo_bloco(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     try {
         return par_de(vazio({R, C}, at::kChar, como->device()), vazio({R, C / blk}, at::kChar, como->device()));
-    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    } catch (...) { return erro_python(); }
 }
 PyObject* novo_cru(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor* como = n == 3 ? tensor(args[0]) : nullptr;
@@ -83,7 +98,7 @@ PyObject* novo_cru(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     try {
         return par_de(vazio({R, C}, at::kInt, como->device()), vazio({R, C}, at::kShort, como->device()));
-    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    } catch (...) { return erro_python(); }
 }
 // novo(like, type, d0, d1, ...): "u1" uint8, "i4" int32
 PyObject* novo(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -95,7 +110,7 @@ PyObject* novo(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     try {
         return THPVariable_Wrap(vazio(at::IntArrayRef(d, n - 2), t[0] == 'u' ? at::kByte : at::kInt, como->device()));
-    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    } catch (...) { return erro_python(); }
 }
 
 // espaco_gemm(address of jt_gemm_ws_bytes, address of jt_stream_atual, like, M, N, K, mode) -> workspace tensor, or None where the product
@@ -114,7 +129,7 @@ PyObject* espaco_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (bytes <= 0) Py_RETURN_NONE;
     try {
         return THPVariable_Wrap(vazio({bytes}, at::kByte, como->device()));
-    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    } catch (...) { return erro_python(); }
 }
 
 // Entry points of the library take pointers and ints (long long for element counts) and return an int: every one of them is an integer
@@ -258,7 +273,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_DECREF(r);
         Py_DECREF(r2);
         return dois;
-    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    } catch (...) { return erro_python(); }
 }
 
 // atencao(address of jt_atencao_ws_bytes, of jt_stream_atual, of the entry point with a workspace, of the raw one without, blk, launch list, op,
@@ -337,7 +352,7 @@ PyObject* atencao(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_DECREF(r);
         Py_XDECREF(Po);
         return dois;
-    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    } catch (...) { return erro_python(); }
 }
 
 PyMethodDef metodos[] = {

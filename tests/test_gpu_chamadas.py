@@ -257,3 +257,18 @@ def test_atencao_com_mais_de_65535_cabecas(amb, via, hd, H):
         oc.lib.jt_atencao_via(0)
     for i, (a, b) in enumerate(zip(out, ref)):
         assert bool((a.view(n, *b.shape) == b).all()), f"output {i}"
+
+
+def test_memoria_esgotada_tem_o_tipo_do_alocador(amb, memoria):
+    """Where an output does not fit, every kind of operator raises what PyTorch's allocator raises, and works again once there is room."""
+    ops, oc, reg = amb
+    G = casos.Gen(41, 32)
+    A, B, (qkv, go, forma) = para_gpu(G.bloco(8192, 2048)), para_gpu(G.bloco(2048, 2048)), _problema(32, 64, 128, 8, 64)
+    c = oc.gemm(B, B, cru=True)
+    memoria(1 << 20)
+    for f in (lambda: oc.relu2(A), lambda: oc.gemm(A, B), lambda: oc.gemm(A, B, cru=True), lambda: oc.gemm_relu2(A, B), lambda: oc.quant(c),
+              lambda: oc.atencao(qkv, *forma), lambda: oc.atencao_quant(qkv, *forma), lambda: oc.rms(A)):
+        with pytest.raises(torch.OutOfMemoryError):
+            f()
+    torch.cuda.set_per_process_memory_fraction(1.0)
+    compara("relu2", oc.relu2(B), spec.Spec(32).relu2(B))
