@@ -73,6 +73,13 @@ PyObject* cru(PyObject*, PyObject* par) {
 
 at::Tensor vazio(at::IntArrayRef forma, at::ScalarType tipo, const at::Device& dev) { return at::detail::empty_cuda(forma, tipo, dev, c10::nullopt); }      // at::empty without the dispatcher
 
+// a workspace; undefined where there is no memory for it (the library then takes the kernels that need none)
+at::Tensor espaco(int64_t bytes, const at::Device& dev) {
+    try {
+        return vazio({bytes}, at::kByte, dev);
+    } catch (const c10::OutOfMemoryError&) { return at::Tensor(); }
+}
+
 PyObject* par_de(at::Tensor a, at::Tensor b) {
     PyObject* r = PyTuple_New(2);
     if (!r) return nullptr;
@@ -115,7 +122,8 @@ PyObject* novo(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // espaco_gemm(address of jt_gemm_ws_bytes, address of jt_stream_atual, like, M, N, K, mode) -> workspace tensor, or None where the product
 // wants none.  The workspace goes back to PyTorch's allocator right after the launch, which is safe only where the library launches on the
-// stream the allocator orders it by: on any other stream there is none, and the library takes the kernel that needs none.
+// stream the allocator orders it by: on any other stream there is none, as where there is no memory for it, and the library takes the kernel
+// that needs none.
 PyObject* espaco_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor* como = n == 7 ? tensor(args[2]) : nullptr;
     if (!como) { PyErr_SetString(PyExc_TypeError, "espaco_gemm(function, function, tensor, M, N, K, mode)"); return nullptr; }
@@ -128,7 +136,9 @@ PyObject* espaco_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const long long bytes = reinterpret_cast<long long (*)(int, int, int, int)>(fb)(d[0], d[1], d[2], d[3]);
     if (bytes <= 0) Py_RETURN_NONE;
     try {
-        return THPVariable_Wrap(vazio({bytes}, at::kByte, como->device()));
+        const at::Tensor ws = espaco(bytes, como->device());
+        if (!ws.defined()) Py_RETURN_NONE;
+        return THPVariable_Wrap(ws);
     } catch (...) { return erro_python(); }
 }
 
@@ -249,7 +259,8 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (reinterpret_cast<void* (*)()>(fs)() == (void*)c10::cuda::getCurrentCUDAStream(dev.index()).stream())
             bytes = reinterpret_cast<long long (*)(int, int, int, int)>(fb)((int)M, (int)N, (int)K, modo);
         int i = 14;                                                // (12, 13: no external row maxima)
-        if (bytes > 0) { ws = vazio({(int64_t)bytes}, at::kByte, dev); p[i++] = (A_)ws.data_ptr(); }
+        if (bytes > 0) ws = espaco(bytes, dev);
+        if (ws.defined()) p[i++] = (A_)ws.data_ptr();
         p[i++] = M; p[i++] = N; p[i++] = K; p[i++] = modo;
         PyObject *ent = PyDict_New(), *forma = Py_BuildValue("(LL)", (long long)M, (long long)N);
         if (!ent || !forma) { Py_XDECREF(ent); Py_XDECREF(forma); return nullptr; }
@@ -263,7 +274,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_DECREF(forma);
         if (kid < 0) return nullptr;
         p[i++] = (A_)kid;
-        const int rc = chama(bytes > 0 ? fw : fe, p, i);
+        const int rc = chama(ws.defined() ? fw : fe, p, i);
         if (rc) return PyLong_FromLong(rc);
         PyObject* r = par_de(std::move(m1), std::move(e1));
         if (!r || !duas) return r;
@@ -309,26 +320,21 @@ PyObject* atencao(PyObject*, PyObject* const* args, Py_ssize_t n) {
         m = vazio({M, C}, blocos_ ? at::kChar : at::kInt, dev);
         e = vazio({M, blocos_ ? C / blk : C}, blocos_ ? at::kChar : at::kShort, dev);
         if (!tras) P = vazio({Bt * H, T, T}, at::kByte, dev);
-        if (bytes > 0) {
-            try {
-                ws = vazio({(int64_t)bytes}, at::kByte, dev);
-            } catch (const c10::OutOfMemoryError&) {
-                if (blocos_) Py_RETURN_NONE;
-                bytes = 0;                                         // the library sees to it
-            }
-        }
+        if (bytes > 0) ws = espaco(bytes, dev);
+        const bool com_ws = ws.defined();
+        if (!com_ws && blocos_) Py_RETURN_NONE;
         A_ p[20];
         int i = 0;
         if (tras) { p[i++] = pg; p[i++] = (A_)tensor(go[1])->data_ptr(); }
         p[i++] = (A_)q0.data_ptr();
         p[i++] = (A_)q1.data_ptr();
         if (tras) p[i++] = pP;
-        if (bytes > 0 && blocos_) { p[i++] = 0; p[i++] = 0; }
+        if (com_ws && blocos_) { p[i++] = 0; p[i++] = 0; }
         p[i++] = (A_)m.data_ptr();
         p[i++] = (A_)e.data_ptr();
-        if (bytes > 0 && !blocos_) { p[i++] = 0; p[i++] = 0; }
+        if (com_ws && !blocos_) { p[i++] = 0; p[i++] = 0; }
         if (!tras) p[i++] = (A_)P.data_ptr();
-        if (bytes > 0) p[i++] = (A_)ws.data_ptr();
+        if (com_ws) p[i++] = (A_)ws.data_ptr();
         p[i++] = Bt; p[i++] = T; p[i++] = H; p[i++] = D; p[i++] = GA;
         if (tras) p[i++] = limite;
         PyObject *ent = PyDict_New(), *forma = Py_BuildValue("(LL)", (long long)M, (long long)C);
@@ -343,7 +349,7 @@ PyObject* atencao(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_XDECREF(forma);
         if (kid < 0) return nullptr;
         p[i++] = (A_)kid;
-        const int rc = chama(bytes > 0 ? fw : fp, p, i);
+        const int rc = chama(com_ws ? fw : fp, p, i);
         if (rc) return PyLong_FromLong(rc);
         PyObject* r = par_de(std::move(m), std::move(e));
         if (!r || tras) return r;

@@ -272,3 +272,17 @@ def test_memoria_esgotada_tem_o_tipo_do_alocador(amb, memoria):
             f()
     torch.cuda.set_per_process_memory_fraction(1.0)
     compara("relu2", oc.relu2(B), spec.Spec(32).relu2(B))
+
+
+@pytest.mark.parametrize("externos", [False, True])
+def test_produto_sem_memoria_para_o_espaco(amb, memoria, externos):
+    """A product whose workspace does not fit beside its output runs on the kernels that need none, with the same bits."""
+    ops, oc, reg = amb
+    G = casos.Gen(43, 32)
+    A, B = para_gpu(G.bloco(4096, 8192, espalha=4)), para_gpu(G.bloco(2048, 8192, espalha=4))
+    kw = dict(RA=oc.max_linha(A), RB=oc.max_linha(B)) if externos else {}
+    ref = oc.gemm(A, B, **kw)
+    assert oc.lib.jt_gemm_ws_bytes(4096, 2048, 8192, 0) > 64 << 20
+    memoria(64 << 20)
+    out = oc.gemm(A, B, **kw)
+    compara("gemm", out, ref)
