@@ -44,7 +44,7 @@ using namespace tc;
 constexpr int NI = 64, TJ = 128;         // queries (or keys) of a tile, keys (or queries) of a window
 constexpr int NTA = 256;                 // threads: 4 lane quarters x 2 halves of 32 columns
 constexpr int SB = 2 * NI;               // columns of a score buffer in tensor memory: hi | lo
-constexpr int GY = 65535;                // limit of a grid's y: heads beyond go to further layers of z
+constexpr int GY = 65535;                // limit of a grid's y: heads beyond go to further launches (y0 = the first head of one)
 constexpr uint32_t idesc(int n, bool b_sem_sinal) {       // kind::i8, D = s32, A = s8, B = s8 or u8, both K-major, M = 128
     return (2u << 4) | (1u << 7) | ((b_sem_sinal ? 0u : 1u) << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
@@ -148,6 +148,7 @@ struct ArgsPrep {
     int* est;                   // backward: the statistics slots [BH][N_EST] to clear (nullptr in the forward)
     int* nrm;                   // forward: [BH][2][ceil(T/128)] largest sum of squares of an aligned row of q (0) / k (1) per 128 tokens
     int BH, T, H, D, GA, blk;
+    int y0;                     // first group of this launch
 };
 __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats that halves hold exactly
     uint32_t r;
@@ -155,7 +156,7 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
     return r;
 }
 
-// grid (pieces of 128 tokens, sequences x groups of 64 / hd heads (GY to a layer), layers x 3 or 4 tensors), 256 threads: 128 tokens of 64 columns - one head of 64, four
+// grid (pieces of 128 tokens, sequences x groups of 64 / hd heads, 3 or 4), 256 threads: 128 tokens of 64 columns - one head of 64, four
 // of 16 or sixteen of 4 - of one tensor.  The pieces of a sequence are a cluster (at most 8), which exchanges the maximum exponents: reading a
 // sequence's exponents in every block was half of the traffic to the cache.  The bound of a plain version (one element at a time in integers, digit bytes stored one by
 // one) was instruction issue, three times the memory time.  So: a thread takes 4 tokens x 8 columns; pairs of elements in f32x2 (a byte
@@ -164,8 +165,9 @@ __device__ __forceinline__ uint32_t par_h(uint64_t x) {            // two floats
 // 16-byte pieces swapped by the column group, without bank conflicts.
 // 16 x 1024 tokens, forward + backward: 16 heads of 64 218 -> 175 us, 16 heads of 16 196 -> 57 us.
 template <int hd, bool PLANO, bool DIG, bool TRA, bool NRM>
-__device__ __forceinline__ void prep_corpo(const ArgsPrep& A, int z, int grupo, uint16_t* dp, uint16_t* dg, int8_t* dt, int* red, uint32_t* tr) {
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, hpc = 64 / hd, gh = (A.H + hpc - 1) / hpc;
+__device__ __forceinline__ void prep_corpo(const ArgsPrep& A, uint16_t* dp, uint16_t* dg, int8_t* dt, int* red, uint32_t* tr) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, z = blockIdx.z, hpc = 64 / hd, gh = (A.H + hpc - 1) / hpc;
+    const unsigned grupo = blockIdx.y + A.y0;
     const int b = grupo / gh, h0 = grupo % gh * hpc;               // first head of the group
     const int T = A.T, D = A.D, blk = A.blk, linha0 = b * T;
     const int8_t* m = z == 3 ? A.gm : A.qm;
@@ -317,21 +319,20 @@ template <int hd>
 __global__ void __launch_bounds__(256, 4) k_at_prep(const ArgsPrep A) {
     __shared__ int red[32 + 2 * 8 * 8];
     __shared__ __align__(16) uint32_t tr[128 * 32];
-    const int nz = A.nrm ? 3 : 4, z = blockIdx.z % nz, grupo = blockIdx.y + blockIdx.z / nz * GY, hpc = 64 / hd;
-    if (grupo >= A.BH / A.H * ((A.H + hpc - 1) / hpc)) return;     // (all pieces of a sequence: the whole cluster)
+    const int z = blockIdx.z;
     uint16_t* dp = z == 0 ? A.plano[0] : z == 1 ? A.plano[1] : z == 2 ? A.plano[2] : A.plano[3];
     uint16_t* dg = z == 0 ? A.dig[0] : z == 1 ? A.dig[1] : z == 2 ? A.dig[2] : A.dig[3];
     int8_t* dt = z == 0 ? A.tra[0] : z == 1 ? A.tra[1] : z == 2 ? A.tra[2] : A.tra[3];
     pdl_espera();
     pdl_solta();
     if (A.nrm) {                                                   // forward: q digits, k plain, v transposed
-        if (dg) prep_corpo<hd, false, true, false, true>(A, z, grupo, dp, dg, dt, red, tr);
-        else if (dp) prep_corpo<hd, true, false, false, true>(A, z, grupo, dp, dg, dt, red, tr);
-        else prep_corpo<hd, false, false, true, false>(A, z, grupo, dp, dg, dt, red, tr);
+        if (dg) prep_corpo<hd, false, true, false, true>(A, dp, dg, dt, red, tr);
+        else if (dp) prep_corpo<hd, true, false, false, true>(A, dp, dg, dt, red, tr);
+        else prep_corpo<hd, false, false, true, false>(A, dp, dg, dt, red, tr);
     } else {                                                       // backward: q, k transposed, v plain, dO digits and transposed
-        if (dg) prep_corpo<hd, false, true, true, false>(A, z, grupo, dp, dg, dt, red, tr);
-        else if (dp) prep_corpo<hd, true, false, false, false>(A, z, grupo, dp, dg, dt, red, tr);
-        else prep_corpo<hd, false, false, true, false>(A, z, grupo, dp, dg, dt, red, tr);
+        if (dg) prep_corpo<hd, false, true, true, false>(A, dp, dg, dt, red, tr);
+        else if (dp) prep_corpo<hd, true, false, false, false>(A, dp, dg, dt, red, tr);
+        else prep_corpo<hd, false, false, true, false>(A, dp, dg, dt, red, tr);
     }
 }
 
@@ -445,14 +446,13 @@ struct ArgsFrente {
     const int* em; const int* nrm;
     int* Oacc; int16_t* Oe; int8_t* Qm; int8_t* QE; uint8_t* P;   // Qm / QE: block output (head dimension 64, block length 32) instead of the raw one
     int BH, T, H, D, hd, GA, kid;
+    int y0;                                                       // first head of this launch
 };
 constexpr uint32_t FR_K = 2 * TILE_N, FR_V = FR_K + TILE_A, FR_P = FR_V + TILE_A, FR_BAR = FR_P + TILE_N;
 constexpr size_t SM_FRENTE = 1024 + FR_BAR + 128 + (6 * NI + 2) * 4;
 
 __global__ void __launch_bounds__(NTA, 3) k_at_frente(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
                                                       const __grid_constant__ CUtensorMap mVt, const ArgsFrente A) {
-    const int bh = blockIdx.y + blockIdx.z * GY;
-    if (bh >= A.BH) return;
     extern __shared__ unsigned char bruto[];
     enum { B_Q = 0, B_K = 1, B_V = 2, B_S = 3, B_O = 4 };
     Base S = comeca(bruto, FR_BAR, 5);
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(NTA, 3) k_at_frente(const __grid_constant__ CU
     int* n_s = i_s + NI;                                           // [2] windows needed, per 32 queries
     const int T = A.T, H = A.H, D = A.D, GA = A.GA, kid = A.kid, hd = A.hd;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2), lt = 32 * quarto + lane;
-    const int tile = gridDim.x - 1 - blockIdx.x, b = bh / H, h = bh % H, i0 = tile * NI, linha0 = b * T;
+    const int tile = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y + A.y0, b = bh / H, h = bh % H, i0 = tile * NI, linha0 = b * T;
     const int gira = (tile + bh) & 3, kq = (quarto + gira) & 3, jl = 32 * kq + lane;      // this warp's keys of a window, this thread's key
     const int j00 = i0 + NI - TJ;                                  // first key of the first window (may lie before the sequence: such rows are masked)
     pdl_espera();
@@ -670,6 +670,7 @@ struct ArgsTras {
     int* zm;                                                                          // [BH][16]: per 64 keys, bit qt = P may have a non-zero among queries 64 qt .. 64 qt + 63
     int8_t* Gm; int8_t* GE;                                                           // block output [M, 3D] instead of the raw one, or nullptr
     int BH, T, H, D, hd, GA, limite, kid, blocos_mapa;
+    int y0;                                                                           // first head of this launch (k_ab_soma, k_ab_saida)
 };
 // The windows of a query tile / of a key tile in which stored P may be non-zero: everywhere else dS and P contribute nothing.  The first
 // window always counts; the bounded variant takes maxima over everything and keeps them all.
@@ -795,8 +796,6 @@ __global__ void __launch_bounds__(NTA, 4) k_ab_max(const __grid_constant__ CUten
 constexpr uint32_t SO_V = 2 * TILE_N, SO_BAR = SO_V + TILE_A;
 constexpr size_t SM_SOMA = 1024 + SO_BAR + 128 + 5 * NI * 4;
 __global__ void __launch_bounds__(NTA, 3) k_ab_soma(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mG, const ArgsTras A) {
-    const int bh = blockIdx.y + blockIdx.z * GY;
-    if (bh >= A.BH) return;
     extern __shared__ unsigned char bruto[];
     __shared__ int red[NTA / 32];
     enum { B_G = 0, B_V = 1, B_S = 2 };
@@ -805,7 +804,7 @@ __global__ void __launch_bounds__(NTA, 3) k_ab_soma(const __grid_constant__ CUte
     int* r_s = reinterpret_cast<int*>(S.smem + SO_BAR + 128);      // [4 lane quarters][64] partial sums
     int* sl_s = r_s + 4 * NI;                                      // [64]
     const int T = A.T, kid = A.kid, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, quarto = wid & 3, q0 = 32 * (wid >> 2);
-    const int qt = gridDim.x - 1 - blockIdx.x, i0 = qt * NI, j00 = i0 + NI - TJ;
+    const int qt = gridDim.x - 1 - blockIdx.x, bh = blockIdx.y + A.y0, i0 = qt * NI, j00 = i0 + NI - TJ;
     const int gira = (qt + bh) & 3, jl = 32 * ((quarto + gira) & 3) + lane;
     const uint32_t t_lane = S.tmem + ((uint32_t)(32 * quarto) << 16);
     int* est = A.est + bh * at::N_EST;
@@ -898,7 +897,7 @@ __global__ void __launch_bounds__(NTA, 3) k_ab_soma(const __grid_constant__ CUte
     termina(S, SB);
 }
 
-// The output kernel.  Three roles (blockIdx.z % 3): 0 key tiles, gk; 1 query tiles, gq; 2 key tiles, gv.
+// The output kernel.  Three roles (blockIdx.z): 0 key tiles, gk; 1 query tiles, gq; 2 key tiles, gv.
 //   gq, gk: scores (lane = the other side's token in the window, column = the tile's token), dS' as digits into an MMA tile
 //           (hi rows 0..63, lo rows 64..127, 128 bytes of window), then D[digit row of k or q][hi | lo column] += X^T . dS'.
 //   gv:     dO^T . P only, both operands straight from memory.
@@ -1091,15 +1090,14 @@ __device__ __forceinline__ void ab_valor(Base& S, const CUtensorMap& mX, const C
 __global__ void __launch_bounds__(NTA, 3) k_ab_saida(const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mGd,
                                                      const __grid_constant__ CUtensorMap mKt, const __grid_constant__ CUtensorMap mQt,
                                                      const __grid_constant__ CUtensorMap mGt, const __grid_constant__ CUtensorMap mP, const ArgsTras A) {
-    const int papel = blockIdx.z % 3, bh = blockIdx.y + blockIdx.z / 3 * GY;
-    if (bh >= A.BH) return;
     extern __shared__ unsigned char bruto[];
     Base S = comeca(bruto, SA_BAR, 5);
     pdl_espera();
     pdl_solta();
+    const int bh = blockIdx.y + A.y0;
     int colunas = NI;
-    if (papel == 0) colunas = ab_saida<true>(S, mV, mGd, mQt, mP, A, bh, blockIdx.x);
-    else if (papel == 1) colunas = ab_saida<false>(S, mGd, mV, mKt, mP, A, bh, gridDim.x - 1 - blockIdx.x);
+    if (blockIdx.z == 0) colunas = ab_saida<true>(S, mV, mGd, mQt, mP, A, bh, blockIdx.x);
+    else if (blockIdx.z == 1) colunas = ab_saida<false>(S, mGd, mV, mKt, mP, A, bh, gridDim.x - 1 - blockIdx.x);
     else ab_valor(S, mGt, mP, A, bh, blockIdx.x);
     termina(S, colunas);
 }
@@ -1117,12 +1115,17 @@ static bool atc_serve(int blk, int T, int H, int D, int GA, bool tras) {
     return (D == H * 64 || D == H * 16 || (D == H * 4 && T > (tras ? 128 : 256))) && T % 32 == 0 && T >= 32 && T <= 1024 && D % blk == 0 &&
            (blk == 32 || blk == 128) && GA >= 0 && GA <= 4;
 }
-// n (sequences x) heads or groups of heads along y, GY to a layer of z
-static dim3 atc_grade(int x, int n, int papeis) { return dim3(x, n < atc::GY ? n : atc::GY, (n + atc::GY - 1) / atc::GY * papeis); }
-static void atc_prep(const atc::ArgsPrep& A, int Bt, int hd, int z, cudaStream_t st) {
+// f(y0, n): one launch for up to GY of the `total` heads (or groups of heads) along a grid's y
+template <typename F>
+static void atc_lancamentos(int total, F f) {
+    for (int y0 = 0; y0 < total; y0 += atc::GY) f(y0, total - y0 < atc::GY ? total - y0 : atc::GY);
+}
+static void atc_prep(atc::ArgsPrep A, int Bt, int hd, int z, cudaStream_t st) {
     const int np = (A.T + 127) / 128, hpc = 64 / hd;
-    const dim3 g = atc_grade(np, Bt * ((A.H + hpc - 1) / hpc), z);
-    lanca_cluster(hd == 64 ? atc::k_at_prep<64> : hd == 16 ? atc::k_at_prep<16> : atc::k_at_prep<4>, g, dim3(256), 0, st, np, A);
+    atc_lancamentos(Bt * ((A.H + hpc - 1) / hpc), [&](int y0, int n) {
+        A.y0 = y0;
+        lanca_cluster(hd == 64 ? atc::k_at_prep<64> : hd == 16 ? atc::k_at_prep<16> : atc::k_at_prep<4>, dim3(np, n, z), dim3(256), 0, st, np, A);
+    });
 }
 
 // Workspace: what the preparation writes.  Forward: head-maximum exponents [BH][4] and the largest squared row norms of q and k per 128 tokens
@@ -1148,15 +1151,18 @@ static int atencao_frente_tc(int blk, const int8_t* qm, const int8_t* qE, int* O
     uint16_t *Qd = reinterpret_cast<uint16_t*>(ws + b_em), *K = reinterpret_cast<uint16_t*>(ws + b_em + 2 * b_lin);
     int8_t* Vt = reinterpret_cast<int8_t*>(ws + b_em + 3 * b_lin);
     atc::ArgsPrep Pp = {qm, qE, nullptr, nullptr, {nullptr, K, nullptr, nullptr}, {Qd, nullptr, nullptr, nullptr}, {nullptr, nullptr, Vt, nullptr},
-                        em, nullptr, nrm, BH, T, H, D, GA, blk};
+                        em, nullptr, nrm, BH, T, H, D, GA, blk, 0};
     atc_prep(Pp, Bt, hd, 3, st);
     CUtensorMap mQ, mK, mVt;
     if (!(faz_mapa_h(&mQ, Qd, 2 * BH * T, 64, 32) && faz_mapa_h(&mK, K, BH * T, 64, 32) && faz_mapa(&mVt, Vt, BH * 128, T, 128)))
         return (int)cudaErrorInvalidValue;
     cudaError_t c = at_smem(atc::k_at_frente, atc::SM_FRENTE);
     if (c != cudaSuccess) return (int)c;
-    const atc::ArgsFrente A = {em, nrm, Oacc, Oe, Qm, QE, P, BH, T, H, D, hd, GA, kid};
-    lanca_pdl(atc::k_at_frente, atc_grade((T + atc::NI - 1) / atc::NI, BH, 1), dim3(atc::NTA), atc::SM_FRENTE, st, mQ, mK, mVt, A);
+    atc::ArgsFrente A = {em, nrm, Oacc, Oe, Qm, QE, P, BH, T, H, D, hd, GA, kid, 0};
+    atc_lancamentos(BH, [&](int y0, int n) {
+        A.y0 = y0;
+        lanca_pdl(atc::k_at_frente, dim3((T + atc::NI - 1) / atc::NI, n), dim3(atc::NTA), atc::SM_FRENTE, st, mQ, mK, mVt, A);
+    });
     return (int)cudaGetLastError();
 }
 
@@ -1174,7 +1180,7 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
     uint16_t *V = (uint16_t*)parte(0), *Gd = (uint16_t*)parte(1);
     int8_t *Qt = (int8_t*)parte(3), *Kt = (int8_t*)parte(4), *Gt = (int8_t*)parte(5);
     atc::ArgsPrep Pp = {qm, qE, gom, goE, {nullptr, nullptr, V, nullptr}, {nullptr, nullptr, nullptr, Gd}, {Qt, Kt, nullptr, Gt},
-                        em, est, nullptr, BH, T, H, D, GA, blk};
+                        em, est, nullptr, BH, T, H, D, GA, blk, 0};
     atc_prep(Pp, Bt, hd, 4, st);
     CUtensorMap mV, mV128, mGd, mKt, mQt, mGt, mP;
     if (!(faz_mapa_h(&mV, V, BH * T, 64, 32) && faz_mapa_h(&mV128, V, BH * T, 64, 128) && faz_mapa_h(&mGd, Gd, 2 * BH * T, 64, 32) &&
@@ -1182,7 +1188,7 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
           faz_mapa(&mP, P, BH * T, T, atc::NI)))
         return (int)cudaErrorInvalidValue;
     // up to two key tiles the first window is all there is: no map
-    const atc::ArgsTras A = {P, Gacc, Ge, est, sl, em, zm, Gm, GE, BH, T, H, D, hd, GA, limite, kid, nt > 2 ? BH * nt : 0};
+    atc::ArgsTras A = {P, Gacc, Ge, est, sl, em, zm, Gm, GE, BH, T, H, D, hd, GA, limite, kid, nt > 2 ? BH * nt : 0, 0};
     cudaError_t c;
     if (limite) {
         at::ArgsTras L = {gom, goE, qm, qE, P, Gacc, Ge, est, sl, nullptr, T, H, D, GA, blk, limite, kid};
@@ -1194,9 +1200,15 @@ static int atencao_tras_tc(int blk, const int8_t* gom, const int8_t* goE, const 
         lanca_pdl(atc::k_ab_max, dim3(A.blocos_mapa + BH * nt), dim3(atc::NTA), atc::SM_MAX, st, mV128, mGd, A);
     }
     if ((c = at_smem(atc::k_ab_soma, atc::SM_SOMA)) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_soma, atc_grade(nt, BH, 1), dim3(atc::NTA), atc::SM_SOMA, st, mV, mGd, A);
+    atc_lancamentos(BH, [&](int y0, int n) {
+        A.y0 = y0;
+        lanca_pdl(atc::k_ab_soma, dim3(nt, n), dim3(atc::NTA), atc::SM_SOMA, st, mV, mGd, A);
+    });
     if ((c = at_smem(atc::k_ab_saida, atc::SM_SAIDA)) != cudaSuccess) return (int)c;
-    lanca_pdl(atc::k_ab_saida, atc_grade(nt, BH, 3), dim3(atc::NTA), atc::SM_SAIDA, st, mV, mGd, mKt, mQt, mGt, mP, A);
+    atc_lancamentos(BH, [&](int y0, int n) {
+        A.y0 = y0;
+        lanca_pdl(atc::k_ab_saida, dim3(nt, n, 3), dim3(atc::NTA), atc::SM_SAIDA, st, mV, mGd, mKt, mQt, mGt, mP, A);
+    });
     return (int)cudaGetLastError();
 }
 
