@@ -600,16 +600,18 @@ static cudaError_t at_smem_ptr(const void* kern, size_t bytes) {
     static int onde[64];                  // the attribute belongs to (kernel, device)
     static size_t quanto[64];
     static int n = 0;
+    static std::mutex trava;              // calls of several threads
     int dev = 0;
     cudaError_t c = cudaGetDevice(&dev);
     if (c != cudaSuccess) return c;
+    std::lock_guard<std::mutex> l(trava);
     int i = 0;
     while (i < n && !(quem[i] == kern && onde[i] == dev)) i++;
     if (i < n && bytes <= quanto[i]) return cudaSuccess;
     c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (c != cudaSuccess) return c;
     if (i == n && n < 64) { quem[n] = kern; onde[n] = dev; n++; }
-    if (i < 64) quanto[i] = bytes;
+    if (i < n) quanto[i] = bytes;
     return cudaSuccess;
 }
 template <typename K>

@@ -145,7 +145,7 @@ PyObject* espaco_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // Entry points of the library take pointers and ints (long long for element counts) and return an int: every one of them is an integer
 // argument of the x86-64 calling convention, passed in a 64-bit register or stack slot of which the callee reads what it declares, so one
 // call through a pointer type with N 64-bit arguments serves every signature with N arguments.
-int chama(void* f, const A_* a, int n) {
+int chama_ja(void* f, const A_* a, int n) {
 #define C_(...) return reinterpret_cast<int (*)(__VA_ARGS__)>(f)
     switch (n) {
         case 1: C_(A_)(a[0]);
@@ -171,6 +171,14 @@ int chama(void* f, const A_* a, int n) {
     }
 #undef C_
     return -1;
+}
+// The call without the interpreter lock, as ctypes makes it: a launch waits while the GPU's queue is full, and other threads go on meanwhile.
+int chama(void* f, const A_* a, int n) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = chama_ja(f, a, n);
+    Py_END_ALLOW_THREADS
+    return rc;
 }
 
 PyObject *S_op, *S_trecho, *S_entradas, *S_forma, *S_A[2], *S_B[2], *S_X[2], *S_qkv[2], *S_go[2], *S_P;

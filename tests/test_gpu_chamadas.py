@@ -2,6 +2,8 @@
 little memory, a first call inside a recording, very many heads.  Everything against the oracle, or against the same operator called
 the plain way."""
 import tempfile
+import threading
+import time
 
 import pytest
 import torch
@@ -286,3 +288,31 @@ def test_produto_sem_memoria_para_o_espaco(amb, memoria, externos):
     memoria(64 << 20)
     out = oc.gemm(A, B, **kw)
     compara("gemm", out, ref)
+
+
+def test_outros_fios_andam_enquanto_um_lancamento_espera(amb):
+    """Launches beyond what the GPU's queue holds wait behind a kernel of about a second; another Python thread runs meanwhile."""
+    ops, oc, reg = amb
+    reg.vigiar = False
+    A = para_gpu(casos.Gen(3, 32).bloco(128, 128))
+    oc.relu2(A)
+    torch.cuda.synchronize()
+    marcas, fim = [], threading.Event()
+
+    def bate():
+        while not fim.is_set():
+            marcas.append(time.perf_counter())
+            time.sleep(0.001)
+
+    fio = threading.Thread(target=bate)
+    fio.start()
+    t0 = time.perf_counter()
+    torch.cuda._sleep(2_000_000_000)
+    for _ in range(4000):
+        oc.relu2(A)
+    dt = time.perf_counter() - t0
+    torch.cuda.synchronize()
+    fim.set()
+    fio.join()
+    assert dt > 0.5, "the launches did not have to wait"
+    assert max(b - a for a, b in zip(marcas, marcas[1:])) < 0.4 * dt
