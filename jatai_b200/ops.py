@@ -143,14 +143,18 @@ class OpsCuda:
         if d is None:
             for n, t in zip(nomes, tensores):
                 self.reg.confere_bloco(n, t)
-            self.reg.falha(f"{nomes}: not block tensors (mantissa and exponent tensors on the GPU, in a tuple)")
+            d = self._nat.blocos(BLK, *(tuple(t) for t in tensores))      # a pair may come in another container than a tuple
+            if d is None:
+                self.reg.falha(f"{nomes}: not block tensors (mantissa and exponent tensors on the GPU)")
         return d
 
     def _cru(self, nome, t):
         d = self._nat.cru(t)
         if d is None:
             self.reg.confere_cru(nome, t)
-            self.reg.falha(f"argument '{nome}' is not a raw tensor of two dimensions")
+            d = self._nat.cru(tuple(t))
+            if d is None:
+                self.reg.falha(f"argument '{nome}' is not a raw tensor of two dimensions")
         return d
 
     # ------------------------------------------------------------------ GEMM family

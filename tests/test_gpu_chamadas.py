@@ -316,3 +316,24 @@ def test_outros_fios_andam_enquanto_um_lancamento_espera(amb):
     fio.join()
     assert dt > 0.5, "the launches did not have to wait"
     assert max(b - a for a, b in zip(marcas, marcas[1:])) < 0.4 * dt
+
+
+def test_pares_em_listas(amb):
+    """A (mantissas, exponents) pair may be a list: every operator gives what it gives for the tuple, and the messages of the checks stay."""
+    from jatai_b200.registro import ErroJatai
+    ops, oc, reg = amb
+    G = casos.Gen(51, 32)
+    A, B, X, W = (para_gpu(G.bloco(256, 256, espalha=4)) for _ in range(4))
+    qkv, go, forma = _problema(32, 2, 64, 2, 64)
+    c, alvo = oc.gemm(A, B, cru=True), torch.randint(0, 256, (256,), device="cuda", dtype=torch.int32)
+    y, cache = oc.rms(A)
+    P = oc.atencao(qkv, *forma)[1]
+    novo = lambda t: tuple(x.clone() for x in t)
+    for f in (lambda k: oc.gemm(k(A), k(B)), lambda k: oc.gemm_soma(k(A), k(B), k(X)), lambda k: oc.gemm_relu2_back(k(A), B, k(X)), lambda k: oc.transpoe(k(A)),
+              lambda k: oc.transpoe2(k(A), k(B)), lambda k: oc.quant(k(c)), lambda k: oc.soma(k(A), B), lambda k: oc.relu2(k(A)), lambda k: oc.rms(k(A)),
+              lambda k: oc.rms_back(k(X), k(y), cache), lambda k: oc.softmax_ce(k(c), alvo), lambda k: oc.momento(k(c), k(novo(X))), lambda k: oc.max_linha(k(A)),
+              lambda k: oc.momento_peso(k(c), k(novo(X)), k(novo(W)), k(novo(B)), 4, True), lambda k: oc.peso(k(novo(W)), k(X), k(novo(B)), 4, True),
+              lambda k: oc.atencao(k(qkv), *forma), lambda k: oc.atencao_back(k(go), k(qkv), P, *forma), lambda k: oc.atencao_quant(k(qkv), *forma)):
+        compara("list", casos.plano(f(list)), casos.plano(f(tuple)))
+    with pytest.raises(ErroJatai, match="argument 'A' is not a valid block tensor"):
+        oc.gemm([A[0], A[1][:1]], B)
