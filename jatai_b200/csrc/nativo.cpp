@@ -6,7 +6,6 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
-#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 namespace {
@@ -15,12 +14,14 @@ typedef long long A_;
 
 inline const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
+PyObject* E_memoria;      // torch.OutOfMemoryError
+
 // in a catch block: the exception in flight as a Python error of the type that PyTorch's own functions raise for it
 PyObject* erro_python() {
     try {
         throw;
     } catch (const c10::OutOfMemoryError& e) {
-        PyErr_SetString(THPException_OutOfMemoryError, e.what_without_backtrace());
+        PyErr_SetString(E_memoria, e.what_without_backtrace());
     } catch (const std::exception& e) {
         PyErr_SetString(PyExc_RuntimeError, e.what());
     } catch (...) {
@@ -385,6 +386,10 @@ PyModuleDef modulo = {PyModuleDef_HEAD_INIT, "_nativo", "host half of the operat
 }  // namespace
 
 PyMODINIT_FUNC PyInit__nativo(void) {
+    PyObject* torch = PyImport_ImportModule("torch");
+    E_memoria = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
+    Py_XDECREF(torch);
+    if (!E_memoria) return nullptr;
     S_op = PyUnicode_InternFromString("op");
     S_trecho = PyUnicode_InternFromString("trecho");
     S_entradas = PyUnicode_InternFromString("entradas");

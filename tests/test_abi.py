@@ -38,3 +38,15 @@ def test_ops_sem_gpu_falha_alto():
     import tempfile
     with pytest.raises(RuntimeError):
         ops.OpsCuda(registro.Registro(tempfile.mkdtemp(), "x", eco=False))
+
+
+def test_modulo_nativo_carrega():
+    """The native half of the launcher loads (every symbol it wants is one PyTorch exports) and refuses what is no tensor."""
+    import pytest
+    from jatai_b200 import build
+    build.build_nativo()
+    import torch
+    from jatai_b200 import _nativo
+    assert _nativo.blocos(32, (torch.zeros(2, 32, dtype=torch.int8), torch.zeros(2, 1, dtype=torch.int8))) is None      # not on a GPU
+    with pytest.raises(TypeError):
+        _nativo.novo_cru(1, 2, 3)
