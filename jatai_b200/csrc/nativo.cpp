@@ -53,8 +53,10 @@ PyObject* blocos(PyObject*, PyObject* const* args, Py_ssize_t n) {
     for (Py_ssize_t i = 1; r && i < n; i++) {
         int64_t R, C;
         if (!bloco_valido(args[i], blk, &R, &C)) { Py_DECREF(r); Py_RETURN_NONE; }
-        PyTuple_SET_ITEM(r, 2 * (i - 1), PyLong_FromLongLong(R));
-        PyTuple_SET_ITEM(r, 2 * (i - 1) + 1, PyLong_FromLongLong(C));
+        PyObject *pr = PyLong_FromLongLong(R), *pc = PyLong_FromLongLong(C);
+        PyTuple_SET_ITEM(r, 2 * (i - 1), pr);
+        PyTuple_SET_ITEM(r, 2 * (i - 1) + 1, pc);
+        if (!pr || !pc) { Py_DECREF(r); return nullptr; }
     }
     return r;
 }
@@ -65,11 +67,7 @@ PyObject* cru(PyObject*, PyObject* par) {
     const at::Tensor *a = tensor(PyTuple_GET_ITEM(par, 0)), *e = tensor(PyTuple_GET_ITEM(par, 1));
     if (!a || !e || a->scalar_type() != at::kInt || e->scalar_type() != at::kShort || !a->is_cuda() || !e->is_cuda()) Py_RETURN_NONE;
     if (a->dim() != 2 || a->sizes() != e->sizes() || !a->is_contiguous() || !e->is_contiguous()) Py_RETURN_NONE;
-    PyObject* r = PyTuple_New(2);
-    if (!r) return nullptr;
-    PyTuple_SET_ITEM(r, 0, PyLong_FromLongLong(a->size(0)));
-    PyTuple_SET_ITEM(r, 1, PyLong_FromLongLong(a->size(1)));
-    return r;
+    return Py_BuildValue("(LL)", (long long)a->size(0), (long long)a->size(1));
 }
 
 at::Tensor vazio(at::IntArrayRef forma, at::ScalarType tipo, const at::Device& dev) { return at::detail::empty_cuda(forma, tipo, dev, c10::nullopt); }      // at::empty without the dispatcher
@@ -82,10 +80,10 @@ at::Tensor espaco(int64_t bytes, const at::Device& dev) {
 }
 
 PyObject* par_de(at::Tensor a, at::Tensor b) {
-    PyObject* r = PyTuple_New(2);
-    if (!r) return nullptr;
-    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(a)));
-    PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(std::move(b)));
+    PyObject *pa = THPVariable_Wrap(std::move(a)), *pb = pa ? THPVariable_Wrap(std::move(b)) : nullptr;
+    PyObject* r = pb ? PyTuple_Pack(2, pa, pb) : nullptr;
+    Py_XDECREF(pa);
+    Py_XDECREF(pb);
     return r;
 }
 
@@ -188,14 +186,11 @@ PyObject *S_op, *S_trecho, *S_entradas, *S_forma, *S_A[2], *S_B[2], *S_X[2], *S_
 Py_ssize_t anota(PyObject* lista, PyObject* op, PyObject* trecho, PyObject* entradas, PyObject* forma) {
     PyObject* d = PyDict_New();
     if (!d) return -1;
-    PyDict_SetItem(d, S_op, op);
-    PyDict_SetItem(d, S_trecho, trecho);
-    PyDict_SetItem(d, S_entradas, entradas);
-    PyDict_SetItem(d, S_forma, forma);
     const Py_ssize_t kid = PyList_GET_SIZE(lista);
-    const int falhou = PyList_Append(lista, d);
+    const bool certo = PyDict_SetItem(d, S_op, op) == 0 && PyDict_SetItem(d, S_trecho, trecho) == 0 && PyDict_SetItem(d, S_entradas, entradas) == 0 &&
+                       PyDict_SetItem(d, S_forma, forma) == 0 && PyList_Append(lista, d) == 0;
     Py_DECREF(d);
-    return falhou ? -1 : kid;
+    return certo ? kid : -1;
 }
 
 // lanca(function address, launch list, op, section, names, tensors, ints, output shape) -> (launch id, return code)
@@ -224,7 +219,7 @@ PyObject* lanca(PyObject*, PyObject* const* args, Py_ssize_t n) {
     PyObject* ent = PyDict_New();
     if (!ent) return nullptr;
     for (Py_ssize_t i = 0; i < nn; i++)
-        if (PyTuple_GET_ITEM(nomes, i) != Py_None) PyDict_SetItem(ent, PyTuple_GET_ITEM(nomes, i), PyTuple_GET_ITEM(ts, i));
+        if (PyTuple_GET_ITEM(nomes, i) != Py_None && PyDict_SetItem(ent, PyTuple_GET_ITEM(nomes, i), PyTuple_GET_ITEM(ts, i)) != 0) { Py_DECREF(ent); return nullptr; }
     const Py_ssize_t kid = anota(lista, args[2], args[3], ent, args[7]);
     Py_DECREF(ent);
     if (kid < 0) return nullptr;
@@ -272,15 +267,13 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (ws.defined()) p[i++] = (A_)ws.data_ptr();
         p[i++] = M; p[i++] = N; p[i++] = K; p[i++] = modo;
         PyObject *ent = PyDict_New(), *forma = Py_BuildValue("(LL)", (long long)M, (long long)N);
-        if (!ent || !forma) { Py_XDECREF(ent); Py_XDECREF(forma); return nullptr; }
-        for (int k = 0; k < 2; k++) {
-            PyDict_SetItem(ent, S_A[k], PyTuple_GET_ITEM(args[9], k));
-            PyDict_SetItem(ent, S_B[k], PyTuple_GET_ITEM(args[10], k));
-            if (tem_x) PyDict_SetItem(ent, S_X[k], PyTuple_GET_ITEM(args[11], k));
-        }
-        const Py_ssize_t kid = anota(args[5], args[6], args[7], ent, forma);
-        Py_DECREF(ent);
-        Py_DECREF(forma);
+        bool certo = ent && forma;
+        for (int k = 0; k < 2 && certo; k++)
+            certo = PyDict_SetItem(ent, S_A[k], PyTuple_GET_ITEM(args[9], k)) == 0 && PyDict_SetItem(ent, S_B[k], PyTuple_GET_ITEM(args[10], k)) == 0 &&
+                    (!tem_x || PyDict_SetItem(ent, S_X[k], PyTuple_GET_ITEM(args[11], k)) == 0);
+        const Py_ssize_t kid = certo ? anota(args[5], args[6], args[7], ent, forma) : -1;
+        Py_XDECREF(ent);
+        Py_XDECREF(forma);
         if (kid < 0) return nullptr;
         p[i++] = (A_)kid;
         const int rc = chama(ws.defined() ? fw : fe, p, i);
@@ -390,17 +383,20 @@ PyMODINIT_FUNC PyInit__nativo(void) {
     E_memoria = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
     Py_XDECREF(torch);
     if (!E_memoria) return nullptr;
-    S_op = PyUnicode_InternFromString("op");
-    S_trecho = PyUnicode_InternFromString("trecho");
-    S_entradas = PyUnicode_InternFromString("entradas");
-    S_forma = PyUnicode_InternFromString("forma");
+    bool certo = true;
+    auto nome = [&](PyObject*& d, const char* t) { certo = certo && (d = PyUnicode_InternFromString(t)) != nullptr; };
+    nome(S_op, "op");
+    nome(S_trecho, "trecho");
+    nome(S_entradas, "entradas");
+    nome(S_forma, "forma");
     for (int k = 0; k < 2; k++) {
-        S_A[k] = PyUnicode_InternFromString(k ? "EA" : "A");
-        S_B[k] = PyUnicode_InternFromString(k ? "EB" : "B");
-        S_X[k] = PyUnicode_InternFromString(k ? "XE" : "X");
-        S_qkv[k] = PyUnicode_InternFromString(k ? "qkvE" : "qkv");
-        S_go[k] = PyUnicode_InternFromString(k ? "goE" : "go");
+        nome(S_A[k], k ? "EA" : "A");
+        nome(S_B[k], k ? "EB" : "B");
+        nome(S_X[k], k ? "XE" : "X");
+        nome(S_qkv[k], k ? "qkvE" : "qkv");
+        nome(S_go[k], k ? "goE" : "go");
     }
-    S_P = PyUnicode_InternFromString("P");
+    nome(S_P, "P");
+    if (!certo) return nullptr;
     return PyModule_Create(&modulo);
 }
