@@ -180,24 +180,42 @@ int chama(void* f, const A_* a, int n) {
     return rc;
 }
 
-PyObject *S_op, *S_trecho, *S_entradas, *S_forma, *S_A[2], *S_B[2], *S_X[2], *S_qkv[2], *S_go[2], *S_P;
+PyObject *S_op, *S_trecho, *S_entradas, *S_forma, *S_A[2], *S_B[2], *S_X[2], *S_qkv[2], *S_go[2], *S_P, *S_registra, *S_depois;
 
-// The launch record {op, trecho, entradas, forma} appended to `lista`; its index, or -1 with a Python error set.
-Py_ssize_t anota(PyObject* lista, PyObject* op, PyObject* trecho, PyObject* entradas, PyObject* forma) {
+// The launch record {op, trecho, entradas, forma}: appended to a list - the registry's own - or, of anything else, given to its method
+// registra(op, entradas, forma).  The launch id, or -1 with a Python error set.
+Py_ssize_t anota(PyObject* reg, PyObject* op, PyObject* trecho, PyObject* entradas, PyObject* forma) {
+    if (!PyList_Check(reg)) {
+        PyObject* r = PyObject_CallMethodObjArgs(reg, S_registra, op, entradas, forma, nullptr);
+        const Py_ssize_t kid = r ? PyLong_AsSsize_t(r) : -1;
+        Py_XDECREF(r);
+        if (kid < 0 && !PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "registra gave no launch id");
+        return kid;
+    }
     PyObject* d = PyDict_New();
     if (!d) return -1;
-    const Py_ssize_t kid = PyList_GET_SIZE(lista);
+    const Py_ssize_t kid = PyList_GET_SIZE(reg);
     const bool certo = PyDict_SetItem(d, S_op, op) == 0 && PyDict_SetItem(d, S_trecho, trecho) == 0 && PyDict_SetItem(d, S_entradas, entradas) == 0 &&
-                       PyDict_SetItem(d, S_forma, forma) == 0 && PyList_Append(lista, d) == 0;
+                       PyDict_SetItem(d, S_forma, forma) == 0 && PyList_Append(reg, d) == 0;
     Py_DECREF(d);
     return certo ? kid : -1;
 }
+// The launch has returned `rc`: a list's owner sees to that; anything else is told, depois(launch id, rc).  False with a Python error set.
+bool avisa(PyObject* reg, Py_ssize_t kid, int rc) {
+    if (PyList_Check(reg)) return true;
+    PyObject *k = PyLong_FromSsize_t(kid), *c = PyLong_FromLong(rc);
+    PyObject* r = k && c ? PyObject_CallMethodObjArgs(reg, S_depois, k, c, nullptr) : nullptr;
+    Py_XDECREF(k);
+    Py_XDECREF(c);
+    Py_XDECREF(r);
+    return r != nullptr;
+}
 
-// lanca(function address, launch list, op, section, names, tensors, ints, output shape) -> (launch id, return code)
+// lanca(function address, launch list or registry, op, section, names, tensors, ints, output shape) -> None, or (launch id, return code)
 // Records the launch ({op, trecho, entradas, forma}; `names` name the first tensors, None skips one) and calls function(pointers..., ints...,
 // launch id).  A None tensor is a null pointer.
 PyObject* lanca(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 8 || !PyList_Check(args[1]) || !PyTuple_Check(args[4]) || !PyTuple_Check(args[5]) || !PyTuple_Check(args[6])) {
+    if (n != 8 || !PyTuple_Check(args[4]) || !PyTuple_Check(args[5]) || !PyTuple_Check(args[6])) {
         PyErr_SetString(PyExc_TypeError, "lanca(function, launches, op, section, names, tensors, ints, shape)");
         return nullptr;
     }
@@ -225,15 +243,16 @@ PyObject* lanca(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (kid < 0) return nullptr;
     a[np + ni] = (A_)kid;
     const int rc = chama(f, a, (int)(np + ni + 1));
-    if (rc == 0) Py_RETURN_NONE;
+    if (!avisa(lista, kid, rc)) return nullptr;
+    if (rc == 0 || !PyList_Check(lista)) Py_RETURN_NONE;
     return Py_BuildValue("(ni)", kid, rc);
 }
 
-// gemm(address of jt_gemm_ws_bytes, of jt_stream_atual, of jt_gemm_ws, of jt_gemm_ext, blk, launch list, op, section, mode, A, B, X or None, two
+// gemm(address of jt_gemm_ws_bytes, of jt_stream_atual, of jt_gemm_ws, of jt_gemm_ext, blk, launch list or registry, op, section, mode, A, B, X or None, two
 // outputs) -> the output (pair), or both; None where an argument is not as it should be (nothing was done), the return code where the launch
 // failed.  The whole of a product in one call: checks, outputs, workspace, record, launch.
 PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 13 || !PyList_Check(args[5])) { PyErr_SetString(PyExc_TypeError, "gemm(4 functions, blk, launches, op, section, mode, A, B, X, two)"); return nullptr; }
+    if (n != 13) { PyErr_SetString(PyExc_TypeError, "gemm(4 functions, blk, launches, op, section, mode, A, B, X, two)"); return nullptr; }
     void *fb = PyLong_AsVoidPtr(args[0]), *fs = PyLong_AsVoidPtr(args[1]), *fw = PyLong_AsVoidPtr(args[2]), *fe = PyLong_AsVoidPtr(args[3]);
     const int64_t blk = PyLong_AsLongLong(args[4]);
     const int modo = (int)PyLong_AsLong(args[8]), duas = PyObject_IsTrue(args[12]);
@@ -277,7 +296,8 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (kid < 0) return nullptr;
         p[i++] = (A_)kid;
         const int rc = chama(ws.defined() ? fw : fe, p, i);
-        if (rc) return PyLong_FromLong(rc);
+        if (!avisa(args[5], kid, rc)) return nullptr;
+        if (rc && PyList_Check(args[5])) return PyLong_FromLong(rc);
         PyObject* r = par_de(std::move(m1), std::move(e1));
         if (!r || !duas) return r;
         PyObject* r2 = par_de(std::move(m2), std::move(e2));
@@ -289,12 +309,12 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     } catch (...) { return erro_python(); }
 }
 
-// atencao(address of jt_atencao_ws_bytes, of jt_stream_atual, of the entry point with a workspace, of the raw one without, blk, launch list, op,
+// atencao(address of jt_atencao_ws_bytes, of jt_stream_atual, of the entry point with a workspace, of the raw one without, blk, launch list or registry, op,
 // section, QKV, dO or None, P or None, Bt, T, H, GA, limit, block outputs) -> forward: (output pair, P), backward (dO and P given): the output
 // pair; None where an argument is not as it should be or there is no workspace for block outputs (nothing was done), the return code
 // where the launch failed.  The whole of an attention call: checks, outputs, workspace, record, launch.
 PyObject* atencao(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 17 || !PyList_Check(args[5])) { PyErr_SetString(PyExc_TypeError, "atencao(4 functions, blk, launches, op, section, QKV, dO, P, Bt, T, H, GA, limit, blocks)"); return nullptr; }
+    if (n != 17) { PyErr_SetString(PyExc_TypeError, "atencao(4 functions, blk, launches, op, section, QKV, dO, P, Bt, T, H, GA, limit, blocks)"); return nullptr; }
     void *fb = PyLong_AsVoidPtr(args[0]), *fs = PyLong_AsVoidPtr(args[1]), *fw = PyLong_AsVoidPtr(args[2]), *fp = PyLong_AsVoidPtr(args[3]);
     const int64_t blk = PyLong_AsLongLong(args[4]), Bt = PyLong_AsLongLong(args[11]), T = PyLong_AsLongLong(args[12]), H = PyLong_AsLongLong(args[13]);
     const int GA = (int)PyLong_AsLong(args[14]), limite = (int)PyLong_AsLong(args[15]), blocos_ = PyObject_IsTrue(args[16]);
@@ -352,7 +372,8 @@ PyObject* atencao(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (kid < 0) return nullptr;
         p[i++] = (A_)kid;
         const int rc = chama(com_ws ? fw : fp, p, i);
-        if (rc) return PyLong_FromLong(rc);
+        if (!avisa(args[5], kid, rc)) return nullptr;
+        if (rc && PyList_Check(args[5])) return PyLong_FromLong(rc);
         PyObject* r = par_de(std::move(m), std::move(e));
         if (!r || tras) return r;
         PyObject* Po = THPVariable_Wrap(std::move(P));
@@ -397,6 +418,8 @@ PyMODINIT_FUNC PyInit__nativo(void) {
         nome(S_go[k], k ? "goE" : "go");
     }
     nome(S_P, "P");
+    nome(S_registra, "registra");
+    nome(S_depois, "depois");
     if (!certo) return nullptr;
     return PyModule_Create(&modulo);
 }

@@ -22,6 +22,8 @@ import os
 
 import torch
 
+from . import registro
+
 BLK = 32
 E_ZERO = -127
 GA = 4                     # guard bits of q/k/v/dO aligned inside a head (reference ops.py:20)
@@ -129,12 +131,14 @@ class OpsCuda:
         """Registers the launch and calls the entry point: pointers of `tensores` (None = null), then `inteiros`, then the launch id.
         `nomes` name the first tensors in the launch record (None leaves one out)."""
         reg = self.reg
-        if reg.perfil:
-            reg.cronometra(op)
+        # The native calls append to the launch list of a plain Registro that times nothing; of any other registry they call registra and depois.
+        if reg.perfil or reg.__class__ is not registro.Registro:
+            self._nat.lanca(self._endereco(fn), reg, op, reg.onde(), nomes, tensores, inteiros, forma)
+            return
         r = self._nat.lanca(self._endereco(fn), reg.lancamentos, op, reg.onde(), nomes, tensores, inteiros, forma)
         if r is not None:
             reg.depois(*r)
-        elif reg.perfil or reg.vigiar:
+        elif reg.vigiar:
             reg.depois(len(reg.lancamentos) - 1, 0)
 
     def _blocos(self, nomes, *tensores):
@@ -160,15 +164,16 @@ class OpsCuda:
     # ------------------------------------------------------------------ GEMM family
     def _gemm(self, op, modo, A, B, X=None, duas=False, RA=None, RB=None):
         reg, nat = self.reg, self._nat
-        if RA is None and RB is None and not reg.perfil:
-            r = nat.gemm(*self._ws, *self._ws_gemm, BLK, reg.lancamentos, op, reg.onde(), modo, A, B, X, duas)
+        if RA is None and RB is None:
+            alheio = reg.perfil or reg.__class__ is not registro.Registro
+            r = nat.gemm(*self._ws, *self._ws_gemm, BLK, reg if alheio else reg.lancamentos, op, reg.onde(), modo, A, B, X, duas)
             if r.__class__ is tuple:
-                if reg.vigiar:
+                if reg.vigiar and not alheio:
                     reg.depois(len(reg.lancamentos) - 1, 0)
                 return r
             if r is not None:
                 reg.depois(len(reg.lancamentos) - 1, r)
-        # with external row maxima, timed, for a library with only the reference's entry points - and what is wrong with an argument
+        # with external row maxima, for a library with only the reference's entry points - and what is wrong with an argument
         if X is None:
             M, K, N, Kb = self._blocos(("A", "B"), A, B)
         else:
@@ -341,15 +346,12 @@ class OpsCuda:
         """The call in one piece, workspace included (`entradas`: the entry points with one and, raw outputs only, without), or None: block
         outputs without a workspace, a library with only the reference's entry points - and what is wrong with an argument."""
         reg = self.reg
-        if reg.perfil:
-            reg.cronometra(op)
-        r = self._nat.atencao(*self._ws_at, *entradas, BLK, reg.lancamentos, op, reg.onde(), QKV, GO, P, Bt, T, H, GA, int(ATENCAO_LIMITE), blocos)
-        if r is None:
-            if reg.perfil:
-                reg.eventos.pop()
-        elif r.__class__ is int:
+        alheio = reg.perfil or reg.__class__ is not registro.Registro
+        r = self._nat.atencao(*self._ws_at, *entradas, BLK, reg if alheio else reg.lancamentos, op, reg.onde(), QKV, GO, P, Bt, T, H, GA,
+                              int(ATENCAO_LIMITE), blocos)
+        if r.__class__ is int:
             reg.depois(len(reg.lancamentos) - 1, r)
-        elif reg.perfil or reg.vigiar:
+        elif r is not None and reg.vigiar and not alheio:
             reg.depois(len(reg.lancamentos) - 1, 0)
         return r
 

@@ -337,3 +337,73 @@ def test_pares_em_listas(amb):
         compara("list", casos.plano(f(list)), casos.plano(f(tuple)))
     with pytest.raises(ErroJatai, match="argument 'A' is not a valid block tensor"):
         oc.gemm([A[0], A[1][:1]], B)
+
+
+def _alguns(oc, A, B, c, qkv, forma):
+    """One launch of each way a launch is made: a product, one with external maxima, an attention, an operator of the general launcher."""
+    return [oc.gemm(A, B), oc.gemm(A, B, cru=True, RA=oc.max_linha(A), RB=oc.max_linha(B)), *oc.atencao_quant(qkv, *forma), oc.quant(c)]
+
+
+@pytest.mark.parametrize("perfil", [False, True])
+def test_registro_de_fora(amb, perfil):
+    """The launcher keeps to the registry's protocol: registra before and depois after every launch of a registry that is not the plain one -
+    one derived from it, and one that has only the reference's methods - with the launch id that registra gave."""
+    from jatai_b200 import registro
+    ops, oc0, reg0 = amb
+    G = casos.Gen(61, 32)
+    A, B = para_gpu(G.bloco(256, 256)), para_gpu(G.bloco(256, 256))
+    c = oc0.gemm(A, B, cru=True)
+    qkv, go, forma = _problema(32, 2, 64, 2, 64)
+    ref = _alguns(oc0, A, B, c, qkv, forma)
+
+    class Derivado(registro.Registro):
+        def registra(self, op, ent, forma):
+            self.visto = getattr(self, "visto", []) + [(op, sorted(ent), tuple(forma))]
+            return super().registra(op, ent, forma)
+
+        def depois(self, kid, rc):
+            self.fim = getattr(self, "fim", []) + [(kid, rc)]
+            super().depois(kid, rc)
+
+    class Minimo:
+        """What jatai_cuda/registro.py:66-116 has of it."""
+        vigiar, lib = False, None
+
+        def __init__(self):
+            self.perfil, self.lancamentos, self.visto, self.fim = perfil, [], [], []
+
+        def onde(self):
+            return "-"
+
+        def registra(self, op, ent, forma):
+            self.visto.append((op, sorted(ent), tuple(forma)))
+            return 100 + len(self.visto) - 1
+
+        def depois(self, kid, rc):
+            self.fim.append((kid, rc))
+
+        def novo_passo(self, p):
+            pass
+
+        def confere_bloco(self, nome, t):
+            pass
+
+        def exige(self, c, msg):
+            assert c, msg
+
+    esperado = [("gemm", ["A", "B", "EA", "EB"], (256, 256)), ("max_linha", ["E"], (256, 1)), ("max_linha", ["E"], (256, 1)),
+                ("gemm_cru", ["A", "B", "EA", "EB"], (256, 256)), ("atencao_quant", ["qkv", "qkvE"], (128, 128)), ("quant", ["acc", "e"], (256, 256))]
+    for reg in (Derivado(tempfile.mkdtemp(), "d", perfil=perfil, eco=False, salvar=False), Minimo()):
+        oc = ops.OpsCuda(reg)
+        reg.novo_passo(0)
+        compara(type(reg).__name__, casos.plano(_alguns(oc, A, B, c, qkv, forma)), casos.plano(ref))
+        assert reg.visto == esperado
+        k0 = 0 if isinstance(reg, registro.Registro) else 100
+        assert reg.fim == [(k0 + i, 0) for i in range(6)]
+    if perfil:
+        plano = registro.Registro(tempfile.mkdtemp(), "p", perfil=True, eco=False, salvar=False)
+        oc = ops.OpsCuda(plano)
+        plano.novo_passo(0)
+        _alguns(oc, A, B, c, qkv, forma)
+        plano.fim_passo()
+        assert sorted(plano.tempos) == sorted({e[0] for e in esperado}) and all(v > 0 for v in plano.tempos.values())
