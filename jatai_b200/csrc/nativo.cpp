@@ -420,6 +420,7 @@ PyMODINIT_FUNC PyInit__nativo(void) {
     nome(S_P, "P");
     nome(S_registra, "registra");
     nome(S_depois, "depois");
-    if (!certo) return nullptr;
-    return PyModule_Create(&modulo);
+    PyObject* m = certo ? PyModule_Create(&modulo) : nullptr;
+    if (m && PyModule_AddStringConstant(m, "MARCA", JT_MARCA) != 0) { Py_DECREF(m); return nullptr; }      // the versions it was built against
+    return m;
 }

@@ -69,6 +69,19 @@ def carrega_biblioteca(caminho=None):
     return lib
 
 
+def carrega_nativo():
+    """The native half of the launcher.  Raises if it has not been built, or was built against another PyTorch or Python."""
+    from . import build
+    como = "build it with `python -m jatai_b200.build`"
+    try:
+        from . import _nativo
+    except ImportError as e:
+        raise RuntimeError(f"{build.SAIDA_NATIVO} does not load ({e}): {como}") from e
+    if _nativo.MARCA != build._marca():
+        raise RuntimeError(f"{build.SAIDA_NATIVO} was built against {_nativo.MARCA}, this is {build._marca()}: {como}")
+    return _nativo
+
+
 def define_blk(blk, lib=None):
     """Select the exponent block length (32 or 128) for this module and for the library."""
     global BLK
@@ -103,8 +116,7 @@ class OpsCuda:
             raise RuntimeError("this library has a fixed block length of 128; call ops.define_blk(128) first")
         if hasattr(self.lib, "jt_pdl"):                           # programmatic dependent launches: JT_PDL=0 switches them off
             self.lib.jt_pdl(0 if os.environ.get("JT_PDL", "1") == "0" else 1)
-        from . import _nativo
-        self._nat = _nativo
+        self._nat = carrega_nativo()
         self._fn = {}                                             # address of every entry point used so far
         self._ws = self._endereco("jt_gemm_ws_bytes"), self._endereco("jt_stream_atual")
         self._ws_gemm = self._endereco("jt_gemm_ws"), self._endereco("jt_gemm_ext")

@@ -50,3 +50,21 @@ def test_modulo_nativo_carrega():
     assert _nativo.blocos(32, (torch.zeros(2, 32, dtype=torch.int8), torch.zeros(2, 1, dtype=torch.int8))) is None      # not on a GPU
     with pytest.raises(TypeError):
         _nativo.novo_cru(1, 2, 3)
+
+
+def test_modulo_nativo_diz_o_que_falta(monkeypatch):
+    """Not built, or built against another PyTorch: the launcher says how to build, and the build does not take the old one for good."""
+    import sys
+    import pytest
+    from jatai_b200 import build, ops
+    build.build_nativo()
+    assert build.nativo_em_dia() and ops.carrega_nativo() is not None
+    monkeypatch.setattr(build, "_marca", lambda: "0.0 python 3.0")
+    assert not build.nativo_em_dia()
+    with pytest.raises(RuntimeError, match="was built against .*`python -m jatai_b200.build"):
+        ops.carrega_nativo()
+    monkeypatch.undo()
+    monkeypatch.setitem(sys.modules, "jatai_b200._nativo", None)
+    monkeypatch.delattr(sys.modules["jatai_b200"], "_nativo", raising=False)
+    with pytest.raises(RuntimeError, match="does not load .*`python -m jatai_b200.build"):
+        ops.carrega_nativo()
