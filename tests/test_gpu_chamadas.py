@@ -265,9 +265,9 @@ def test_memoria_esgotada_tem_o_tipo_do_alocador(amb, memoria):
     """Where an output does not fit, every kind of operator raises what PyTorch's allocator raises, and works again once there is room."""
     ops, oc, reg = amb
     G = casos.Gen(41, 32)
-    A, B, (qkv, go, forma) = para_gpu(G.bloco(8192, 2048)), para_gpu(G.bloco(2048, 2048)), _problema(32, 64, 128, 8, 64)
-    c = oc.gemm(B, B, cru=True)
-    memoria(1 << 20)
+    A, B, (qkv, go, forma) = para_gpu(G.bloco(16384, 2048)), para_gpu(G.bloco(2048, 2048)), _problema(32, 64, 128, 32, 64)
+    c = oc.gemm(A, B, cru=True)
+    memoria(1 << 20)                               # (every call wants 32 MB somewhere: more than what is free in a segment that is in use)
     for f in (lambda: oc.relu2(A), lambda: oc.gemm(A, B), lambda: oc.gemm(A, B, cru=True), lambda: oc.gemm_relu2(A, B), lambda: oc.quant(c),
               lambda: oc.atencao(qkv, *forma), lambda: oc.atencao_quant(qkv, *forma), lambda: oc.rms(A)):
         with pytest.raises(torch.OutOfMemoryError):
@@ -407,3 +407,84 @@ def test_registro_de_fora(amb, perfil):
         _alguns(oc, A, B, c, qkv, forma)
         plano.fim_passo()
         assert sorted(plano.tempos) == sorted({e[0] for e in esperado}) and all(v > 0 for v in plano.tempos.values())
+
+
+def _tok_fora(oc):
+    W = para_gpu(casos.Gen(3, 32).bloco(256, 128))
+    return W, torch.full((64,), 300, dtype=torch.int32, device="cuda")
+
+
+def test_registro_de_erros_limpo_antes_de_lido(amb):
+    """The record is cleared in the order of a stream and read after that: a sentinel of the step before does not come back."""
+    ops, oc, reg = amb
+    reg.vigiar = False
+    W, tok = _tok_fora(oc)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    try:
+        with torch.cuda.stream(s):
+            oc.lib.jt_stream(s.cuda_stream)
+            oc.embed(W, tok)
+            torch.cuda.synchronize()
+            torch.cuda._sleep(200_000_000)
+            reg.novo_passo(1)
+            reg.confere_device()
+    finally:
+        oc.lib.jt_stream(None)
+
+
+@pytest.mark.parametrize("n", [1, 20])
+def test_registro_de_erros_limpo_antes_de_outra_corrente(amb, n):
+    """A clearing that is still queued on one stream does not wipe out what a launch on another one finds afterwards, whichever of n it is."""
+    from jatai_b200.registro import ErroJatai
+    ops, oc, reg = amb
+    reg.vigiar = False
+    W, tok = _tok_fora(oc)
+    bom = torch.zeros_like(tok)
+    a, outras = torch.cuda.Stream(), [torch.cuda.Stream() for _ in range(n)]
+    torch.cuda.synchronize()
+    try:
+        with torch.cuda.stream(a):
+            oc.lib.jt_stream(a.cuda_stream)
+            torch.cuda._sleep(200_000_000)
+            reg.novo_passo(1)
+        for i, b in enumerate(outras):
+            with torch.cuda.stream(b):
+                oc.lib.jt_stream(b.cuda_stream)
+                oc.embed(W, tok if i == n - 1 else bom)
+        oc.lib.jt_stream(a.cuda_stream)
+        with torch.cuda.stream(a):
+            oc.embed(W, bom)
+        torch.cuda.synchronize()
+        with pytest.raises(ErroJatai, match="outside the vocabulary"):
+            reg.confere_device()
+    finally:
+        oc.lib.jt_stream(None)
+
+
+def test_registro_de_erros_limpo_antes_de_uma_repeticao(amb):
+    """The same for a recorded step that is replayed on a stream which is not the library's."""
+    from jatai_b200 import modelo
+    from jatai_b200.registro import ErroJatai
+    ops, oc, reg = amb
+    reg.vigiar = False
+    m = modelo.Modelo(256, 128, 2, 256, 1, 0, "cuda", oc, reg)
+    x = torch.randint(0, 256, (2, 64), device="cuda")
+    m.passo(x, x, k_lr=4)
+    g = modelo.PassoGravado(m, 2, 64, 4)
+    ruim = x.clone()
+    ruim[1, 17] = 300
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    try:
+        with torch.cuda.stream(a):
+            oc.lib.jt_stream(a.cuda_stream)
+            torch.cuda._sleep(200_000_000)
+            reg.novo_passo(1)
+        with torch.cuda.stream(b):
+            g(ruim, x)
+        torch.cuda.synchronize()
+        with pytest.raises(ErroJatai, match="forward / embedding"):
+            reg.confere_device()
+    finally:
+        oc.lib.jt_stream(None)
