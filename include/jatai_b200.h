@@ -35,9 +35,10 @@ extern "C" {
 
 /* ---- device error record and control --------------------------------------------------------------- */
 /* out[0..5] = n events, code, kid, flat index into the output, value, extra.  Returns n, or -cudaError.
- * Synchronises.  Codes 1..6 as in the reference (jatai_cuda.cu:22), 7 = a bounded in-kernel wait expired.
+ * Waits for the stream set with jt_stream.  Codes 1..6 as in the reference (jatai_cuda.cu:22), 7 = a bounded in-kernel wait expired.
  * jatai_cuda.cu:1062 */
 int jt_erro_le(long long* out);
+/* Clears the record on the stream set with jt_stream, without waiting for it; a stream set later waits for the clearing. */
 int jt_erro_limpa(void);                                   /* jatai_cuda.cu:1069 */
 int jt_sincroniza(void);                                   /* jatai_cuda.cu:1073 */
 void jt_stream(void* cuda_stream);                         /* jatai_cuda.cu:1088 */

@@ -226,8 +226,29 @@ static bool ws_serve(const void* ws) { return ws && ((uintptr_t)ws & 127) == 0; 
 extern "C" {
 
 // ---------------------------------------------------------------------------------------------- control
+// Where the error record was last cleared: that happens in the order of one stream, and a launch on another one must not come before it.
+static struct { cudaEvent_t ev[64]; int dev; cudaStream_t onde, esperam[16]; int n; bool pendente; } g_limpa;
+static void espera_limpeza(cudaStream_t st) {
+    if (!g_limpa.pendente || st == g_limpa.onde) return;
+    for (int i = 0; i < g_limpa.n; i++)
+        if (g_limpa.esperam[i] == st) return;
+    // (launches that are being captured run when the graph is launched, on a stream of its caller's choice)
+    int dev = -1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev != g_limpa.dev || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return;
+    }
+    if (g_limpa.n == 16) {                 // more streams than there is room for: wait here
+        if (cudaEventSynchronize(g_limpa.ev[dev]) == cudaSuccess) g_limpa.pendente = false;
+        return;
+    }
+    if (cudaStreamWaitEvent(st, g_limpa.ev[dev], 0) == cudaSuccess) g_limpa.esperam[g_limpa.n++] = st;
+}
 int jt_erro_le(long long* out) {
     Erro e;
+    // the launches and the clearing before this call are on the stream set with jt_stream or ordered before it
+    (void)cudaStreamSynchronize(g_stream);
     cudaError_t c = cudaMemcpyFromSymbol(&e, g_erro, sizeof(Erro));
     if (c != cudaSuccess) return -(int)c;
     out[0] = e.n; out[1] = e.codigo; out[2] = e.kid; out[3] = e.idx; out[4] = e.valor; out[5] = e.aux;
@@ -252,7 +273,8 @@ int jt_teste_espera(int* saiu, int kid) {
 }
 // Programmatic dependent launch of the kernels that support it (0 = plain stream order).
 int jt_pdl(int ligado) { pdl_ligado() = ligado ? 1 : 0; return 0; }
-// Clears the error record, in the order of the launches (on the stream set with jt_stream): a step that begins does not wait for the GPU.
+// Clears the error record, in the order of the launches: on the stream set with jt_stream, and before the launches that follow on any other one
+// it is set to.  A step that begins does not wait for the GPU.
 int jt_erro_limpa() {
     static void* onde[64];                 // address of the record, per device
     int dev = 0;
@@ -260,10 +282,21 @@ int jt_erro_limpa() {
     if (c != cudaSuccess) return (int)c;
     if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
     if (!onde[dev] && (c = cudaGetSymbolAddress(&onde[dev], g_erro)) != cudaSuccess) return (int)c;
-    return (int)cudaMemsetAsync(onde[dev], 0, sizeof(Erro), g_stream);
+    if ((c = cudaMemsetAsync(onde[dev], 0, sizeof(Erro), g_stream)) != cudaSuccess) return (int)c;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    g_limpa.pendente = cudaStreamIsCapturing(g_stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    if (!g_limpa.pendente) return 0;
+    if (!g_limpa.ev[dev] && (c = cudaEventCreateWithFlags(&g_limpa.ev[dev], cudaEventDisableTiming)) != cudaSuccess) return (int)c;
+    g_limpa.dev = dev;
+    g_limpa.onde = g_stream;
+    g_limpa.n = 0;
+    return (int)cudaEventRecord(g_limpa.ev[dev], g_stream);
 }
 int jt_sincroniza() { return (int)cudaDeviceSynchronize(); }
-void jt_stream(void* st) { g_stream = (cudaStream_t)st; }
+void jt_stream(void* st) {
+    g_stream = (cudaStream_t)st;
+    espera_limpeza(g_stream);
+}
 void* jt_stream_atual() { return (void*)g_stream; }
 void jt_gemm_split(int alvo) { g_alvo_ctas = alvo > 0 ? alvo : 148; }
 void jt_gemm_bm(int) {}

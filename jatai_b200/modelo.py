@@ -475,10 +475,21 @@ class PassoGravado:
         self.coletivos_por_passo = 0 if red is None else 2 * len(self._M)
         self.reg.info(f"step recorded in {len(self.grafos)} CUDA graph(s): {len(self.lancamentos)} launches", lancamentos=len(self.lancamentos))
 
+    def _na_ordem(self):
+        """A replay goes to PyTorch's stream.  Where the library's is another one (the error record is cleared there), it is set to this
+        one for a moment: what is then queued here waits for the clearing."""
+        lib = self.m.ops.lib
+        if hasattr(lib, "jt_stream_atual"):
+            dela, esta = lib.jt_stream_atual(), torch.cuda.current_stream().cuda_stream
+            if (dela or 0) != esta:
+                lib.jt_stream(esta)
+                lib.jt_stream(dela)
+
     def __call__(self, tok, alvo):
         self.tok.copy_(tok)
         self.alvo.copy_(alvo)
         self.reg.lancamentos = self.lancamentos
+        self._na_ordem()
         if len(self.grafos) == 1:
             self.grafos[0].replay()
             return self.perda
