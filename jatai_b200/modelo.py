@@ -289,6 +289,22 @@ class Modelo:
         stream joined, so that a caller can end a CUDA graph there and put a collective between two pieces (data
         parallel: the weight-gradient operands of the piece just finished are the new entries of self._adiados).  The loss
         tensor is left in self._perda."""
+        try:
+            yield from self._em_trechos(tok, alvo, treina, k_lr, cortes)
+        except BaseException:                                      # (GeneratorExit too: a caller that stops between two pieces)
+            self._abandona()
+            raise
+
+    def _abandona(self):
+        """A step that ends early: what the side streams still read goes back only after the main stream has joined them."""
+        if self._ramo is not None:
+            try:
+                self._junta_lado()
+            except RuntimeError:
+                pass                                               # a recording that has failed joins nothing, and nothing runs
+        self._presos = []
+
+    def _em_trechos(self, tok, alvo, treina, k_lr, cortes):
         ops, reg, p = self.ops, self.reg, self.p
         Bt, T = tok.shape
         tok = tok.reshape(-1).to(torch.int32).contiguous()

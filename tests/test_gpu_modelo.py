@@ -88,3 +88,41 @@ def test_sentinela_dentro_do_grafo():
         reg.fim_passo()
     msg = str(ei.value)
     assert "embed" in msg and "forward / embedding" in msg and f"linha {T + 17}, coluna 0" in msg and "300" in msg
+
+
+def test_passo_abandonado_espera_pelas_correntes_ao_lado():
+    """A step that an exception ends while a side stream still reads its tensors: the main stream joins that stream before it goes on, so
+    that memory given back is not written under it; and the model steps on as one that never failed."""
+    from jatai_b200 import modelo, ops, registro
+    ops.define_blk(32)
+
+    def novo():
+        reg = registro.Registro(tempfile.mkdtemp(), "a", eco=False, salvar=False)
+        oc = ops.OpsCuda(reg)
+        reg.novo_passo(0)
+        return modelo.Modelo(256, 512, 8, 512, 2, 0, "cuda", oc, reg), oc
+    m, oc = novo()
+    x = torch.randint(0, 256, (8, 256), generator=torch.Generator().manual_seed(1)).cuda()
+    assert x.numel() * m.D >= m.RAMO_MINIMO                       # the eager step uses a side stream
+    par = oc.transpoe2
+
+    def lento(*a):
+        torch.cuda._sleep(400_000_000)                            # on the side stream
+        return par(*a)
+
+    def cai(*a):
+        raise ValueError("no more")
+    oc.transpoe2, oc.rms_back = lento, cai                        # the first weight gradient, then the next operator of the main chain
+    with pytest.raises(ValueError):
+        m.passo(x, x, k_lr=4)
+    fim = torch.cuda.current_stream().record_event()
+    fim.synchronize()
+    assert m._lados[0].query(), "the main stream went on while the side stream was reading"
+    assert not m._presos
+    del oc.transpoe2, oc.rms_back
+    a, _ = novo()
+    for k in range(2):
+        a.passo(x, x, k_lr=4)
+        m.passo(x, x, k_lr=4)
+    for i, (u, v) in enumerate(zip(_estado(a), _estado(m))):
+        assert torch.equal(u, v), f"state tensor {i}"
