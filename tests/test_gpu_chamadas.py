@@ -269,10 +269,11 @@ def test_memoria_esgotada_tem_o_tipo_do_alocador(amb, memoria):
     G = casos.Gen(41, 32)
     A, B, (qkv, go, forma) = para_gpu(G.bloco(16384, 2048)), para_gpu(G.bloco(2048, 2048)), _problema(32, 64, 128, 32, 64)
     c = oc.gemm(A, B, cru=True)
-    memoria(1 << 20)                               # (every call wants 32 MB somewhere: more than what is free in a segment that is in use)
+    # (every call wants 32 MB somewhere: more than what is free in a segment that is in use)
     for nome, f in (("relu2", lambda: oc.relu2(A)), ("gemm", lambda: oc.gemm(A, B)), ("gemm_cru", lambda: oc.gemm(A, B, cru=True)),
                     ("gemm_relu2", lambda: oc.gemm_relu2(A, B)), ("quant", lambda: oc.quant(c)), ("atencao", lambda: oc.atencao(qkv, *forma)),
                     ("atencao_quant", lambda: oc.atencao_quant(qkv, *forma)), ("rms", lambda: oc.rms(A))):
+        memoria(1 << 20)
         try:
             f()
             raise AssertionError(f"{nome} found memory; {torch.cuda.memory_reserved() - torch.cuda.memory_allocated()} bytes were free")
