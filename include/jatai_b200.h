@@ -96,9 +96,9 @@ int jt_atencao(const void* qm, const void* qE, void* Oacc, void* Oe, void* P, in
 int jt_atencao_back(const void* gom, const void* goE, const void* qm, const void* qE, const void* P, void* Gacc, void* Ge,
                     int Bt, int T, int H, int D, int GA, int limite, int kid);
 int jt_softmax_ce(const void* acc, const void* e, const void* alvo, void* gm, void* gE, void* d_alvo, void* soma,
-                  int M, int V, int log2M, int kid);
-/* loss of every row of jt_softmax_ce's outputs (report only): perda[i] = d_alvo[i] / 256 + log(soma[i] / 4096), double precision */
-int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid);                                                            /* jatai_cuda.cu:1195 */
+                  int M, int V, int log2M, int kid);                                                            /* jatai_cuda.cu:1195 */
+/* No counterpart in the reference: loss of every row of jt_softmax_ce's outputs (report only): perda[i] = d_alvo[i] / 256 + log(soma[i] / 4096), double precision */
+int jt_perda(const void* d_alvo, const void* soma, void* perda, int M, int kid);
 
 /* The reference's 16-bit residual stream (opt-in ablation, no int64 specification).  Exported so that a launcher
  * that looks the symbols up keeps working; each returns cudaErrorNotSupported.  jatai_cuda.cu:1074-1086 */
@@ -112,8 +112,8 @@ int jt_soma16(const void* xm, const void* xE, const void* ym, const void* yE, vo
 int jt_blk(int blk);
 int jt_blk_atual(void);
 /* GEMM path: 0 automatic | 1 tensor cores, refused (cudaErrorInvalidValue) on a shape they do not take | 2 CUDA cores (dp4a) |
- * 3 tensor cores with every K-block rounded by a float-to-int conversion | 4 half-precision tensor pipe, forced (block 32's default rounds with an FMA against
- * 1.5*2^23 after a range check, and converts only the columns that fail it; both are exact for every input). */
+ * 3 tensor cores with every K-block rounded by a float-to-int conversion (path 1 rounds block 32 with an FMA against 1.5*2^23 after a range
+ * check, and converts only the columns that fail it; both are exact for every input) | 4 half-precision tensor pipe (jt_gemm_ws). */
 int jt_gemm_via(int via);
 /* jt_quant(jt_atencao(...)) / jt_quant(jt_atencao_back(...)) with the quantisation done in the attention kernels' output stage:
  * Om, OE = block tensor [Bt*T, D]; Gm, GE = block tensor [Bt*T, 3D] (gq | gk | gv); other arguments as in jt_atencao /

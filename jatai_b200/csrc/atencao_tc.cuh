@@ -21,7 +21,7 @@
 // reference's slopes P is exactly zero a few dozen keys behind the diagonal, so one window is nearly always all there is: the forward
 // works out after the first window how many it needs, the backward reads a map of the non-zero parts of P.  The one-window case keeps
 // everything in registers between the passes (scores, exponentials, P); with more windows each pass computes the scores again.
-// Between load, MMA and drain a block has little to overlap, so the overlap comes from two blocks per SM.
+// Between load, MMA and drain a block has little to overlap, so the overlap comes from three blocks per SM (k_ab_max: four).
 //
 // Orientation of every score-like product of a query tile: tensor-memory lane = key (M = 128 keys of a window), column = query; a
 // thread of the drain owns one key and 32 queries.  Stored P is key-major, so that thread reads or writes 32 contiguous bytes of P.

@@ -13,9 +13,9 @@
 // That leaves the CUDA cores ONE packed addition per two element-steps - r + 1.5 * 2^23 rounds half to even at integer granularity -
 // and one three-input integer addition per two element-steps (two K-blocks at a time): no exponent table, no scaling, no int -> float
 // conversion.  The rounding is exact while |r| < 2^22, i.e. |p| 2^-(sa+sb) < 2^18.  Block 32: k_prep_h leaves, per 32 rows and K-block,
-// the largest squared norm of a block scaled by 4^-s; by Cauchy-Schwarz the bound holds for a warp's 32 x 64 outputs whenever the product
-// of its two norms is below 2^36, which a warp evaluates for 32 K-blocks at once; where it does not hold, and always with block 128 (a
-// quarter of the drains), the results' exponent fields are checked and a failing warp reads the accumulators again and converts.
+// the largest squared norm of a block scaled by 4^-s; by Cauchy-Schwarz the bound holds for a warp's 32 x 32 outputs whenever the product
+// of its two norms is below 2^36, which a warp evaluates for 32 K-blocks at once; where it does not hold, it rounds by conversion.  Block 128
+// (a quarter of the drains): the results' exponent fields are checked, and a warp in which one has left the window converts.
 #pragma once
 #include "gemm_tc.cuh"
 
@@ -179,25 +179,13 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t da, uint64_t d
                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
                  ::"r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(acumula) : "memory");
 }
-// 8, 16 or 32 consecutive columns of this lane, asynchronous: the registers may be used after tmem_pronto on them
-__device__ __forceinline__ void tmem_pede(uint32_t t, uint32_t (&d)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : JT_O4(d, 0), JT_O4(d, 4) : "r"(t) : "memory");
-}
+// 16 consecutive columns of this lane, asynchronous: the registers may be used after tmem_pronto on them
 __device__ __forceinline__ void tmem_pede(uint32_t t, uint32_t (&d)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" : JT_O16(d, 0) : "r"(t) : "memory");
 }
-__device__ __forceinline__ void tmem_pede(uint32_t t, uint32_t (&d)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
-                 "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];" : JT_O32(d, 0) : "r"(t) : "memory");
-}
 #define JT_IO4(a, i) "+r"(a[i]), "+r"(a[i + 1]), "+r"(a[i + 2]), "+r"(a[i + 3])
 #define JT_IO16(a, i) JT_IO4(a, i), JT_IO4(a, i + 4), JT_IO4(a, i + 8), JT_IO4(a, i + 12)
-__device__ __forceinline__ void tmem_pronto(uint32_t (&a)[8]) { asm volatile("tcgen05.wait::ld.sync.aligned;" : JT_IO4(a, 0), JT_IO4(a, 4)::"memory"); }
 __device__ __forceinline__ void tmem_pronto(uint32_t (&a)[16]) { asm volatile("tcgen05.wait::ld.sync.aligned;" : JT_IO16(a, 0)::"memory"); }
-__device__ __forceinline__ void tmem_pronto(uint32_t (&a)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" : JT_IO16(a, 0)::"memory");
-    asm volatile("" : JT_IO16(a, 16)::"memory");                            // (an asm statement takes 30 operands: the rest is tied to the wait by order)
-}
 // two fp32 additions in one instruction: r + 1.5 * 2^23, the rounding of the specification
 __device__ __forceinline__ void soma_magia(uint32_t& a, uint32_t& b) {
     asm volatile("{\n .reg .b64 t;\n mov.b64 t, {%0, %1};\n add.rn.f32x2 t, t, %2;\n mov.b64 {%0, %1}, t;\n}" : "+r"(a), "+r"(b) : "l"(par(MAGIA, MAGIA)));

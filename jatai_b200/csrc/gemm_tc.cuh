@@ -143,16 +143,7 @@ __device__ __forceinline__ void tmem_le32(uint32_t taddr, uint32_t (&d)[32]) {
         : "memory");
 }
 
-// 16 consecutive columns of this thread's lane from each of two tensor-memory addresses (two K slices); one wait for both
-__device__ __forceinline__ void tmem_le16x2(uint32_t ta, uint32_t tb, uint32_t (&a)[16], uint32_t (&b)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n"
-        "tcgen05.wait::ld.sync.aligned;\n"
-        : JT_O16(a, 0), JT_O16(b, 0)
-        : "r"(ta), "r"(tb)
-        : "memory");
-}
+// 8 consecutive columns of this thread's lane from each of two tensor-memory addresses (two K slices); one wait for both
 __device__ __forceinline__ void tmem_le8x2(uint32_t ta, uint32_t tb, uint32_t (&a)[8], uint32_t (&b)[8]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n"

@@ -29,9 +29,9 @@ using namespace jt;
 static cudaStream_t g_stream = 0;
 static int g_blk = 32;               // exponent block length: 32 (native) or 128 (the reference's format)
 static int g_via = 0;                // GEMM path: 0 automatic | 1 tensor core (forced) | 2 CUDA cores | 3 tensor core, rounding by conversion | 4 half-precision tensor pipe (forced)
-static int g_alvo_ctas = 148;
+static int g_alvo_ctas = 148;        // split-K of raw GEMMs aims at this many CTAs
 static int g_at_via = 0;             // attention path: 0 automatic (tensor cores; one CTA per head for short sequences of heads of 4) | 1 the tiled CUDA-core kernels
-static int g_tn = 0;                 // tile width of the tensor-core GEMM: 0 automatic | 64 | 128        // split-K of raw GEMMs aims at this many CTAs
+static int g_tn = 0;                 // tile width of the tensor-core GEMM: 0 automatic | 64 | 128
 
 static int fim() { return (int)cudaGetLastError(); }
 static unsigned nblocos16(long long n16) { return (unsigned)((n16 + 255) / 256); }
