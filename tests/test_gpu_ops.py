@@ -310,17 +310,20 @@ def test_gemm_largura_do_tile(amb, nome, blk, f, tn):
 @pytest.mark.parametrize("tn", [64, 128])
 @pytest.mark.parametrize("caso", ["expoentes afastados", "linhas nulas", "acumuladores grandes"])
 @pytest.mark.parametrize("op", ["gemm", "gemm_soma", "gemm_relu2", "gemm_relu2_back"])
-def test_gemm_estagio_de_saida(amb, op, caso, tn):
+@pytest.mark.parametrize("blk,via", [(32, 0), (32, 4), (128, 0), (128, 4)])
+def test_gemm_estagio_de_saida(amb, op, caso, tn, blk, via):
     """The output stage of the tensor-core GEMM quantises in fp32 when that is exact and in integers otherwise.  These
     inputs force the integer side: column exponents of one block more than 64 apart, all-zero rows of B (row maximum
-    -127 next to ordinary rows), accumulators at or above 2^24 - each against the specification."""
+    -127 next to ordinary rows), accumulators at or above 2^24 - each against the specification, on the 8-bit kernel (which
+    these sizes take by themselves) and on the half-precision one, which has its own tables for that decision."""
     ops, oc, reg = amb
-    ops.define_blk(32)
-    oc.lib.jt_gemm_via(0)
-    assert oc.lib.jt_gemm_tn(tn) == 0
+    if blk == 128 and tn == 64:
+        pytest.skip("64-column tiles exist for block 32 only")
+    ops.define_blk(blk)
+    assert oc.lib.jt_gemm_via(via) == 0 and oc.lib.jt_gemm_tn(tn) == 0
     try:
         reg.novo_passo(0)
-        G = casos.Gen(4242, 32)
+        G = casos.Gen(4242, blk)
         M, K, N = 256, 512, 256
         A, B = G.bloco(M, K, espalha=2), G.bloco(N, K, espalha=2)
         if caso == "expoentes afastados":
@@ -336,9 +339,11 @@ def test_gemm_estagio_de_saida(amb, op, caso, tn):
         args = {"gemm": (A, B), "gemm_soma": (A, B, X), "gemm_relu2": (A, B), "gemm_relu2_back": (A, B, X)}[op]
         outs = casos.roda(oc, op, tuple(para_gpu(a) for a in args), {})
         torch.cuda.synchronize()
-        compara(f"{op} {caso} tn {tn}", outs, casos.roda(spec.Spec(32), op, args, {}))
+        compara(f"{op} {caso} tn {tn} blk {blk} via {via}", outs, casos.roda(spec.Spec(blk), op, args, {}))
     finally:
         oc.lib.jt_gemm_tn(0)
+        oc.lib.jt_gemm_via(0)
+        ops.define_blk(32)
 
 
 @pytest.mark.parametrize("blk", [32, 128])
@@ -414,14 +419,15 @@ def test_rms_back_soma_junto(amb, blk, M, D):
 
 @pytest.mark.parametrize("tn", [64, 128])
 @pytest.mark.parametrize("caso", ["tudo +127", "sinais alternados", "uma linha saturada", "um bloco saturado por linha"])
-def test_gemm_produtos_parciais_grandes(amb, caso, tn):
+@pytest.mark.parametrize("via", [0, 4])
+def test_gemm_produtos_parciais_grandes(amb, caso, tn, via):
     """Partial products at and above 2^18 with no alignment shift (s = 0): the inputs on which rounding by an FMA against
-    1.5*2^23 would leave its exact range.  The kernel must find them (a range check on the biased patterns) and round those
-    columns by conversion - in whole tiles, in single rows and in single K-blocks, for positive and negative products."""
+    1.5*2^23 would leave its exact range.  The kernels must find them (the 8-bit one, which these sizes take by themselves, by a range check
+    on the biased patterns, the half-precision one by the norms of the K-blocks) and round those by conversion - in whole
+    tiles, in single rows and in single K-blocks, for positive and negative products."""
     ops, oc, reg = amb
     ops.define_blk(32)
-    oc.lib.jt_gemm_via(0)
-    assert oc.lib.jt_gemm_tn(tn) == 0
+    assert oc.lib.jt_gemm_via(via) == 0 and oc.lib.jt_gemm_tn(tn) == 0
     try:
         reg.novo_passo(0)
         G = casos.Gen(8181, 32)
@@ -444,9 +450,10 @@ def test_gemm_produtos_parciais_grandes(amb, caso, tn):
         for cru in (False, True):
             outs = casos.plano(oc.gemm(para_gpu(A), para_gpu(B), cru=cru))
             torch.cuda.synchronize()
-            compara(f"gemm {caso} tn {tn} cru {cru}", outs, casos.plano(spec.Spec(32).gemm(A, B, cru=cru)))
+            compara(f"gemm {caso} tn {tn} via {via} cru {cru}", outs, casos.plano(spec.Spec(32).gemm(A, B, cru=cru)))
     finally:
         oc.lib.jt_gemm_tn(0)
+        oc.lib.jt_gemm_via(0)
 
 
 @pytest.mark.parametrize("limite", [False, True])
@@ -640,10 +647,10 @@ def test_atencao_janelas(amb, blk, Bt, T, H, D, e0, longe):
     G = casos.Gen(911 + T + H + D, blk)
     qkv, go = G.bloco(Bt * T, 3 * D, e0=e0, espalha=4, zera=0.02), G.bloco(Bt * T, D, e0=-20, espalha=4)
     s = spec.Spec(blk)
-    o_r, P = s.atencao(qkv, Bt, T, H)
+    o_r, P_r = s.atencao(qkv, Bt, T, H)
     try:
         o_c, P_c = oc.atencao(para_gpu(qkv), Bt, T, H)
-        P = P.clone()
+        P = P_r.clone()
         for n in range(longe):                       # [Bt*H, T (keys), T (queries)]
             j = (37 * n) % (T // 4)
             P[n % (Bt * H), j, T - 1 - 29 * n] = 200
@@ -653,7 +660,7 @@ def test_atencao_janelas(amb, blk, Bt, T, H, D, e0, longe):
         torch.cuda.synchronize()
     finally:
         ops.define_blk(32)
-    compara(f"atencao T {T} H {H} D {D}", list(o_c), list(o_r))
+    compara(f"atencao T {T} H {H} D {D}", [*o_c, P_c], [*o_r, P_r])
     compara(f"atencao_back T {T} H {H} D {D}", list(g_c), list(g_r))
 
 
