@@ -22,7 +22,7 @@ import os
 
 import torch
 
-from . import registro
+from .registro import Registro
 
 BLK = 32
 E_ZERO = -127
@@ -144,7 +144,7 @@ class OpsCuda:
         `nomes` name the first tensors in the launch record (None leaves one out)."""
         reg = self.reg
         # The native calls append to the launch list of a plain Registro that times nothing; of any other registry they call registra and depois.
-        if reg.perfil or reg.__class__ is not registro.Registro:
+        if reg.perfil or reg.__class__ is not Registro:
             self._nat.lanca(self._endereco(fn), reg, op, reg.onde(), nomes, tensores, inteiros, forma)
             return
         r = self._nat.lanca(self._endereco(fn), reg.lancamentos, op, reg.onde(), nomes, tensores, inteiros, forma)
@@ -177,7 +177,7 @@ class OpsCuda:
     def _gemm(self, op, modo, A, B, X=None, duas=False, RA=None, RB=None):
         reg, nat = self.reg, self._nat
         if RA is None and RB is None:
-            alheio = reg.perfil or reg.__class__ is not registro.Registro
+            alheio = reg.perfil or reg.__class__ is not Registro
             r = nat.gemm(*self._ws, *self._ws_gemm, BLK, reg if alheio else reg.lancamentos, op, reg.onde(), modo, A, B, X, duas)
             if r.__class__ is tuple:
                 if reg.vigiar and not alheio:
@@ -358,7 +358,7 @@ class OpsCuda:
         """The call in one piece, workspace included (`entradas`: the entry points with one and, raw outputs only, without), or None: block
         outputs without a workspace, a library with only the reference's entry points - and what is wrong with an argument."""
         reg = self.reg
-        alheio = reg.perfil or reg.__class__ is not registro.Registro
+        alheio = reg.perfil or reg.__class__ is not Registro
         r = self._nat.atencao(*self._ws_at, *entradas, BLK, reg if alheio else reg.lancamentos, op, reg.onde(), QKV, GO, P, Bt, T, H, GA,
                               int(ATENCAO_LIMITE), blocos)
         if r.__class__ is int:
