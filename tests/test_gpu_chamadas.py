@@ -90,6 +90,8 @@ def _limita_torch(folga):
 
 @pytest.fixture
 def memoria(amb):
+    gc.collect()
+    torch.cuda.empty_cache()                           # (else the test's tensors may share a segment with a large free rest of an earlier test's)
     yield _limita_torch
     torch.cuda.set_per_process_memory_fraction(1.0)
     amb[1].lib.jt_espaco_limite(0)
