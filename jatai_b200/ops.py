@@ -142,12 +142,12 @@ class OpsCuda:
     def _lanca(self, op, fn, tensores, inteiros, nomes, forma):
         """Registers the launch and calls the entry point: pointers of `tensores` (None = null), then `inteiros`, then the launch id.
         `nomes` name the first tensors in the launch record (None leaves one out)."""
-        reg = self.reg
+        reg, f = self.reg, self._fn.get(fn) or self._endereco(fn)
         # The native calls append to the launch list of a plain Registro that times nothing; of any other registry they call registra and depois.
         if reg.perfil or reg.__class__ is not Registro:
-            self._nat.lanca(self._endereco(fn), reg, op, reg.onde(), nomes, tensores, inteiros, forma)
+            self._nat.lanca(f, reg, op, reg.onde(), nomes, tensores, inteiros, forma)
             return
-        r = self._nat.lanca(self._endereco(fn), reg.lancamentos, op, reg.onde(), nomes, tensores, inteiros, forma)
+        r = self._nat.lanca(f, reg.lancamentos, op, reg.onde(), nomes, tensores, inteiros, forma)
         if r is not None:
             reg.depois(*r)
         elif reg.vigiar:

@@ -37,7 +37,12 @@ def test_rotulos_depois_de_um_erro():
         with r.trecho("fim"):
             r.confere_device()
     assert r.onde() == "-"
+    with pytest.raises(registro.ErroJatai, match="forward / embedding"):
+        r.confere_device()
+    assert r.onde() == "-"
     with r.trecho("a"):
+        with pytest.raises(registro.ErroJatai, match="forward / embedding"):
+            r.confere_device()
         assert r.onde() == "a"
     assert r.onde() == "-"
 
