@@ -138,7 +138,9 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
     return M > 0 && N > 0 && K > 0 && M % 64 == 0 && N % TN == 0 && K % blk == 0 && K % 32 == 0 && modo >= 0 && modo <= 4;
 }
 // Estimated times of the GEMM kernels in microseconds (measured at 128..16384 rows, 128..4096 columns, K = 128..16384): waves of tiles
-// times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels.
+// times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels: against the
+// kernels forced one by one at 44 sizes the choice is within 1 % of the best, but for six sizes where it loses 3 to 7 % (1536 x 512 x 4096 raw 44.3 us against
+// 41.7 with 128-wide tiles, 3072 x 1024 x 16384 raw 256 against 240 with 64-wide ones, block 128 at 4096 x 1024 x 1024 23.1 against 21.6).
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
 static Custos custos_gemm(int blk, int M, int N, int K) {
     const double n = (K + 63) / 64;
