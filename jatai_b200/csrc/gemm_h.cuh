@@ -16,6 +16,12 @@
 // the largest squared norm of a block scaled by 4^-s; by Cauchy-Schwarz the bound holds for a warp's 32 x 32 outputs whenever the product
 // of its two norms is below 2^36, which a warp evaluates for 32 K-blocks at once; where it does not hold, it rounds by conversion.  Block 128
 // (a quarter of the drains): the results' exponent fields are checked, and a warp in which one has left the window converts.
+//
+// Where sa + sb <= 4 nothing is rounded at all: r is a whole number.  A tile in which that holds for every K-block (what a step multiplies by
+// its weights nearly always is: normalised rows and weights have block exponents one or two apart) need not be drained K-block by
+// K-block; its chunks add up in tensor memory, in fp32, exactly while the sum of the bounds stays below 2^24 last places.  Large
+// products with K <= 1024 look for it, with the norms and the largest shift that k_prep_h leaves.  Drained once, a tile is bound by what
+// issues its MMAs (480 cycles a chunk, against 790 for a rounded one): 16384 x 4096 x 1024 with ReLU^2 290 -> 185 us, 16384 x 1024 x 1024 77 -> 55.
 #pragma once
 #include "gemm_tc.cuh"
 
@@ -26,11 +32,12 @@ using namespace tc;
 
 constexpr int KH = 64;                                     // K elements per operand stage: 128 bytes of f16, one swizzle row
 constexpr float LIM_NORMA = 68719000000.0f;               // just below 2^36 (the product of two fp32 roundings included)
+constexpr float LIM_SOMA = 16770000.0f;                    // just below 2^24
 
 // ------------------------------------------------------------------------------------------ operand preparation
 struct ArgsPrepH {
     const int8_t* m[2]; const int8_t* E[2]; const int8_t* Rext[2];      // A and B: mantissas, exponents, external row maxima or nullptr
-    uint16_t* h[2]; int8_t* R[2]; float* nrm[2];                         // f16 operands, row maxima, norms [ceil(rows/32)][K/32] (block 32)
+    uint16_t* h[2]; int8_t* R[2]; uint32_t* nrm[2];                      // f16 operands, row maxima, bounds [ceil(rows/32)][K/32] (block 32)
     int linhas[2], ctas0;                                                // rows of each; CTAs of A (B's follow)
     int K;
 };
@@ -49,6 +56,9 @@ __device__ __forceinline__ uint32_t dois_h(float v) {
     return r;
 }
 
+// A bound is one word per 32 rows and K-block: the largest squared norm of a block of the group, scaled by 4^-s, as a float rounded up
+// to 18 bits of mantissa, and in the five bits that leaves free the largest s of a block that is not zero.
+//
 // One CTA of 256 threads: 32 rows x 512 columns of one operand; a warp takes 4 rows, a lane 16 consecutive elements of each.  Bound by
 // memory (1 byte in, 2 out per element); the exponents of the whole row are read by every CTA of the row (K / 32 bytes, from L2).
 template <int BLK>
@@ -56,6 +66,7 @@ __global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
     pdl_espera();
     pdl_solta();
     __shared__ float nrm_s[8][16];
+    __shared__ int smax_s[8][16];
     const int q = (int)blockIdx.x >= P.ctas0, cta = (int)blockIdx.x - (q ? P.ctas0 : 0);
     const int K = P.K, nb = K / BLK, nfx = (K + 511) / 512, c0 = (cta % nfx) * 512, g32 = cta / nfx;
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, c = c0 + lane * 16;
@@ -93,6 +104,7 @@ __global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
         for (int i = 0; i < 4; i++) r[i] = __reduce_max_sync(FULL, r[i]);
     }
     float nmax = 0.f;
+    int smax = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int s = r[i] - e[i];
@@ -114,7 +126,9 @@ __global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
             n = __dp4a((int)v[i].z, (int)v[i].z, n);
             n = __dp4a((int)v[i].w, (int)v[i].w, n);
             n += __shfl_xor_sync(FULL, n, 1);
+            // (a block of zeros, or one so far down that its operand is zero, adds nothing)
             nmax = fmaxf(nmax, (float)n * (s <= 26 ? pot2(-2 * s) : 0.f));
+            smax = max(smax, n != 0 && s <= 26 ? s : 0);
         }
     }
     if (c0 == 0 && lane < 4 && l0 + lane < linhas) {
@@ -122,13 +136,15 @@ __global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
         (q ? P.R[1] : P.R[0])[l0 + lane] = (int8_t)rr;
     }
     if (BLK == 32) {
-        if ((lane & 1) == 0) nrm_s[wid][lane >> 1] = nmax;
+        // (the low five bits of a norm rounded up are free for the shift)
+        if ((lane & 1) == 0) { nrm_s[wid][lane >> 1] = nmax; smax_s[wid][lane >> 1] = smax; }
         __syncthreads();
         if (threadIdx.x < 16 && c0 / 32 + (int)threadIdx.x < nb) {
             float n = 0.f;
+            int sm = 0;
 #pragma unroll
-            for (int w = 0; w < 8; w++) n = fmaxf(n, nrm_s[w][threadIdx.x]);
-            (q ? P.nrm[1] : P.nrm[0])[(size_t)g32 * nb + c0 / 32 + threadIdx.x] = n;
+            for (int w = 0; w < 8; w++) { n = fmaxf(n, nrm_s[w][threadIdx.x]); sm = max(sm, smax_s[w][threadIdx.x]); }
+            (q ? P.nrm[1] : P.nrm[0])[(size_t)g32 * nb + c0 / 32 + threadIdx.x] = ((__float_as_uint(n) + 31u) & ~31u) | (uint32_t)sm;
         }
     }
 }
@@ -150,15 +166,15 @@ struct CfgH {
     static constexpr int N_MW = 2, N_THR = N_EPI + 32 + 32 * N_MW;          // multiplying warps: each takes every N_MW-th stage
     static_assert(NS >= N_MW && COLS == 32, "");
     static constexpr uint32_t B_BYTES = TNv * 128, STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int NST = 4;
+    static constexpr int NST = 4, NPL = 8;                                  // NPL: tiles whose plans are kept (the loads are at most 6 ahead of a drain)
     // the staged accumulators: memory of their own where the loads of the next tile go on meanwhile, else the operand ring (when a
     // drain thread stores them it has seen the commit of the last MMA)
     static constexpr uint32_t ACC_BYTES = TM * (TNv + 4) * 4, OFF_ACC = PERSISTE ? NST * STAGE_BYTES : 0;
     static_assert(PERSISTE || ACC_BYTES <= NST * STAGE_BYTES, "staged accumulators must fit in the operand ring");
     static constexpr uint32_t OFF_RA = PERSISTE ? OFF_ACC + ACC_BYTES : NST * STAGE_BYTES, OFF_RB = OFF_RA + TM * 4, OFF_RBF = OFF_RB + TNv * 4,
                               OFF_RBM = OFF_RBF + TNv * 4;
-    static constexpr uint32_t OFF_BAR = OFF_RBM + 32, OFF_MISC = OFF_BAR + (2 * NST + 2 * NS) * 8;
-    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;            // + slack to align the base to 1024 bytes
+    static constexpr uint32_t OFF_BAR = OFF_RBM + 32, OFF_MISC = OFF_BAR + (2 * NST + 2 * NS + NPL + 1) * 8;
+    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + NPL * 4 + 1024;            // + slack to align the base to 1024 bytes
     static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
     // instruction descriptor kind::f16: D = f32, A = B = f16, both K-major, N = TNv, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
@@ -225,13 +241,17 @@ __device__ __forceinline__ int4 le_vizinho(uint32_t end, int bloco) {
     return v;
 }
 
-template <int BLK, int MODO, int TNv, bool GRUPO>
+// SOMA: tiles in which nothing is rounded add up in tensor memory (128-wide tiles of block 32; the 64-wide ones have no registers for the second
+// drain, and block 128 drains every four MMAs as it is).  A template parameter: with the second drain in the kernel the loop of the rounded
+// tiles comes out 3 to 10 % slower.
+template <int BLK, int MODO, int TNv, bool GRUPO, bool SOMA>
 __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k_gemm_h(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                                                       const int8_t* __restrict__ RA, const int8_t* __restrict__ RB, const float* __restrict__ nA,
-                                                       const float* __restrict__ nB, SaidaGemm S, int M, int N, int K, Grade Gr, int kid) {
+                                                       const int8_t* __restrict__ RA, const int8_t* __restrict__ RB, const uint32_t* __restrict__ nA,
+                                                       const uint32_t* __restrict__ nB, SaidaGemm S, int M, int N, int K, Grade Gr, int kid) {
     using C_ = CfgH<TNv, BLK>;
-    constexpr int NST = C_::NST, NS = C_::NS, COLS = C_::COLS, LV = 16, N_EPI = C_::N_EPI, N_DW = C_::N_DW, N_MW = C_::N_MW;
+    constexpr int NST = C_::NST, NS = C_::NS, NPL = C_::NPL, COLS = C_::COLS, LV = 16, N_EPI = C_::N_EPI, N_DW = C_::N_DW, N_MW = C_::N_MW;
     constexpr int CB = BLK == 32 ? 1 : 2;                                   // chunks per tensor-memory stage: two K-blocks of 32, or one of 128
+    static_assert(!SOMA || (TNv == 128 && BLK == 32 && !GRUPO), "");
     extern __shared__ unsigned char smem_bruto[];
     unsigned char* smem = smem_bruto + ((1024u - (smem_u32(smem_bruto) & 1023u)) & 1023u);      // stays in the shared address space
     const uint32_t sbase = smem_u32(smem);
@@ -240,9 +260,10 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     int* RBs = reinterpret_cast<int*>(smem + C_::OFF_RB);
     float* RBf = reinterpret_cast<float*>(smem + C_::OFF_RBF);
     int* RBm = reinterpret_cast<int*>(smem + C_::OFF_RBM);
-    const uint32_t bar_full = sbase + C_::OFF_BAR, bar_empty = bar_full + NST * 8, bar_tfull = bar_empty + NST * 8, bar_tempty = bar_tfull + NS * 8;
+    const uint32_t bar_full = sbase + C_::OFF_BAR, bar_empty = bar_full + NST * 8, bar_tfull = bar_empty + NST * 8, bar_tempty = bar_tfull + NS * 8, bar_plano = bar_tempty + NS * 8, bar_vez = bar_plano + NPL * 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C_::OFF_MISC);
     volatile int* aborta = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 4);
+    volatile int* plano = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 16);
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int ntiles = Gr.nx * Gr.ny * Gr.partes, npedT = (K + KH - 1) / KH;
     static_assert(!GRUPO || !C_::PERSISTE, "");
@@ -252,6 +273,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     if (tid == 0) {
         for (int i = 0; i < NST; i++) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
         for (int i = 0; i < NS; i++) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, N_DW); }
+        for (int i = 0; i < NPL; i++) mbar_init(bar_plano + 8 * i, 1);
+        mbar_init(bar_vez, 1);
         *aborta = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -271,16 +294,78 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     // is how few instructions a chunk takes them (with one lane in a divergent branch the multiplying warp took 680 cycles a chunk and
     // bounded the kernel).
     if (wid == N_DW) {
-        // ------------------------------------------------------------------ loads
+        // ------------------------------------------------------------------ loads, and each tile's plan: how many chunks of K add up in
+        // tensor memory before a drain; 0: every K-block is drained and rounded.  Chunks can add up where none of their products is rounded
+        // (shift <= 4) and their sums stay below 2^24 last places of the finest product, 2^(4 - largest shift), by Cauchy-Schwarz for the
+        // whole tile.  A tile that fails anywhere is rounded throughout; that is nearly always known by its first 32 K-blocks.
+        const int nb = K / 32, gA = (M + 31) / 32;
+        uint32_t pv[4 + TNv / 32];                                           // the bounds of 32 K-blocks
+        auto pede = [&](int tile, int u0) {
+            const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, f = (tile / (Gr.nx * Gr.ny) * Gr.ppp + u0) * 2 + lane;
+#pragma unroll
+            for (int g = 0; g < 4; g++) pv[g] = f < nb ? nA[(size_t)min(m0 / 32 + g, gA - 1) * nb + f] : 0u;
+#pragma unroll
+            for (int g = 0; g < TNv / 32; g++) pv[4 + g] = f < nb ? nB[(size_t)(n0 / 32 + g) * nb + f] : 0u;
+        };
+        // the plan of a tile whose first 32 K-blocks' bounds have been asked for
+        auto planeja = [&](int tile) -> int {
+            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nuni = min(Gr.ppp, npedT - ped0);
+            unsigned serve = 0x1Fu;                                          // bit k: all aligned groups of 2^k units so far
+            for (int u0 = 0;;) {
+                uint32_t sa = 0, sb = 0;
+                float ma = 0.f, mb = 0.f;
+#pragma unroll
+                for (int g = 0; g < 4; g++) { sa = max(sa, pv[g] & 31u); ma = fmaxf(ma, __uint_as_float(pv[g])); }
+#pragma unroll
+                for (int g = 0; g < TNv / 32; g++) { sb = max(sb, pv[4 + g] & 31u); mb = fmaxf(mb, __uint_as_float(pv[4 + g])); }
+                if (u0 + lane / 2 >= nuni) ma = 0.f;                         // (another K range's)
+                int sh = ma > 0.f && mb > 0.f ? (int)(sa + sb) : 0;
+                float lim = sqrtf(ma) * sqrtf(mb) * 1.0001f;                 // of what the K-block adds to any sum, 2^-4
+                sh = max(sh, __shfl_xor_sync(FULL, sh, 1));
+                lim += __shfl_xor_sync(FULL, lim, 1);
+#pragma unroll
+                for (int k = 0; k < 5; k++) {
+                    if (!__all_sync(FULL, sh <= GG && lim * pot2(min(sh, GG)) < LIM_SOMA)) {
+                        if (k <= 1) return 0;                                // (single units: the drain as it is)
+                        serve &= (1u << k) - 1;
+                        break;
+                    }
+                    sh = max(sh, __shfl_xor_sync(FULL, sh, 2 << k));
+                    lim += __shfl_xor_sync(FULL, lim, 2 << k);
+                }
+                u0 += 16;
+                if (u0 >= nuni) return 1 << (31 - __clz(serve));
+                pede(tile, u0);
+            }
+        };
         if (*reinterpret_cast<volatile int*>(&g_sem_cargas) == 0) {
             const bool eleito = elege();
+            uint32_t nt = 0;
+            auto publica = [&](int tile) {
+                const int n = planeja(tile);
+                if (eleito) {
+                    plano[nt % NPL] = n;
+                    mbar_arrive(bar_plano + 8 * (nt % NPL));
+                }
+                nt++;
+            };
+            if (SOMA && tile0() < ntiles) pede(tile0(), 0);
             int s = 0;
             uint32_t fase = 1;
             bool ok = true;
             for (int tile = tile0(); tile < ntiles && ok; tile += GRUPO ? ntiles : gridDim.x) {
                 const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp;
                 const int xf = min(ped0 + Gr.ppp, npedT) * KH;
+                // A tile's plan is made while the one before is being loaded, the first one's behind its first loads
+                const bool primeira = tile == tile0();
+                const int prox = tile + (GRUPO ? ntiles : (int)gridDim.x), xu = max(xf - KH, 0);
+                const int xp = min(ped0 * KH + (primeira ? NST * KH : 0), xu), xq = min(xp + 2 * KH, xu);
                 for (int x = ped0 * KH; x < xf; x += KH) {
+                    if (SOMA && x == xp) {
+                        if (primeira) publica(tile);
+                        if (prox < ntiles) pede(prox, 0);
+                    }
+                    if (SOMA && x == xq && prox < ntiles) publica(prox);
                     ok = __all_sync(FULL, espera(bar_empty + 8 * s, fase, aborta, kid, 1));
                     if (!ok) break;
                     if (eleito) {
@@ -298,10 +383,55 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         const bool eleito = elege();
         const uint64_t da0 = desc_sw128(sbase), db0 = desc_sw128(sbase + A_BYTES);
         int s = 0, t = 0, vez = wid - N_DW - 1;
-        uint32_t fase = 0, fase_t = 1;
+        uint32_t fase = 0, fase_t = 1, nt = 0, nsoma = 0;                    // tiles so far, and those that added up in tensor memory
         bool ok = true;
-        for (int tile = tile0(); tile < ntiles && ok; tile += GRUPO ? ntiles : gridDim.x) {
+        for (int tile = tile0(); tile < ntiles && ok; tile += GRUPO ? ntiles : gridDim.x, nt++) {
+            int junta = 0;
+            if constexpr (SOMA) {
+                ok = __all_sync(FULL, espera(bar_plano + 8 * (nt % NPL), nt / NPL & 1, aborta, kid, 7));
+                if (!ok) break;
+                junta = plano[nt % NPL];
+            }
+            // A chunk's place in the ring is known by a parity, so a warp may look at it only when the chunk NST before it has been loaded.  In a
+            // rounded tile that is so by itself, the other warp being one stage away.  A tile that adds up belongs to one warp, each other
+            // one to this warp; whoever comes next waits until its MMAs are issued.
+            if (SOMA && nsoma && ((nsoma - 1) & 1) != (uint32_t)(wid - N_DW - 1)) {
+                ok = __all_sync(FULL, espera(bar_vez, (nsoma - 1) & 1, aborta, kid, 8));
+                if (!ok) break;
+            }
             const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
+            if (SOMA && junta) {
+                const int nuni = nped / CB, net = (nuni + junta - 1) / junta;
+                if ((nsoma & 1) == (uint32_t)(wid - N_DW - 1)) {
+                    for (int u0 = 0; u0 < nuni && ok; u0 += junta) {
+                        const int nc = min(junta, nuni - u0) * CB;
+                        const uint32_t d = tmem + t * (C_::G * TNv);
+                        ok = __all_sync(FULL, espera(bar_tempty + 8 * t, fase_t, aborta, kid, 3));
+                        for (int i = 0; i < nc && ok; i++) {
+                            ok = __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
+                            tc_fence_depois();
+                            const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
+                            if (eleito && ok) {
+#pragma unroll
+                                for (int q = 0; q < 4; q++) mma_f16(d, da + 2 * q, db + 2 * q, C_::IDESC, i | q);
+                                if (i == nc - 1) tc_commit(bar_tfull + 8 * t);
+                                tc_commit(bar_empty + 8 * s);
+                            }
+                            if (++s == NST) { s = 0; fase ^= 1; }
+                        }
+                        if (++t == NS) { t = 0; fase_t ^= 1; }
+                    }
+                    if (eleito && ok) mbar_arrive(bar_vez);
+                } else {
+                    fase ^= (s + nped) / NST & 1;
+                    s = (s + nped) % NST;
+                    fase_t ^= (t + net) / NS & 1;
+                    t = (t + net) % NS;
+                }
+                vez = wid - N_DW - 1;
+                nsoma++;
+                continue;
+            }
             for (int i = 0; i < nped && ok; i += CB) {
                 const bool minha = vez == 0;
                 vez = minha ? N_MW - 1 : vez - 1;
@@ -337,7 +467,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         const int quarto = wid & 3, cg = wid >> 2, lin = quarto * 32 + lane;
         const uint32_t base = tmem + ((uint32_t)(quarto * 32) << 16) + cg * COLS;
         int t = 0;
-        uint32_t fase_t = 0;
+        uint32_t fase_t = 0, nt = 0;
         // waits for the next stage (a wait that gives up makes all later ones return at once) / hands it back, its contents in registers
         auto recebe = [&]() {
             espera(bar_tfull + 8 * t, fase_t, aborta, kid, 4);
@@ -350,17 +480,75 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
             if (++t == NS) { t = 0; fase_t ^= 1; }
         };
-        for (int tile = tile0(); tile < ntiles; tile += GRUPO ? ntiles : gridDim.x) {
+        for (int tile = tile0(); tile < ntiles; tile += GRUPO ? ntiles : gridDim.x, nt++) {
             const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, parte = tile / (Gr.nx * Gr.ny), ped0 = parte * Gr.ppp;
             const int nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
             // the row maxima, wanted by the output stage: read now, stored to shared memory after the main loop
             int ra = 0, rb = 0;
             if (tid < TM) ra = m0 + tid < M ? (int)RA[m0 + tid] : 0;
             if (tid < TNv) rb = RB[n0 + tid];
-            int acc[COLS];
+            constexpr int PITCHv = TNv + 4;
+            // what the output stage needs goes to shared memory
+            auto tabelas = [&]() {
+                if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
+                if (tid < TM) RAs[tid] = ra;
+                if (tid < TNv) {
+                    RBs[tid] = rb;
+                    if (MODO != 1) {
+                        // what the fp32 path of the output stage needs: each block's extreme column exponents and the column scales
+                        int mn = __reduce_min_sync(FULL, rb), mx = __reduce_max_sync(FULL, rb);
+                        if (lane == 0) { RBm[wid] = mn; RBm[4 + wid] = mx; }
+                        if (BLK > 32) {                                          // one block over the four warps: place 0 gets its extremes
+                            asm volatile("bar.sync 3, %0;" ::"n"(TNv) : "memory");
+                            mn = min(min(RBm[0], RBm[1]), min(RBm[2], RBm[3]));
+                            mx = max(max(RBm[4], RBm[5]), max(RBm[6], RBm[7]));
+                            if (tid == 0) { RBm[0] = mn; RBm[4] = mx; }
+                        }
+                        RBf[tid] = pot2(min(rb - mn, 100));
+                    }
+                }
+            };
+            int junta = 0;
+            if constexpr (SOMA) junta = __all_sync(FULL, espera(bar_plano + 8 * (nt % NPL), nt / NPL & 1, aborta, kid, 9)) ? plano[nt % NPL] : 0;
+            if (SOMA && junta) {
+                // Sums of whole numbers, straight to shared memory (and added there where a tile has several): with accumulators in registers
+                // this way in and the rounding one out of the loops share them, which costs the rounding loop 5 %.
+                tabelas();
+                for (int u = 0; u < nped / CB; u += junta) {
+                    const uint32_t ta = base + t * (C_::G * TNv);
+                    recebe();
 #pragma unroll
-            for (int j = 0; j < COLS; j++) acc[j] = 0;
-            if constexpr (BLK == 32) {
+                    for (int o = 0; o < COLS; o += LV) {
+                        uint32_t a[LV], v[LV], fora = 0;
+                        tmem_pede(ta + o, a);
+                        tmem_pronto(a);
+                        if (o + LV == COLS) devolve();
+                        // (the exponent field of every sum with the constant must be that of 1.5 * 2^23, else the warp converts)
+#pragma unroll
+                        for (int k = 0; k < LV; k += 2) {
+                            v[k] = a[k]; v[k + 1] = a[k + 1];
+                            soma_magia(v[k], v[k + 1]);
+                            fora |= (v[k] ^ MAGIA) | (v[k + 1] ^ MAGIA);
+                            v[k] -= MAGIA; v[k + 1] -= MAGIA;
+                        }
+                        if (__any_sync(FULL, (fora & 0xFF800000u) != 0)) {
+#pragma unroll
+                            for (int k = 0; k < LV; k++) v[k] = (uint32_t)__float2int_rn(__uint_as_float(a[k]));
+                        }
+                        uint4* d = reinterpret_cast<uint4*>(acc_s + lin * PITCHv + cg * COLS + o);
+#pragma unroll
+                        for (int k = 0; k < LV / 4; k++) {
+                            uint4 w = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                            if (u) { const uint4 z = d[k]; w.x += z.x; w.y += z.y; w.z += z.z; w.w += z.w; }
+                            d[k] = w;
+                        }
+                    }
+                }
+            } else {
+                int acc[COLS];
+#pragma unroll
+                for (int j = 0; j < COLS; j++) acc[j] = 0;
+                if constexpr (BLK == 32) {
                 const int nb = K / 32;
                 unsigned suspeitos = 0;                                      // bit k: K-block (c & ~15) * 2 + k of this range may leave the exact window
                 for (int c = 0; c < nped; c++) {
@@ -369,8 +557,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                         const int f = (ped0 + c) * 2 + lane;
                         float pa = 0.f, pb = 0.f;
                         if (f < nb) {
-                            pa = nA[(size_t)min(m0 / 32 + quarto, (M + 31) / 32 - 1) * nb + f];
-                            pb = nB[(size_t)((n0 + cg * COLS) / 32) * nb + f];
+                            pa = __uint_as_float(nA[(size_t)min(m0 / 32 + quarto, (M + 31) / 32 - 1) * nb + f]);
+                            pb = __uint_as_float(nB[(size_t)((n0 + cg * COLS) / 32) * nb + f]);
                         }
                         suspeitos = __ballot_sync(FULL, pa * pb >= LIM_NORMA);
                     }
@@ -427,29 +615,13 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                     }
                 }
             }
-            const uint32_t vies = (uint32_t)(BLK == 32 ? nped * 2 : nped / 2) * MAGIA;
-            constexpr int PITCHv = TNv + 4;
-            if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
-            if (tid < TM) RAs[tid] = ra;
-            if (tid < TNv) {
-                RBs[tid] = rb;
-                if (MODO != 1) {
-                    // what the fp32 path of the output stage needs: each block's extreme column exponents and the column scales
-                    int mn = __reduce_min_sync(FULL, rb), mx = __reduce_max_sync(FULL, rb);
-                    if (lane == 0) { RBm[wid] = mn; RBm[4 + wid] = mx; }
-                    if (BLK > 32) {                                          // one block over the four warps: place 0 gets its extremes
-                        asm volatile("bar.sync 3, %0;" ::"n"(TNv) : "memory");
-                        mn = min(min(RBm[0], RBm[1]), min(RBm[2], RBm[3]));
-                        mx = max(max(RBm[4], RBm[5]), max(RBm[6], RBm[7]));
-                        if (tid == 0) { RBm[0] = mn; RBm[4] = mx; }
-                    }
-                    RBf[tid] = pot2(min(rb - mn, 100));
-                }
-            }
+                const uint32_t vies = (uint32_t)(BLK == 32 ? nped * 2 : nped / 2) * MAGIA;
+                tabelas();
 #pragma unroll
-            for (int j = 0; j < COLS; j += 4)
-                *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * COLS + j) =
-                    make_int4((int)((uint32_t)acc[j] - vies), (int)((uint32_t)acc[j + 1] - vies), (int)((uint32_t)acc[j + 2] - vies), (int)((uint32_t)acc[j + 3] - vies));
+                for (int j = 0; j < COLS; j += 4)
+                    *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * COLS + j) =
+                        make_int4((int)((uint32_t)acc[j] - vies), (int)((uint32_t)acc[j + 1] - vies), (int)((uint32_t)acc[j + 2] - vies), (int)((uint32_t)acc[j + 3] - vies));
+            }
             asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
             if constexpr (!GRUPO) epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s, RAs, RBs, min(TM, M - m0), m0, n0, N, S, Gr.partes > 1, parte == 0, kid, tid, RBf, RBm);
             else {

@@ -456,6 +456,66 @@ def test_gemm_produtos_parciais_grandes(amb, caso, tn, via):
         oc.lib.jt_gemm_via(0)
 
 
+@pytest.mark.parametrize("caso", ["um expoente", "dois", "saturado", "saturado a 4", "sem blocos", "um bloco fora"])
+@pytest.mark.parametrize("M,N,K", [(64, 128, 32), (192, 256, 160), (128, 128, 992), (128, 128, 1024)])
+def test_gemm_somas_em_memoria_de_tensor(amb, caso, M, N, K):
+    """Tiles whose K-blocks need no rounding (exponents within 4 of their rows' maxima, both sides together) add up in tensor memory: one
+    sum, several where the bound on the sums (2^24 last places) splits them, and none where one K-block of one row lies further down."""
+    ops, oc, reg = amb
+    ops.define_blk(32)
+    assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(128) == 0
+    try:
+        reg.novo_passo(0)
+        G = casos.Gen(77, 32)
+        A, B = G.bloco(M, K, espalha=0), G.bloco(N, K, espalha=0)
+        nb = K // 32
+        if caso == "dois":                            # shifts 0 to 2 on either side
+            A, B = (A[0], -8 - torch.randint(0, 3, (M, nb), generator=G.g).to(torch.int8)), (B[0], -8 - torch.randint(0, 3, (N, nb), generator=G.g).to(torch.int8))
+        elif caso.startswith("saturado"):             # the largest sums there are; "a 4": in units of 1, all but the first K-block
+            A, B = (torch.full_like(A[0], 127), A[1].clone()), (torch.full_like(B[0], -127), B[1].clone())
+            if caso == "saturado a 4":
+                A[1][:, 1:] -= 4
+        elif caso == "sem blocos":                    # all-zero K-blocks, exponents far down: they round nothing
+            A[0][:, 32:64] = 0
+            A[1][:, 1:2] = -127
+        elif caso == "um bloco fora":
+            A[1][M // 2, nb - 1] -= 5
+            A[0][M // 2] |= 1
+        for cru in (False, True):
+            outs = casos.plano(oc.gemm(para_gpu(A), para_gpu(B), cru=cru))
+            torch.cuda.synchronize()
+            compara(f"gemm {caso} {M}x{N}x{K} cru {cru}", outs, casos.plano(spec.Spec(32).gemm(A, B, cru=cru)))
+    finally:
+        oc.lib.jt_gemm_tn(0)
+        oc.lib.jt_gemm_via(0)
+
+
+@pytest.mark.parametrize("K", [64, 96, 512, 1024])
+def test_gemm_somas_e_arredondamentos_alternados(amb, K):
+    """More tiles than SMs, so that a block works through several: some add up in tensor memory, some round, in every order."""
+    ops, oc, reg = amb
+    ops.define_blk(32)
+    g = torch.Generator(device=DEV).manual_seed(K)
+    M, N = 2560, 1024                                 # 160 tiles
+    def bloco(R, quem):
+        m = torch.randint(-127, 128, (R, K), generator=g, device=DEV, dtype=torch.int32).to(torch.int8)
+        e = torch.randint(-8, -6, (R, K // 32), generator=g, device=DEV, dtype=torch.int32)
+        e -= 6 * (torch.randint(0, 2, (R // 128,), generator=g, device=DEV).repeat_interleave(128)[:, None] * torch.randint(0, 2, e.shape, generator=g, device=DEV)) * quem
+        return m, e.to(torch.int8)
+    A, B = bloco(M, 1), bloco(N, 0)
+    reg.novo_passo(0)
+    try:
+        for cru in (False, True):
+            assert oc.lib.jt_gemm_via(2) == 0
+            quer = oc.gemm(A, B, cru=cru)
+            assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(128) == 0
+            tem = oc.gemm(A, B, cru=cru)
+            assert all(torch.equal(x, y) for x, y in zip(quer, tem))
+    finally:
+        oc.lib.jt_gemm_tn(0)
+        oc.lib.jt_gemm_via(0)
+
+
 @pytest.mark.parametrize("limite", [False, True])
 @pytest.mark.parametrize("blk,Bt,T,H,D", [(32, 2, 128, 2, 128), (32, 1, 192, 2, 128), (32, 1, 160, 2, 128), (32, 2, 256, 8, 512), (128, 2, 128, 2, 128),
                                          (32, 1, 704, 1, 64), (32, 1, 320, 3, 192)])
