@@ -24,6 +24,7 @@
 // issues its MMAs (480 cycles a chunk, against 790 for a rounded one): 16384 x 4096 x 1024 with ReLU^2 290 -> 185 us, 16384 x 1024 x 1024 77 -> 55.
 #pragma once
 #include "gemm_tc.cuh"
+#include "gemm_h_ordem.cuh"
 
 namespace jt {
 namespace th {
@@ -163,10 +164,9 @@ struct CfgH {
     static constexpr int COLS = TNv / (N_DW / 4);                           // accumulator columns of a drain thread: 32
     static constexpr int G = BLK == 32 ? 2 : 1;                             // K-blocks handed over together
     static constexpr int NS = 512 / CTAS / (G * TNv);                       // tensor-memory stages of G x TNv columns
-    static constexpr int N_MW = 2, N_THR = N_EPI + 32 + 32 * N_MW;          // multiplying warps: each takes every N_MW-th stage
+    static constexpr int N_THR = N_EPI + 32 + 32 * N_MW;          // multiplying warps: each takes every N_MW-th stage
     static_assert(NS >= N_MW && COLS == 32, "");
     static constexpr uint32_t B_BYTES = TNv * 128, STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int NST = 4, NPL = 8;                                  // NPL: tiles whose plans are kept (the loads are at most 6 ahead of a drain)
     // the staged accumulators: memory of their own where the loads of the next tile go on meanwhile, else the operand ring (when a
     // drain thread stores them it has seen the commit of the last MMA)
     static constexpr uint32_t ACC_BYTES = TM * (TNv + 4) * 4, OFF_ACC = PERSISTE ? NST * STAGE_BYTES : 0;
@@ -179,11 +179,6 @@ struct CfgH {
     // instruction descriptor kind::f16: D = f32, A = B = f16, both K-major, N = TNv, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 };
-// how the tiles are numbered: columns fastest, then rows, then K ranges
-// With GRUPO the K ranges of a tile are the blocks of a cluster (one tile per block): each leaves its accumulators in shared memory, and each
-// puts out 1 / partes of the rows, summed over the cluster.
-struct Grade { int nx, ny, partes, ppp; };                                  // tiles per row and column, K ranges, 64-element chunks per range
-
 // one lane of a converged warp
 __device__ __forceinline__ bool elege() {
     uint32_t p;
@@ -249,7 +244,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                                                        const int8_t* __restrict__ RA, const int8_t* __restrict__ RB, const uint32_t* __restrict__ nA,
                                                        const uint32_t* __restrict__ nB, SaidaGemm S, int M, int N, int K, Grade Gr, int kid) {
     using C_ = CfgH<TNv, BLK>;
-    constexpr int NST = C_::NST, NS = C_::NS, NPL = C_::NPL, COLS = C_::COLS, LV = 16, N_EPI = C_::N_EPI, N_DW = C_::N_DW, N_MW = C_::N_MW;
+    constexpr int NS = C_::NS, COLS = C_::COLS, LV = 16, N_EPI = C_::N_EPI, N_DW = C_::N_DW;
     constexpr int CB = BLK == 32 ? 1 : 2;                                   // chunks per tensor-memory stage: two K-blocks of 32, or one of 128
     static_assert(!SOMA || (TNv == 128 && BLK == 32 && !GRUPO), "");
     extern __shared__ unsigned char smem_bruto[];
@@ -267,8 +262,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int ntiles = Gr.nx * Gr.ny * Gr.partes, npedT = (K + KH - 1) / KH;
     static_assert(!GRUPO || !C_::PERSISTE, "");
-    // the first tile of this block: in a cluster the K ranges lie next to each other
-    auto tile0 = [&]() -> int { return GRUPO ? (int)blockIdx.x / Gr.partes + (int)blockIdx.x % Gr.partes * (Gr.nx * Gr.ny) : (int)blockIdx.x; };
+    // the tiles of this block: in a cluster the K ranges lie next to each other
+    const Percurso Pc = {GRUPO ? (int)blockIdx.x / Gr.partes + (int)blockIdx.x % Gr.partes * (Gr.nx * Gr.ny) : (int)blockIdx.x, GRUPO ? ntiles : (int)gridDim.x, ntiles, npedT};
 
     if (tid == 0) {
         for (int i = 0; i < NST; i++) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
@@ -298,170 +293,121 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         // tensor memory before a drain; 0: every K-block is drained and rounded.  Chunks can add up where none of their products is rounded
         // (shift <= 4) and their sums stay below 2^24 last places of the finest product, 2^(4 - largest shift), by Cauchy-Schwarz for the
         // whole tile.  A tile that fails anywhere is rounded throughout; that is nearly always known by its first 32 K-blocks.
-        const int nb = K / 32, gA = (M + 31) / 32;
-        uint32_t pv[4 + TNv / 32];                                           // the bounds of 32 K-blocks
-        auto pede = [&](int tile, int u0) {
-            const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, f = (tile / (Gr.nx * Gr.ny) * Gr.ppp + u0) * 2 + lane;
+        struct {
+            const CUtensorMap *mapA, *mapB;
+            const uint32_t *nA, *nB;
+            volatile int *aborta, *plano;
+            Grade Gr;
+            uint32_t sbase, bar_full, bar_empty, bar_plano;
+            int lane, kid, nb, gA, npedT;
+            bool eleito;
+            int n0, m0;                                                      // of the tile that is being loaded
+            uint32_t pv[4 + TNv / 32];                                       // the bounds of 32 K-blocks
+            __device__ __forceinline__ void pede(int tile, int u0 = 0) {
+                const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, f = (ped_ini(Gr, tile) + u0) * 2 + lane;
 #pragma unroll
-            for (int g = 0; g < 4; g++) pv[g] = f < nb ? nA[(size_t)min(m0 / 32 + g, gA - 1) * nb + f] : 0u;
+                for (int g = 0; g < 4; g++) pv[g] = f < nb ? nA[(size_t)min(m0 / 32 + g, gA - 1) * nb + f] : 0u;
 #pragma unroll
-            for (int g = 0; g < TNv / 32; g++) pv[4 + g] = f < nb ? nB[(size_t)(n0 / 32 + g) * nb + f] : 0u;
-        };
-        // the plan of a tile whose first 32 K-blocks' bounds have been asked for
-        auto planeja = [&](int tile) -> int {
-            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nuni = min(Gr.ppp, npedT - ped0);
-            unsigned serve = 0x1Fu;                                          // bit k: all aligned groups of 2^k units so far
-            for (int u0 = 0;;) {
-                uint32_t sa = 0, sb = 0;
-                float ma = 0.f, mb = 0.f;
-#pragma unroll
-                for (int g = 0; g < 4; g++) { sa = max(sa, pv[g] & 31u); ma = fmaxf(ma, __uint_as_float(pv[g])); }
-#pragma unroll
-                for (int g = 0; g < TNv / 32; g++) { sb = max(sb, pv[4 + g] & 31u); mb = fmaxf(mb, __uint_as_float(pv[4 + g])); }
-                if (u0 + lane / 2 >= nuni) ma = 0.f;                         // (another K range's)
-                int sh = ma > 0.f && mb > 0.f ? (int)(sa + sb) : 0;
-                float lim = sqrtf(ma) * sqrtf(mb) * 1.0001f;                 // of what the K-block adds to any sum, 2^-4
-                sh = max(sh, __shfl_xor_sync(FULL, sh, 1));
-                lim += __shfl_xor_sync(FULL, lim, 1);
-#pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    if (!__all_sync(FULL, sh <= GG && lim * pot2(min(sh, GG)) < LIM_SOMA)) {
-                        if (k <= 1) return 0;                                // (single units: the drain as it is)
-                        serve &= (1u << k) - 1;
-                        break;
-                    }
-                    sh = max(sh, __shfl_xor_sync(FULL, sh, 2 << k));
-                    lim += __shfl_xor_sync(FULL, lim, 2 << k);
-                }
-                u0 += 16;
-                if (u0 >= nuni) return 1 << (31 - __clz(serve));
-                pede(tile, u0);
+                for (int g = 0; g < TNv / 32; g++) pv[4 + g] = f < nb ? nB[(size_t)(n0 / 32 + g) * nb + f] : 0u;
             }
-        };
-        if (*reinterpret_cast<volatile int*>(&g_sem_cargas) == 0) {
-            const bool eleito = elege();
-            uint32_t nt = 0;
-            auto publica = [&](int tile) {
+            // the plan of a tile whose first 32 K-blocks' bounds have been asked for
+            __device__ __forceinline__ int planeja(int tile) {
+                const int nuni = min(Gr.ppp, npedT - ped_ini(Gr, tile));
+                unsigned serve = 0x1Fu;                                      // bit k: all aligned groups of 2^k units so far
+                for (int u0 = 0;;) {
+                    uint32_t sa = 0, sb = 0;
+                    float ma = 0.f, mb = 0.f;
+#pragma unroll
+                    for (int g = 0; g < 4; g++) { sa = max(sa, pv[g] & 31u); ma = fmaxf(ma, __uint_as_float(pv[g])); }
+#pragma unroll
+                    for (int g = 0; g < TNv / 32; g++) { sb = max(sb, pv[4 + g] & 31u); mb = fmaxf(mb, __uint_as_float(pv[4 + g])); }
+                    if (u0 + lane / 2 >= nuni) ma = 0.f;                     // (another K range's)
+                    int sh = ma > 0.f && mb > 0.f ? (int)(sa + sb) : 0;
+                    float lim = sqrtf(ma) * sqrtf(mb) * 1.0001f;             // of what the K-block adds to any sum, 2^-4
+                    sh = max(sh, __shfl_xor_sync(FULL, sh, 1));
+                    lim += __shfl_xor_sync(FULL, lim, 1);
+#pragma unroll
+                    for (int k = 0; k < 5; k++) {
+                        if (!__all_sync(FULL, sh <= GG && lim * pot2(min(sh, GG)) < LIM_SOMA)) {
+                            if (k <= 1) return 0;                            // (single units: the drain as it is)
+                            serve &= (1u << k) - 1;
+                            break;
+                        }
+                        sh = max(sh, __shfl_xor_sync(FULL, sh, 2 << k));
+                        lim += __shfl_xor_sync(FULL, lim, 2 << k);
+                    }
+                    u0 += 16;
+                    if (u0 >= nuni) return 1 << (31 - __clz(serve));
+                    pede(tile, u0);
+                }
+            }
+            __device__ __forceinline__ void publica(int tile, uint32_t nt) {
                 const int n = planeja(tile);
                 if (eleito) {
                     plano[nt % NPL] = n;
                     mbar_arrive(bar_plano + 8 * (nt % NPL));
                 }
-                nt++;
-            };
-            if (SOMA && tile0() < ntiles) pede(tile0(), 0);
-            int s = 0;
-            uint32_t fase = 1;
-            bool ok = true;
-            for (int tile = tile0(); tile < ntiles && ok; tile += GRUPO ? ntiles : gridDim.x) {
-                const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp;
-                const int xf = min(ped0 + Gr.ppp, npedT) * KH;
-                // A tile's plan is made while the one before is being loaded, the first one's behind its first loads
-                const bool primeira = tile == tile0();
-                const int prox = tile + (GRUPO ? ntiles : (int)gridDim.x), xu = max(xf - KH, 0);
-                const int xp = min(ped0 * KH + (primeira ? NST * KH : 0), xu), xq = min(xp + 2 * KH, xu);
-                for (int x = ped0 * KH; x < xf; x += KH) {
-                    if (SOMA && x == xp) {
-                        if (primeira) publica(tile);
-                        if (prox < ntiles) pede(prox, 0);
-                    }
-                    if (SOMA && x == xq && prox < ntiles) publica(prox);
-                    ok = __all_sync(FULL, espera(bar_empty + 8 * s, fase, aborta, kid, 1));
-                    if (!ok) break;
-                    if (eleito) {
-                        mbar_expect_tx(bar_full + 8 * s, C_::STAGE_BYTES);
-                        tma_2d(sbase + s * C_::STAGE_BYTES, &mapA, x, m0, bar_full + 8 * s);
-                        tma_2d(sbase + s * C_::STAGE_BYTES + A_BYTES, &mapB, x, n0, bar_full + 8 * s);
-                    }
-                    if (++s == NST) { s = 0; fase ^= 1; }
+            }
+            __device__ __forceinline__ bool vazio(int s, uint32_t fase) { return __all_sync(FULL, espera(bar_empty + 8 * s, fase, aborta, kid, 1)); }
+            __device__ __forceinline__ void tile(int tile) { n0 = tile % Gr.nx * TNv; m0 = tile / Gr.nx % Gr.ny * TM; }
+            __device__ __forceinline__ void carrega(int s, int c) {
+                if (eleito) {
+                    mbar_expect_tx(bar_full + 8 * s, C_::STAGE_BYTES);
+                    tma_2d(sbase + s * C_::STAGE_BYTES, mapA, c * KH, m0, bar_full + 8 * s);
+                    tma_2d(sbase + s * C_::STAGE_BYTES + A_BYTES, mapB, c * KH, n0, bar_full + 8 * s);
                 }
             }
-        }
+        } v = {&mapA, &mapB, nA, nB, aborta, plano, Gr, sbase, bar_full, bar_empty, bar_plano, lane, kid, K / 32, (M + 31) / 32, npedT, elege()};
+        if (*reinterpret_cast<volatile int*>(&g_sem_cargas) == 0) laco_cargas<SOMA>(v, Gr, Pc);
     } else if (wid > N_DW) {
-        // ------------------------------------------------------------------ MMAs.  A chunk takes a warp ~500 cycles of waits and issue, its
-        // MMAs 256: two warps take the stages in turn (every stage starts a sum of its own).
-        const bool eleito = elege();
-        const uint64_t da0 = desc_sw128(sbase), db0 = desc_sw128(sbase + A_BYTES);
-        int s = 0, t = 0, vez = wid - N_DW - 1;
-        uint32_t fase = 0, fase_t = 1, nt = 0, nsoma = 0;                    // tiles so far, and those that added up in tensor memory
-        bool ok = true;
-        for (int tile = tile0(); tile < ntiles && ok; tile += GRUPO ? ntiles : gridDim.x, nt++) {
-            int junta = 0;
-            if constexpr (SOMA) {
-                ok = __all_sync(FULL, espera(bar_plano + 8 * (nt % NPL), nt / NPL & 1, aborta, kid, 7));
-                if (!ok) break;
-                junta = plano[nt % NPL];
+        // ------------------------------------------------------------------ MMAs
+        struct {
+            volatile int *aborta, *planos;
+            uint32_t tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_vez;
+            uint64_t da0, db0;
+            int kid;
+            bool eleito;
+            __device__ __forceinline__ void tile(int) {}
+            __device__ __forceinline__ bool plano(uint32_t nt, int& junta) {
+                const bool ok = __all_sync(FULL, espera(bar_plano + 8 * (nt % NPL), nt / NPL & 1, aborta, kid, 7));
+                if (ok) junta = planos[nt % NPL];
+                return ok;
             }
-            // A chunk's place in the ring is known by a parity, so a warp may look at it only when the chunk NST before it has been loaded.  In a
-            // rounded tile that is so by itself, the other warp being one stage away.  A tile that adds up belongs to one warp, each other
-            // one to this warp; whoever comes next waits until its MMAs are issued.
-            if (SOMA && nsoma && ((nsoma - 1) & 1) != (uint32_t)(wid - N_DW - 1)) {
-                ok = __all_sync(FULL, espera(bar_vez, (nsoma - 1) & 1, aborta, kid, 8));
-                if (!ok) break;
+            __device__ __forceinline__ bool vez(uint32_t fase) { return __all_sync(FULL, espera(bar_vez, fase, aborta, kid, 8)); }
+            __device__ __forceinline__ void passa_vez() { if (eleito) mbar_arrive(bar_vez); }
+            __device__ __forceinline__ bool livre(int t, uint32_t fase) { return __all_sync(FULL, espera(bar_tempty + 8 * t, fase, aborta, kid, 3)); }
+            __device__ __forceinline__ bool cheio(int s, uint32_t fase) {
+                const bool ok = __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
+                tc_fence_depois();
+                return ok;
             }
-            const int ped0 = tile / (Gr.nx * Gr.ny) * Gr.ppp, nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
-            if (SOMA && junta) {
-                const int nuni = nped / CB, net = (nuni + junta - 1) / junta;
-                if ((nsoma & 1) == (uint32_t)(wid - N_DW - 1)) {
-                    for (int u0 = 0; u0 < nuni && ok; u0 += junta) {
-                        const int nc = min(junta, nuni - u0) * CB;
-                        const uint32_t d = tmem + t * (C_::G * TNv);
-                        ok = __all_sync(FULL, espera(bar_tempty + 8 * t, fase_t, aborta, kid, 3));
-                        for (int i = 0; i < nc && ok; i++) {
-                            ok = __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
-                            tc_fence_depois();
-                            const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
-                            if (eleito && ok) {
-#pragma unroll
-                                for (int q = 0; q < 4; q++) mma_f16(d, da + 2 * q, db + 2 * q, C_::IDESC, i | q);
-                                if (i == nc - 1) tc_commit(bar_tfull + 8 * t);
-                                tc_commit(bar_empty + 8 * s);
-                            }
-                            if (++s == NST) { s = 0; fase ^= 1; }
-                        }
-                        if (++t == NS) { t = 0; fase_t ^= 1; }
-                    }
-                    if (eleito && ok) mbar_arrive(bar_vez);
+            __device__ __forceinline__ void arredonda(int s, int t, int j, bool certo, int) {
+                const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
+                const uint32_t d = tmem + t * (C_::G * TNv);
+                if (!(eleito && certo)) return;
+                if (BLK == 32) {
+                    mma_f16(d, da, db, C_::IDESC, 0);                       // +32 bytes (16 elements of K) per instruction
+                    mma_f16(d, da + 2, db + 2, C_::IDESC, 1);
+                    mma_f16(d + TNv, da + 4, db + 4, C_::IDESC, 0);
+                    mma_f16(d + TNv, da + 6, db + 6, C_::IDESC, 1);
                 } else {
-                    fase ^= (s + nped) / NST & 1;
-                    s = (s + nped) % NST;
-                    fase_t ^= (t + net) / NS & 1;
-                    t = (t + net) % NS;
-                }
-                vez = wid - N_DW - 1;
-                nsoma++;
-                continue;
-            }
-            for (int i = 0; i < nped && ok; i += CB) {
-                const bool minha = vez == 0;
-                vez = minha ? N_MW - 1 : vez - 1;
-                if (minha) ok = __all_sync(FULL, espera(bar_tempty + 8 * t, fase_t, aborta, kid, 3));
 #pragma unroll
-                for (int j = 0; j < CB; j++) {
-                    if (minha && ok) {
-                        ok = __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
-                        tc_fence_depois();
-                        const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
-                        const uint32_t d = tmem + t * (C_::G * TNv);
-                        if (eleito && ok) {
-                            if (BLK == 32) {
-                                mma_f16(d, da, db, C_::IDESC, 0);                   // +32 bytes (16 elements of K) per instruction
-                                mma_f16(d, da + 2, db + 2, C_::IDESC, 1);
-                                mma_f16(d + TNv, da + 4, db + 4, C_::IDESC, 0);
-                                mma_f16(d + TNv, da + 6, db + 6, C_::IDESC, 1);
-                            } else {
-#pragma unroll
-                                for (int q = 0; q < 4; q++) mma_f16(d, da + 2 * q, db + 2 * q, C_::IDESC, j | q);
-                            }
-                            if (j == CB - 1) tc_commit(bar_tfull + 8 * t);
-                            tc_commit(bar_empty + 8 * s);
-                        }
-                    }
-                    if (++s == NST) { s = 0; fase ^= 1; }
+                    for (int q = 0; q < 4; q++) mma_f16(d, da + 2 * q, db + 2 * q, C_::IDESC, j | q);
                 }
-                if (++t == NS) { t = 0; fase_t ^= 1; }
+                if (j == CB - 1) tc_commit(bar_tfull + 8 * t);
+                tc_commit(bar_empty + 8 * s);
             }
-        }
+            __device__ __forceinline__ void soma(int s, int t, int i, bool fim, bool certo, int) {
+                const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
+                const uint32_t d = tmem + t * (C_::G * TNv);
+                if (!(eleito && certo)) return;
+#pragma unroll
+                for (int q = 0; q < 4; q++) mma_f16(d, da + 2 * q, db + 2 * q, C_::IDESC, i | q);
+                if (fim) tc_commit(bar_tfull + 8 * t);
+                tc_commit(bar_empty + 8 * s);
+            }
+        } v = {aborta, plano, tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_vez, desc_sw128(sbase), desc_sw128(sbase + A_BYTES), kid, elege()};
+        laco_produtos<SOMA, NS, CB>(v, Gr, Pc, wid - N_DW - 1);
     } else {
         // ------------------------------------------------------------------ drain + output stage
         const int quarto = wid & 3, cg = wid >> 2, lin = quarto * 32 + lane;
@@ -480,7 +426,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
             if (++t == NS) { t = 0; fase_t ^= 1; }
         };
-        for (int tile = tile0(); tile < ntiles; tile += GRUPO ? ntiles : gridDim.x, nt++) {
+        for (int tile = Pc.tile0; tile < ntiles; tile += Pc.passo, nt++) {
             const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, parte = tile / (Gr.nx * Gr.ny), ped0 = parte * Gr.ppp;
             const int nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
             // the row maxima, wanted by the output stage: read now, stored to shared memory after the main loop

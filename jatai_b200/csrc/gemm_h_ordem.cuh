@@ -1,0 +1,131 @@
+// The order of barriers in k_gemm_h: the loops of the warp that loads and of the warps that multiply.  They are written over an object that does what
+// they ask for.  In the kernel (gemm_h.cuh) that is the barriers, the copies and the MMAs; the test of the order compiles the same loops
+// for the host, over barriers that complete in any order the hardware may choose.
+#pragma once
+#ifdef __CUDACC__
+#define JT_LACO __device__ __forceinline__
+#define JT_DESENROLA _Pragma("unroll")
+#else
+#define JT_LACO inline
+#define JT_DESENROLA
+#endif
+
+namespace jt {
+namespace th {
+
+constexpr int NST = 4, NPL = 8, N_MW = 2;                                   // places of the operand ring, plans kept, multiplying warps
+
+// how the tiles are numbered: columns fastest, then rows, then K ranges
+// With GRUPO the K ranges of a tile are the blocks of a cluster (one tile per block): each leaves its accumulators in shared memory, and each
+// puts out 1 / partes of the rows, summed over the cluster.
+struct Grade { int nx, ny, partes, ppp; };                                  // tiles per row and column, K ranges, 64-element chunks per range
+struct Percurso { int tile0, passo, ntiles, npedT; };                       // a block's tiles: tile0, tile0 + passo, ...; chunks of the whole K
+
+// first chunk of a tile and the one after its last
+JT_LACO int ped_ini(const Grade& G, int tile) { return tile / (G.nx * G.ny) * G.ppp; }
+JT_LACO int ped_fim(const Grade& G, const Percurso& P, int tile) { const int f = ped_ini(G, tile) + G.ppp; return f < P.npedT ? f : P.npedT; }
+
+// ------------------------------------------------------------------------------------------ loads
+// v: vazio(s, phase)  waits until place s of the operand ring has been read (false: given up)
+//    tile(tile)      the tile whose chunks follow;  carrega(s, c)  has its chunk c copied there
+//    pede(tile), publica(tile, nt)  ask for what the tile's plan is made of; make the plan and hand it over as that of the block's nt-th tile
+template <bool SOMA, class V>
+JT_LACO void laco_cargas(V& v, const Grade& G, const Percurso& P) {
+    if (SOMA && P.tile0 < P.ntiles) v.pede(P.tile0);
+    int s = 0;
+    unsigned fase = 1, nt = 0;
+    bool ok = true;
+    for (int tile = P.tile0; tile < P.ntiles && ok; tile += P.passo) {
+        const int c0 = ped_ini(G, tile), cf = ped_fim(G, P, tile);
+        v.tile(tile);
+        // A tile's plan is made while the one before is being loaded, the first one's behind its first loads
+        const bool primeira = tile == P.tile0;
+        const int prox = tile + P.passo, cu = cf - 1 > 0 ? cf - 1 : 0;
+        const int x = c0 + (primeira ? NST : 0), cp = x < cu ? x : cu, cq = cp + 2 < cu ? cp + 2 : cu;
+        for (int c = c0; c < cf; c++) {
+            if (SOMA && c == cp) {
+                if (primeira) v.publica(tile, nt++);
+                if (prox < P.ntiles) v.pede(prox);
+            }
+            if (SOMA && c == cq && prox < P.ntiles) v.publica(prox, nt++);
+            ok = v.vazio(s, fase);
+            if (!ok) break;
+            v.carrega(s, c);
+            if (++s == NST) { s = 0; fase ^= 1; }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------ MMAs
+// A chunk takes a warp ~500 cycles of waits and issue, its MMAs 256: two warps take the stages of a rounded tile in turn (every stage starts a
+// sum of its own).  NS: tensor-memory stages; CB: chunks per stage that is rounded; eu: this warp's number.
+// v: plano(nt, junta)  waits for the plan of the block's nt-th tile
+//    livre(t, phase)   waits until tensor-memory stage t has been drained
+//    cheio(s, phase)   waits until place s of the ring has been loaded
+//    arredonda(s, t, j, certo, c) / soma(s, t, i, fim, certo, c)  if `certo`, issue the MMAs of chunk c onto stage t: chunk j of a stage that is rounded / chunk i of a sum,
+//                      `fim` its last; each commits the ring's place, the last of a stage the stage too
+//    vez(phase), passa_vez()  the hand-over behind a tile that adds up
+// All waits return false when they have given up.
+template <bool SOMA, int NS, int CB, class V>
+JT_LACO void laco_produtos(V& v, const Grade& G, const Percurso& P, int eu) {
+    int s = 0, t = 0, vez = eu;
+    unsigned fase = 0, fase_t = 1, nt = 0, nsoma = 0;                       // tiles so far, and those that added up in tensor memory
+    bool ok = true;
+    for (int tile = P.tile0; tile < P.ntiles && ok; tile += P.passo, nt++) {
+        v.tile(tile);
+        int junta = 0;
+        if (SOMA) {
+            ok = v.plano(nt, junta);
+            if (!ok) break;
+        }
+        // A chunk's place in the ring is known by a parity, so a warp may look at it only when the chunk NST before it has been loaded.  In a
+        // rounded tile that is so by itself, the other warp being one stage away.  A tile that adds up belongs to one warp, each other
+        // one to this warp; whoever comes next waits until its MMAs are issued.
+        if (SOMA && nsoma && ((nsoma - 1) & 1) != (unsigned)eu) {
+            ok = v.vez((nsoma - 1) & 1);
+            if (!ok) break;
+        }
+        const int c0 = ped_ini(G, tile), cf = ped_fim(G, P, tile), nped = cf > c0 ? cf - c0 : 0;
+        if (SOMA && junta) {
+            const int nuni = nped / CB, net = (nuni + junta - 1) / junta;
+            if ((nsoma & 1) == (unsigned)eu) {
+                for (int u0 = 0; u0 < nuni && ok; u0 += junta) {
+                    const int nc = (junta < nuni - u0 ? junta : nuni - u0) * CB;
+                    ok = v.livre(t, fase_t);
+                    for (int i = 0; i < nc && ok; i++) {
+                        ok = v.cheio(s, fase);
+                        v.soma(s, t, i, i == nc - 1, ok, c0 + u0 * CB + i);
+                        if (++s == NST) { s = 0; fase ^= 1; }
+                    }
+                    if (++t == NS) { t = 0; fase_t ^= 1; }
+                }
+                if (ok) v.passa_vez();
+            } else {
+                fase ^= (s + nped) / NST & 1;
+                s = (s + nped) % NST;
+                fase_t ^= (t + net) / NS & 1;
+                t = (t + net) % NS;
+            }
+            vez = eu;
+            nsoma++;
+            continue;
+        }
+        for (int i = 0; i < nped && ok; i += CB) {
+            const bool minha = vez == 0;
+            vez = minha ? N_MW - 1 : vez - 1;
+            if (minha) ok = v.livre(t, fase_t);
+JT_DESENROLA
+            for (int j = 0; j < CB; j++) {
+                if (minha && ok) {
+                    ok = v.cheio(s, fase);
+                    v.arredonda(s, t, j, ok, c0 + i + j);
+                }
+                if (++s == NST) { s = 0; fase ^= 1; }
+            }
+            if (++t == NS) { t = 0; fase_t ^= 1; }
+        }
+    }
+}
+
+}  // namespace th
+}  // namespace jt
