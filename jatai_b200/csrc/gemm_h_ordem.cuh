@@ -13,7 +13,11 @@
 namespace jt {
 namespace th {
 
-constexpr int NST = 4, NPL = 8, N_MW = 2;                                   // places of the operand ring, plans kept, multiplying warps
+constexpr int NST = 4, N_MW = 2;                                            // places of the operand ring, multiplying warps
+// Plans kept.  With one chunk per tile the loading warp has plan n + 1 ready when tile n - 5 has been multiplied.  A drain warp has read those up to
+// n - 7 by then.  A multiplying warp may be three tiles behind (its own sum, then a rounded tile, a sum and a rounded tile of the
+// other warp's): it has read those up to n - 9.
+constexpr int NPL = 16;
 
 // how the tiles are numbered: columns fastest, then rows, then K ranges
 // With GRUPO the K ranges of a tile are the blocks of a cluster (one tile per block): each leaves its accumulators in shared memory, and each

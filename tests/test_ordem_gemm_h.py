@@ -23,3 +23,9 @@ def test_cada_pedaco_uma_vez(programa, tiles, pedacos):
         pedacos *= 2                                   # (a K-block of 128 is two chunks)
     r = subprocess.run([programa, tiles, str(pedacos), "400"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_um_pedaco_por_tile(programa):
+    """Tiles of one chunk (K <= 64), rounded and summed ones in any order: a multiplying warp that falls behind still finds its plans."""
+    r = subprocess.run([programa, "mixed", "1", "2000"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
