@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     int* RBs = reinterpret_cast<int*>(smem + C_::OFF_RB);
     float* RBf = reinterpret_cast<float*>(smem + C_::OFF_RBF);
     int* RBm = reinterpret_cast<int*>(smem + C_::OFF_RBM);
-    const uint32_t bar_full = sbase + C_::OFF_BAR, bar_empty = bar_full + NST * 8, bar_tfull = bar_empty + NST * 8, bar_tempty = bar_tfull + NS * 8, bar_plano = bar_tempty + NS * 8, bar_vez = bar_plano + NPL * 8;
+    const uint32_t bar_full = sbase + C_::OFF_BAR, bar_empty = bar_full + NST * 8, bar_tfull = bar_empty + NST * 8, bar_tempty = bar_tfull + NS * 8, bar_plano = bar_tempty + NS * 8, bar_encontro = bar_plano + NPL * 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C_::OFF_MISC);
     volatile int* aborta = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 4);
     volatile int* plano = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 16);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         for (int i = 0; i < NST; i++) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
         for (int i = 0; i < NS; i++) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, N_DW); }
         for (int i = 0; i < NPL; i++) mbar_init(bar_plano + 8 * i, 1);
-        mbar_init(bar_vez, 1);
+        mbar_init(bar_encontro, N_MW);
         *aborta = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         // ------------------------------------------------------------------ MMAs
         struct {
             volatile int *aborta, *planos;
-            uint32_t tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_vez;
+            uint32_t tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_encontro;
             uint64_t da0, db0;
             int kid;
             bool eleito;
@@ -373,8 +373,11 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                 if (ok) junta = planos[nt % NPL];
                 return ok;
             }
-            __device__ __forceinline__ bool vez(uint32_t fase) { return __all_sync(FULL, espera(bar_vez, fase, aborta, kid, 8)); }
-            __device__ __forceinline__ void passa_vez() { if (eleito) mbar_arrive(bar_vez); }
+            __device__ __forceinline__ bool encontra(uint32_t fase) {
+                __syncwarp();
+                if (eleito) mbar_arrive(bar_encontro);
+                return __all_sync(FULL, espera(bar_encontro, fase, aborta, kid, 8));
+            }
             __device__ __forceinline__ bool livre(int t, uint32_t fase) { return __all_sync(FULL, espera(bar_tempty + 8 * t, fase, aborta, kid, 3)); }
             __device__ __forceinline__ bool cheio(int s, uint32_t fase) {
                 const bool ok = __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
@@ -406,7 +409,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                 if (fim) tc_commit(bar_tfull + 8 * t);
                 tc_commit(bar_empty + 8 * s);
             }
-        } v = {aborta, plano, tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_vez, desc_sw128(sbase), desc_sw128(sbase + A_BYTES), kid, elege()};
+        } v = {aborta, plano, tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_encontro, desc_sw128(sbase), desc_sw128(sbase + A_BYTES), kid, elege()};
         laco_produtos<SOMA, NS, CB>(v, Gr, Pc, wid - N_DW - 1);
     } else {
         // ------------------------------------------------------------------ drain + output stage

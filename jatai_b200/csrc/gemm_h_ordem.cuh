@@ -14,9 +14,8 @@ namespace jt {
 namespace th {
 
 constexpr int NST = 4, N_MW = 2;                                            // places of the operand ring, multiplying warps
-// Plans kept.  With one chunk per tile the loading warp has plan n + 1 ready when tile n - 5 has been multiplied.  A drain warp has read those up to
-// n - 7 by then.  A multiplying warp may be three tiles behind (its own sum, then a rounded tile, a sum and a rounded tile of the
-// other warp's): it has read those up to n - 9.
+// Plans kept.  With one chunk per tile the loading warp has plan n + 1 ready when tile n - 5 has been multiplied; the drain warps have read those up to
+// n - 7 by then, the multiplying warps, which take rounded tiles in turn and meet at those that add up, those up to n - 6.
 constexpr int NPL = 16;
 
 // how the tiles are numbered: columns fastest, then rows, then K ranges
@@ -68,13 +67,13 @@ JT_LACO void laco_cargas(V& v, const Grade& G, const Percurso& P) {
 //    cheio(s, phase)   waits until place s of the ring has been loaded
 //    arredonda(s, t, j, certo, c) / soma(s, t, i, fim, certo, c)  if `certo`, issue the MMAs of chunk c onto stage t: chunk j of a stage that is rounded / chunk i of a sum,
 //                      `fim` its last; each commits the ring's place, the last of a stage the stage too
-//    vez(phase), passa_vez()  the hand-over behind a tile that adds up
+//    encontra(phase)   arrives where the multiplying warps meet and waits for the other
 // All waits return false when they have given up.
 template <bool SOMA, int NS, int CB, class V>
 JT_LACO void laco_produtos(V& v, const Grade& G, const Percurso& P, int eu) {
     int s = 0, t = 0, vez = eu;
-    unsigned fase = 0, fase_t = 1, nt = 0, nsoma = 0;                       // tiles so far, and those that added up in tensor memory
-    bool ok = true;
+    unsigned fase = 0, fase_t = 1, nt = 0, encontros = 0;
+    bool ok = true, soma_antes = false;
     for (int tile = P.tile0; tile < P.ntiles && ok; tile += P.passo, nt++) {
         v.tile(tile);
         int junta = 0;
@@ -82,17 +81,19 @@ JT_LACO void laco_produtos(V& v, const Grade& G, const Percurso& P, int eu) {
             ok = v.plano(nt, junta);
             if (!ok) break;
         }
-        // A chunk's place in the ring is known by a parity, so a warp may look at it only when the chunk NST before it has been loaded.  In a
-        // rounded tile that is so by itself, the other warp being one stage away.  A tile that adds up belongs to one warp, each other
-        // one to this warp; whoever comes next waits until its MMAs are issued.
-        if (SOMA && nsoma && ((nsoma - 1) & 1) != (unsigned)eu) {
-            ok = v.vez((nsoma - 1) & 1);
+        // A phase is known by its parity, so a warp may look at a place of the ring only when it is known that the chunk NST before has been loaded, and
+        // at a stage only when its drain before last is known.  Within a rounded tile the waits for the stages see to both, the other warp
+        // being one stage away.  A tile that adds up is one warp's, which does not see what the other waits for: around one the warps
+        // meet, and what the tiles before it waited for has then come for both.
+        if (SOMA && (junta || soma_antes)) {
+            ok = v.encontra(encontros++ & 1);
             if (!ok) break;
         }
+        soma_antes = junta;
         const int c0 = ped_ini(G, tile), cf = ped_fim(G, P, tile), nped = cf > c0 ? cf - c0 : 0;
         if (SOMA && junta) {
             const int nuni = nped / CB, net = (nuni + junta - 1) / junta;
-            if ((nsoma & 1) == (unsigned)eu) {
+            if (eu == 0) {
                 for (int u0 = 0; u0 < nuni && ok; u0 += junta) {
                     const int nc = (junta < nuni - u0 ? junta : nuni - u0) * CB;
                     ok = v.livre(t, fase_t);
@@ -103,15 +104,12 @@ JT_LACO void laco_produtos(V& v, const Grade& G, const Percurso& P, int eu) {
                     }
                     if (++t == NS) { t = 0; fase_t ^= 1; }
                 }
-                if (ok) v.passa_vez();
             } else {
                 fase ^= (s + nped) / NST & 1;
                 s = (s + nped) % NST;
                 fase_t ^= (t + net) / NS & 1;
                 t = (t + net) % NS;
             }
-            vez = eu;
-            nsoma++;
             continue;
         }
         for (int i = 0; i < nped && ok; i += CB) {

@@ -113,7 +113,7 @@ struct Bloco {
     std::vector<int> planos_certos;
     Grade G;
     Percurso P;
-    Barra cheio[NST], vazio[NST], tcheio[NS], tlivre[NS], plano_b[NPL], vez_b;
+    Barra cheio[NST], vazio[NST], tcheio[NS], tlivre[NS], plano_b[NPL], encontro_b;
     int planos[NPL] = {};
     struct Lugar { int tile = -1, c = -1; bool vem = false; } anel[NST];
     struct Estagio { int tile = -1; std::vector<int> c; int le = 0; bool usado = false; } tmem[NS];
@@ -129,7 +129,7 @@ struct Bloco {
         for (auto& b : tcheio) b.cria(S, 1);
         for (auto& b : tlivre) b.cria(S, N_DW);
         for (auto& b : plano_b) b.cria(S, 1);
-        vez_b.cria(S, 1);
+        encontro_b.cria(S, N_MW);
     }
 
     struct Carrega {
@@ -177,8 +177,7 @@ struct Bloco {
             if (junta != B.planos_certos[t]) throw Falha{"a multiplying warp reads another tile's plan"};
             return ok;
         }
-        bool vez(unsigned fase) { return B.vez_b.espera(fase); }
-        void passa_vez() { B.vez_b.chega(); }
+        bool encontra(unsigned fase) { B.encontro_b.chega(); return B.encontro_b.espera(fase); }
         bool livre(int s, unsigned fase) { return B.tlivre[s].espera(fase); }
         bool cheio(int s, unsigned fase) { return B.cheio[s].espera(fase); }
         void arredonda(int s, int st, int j, bool, int c) { B.emite(s, st, j == 0, j == CB - 1, t, c); B.S.passa(B.S.demora(0.2)); }

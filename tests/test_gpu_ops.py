@@ -516,6 +516,39 @@ def test_gemm_somas_e_arredondamentos_alternados(amb, K):
         oc.lib.jt_gemm_via(0)
 
 
+@pytest.mark.parametrize("op", ["gemm", "gemm_soma", "gemm_relu2", "gemm_relu2_back"])
+@pytest.mark.parametrize("K,arredonda", [(64, 0.5), (96, 0.3), (320, 0.5), (512, 0.8), (1024, 0.1), (1024, 0.5)])
+def test_gemm_somas_e_arredondamentos_treze_tiles_por_bloco(amb, K, arredonda, op):
+    """2032 tiles, 13 or 14 to a block, in random order: tiles that round (a share of the bands of 128 rows), that add up in one sum, and in sums of 8, 4
+    and 2 chunks (blocks at the ends of the mantissas' range, up to 1, 2 or 3 places below their rows' maxima).  Every output stage that
+    the summing kernel has, the last band of rows half full, against the CUDA-core kernel."""
+    ops, oc, reg = amb
+    ops.define_blk(32)
+    g = torch.Generator(device=DEV).manual_seed(1000 * K + int(10 * arredonda))
+    M, N = 127 * 128 - 64, 2048
+    ints = lambda a, b, forma: torch.randint(a, b + 1, forma, generator=g, device=DEV, dtype=torch.int32)
+    faixa = torch.arange(M, device=DEV) // 128
+    arr = (torch.rand(127, generator=g, device=DEV) < arredonda)[faixa]
+    desce = ints(0, 3, (127,))[faixa]                              # 0: one sum; 1 to 3: several
+    m = torch.where((desce > 0)[:, None], 254 * ints(0, 1, (M, K)) - 127, ints(-127, 127, (M, K)))
+    e = -8 - torch.remainder(ints(0, 1 << 20, (M, K // 32)), (desce + 1)[:, None])
+    e -= 9 * (arr[:, None] & (ints(0, 2, e.shape) == 0)).to(torch.int32)
+    A = (m.to(torch.int8), e.to(torch.int8))
+    B = ((254 * ints(0, 1, (N, K)) - 127).to(torch.int8), torch.full((N, K // 32), -8, device=DEV, dtype=torch.int8))
+    X = (ints(-127, 127, (M, N)).to(torch.int8), ints(-12, -4, (M, N // 32)).to(torch.int8))
+    args = {"gemm": (A, B), "gemm_soma": (A, B, X), "gemm_relu2": (A, B), "gemm_relu2_back": (A, B, X)}[op]
+    reg.novo_passo(0)
+    try:
+        assert oc.lib.jt_gemm_via(2) == 0
+        quer = casos.roda(oc, op, args, {})
+        assert oc.lib.jt_gemm_via(4) == 0
+        for _ in range(3):
+            tem = casos.roda(oc, op, args, {})
+            assert len(quer) == len(tem) and all(torch.equal(x, y) for x, y in zip(quer, tem))
+    finally:
+        oc.lib.jt_gemm_via(0)
+
+
 @pytest.mark.parametrize("limite", [False, True])
 @pytest.mark.parametrize("blk,Bt,T,H,D", [(32, 2, 128, 2, 128), (32, 1, 192, 2, 128), (32, 1, 160, 2, 128), (32, 2, 256, 8, 512), (128, 2, 128, 2, 128),
                                          (32, 1, 704, 1, 64), (32, 1, 320, 3, 192)])

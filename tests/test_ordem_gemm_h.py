@@ -29,3 +29,11 @@ def test_um_pedaco_por_tile(programa):
     """Tiles of one chunk (K <= 64), rounded and summed ones in any order: a multiplying warp that falls behind still finds its plans."""
     r = subprocess.run([programa, "mixed", "1", "2000"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("pedacos", [2, 3, 4, 5, 8, 12, 16])
+def test_arredondados_e_somados(programa, pedacos):
+    """Rounded and summed tiles in any order, sums of 2 to 16 chunks: no multiplying warp takes a chunk for loaded, or a stage for drained, by the parity
+    of a phase that it has not followed."""
+    r = subprocess.run([programa, "mixed", str(pedacos), "2000"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
