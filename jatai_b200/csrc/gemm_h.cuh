@@ -20,8 +20,8 @@
 // Where sa + sb <= 4 nothing is rounded at all: r is a whole number.  A tile in which that holds for every K-block (what a step multiplies by
 // its weights nearly always is: normalised rows and weights have block exponents one or two apart) need not be drained K-block by
 // K-block; its chunks add up in tensor memory, in fp32, exactly while the sum of the bounds stays below 2^24 last places.  Large
-// products with K <= 1024 look for it, with the norms and the largest shift that k_prep_h leaves.  Drained once, a tile is bound by what
-// issues its MMAs (480 cycles a chunk, against 790 for a rounded one): 16384 x 4096 x 1024 with ReLU^2 290 -> 185 us, 16384 x 1024 x 1024 77 -> 55.
+// products with K <= 1024 look for it, with the norms and the largest shift that k_prep_h leaves: 16384 x 4096 x 1024 with ReLU^2 290 -> 168 us,
+// 16384 x 1024 x 1024 77 -> 50.5.  Drained once, a tile waits for nothing but its operands, its MMAs and the output stage of the one before.
 #pragma once
 #include "gemm_tc.cuh"
 #include "gemm_h_ordem.cuh"
@@ -34,6 +34,7 @@ using namespace tc;
 constexpr int KH = 64;                                     // K elements per operand stage: 128 bytes of f16, one swizzle row
 constexpr float LIM_NORMA = 68719000000.0f;               // just below 2^36 (the product of two fp32 roundings included)
 constexpr float LIM_SOMA = 16770000.0f;                    // just below 2^24
+constexpr int N_PLANOS = 2048;                             // tiles of a block whose plans are kept, a byte each
 
 // ------------------------------------------------------------------------------------------ operand preparation
 struct ArgsPrepH {
@@ -173,8 +174,8 @@ struct CfgH {
     static_assert(PERSISTE || ACC_BYTES <= NST * STAGE_BYTES, "staged accumulators must fit in the operand ring");
     static constexpr uint32_t OFF_RA = PERSISTE ? OFF_ACC + ACC_BYTES : NST * STAGE_BYTES, OFF_RB = OFF_RA + TM * 4, OFF_RBF = OFF_RB + TNv * 4,
                               OFF_RBM = OFF_RBF + TNv * 4;
-    static constexpr uint32_t OFF_BAR = OFF_RBM + 32, OFF_MISC = OFF_BAR + (2 * NST + 2 * NS + NPL + 1) * 8;
-    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + NPL * 4 + 1024;            // + slack to align the base to 1024 bytes
+    static constexpr uint32_t OFF_BAR = OFF_RBM + 32, OFF_MISC = OFF_BAR + (2 * NST + 2 * NS + 1) * 8;
+    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + (PERSISTE && BLK == 32 ? N_PLANOS : 0) + 1024;            // + slack to align the base to 1024 bytes
     static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
     // instruction descriptor kind::f16: D = f32, A = B = f16, both K-major, N = TNv, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
@@ -236,9 +237,18 @@ __device__ __forceinline__ int4 le_vizinho(uint32_t end, int bloco) {
     return v;
 }
 
+template <bool B> struct Logico { static constexpr bool v = B; };
+// a barrier of the first and last warps (not the loading one) that tells each whether any thread said yes
+template <int N>
+__device__ __forceinline__ bool barreira_ou(bool sim) {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, 2, %2, p;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(r) : "r"((uint32_t)sim), "n"(N) : "memory");
+    return r != 0;
+}
+
 // SOMA: tiles in which nothing is rounded add up in tensor memory (128-wide tiles of block 32; the 64-wide ones have no registers for the second
-// drain, and block 128 drains every four MMAs as it is).  A template parameter: with the second drain in the kernel the loop of the rounded
-// tiles comes out 3 to 10 % slower.
+// drain, and block 128 drains every four MMAs as it is).  The loops with and without sums are both in the kernel: with the second drain in
+// them the loops that round come out up to 5 % slower.
 template <int BLK, int MODO, int TNv, bool GRUPO, bool SOMA>
 __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k_gemm_h(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                                                        const int8_t* __restrict__ RA, const int8_t* __restrict__ RB, const uint32_t* __restrict__ nA,
@@ -255,10 +265,10 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     int* RBs = reinterpret_cast<int*>(smem + C_::OFF_RB);
     float* RBf = reinterpret_cast<float*>(smem + C_::OFF_RBF);
     int* RBm = reinterpret_cast<int*>(smem + C_::OFF_RBM);
-    const uint32_t bar_full = sbase + C_::OFF_BAR, bar_empty = bar_full + NST * 8, bar_tfull = bar_empty + NST * 8, bar_tempty = bar_tfull + NS * 8, bar_plano = bar_tempty + NS * 8, bar_encontro = bar_plano + NPL * 8;
+    const uint32_t bar_full = sbase + C_::OFF_BAR, bar_empty = bar_full + NST * 8, bar_tfull = bar_empty + NST * 8, bar_tempty = bar_tfull + NS * 8, bar_encontro = bar_tempty + NS * 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C_::OFF_MISC);
     volatile int* aborta = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 4);
-    volatile int* plano = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 16);
+    unsigned char* planos = smem + C_::OFF_MISC + 16;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int ntiles = Gr.nx * Gr.ny * Gr.partes, npedT = (K + KH - 1) / KH;
     static_assert(!GRUPO || !C_::PERSISTE, "");
@@ -268,7 +278,6 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     if (tid == 0) {
         for (int i = 0; i < NST; i++) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
         for (int i = 0; i < NS; i++) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, N_DW); }
-        for (int i = 0; i < NPL; i++) mbar_init(bar_plano + 8 * i, 1);
         mbar_init(bar_encontro, N_MW);
         *aborta = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -284,70 +293,55 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     pdl_espera();                                  // everything above touches no global memory: it overlaps the predecessor's tail
     pdl_solta();
 
+    // The plans of this block's tiles: how many chunks of K add up in tensor memory before a drain; 0: every K-block is drained and rounded.  Chunks
+    // can add up where none of their products is rounded (shift <= 4) and their sums stay below 2^24 last places of the finest product,
+    // 2^(4 - largest shift), by Cauchy-Schwarz for the whole tile.  A tile that fails anywhere is rounded throughout.  The drain warps make all
+    // of them, a tile each at a time, while the first operands are on their way; a block without a tile that adds up takes the loops
+    // without sums.  (Made by the loading warp tile by tile and waited for by everyone, they cost a tile up to 1000 cycles.  With exponents
+    // that round: no sums at all / plans tile by tile / as it is 75.6 / 79.2 / 74.6 us for 16384 x 1024 x 1024, 213 / 227 / 209 for
+    // 16384 x 4096 x 512 with the sum, 289 / 305 / 293 for 16384 x 4096 x 1024 with ReLU^2.  With exponents that do not: 77 / 55 / 50.5, 214 / 143 / 137, 290 / 187 / 168.)
+    bool somas = false;
+    if (SOMA && wid != N_DW) {
+        const int nb = K / 32, gA = (M + 31) / 32;
+        for (int nt = wid, tile = Pc.tile0 + wid * Pc.passo; wid < N_DW && tile < ntiles; nt += N_DW, tile += N_DW * Pc.passo) {
+            const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx * TM;       // (one K range, of at most 32 K-blocks: a lane each)
+            uint32_t sa = 0, sb = 0;
+            float ma = 0.f, mb = 0.f;
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                const uint32_t a = lane < nb ? nA[(size_t)min(m0 / 32 + g, gA - 1) * nb + lane] : 0u, b = lane < nb ? nB[(size_t)(n0 / 32 + g) * nb + lane] : 0u;
+                sa = max(sa, a & 31u); ma = fmaxf(ma, __uint_as_float(a));
+                sb = max(sb, b & 31u); mb = fmaxf(mb, __uint_as_float(b));
+            }
+            int sh = ma > 0.f && mb > 0.f ? (int)(sa + sb) : 0, junta = 0;
+            float lim = sqrtf(ma) * sqrtf(mb) * 1.0001f;                     // of what the K-block adds to any sum, 2^-4
+#pragma unroll
+            for (int k = 0; k < 5; k++) {                                    // all aligned groups of 2^k chunks, from 2 on (single ones: the drain as it is)
+                sh = max(sh, __shfl_xor_sync(FULL, sh, 1 << k));
+                lim += __shfl_xor_sync(FULL, lim, 1 << k);
+                if (!__all_sync(FULL, sh <= GG && lim * pot2(min(sh, GG)) < LIM_SOMA)) break;
+                if (k) junta = 1 << k;
+            }
+            if (lane == 0) planos[nt] = (unsigned char)junta;
+            somas |= junta != 0;
+        }
+        somas = barreira_ou<(N_DW + N_MW) * 32>(somas);
+    }
+
     // The loading and the multiplying warps run their loops as whole warps, with one elected lane for the asynchronous instructions: the
     // addresses and descriptors then live in uniform registers.  They share their schedulers with busy drain warps, so what counts
     // is how few instructions a chunk takes them (with one lane in a divergent branch the multiplying warp took 680 cycles a chunk and
     // bounded the kernel).
     if (wid == N_DW) {
-        // ------------------------------------------------------------------ loads, and each tile's plan: how many chunks of K add up in
-        // tensor memory before a drain; 0: every K-block is drained and rounded.  Chunks can add up where none of their products is rounded
-        // (shift <= 4) and their sums stay below 2^24 last places of the finest product, 2^(4 - largest shift), by Cauchy-Schwarz for the
-        // whole tile.  A tile that fails anywhere is rounded throughout; that is nearly always known by its first 32 K-blocks.
+        // ------------------------------------------------------------------ loads
         struct {
             const CUtensorMap *mapA, *mapB;
-            const uint32_t *nA, *nB;
-            volatile int *aborta, *plano;
+            volatile int* aborta;
             Grade Gr;
-            uint32_t sbase, bar_full, bar_empty, bar_plano;
-            int lane, kid, nb, gA, npedT;
+            uint32_t sbase, bar_full, bar_empty;
+            int kid;
             bool eleito;
             int n0, m0;                                                      // of the tile that is being loaded
-            uint32_t pv[4 + TNv / 32];                                       // the bounds of 32 K-blocks
-            __device__ __forceinline__ void pede(int tile, int u0 = 0) {
-                const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, f = (ped_ini(Gr, tile) + u0) * 2 + lane;
-#pragma unroll
-                for (int g = 0; g < 4; g++) pv[g] = f < nb ? nA[(size_t)min(m0 / 32 + g, gA - 1) * nb + f] : 0u;
-#pragma unroll
-                for (int g = 0; g < TNv / 32; g++) pv[4 + g] = f < nb ? nB[(size_t)(n0 / 32 + g) * nb + f] : 0u;
-            }
-            // the plan of a tile whose first 32 K-blocks' bounds have been asked for
-            __device__ __forceinline__ int planeja(int tile) {
-                const int nuni = min(Gr.ppp, npedT - ped_ini(Gr, tile));
-                unsigned serve = 0x1Fu;                                      // bit k: all aligned groups of 2^k units so far
-                for (int u0 = 0;;) {
-                    uint32_t sa = 0, sb = 0;
-                    float ma = 0.f, mb = 0.f;
-#pragma unroll
-                    for (int g = 0; g < 4; g++) { sa = max(sa, pv[g] & 31u); ma = fmaxf(ma, __uint_as_float(pv[g])); }
-#pragma unroll
-                    for (int g = 0; g < TNv / 32; g++) { sb = max(sb, pv[4 + g] & 31u); mb = fmaxf(mb, __uint_as_float(pv[4 + g])); }
-                    if (u0 + lane / 2 >= nuni) ma = 0.f;                     // (another K range's)
-                    int sh = ma > 0.f && mb > 0.f ? (int)(sa + sb) : 0;
-                    float lim = sqrtf(ma) * sqrtf(mb) * 1.0001f;             // of what the K-block adds to any sum, 2^-4
-                    sh = max(sh, __shfl_xor_sync(FULL, sh, 1));
-                    lim += __shfl_xor_sync(FULL, lim, 1);
-#pragma unroll
-                    for (int k = 0; k < 5; k++) {
-                        if (!__all_sync(FULL, sh <= GG && lim * pot2(min(sh, GG)) < LIM_SOMA)) {
-                            if (k <= 1) return 0;                            // (single units: the drain as it is)
-                            serve &= (1u << k) - 1;
-                            break;
-                        }
-                        sh = max(sh, __shfl_xor_sync(FULL, sh, 2 << k));
-                        lim += __shfl_xor_sync(FULL, lim, 2 << k);
-                    }
-                    u0 += 16;
-                    if (u0 >= nuni) return 1 << (31 - __clz(serve));
-                    pede(tile, u0);
-                }
-            }
-            __device__ __forceinline__ void publica(int tile, uint32_t nt) {
-                const int n = planeja(tile);
-                if (eleito) {
-                    plano[nt % NPL] = n;
-                    mbar_arrive(bar_plano + 8 * (nt % NPL));
-                }
-            }
             __device__ __forceinline__ bool vazio(int s, uint32_t fase) { return __all_sync(FULL, espera(bar_empty + 8 * s, fase, aborta, kid, 1)); }
             __device__ __forceinline__ void tile(int tile) { n0 = tile % Gr.nx * TNv; m0 = tile / Gr.nx % Gr.ny * TM; }
             __device__ __forceinline__ void carrega(int s, int c) {
@@ -357,22 +351,19 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                     tma_2d(sbase + s * C_::STAGE_BYTES + A_BYTES, mapB, c * KH, n0, bar_full + 8 * s);
                 }
             }
-        } v = {&mapA, &mapB, nA, nB, aborta, plano, Gr, sbase, bar_full, bar_empty, bar_plano, lane, kid, K / 32, (M + 31) / 32, npedT, elege()};
-        if (*reinterpret_cast<volatile int*>(&g_sem_cargas) == 0) laco_cargas<SOMA>(v, Gr, Pc);
+        } v = {&mapA, &mapB, aborta, Gr, sbase, bar_full, bar_empty, kid, elege()};
+        if (*reinterpret_cast<volatile int*>(&g_sem_cargas) == 0) laco_cargas(v, Gr, Pc);
     } else if (wid > N_DW) {
         // ------------------------------------------------------------------ MMAs
         struct {
-            volatile int *aborta, *planos;
-            uint32_t tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_encontro;
+            volatile int* aborta;
+            const unsigned char* planos;
+            uint32_t tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_encontro;
             uint64_t da0, db0;
             int kid;
             bool eleito;
             __device__ __forceinline__ void tile(int) {}
-            __device__ __forceinline__ bool plano(uint32_t nt, int& junta) {
-                const bool ok = __all_sync(FULL, espera(bar_plano + 8 * (nt % NPL), nt / NPL & 1, aborta, kid, 7));
-                if (ok) junta = planos[nt % NPL];
-                return ok;
-            }
+            __device__ __forceinline__ int plano(uint32_t nt) { return planos[nt]; }
             __device__ __forceinline__ bool encontra(uint32_t fase) {
                 __syncwarp();
                 if (eleito) mbar_arrive(bar_encontro);
@@ -409,186 +400,191 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                 if (fim) tc_commit(bar_tfull + 8 * t);
                 tc_commit(bar_empty + 8 * s);
             }
-        } v = {aborta, plano, tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_plano, bar_encontro, desc_sw128(sbase), desc_sw128(sbase + A_BYTES), kid, elege()};
-        laco_produtos<SOMA, NS, CB>(v, Gr, Pc, wid - N_DW - 1);
+        } v = {aborta, planos, tmem, bar_full, bar_empty, bar_tfull, bar_tempty, bar_encontro, desc_sw128(sbase), desc_sw128(sbase + A_BYTES), kid, elege()};
+        if (SOMA && somas) laco_produtos<true, NS, CB>(v, Gr, Pc, wid - N_DW - 1);
+        else laco_produtos<false, NS, CB>(v, Gr, Pc, wid - N_DW - 1);
     } else {
         // ------------------------------------------------------------------ drain + output stage
         const int quarto = wid & 3, cg = wid >> 2, lin = quarto * 32 + lane;
         const uint32_t base = tmem + ((uint32_t)(quarto * 32) << 16) + cg * COLS;
-        int t = 0;
-        uint32_t fase_t = 0, nt = 0;
-        // waits for the next stage (a wait that gives up makes all later ones return at once) / hands it back, its contents in registers
-        auto recebe = [&]() {
-            espera(bar_tfull + 8 * t, fase_t, aborta, kid, 4);
-            __syncwarp();
-            tc_fence_depois();
-        };
-        auto devolve = [&]() {
-            tc_fence_antes();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
-            if (++t == NS) { t = 0; fase_t ^= 1; }
-        };
-        for (int tile = Pc.tile0; tile < ntiles; tile += Pc.passo, nt++) {
-            const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, parte = tile / (Gr.nx * Gr.ny), ped0 = parte * Gr.ppp;
-            const int nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
-            // the row maxima, wanted by the output stage: read now, stored to shared memory after the main loop
-            int ra = 0, rb = 0;
-            if (tid < TM) ra = m0 + tid < M ? (int)RA[m0 + tid] : 0;
-            if (tid < TNv) rb = RB[n0 + tid];
-            constexpr int PITCHv = TNv + 4;
-            // what the output stage needs goes to shared memory
-            auto tabelas = [&]() {
-                if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
-                if (tid < TM) RAs[tid] = ra;
-                if (tid < TNv) {
-                    RBs[tid] = rb;
-                    if (MODO != 1) {
-                        // what the fp32 path of the output stage needs: each block's extreme column exponents and the column scales
-                        int mn = __reduce_min_sync(FULL, rb), mx = __reduce_max_sync(FULL, rb);
-                        if (lane == 0) { RBm[wid] = mn; RBm[4 + wid] = mx; }
-                        if (BLK > 32) {                                          // one block over the four warps: place 0 gets its extremes
-                            asm volatile("bar.sync 3, %0;" ::"n"(TNv) : "memory");
-                            mn = min(min(RBm[0], RBm[1]), min(RBm[2], RBm[3]));
-                            mx = max(max(RBm[4], RBm[5]), max(RBm[6], RBm[7]));
-                            if (tid == 0) { RBm[0] = mn; RBm[4] = mx; }
-                        }
-                        RBf[tid] = pot2(min(rb - mn, 100));
-                    }
-                }
+        auto drena = [&](auto misto) {
+            constexpr bool MISTO = decltype(misto)::v;
+            int t = 0;
+            uint32_t fase_t = 0, nt = 0;
+            // waits for the next stage (a wait that gives up makes all later ones return at once) / hands it back, its contents in registers
+            auto recebe = [&]() {
+                espera(bar_tfull + 8 * t, fase_t, aborta, kid, 4);
+                __syncwarp();
+                tc_fence_depois();
             };
-            int junta = 0;
-            if constexpr (SOMA) junta = __all_sync(FULL, espera(bar_plano + 8 * (nt % NPL), nt / NPL & 1, aborta, kid, 9)) ? plano[nt % NPL] : 0;
-            if (SOMA && junta) {
-                // Sums of whole numbers, straight to shared memory (and added there where a tile has several): with accumulators in registers
-                // this way in and the rounding one out of the loops share them, which costs the rounding loop 5 %.
-                tabelas();
-                for (int u = 0; u < nped / CB; u += junta) {
-                    const uint32_t ta = base + t * (C_::G * TNv);
-                    recebe();
-#pragma unroll
-                    for (int o = 0; o < COLS; o += LV) {
-                        uint32_t a[LV], v[LV], fora = 0;
-                        tmem_pede(ta + o, a);
-                        tmem_pronto(a);
-                        if (o + LV == COLS) devolve();
-                        // (the exponent field of every sum with the constant must be that of 1.5 * 2^23, else the warp converts)
-#pragma unroll
-                        for (int k = 0; k < LV; k += 2) {
-                            v[k] = a[k]; v[k + 1] = a[k + 1];
-                            soma_magia(v[k], v[k + 1]);
-                            fora |= (v[k] ^ MAGIA) | (v[k + 1] ^ MAGIA);
-                            v[k] -= MAGIA; v[k + 1] -= MAGIA;
-                        }
-                        if (__any_sync(FULL, (fora & 0xFF800000u) != 0)) {
-#pragma unroll
-                            for (int k = 0; k < LV; k++) v[k] = (uint32_t)__float2int_rn(__uint_as_float(a[k]));
-                        }
-                        uint4* d = reinterpret_cast<uint4*>(acc_s + lin * PITCHv + cg * COLS + o);
-#pragma unroll
-                        for (int k = 0; k < LV / 4; k++) {
-                            uint4 w = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-                            if (u) { const uint4 z = d[k]; w.x += z.x; w.y += z.y; w.z += z.z; w.w += z.w; }
-                            d[k] = w;
+            auto devolve = [&]() {
+                tc_fence_antes();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
+                if (++t == NS) { t = 0; fase_t ^= 1; }
+            };
+            for (int tile = Pc.tile0; tile < ntiles; tile += Pc.passo, nt++) {
+                const int n0 = tile % Gr.nx * TNv, m0 = tile / Gr.nx % Gr.ny * TM, parte = tile / (Gr.nx * Gr.ny), ped0 = parte * Gr.ppp;
+                const int nped = GRUPO ? max(min(Gr.ppp, npedT - ped0), 0) : min(Gr.ppp, npedT - ped0);
+                // the row maxima, wanted by the output stage: read now, stored to shared memory after the main loop
+                int ra = 0, rb = 0;
+                if (tid < TM) ra = m0 + tid < M ? (int)RA[m0 + tid] : 0;
+                if (tid < TNv) rb = RB[n0 + tid];
+                constexpr int PITCHv = TNv + 4;
+                // what the output stage needs goes to shared memory
+                auto tabelas = [&]() {
+                    if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
+                    if (tid < TM) RAs[tid] = ra;
+                    if (tid < TNv) {
+                        RBs[tid] = rb;
+                        if (MODO != 1) {
+                            // what the fp32 path of the output stage needs: each block's extreme column exponents and the column scales
+                            int mn = __reduce_min_sync(FULL, rb), mx = __reduce_max_sync(FULL, rb);
+                            if (lane == 0) { RBm[wid] = mn; RBm[4 + wid] = mx; }
+                            if (BLK > 32) {                                          // one block over the four warps: place 0 gets its extremes
+                                asm volatile("bar.sync 3, %0;" ::"n"(TNv) : "memory");
+                                mn = min(min(RBm[0], RBm[1]), min(RBm[2], RBm[3]));
+                                mx = max(max(RBm[4], RBm[5]), max(RBm[6], RBm[7]));
+                                if (tid == 0) { RBm[0] = mn; RBm[4] = mx; }
+                            }
+                            RBf[tid] = pot2(min(rb - mn, 100));
                         }
                     }
-                }
-            } else {
-                int acc[COLS];
-#pragma unroll
-                for (int j = 0; j < COLS; j++) acc[j] = 0;
-                if constexpr (BLK == 32) {
-                const int nb = K / 32;
-                unsigned suspeitos = 0;                                      // bit k: K-block (c & ~15) * 2 + k of this range may leave the exact window
-                for (int c = 0; c < nped; c++) {
-                    if ((c & 15) == 0) {
-                        // 32 K-blocks ahead: this warp's largest squared norms of A (32 rows) and B (32 columns)
-                        const int f = (ped0 + c) * 2 + lane;
-                        float pa = 0.f, pb = 0.f;
-                        if (f < nb) {
-                            pa = __uint_as_float(nA[(size_t)min(m0 / 32 + quarto, (M + 31) / 32 - 1) * nb + f]);
-                            pb = __uint_as_float(nB[(size_t)((n0 + cg * COLS) / 32) * nb + f]);
-                        }
-                        suspeitos = __ballot_sync(FULL, pa * pb >= LIM_NORMA);
-                    }
-                    const uint32_t ta = base + t * (2 * TNv);
-                    const bool certo = ((suspeitos >> (2 * (c & 15))) & 3u) == 0;
-                    recebe();
-                    if (certo) {
+                };
+                const int junta = MISTO ? planos[nt] : 0;
+                if (MISTO && junta) {
+                    // Sums of whole numbers, straight to shared memory (and added there where a tile has several): with accumulators in registers
+                    // this way in and the rounding one out of the loops share them, which costs the rounding loop 5 %.
+                    tabelas();
+                    for (int u = 0; u < nped / CB; u += junta) {
+                        const uint32_t ta = base + t * (C_::G * TNv);
+                        recebe();
 #pragma unroll
                         for (int o = 0; o < COLS; o += LV) {
-                            uint32_t a[LV], b[LV];
+                            uint32_t a[LV], v[LV], fora = 0;
                             tmem_pede(ta + o, a);
-                            tmem_pede(ta + TNv + o, b);
                             tmem_pronto(a);
-                            tmem_pronto(b);
                             if (o + LV == COLS) devolve();
-                            junta_lote(a, b, acc, o);
+                            // (the exponent field of every sum with the constant must be that of 1.5 * 2^23, else the warp converts)
+#pragma unroll
+                            for (int k = 0; k < LV; k += 2) {
+                                v[k] = a[k]; v[k + 1] = a[k + 1];
+                                soma_magia(v[k], v[k + 1]);
+                                fora |= (v[k] ^ MAGIA) | (v[k + 1] ^ MAGIA);
+                                v[k] -= MAGIA; v[k + 1] -= MAGIA;
+                            }
+                            if (__any_sync(FULL, (fora & 0xFF800000u) != 0)) {
+#pragma unroll
+                                for (int k = 0; k < LV; k++) v[k] = (uint32_t)__float2int_rn(__uint_as_float(a[k]));
+                            }
+                            uint4* d = reinterpret_cast<uint4*>(acc_s + lin * PITCHv + cg * COLS + o);
+#pragma unroll
+                            for (int k = 0; k < LV / 4; k++) {
+                                uint4 w = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                                if (u) { const uint4 z = d[k]; w.x += z.x; w.y += z.y; w.z += z.z; w.w += z.w; }
+                                d[k] = w;
+                            }
+                        }
+                    }
+                } else {
+                    int acc[COLS];
+#pragma unroll
+                    for (int j = 0; j < COLS; j++) acc[j] = 0;
+                    if constexpr (BLK == 32) {
+                        const int nb = K / 32;
+                        unsigned suspeitos = 0;                                      // bit k: K-block (c & ~15) * 2 + k of this range may leave the exact window
+                        for (int c = 0; c < nped; c++) {
+                            if ((c & 15) == 0) {
+                                // 32 K-blocks ahead: this warp's largest squared norms of A (32 rows) and B (32 columns)
+                                const int f = (ped0 + c) * 2 + lane;
+                                float pa = 0.f, pb = 0.f;
+                                if (f < nb) {
+                                    pa = __uint_as_float(nA[(size_t)min(m0 / 32 + quarto, (M + 31) / 32 - 1) * nb + f]);
+                                    pb = __uint_as_float(nB[(size_t)((n0 + cg * COLS) / 32) * nb + f]);
+                                }
+                                suspeitos = __ballot_sync(FULL, pa * pb >= LIM_NORMA);
+                            }
+                            const uint32_t ta = base + t * (2 * TNv);
+                            const bool certo = ((suspeitos >> (2 * (c & 15))) & 3u) == 0;
+                            recebe();
+                            if (certo) {
+#pragma unroll
+                                for (int o = 0; o < COLS; o += LV) {
+                                    uint32_t a[LV], b[LV];
+                                    tmem_pede(ta + o, a);
+                                    tmem_pede(ta + TNv + o, b);
+                                    tmem_pronto(a);
+                                    tmem_pronto(b);
+                                    if (o + LV == COLS) devolve();
+                                    junta_lote(a, b, acc, o);
+                                }
+                            } else {
+#pragma unroll
+                                for (int o = 0; o < COLS; o += LV) {
+                                    uint32_t a[LV], b[LV];
+                                    tmem_pede(ta + o, a);
+                                    tmem_pede(ta + TNv + o, b);
+                                    tmem_pronto(a);
+                                    tmem_pronto(b);
+                                    converte_lote(a, b, acc, o);
+                                }
+                                devolve();
+                            }
                         }
                     } else {
+                        for (int c = 0; c < nped / 2; c++) {
+                            const uint32_t ta = base + t * TNv;
+                            recebe();
 #pragma unroll
-                        for (int o = 0; o < COLS; o += LV) {
-                            uint32_t a[LV], b[LV];
-                            tmem_pede(ta + o, a);
-                            tmem_pede(ta + TNv + o, b);
-                            tmem_pronto(a);
-                            tmem_pronto(b);
-                            converte_lote(a, b, acc, o);
+                            for (int o = 0; o < COLS; o += LV) {
+                                uint32_t a[LV], x[LV], fora = 0;
+                                tmem_pede(ta + o, a);
+                                tmem_pronto(a);
+                                if (o + LV == COLS) devolve();
+                                // (the exponent field of every sum must be that of 1.5 * 2^23)
+#pragma unroll
+                                for (int k = 0; k < LV; k += 2) {
+                                    x[k] = a[k]; x[k + 1] = a[k + 1];
+                                    soma_magia(x[k], x[k + 1]);
+                                    fora |= (x[k] ^ MAGIA) | (x[k + 1] ^ MAGIA);
+                                }
+                                if (__any_sync(FULL, (fora & 0xFF800000u) != 0)) {
+#pragma unroll
+                                    for (int k = 0; k < LV; k++) x[k] = (uint32_t)__float2int_rn(__uint_as_float(a[k])) + MAGIA;
+                                }
+#pragma unroll
+                                for (int k = 0; k < LV; k++) acc[o + k] += (int)x[k];
+                            }
                         }
-                        devolve();
                     }
-                }
-            } else {
-                for (int c = 0; c < nped / 2; c++) {
-                    const uint32_t ta = base + t * TNv;
-                    recebe();
+                    const uint32_t vies = (uint32_t)(BLK == 32 ? nped * 2 : nped / 2) * MAGIA;
+                    tabelas();
 #pragma unroll
-                    for (int o = 0; o < COLS; o += LV) {
-                        uint32_t a[LV], x[LV], fora = 0;
-                        tmem_pede(ta + o, a);
-                        tmem_pronto(a);
-                        if (o + LV == COLS) devolve();
-                        // (the exponent field of every sum must be that of 1.5 * 2^23)
-#pragma unroll
-                        for (int k = 0; k < LV; k += 2) {
-                            x[k] = a[k]; x[k + 1] = a[k + 1];
-                            soma_magia(x[k], x[k + 1]);
-                            fora |= (x[k] ^ MAGIA) | (x[k + 1] ^ MAGIA);
-                        }
-                        if (__any_sync(FULL, (fora & 0xFF800000u) != 0)) {
-#pragma unroll
-                            for (int k = 0; k < LV; k++) x[k] = (uint32_t)__float2int_rn(__uint_as_float(a[k])) + MAGIA;
-                        }
-#pragma unroll
-                        for (int k = 0; k < LV; k++) acc[o + k] += (int)x[k];
-                    }
-                }
-            }
-                const uint32_t vies = (uint32_t)(BLK == 32 ? nped * 2 : nped / 2) * MAGIA;
-                tabelas();
-#pragma unroll
-                for (int j = 0; j < COLS; j += 4)
-                    *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * COLS + j) =
-                        make_int4((int)((uint32_t)acc[j] - vies), (int)((uint32_t)acc[j + 1] - vies), (int)((uint32_t)acc[j + 2] - vies), (int)((uint32_t)acc[j + 3] - vies));
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
-            if constexpr (!GRUPO) epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s, RAs, RBs, min(TM, M - m0), m0, n0, N, S, Gr.partes > 1, parte == 0, kid, tid, RBf, RBm);
-            else {
-                grupo_barreira();                                            // every block's accumulators are there
-                const int lr = TM / Gr.partes, r0 = parte * lr;              // the rows this block puts out
-                for (int t = tid; t < lr * (TNv / 4); t += N_EPI) {
-                    const int o = (r0 + t / (TNv / 4)) * PITCHv + t % (TNv / 4) * 4;
-                    int4 v = *reinterpret_cast<const int4*>(acc_s + o);
-                    for (int k = 1; k < Gr.partes; k++) {
-                        const int4 x = le_vizinho(smem_u32(acc_s + o), (parte + k) % Gr.partes);
-                        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-                    }
-                    *reinterpret_cast<int4*>(acc_s + o) = v;                 // (only this block reads these rows of its own)
+                    for (int j = 0; j < COLS; j += 4)
+                        *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * COLS + j) =
+                            make_int4((int)((uint32_t)acc[j] - vies), (int)((uint32_t)acc[j + 1] - vies), (int)((uint32_t)acc[j + 2] - vies), (int)((uint32_t)acc[j + 3] - vies));
                 }
                 asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
-                epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s + r0 * PITCHv, RAs + r0, RBs, min(lr, max(M - m0 - r0, 0)), m0 + r0, n0, N, S, false, true, kid, tid, RBf, RBm);
+                if constexpr (!GRUPO) epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s, RAs, RBs, min(TM, M - m0), m0, n0, N, S, Gr.partes > 1, parte == 0, kid, tid, RBf, RBm);
+                else {
+                    grupo_barreira();                                            // every block's accumulators are there
+                    const int lr = TM / Gr.partes, r0 = parte * lr;              // the rows this block puts out
+                    for (int t = tid; t < lr * (TNv / 4); t += N_EPI) {
+                        const int o = (r0 + t / (TNv / 4)) * PITCHv + t % (TNv / 4) * 4;
+                        int4 v = *reinterpret_cast<const int4*>(acc_s + o);
+                        for (int k = 1; k < Gr.partes; k++) {
+                            const int4 x = le_vizinho(smem_u32(acc_s + o), (parte + k) % Gr.partes);
+                            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+                        }
+                        *reinterpret_cast<int4*>(acc_s + o) = v;                 // (only this block reads these rows of its own)
+                    }
+                    asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
+                    epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s + r0 * PITCHv, RAs + r0, RBs, min(lr, max(M - m0 - r0, 0)), m0 + r0, n0, N, S, false, true, kid, tid, RBf, RBm);
+                }
             }
-        }
+        };
+        if (SOMA && somas) drena(Logico<SOMA>{});
+        else drena(Logico<false>{});
     }
     if constexpr (GRUPO) {
         __syncwarp();

@@ -14,9 +14,6 @@ namespace jt {
 namespace th {
 
 constexpr int NST = 4, N_MW = 2;                                            // places of the operand ring, multiplying warps
-// Plans kept.  With one chunk per tile the loading warp has plan n + 1 ready when tile n - 5 has been multiplied; the drain warps have read those up to
-// n - 7 by then, the multiplying warps, which take rounded tiles in turn and meet at those that add up, those up to n - 6.
-constexpr int NPL = 16;
 
 // how the tiles are numbered: columns fastest, then rows, then K ranges
 // With GRUPO the K ranges of a tile are the blocks of a cluster (one tile per block): each leaves its accumulators in shared memory, and each
@@ -30,27 +27,17 @@ JT_LACO int ped_fim(const Grade& G, const Percurso& P, int tile) { const int f =
 
 // ------------------------------------------------------------------------------------------ loads
 // v: vazio(s, phase)  waits until place s of the operand ring has been read (false: given up)
-//    tile(tile)      the tile whose chunks follow;  carrega(s, c)  has its chunk c copied there
-//    pede(tile), publica(tile, nt)  ask for what the tile's plan is made of; make the plan and hand it over as that of the block's nt-th tile
-template <bool SOMA, class V>
+//    tile(tile)          the tile whose chunks follow
+//    carrega(s, c)       has its chunk c copied there
+template <class V>
 JT_LACO void laco_cargas(V& v, const Grade& G, const Percurso& P) {
-    if (SOMA && P.tile0 < P.ntiles) v.pede(P.tile0);
     int s = 0;
-    unsigned fase = 1, nt = 0;
+    unsigned fase = 1;
     bool ok = true;
     for (int tile = P.tile0; tile < P.ntiles && ok; tile += P.passo) {
-        const int c0 = ped_ini(G, tile), cf = ped_fim(G, P, tile);
         v.tile(tile);
-        // A tile's plan is made while the one before is being loaded, the first one's behind its first loads
-        const bool primeira = tile == P.tile0;
-        const int prox = tile + P.passo, cu = cf - 1 > 0 ? cf - 1 : 0;
-        const int x = c0 + (primeira ? NST : 0), cp = x < cu ? x : cu, cq = cp + 2 < cu ? cp + 2 : cu;
-        for (int c = c0; c < cf; c++) {
-            if (SOMA && c == cp) {
-                if (primeira) v.publica(tile, nt++);
-                if (prox < P.ntiles) v.pede(prox);
-            }
-            if (SOMA && c == cq && prox < P.ntiles) v.publica(prox, nt++);
+        const int cf = ped_fim(G, P, tile);
+        for (int c = ped_ini(G, tile); c < cf; c++) {
             ok = v.vazio(s, fase);
             if (!ok) break;
             v.carrega(s, c);
@@ -62,7 +49,8 @@ JT_LACO void laco_cargas(V& v, const Grade& G, const Percurso& P) {
 // ------------------------------------------------------------------------------------------ MMAs
 // A chunk takes a warp ~500 cycles of waits and issue, its MMAs 256: two warps take the stages of a rounded tile in turn (every stage starts a
 // sum of its own).  NS: tensor-memory stages; CB: chunks per stage that is rounded; eu: this warp's number.
-// v: plano(nt, junta)  waits for the plan of the block's nt-th tile
+// SOMA: with tiles that add up.  v: tile(tile)  the tile whose chunks follow
+//    plano(nt)         chunks per sum of the block's nt-th tile, 0: it is rounded
 //    livre(t, phase)   waits until tensor-memory stage t has been drained
 //    cheio(s, phase)   waits until place s of the ring has been loaded
 //    arredonda(s, t, j, certo, c) / soma(s, t, i, fim, certo, c)  if `certo`, issue the MMAs of chunk c onto stage t: chunk j of a stage that is rounded / chunk i of a sum,
@@ -76,11 +64,7 @@ JT_LACO void laco_produtos(V& v, const Grade& G, const Percurso& P, int eu) {
     bool ok = true, soma_antes = false;
     for (int tile = P.tile0; tile < P.ntiles && ok; tile += P.passo, nt++) {
         v.tile(tile);
-        int junta = 0;
-        if (SOMA) {
-            ok = v.plano(nt, junta);
-            if (!ok) break;
-        }
+        const int junta = SOMA ? v.plano(nt) : 0;
         // A phase is known by its parity, so a warp may look at a place of the ring only when it is known that the chunk NST before has been loaded, and
         // at a stage only when its drain before last is known.  Within a rounded tile the waits for the stages see to both, the other warp
         // being one stage away.  A tile that adds up is one warp's, which does not see what the other waits for: around one the warps

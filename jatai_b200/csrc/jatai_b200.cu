@@ -208,12 +208,12 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
         cudaError_t c = cudaMemsetAsync(S.C32, 0, (size_t)M * N * sizeof(int), g_stream);
         if (c != cudaSuccess) return (int)c;
     }
-    // Whether tiles may add up in tensor memory where nothing is rounded.  It depends on the data, which the host does not see: what a step multiplies
-    // by its weights (K = the model's width, at most 1024) nearly always qualifies, products over tokens or over the hidden layer (K from
-    // 1024 up) mostly do not, and a tile that does not pays for having been looked at.  From four tiles per SM the gain is 28 to 36 % (16384 x
-    // 1024..4096 x 1024), the price about 5 %; at one or two tiles it is 8 % against 10 (2048 x 2048 x 512: 19.0 -> 17.5 and 18.8 -> 20.8 us).
-    // (A forced width takes it at any size.)
-    const bool soma = !estreito && K <= 1024 && partes == 1 && (tiles >= 4 * N_SM || g_tn == 128);
+    // Whether tiles may add up in tensor memory where nothing is rounded.  It depends on the data, which the host does not see: each block looks at its
+    // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  From four tiles per SM on the gain where tiles qualify is
+    // 10 to 45 % (16384 x 1024 x 64 28.1 -> 25.1 us, 16384 x 4096 x 1024 290 -> 168; K = 128 with 16 tiles per SM is bound by its output: 151 either way), the price where
+    // none does at most 1.2 % (16384 x 4096 x 1024 with ReLU^2 289 -> 293).  Fewer tiles per SM, larger K and raw outputs keep the kernel
+    // without sums: not measured since the plans are made at a block's start.  (A forced width takes it at any size.)
+    const bool soma = !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (tiles >= 4 * N_SM || g_tn == 128);
 #define JT_H(MD)                                                                                                                            \
     case MD:                                                                                                                                \
         if constexpr (BLK == 32)                                                                                                            \

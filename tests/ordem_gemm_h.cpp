@@ -110,25 +110,23 @@ template <int NS, int CB>
 struct Bloco {
     Sim& S;
     const int n_ped;
-    std::vector<int> planos_certos;
+    std::vector<int> planos;
     Grade G;
     Percurso P;
-    Barra cheio[NST], vazio[NST], tcheio[NS], tlivre[NS], plano_b[NPL], encontro_b;
-    int planos[NPL] = {};
+    Barra cheio[NST], vazio[NST], tcheio[NS], tlivre[NS], encontro_b;
     struct Lugar { int tile = -1, c = -1; bool vem = false; } anel[NST];
     struct Estagio { int tile = -1; std::vector<int> c; int le = 0; bool usado = false; } tmem[NS];
     std::vector<int> postos;                             // chunks put out, tile after tile
     double fim_mma = 0;
 
-    Bloco(Sim& s, int ped, std::vector<int> pl) : S(s), n_ped(ped), planos_certos(std::move(pl)) {
-        const int n = (int)planos_certos.size();
+    Bloco(Sim& s, int ped, std::vector<int> pl) : S(s), n_ped(ped), planos(std::move(pl)) {
+        const int n = (int)planos.size();
         G = {1, n, 1, ped};
         P = {0, 1, n, ped};
         for (auto& b : cheio) b.cria(S, 1);
         for (auto& b : vazio) b.cria(S, 1);
         for (auto& b : tcheio) b.cria(S, 1);
         for (auto& b : tlivre) b.cria(S, N_DW);
-        for (auto& b : plano_b) b.cria(S, 1);
         encontro_b.cria(S, N_MW);
     }
 
@@ -136,12 +134,6 @@ struct Bloco {
         Bloco& B;
         int t = 0;
         void tile(int x) { t = x; }
-        void pede(int) {}
-        void publica(int tile, unsigned nt) {
-            B.S.passa(B.S.demora(0.2));
-            B.planos[nt % NPL] = B.planos_certos[tile];
-            B.plano_b[nt % NPL].chega();
-        }
         bool vazio(int s, unsigned fase) { return B.vazio[s].espera(fase); }
         void carrega(int s, int c) {
             Lugar& l = B.anel[s];
@@ -171,12 +163,7 @@ struct Bloco {
         Bloco& B;
         int t = 0;
         void tile(int x) { t = x; }
-        bool plano(unsigned nt, int& junta) {
-            const bool ok = B.plano_b[nt % NPL].espera(nt / NPL & 1);
-            junta = B.planos[nt % NPL];
-            if (junta != B.planos_certos[t]) throw Falha{"a multiplying warp reads another tile's plan"};
-            return ok;
-        }
+        int plano(unsigned nt) { return B.planos[nt]; }
         bool encontra(unsigned fase) { B.encontro_b.chega(); return B.encontro_b.espera(fase); }
         bool livre(int s, unsigned fase) { return B.tlivre[s].espera(fase); }
         bool cheio(int s, unsigned fase) { return B.cheio[s].espera(fase); }
@@ -186,14 +173,9 @@ struct Bloco {
     template <bool SOMA>
     void drena(bool anota) {
         int t = 0;
-        unsigned fase = 0, nt = 0;
-        for (int tile = 0; tile < P.ntiles; tile++, nt++) {
-            int junta = 0;
-            if (SOMA) {
-                plano_b[nt % NPL].espera(nt / NPL & 1);
-                junta = planos[nt % NPL];
-                if (junta != planos_certos[tile]) throw Falha{"a drain warp reads another tile's plan"};
-            }
+        unsigned fase = 0;
+        for (int tile = 0; tile < P.ntiles; tile++) {
+            const int junta = SOMA ? planos[tile] : 0;
             for (int c = 0; c < n_ped; c += junta ? junta : CB) {
                 tcheio[t].espera(fase);
                 Estagio& e = tmem[t];
@@ -213,7 +195,7 @@ struct Bloco {
     const char* roda() {
         Carrega vc{*this};
         std::vector<Multiplica> vm(N_MW, Multiplica{*this});
-        S.nova([&] { laco_cargas<SOMA>(vc, G, P); });
+        S.nova([&] { laco_cargas(vc, G, P); });
         for (int w = 0; w < N_MW; w++) S.nova([&, w] { laco_produtos<SOMA, NS, CB>(vm[w], G, P, w); });
         for (int w = 0; w < N_DW; w++) S.nova([&, w] { drena<SOMA>(w == 0); });
         S.roda();
