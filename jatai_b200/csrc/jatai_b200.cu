@@ -189,7 +189,6 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     uint32_t *nA = (uint32_t*)(ws + e.nA), *nB = (uint32_t*)(ws + e.nB);
     const int nfx = (K + 511) / 512, ctasA = (M + 31) / 32 * nfx, ctasB = N / 32 * nfx;
     th::ArgsPrepH P = {{A, B}, {EA, EB}, {RA, RB}, {Ah, Bh}, {RAw, RBw}, {nA, nB}, {M, N}, ctasA, K};
-    lanca_pdl(th::k_prep_h<BLK>, dim3(ctasA + ctasB), dim3(256), 0, g_stream, P);
     const Custos c = custos_gemm(BLK, M, N, K);
     const bool estreito = BLK == 32 && g_tn != 128 && (g_tn == 64 || c.h64 < c.h128);
     const int tn = estreito ? 64 : TN;
@@ -204,16 +203,19 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     const int ppp = ((nped + partes - 1) / partes + uni - 1) / uni * uni;
     if (!grupo) partes = (nped + ppp - 1) / ppp;                   // (in a cluster a block without chunks adds zeros)
     const th::Grade G = {N / tn, (M + 127) / 128, partes, ppp};
+    // Whether tiles may add up in tensor memory where nothing is rounded.  It depends on the data, which the host does not see: each block looks at its
+    // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  From four tiles per SM on the gain where tiles qualify is
+    // 10 to 45 % (16384 x 1024 x 64 28.1 -> 25.1 us, 16384 x 4096 x 1024 with ReLU^2 290 -> 168), the price where none does at most 1.2 % (the
+    // latter, 289 -> 293).  Fewer tiles per SM, larger K and raw outputs keep the kernel without sums: not measured since the plans are
+    // made at a block's start.  (A forced width takes it at any size.)
+    const bool soma = BLK == 32 && modo != 1 && !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (tiles >= 4 * N_SM || g_tn == 128);
+    // The bounds with the shift serve every product.  Long rows are prepared faster without it (4096 x 1024 x 16384 raw 271 -> 267 us, the preparation
+    // 55.2 -> 51.5), shorter ones with it (1536 x 512 x 4096 raw 42.8 against 43.0 us, 2048 x 512 x 2048 20.7 against 20.9).
+    lanca_pdl(soma || K < 8192 ? th::k_prep_h<BLK, BLK == 32> : th::k_prep_h<BLK, false>, dim3(ctasA + ctasB), dim3(256), 0, g_stream, P);
     if (partes > 1 && !grupo) {
         cudaError_t c = cudaMemsetAsync(S.C32, 0, (size_t)M * N * sizeof(int), g_stream);
         if (c != cudaSuccess) return (int)c;
     }
-    // Whether tiles may add up in tensor memory where nothing is rounded.  It depends on the data, which the host does not see: each block looks at its
-    // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  From four tiles per SM on the gain where tiles qualify is
-    // 10 to 45 % (16384 x 1024 x 64 28.1 -> 25.1 us, 16384 x 4096 x 1024 290 -> 168; K = 128 with 16 tiles per SM is bound by its output: 151 either way), the price where
-    // none does at most 1.2 % (16384 x 4096 x 1024 with ReLU^2 289 -> 293).  Fewer tiles per SM, larger K and raw outputs keep the kernel
-    // without sums: not measured since the plans are made at a block's start.  (A forced width takes it at any size.)
-    const bool soma = !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (tiles >= 4 * N_SM || g_tn == 128);
 #define JT_H(MD)                                                                                                                            \
     case MD:                                                                                                                                \
         if constexpr (BLK == 32)                                                                                                            \
