@@ -141,6 +141,9 @@ int jt_atencao_via(int via);
 /* Tile width of the tensor-core GEMM: 0 automatic (64 columns when 128-column tiles would leave most SMs idle, block
  * 32 only) | 64 | 128. */
 int jt_gemm_tn(int tn);
+/* Half-precision products whose blocks look for tiles that add up in tensor memory: 0 automatic | 1 none | 2 every one that can (block 32,
+ * 128-column tiles, K <= 1024, a block output).  Same bits either way. */
+int jt_gemm_somas(int quando);
 /* jt_gemm_f with optional externally supplied row-maximum exponents RA[M], RB[N] (int8).  A data-parallel rank
  * passes the maxima over all ranks, so that the int32 partial sums of all ranks share one exponent and their
  * integer sum equals the single-GPU result (the reference's split-K argument, jatai_cuda.cu:214-216). */

@@ -32,6 +32,7 @@ static int g_via = 0;                // GEMM path: 0 automatic | 1 tensor core (
 static int g_alvo_ctas = 148;        // split-K of raw GEMMs aims at this many CTAs
 static int g_at_via = 0;             // attention path: 0 automatic (tensor cores; one CTA per head for short sequences of heads of 4) | 1 the tiled CUDA-core kernels
 static int g_tn = 0;                 // tile width of the tensor-core GEMM: 0 automatic | 64 | 128
+static int g_somas = 0;              // products whose blocks look for tiles that add up in tensor memory: 0 automatic | 1 none | 2 every one that can
 
 static int fim() { return (int)cudaGetLastError(); }
 static unsigned nblocos16(long long n16) { return (unsigned)((n16 + 255) / 256); }
@@ -207,8 +208,8 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  From four tiles per SM on the gain where tiles qualify is
     // 10 to 45 % (16384 x 1024 x 64 28.1 -> 25.1 us, 16384 x 4096 x 1024 with ReLU^2 290 -> 168), the price where none does at most 1.2 % (the
     // latter, 289 -> 293).  Fewer tiles per SM, larger K and raw outputs keep the kernel without sums: not measured since the plans are
-    // made at a block's start.  (A forced width takes it at any size.)
-    const bool soma = BLK == 32 && modo != 1 && !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (tiles >= 4 * N_SM || g_tn == 128);
+    // made at a block's start.
+    const bool soma = BLK == 32 && modo != 1 && !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (g_somas == 2 || (g_somas == 0 && tiles >= 4 * N_SM));
     // The bounds with the shift serve every product.  Long rows are prepared faster without it (4096 x 1024 x 16384 raw 271 -> 267 us, the preparation
     // 55.2 -> 51.5), shorter ones with it (1536 x 512 x 4096 raw 42.8 against 43.0 us, 2048 x 512 x 2048 20.7 against 20.9).
     lanca_pdl(soma || K < 8192 ? th::k_prep_h<BLK, BLK == 32> : th::k_prep_h<BLK, false>, dim3(ctasA + ctasB), dim3(256), 0, g_stream, P);
@@ -323,6 +324,11 @@ int jt_blk_atual() { return g_blk; }
 int jt_gemm_tn(int tn) {
     if (tn != 0 && tn != 64 && tn != 128) return (int)cudaErrorInvalidValue;
     g_tn = tn;
+    return 0;
+}
+int jt_gemm_somas(int quando) {
+    if (quando < 0 || quando > 2) return (int)cudaErrorInvalidValue;
+    g_somas = quando;
     return 0;
 }
 int jt_gemm_via(int via) {

@@ -142,6 +142,11 @@ def test_gemm_formas(amb, blk, M, N, K, cru):
     compara(f"gemm {M}x{N}x{K}", casos.plano(out), casos.plano(spec.Spec(blk).gemm(A, B, cru=cru)))
 
 
+def _somas(blk, tn, K):
+    """The values of jt_gemm_somas that mean different kernels for a half-precision product: one, or without sums and with them."""
+    return (1, 2) if blk == 32 and tn == 128 and K <= 1024 else (0,)
+
+
 @pytest.mark.parametrize("tn", [64, 128])
 @pytest.mark.parametrize("blk,M,N,K", [(32, 64, 128, 32), (32, 128, 128, 96), (32, 192, 256, 2080), (32, 320, 384, 512), (32, 2432, 1408, 160), (32, 128, 128, 8192),
                                        (32, 320, 128, 544), (32, 192, 256, 1056),
@@ -163,12 +168,16 @@ def test_gemm_meia_precisao(amb, blk, M, N, K, tn):
         B[1][7::32] = -8
         s = spec.Spec(blk)
         for op, args, kw in (("gemm", (A, B), {}), ("gemm", (A, B), dict(cru=True)), ("gemm_soma", (A, B, X), {}), ("gemm_relu2", (A, B), {}), ("gemm_relu2_back", (A, B, X), {})):
-            outs = casos.roda(oc, op, args, kw)
-            torch.cuda.synchronize()
-            compara(f"{op} {kw} {M}x{N}x{K} blk {blk} tn {tn}", outs, casos.roda(s, op, args, kw))
+            quer = casos.roda(s, op, args, kw)
+            for somas in _somas(blk, tn, K):
+                assert oc.lib.jt_gemm_somas(somas) == 0
+                outs = casos.roda(oc, op, args, kw)
+                torch.cuda.synchronize()
+                compara(f"{op} {kw} {M}x{N}x{K} blk {blk} tn {tn} somas {somas}", outs, quer)
     finally:
         oc.lib.jt_gemm_via(0)
         oc.lib.jt_gemm_tn(0)
+        oc.lib.jt_gemm_somas(0)
         ops.define_blk(32)
 
 
@@ -337,12 +346,16 @@ def test_gemm_estagio_de_saida(amb, op, caso, tn, blk, via):
             B = (torch.full_like(B[0], 127), torch.full_like(B[1], -8))
         X = G.bloco(M, N, espalha=3)
         args = {"gemm": (A, B), "gemm_soma": (A, B, X), "gemm_relu2": (A, B), "gemm_relu2_back": (A, B, X)}[op]
-        outs = casos.roda(oc, op, tuple(para_gpu(a) for a in args), {})
-        torch.cuda.synchronize()
-        compara(f"{op} {caso} tn {tn} blk {blk} via {via}", outs, casos.roda(spec.Spec(blk), op, args, {}))
+        quer = casos.roda(spec.Spec(blk), op, args, {})
+        for somas in _somas(blk, tn, K) if via == 4 else (0,):
+            assert oc.lib.jt_gemm_somas(somas) == 0
+            outs = casos.roda(oc, op, tuple(para_gpu(a) for a in args), {})
+            torch.cuda.synchronize()
+            compara(f"{op} {caso} tn {tn} blk {blk} via {via} somas {somas}", outs, quer)
     finally:
         oc.lib.jt_gemm_tn(0)
         oc.lib.jt_gemm_via(0)
+        oc.lib.jt_gemm_somas(0)
         ops.define_blk(32)
 
 
@@ -424,7 +437,8 @@ def test_gemm_produtos_parciais_grandes(amb, caso, tn, via):
     """Partial products at and above 2^18 with no alignment shift (s = 0): the inputs on which rounding by an FMA against
     1.5*2^23 would leave its exact range.  The kernels must find them (the 8-bit one, which these sizes take by themselves, by a range check
     on the biased patterns, the half-precision one by the norms of the K-blocks) and round those by conversion - in whole
-    tiles, in single rows and in single K-blocks, for positive and negative products."""
+    tiles, in single rows and in single K-blocks, for positive and negative products.  (Without shifts nothing is rounded, so the half-precision
+    kernel runs without sums in tensor memory, where it converts, and with them, where it adds up 2 to 16 chunks.)"""
     ops, oc, reg = amb
     ops.define_blk(32)
     assert oc.lib.jt_gemm_via(via) == 0 and oc.lib.jt_gemm_tn(tn) == 0
@@ -448,22 +462,28 @@ def test_gemm_produtos_parciais_grandes(amb, caso, tn, via):
                 A[0][i, 32 * b:32 * b + 32] = 127 if i % 2 else -127
             B = (torch.full_like(B[0], 127), B[1])
         for cru in (False, True):
-            outs = casos.plano(oc.gemm(para_gpu(A), para_gpu(B), cru=cru))
-            torch.cuda.synchronize()
-            compara(f"gemm {caso} tn {tn} via {via} cru {cru}", outs, casos.plano(spec.Spec(32).gemm(A, B, cru=cru)))
+            quer = casos.plano(spec.Spec(32).gemm(A, B, cru=cru))
+            for somas in _somas(32, tn, K) if via == 4 and not cru else (0,):
+                assert oc.lib.jt_gemm_somas(somas) == 0
+                outs = casos.plano(oc.gemm(para_gpu(A), para_gpu(B), cru=cru))
+                torch.cuda.synchronize()
+                compara(f"gemm {caso} tn {tn} via {via} cru {cru} somas {somas}", outs, quer)
     finally:
         oc.lib.jt_gemm_tn(0)
         oc.lib.jt_gemm_via(0)
+        oc.lib.jt_gemm_somas(0)
 
 
 @pytest.mark.parametrize("caso", ["um expoente", "dois", "saturado", "saturado a 4", "sem blocos", "um bloco fora"])
+@pytest.mark.parametrize("op", ["gemm", "gemm_soma", "gemm_relu2", "gemm_relu2_back"])
 @pytest.mark.parametrize("M,N,K", [(64, 128, 32), (192, 256, 160), (128, 128, 992), (128, 128, 1024)])
-def test_gemm_somas_em_memoria_de_tensor(amb, caso, M, N, K):
+def test_gemm_somas_em_memoria_de_tensor(amb, caso, M, N, K, op):
     """Tiles whose K-blocks need no rounding (exponents within 4 of their rows' maxima, both sides together) add up in tensor memory: one
-    sum, several where the bound on the sums (2^24 last places) splits them, and none where one K-block of one row lies further down."""
+    sum, several where the bound on the sums (2^24 last places) splits them, and none where one K-block of one row lies further down.  In
+    every output stage that has sums, with rows that fill no tile."""
     ops, oc, reg = amb
     ops.define_blk(32)
-    assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(128) == 0
+    assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(128) == 0 and oc.lib.jt_gemm_somas(2) == 0
     try:
         reg.novo_passo(0)
         G = casos.Gen(77, 32)
@@ -481,18 +501,20 @@ def test_gemm_somas_em_memoria_de_tensor(amb, caso, M, N, K):
         elif caso == "um bloco fora":
             A[1][M // 2, nb - 1] -= 5
             A[0][M // 2] |= 1
-        for cru in (False, True):
-            outs = casos.plano(oc.gemm(para_gpu(A), para_gpu(B), cru=cru))
-            torch.cuda.synchronize()
-            compara(f"gemm {caso} {M}x{N}x{K} cru {cru}", outs, casos.plano(spec.Spec(32).gemm(A, B, cru=cru)))
+        args = (A, B, G.bloco(M, N, espalha=3)) if op in ("gemm_soma", "gemm_relu2_back") else (A, B)
+        outs = casos.roda(oc, op, tuple(para_gpu(a) for a in args), {})
+        torch.cuda.synchronize()
+        compara(f"{op} {caso} {M}x{N}x{K}", outs, casos.roda(spec.Spec(32), op, args, {}))
     finally:
         oc.lib.jt_gemm_tn(0)
         oc.lib.jt_gemm_via(0)
+        oc.lib.jt_gemm_somas(0)
 
 
 @pytest.mark.parametrize("K", [64, 96, 512, 1024])
 def test_gemm_somas_e_arredondamentos_alternados(amb, K):
-    """More tiles than SMs, so that a block works through several: some add up in tensor memory, some round, in every order."""
+    """160 tiles, a few more than SMs: most blocks have one, twelve have two, each of which adds up or rounds.  Raw outputs, which have no sums, beside
+    the block outputs."""
     ops, oc, reg = amb
     ops.define_blk(32)
     g = torch.Generator(device=DEV).manual_seed(K)
@@ -508,12 +530,13 @@ def test_gemm_somas_e_arredondamentos_alternados(amb, K):
         for cru in (False, True):
             assert oc.lib.jt_gemm_via(2) == 0
             quer = oc.gemm(A, B, cru=cru)
-            assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(128) == 0
+            assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(128) == 0 and oc.lib.jt_gemm_somas(2) == 0
             tem = oc.gemm(A, B, cru=cru)
             assert all(torch.equal(x, y) for x, y in zip(quer, tem))
     finally:
         oc.lib.jt_gemm_tn(0)
         oc.lib.jt_gemm_via(0)
+        oc.lib.jt_gemm_somas(0)
 
 
 @pytest.mark.parametrize("op", ["gemm", "gemm_soma", "gemm_relu2", "gemm_relu2_back"])
@@ -541,9 +564,34 @@ def test_gemm_somas_e_arredondamentos_treze_tiles_por_bloco(amb, K, arredonda, o
     try:
         assert oc.lib.jt_gemm_via(2) == 0
         quer = casos.roda(oc, op, args, {})
-        assert oc.lib.jt_gemm_via(4) == 0
+        assert oc.lib.jt_gemm_via(4) == 0 and oc.lib.jt_gemm_tn(128) == 0 and oc.lib.jt_gemm_somas(2) == 0
         for _ in range(3):
             tem = casos.roda(oc, op, args, {})
+            assert len(quer) == len(tem) and all(torch.equal(x, y) for x, y in zip(quer, tem))
+    finally:
+        oc.lib.jt_gemm_tn(0)
+        oc.lib.jt_gemm_via(0)
+        oc.lib.jt_gemm_somas(0)
+
+
+@pytest.mark.parametrize("op", ["gemm", "gemm_relu2"])
+@pytest.mark.parametrize("afasta", [1, 9])
+@pytest.mark.parametrize("M,K", [(37 * 128, 1024), (36 * 128, 1024), (37 * 128, 1056), (37 * 128 - 64, 32), (37 * 128, 64)])
+def test_gemm_somas_regra(amb, M, K, afasta, op):
+    """Both sides of the lines of the automatic choice (592 tiles against 576, K = 1024 against 1056, the smallest K), with exponents that round
+    nothing and with exponents that round everywhere, against the CUDA-core kernel."""
+    ops, oc, reg = amb
+    ops.define_blk(32)
+    g = torch.Generator(device=DEV).manual_seed(M + K + afasta)
+    ints = lambda a, b, forma: torch.randint(a, b + 1, forma, generator=g, device=DEV, dtype=torch.int32).to(torch.int8)
+    A, B = ((ints(-127, 127, (R, K)), ints(-8, -9 + afasta, (R, K // 32))) for R in (M, 2048))
+    reg.novo_passo(0)
+    try:
+        assert oc.lib.jt_gemm_via(2) == 0
+        quer = casos.roda(oc, op, (A, B), {})
+        for via in (0, 4):
+            assert oc.lib.jt_gemm_via(via) == 0
+            tem = casos.roda(oc, op, (A, B), {})
             assert len(quer) == len(tem) and all(torch.equal(x, y) for x, y in zip(quer, tem))
     finally:
         oc.lib.jt_gemm_via(0)
