@@ -140,8 +140,9 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
 }
 // Estimated times of the GEMM kernels in microseconds (measured at 128..16384 rows, 128..4096 columns, K = 128..16384): waves of tiles
 // times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels: against the
-// kernels forced one by one at 44 sizes the choice is within 1 % of the best, but for six sizes where it loses 3 to 7 % (1536 x 512 x 4096 raw 44.3 us against
-// 41.7 with 128-wide tiles, 3072 x 1024 x 16384 raw 256 against 240 with 64-wide ones, block 128 at 4096 x 1024 x 1024 23.1 against 21.6).
+// kernels forced one by one at 49 sizes the choice loses more than 3 % at six (1536 x 512 x 4096 raw 43.1 us against 41.0 and 1024 x 1024 x 16384 raw 107
+// against 100.5 with 128-wide tiles, 3072 x 1024 x 16384 raw 258 against 239 with 64-wide ones, block 128 at 4096 x 1024 x 1024 21.6 against 20.1 and
+// 2048 x 256 x 1024 13.0 against 12.5, and 16384 x 4096 x 128, where the 8-bit path takes 152 us instead of the 59 of the model and the half-precision one 105).
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
 static Custos custos_gemm(int blk, int M, int N, int K) {
     const double n = (K + 63) / 64;
@@ -206,9 +207,9 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     const th::Grade G = {N / tn, (M + 127) / 128, partes, ppp};
     // Whether tiles may add up in tensor memory where nothing is rounded.  It depends on the data, which the host does not see: each block looks at its
     // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  From four tiles per SM on the gain where tiles qualify is
-    // 10 to 45 % (16384 x 1024 x 64 28.1 -> 25.1 us, 16384 x 4096 x 1024 with ReLU^2 290 -> 168), the price where none does at most 1.2 % (the
-    // latter, 289 -> 293).  Fewer tiles per SM, larger K and raw outputs keep the kernel without sums: not measured since the plans are
-    // made at a block's start.
+    // 10 to 45 % (16384 x 1024 x 64 27.9 -> 25.1 us, 16384 x 4096 x 1024 with ReLU^2 290 -> 168), the price where none does at most 1.2 % (the
+    // latter, 289 -> 293).  The line was drawn when a look cost a tile 1000 cycles; now it would pay with fewer tiles too (2048 x 1536 x 512
+    // 17.6 -> 13.7 us where tiles qualify, 17.6 either way where none does).  Larger K and raw outputs are not measured.
     const bool soma = BLK == 32 && modo != 1 && !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (g_somas == 2 || (g_somas == 0 && tiles >= 4 * N_SM));
     // The bounds with the shift serve every product.  Long rows are prepared faster without it (4096 x 1024 x 16384 raw 271 -> 267 us, the preparation
     // 55.2 -> 51.5), shorter ones with it (1536 x 512 x 4096 raw 42.8 against 43.0 us, 2048 x 512 x 2048 20.7 against 20.9).
