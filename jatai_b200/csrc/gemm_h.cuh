@@ -20,8 +20,8 @@
 // Where sa + sb <= 4 nothing is rounded at all: r is a whole number.  A tile in which that holds for every K-block (what a step multiplies by
 // its weights nearly always is: normalised rows and weights have block exponents one or two apart) need not be drained K-block by
 // K-block; its chunks add up in tensor memory, in fp32, exactly while the sum of the bounds stays below 2^24 last places.  Large
-// products with K <= 1024 look for it, with the norms and the largest shift that k_prep_h leaves: 16384 x 4096 x 1024 with ReLU^2 290 -> 168 us,
-// 16384 x 1024 x 1024 77 -> 50.5.  Drained once, a tile waits for nothing but its operands, its MMAs and the output stage of the one before.
+// products with K <= 1024 look for it, with the norms and the largest shift that k_prep_h leaves: 16384 x 4096 x 1024 with ReLU^2 256 -> 167 us,
+// 16384 x 1024 x 1024 69 -> 50.5.  Drained once, a tile waits for nothing but its operands, its MMAs and the output stage of the one before.
 #pragma once
 #include "gemm_tc.cuh"
 #include "gemm_h_ordem.cuh"
@@ -159,31 +159,37 @@ __global__ void __launch_bounds__(256) k_prep_h(const ArgsPrepH P) {
 }
 
 // ------------------------------------------------------------------------------------------ the product
-// A CTA works through 128 x TNv tiles of C (each optionally one K range of it); 4 x NCG drain warps, one warp that loads and one or two
-// that multiply.
-//   TNv 128, 16 drain warps, one CTA per SM, persistent: while the drain warps put a tile out, the next one's operands are already
-//           being loaded and multiplied
-//   TNv 64, 8 drain warps, two CTAs per SM, one tile each (block 32): where 128-wide tiles would leave SMs without work; where even these
-//           do, the K ranges of a tile go to a cluster of 2 to 8 CTAs (512 x 512 x 2048: 17.6 -> 12.2 us)
+// A CTA works through 128 x TNv tiles of C (each optionally one K range of it); 16 drain warps, one warp that loads and two that multiply.  One CTA per
+// SM, persistent: while the drain warps put a tile out, the next one's operands are already being loaded and multiplied.
+//   TNv 128: a drain warp has 32 rows x 32 columns, tensor memory two stages of a chunk
+//   TNv 64, block 32: 32 rows x 16 columns, four stages.  For products of up to 148 such tiles; where these leave SMs without work, the K ranges of
+//           a tile go to a cluster of 2 to 8 CTAs (512 x 512 x 2048 raw: 14.3 -> 11.2 us).  (Two CTAs of 8 drain warps x 32 columns on an SM before:
+//           with two warps to a scheduler a chunk took 600 cycles, its instructions' latencies one after the other, now 310: 2048 x 512 x 2048
+//           with the sum 20.8 -> 17.7 us, 2048 x 512 x 4096 raw 44.9 -> 26.8, in one K range instead of two that add atomically.)
+// What bounds a rounded chunk is the drain warps' instructions: the stage they want is nearly always there (a wait takes 76 cycles when it is, 100 on
+// average).  128 wide, 4096 x 4096 x 4096: 138 instructions a warp and chunk, of which 64 add, 790 cycles -> 110, 650.  What it took: the look at the norms
+// once per 16 chunks instead of a test in each, and their loads 16 chunks ahead (834 -> 783 us for 16384 x 4096 x 4096); the multiplying warps
+// look at the ring before the stage, so that what they wait for last is what comes last (-> 741); warp numbers known to be uniform and the
+// two stages' addresses by one bit (-> 706 -> 684).  Measured and not kept: 8 columns of both K-blocks on their way while 8 are added (1030: twice
+// the loads and waits); 8 drain warps of 64 columns with up to 232 registers, loads of 32 columns, the whole stage in registers at once or in halves
+// (875 to 905: two warps to a scheduler); 16 warps with 112 registers and loads of 32 columns (835); a look at the next stage before the additions (750).
 template <int TNv, int BLK>
 struct CfgH {
-    static constexpr bool PERSISTE = TNv == 128;
-    static constexpr int CTAS = PERSISTE ? 1 : 2, N_DW = PERSISTE ? 16 : 8, N_EPI = N_DW * 32;
-    static constexpr int COLS = TNv / (N_DW / 4);                           // accumulator columns of a drain thread: 32
+    static constexpr int N_DW = 16, N_EPI = N_DW * 32;
+    static constexpr int COLS = TNv / (N_DW / 4);                           // accumulator columns of a drain thread: 32 or 16
     static constexpr int G = BLK == 32 ? 2 : 1;                             // K-blocks handed over together
-    static constexpr int NS = 512 / CTAS / (G * TNv);                       // tensor-memory stages of G x TNv columns
+    static constexpr int NS = 512 / (G * TNv);                       // tensor-memory stages of G x TNv columns
     static constexpr int N_THR = N_EPI + 32 + 32 * N_MW;          // multiplying warps: each takes every N_MW-th stage
-    static_assert(NS >= N_MW && COLS == 32, "");
+    static_assert(NS >= N_MW && (COLS == 32 || COLS == 16), "");
     static constexpr uint32_t B_BYTES = TNv * 128, STAGE_BYTES = A_BYTES + B_BYTES;
-    // the staged accumulators: memory of their own where the loads of the next tile go on meanwhile, else the operand ring (when a
-    // drain thread stores them it has seen the commit of the last MMA)
-    static constexpr uint32_t ACC_BYTES = TM * (TNv + 4) * 4, OFF_ACC = PERSISTE ? NST * STAGE_BYTES : 0;
-    static_assert(PERSISTE || ACC_BYTES <= NST * STAGE_BYTES, "staged accumulators must fit in the operand ring");
-    static constexpr uint32_t OFF_RA = PERSISTE ? OFF_ACC + ACC_BYTES : NST * STAGE_BYTES, OFF_RB = OFF_RA + TM * 4, OFF_RBF = OFF_RB + TNv * 4,
+    // the staged accumulators have memory of their own: the loads of the next tile go on meanwhile
+    static constexpr uint32_t ACC_BYTES = TM * (TNv + 4) * 4, OFF_ACC = NST * STAGE_BYTES;
+    static constexpr uint32_t OFF_RA = OFF_ACC + ACC_BYTES, OFF_RB = OFF_RA + TM * 4, OFF_RBF = OFF_RB + TNv * 4,
                               OFF_RBM = OFF_RBF + TNv * 4;
     static constexpr uint32_t OFF_BAR = OFF_RBM + 32, OFF_MISC = OFF_BAR + (2 * NST + 2 * NS + 1) * 8;
-    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + (PERSISTE && BLK == 32 ? N_PLANOS : 0) + 1024;            // + slack to align the base to 1024 bytes
-    static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
+    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + (TNv == 128 && BLK == 32 ? N_PLANOS : 0) + 1024;            // + slack to align the base to 1024 bytes
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a CTA");
+    static_assert(OFF_BAR % 16 == 0, "the drain warps turn from one stage's barrier to the other's by a bit of the address");
     // instruction descriptor kind::f16: D = f32, A = B = f16, both K-major, N = TNv, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 };
@@ -257,7 +263,7 @@ __device__ __forceinline__ bool barreira_ou(bool sim) {
 // drain, and block 128 drains every four MMAs as it is).  The loops with and without sums are both in the kernel: with the second drain in
 // them the loops that round come out up to 5 % slower.
 template <int BLK, int MODO, int TNv, bool GRUPO, bool SOMA>
-__global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k_gemm_h(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+__global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, 1) k_gemm_h(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                                                        const int8_t* __restrict__ RA, const int8_t* __restrict__ RB, const uint32_t* __restrict__ nA,
                                                        const uint32_t* __restrict__ nB, SaidaGemm S, int M, int N, int K, Grade Gr, int kid) {
     using C_ = CfgH<TNv, BLK>;
@@ -276,9 +282,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C_::OFF_MISC);
     volatile int* aborta = reinterpret_cast<volatile int*>(smem + C_::OFF_MISC + 4);
     unsigned char* planos = smem + C_::OFF_MISC + 16;
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, wid = __shfl_sync(FULL, tid >> 5, 0), lane = tid & 31;
     const int ntiles = Gr.nx * Gr.ny * Gr.partes, npedT = (K + KH - 1) / KH;
-    static_assert(!GRUPO || !C_::PERSISTE, "");
     // the tiles of this block: in a cluster the K ranges lie next to each other
     const Percurso Pc = {GRUPO ? (int)blockIdx.x / Gr.partes + (int)blockIdx.x % Gr.partes * (Gr.nx * Gr.ny) : (int)blockIdx.x, GRUPO ? ntiles : (int)gridDim.x, ntiles, npedT};
 
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (wid == N_DW) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512 / C_::CTAS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_antes();
@@ -378,11 +383,10 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
             }
             __device__ __forceinline__ bool livre(int t, uint32_t fase) { return __all_sync(FULL, espera(bar_tempty + 8 * t, fase, aborta, kid, 3)); }
             __device__ __forceinline__ bool cheio(int s, uint32_t fase) {
-                const bool ok = __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
-                tc_fence_depois();
-                return ok;
+                return __all_sync(FULL, espera(bar_full + 8 * s, fase, aborta, kid, 2));
             }
             __device__ __forceinline__ void arredonda(int s, int t, int j, bool certo, int) {
+                tc_fence_depois();
                 const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
                 const uint32_t d = tmem + t * (C_::G * TNv);
                 if (!(eleito && certo)) return;
@@ -399,6 +403,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                 tc_commit(bar_empty + 8 * s);
             }
             __device__ __forceinline__ void soma(int s, int t, int i, bool fim, bool certo, int) {
+                tc_fence_depois();
                 const uint64_t da = da0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4)), db = db0 + (uint32_t)(s * (C_::STAGE_BYTES >> 4));
                 const uint32_t d = tmem + t * (C_::G * TNv);
                 if (!(eleito && certo)) return;
@@ -416,19 +421,26 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
         const uint32_t base = tmem + ((uint32_t)(quarto * 32) << 16) + cg * COLS;
         auto drena = [&](auto misto) {
             constexpr bool MISTO = decltype(misto)::v;
-            int t = 0;
-            uint32_t fase_t = 0, nt = 0;
+            // the stage at hand: its columns, its barrier, the drains before it
+            uint32_t ta = base, bt = bar_tfull, n_t = 0, nt = 0;
             // waits for the next stage (a wait that gives up makes all later ones return at once) / hands it back, its contents in registers
             auto recebe = [&]() {
-                espera(bar_tfull + 8 * t, fase_t, aborta, kid, 4);
+                espera(bt, n_t / NS & 1, aborta, kid, 4);
                 __syncwarp();
                 tc_fence_depois();
             };
             auto devolve = [&]() {
                 tc_fence_antes();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_tempty + 8 * t);
-                if (++t == NS) { t = 0; fase_t ^= 1; }
+                if (lane == 0) mbar_arrive(bt + (bar_tempty - bar_tfull));
+                n_t++;
+                if constexpr (NS == 2) {
+                    ta ^= C_::G * TNv;
+                    bt ^= 8;
+                } else {
+                    ta = base + n_t % NS * (C_::G * TNv);
+                    bt = bar_tfull + n_t % NS * 8;
+                }
             };
             // The next tile.  With the bounds in registers from above, or a signed step, the loop of raw products comes out 3 % slower (4096 x 1024 x 16384
             // 268 -> 278 us); where there are sums it is the other way round (16384 x 4096 x 512 209 us against 213).
@@ -446,7 +458,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                 constexpr int PITCHv = TNv + 4;
                 // what the output stage needs goes to shared memory
                 auto tabelas = [&]() {
-                    if (C_::PERSISTE && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
+                    if (!GRUPO && tile != (int)blockIdx.x) asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");      // the previous tile is out
                     if (tid < TM) RAs[tid] = ra;
                     if (tid < TNv) {
                         RBs[tid] = rb;
@@ -470,12 +482,12 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
                     // this way in and the rounding one out of the loops share them, which costs the rounding loop 5 %.
                     tabelas();
                     for (int u = 0; u < nped / CB; u += junta) {
-                        const uint32_t ta = base + t * (C_::G * TNv);
                         recebe();
+                        const uint32_t te = ta;
 #pragma unroll
                         for (int o = 0; o < COLS; o += LV) {
                             uint32_t a[LV], v[LV], fora = 0;
-                            tmem_pede(ta + o, a);
+                            tmem_pede(te + o, a);
                             tmem_pronto(a);
                             if (o + LV == COLS) devolve();
                             // (the exponent field of every sum with the constant must be that of 1.5 * 2^23, else the warp converts)
@@ -504,54 +516,64 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
 #pragma unroll
                     for (int j = 0; j < COLS; j++) acc[j] = 0;
                     if constexpr (BLK == 32) {
-                        const int nb = K / 32;
-                        unsigned suspeitos = 0;                                      // bit k: K-block (c & ~15) * 2 + k of this range may leave the exact window
-                        for (int c = 0; c < nped; c++) {
-                            if ((c & 15) == 0) {
-                                // 32 K-blocks ahead: this warp's largest squared norms of A (32 rows) and B (32 columns)
-                                const int f = (ped0 + c) * 2 + lane;
-                                float pa = 0.f, pb = 0.f;
-                                if (f < nb) {
-                                    pa = __uint_as_float(nA[(size_t)min(m0 / 32 + quarto, (M + 31) / 32 - 1) * nb + f]);
-                                    pb = __uint_as_float(nB[(size_t)((n0 + cg * COLS) / 32) * nb + f]);
-                                }
-                                suspeitos = __ballot_sync(FULL, pa * pb >= LIM_NORMA);
-                            }
-                            const uint32_t ta = base + t * (2 * TNv);
-                            const bool certo = ((suspeitos >> (2 * (c & 15))) & 3u) == 0;
-                            recebe();
-                            if (certo) {
+                        // the largest squared norms of this warp's 32 rows of A and of its columns' 32 of B, a lane per K-block, 16 chunks at a time
+                        const int nb = K / 32, fb = min(nb, (ped0 + nped) * 2);
+                        const uint32_t *pA = nA + (size_t)min(m0 / 32 + quarto, (M + 31) / 32 - 1) * nb, *pB = nB + (size_t)((n0 + cg * COLS) / 32) * nb;
+                        float na = 0.f, nbm = 0.f;
+                        auto normas = [&](int c0) {
+                            const int f = (ped0 + c0) * 2 + lane;
+                            na = nbm = 0.f;
+                            if (f < fb) { na = __uint_as_float(pA[f]); nbm = __uint_as_float(pB[f]); }
+                        };
+                        normas(0);
+                        for (int c0 = 0; c0 < nped; c0 += 16) {
+                            unsigned suspeitos = __ballot_sync(FULL, na * nbm >= LIM_NORMA);      // bits 2 c, 2 c + 1: the K-blocks of chunk c may leave the exact window
+                            const int cf = min(nped - c0, 16);
+                            normas(c0 + 16);                                     // (on their way while these chunks are added: waited for here they cost 500 cycles)
+                            if (suspeitos == 0) {
+#pragma unroll 1
+                                for (int c = 0; c < cf; c++) {
+                                    recebe();
+                                    const uint32_t te = ta;
 #pragma unroll
-                                for (int o = 0; o < COLS; o += LV) {
-                                    uint32_t a[LV], b[LV];
-                                    tmem_pede(ta + o, a);
-                                    tmem_pede(ta + TNv + o, b);
-                                    tmem_pronto(a);
-                                    tmem_pronto(b);
-                                    if (o + LV == COLS) devolve();
-                                    junta_lote(a, b, acc, o);
+                                    for (int o = 0; o < COLS; o += LV) {
+                                        uint32_t a[LV], b[LV];
+                                        tmem_pede(te + o, a);
+                                        tmem_pede(te + TNv + o, b);
+                                        tmem_pronto(a);
+                                        tmem_pronto(b);
+                                        if (o + LV == COLS) devolve();
+                                        junta_lote(a, b, acc, o);
+                                    }
                                 }
                             } else {
+#pragma unroll 1
+                                for (int c = 0; c < cf; c++, suspeitos >>= 2) {
+                                    recebe();
+                                    const uint32_t te = ta;
+                                    const bool certo = (suspeitos & 3u) == 0;
 #pragma unroll
-                                for (int o = 0; o < COLS; o += LV) {
-                                    uint32_t a[LV], b[LV];
-                                    tmem_pede(ta + o, a);
-                                    tmem_pede(ta + TNv + o, b);
-                                    tmem_pronto(a);
-                                    tmem_pronto(b);
-                                    converte_lote(a, b, acc, o);
+                                    for (int o = 0; o < COLS; o += LV) {
+                                        uint32_t a[LV], b[LV];
+                                        tmem_pede(te + o, a);
+                                        tmem_pede(te + TNv + o, b);
+                                        tmem_pronto(a);
+                                        tmem_pronto(b);
+                                        if (o + LV == COLS) devolve();
+                                        if (certo) junta_lote(a, b, acc, o);
+                                        else converte_lote(a, b, acc, o);
+                                    }
                                 }
-                                devolve();
                             }
                         }
                     } else {
                         for (int c = 0; c < nped / 2; c++) {
-                            const uint32_t ta = base + t * TNv;
                             recebe();
+                            const uint32_t te = ta;
 #pragma unroll
                             for (int o = 0; o < COLS; o += LV) {
                                 uint32_t a[LV], x[LV], fora = 0;
-                                tmem_pede(ta + o, a);
+                                tmem_pede(te + o, a);
                                 tmem_pronto(a);
                                 if (o + LV == COLS) devolve();
                                 // (the exponent field of every sum must be that of 1.5 * 2^23)
@@ -608,7 +630,7 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, CfgH<TNv, BLK>::CTAS) k
     __syncthreads();
     if (wid == N_DW) {
         tc_fence_depois();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512 / C_::CTAS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
     }
 }
 

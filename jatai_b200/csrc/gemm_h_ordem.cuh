@@ -66,8 +66,9 @@ JT_LACO void laco_produtos(V& v, const Grade& G, const Percurso& P, int eu) {
         v.tile(tile);
         const int junta = SOMA ? v.plano(nt) : 0;
         // A phase is known by its parity, so a warp may look at a place of the ring only when it is known that the chunk NST before has been loaded, and
-        // at a stage only when its drain before last is known.  Within a rounded tile the waits for the stages see to both, the other warp
-        // being one stage away.  A tile that adds up is one warp's, which does not see what the other waits for: around one the warps
+        // at a stage only when its drain before last is known.  Within rounded tiles a warp's own waits see to both: the places and the stages that
+        // it takes are the same ones again and again, so it has itself waited for what was there before (in either order: the place first, because the
+        // chunk is there by then, and the stage, which is not, last).  A tile that adds up is one warp's, which does not see what the other waits for: around one the warps
         // meet, and what the tiles before it waited for has then come for both.
         if (SOMA && (junta || soma_antes)) {
             ok = v.encontra(encontros++ & 1);
@@ -99,11 +100,11 @@ JT_LACO void laco_produtos(V& v, const Grade& G, const Percurso& P, int eu) {
         for (int i = 0; i < nped && ok; i += CB) {
             const bool minha = vez == 0;
             vez = minha ? N_MW - 1 : vez - 1;
-            if (minha) ok = v.livre(t, fase_t);
 JT_DESENROLA
             for (int j = 0; j < CB; j++) {
                 if (minha && ok) {
                     ok = v.cheio(s, fase);
+                    if (j == 0) ok = ok && v.livre(t, fase_t);
                     v.arredonda(s, t, j, ok, c0 + i + j);
                 }
                 if (++s == NST) { s = 0; fase ^= 1; }

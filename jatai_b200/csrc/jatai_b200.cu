@@ -138,36 +138,42 @@ static EspacoH espaco_h(int M, int N, int K) {
 static bool forma_gemm(int blk, int M, int N, int K, int modo) {
     return M > 0 && N > 0 && K > 0 && M % 64 == 0 && N % TN == 0 && K % blk == 0 && K % 32 == 0 && modo >= 0 && modo <= 4;
 }
-// Estimated times of the GEMM kernels in microseconds (measured at 128..16384 rows, 128..4096 columns, K = 128..16384): waves of tiles
+// Estimated times of the GEMM kernels in microseconds (measured at 64..16384 rows, 128..4096 columns, K = 64..16384): waves of tiles
 // times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels: against the
-// kernels forced one by one at 49 sizes the choice loses more than 3 % at six (1536 x 512 x 4096 raw 43.1 us against 41.0 and 1024 x 1024 x 16384 raw 107
-// against 100.5 with 128-wide tiles, 3072 x 1024 x 16384 raw 258 against 239 with 64-wide ones, block 128 at 4096 x 1024 x 1024 21.6 against 20.1 and
-// 2048 x 256 x 1024 13.0 against 12.5, and 16384 x 4096 x 128, where the 8-bit path takes 152 us instead of the 59 of the model and the half-precision one 105).
+// kernels forced one by one at 70 sizes the choice loses more than 3 % at two (128 x 128 x 512 8.4 us against 8.1 with the 8-bit kernel, 2048 x 1536 x 512
+// 15.8 against 15.4 where every tile rounds: it looks for sums; they are worth 16.2 -> 13.2 where none does).
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
-static Custos custos_gemm(int blk, int M, int N, int K) {
+static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
     const double n = (K + 63) / 64;
     const long long t128 = (long long)(N / 128) * ((M + 127) / 128), t64 = 2 * t128;
     auto ondas = [](long long t, int vagas) { return (double)((t + vagas - 1) / vagas); };
     const double prep = 4.0 + (double)(M + N) * K * 3 / 4e6;                            // k_prep_h: a launch, and 3 bytes per element at 4 TB/s
     Custos c;
-    c.h128 = prep + ondas(t128, N_SM) * (n * (blk == 32 ? 0.41 : 0.28) + 1.5);
-    c.h64 = blk == 32 ? prep + (t64 <= N_SM ? n * 0.31 + 2.5 : ondas(t64, 2 * N_SM) * (n * 0.45 + 2.0)) : 1e9;
     c.grupo = 1;
-    // K ranges over a cluster while every block still has an SM for itself and keeps 4 chunks.  (Two to an SM, the blocks of 128 tiles in
-    // two ranges take longer than 128 blocks: 2048 x 512 x 2048 20.8 us against 19.3.)
-    for (int g = 2; blk == 32 && g <= 8 && t64 * g <= N_SM && n >= 4 * g; g *= 2) {
-        const double t = prep + (n / g) * 0.31 + 3.5;
-        if (t < c.h64) { c.h64 = t; c.grupo = g; }
+    // 64-wide tiles read 1.5 times as much for an output element.  With all SMs at it, or operands beyond 48 MB, they wait for the cache
+    // (0.26 to 0.30 us a chunk): 4096 x 4096 x 4096 263 us, 183 with 128-wide ones.  So they have one wave or none.
+    const double p64 = (double)(M + N) * K * 2 > 48e6 ? 0.28 : 0.18;
+    c.h64 = blk == 32 && t64 <= N_SM ? prep + n * p64 + 2.9 : 1e9;
+    if (blk == 32) {
+        int partes = 1;                                                                 // (gemm_h: raw outputs of few 128-wide tiles, clearing and atomic additions 15 us)
+        while (cru && t128 * partes * 2 <= N_SM && n >= partes * 64) partes *= 2;
+        c.h128 = prep + ondas(t128 * partes, N_SM) * (n / partes * 0.31 + 2.4) + (partes > 1 ? 15.0 : 0.0);
+    } else
+        c.h128 = prep + 1.5 + ondas(t128, N_SM) * (n * 0.25 + 1.7);
+    // K ranges over a cluster while every block has an SM for itself (132 blocks in clusters of 4, 120 in clusters of 8 are at work at once) and keeps 4 chunks
+    for (int g = 2; blk == 32 && g <= 8 && t64 * g <= (g == 8 ? 120 : g == 4 ? 132 : N_SM) && n >= 4 * g; g *= 2) {
+        const double x = prep + n / g * p64 + 3.9;
+        if (x < c.h64) { c.h64 = x; c.grupo = g; }
     }
     if (M % tc::TM || K % tc::KC) c.i8 = 1e9;                                           // whole tiles only
-    else if (blk == 32) c.i8 = 2.5 + (t64 <= N_SM ? n * 0.75 : ondas(t64, 2 * N_SM) * n * 1.0);
-    else c.i8 = 2.5 + ondas(t128, N_SM) * (n * (t128 <= N_SM ? 0.58 : 0.43) + 1.0);
+    else if (blk == 32) c.i8 = t64 <= N_SM ? n * 0.68 + 3.0 : 2.5 + ondas(t64, 2 * N_SM) * (n * 0.85 + 3.0);
+    else c.i8 = 2.5 + (t128 <= N_SM ? n * 0.55 + 1.0 : ondas(t128, N_SM) * (n * 0.41 + 3.0));
     return c;
 }
 // whether a caller with a workspace takes the half-precision path
-static bool usa_h(int M, int N, int K) {
+static bool usa_h(int M, int N, int K, int modo) {
     if (g_via != 0) return g_via == 4;
-    const Custos c = custos_gemm(g_blk, M, N, K);
+    const Custos c = custos_gemm(g_blk, M, N, K, modo == 1);
     return (c.h64 < c.h128 ? c.h64 : c.h128) < c.i8;
 }
 template <int BLK, int MODO, int TNv, bool GRUPO, bool SOMA = false>
@@ -179,7 +185,7 @@ static int lanca_h(const CUtensorMap& mA, const CUtensorMap& mB, const int8_t* R
     if (c != cudaSuccess) return (int)c;
     const int tiles = G.nx * G.ny * G.partes;
     if (GRUPO) lanca_cluster(k, dim3(tiles), dim3(C_::N_THR), C_::SMEM_BYTES, g_stream, G.partes, mA, mB, RA, RB, nA, nB, S, M, N, K, G, kid);
-    else lanca_pdl(k, dim3(C_::PERSISTE && tiles > N_SM ? N_SM : tiles), dim3(C_::N_THR), C_::SMEM_BYTES, g_stream, mA, mB, RA, RB, nA, nB, S, M, N, K, G, kid);
+    else lanca_pdl(k, dim3(tiles > N_SM ? N_SM : tiles), dim3(C_::N_THR), C_::SMEM_BYTES, g_stream, mA, mB, RA, RB, nA, nB, S, M, N, K, G, kid);
     return fim();
 }
 template <int BLK>
@@ -191,7 +197,7 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     uint32_t *nA = (uint32_t*)(ws + e.nA), *nB = (uint32_t*)(ws + e.nB);
     const int nfx = (K + 511) / 512, ctasA = (M + 31) / 32 * nfx, ctasB = N / 32 * nfx;
     th::ArgsPrepH P = {{A, B}, {EA, EB}, {RA, RB}, {Ah, Bh}, {RAw, RBw}, {nA, nB}, {M, N}, ctasA, K};
-    const Custos c = custos_gemm(BLK, M, N, K);
+    const Custos c = custos_gemm(BLK, M, N, K, modo == 1);
     const bool estreito = BLK == 32 && g_tn != 128 && (g_tn == 64 || c.h64 < c.h128);
     const int tn = estreito ? 64 : TN;
     CUtensorMap mA, mB;
@@ -201,16 +207,16 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     const bool grupo = estreito && c.grupo > 1;
     int partes = grupo ? c.grupo : 1;
     if (modo == 1 && !grupo)
-        while (tiles * partes * 2 <= (estreito ? 2 : 1) * g_alvo_ctas && nped >= partes * 2 * 32) partes *= 2;
+        while (tiles * partes * 2 <= g_alvo_ctas && nped >= partes * 2 * 32) partes *= 2;
     const int ppp = ((nped + partes - 1) / partes + uni - 1) / uni * uni;
     if (!grupo) partes = (nped + ppp - 1) / ppp;                   // (in a cluster a block without chunks adds zeros)
     const th::Grade G = {N / tn, (M + 127) / 128, partes, ppp};
     // Whether tiles may add up in tensor memory where nothing is rounded.  It depends on the data, which the host does not see: each block looks at its
-    // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  From four tiles per SM on the gain where tiles qualify is
-    // 10 to 45 % (16384 x 1024 x 64 27.9 -> 25.1 us, 16384 x 4096 x 1024 with ReLU^2 290 -> 168), the price where none does at most 1.2 % (the
-    // latter, 289 -> 293).  The line was drawn when a look cost a tile 1000 cycles; now it would pay with fewer tiles too (2048 x 1536 x 512
-    // 17.6 -> 13.7 us where tiles qualify, 17.6 either way where none does).  Larger K and raw outputs are not measured.
-    const bool soma = BLK == 32 && modo != 1 && !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (g_somas == 2 || (g_somas == 0 && tiles >= 4 * N_SM));
+    // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  With more than one tile per SM the gain where tiles qualify is 5 to 35 %
+    // (2048 x 1536 x 512 16.2 -> 13.2 us, 4096 x 1024 x 1024 24.4 -> 19.9, 16384 x 4096 x 1024 with ReLU^2 256 -> 167), the price where none does at most 4 %
+    // (15.4 -> 15.8, 23.2 -> 23.6, 247 -> 256).  With fewer the two are alike (4096 x 512 x 512 11.1 -> 10.5, 10.4 -> 10.9).  Larger K and raw
+    // outputs are not measured.
+    const bool soma = BLK == 32 && modo != 1 && !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (g_somas == 2 || (g_somas == 0 && tiles > N_SM));
     // The bounds with the shift serve every product.  Long rows are prepared faster without it (4096 x 1024 x 16384 raw 271 -> 267 us, the preparation
     // 55.2 -> 51.5), shorter ones with it (1536 x 512 x 4096 raw 42.8 against 43.0 us, 2048 x 512 x 2048 20.7 against 20.9).
     lanca_pdl(soma || K < 8192 ? th::k_prep_h<BLK, BLK == 32> : th::k_prep_h<BLK, false>, dim3(ctasA + ctasB), dim3(256), 0, g_stream, P);
@@ -358,14 +364,14 @@ int jt_gemm(const void* A, const void* EA, const void* B, const void* EB, void* 
 }
 // Workspace of jt_gemm_ws for these sizes, in bytes; 0: the call would not use one (jt_gemm_ext is the same).
 long long jt_gemm_ws_bytes(int M, int N, int K, int modo) {
-    if (!forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K)) return 0;
+    if (!forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K, modo)) return 0;
     return (long long)espaco_h(M, N, K).total;
 }
 // jt_gemm_ext with a workspace of at least jt_gemm_ws_bytes bytes (128-byte aligned, private to this call until its kernels are done)
 int jt_gemm_ws(const void* A, const void* EA, const void* B, const void* EB, void* Cm, void* CE, void* C32, void* Ce, const void* Xm, const void* XE,
                void* Om2, void* OE2, const void* RA, const void* RB, void* ws, int M, int N, int K, int modo, int kid) {
     const bool alinhado = (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
-    if (!ws_serve(ws) || !alinhado || !forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K))
+    if (!ws_serve(ws) || !alinhado || !forma_gemm(g_blk, M, N, K, modo) || !usa_h(M, N, K, modo))
         return jt_gemm_ext(A, EA, B, EB, Cm, CE, C32, Ce, Xm, XE, Om2, OE2, RA, RB, M, N, K, modo, kid);
     SaidaGemm S = {(int8_t*)Cm, (int8_t*)CE, (int*)C32, (int16_t*)Ce, (const int8_t*)Xm, (const int8_t*)XE, (int8_t*)Om2, (int8_t*)OE2};
     if (modo == 1 ? (!C32 || !Ce) : (!Cm || !CE)) return (int)cudaErrorInvalidValue;

@@ -1,6 +1,6 @@
 // The loops of jatai_b200/csrc/gemm_h_ordem.cuh over simulated barriers: loads complete in any order (each one's latency is drawn, some are very
 // late), warps stall anywhere.  Each drawn schedule must multiply what was asked for, put every stage out once and end.
-//   ordem_gemm_h KIND CHUNKS SCHEDULES      KIND: plain (the kernel that only rounds), plain128 (its form for block 128), round, sum, mixed
+//   ordem_gemm_h KIND CHUNKS SCHEDULES      KIND: plain (the kernel that only rounds), plain64 / plain128 (its forms for 64-wide tiles / block 128), round, sum, mixed
 // Exit 0: all schedules are right; 1: the first one that is not is printed.
 #include <ucontext.h>
 
@@ -219,6 +219,7 @@ int main(int argc, char** argv) {
         const int parte = 2 << (S.rng() % 4);             // chunks per sum: 2 to 16
         for (int& x : planos) x = kind == "sum" || (kind == "mixed" && S.unif() < p) ? parte : 0;
         const char* erro = kind == "plain128" ? Bloco<4, 2>(S, ped, planos).roda<false>()
+                           : kind == "plain64" ? Bloco<4, 1>(S, ped, planos).roda<false>()
                            : kind == "plain"  ? Bloco<2, 1>(S, ped, planos).roda<false>()
                                               : Bloco<2, 1>(S, ped, planos).roda<true>();
         if (erro) {

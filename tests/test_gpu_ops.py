@@ -181,6 +181,13 @@ def test_gemm_meia_precisao(amb, blk, M, N, K, tn):
         ops.define_blk(32)
 
 
+@pytest.mark.parametrize("M,N,K", [(2432, 1024, 1056), (2368, 1024, 96), (1088, 1024, 4160), (960, 128, 2048), (1024, 128, 2080)])
+def test_gemm_meia_precisao_64_ondas_e_grupos(amb, M, N, K):
+    """The same with 64-wide tiles: two or three per block, with whole chunks and half ones; more than 32 K-blocks; 15 and 16 tiles, on either side of what
+    goes to clusters of 8."""
+    test_gemm_meia_precisao(amb, 32, M, N, K, 64)
+
+
 def test_gemm_maximos_externos(amb):
     """Row maxima supplied by the caller (the data-parallel path): two K halves with the global maxima add up to
     the full GEMM, bit for bit."""

@@ -15,7 +15,7 @@ def programa(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("tiles", ["plain", "plain128", "round", "sum"])
+@pytest.mark.parametrize("tiles", ["plain", "plain64", "plain128", "round", "sum"])
 @pytest.mark.parametrize("pedacos", [1, 2, 3, 8, 16])
 def test_cada_pedaco_uma_vez(programa, tiles, pedacos):
     """28 tiles of one kind: every chunk is multiplied when it has been loaded and put out once, in its order, and every wait ends."""
