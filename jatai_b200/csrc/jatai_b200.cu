@@ -27,6 +27,7 @@ using namespace jt;
 
 // ---------------------------------------------------------------------------------------------- host state
 static cudaStream_t g_stream = 0;
+static bool g_ao_lado = false;       // the launches to come run beside another chain of launches (jt_stream_ao_lado)
 static int g_blk = 32;               // exponent block length: 32 (native) or 128 (the reference's format)
 static int g_via = 0;                // GEMM path: 0 automatic | 1 tensor core (forced) | 2 CUDA cores | 3 tensor core, rounding by conversion | 4 half-precision tensor pipe (forced)
 static int g_alvo_ctas = 148;        // split-K of raw GEMMs aims at this many CTAs
@@ -142,6 +143,7 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
 // times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels: against the
 // kernels forced one by one at 70 sizes the choice loses more than 3 % at two (128 x 128 x 512 8.4 us against 8.1 with the 8-bit kernel, 2048 x 1536 x 512
 // 15.8 against 15.4 where every tile rounds: it looks for sums; they are worth 16.2 -> 13.2 where none does).
+constexpr int N_LADO = 48;                                           // most blocks of a product beside another chain whose tiles are not the largest
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
 static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
     const double n = (K + 63) / 64;
@@ -152,16 +154,21 @@ static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
     c.grupo = 1;
     // 64-wide tiles read 1.5 times as much for an output element.  With all SMs at it, or operands beyond 48 MB, they wait for the cache
     // (0.26 to 0.30 us a chunk): 4096 x 4096 x 4096 263 us, 183 with 128-wide ones.  So they have one wave or none.
+    // Beside another chain (jt_stream_ao_lado) it is the SMs' time that counts: as many 64-wide tiles as fill the chip, and K ranges over clusters, are
+    // done sooner but hold more SMs (2048 x 512 x 2048 raw 17.3 us on 128 SMs or 22.8 on 64).  A third of the chip is free for them (a short step's
+    // chains are long ones): the 12-layer step takes 3082 to 3172 us without a limit, 3073 with one of 24 or 48 blocks, 3077 with none at all,
+    // 6 layers of 4096 tokens x 256 columns 1261, 1195, 1149, 1166, 5 layers of 4096 x 128 799, 794, 799, 814.
+    const int vagas = g_ao_lado ? N_LADO : N_SM;
     const double p64 = (double)(M + N) * K * 2 > 48e6 ? 0.28 : 0.18;
-    c.h64 = blk == 32 && t64 <= N_SM ? prep + n * p64 + 2.9 : 1e9;
+    c.h64 = blk == 32 && t64 <= vagas ? prep + n * p64 + 2.9 : 1e9;
     if (blk == 32) {
         int partes = 1;                                                                 // (gemm_h: raw outputs of few 128-wide tiles, clearing and atomic additions 15 us)
-        while (cru && t128 * partes * 2 <= N_SM && n >= partes * 64) partes *= 2;
+        while (cru && !g_ao_lado && t128 * partes * 2 <= N_SM && n >= partes * 64) partes *= 2;
         c.h128 = prep + ondas(t128 * partes, N_SM) * (n / partes * 0.31 + 2.4) + (partes > 1 ? 15.0 : 0.0);
     } else
         c.h128 = prep + 1.5 + ondas(t128, N_SM) * (n * 0.25 + 1.7);
     // K ranges over a cluster while every block has an SM for itself (132 blocks in clusters of 4, 120 in clusters of 8 are at work at once) and keeps 4 chunks
-    for (int g = 2; blk == 32 && g <= 8 && t64 * g <= (g == 8 ? 120 : g == 4 ? 132 : N_SM) && n >= 4 * g; g *= 2) {
+    for (int g = 2; blk == 32 && g <= 8 && t64 * g <= vagas && t64 * g <= (g == 8 ? 120 : g == 4 ? 132 : N_SM) && n >= 4 * g; g *= 2) {
         const double x = prep + n / g * p64 + 3.9;
         if (x < c.h64) { c.h64 = x; c.grupo = g; }
     }
@@ -206,7 +213,7 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     const long long tiles = (long long)(N / tn) * ((M + 127) / 128);
     const bool grupo = estreito && c.grupo > 1;
     int partes = grupo ? c.grupo : 1;
-    if (modo == 1 && !grupo)
+    if (modo == 1 && !grupo && !g_ao_lado)
         while (tiles * partes * 2 <= g_alvo_ctas && nped >= partes * 2 * 32) partes *= 2;
     const int ppp = ((nped + partes - 1) / partes + uni - 1) / uni * uni;
     if (!grupo) partes = (nped + ppp - 1) / ppp;                   // (in a cluster a block without chunks adds zeros)
@@ -314,8 +321,15 @@ int jt_erro_limpa() {
 }
 int jt_sincroniza() { return (int)cudaDeviceSynchronize(); }
 void jt_stream(void* st) {
+    g_ao_lado = false;
     g_stream = (cudaStream_t)st;
     espera_limpeza(g_stream);
+}
+// jt_stream for a chain of launches that runs beside another one, until the next jt_stream: products then take no more SMs than their tiles need
+// (custos_gemm).  The results are the same.
+void jt_stream_ao_lado(void* st) {
+    jt_stream(st);
+    g_ao_lado = true;
 }
 void* jt_stream_atual() { return (void*)g_stream; }
 void jt_gemm_split(int alvo) { g_alvo_ctas = alvo > 0 ? alvo : 148; }

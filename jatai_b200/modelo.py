@@ -157,8 +157,9 @@ class Modelo:
         ramo = self._ramo[faixa]
         self._usadas.add(faixa)
         ramo.wait_event(self._ev[0])
+        lib = self.ops.lib
         with torch.cuda.stream(ramo):
-            self.ops.lib.jt_stream(ramo.cuda_stream)
+            (lib.jt_stream_ao_lado if hasattr(lib, "jt_stream_ao_lado") else lib.jt_stream)(ramo.cuda_stream)
             try:
                 yield
             finally:

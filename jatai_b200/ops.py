@@ -61,6 +61,9 @@ def carrega_biblioteca(caminho=None):
     for f in _INT_FUNCS:
         if hasattr(lib, f):
             getattr(lib, f).restype = ctypes.c_int
+    if hasattr(lib, "jt_stream_ao_lado"):
+        lib.jt_stream_ao_lado.argtypes = [ctypes.c_void_p]
+        lib.jt_stream_ao_lado.restype = None
     if hasattr(lib, "jt_gemm_ws_bytes"):
         lib.jt_gemm_ws_bytes.restype = ctypes.c_longlong
         lib.jt_atencao_ws_bytes.restype = ctypes.c_longlong

@@ -497,3 +497,24 @@ def test_registro_de_erros_limpo_antes_de_uma_repeticao(amb):
             reg.confere_device()
     finally:
         oc.lib.jt_stream(None)
+
+
+@pytest.mark.parametrize("M,N,K,cru", [(512, 512, 2048, True), (2048, 512, 2048, True), (128, 128, 4096, True), (1024, 1024, 8192, True), (2048, 512, 1536, False)])
+def test_ao_lado_mesmos_bits(amb, M, N, K, cru):
+    """jt_stream_ao_lado changes how a product is cut (clusters, 64-wide tiles, K ranges), not what it gives; jt_stream takes it back."""
+    ops, oc, reg = amb
+    ops.define_blk(32)
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    ints = lambda a, b, forma: torch.randint(a, b + 1, forma, generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    A, B = ((ints(-127, 127, (R, K)), ints(-12, -4, (R, K // 32))) for R in (M, N))
+    reg.novo_passo(0)
+    try:
+        quer = oc.gemm(A, B, cru=cru)
+        oc.lib.jt_stream_ao_lado(None)
+        tem = oc.gemm(A, B, cru=cru)
+        oc.lib.jt_stream(None)
+        outra = oc.gemm(A, B, cru=cru)
+    finally:
+        oc.lib.jt_stream(None)
+    for x, y, z in zip(quer, tem, outra):
+        assert torch.equal(x, y) and torch.equal(x, z)
