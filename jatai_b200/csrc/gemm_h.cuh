@@ -193,12 +193,6 @@ struct CfgH {
     // instruction descriptor kind::f16: D = f32, A = B = f16, both K-major, N = TNv, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 };
-// one lane of a converged warp
-__device__ __forceinline__ bool elege() {
-    uint32_t p;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acumula) {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"

@@ -10,7 +10,9 @@
 // instruction starts a fresh accumulator (tensor-memory stage) that is drained, aligned and added in registers;
 // with BLK = 128 four instructions accumulate in tensor memory before one drain.
 //
-// CTA = one 128 x TNv tile of C (optionally one K range of it: split-K for raw outputs), 2 + TNv / 8 warps (TNv = 128 below):
+// CTA = one 128 x TNv tile of C (optionally one K range of it: split-K for raw outputs), 2 + 16 warps (TNv = 128 below).  64-wide tiles: two CTAs of 2 + 8 warps
+// per SM where there are more of them than SMs, else one of 2 + 16 warps of 16 columns each with eight tensor-memory stages: four
+// warps to a scheduler instead of two (2048 x 512 x 512 8.4 -> 7.7 us, 2048 x 512 x 2048 23.9 -> 21.4; the multiplying warp goes through its loop converged):
 //   warp 0       TMA producer (one lane): A and B tiles of 128 rows x 128 bytes of K, SWIZZLE_128B, NST-stage ring;
 //                all 32 lanes also build, ahead of the drain, the table of column scales 2^-(RB_j - eb_jb) it reads
 //   warp 1       allocates tensor memory, issues the MMAs (one thread), frees tensor memory
@@ -25,13 +27,16 @@
 namespace jt {
 namespace tc {
 
-constexpr int TM = 128, KC = 128, NST = 4, NTM = 4, NTB = 4;
+constexpr int TM = 128, KC = 128, NST = 4, NTB = 4;
 constexpr uint32_t A_BYTES = TM * KC;
 // everything that depends on the tile width TNv (columns of C per CTA): 128, or 64 for shapes whose 128-wide tiling
 // would leave most SMs without a CTA (block 32 only: a 128-column exponent block does not fit a 64-column tile)
-template <int TNv, int VIA>
+template <int TNv, int VIA, bool SO>
 struct Cfg {
-    static constexpr int N_DW = TNv / 8;                       // drain warps: 4 lane quarters x (TNv / 32) column groups
+    // drain warps: 4 lane quarters x column groups of 32, or (SO: a 64-wide tile alone on its SM) of 16
+    static constexpr int N_DW = SO ? 16 : TNv / 8, COLS = TNv * 4 / N_DW;
+    static constexpr int NTM = SO ? 8 : 4;                     // tensor-memory stages
+    static_assert(!SO || (TNv == 64 && VIA == 1), "");
     static constexpr int N_EPI = N_DW * 32, N_THR = 64 + N_EPI, PITCHv = TNv + 4;
     static constexpr uint32_t B_BYTES = TNv * KC, STAGE_BYTES = A_BYTES + B_BYTES;
     // the staged accumulators of the output stage reuse the operand ring: when a drain thread stores its accumulators
@@ -49,7 +54,7 @@ struct Cfg {
     static constexpr uint32_t SMEM_BYTES = OFF_C127 + 1024 + 1024;          // + slack to align the base to 1024 bytes
     // 64-column tiles: two CTAs per SM (2 x 256 columns of tensor memory, 2 x ~100 KB of shared memory, <= 102 registers):
     // the prologue and the output stage of one overlap the main loop of the other
-    static constexpr int CTAS_SM = TNv == 64 ? 2 : 1;
+    static constexpr int CTAS_SM = TNv == 64 && !SO ? 2 : 1;
     // instruction descriptor kind::i8: D = s32, A = B = s8, both K-major, N = TNv, M = 128
     static constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TNv >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 };
@@ -119,6 +124,12 @@ __device__ __forceinline__ void tc_fence_depois() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// one lane of a converged warp
+__device__ __forceinline__ bool elege() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acumula) {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
                  " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
@@ -167,13 +178,14 @@ __device__ __forceinline__ void tmem_le8x2(uint32_t ta, uint32_t tb, uint32_t (&
 //        those of 1.5*2^23 reads the half chunk again (the stages are handed back only after this vote), takes the fast results
 //        off and adds VIA 2's conversions instead.
 // VIA 2: exact float product, cvt.rni to int (valid for every input; block 128, where four MMAs accumulate before a drain).
-template <int BLK, int MODO, int VIA, int TNv>
-__global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) k_gemm_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+template <int BLK, int MODO, int VIA, int TNv, bool SO>
+__global__ void __launch_bounds__(Cfg<TNv, VIA, SO>::N_THR, Cfg<TNv, VIA, SO>::CTAS_SM) k_gemm_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                                                       const int8_t* __restrict__ EA, const int8_t* __restrict__ EB,
                                                       const int8_t* __restrict__ RAg, const int8_t* __restrict__ RBg, SaidaGemm S, int M, int N,
                                                       int K, int pedacos_por_parte, int kid) {
     constexpr int NQ = KC / BLK;                 // K-blocks per 128-byte chunk: 4 (BLK 32) or 1 (BLK 128)
-    using C_ = Cfg<TNv, VIA>;
+    using C_ = Cfg<TNv, VIA, SO>;
+    constexpr int NTM = C_::NTM, COLS = C_::COLS;
     constexpr int N_DW = C_::N_DW, N_EPI = C_::N_EPI, PITCHv = C_::PITCHv;
     constexpr bool PARES = BLK == 32 && VIA == 1;
     static_assert(VIA != 1 || BLK == 32, "the FMA rounding is written for one MMA per drain");
@@ -195,7 +207,7 @@ __global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC);
     volatile int* aborta = reinterpret_cast<volatile int*>(smem + OFF_MISC + 4);
 
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, wid = __shfl_sync(FULL, tid >> 5, 0), lane = tid & 31;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TNv;
     const int nb = K / BLK;
     const int ped0 = blockIdx.z * pedacos_por_parte;             // first 128-byte chunk of this CTA's K range
@@ -278,57 +290,48 @@ __global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) 
             if (i + 1 < pedacos_por_parte) le_w(i + 1);
         }
     } else if (wid == 1) {
-        // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            int f = 0;
-            bool ok = true;
-            const uint64_t d127 = desc_sw128(sbase + C_::OFF_C127) & ~((uint64_t)0x3FFF << 32);
-            for (int i = 0; i < pedacos_por_parte && ok; i++) {
-                const int s = i % NST;
-                if (!espera(bar_full + 8 * s, (i / NST) & 1, aborta, kid, 2)) break;
-                tc_fence_depois();
-                const uint64_t da = desc_sw128(sbase + s * STAGE_BYTES), db = desc_sw128(sbase + s * STAGE_BYTES + A_BYTES);
-                if (BLK == 32 && VIA == 1) {
-                    // two slices per hand-over (the drain takes them together): barriers of the even stages only.  The constant
-                    // product 32 * 127 * 127 goes in first (every 8-row group of both operands is the same 1 KB of the byte 127:
-                    // group stride 0), the slices' products on top of it.
+        // ------------------------------------------------------------------ MMA issuer: the whole warp goes through the loop, one elected lane issues (the
+        // addresses and descriptors then live in uniform registers)
+        const bool eleito = elege();
+        int f = 0;
+        bool ok = true;
+        const uint64_t d127 = desc_sw128(sbase + C_::OFF_C127) & ~((uint64_t)0x3FFF << 32);
+        for (int i = 0; i < pedacos_por_parte && ok; i++) {
+            const int s = i % NST;
+            ok = __all_sync(FULL, espera(bar_full + 8 * s, (i / NST) & 1, aborta, kid, 2));
+            if (!ok) break;
+            const uint64_t da = desc_sw128(sbase + s * STAGE_BYTES), db = desc_sw128(sbase + s * STAGE_BYTES + A_BYTES);
+            // PARES: two slices per hand-over (the drain takes them together), barriers of the even stages only
+            constexpr int FQ = PARES ? 2 : BLK == 32 ? 1 : 4;       // MMAs of K = 32 per hand-over
 #pragma unroll
-                    for (int q = 0; q < 4; q += 2, f += 2) {
-                        const int t = f % NTM;
-                        if (!espera(bar_tempty + 8 * t, ((f / NTM) & 1) ^ 1, aborta, kid, 3)) { ok = false; break; }
-                        tc_fence_depois();
+            for (int q = 0; q < 4; q += FQ) {
+                const int t = f % NTM;
+                ok = __all_sync(FULL, espera(bar_tempty + 8 * t, ((f / NTM) & 1) ^ 1, aborta, kid, 3));
+                if (!ok) break;
+                tc_fence_depois();
+                if (eleito) {
+                    if (PARES) {
+                        // the constant product 32 * 127 * 127 goes in first (every 8-row group of both operands is the same 1 KB of the byte 127:
+                        // group stride 0), the slices' products on top of it
                         tc_mma_i8(tmem + t * TNv, d127, d127, IDESC, 0);
                         tc_mma_i8(tmem + (t + 1) * TNv, d127, d127, IDESC, 0);
                         tc_mma_i8(tmem + t * TNv, da + 2 * q, db + 2 * q, IDESC, 1);               // +32 bytes of K per instruction
                         tc_mma_i8(tmem + (t + 1) * TNv, da + 2 * q + 2, db + 2 * q + 2, IDESC, 1);
-                        tc_commit(bar_tfull + 8 * t);
-                    }
-                } else if (BLK == 32) {
+                    } else {
 #pragma unroll
-                    for (int q = 0; q < 4; q++, f++) {
-                        const int t = f % NTM;
-                        if (!espera(bar_tempty + 8 * t, ((f / NTM) & 1) ^ 1, aborta, kid, 3)) { ok = false; break; }
-                        tc_fence_depois();
-                        tc_mma_i8(tmem + t * TNv, da + 2 * q, db + 2 * q, IDESC, 0);               // +32 bytes of K per instruction
-                        tc_commit(bar_tfull + 8 * t);
+                        for (int r = 0; r < FQ; r++) tc_mma_i8(tmem + t * TNv, da + 2 * (q + r), db + 2 * (q + r), IDESC, r > 0);
                     }
-                } else {
-                    const int t = f % NTM;
-                    if (!espera(bar_tempty + 8 * t, ((f / NTM) & 1) ^ 1, aborta, kid, 3)) break;
-                    tc_fence_depois();
-#pragma unroll
-                    for (int q = 0; q < 4; q++) tc_mma_i8(tmem + t * TNv, da + 2 * q, db + 2 * q, IDESC, q > 0);
                     tc_commit(bar_tfull + 8 * t);
-                    f++;
+                    if (q + FQ == 4) tc_commit(bar_empty + 8 * s);
                 }
-                tc_commit(bar_empty + 8 * s);
+                f += PARES ? 2 : 1;
             }
         }
     } else {
         // ------------------------------------------------------------------ drain + output stage
         const int et = tid - 64;                                  // 0..511
         const int quarto = wid & 3;                               // tensor-memory lanes this warp may read
-        const int cg = (wid - 2) >> 2;                            // column group of 32 within the tile
+        const int cg = (wid - 2) >> 2;                            // column group within the tile
         const int lin = quarto * 32 + lane;                       // row of the tile = tensor-memory lane
         const int8_t* ea_lin = EA + (size_t)(m0 + lin) * nb + (size_t)ped0 * NQ;
         auto le_exp = [&](int c) -> uint32_t {
@@ -372,13 +375,13 @@ __global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) 
             } else if (lane == 0) { RBm[b] = mn; RBm[4 + b] = mx; }
             RBf[et] = pot2(min(rb - mn, 100));
         }
-        int acc[32];
+        int acc[COLS];
 #pragma unroll
-        for (int j = 0; j < 32; j++) acc[j] = 0;
+        for (int j = 0; j < COLS; j++) acc[j] = 0;
         int f = 0;
         bool ok = true;
         if constexpr (PARES) {
-            static_assert(NQ == NTM, "one tensor-memory stage per K-block of a chunk");
+            static_assert(NTM % NQ == 0, "whole chunks of one tensor-memory stage per K-block");
             const uint64_t magia2 = par_f(MAGIA_F, MAGIA_F);
             for (int c = 0; c < pedacos_por_parte && ok; c++) {
                 const int sl = c % NTB;
@@ -387,19 +390,19 @@ __global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) 
                 if (!ok) break;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const int t0 = 2 * h, t1 = 2 * h + 1;
-                    ok = __all_sync(FULL, espera(bar_tfull + 8 * t0, c & 1, aborta, kid, 4));      // one hand-over for both stages
+                    const int t0 = c % (NTM / NQ) * NQ + 2 * h, t1 = t0 + 1;
+                    ok = __all_sync(FULL, espera(bar_tfull + 8 * t0, c / (NTM / NQ) & 1, aborta, kid, 4));      // one hand-over for both stages
                     if (!ok) break;
                     tc_fence_depois();
                     const int sa0 = min(RA - (int)(int8_t)(eaw >> (16 * h)), 40), sa1 = min(RA - (int)(int8_t)(eaw >> (16 * h + 8)), 40);
-                    const uint32_t base_h = tmem + ((uint32_t)(quarto * 32) << 16) + cg * 32;
-                    const float* tb_h = tabB + (sl * 4 + t0) * TNv + cg * 32;
+                    const uint32_t base_h = tmem + ((uint32_t)(quarto * 32) << 16) + cg * COLS;
+                    const float* tb_h = tabB + (sl * 4 + 2 * h) * TNv + cg * COLS;
                     const float fa0 = pot2(123 - sa0), fa1 = pot2(123 - sa1);
                     const float cn0 = -(float)DESLOC * pot2(GG - 30 - sa0), cn1 = -(float)DESLOC * pot2(GG - 30 - sa1);
                     const uint64_t fa0p = par_f(fa0, fa0), fa1p = par_f(fa1, fa1), cn0p = par_f(cn0, cn0), cn1p = par_f(cn1, cn1);
                     uint32_t ou = 0;
 #pragma unroll
-                    for (int hf = 0; hf < 4; hf++) {                   // 8 columns of two slices at a time
+                    for (int hf = 0; hf < COLS / 8; hf++) {                   // 8 columns of two slices at a time
                         uint32_t d0[8], d1[8];                         // p' = p + 32*127^2: as floats, the subnormals p' * 2^-149
                         tmem_le8x2(base_h + hf * 8 + t0 * TNv, base_h + hf * 8 + t1 * TNv, d0, d1);
                         const float* tb0 = tb_h + hf * 8;
@@ -427,7 +430,7 @@ __global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) 
                         // some result left the window of the rounding constant: take the fast results off again, add the conversions
                         const float ga0 = pot2(GG - 30 - sa0), ga1 = pot2(GG - 30 - sa1);
 #pragma unroll 1
-                        for (int hf = 0; hf < 4; hf++) {
+                        for (int hf = 0; hf < COLS / 8; hf++) {
                             uint32_t d0[8], d1[8];
                             tmem_le8x2(base_h + hf * 8 + t0 * TNv, base_h + hf * 8 + t1 * TNv, d0, d1);
                             const float* tb0 = tb_h + hf * 8;
@@ -441,7 +444,7 @@ __global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) 
                                 const int dif = (int)((uint32_t)ex0 + MAGIA - rap0) + (int)((uint32_t)ex1 + MAGIA - rap1);
                                 // the accumulator is a compile-time register only under full unrolling: select by hf
 #pragma unroll
-                                for (int g = 0; g < 4; g++) acc[g * 8 + k] += g == hf ? dif : 0;
+                                for (int g = 0; g < COLS / 8; g++) acc[g * 8 + k] += g == hf ? dif : 0;
                             }
                         }
                     }
@@ -496,11 +499,11 @@ __global__ void __launch_bounds__(Cfg<TNv, VIA>::N_THR, Cfg<TNv, VIA>::CTAS_SM) 
         if (PARES) {
             const uint32_t vies = (uint32_t)nfatias * MAGIA;
 #pragma unroll
-            for (int j = 0; j < 32; j++) acc[j] = (int)((uint32_t)acc[j] - vies);
+            for (int j = 0; j < COLS; j++) acc[j] = (int)((uint32_t)acc[j] - vies);
         }
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * 32 + j) = make_int4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+        for (int j = 0; j < COLS; j += 4)
+            *reinterpret_cast<int4*>(acc_s + lin * PITCHv + cg * COLS + j) = make_int4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
         // the only barrier of the drain warps: reached by every drain thread exactly once, aborted or not
         asm volatile("bar.sync 1, %0;" ::"n"(N_EPI) : "memory");
         epilogo_tile<BLK, MODO, N_EPI, TNv>(acc_s, RAs, RBs, TM, m0, n0, N, S, gridDim.z > 1, blockIdx.z == 0, kid, et, RBf, RBm);

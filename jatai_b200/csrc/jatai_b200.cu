@@ -40,12 +40,12 @@ static unsigned nblocos16(long long n16) { return (unsigned)((n16 + 255) / 256);
 static unsigned nblocos_128(long long n16) { return (unsigned)((n16 + 127) / 128); }
 static unsigned nblocos16u(long long n16, int U) { return (unsigned)((n16 + 256LL * U - 1) / (256LL * U)); }      // U chunks per thread
 
-template <int BLK, int MODO, int VIA, int TNv>
+template <int BLK, int MODO, int VIA, int TNv, bool SO = false>
 static int lanca_tc(const CUtensorMap& mA, const CUtensorMap& mB, const int8_t* EA, const int8_t* EB, const int8_t* RA, const int8_t* RB,
                     const SaidaGemm& S, int M, int N, int K, int partes, int kid) {
     static bool feito[64];                 // kernel attributes are per device
-    using C_ = tc::Cfg<TNv, VIA>;
-    auto k = tc::k_gemm_tc<BLK, MODO, VIA, TNv>;
+    using C_ = tc::Cfg<TNv, VIA, SO>;
+    auto k = tc::k_gemm_tc<BLK, MODO, VIA, TNv, SO>;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
     bool& pronto = feito[dev];
@@ -96,6 +96,7 @@ static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const in
     int partes = 1;
     if (modo == 1)
         while (partes * (usa_tc ? 16 : 2) <= unidades && tiles * partes * 2 <= g_alvo_ctas && unidades % (partes * 2) == 0) partes *= 2;
+    const bool so = estreito && tiles * partes <= N_SM;
     if (partes > 1) {
         cudaError_t c = cudaMemsetAsync(S.C32, 0, (size_t)M * N * sizeof(int), g_stream);
         if (c != cudaSuccess) return (int)c;
@@ -107,6 +108,7 @@ static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const in
         if constexpr (BLK == 32) {                                                                                   \
             if (estreito) {                                                                                          \
                 if (g_via == 3) return lanca_tc<32, MD, 2, 64>(mA, mB, EA, EB, RA, RB, S, M, N, K, partes, kid);     \
+                if (so) return lanca_tc<32, MD, 1, 64, true>(mA, mB, EA, EB, RA, RB, S, M, N, K, partes, kid);       \
                 return lanca_tc<32, MD, 1, 64>(mA, mB, EA, EB, RA, RB, S, M, N, K, partes, kid);                     \
             }                                                                                                        \
             if (g_via == 3) return lanca_tc<32, MD, 2, 128>(mA, mB, EA, EB, RA, RB, S, M, N, K, partes, kid);        \
@@ -141,8 +143,9 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
 }
 // Estimated times of the GEMM kernels in microseconds (measured at 64..16384 rows, 128..4096 columns, K = 64..16384): waves of tiles
 // times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels: against the
-// kernels forced one by one at 70 sizes the choice loses more than 3 % at two (128 x 128 x 512 8.4 us against 8.1 with the 8-bit kernel, 2048 x 1536 x 512
-// 15.8 against 15.4 where every tile rounds: it looks for sums; they are worth 16.2 -> 13.2 where none does).
+// kernels forced one by one at 70 sizes the choice loses more than 3 % at three where every tile rounds, because it looks for sums (2048 x 1536 x 512 15.8 us
+// against 15.4, 2048 x 2048 x 512 with ReLU^2 18.3 against 17.7, 16384 x 4096 x 1024 256 against 248; where none rounds they are worth 16.2 -> 13.2, 18.0 -> 15.1,
+// 256 -> 167), at 8192 x 512 x 128 (14.6 against 13.7 with the 8-bit kernel) and, block 128, at 1024 x 512 x 4096 raw (34.8 against 25.2).
 constexpr int N_LADO = 48;                                           // most blocks of a product beside another chain whose tiles are not the largest
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
 static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
@@ -173,7 +176,7 @@ static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
         if (x < c.h64) { c.h64 = x; c.grupo = g; }
     }
     if (M % tc::TM || K % tc::KC) c.i8 = 1e9;                                           // whole tiles only
-    else if (blk == 32) c.i8 = t64 <= N_SM ? n * 0.68 + 3.0 : 2.5 + ondas(t64, 2 * N_SM) * (n * 0.85 + 3.0);
+    else if (blk == 32) c.i8 = t64 <= N_SM ? n * 0.55 + 3.4 : 2.5 + ondas(t64, 2 * N_SM) * (n * 0.80 + 3.2);
     else c.i8 = 2.5 + (t128 <= N_SM ? n * 0.55 + 1.0 : ondas(t128, N_SM) * (n * 0.41 + 3.0));
     return c;
 }
