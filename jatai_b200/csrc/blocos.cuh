@@ -473,6 +473,9 @@ __device__ __forceinline__ void max4_atomico(int8_t* p, uint32_t meu) {
 // top = max(e + bitlen(v)) through its exponent field, and one FFMA against 1.5*2^23 rounds v * 2^(e - E) half to even
 // (|result| <= 127, inside the window).  A transposed block can never need the "one more bit" retry (|m| <= 127 going in).  Rows whose
 // exponents are more than 100 apart take integers.  Block 128: the four warps of a CTA (128 rows) exchange their columns' tops first.
+// Block 32: where the exponents lie at most 24 apart, two rows at a time in halves, which are as exact there (4 instructions an element instead of 11; the
+// rows' factors go through shared memory as halves).  16384 x (4096 + 1024) 65.7 -> 59.5 us, 2048 x (512 + 2048) 7.4 -> 6.95: what is left is the
+// latency of a warp's 32 loads at 16 warps an SM (128 registers, for the fp32 form).
 // CPT = 4: a lane does its 4 columns; CPT = 1, for matrices that would leave SMs idle: four warps share the 32 x 128 piece, a column each.
 // (Tiles staged in shared memory before, two shared loads per element: 16384 x (4096 + 1024) 95 -> 66 us, block 128 154 -> 50 us; 128 x 128
 // 6.4 -> 2.1 us.)
@@ -532,6 +535,80 @@ __device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int 
     const uint32_t longe = __reduce_or_sync(FULL, __vcmpgtu4(d4, 0x64646464u) & ~__vcmpeq4(ew, 0x81818181u));
     const int bl = lane >> 3, eref = (int)(int8_t)(mx4 >> (8 * bl));
     const bool largo = (longe >> (8 * bl)) & 1;
+    uint32_t emax4 = 0x80808080u;                                  // the new exponents of this lane's columns, -128 where it has none
+    if constexpr (BLK == 32) {
+        // In halves, two rows at a time: with exponents at most 24 apart (all-zero blocks apart) a mantissa times 2^(e - eref) is exact, the largest gives the
+        // block's exponent, and one fused multiply-add against 1.5 * 2^10 rounds half to even while the factor is at most 2^15 (a column
+        // whose largest element lies further below the largest exponent of its 32-column block: fp32, the whole warp).
+        __shared__ __align__(16) uint16_t esc_s[4][4][32];         // per warp and block: the rows' factors
+        const bool perto = __reduce_or_sync(FULL, __vcmpgtu4(d4, 0x18181818u) & ~__vcmpeq4(ew, 0x81818181u)) == 0;
+        if (perto) {
+            const uint32_t d24 = __vminu4(d4, 0x18181818u);
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const int d = (d24 >> (8 * b)) & 0xff;
+                esc_s[wid][b][lane] = d <= 14 ? (uint16_t)((15 - d) << 10) : (uint16_t)(1 << (24 - d));      // 2^-d
+            }
+            __syncwarp();
+            uint32_t he[16], t[CPT][16], mx[CPT];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint4 x = reinterpret_cast<const uint4*>(esc_s[wid][bl])[j];
+                he[4 * j] = x.x; he[4 * j + 1] = x.y; he[4 * j + 2] = x.z; he[4 * j + 3] = x.w;
+            }
+#pragma unroll
+            for (int c = 0; c < CPT; c++) mx[c] = 0;
+            const uint32_t qual = CPT == 1 ? (uint32_t)(k0 | (k0 + 4) << 4) : 0x5140u;
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                uint32_t hb, x[2];
+                asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(hb) : "r"(he[j]), "r"(0xE480E480u));                  // -1152 of them
+                x[0] = __byte_perm(w[2 * j], w[2 * j + 1], qual);
+                if (CPT > 1) x[1] = __byte_perm(w[2 * j], w[2 * j + 1], 0x7362);
+#pragma unroll
+                for (int c = 0; c < CPT; c++) {
+                    const uint32_t a = __byte_perm(x[c >> 1], 0x64646464u, c & 1 ? 0x4342 : 0x4140);       // 1152 + m
+                    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(t[c][j]) : "r"(a), "r"(he[j]), "r"(hb));
+                    asm("max.f16x2 %0, %0, %1;" : "+r"(mx[c]) : "r"(t[c][j] & 0x7FFF7FFFu));
+                }
+            }
+            int Eo[CPT];
+            bool serve = true;
+#pragma unroll
+            for (int c = 0; c < CPT; c++) {
+                const uint32_t m = max(mx[c] & 0xFFFFu, mx[c] >> 16);                                       // (not negative: ordered like their bits)
+                float f;
+                asm("{\n .reg .b16 h;\n cvt.u16.u32 h, %1;\n cvt.f32.f16 %0, h;\n}" : "=f"(f) : "r"(m));
+                Eo[c] = m == 0 ? SEM_TOPO : eref + (__float_as_int(f) >> 23) - 126 - 7;
+                serve = serve && (m == 0 || eref - Eo[c] <= 15);
+            }
+            if (__all_sync(FULL, serve)) {
+#pragma unroll
+                for (int c = 0; c < CPT; c++) {
+                    const int k = k0 + c;
+                    const size_t col = (size_t)col0 + k;
+                    const bool morto = Eo[c] < -126;
+                    if (dentro && Eo[c] > 126) reporta(E_EXP, kid, (long long)col * R + lin0, Eo[c], eref);
+                    const uint32_t B = morto ? 0u : (uint32_t)(15 + eref - Eo[c]) << 10, B2 = B | B << 16;  // 2^(eref - Eo)
+                    if (morto) Eo[c] = E_ZERO;
+                    if (dentro) {
+                        uint32_t q[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j++) asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(q[j]) : "r"(t[c][j]), "r"(B2), "r"(0x66006600u));
+                        uint4* dst = reinterpret_cast<uint4*>(A.Y + col * R + lin0);
+#pragma unroll
+                        for (int h = 0; h < 2; h++)
+                            dst[h] = make_uint4(__byte_perm(q[8 * h], q[8 * h + 1], 0x6420), __byte_perm(q[8 * h + 2], q[8 * h + 3], 0x6420),
+                                                __byte_perm(q[8 * h + 4], q[8 * h + 5], 0x6420), __byte_perm(q[8 * h + 6], q[8 * h + 7], 0x6420));
+                        A.EY[col * nby + lin0 / BLK] = (int8_t)Eo[c];
+                    }
+                    emax4 = (emax4 & ~(0xffu << (8 * k))) | ((uint32_t)(uint8_t)(int8_t)Eo[c] << (8 * k));
+                }
+                if (A.RM != nullptr && dentro) max4_atomico(A.RM + col0, emax4);
+                return;
+            }
+        }
+    }
     d4 = __vminu4(d4, 0x7f7f7f7fu);
     float fa[32];                                                  // 2^(e - eref)
 #pragma unroll
@@ -541,7 +618,6 @@ __device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int 
     };
     auto topo_de = [&](float mx) { return mx == 0.f ? SEM_TOPO : eref + (__float_as_int(mx) >> 23) - 126; };       // e + bitlen of the largest
     const int8_t *px0 = A.X + (size_t)lin0 * C + (dentro ? col0 : 0), *pe0 = A.EX + (size_t)lin0 * nbx + (dentro ? col0 : 0) / BLK;      // (cold path)
-    uint32_t emax4 = 0x80808080u;                                  // the new exponents of this lane's columns, -128 where it has none
     if (BLK == 128) {
         float mx[CPT];
 #pragma unroll

@@ -864,3 +864,30 @@ def test_atencao_back_com_P_alterado(amb):
     g_c = oc.atencao_back(para_gpu(go), para_gpu(qkv), para_gpu(P), Bt, T, H)
     torch.cuda.synchronize()
     compara("atencao_back with hand-zeroed tiles of P", list(g_c), list(g_r))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,C", [(128, 192), (256, 64), (8192, 1088)])
+@pytest.mark.parametrize("afasta,fundo", [(0, 0), (14, 0), (15, 8), (24, 9), (24, 10), (25, 0), (100, 0), (101, 0)])
+def test_transpoe_metades_e_fp32(amb, R, C, afasta, fundo):
+    """The transposition in halves up to its limits and beyond: rows whose exponents lie `afasta` below their neighbours' (24 is the last that halves hold, 100 the last
+    for fp32), zero blocks, columns that only the lower rows have and, with `fundo`, columns whose largest element lies so far down
+    that the factor is 2^15 or 2^16."""
+    ops, oc, reg = amb
+    ops.define_blk(32)
+    reg.novo_passo(0)
+    G = casos.Gen(R + C + afasta, 32)
+    m, E = G.bloco(R, C, e0=-10, espalha=0, zera=0.05)
+    zero = E == -127
+    E[1::3] -= afasta
+    E[zero] = -127
+    m[::3, 5::64] = 0
+    m[2::3, 5::64] = 0
+    if fundo:                                            # 1 at 2^-fundo, or nothing: Eo = -fundo - 6
+        m[:, 9::64] = 0
+        m[1::3, 9::64] = 1
+        E[1::3] = torch.where(zero[1::3], E[1::3], torch.full_like(E[1::3], -10 - fundo))
+    X = para_gpu((m, E))
+    out = oc.transpoe(X)
+    torch.cuda.synchronize()
+    compara(f"transpoe {R}x{C} afasta {afasta} fundo {fundo}", list(out), list(spec.Spec(32).transpoe(X)))
