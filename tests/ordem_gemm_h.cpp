@@ -162,12 +162,18 @@ struct Bloco {
     struct Multiplica {
         Bloco& B;
         int t = 0;
+        char ultima = 0;                                 // the last wait: for a stage or for a place
         void tile(int x) { t = x; }
         int plano(unsigned nt) { return B.planos[nt]; }
         bool encontra(unsigned fase) { B.encontro_b.chega(); return B.encontro_b.espera(fase); }
-        bool livre(int s, unsigned fase) { return B.tlivre[s].espera(fase); }
-        bool cheio(int s, unsigned fase) { return B.cheio[s].espera(fase); }
-        void arredonda(int s, int st, int j, bool, int c) { B.emite(s, st, j == 0, j == CB - 1, t, c); B.S.passa(B.S.demora(0.2)); }
+        bool livre(int s, unsigned fase) { ultima = 'e'; return B.tlivre[s].espera(fase); }
+        bool cheio(int s, unsigned fase) { ultima = 'l'; return B.cheio[s].espera(fase); }
+        void arredonda(int s, int st, int j, bool, int c) {
+            // (stages of one chunk are drained more slowly than chunks are loaded, four stages of two are not)
+            if (ultima != (CB == 1 ? 'e' : 'l')) throw Falha{"the wait for what comes first is the last one"};
+            B.emite(s, st, j == 0, j == CB - 1, t, c);
+            B.S.passa(B.S.demora(0.2));
+        }
         void soma(int s, int st, int i, bool fim, bool, int c) { B.emite(s, st, i == 0, fim, t, c); B.S.passa(B.S.demora(0.2)); }
     };
     template <bool SOMA>
