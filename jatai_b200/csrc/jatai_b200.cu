@@ -71,18 +71,19 @@ static int lanca_simt(const int8_t* A, const int8_t* EA, const int8_t* B, const 
     return fim();
 }
 
+// Whether the 8-bit kernel takes 64-column tiles (block 32 only) for a product of t 128 x 128 ones.  Up to 148 of them have an SM each and 16 drain warps: a tile takes
+// 0.6 to 0.8 of a 128-column one (2048 x 512 x 512 7.9 us against 10.8, K = 2048 20.6 against 29.8).  From 75 to 148 128-column tiles these have an SM
+// each, where two 64-column ones on an SM take longer (2048 x 768 x 512 12.0 us against 10.9, K = 2048 35.1 against 29.8).  Beyond, the pairs run without
+// wave boundaries (about 1.03 t/148 + 0.3 rounds of a 128-column tile) against ceil(t/148) whole rounds: 160 tiles, K = 512 17.9 us against 20.0,
+// 256 tiles 22.3 against 20.5.
+static bool estreito_i8(long long t) { return 2 * t <= N_SM || (t > N_SM && 1.03 * (double)t / N_SM + 0.3 < (double)((t + N_SM - 1) / N_SM)); }
 template <int BLK>
 static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const int8_t* EB, const int8_t* RA, const int8_t* RB,
                     const SaidaGemm& S, int M, int N, int K, int modo, int kid) {
     if (M <= 0 || N <= 0 || K <= 0 || M % 64 || N % TN || K % BLK || K % 32 || modo < 0 || modo > 4) return (int)cudaErrorInvalidValue;
     const bool alinhado = (((uintptr_t)A | (uintptr_t)B) & 15) == 0 && (((uintptr_t)EA | (uintptr_t)EB) & 3) == 0;
     bool usa_tc = g_via != 2 && M % tc::TM == 0 && K % tc::KC == 0 && alinhado;
-    // 64-column tiles (block 32 only), two CTAs per SM.  Alone on an SM such a tile takes ~0.77 of a 128-column one, so they
-    // win when 128-column tiles would leave half of the 148 SMs without a CTA; beyond that the pairs run without wave
-    // boundaries (~1.03 t/148 + 0.3 rounds of a 128-column tile, measured) against ceil(t/148) whole rounds
-    const long long tiles128 = (long long)(N / TN) * (M / tc::TM);
-    const double r128 = (double)((tiles128 + 147) / 148), r64 = 1.03 * (double)tiles128 / 148.0 + 0.3;
-    const bool estreito = BLK == 32 && usa_tc && g_tn != 128 && (g_tn == 64 || 2 * tiles128 <= 148 || r64 < r128);
+    const bool estreito = BLK == 32 && usa_tc && g_tn != 128 && (g_tn == 64 || estreito_i8((long long)(N / TN) * (M / tc::TM)));
     const int tn = estreito ? 64 : TN;
     CUtensorMap mA, mB;
     // a shape the tensor-core kernel takes never falls back silently: a tensor map that can not be encoded is an error

@@ -1,0 +1,82 @@
+"""Which kernel a call takes and with how many blocks (read from a recording of the call), and the kernels' forms that only particular sizes or data reach,
+each against the specification or the CUDA-core kernel."""
+import ctypes
+import tempfile
+
+import pytest
+import torch
+
+import casos
+from test_gpu_ops import compara
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def amb():
+    from jatai_b200 import ops, registro
+    ops.define_blk(32)
+    reg = registro.Registro(tempfile.mkdtemp(), "rotas", vigiar=True, eco=False, salvar=False)
+    oc = ops.OpsCuda(reg)
+    reg.novo_passo(0)
+    yield ops, oc, reg
+    ops.define_blk(32)
+    oc.lib.jt_gemm_via(0)
+    oc.lib.jt_gemm_tn(0)
+
+
+class _Lancamento(ctypes.Structure):                     # CUDA_KERNEL_NODE_PARAMS
+    _fields_ = [("func", ctypes.c_void_p), ("grade", ctypes.c_uint * 3), ("bloco", ctypes.c_uint * 3), ("smem", ctypes.c_uint),
+                ("args", ctypes.c_void_p), ("extra", ctypes.c_void_p), ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
+
+
+def lancamentos(oc, f, ao_lado=False):
+    """The kernels that f launches: (name, blocks)."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    f()                                                  # (kernel attributes are set at a first launch)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    vigiar, oc.reg.vigiar = oc.reg.vigiar, False         # (the check after each operator waits for the GPU)
+    try:
+        with torch.cuda.graph(g):
+            (oc.lib.jt_stream_ao_lado if ao_lado else oc.lib.jt_stream)(torch.cuda.current_stream().cuda_stream)
+            f()
+    finally:
+        oc.lib.jt_stream(None)
+        oc.reg.vigiar = vigiar
+    grafo, n = ctypes.c_void_p(g.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert cu.cuGraphGetNodes(grafo, None, ctypes.byref(n)) == 0
+    nos = (ctypes.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(grafo, nos, ctypes.byref(n)) == 0
+    r = []
+    for no in nos:
+        tipo = ctypes.c_int(-1)
+        assert cu.cuGraphNodeGetType(ctypes.c_void_p(no), ctypes.byref(tipo)) == 0
+        if tipo.value != 0:
+            continue
+        p, nome = _Lancamento(), ctypes.c_char_p()
+        assert cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(no), ctypes.byref(p)) == 0
+        assert (cu.cuKernelGetName(ctypes.byref(nome), ctypes.c_void_p(p.kern)) if p.kern else cu.cuFuncGetName(ctypes.byref(nome), ctypes.c_void_p(p.func))) == 0
+        r.append((nome.value.decode(), p.grade[0] * p.grade[1] * p.grade[2]))
+    return r
+
+
+def inteiros(semente):
+    g = torch.Generator(device="cuda").manual_seed(semente)
+    return lambda a, b, forma: torch.randint(a, b + 1, forma, generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+
+
+# ------------------------------------------------------------------------------------------------ products
+@pytest.mark.parametrize("M,N,largura,so", [(9472, 128, 64, 1), (9600, 128, 128, 0), (2048, 768, 128, 0), (18944, 128, 128, 0), (2048, 1280, 64, 0), (4096, 1024, 128, 0)])
+@pytest.mark.parametrize("cru", [False, True])
+def test_gemm_8_bits_largura(amb, M, N, largura, so, cru):
+    """The 8-bit kernel's tiles by their number: 74 (64 wide, an SM each), 75, 96 and 148 (128 wide), 160 (64 wide, two to an SM), 256 (128 wide, two rounds)."""
+    ops, oc, reg = amb
+    ints = inteiros(M + N)
+    A, B = ((ints(-127, 127, (R, 256)), ints(-12, -4, (R, 8))) for R in (M, N))
+    f = lambda: list(oc.gemm(A, B, cru=cru))
+    assert oc.lib.jt_gemm_via(2) == 0
+    quer = f()
+    assert oc.lib.jt_gemm_via(1) == 0
+    assert [n for n, b in lancamentos(oc, f) if "k_gemm_tc" in n and f"ELi{largura}ELb{so}E" in n and b == M // 128 * (N // largura)]
+    compara(f"{M}x{N}x256 cru {cru}", f(), quer)
