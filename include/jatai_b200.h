@@ -159,8 +159,8 @@ int jt_gemm_ws(const void* A, const void* EA, const void* B, const void* EB, voi
                int M, int N, int K, int modo, int kid);
 /* The stream set with jt_stream. */
 void* jt_stream_atual(void);
-/* jt_stream for launches that run beside another chain of launches, until the next jt_stream: products then take no more SMs than their tiles need.
- * Same results. */
+/* jt_stream for launches that run beside another chain of launches, until the next jt_stream: a product of a tensor-core kernel then has a block for each of
+ * its 128 x 128 tiles at most, or 48 (64-wide tiles, K ranges).  Same results. */
 void jt_stream_ao_lado(void* cuda_stream);
 /* R8[i] = max over the nb block exponents of row i of E (int8 [linhas, nb]): the RA / RB above. */
 int jt_max_linha(const void* E, void* R8, int linhas, int nb, int kid);

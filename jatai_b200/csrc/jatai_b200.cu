@@ -71,12 +71,17 @@ static int lanca_simt(const int8_t* A, const int8_t* EA, const int8_t* B, const 
     return fim();
 }
 
+// Beside another chain (jt_stream_ao_lado): most blocks of a product that has more of them than 128 x 128 tiles (64-column tiles, K ranges).
+constexpr int N_LADO = 48;
 // Whether the 8-bit kernel takes 64-column tiles (block 32 only) for a product of t 128 x 128 ones.  Up to 148 of them have an SM each and 16 drain warps: a tile takes
 // 0.6 to 0.8 of a 128-column one (2048 x 512 x 512 7.9 us against 10.8, K = 2048 20.6 against 29.8).  From 75 to 148 128-column tiles these have an SM
 // each, where two 64-column ones on an SM take longer (2048 x 768 x 512 12.0 us against 10.9, K = 2048 35.1 against 29.8).  Beyond, the pairs run without
 // wave boundaries (about 1.03 t/148 + 0.3 rounds of a 128-column tile) against ceil(t/148) whole rounds: 160 tiles, K = 512 17.9 us against 20.0,
 // 256 tiles 22.3 against 20.5.
-static bool estreito_i8(long long t) { return 2 * t <= N_SM || (t > N_SM && 1.03 * (double)t / N_SM + 0.3 < (double)((t + N_SM - 1) / N_SM)); }
+static bool estreito_i8(long long t) {
+    if (g_ao_lado && 2 * t > N_LADO) return false;
+    return 2 * t <= N_SM || (t > N_SM && 1.03 * (double)t / N_SM + 0.3 < (double)((t + N_SM - 1) / N_SM));
+}
 template <int BLK>
 static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const int8_t* EB, const int8_t* RA, const int8_t* RB,
                     const SaidaGemm& S, int M, int N, int K, int modo, int kid) {
@@ -95,8 +100,9 @@ static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const in
     const int unidades = usa_tc ? K / tc::KC : K / BLK;            // indivisible K units of the chosen kernel
     const long long tiles = usa_tc ? (long long)(N / tn) * (M / tc::TM) : (long long)(N / TN) * (M / 64);
     int partes = 1;
+    const int alvo = g_ao_lado && g_alvo_ctas > N_LADO ? N_LADO : g_alvo_ctas;
     if (modo == 1)
-        while (partes * (usa_tc ? 16 : 2) <= unidades && tiles * partes * 2 <= g_alvo_ctas && unidades % (partes * 2) == 0) partes *= 2;
+        while (partes * (usa_tc ? 16 : 2) <= unidades && tiles * partes * 2 <= alvo && unidades % (partes * 2) == 0) partes *= 2;
     const bool so = estreito && tiles * partes <= N_SM;
     if (partes > 1) {
         cudaError_t c = cudaMemsetAsync(S.C32, 0, (size_t)M * N * sizeof(int), g_stream);
@@ -147,7 +153,6 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
 // kernels forced one by one at 70 sizes the choice loses more than 3 % at three where every tile rounds, because it looks for sums (2048 x 1536 x 512 15.8 us
 // against 15.4, 2048 x 2048 x 512 with ReLU^2 18.3 against 17.7, 16384 x 4096 x 1024 256 against 248; where none rounds they are worth 16.2 -> 13.2, 18.0 -> 15.1,
 // 256 -> 167), at 8192 x 512 x 128 (14.6 against 13.7 with the 8-bit kernel) and, block 128, at 1024 x 512 x 4096 raw (34.8 against 25.2).
-constexpr int N_LADO = 48;                                           // most blocks of a product beside another chain whose tiles are not the largest
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
 static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
     const double n = (K + 63) / 64;
@@ -160,8 +165,9 @@ static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
     // (0.26 to 0.30 us a chunk): 4096 x 4096 x 4096 263 us, 183 with 128-wide ones.  So they have one wave or none.
     // Beside another chain (jt_stream_ao_lado) it is the SMs' time that counts: as many 64-wide tiles as fill the chip, and K ranges over clusters, are
     // done sooner but hold more SMs (2048 x 512 x 2048 raw 17.3 us on 128 SMs or 22.8 on 64).  A third of the chip is free for them (a short step's
-    // chains are long ones): the 12-layer step takes 3082 to 3172 us without a limit, 3073 with one of 24 or 48 blocks, 3077 with none at all,
-    // 6 layers of 4096 tokens x 256 columns 1261, 1195, 1149, 1166, 5 layers of 4096 x 128 799, 794, 799, 814.
+    // chains are long ones), in the half-precision kernel and in the 8-bit one: N_LADO blocks.  Steps with 24, 36 or 48: 6 layers of
+    // 512 columns 1184, 1194, 1193 us with 1024 tokens (1259 before the 8-bit kernel kept to it), 1027, 1016, 1017 with 512; 6 layers of 4096 tokens x 256
+    // columns 1388, 1410, 1416; 12 layers of 2048 x 512 3120 each.
     const int vagas = g_ao_lado ? N_LADO : N_SM;
     const double p64 = (double)(M + N) * K * 2 > 48e6 ? 0.28 : 0.18;
     c.h64 = blk == 32 && t64 <= vagas ? prep + n * p64 + 2.9 : 1e9;
@@ -177,6 +183,7 @@ static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
         if (x < c.h64) { c.h64 = x; c.grupo = g; }
     }
     if (M % tc::TM || K % tc::KC) c.i8 = 1e9;                                           // whole tiles only
+    else if (blk == 32 && g_ao_lado && !estreito_i8(t128)) c.i8 = 0.5 + ondas(t128, N_SM) * (n * 0.79 + 4.0 + (cru ? 2.2 : 0.0));
     else if (blk == 32) c.i8 = t64 <= N_SM ? n * 0.55 + 3.4 : 2.5 + ondas(t64, 2 * N_SM) * (n * 0.80 + 3.2);
     else c.i8 = 2.5 + (t128 <= N_SM ? n * 0.55 + 1.0 : ondas(t128, N_SM) * (n * 0.41 + 3.0));
     return c;
@@ -329,8 +336,8 @@ void jt_stream(void* st) {
     g_stream = (cudaStream_t)st;
     espera_limpeza(g_stream);
 }
-// jt_stream for a chain of launches that runs beside another one, until the next jt_stream: products then take no more SMs than their tiles need
-// (custos_gemm).  The results are the same.
+// jt_stream for a chain of launches that runs beside another one, until the next jt_stream: a product of either tensor-core kernel then has a block for each of its
+// 128 x 128 tiles at most, or N_LADO.  The results are the same.
 void jt_stream_ao_lado(void* st) {
     jt_stream(st);
     g_ao_lado = true;

@@ -80,3 +80,40 @@ def test_gemm_8_bits_largura(amb, M, N, largura, so, cru):
     assert oc.lib.jt_gemm_via(1) == 0
     assert [n for n, b in lancamentos(oc, f) if "k_gemm_tc" in n and f"ELi{largura}ELb{so}E" in n and b == M // 128 * (N // largura)]
     compara(f"{M}x{N}x256 cru {cru}", f(), quer)
+
+
+# ------------------------------------------------------------------------------------------------ beside another chain
+LADO = 48                                                # most blocks of a product there that has more of them than 128 x 128 tiles
+
+
+@pytest.mark.parametrize("via", [0, 1])
+@pytest.mark.parametrize("M,N,K,cru", [(1536, 512, 1024, True), (2048, 512, 1024, True), (512, 2048, 1024, True), (1024, 512, 512, True), (2048, 512, 512, False),
+                                       (512, 512, 256, True), (256, 256, 4096, True), (384, 1024, 4096, True), (512, 384, 128, False), (10240, 128, 128, False)])
+def test_ao_lado_blocos(amb, M, N, K, cru, via):
+    """Under jt_stream_ao_lado a product of any kernel has at most 48 blocks, or one for each of its 128 x 128 tiles, and gives the same bits."""
+    ops, oc, reg = amb
+    ints = inteiros(M + N + K)
+    A, B = ((ints(-127, 127, (R, K)), ints(-12, -4, (R, K // 32))) for R in (M, N))
+    assert oc.lib.jt_gemm_via(via) == 0
+    f = lambda: oc.gemm(A, B, cru=cru)
+    quer = f()
+    blocos = [b for n, b in lancamentos(oc, f, ao_lado=True) if "k_gemm" in n]
+    assert len(blocos) == 1 and blocos[0] <= max(LADO, (M // 128) * (N // 128))
+    try:
+        oc.lib.jt_stream_ao_lado(None)
+        tem = f()
+    finally:
+        oc.lib.jt_stream(None)
+    torch.cuda.synchronize()
+    compara(f"{M}x{N}x{K} cru {cru} via {via}", list(tem), list(quer))
+
+
+@pytest.mark.parametrize("M,N,K", [(1536, 512, 1024), (2048, 512, 1024), (512, 2048, 1024)])
+def test_ao_lado_o_mesmo_nucleo(amb, M, N, K):
+    """What takes the half-precision kernel alone takes it beside another chain too: that 64-wide tiles are ruled out there does not send it to the 8-bit kernel."""
+    ops, oc, reg = amb
+    ints = inteiros(M + N + K)
+    A, B = ((ints(-127, 127, (R, K)), ints(-12, -4, (R, K // 32))) for R in (M, N))
+    f = lambda: oc.gemm(A, B, cru=True)
+    for ao_lado in (False, True):
+        assert [n for n, _ in lancamentos(oc, f, ao_lado) if "k_gemm_h" in n]
