@@ -154,11 +154,16 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
 // against 15.4, 2048 x 2048 x 512 with ReLU^2 18.3 against 17.7, 16384 x 4096 x 1024 256 against 248; where none rounds they are worth 16.2 -> 13.2, 18.0 -> 15.1,
 // 256 -> 167), at 8192 x 512 x 128 (14.6 against 13.7 with the 8-bit kernel) and, block 128, at 1024 x 512 x 4096 raw (34.8 against 25.2).
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
-static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
+static Custos custos_gemm(int blk, int M, int N, int K, int modo) {
+    const bool cru = modo == 1;
     const double n = (K + 63) / 64;
     const long long t128 = (long long)(N / 128) * ((M + 127) / 128), t64 = 2 * t128;
     auto ondas = [](long long t, int vagas) { return (double)((t + vagas - 1) / vagas); };
-    const double prep = 4.0 + (double)(M + N) * K * 3 / 4e6;                            // k_prep_h: a launch, and 3 bytes per element at 4 TB/s
+    const double prep = 4.0 + (double)(M + N) * K * 3 / 4.8e6;                          // k_prep_h: a launch, and 3 bytes per element at 4.8 TB/s
+    // What a raw output, or the backward of ReLU^2, costs a wave of tiles more than a block output does.  With it, short K is where the lines lie for products of more tiles than
+    // 64-wide ones have SMs: 2048 x 1536 x 128 9.8 us with the 8-bit kernel and 11.5 with the half-precision one, raw 13.0 and 16.5, 2048 x 640 x 256
+    // 7.8 and 8.7; 2048 x 1536 x 256 12.8 and 13.1, or 11.5 with exponents that round nothing.
+    auto saida = [&](double crua, double relu2_back) { return cru ? crua : modo == 4 ? relu2_back : 0.0; };
     Custos c;
     c.grupo = 1;
     // 64-wide tiles read 1.5 times as much for an output element.  With all SMs at it, or operands beyond 48 MB, they wait for the cache
@@ -174,7 +179,7 @@ static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
     if (blk == 32) {
         int partes = 1;                                                                 // (gemm_h: raw outputs of few 128-wide tiles, clearing and atomic additions 15 us)
         while (cru && !g_ao_lado && t128 * partes * 2 <= N_SM && n >= partes * 64) partes *= 2;
-        c.h128 = prep + ondas(t128 * partes, N_SM) * (n / partes * 0.31 + 2.4) + (partes > 1 ? 15.0 : 0.0);
+        c.h128 = prep + 1.0 + ondas(t128 * partes, N_SM) * (n / partes * 0.31 + 2.4 + saida(2.6, 1.5)) + (partes > 1 ? 15.0 : 0.0);
     } else
         c.h128 = prep + 1.5 + ondas(t128, N_SM) * (n * 0.25 + 1.7);
     // K ranges over a cluster while every block has an SM for itself (132 blocks in clusters of 4, 120 in clusters of 8 are at work at once) and keeps 4 chunks
@@ -183,15 +188,15 @@ static Custos custos_gemm(int blk, int M, int N, int K, bool cru) {
         if (x < c.h64) { c.h64 = x; c.grupo = g; }
     }
     if (M % tc::TM || K % tc::KC) c.i8 = 1e9;                                           // whole tiles only
-    else if (blk == 32 && g_ao_lado && !estreito_i8(t128)) c.i8 = 0.5 + ondas(t128, N_SM) * (n * 0.79 + 4.0 + (cru ? 2.2 : 0.0));
-    else if (blk == 32) c.i8 = t64 <= N_SM ? n * 0.55 + 3.4 : 2.5 + ondas(t64, 2 * N_SM) * (n * 0.80 + 3.2);
+    else if (blk == 32 && estreito_i8(t128)) c.i8 = t64 <= N_SM ? n * 0.55 + 3.4 : ondas(t64, 2 * N_SM) * (n * 0.76 + 3.4 + saida(1.75, 0.9));
+    else if (blk == 32) c.i8 = 0.5 + ondas(t128, N_SM) * (n * 0.79 + 4.0 + saida(2.2, 1.25));
     else c.i8 = 2.5 + (t128 <= N_SM ? n * 0.55 + 1.0 : ondas(t128, N_SM) * (n * 0.41 + 3.0));
     return c;
 }
 // whether a caller with a workspace takes the half-precision path
 static bool usa_h(int M, int N, int K, int modo) {
     if (g_via != 0) return g_via == 4;
-    const Custos c = custos_gemm(g_blk, M, N, K, modo == 1);
+    const Custos c = custos_gemm(g_blk, M, N, K, modo);
     return (c.h64 < c.h128 ? c.h64 : c.h128) < c.i8;
 }
 template <int BLK, int MODO, int TNv, bool GRUPO, bool SOMA = false>
@@ -215,7 +220,7 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     uint32_t *nA = (uint32_t*)(ws + e.nA), *nB = (uint32_t*)(ws + e.nB);
     const int nfx = (K + 511) / 512, ctasA = (M + 31) / 32 * nfx, ctasB = N / 32 * nfx;
     th::ArgsPrepH P = {{A, B}, {EA, EB}, {RA, RB}, {Ah, Bh}, {RAw, RBw}, {nA, nB}, {M, N}, ctasA, K};
-    const Custos c = custos_gemm(BLK, M, N, K, modo == 1);
+    const Custos c = custos_gemm(BLK, M, N, K, modo);
     const bool estreito = BLK == 32 && g_tn != 128 && (g_tn == 64 || c.h64 < c.h128);
     const int tn = estreito ? 64 : TN;
     CUtensorMap mA, mB;

@@ -82,6 +82,22 @@ def test_gemm_8_bits_largura(amb, M, N, largura, so, cru):
     compara(f"{M}x{N}x256 cru {cru}", f(), quer)
 
 
+@pytest.mark.parametrize("M,N,K,op,nucleo", [(2048, 640, 128, "gemm", "tc"), (2048, 640, 256, "gemm cru", "tc"), (1920, 1024, 256, "gemm", "tc"), (2048, 1536, 128, "gemm", "tc"),
+                                             (2048, 1536, 128, "gemm cru", "tc"), (8192, 512, 128, "gemm cru", "tc"), (2048, 1280, 256, "gemm_relu2_back", "tc"),
+                                             (2048, 1536, 512, "gemm", "h"), (2048, 2048, 256, "gemm", "h"), (4096, 2048, 128, "gemm", "h"), (2048, 1024, 1024, "gemm cru", "h")])
+def test_gemm_escolha_com_K_curto(amb, M, N, K, op, nucleo):
+    """Products of one to four rounds of tiles and short K take the kernel that is measured to be faster: the 8-bit one up to K = 128 or 256, by the output."""
+    ops, oc, reg = amb
+    ints = inteiros(M + K)
+    A, B, X = (ints(-127, 127, (M, K)), ints(-9, -8, (M, K // 32))), (ints(-127, 127, (N, K)), ints(-9, -8, (N, K // 32))), (ints(-127, 127, (M, N)), ints(-12, -4, (M, N // 32)))
+    f = lambda: casos.roda(oc, op.split()[0], (A, B, X) if "back" in op else (A, B), dict(cru=True) if "cru" in op else {})
+    assert oc.lib.jt_gemm_via(2) == 0
+    quer = f()
+    assert oc.lib.jt_gemm_via(0) == 0
+    assert [n for n, _ in lancamentos(oc, f) if f"k_gemm_{nucleo}" in n]
+    compara(f"{op} {M}x{N}x{K}", f(), quer)
+
+
 # ------------------------------------------------------------------------------------------------ beside another chain
 LADO = 48                                                # most blocks of a product there that has more of them than 128 x 128 tiles
 
