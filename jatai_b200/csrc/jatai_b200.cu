@@ -82,6 +82,21 @@ static bool estreito_i8(long long t) {
     if (g_ao_lado && 2 * t > N_LADO) return false;
     return 2 * t <= N_SM || (t > N_SM && 1.03 * (double)t / N_SM + 0.3 < (double)((t + N_SM - 1) / N_SM));
 }
+// K ranges of a raw product of block 128, estimated in microseconds: a 64-element chunk of one wave of tiles takes the 8-bit kernel 0.345 and the half-precision one 0.20,
+// clearing the output and adding the ranges atomically 10 and 0.6 for every MB that is added.  8-bit kernel: 256 x 256 x 2048 17.2 in one range, 22.7 in two,
+// K = 4096 28.1 in one, 19.0 in sixteen; half precision: 1024 x 512 x 4096 25.6 in one, 34.4 in two, 512 x 512 x 16384 70 in one, 40 in eight.
+constexpr double I8_B128 = 0.345, H_B128 = 0.20;
+static double soma_partes(int M, int N, int partes) { return partes > 1 ? 10.0 + (double)M * N * partes / 4.2e5 : 0.0; }
+static int partes_b128(int M, int N, int K, double pedaco, bool iguais) {
+    const long long t = (long long)(N / 128) * ((M + 127) / 128);
+    const double n = (K + 63) / 64;
+    int melhor = 1;
+    // Beside another chain none: a step of 6 layers with 4096 tokens x 256 columns took 1368 us with up to 48 blocks of them, 1342 without.
+    if (g_ao_lado) return 1;
+    for (int p = 2; t * p <= g_alvo_ctas && K / 128 >= 2 * p && (!iguais || K / 128 % p == 0); p *= 2)      // (two blocks at least; of equal length for the 8-bit kernel)
+        if (n / p * pedaco + soma_partes(M, N, p) < n / melhor * pedaco + soma_partes(M, N, melhor)) melhor = p;
+    return melhor;
+}
 template <int BLK>
 static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const int8_t* EB, const int8_t* RA, const int8_t* RB,
                     const SaidaGemm& S, int M, int N, int K, int modo, int kid) {
@@ -97,11 +112,13 @@ static int gemm_blk(const int8_t* A, const int8_t* EA, const int8_t* B, const in
     // split-K (raw output only): powers of two while the grid stays below the target and the K range divides evenly.  Clearing the output and
     // adding atomically cost 6 to 9 us, a unit of the tensor-core kernel takes 1.2: a part keeps at least 8 (512 x 256 x 256: 13.8 us in
     // two parts, 6.8 in one).
+    // Block 128 takes what partes_b128 finds best.
     const int unidades = usa_tc ? K / tc::KC : K / BLK;            // indivisible K units of the chosen kernel
     const long long tiles = usa_tc ? (long long)(N / tn) * (M / tc::TM) : (long long)(N / TN) * (M / 64);
     int partes = 1;
     const int alvo = g_ao_lado && g_alvo_ctas > N_LADO ? N_LADO : g_alvo_ctas;
-    if (modo == 1)
+    if (modo == 1 && BLK == 128 && usa_tc) partes = partes_b128(M, N, K, I8_B128, true);
+    else if (modo == 1)
         while (partes * (usa_tc ? 16 : 2) <= unidades && tiles * partes * 2 <= alvo && unidades % (partes * 2) == 0) partes *= 2;
     const bool so = estreito && tiles * partes <= N_SM;
     if (partes > 1) {
@@ -159,7 +176,7 @@ static Custos custos_gemm(int blk, int M, int N, int K, int modo) {
     const double n = (K + 63) / 64;
     const long long t128 = (long long)(N / 128) * ((M + 127) / 128), t64 = 2 * t128;
     auto ondas = [](long long t, int vagas) { return (double)((t + vagas - 1) / vagas); };
-    const double prep = 4.0 + (double)(M + N) * K * 3 / 4.8e6;                          // k_prep_h: a launch, and 3 bytes per element at 4.8 TB/s
+    const double prep = 4.0 + (double)(M + N) * K * 3 / (blk == 32 ? 4.8e6 : 5.3e6);    // k_prep_h: a launch, and 3 bytes per element at 4.8 TB/s (block 128: 5.3)
     // What a raw output, or the backward of ReLU^2, costs a wave of tiles more than a block output does.  With it, short K is where the lines lie for products of more tiles than
     // 64-wide ones have SMs: 2048 x 1536 x 128 9.8 us with the 8-bit kernel and 11.5 with the half-precision one, raw 13.0 and 16.5, 2048 x 640 x 256
     // 7.8 and 8.7; 2048 x 1536 x 256 12.8 and 13.1, or 11.5 with exponents that round nothing.
@@ -180,8 +197,11 @@ static Custos custos_gemm(int blk, int M, int N, int K, int modo) {
         int partes = 1;                                                                 // (gemm_h: raw outputs of few 128-wide tiles, clearing and atomic additions 15 us)
         while (cru && !g_ao_lado && t128 * partes * 2 <= N_SM && n >= partes * 64) partes *= 2;
         c.h128 = prep + 1.0 + ondas(t128 * partes, N_SM) * (n / partes * 0.31 + 2.4 + saida(2.6, 1.5)) + (partes > 1 ? 15.0 : 0.0);
-    } else
-        c.h128 = prep + 1.5 + ondas(t128, N_SM) * (n * 0.25 + 1.7);
+    } else {
+        // (several waves of tiles wait for the cache: 0.25 a chunk.  12288 x 640 x 11136 raw 295 us, 275 with the 8-bit kernel; 8192 x 2048 x 2048 99.5 and 121.5)
+        const int partes = cru ? partes_b128(M, N, K, H_B128, false) : 1;
+        c.h128 = prep + (t128 <= N_SM ? 3.4 + n / partes * H_B128 + soma_partes(M, N, partes) + (cru ? 1.9 : 0.0) : 1.7 + ondas(t128, N_SM) * (n * 0.25 + (cru ? 4.2 : 1.7)));
+    }
     // K ranges over a cluster while every block has an SM for itself (132 blocks in clusters of 4, 120 in clusters of 8 are at work at once) and keeps 4 chunks
     for (int g = 2; blk == 32 && g <= 8 && t64 * g <= vagas && t64 * g <= (g == 8 ? 120 : g == 4 ? 132 : N_SM) && n >= 4 * g; g *= 2) {
         const double x = prep + n / g * p64 + 3.9;
@@ -190,7 +210,10 @@ static Custos custos_gemm(int blk, int M, int N, int K, int modo) {
     if (M % tc::TM || K % tc::KC) c.i8 = 1e9;                                           // whole tiles only
     else if (blk == 32 && estreito_i8(t128)) c.i8 = t64 <= N_SM ? n * 0.55 + 3.4 : ondas(t64, 2 * N_SM) * (n * 0.76 + 3.4 + saida(1.75, 0.9));
     else if (blk == 32) c.i8 = 0.5 + ondas(t128, N_SM) * (n * 0.79 + 4.0 + saida(2.2, 1.25));
-    else c.i8 = 2.5 + (t128 <= N_SM ? n * 0.55 + 1.0 : ondas(t128, N_SM) * (n * 0.41 + 3.0));
+    else {
+        const int partes = cru ? partes_b128(M, N, K, I8_B128, true) : 1;
+        c.i8 = t128 > N_SM ? 2.5 + ondas(t128, N_SM) * (cru ? n * 0.365 + 5.0 : n * 0.41 + 3.0) : cru ? 6.3 + n / partes * I8_B128 + soma_partes(M, N, partes) : 4.6 + n * 0.375;
+    }
     return c;
 }
 // whether a caller with a workspace takes the half-precision path
@@ -229,7 +252,8 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     const long long tiles = (long long)(N / tn) * ((M + 127) / 128);
     const bool grupo = estreito && c.grupo > 1;
     int partes = grupo ? c.grupo : 1;
-    if (modo == 1 && !grupo && !g_ao_lado)
+    if (modo == 1 && BLK == 128) partes = partes_b128(M, N, K, H_B128, false);
+    else if (modo == 1 && !grupo && !g_ao_lado)
         while (tiles * partes * 2 <= g_alvo_ctas && nped >= partes * 2 * 32) partes *= 2;
     const int ppp = ((nped + partes - 1) / partes + uni - 1) / uni * uni;
     if (!grupo) partes = (nped + ppp - 1) / ppp;                   // (in a cluster a block without chunks adds zeros)

@@ -98,6 +98,23 @@ def test_gemm_escolha_com_K_curto(amb, M, N, K, op, nucleo):
     compara(f"{op} {M}x{N}x{K}", f(), quer)
 
 
+@pytest.mark.parametrize("M,N,K,via,nucleo,blocos", [(1024, 512, 4096, 0, "h", 32), (256, 256, 2048, 1, "tc", 4), (256, 256, 4096, 0, "tc", 64), (512, 512, 8192, 0, "tc", 128),
+                                                     (256, 256, 4224, 1, "tc", 4), (512, 256, 4608, 1, "tc", 32), (320, 512, 8320, 0, "h", 96), (128, 128, 16384, 4, "h", 32),
+                                                     (1024, 1024, 4096, 4, "h", 64), (12288, 640, 4096, 0, "tc", 480)])
+def test_gemm_bloco_128_partes(amb, M, N, K, via, nucleo, blocos):
+    """Raw products of block 128 and few tiles: K ranges where they are worth what clearing and adding cost, by the kernel that is faster with them."""
+    ops, oc, reg = amb
+    ops.define_blk(128)
+    ints = inteiros(M + N + K)
+    A, B = ((ints(-127, 127, (R, K)), ints(-12, -4, (R, K // 128))) for R in (M, N))
+    f = lambda: list(oc.gemm(A, B, cru=True))
+    assert oc.lib.jt_gemm_via(2) == 0
+    quer = f()
+    assert oc.lib.jt_gemm_via(via) == 0
+    assert [b for n, b in lancamentos(oc, f) if f"k_gemm_{nucleo}" in n] == [blocos]
+    compara(f"{M}x{N}x{K} via {via}", f(), quer)
+
+
 # ------------------------------------------------------------------------------------------------ beside another chain
 LADO = 48                                                # most blocks of a product there that has more of them than 128 x 128 tiles
 
