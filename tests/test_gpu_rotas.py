@@ -7,7 +7,8 @@ import pytest
 import torch
 
 import casos
-from test_gpu_ops import compara
+from oracle import spec
+from test_gpu_ops import compara, para_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -64,6 +65,60 @@ def lancamentos(oc, f, ao_lado=False):
 def inteiros(semente):
     g = torch.Generator(device="cuda").manual_seed(semente)
     return lambda a, b, forma: torch.randint(a, b + 1, forma, generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+
+
+# ------------------------------------------------------------------------------------------------ transposition
+def em_metades(X, colunas):
+    """How many (32 rows x 128 columns, columns a lane) pieces meet both conditions of the transposition in halves, of how many: exponents at most 24 apart,
+    all-zero blocks aside, and no column whose largest element lies so far down that its factor exceeds 2^15."""
+    m, E = (t.to(torch.int64) for t in X)
+    R, C = m.shape
+    falta = -C % 128
+    m = torch.nn.functional.pad(m, (0, falta)).reshape(R // 32, 32, -1, 4, 32)
+    E = torch.nn.functional.pad(E, (0, falta // 32), value=casos.E_ZERO).reshape(R // 32, 32, -1, 4)
+    ref = E.amax(1, keepdim=True)
+    perto = ((ref - E <= 24) | (E == casos.E_ZERO)).all(3).all(1)
+    # log2 of a column's largest element: a mantissa below 2^b at exponent e counts b + e
+    bits = torch.frexp(m.abs().to(torch.float64))[1].to(torch.int64)
+    topo = torch.where(m != 0, bits + E[..., None], torch.full_like(m, -1000)).amax(1)
+    serve = (topo == -1000) | (ref[:, 0, :, :, None] - (topo - 7) <= 15)
+    serve = serve.reshape(*serve.shape[:3], 8, 4)        # 8 lanes of 4 columns in a block
+    serve = serve.all(4).all(3).all(2) if colunas == 4 else serve.all(3).all(2)
+    return int((perto[..., None] & serve.reshape(*perto.shape, -1)).sum()), serve.numel()
+
+
+@pytest.mark.parametrize("R,C,colunas", [(128, 192, 1), (8192, 1088, 4)])
+@pytest.mark.parametrize("afasta", [14, 15, 20, 24])
+def test_transpoe_metades_todos_os_fatores(amb, R, C, colunas, afasta):
+    """Every factor 2^0 to 2^-afasta of the transposition in halves, subnormal ones among them, beside rows at the block's largest exponent, so that every piece
+    is put out in halves."""
+    ops, oc, reg = amb
+    G = casos.Gen(R + C + afasta, 32)
+    m, E = G.bloco(R, C, e0=-10, espalha=0, zera=0.05)
+    zero = E == casos.E_ZERO
+    E[1::3] -= torch.randint(0, afasta + 1, E[1::3].shape, generator=G.g).to(torch.int8)
+    E[1::12] = -10 - afasta
+    E[zero] = casos.E_ZERO
+    tem, de = em_metades((m, E), colunas)
+    assert tem == de
+    X = para_gpu((m, E))
+    compara(f"transpoe {R}x{C} afasta {afasta}", list(oc.transpoe(X)), list(spec.Spec(32).transpoe(X)))
+
+
+@pytest.mark.parametrize("R,C,colunas", [(128, 192, 1), (8192, 1088, 4)])
+@pytest.mark.parametrize("fundo", [8, 9, 10])
+def test_transpoe_metades_fatores_grandes(amb, R, C, colunas, fundo):
+    """In one block of four, a column that holds nothing but ones `fundo` below the largest exponent: its factor is 2^14, 2^15 (the last that halves hold) or 2^16."""
+    ops, oc, reg = amb
+    G = casos.Gen(R + C + fundo, 32)
+    m, E = G.bloco(R, C, e0=-10, espalha=0)
+    E[1::3, 1::4] = -10 - fundo
+    m[:, 41::128] = 0
+    m[1::3, 41::128] = 1
+    tem, de = em_metades((m, E), colunas)
+    assert tem == de if fundo <= 9 else tem < de
+    X = para_gpu((m, E))
+    compara(f"transpoe {R}x{C} fundo {fundo}", list(oc.transpoe(X)), list(spec.Spec(32).transpoe(X)))
 
 
 # ------------------------------------------------------------------------------------------------ products
