@@ -170,6 +170,35 @@ def test_gemm_bloco_128_partes(amb, M, N, K, via, nucleo, blocos):
     compara(f"{M}x{N}x{K} via {via}", f(), quer)
 
 
+@pytest.mark.parametrize("caso", ["comum", "saturados", "expoentes afastados", "linhas nulas", "acumuladores grandes"])
+@pytest.mark.parametrize("op", ["gemm", "gemm cru", "gemm_soma", "gemm_relu2", "gemm_relu2_back"])
+def test_gemm_64_dois_por_sm(amb, op, caso):
+    """The 8-bit kernel's 64-wide tiles with two blocks on an SM (more than 148 of them) in every output mode: the rounding's range check and the output stage's
+    integer side as well as the ordinary ones."""
+    ops, oc, reg = amb
+    M, N, K = 2432, 1024, 512
+    G = casos.Gen(4243, 32)
+    A, B, X = G.bloco(M, K, espalha=2 if caso != "comum" else 8, zera=0.05 if caso == "comum" else 0.0), G.bloco(N, K, espalha=2), G.bloco(M, N, espalha=3)
+    if caso == "saturados":
+        A[0][5::64], B[0][7::32] = 127, -127
+        A[1][5::64], B[1][7::32] = -8, -8
+    elif caso == "expoentes afastados":
+        B[1][0::2] -= 50
+        B[1][1::2] += 20
+    elif caso == "linhas nulas":
+        B[0][::3], B[1][::3] = 0, casos.E_ZERO
+    elif caso == "acumuladores grandes":
+        A, B = (torch.full_like(A[0], 127), torch.full_like(A[1], -8)), (torch.full_like(B[0], 127), torch.full_like(B[1], -8))
+    A, B, X = para_gpu(A), para_gpu(B), para_gpu(X)
+    args, kw = ((A, B, X) if op in ("gemm_soma", "gemm_relu2_back") else (A, B)), (dict(cru=True) if op == "gemm cru" else {})
+    assert oc.lib.jt_gemm_via(1) == 0 and oc.lib.jt_gemm_tn(64) == 0
+    f = lambda: casos.roda(oc, op.split()[0], args, kw)
+    assert [(n, b) for n, b in lancamentos(oc, f) if "k_gemm_tc" in n and "ELi1ELi64ELb0E" in n and b == 304]
+    tem = f()
+    torch.cuda.synchronize()
+    compara(f"{op} {caso}", tem, casos.roda(spec.Spec(32), op.split()[0], args, kw))
+
+
 # ------------------------------------------------------------------------------------------------ beside another chain
 LADO = 48                                                # most blocks of a product there that has more of them than 128 x 128 tiles
 
