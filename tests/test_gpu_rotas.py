@@ -199,6 +199,24 @@ def test_gemm_64_dois_por_sm(amb, op, caso):
     compara(f"{op} {caso}", tem, casos.roda(spec.Spec(32), op.split()[0], args, kw))
 
 
+@pytest.mark.parametrize("M,N,soma", [(4736, 512, False), (19072, 128, True)])
+@pytest.mark.parametrize("op", ["gemm", "gemm_relu2"])
+@pytest.mark.parametrize("afasta", [0, 12])
+def test_gemm_somas_linha(amb, M, N, soma, op, afasta):
+    """148 tiles, a tile per SM, and 149: from there on half-precision products look for tiles that add up in tensor memory.  With exponents that round nothing
+    and with ones that round everywhere."""
+    ops, oc, reg = amb
+    K = 512
+    ints = inteiros(M + afasta)
+    A, B = ((ints(-127, 127, (R, K)), ints(-9 - afasta, -8, (R, K // 32))) for R in (M, N))
+    assert oc.lib.jt_gemm_via(2) == 0
+    quer = casos.roda(oc, op, (A, B), {})
+    assert oc.lib.jt_gemm_via(4) == 0
+    f = lambda: casos.roda(oc, op, (A, B), {})
+    assert [n for n, _ in lancamentos(oc, f) if "k_gemm_h" in n and f"ELi128ELb0ELb{int(soma)}E" in n]
+    compara(f"{op} {M}x{N}x{K} afasta {afasta}", f(), quer)
+
+
 # ------------------------------------------------------------------------------------------------ beside another chain
 LADO = 48                                                # most blocks of a product there that has more of them than 128 x 128 tiles
 
