@@ -253,8 +253,8 @@ __device__ __forceinline__ bool barreira_ou(bool sim) {
     return r != 0;
 }
 
-// SOMA: tiles in which nothing is rounded add up in tensor memory (128-wide tiles of block 32; the 64-wide ones have no registers for the second
-// drain, and block 128 drains every four MMAs as it is).  The loops with and without sums are both in the kernel: with the second drain in
+// SOMA: tiles in which nothing is rounded add up in tensor memory (128-wide tiles of block 32; 64-wide ones, one tile to an SM, were not tried with
+// it, and block 128 drains every four MMAs as it is).  The loops with and without sums are both in the kernel: with the second drain in
 // them the loops that round come out up to 5 % slower.
 template <int BLK, int MODO, int TNv, bool GRUPO, bool SOMA>
 __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, 1) k_gemm_h(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, 1) k_gemm_h(const __gri
     // can add up where none of their products is rounded (shift <= 4) and their sums stay below 2^24 last places of the finest product,
     // 2^(4 - largest shift), by Cauchy-Schwarz for the whole tile.  A tile that fails anywhere is rounded throughout.  The drain warps make all
     // of them, a tile each at a time, while the first operands are on their way; a block without a tile that adds up takes the loops
-    // without sums.  (Made by the loading warp tile by tile and waited for by everyone, they cost a tile up to 1000 cycles.  With exponents
-    // that round: no sums at all / plans tile by tile / as it is 75.6 / 79.2 / 74.6 us for 16384 x 1024 x 1024, 213 / 227 / 209 for
+    // without sums.  (Made by the loading warp tile by tile and waited for by everyone, they cost a tile up to 1000 cycles.  With the rounding loops of that
+    // time, 138 instructions a chunk, and exponents that round: no sums at all / plans tile by tile / made here 75.6 / 79.2 / 74.6 us for 16384 x 1024 x 1024, 213 / 227 / 209 for
     // 16384 x 4096 x 512 with the sum, 289 / 305 / 293 for 16384 x 4096 x 1024 with ReLU^2.  With exponents that do not: 77 / 55 / 50.5, 214 / 143 / 137, 290 / 187 / 168.)
     bool somas = false;
     if (SOMA && wid != N_DW) {
@@ -436,8 +436,8 @@ __global__ void __launch_bounds__(CfgH<TNv, BLK>::N_THR, 1) k_gemm_h(const __gri
                     bt = bar_tfull + n_t % NS * 8;
                 }
             };
-            // The next tile.  With the bounds in registers from above, or a signed step, the loop of raw products comes out 3 % slower (4096 x 1024 x 16384
-            // 268 -> 278 us); where there are sums it is the other way round (16384 x 4096 x 512 209 us against 213).
+            // The next tile.  With the bounds in registers from above, or a signed step, the loop of raw products came out 3 % slower (4096 x 1024 x 16384
+            // 268 -> 278 us, now 235); where there are sums it was the other way round (16384 x 4096 x 512 209 us against 213, now 196).
             auto seguinte = [&](int tile) -> int {
                 if constexpr (SOMA) return tile + Pc.passo;
                 else return (int)((uint32_t)tile + (GRUPO ? (uint32_t)ntiles : gridDim.x));

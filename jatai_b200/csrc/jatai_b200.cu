@@ -167,9 +167,10 @@ static bool forma_gemm(int blk, int M, int N, int K, int modo) {
 }
 // Estimated times of the GEMM kernels in microseconds (measured at 64..16384 rows, 128..4096 columns, K = 64..16384): waves of tiles
 // times (64-element chunks of K x time per chunk + the start and end of a tile).  They place the lines between the kernels: against the
-// kernels forced one by one at 70 sizes the choice loses more than 3 % at three where every tile rounds, because it looks for sums (2048 x 1536 x 512 15.8 us
-// against 15.4, 2048 x 2048 x 512 with ReLU^2 18.3 against 17.7, 16384 x 4096 x 1024 256 against 248; where none rounds they are worth 16.2 -> 13.2, 18.0 -> 15.1,
-// 256 -> 167), at 8192 x 512 x 128 (14.6 against 13.7 with the 8-bit kernel) and, block 128, at 1024 x 512 x 4096 raw (34.8 against 25.2).
+// kernels forced one by one at 70 sizes the choice loses more than 3 % (3.1 to 5) at ten where every tile rounds, because it looks for sums (2048 x 1536 x 512
+// 16.6 us against 16.0, 16384 x 4096 x 1024 with ReLU^2 258 against 250; where none rounds they are worth 16.4 -> 13.8 and 257 -> 169), and at 2048 x 1024 x 1024
+// where none rounds, since 128 tiles do not look (15.2 against 14.1).  Outside of these sizes: K = 256 with 160 to 192 tiles that round (13.2 against 12.7 with the
+// 8-bit kernel), 256 tiles of K = 128 (11.9 and 11.4), and, block 128, 2048 x 1024 x 16384 raw (109 and 103).
 struct Custos { double i8, h64, h128; int grupo; };                  // grupo: blocks of a cluster per 64-wide tile
 static Custos custos_gemm(int blk, int M, int N, int K, int modo) {
     const bool cru = modo == 1;
@@ -259,10 +260,10 @@ static int gemm_h(const int8_t* A, const int8_t* EA, const int8_t* B, const int8
     if (!grupo) partes = (nped + ppp - 1) / ppp;                   // (in a cluster a block without chunks adds zeros)
     const th::Grade G = {N / tn, (M + 127) / 128, partes, ppp};
     // Whether tiles may add up in tensor memory where nothing is rounded.  It depends on the data, which the host does not see: each block looks at its
-    // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  With more than one tile per SM the gain where tiles qualify is 5 to 35 %
-    // (2048 x 1536 x 512 16.2 -> 13.2 us, 4096 x 1024 x 1024 24.4 -> 19.9, 16384 x 4096 x 1024 with ReLU^2 256 -> 167), the price where none does at most 4 %
-    // (15.4 -> 15.8, 23.2 -> 23.6, 247 -> 256).  With fewer the two are alike (4096 x 512 x 512 11.1 -> 10.5, 10.4 -> 10.9).  Larger K and raw
-    // outputs are not measured.
+    // tiles (k_gemm_h).  K <= 1024: the bounds of a tile are one word per lane.  With more than one tile per SM the gain where tiles qualify is 15 to 35 %
+    // (2048 x 1536 x 512 16.4 -> 13.8 us, 4096 x 1024 x 1024 24.3 -> 20.2, 16384 x 4096 x 1024 with ReLU^2 257 -> 169; K <= 128 3 to 12 %), the price where
+    // none does 1 to 5 % (16.0 -> 16.6, 23.4 -> 24.3, 250 -> 258).  With fewer both are about 5 % (4096 x 512 x 512 11.4 -> 10.8, 11.0 -> 11.7; 2048 x 1024 x 1024 15.2 -> 14.1,
+    // 14.9 -> 15.3).  Larger K and raw outputs are not measured.
     const bool soma = BLK == 32 && modo != 1 && !estreito && K <= 1024 && partes == 1 && tiles <= (long long)th::N_PLANOS * N_SM && (g_somas == 2 || (g_somas == 0 && tiles > N_SM));
     // The bounds with the shift serve every product.  Long rows are prepared faster without it (4096 x 1024 x 16384 raw 271 -> 267 us, the preparation
     // 55.2 -> 51.5), shorter ones with it (1536 x 512 x 4096 raw 42.8 against 43.0 us, 2048 x 512 x 2048 20.7 against 20.9).
