@@ -495,6 +495,7 @@ __device__ __noinline__ void transpoe_grava_lento(const int8_t* X, const int8_t*
     }
 }
 
+template <bool B> struct SimNao { static constexpr bool v = B; };
 template <int BLK, int CPT>
 __device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int c0, int R, int kid) {
     pdl_espera();
@@ -538,16 +539,19 @@ __device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int 
     uint32_t emax4 = 0x80808080u;                                  // the new exponents of this lane's columns, -128 where it has none
     if constexpr (BLK == 32) {
         // In halves, two rows at a time: with exponents at most 24 apart (all-zero blocks apart) a mantissa times 2^(e - eref) is exact, the largest gives the
-        // block's exponent, and one fused multiply-add against 1.5 * 2^10 rounds half to even while the factor is at most 2^15 (a column
-        // whose largest element lies further below the largest exponent of its 32-column block: fp32, the whole warp).
+        // block's exponent, and one fused multiply-add against 1.5 * 2^10 rounds half to even.  Its factor is at most 2^15: a column whose largest element lies
+        // further below the largest exponent of its 32-column block (2^30 at most) is multiplied by 2^15 first, which is exact, where a lane has one column.  (Left to
+        // fp32, the whole warp, such columns cost 4 to 6 % more than without halves: 2048 x 512 with few small elements 3.44 us, 3.30 without halves, 3.17 so.
+        // With four columns a lane, fp32: the second form of the output there costs every other input 1.5 %, 16384 x 4096 45.8 -> 46.7.)
+        // An all-zero block's row may lie anywhere below; beyond 24 its factor is 0.  Should its mantissas not be cleared, that is what they come to where
+        // the column's new exponent is -119 or more: at least eref - 15 >= -117 with one factor, eref - 30 >= -110 with two from eref = -80 on, and fp32 below that.
         __shared__ __align__(16) uint16_t esc_s[4][4][32];         // per warp and block: the rows' factors
         const bool perto = __reduce_or_sync(FULL, __vcmpgtu4(d4, 0x18181818u) & ~__vcmpeq4(ew, 0x81818181u)) == 0;
         if (perto) {
-            const uint32_t d24 = __vminu4(d4, 0x18181818u);
 #pragma unroll
             for (int b = 0; b < 4; b++) {
-                const int d = (d24 >> (8 * b)) & 0xff;
-                esc_s[wid][b][lane] = d <= 14 ? (uint16_t)((15 - d) << 10) : (uint16_t)(1 << (24 - d));      // 2^-d
+                const int d = (d4 >> (8 * b)) & 0xff;
+                esc_s[wid][b][lane] = d <= 14 ? (uint16_t)((15 - d) << 10) : d <= 24 ? (uint16_t)(1 << (24 - d)) : (uint16_t)0;      // 2^-d
             }
             __syncwarp();
             uint32_t he[16], t[CPT][16], mx[CPT];
@@ -573,7 +577,7 @@ __device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int 
                 }
             }
             int Eo[CPT];
-            bool serve = true;
+            bool serve = true;                                     // the factors of this lane's columns are 2^15 at most
 #pragma unroll
             for (int c = 0; c < CPT; c++) {
                 const uint32_t m = max(mx[c] & 0xFFFFu, mx[c] >> 16);                                       // (not negative: ordered like their bits)
@@ -582,14 +586,21 @@ __device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int 
                 Eo[c] = m == 0 ? SEM_TOPO : eref + (__float_as_int(f) >> 23) - 126 - 7;
                 serve = serve && (m == 0 || eref - Eo[c] <= 15);
             }
-            if (__all_sync(FULL, serve)) {
+            auto grava = [&](auto longe15) {                       // longe15: some factor is beyond 2^15
 #pragma unroll
                 for (int c = 0; c < CPT; c++) {
                     const int k = k0 + c;
                     const size_t col = (size_t)col0 + k;
                     const bool morto = Eo[c] < -126;
                     if (dentro && Eo[c] > 126) reporta(E_EXP, kid, (long long)col * R + lin0, Eo[c], eref);
-                    const uint32_t B = morto ? 0u : (uint32_t)(15 + eref - Eo[c]) << 10, B2 = B | B << 16;  // 2^(eref - Eo)
+                    int kB = eref - Eo[c];                                                                  // 2^kB
+                    if constexpr (decltype(longe15)::v) {
+                        const uint32_t A2 = kB > 15 ? 0x78007800u : 0x3C003C00u;                            // 2^15 (an empty column's zeros too) or 1
+#pragma unroll
+                        for (int j = 0; j < 16; j++) asm("mul.rn.f16x2 %0, %0, %1;" : "+r"(t[c][j]) : "r"(A2));
+                        if (kB > 15) kB -= 15;
+                    }
+                    const uint32_t B = morto ? 0u : (uint32_t)(15 + kB) << 10, B2 = B | B << 16;
                     if (morto) Eo[c] = E_ZERO;
                     if (dentro) {
                         uint32_t q[16];
@@ -605,6 +616,13 @@ __device__ __forceinline__ void transpoe_corpo(const ArgsTransp& A, int r0, int 
                     emax4 = (emax4 & ~(0xffu << (8 * k))) | ((uint32_t)(uint8_t)(int8_t)Eo[c] << (8 * k));
                 }
                 if (A.RM != nullptr && dentro) max4_atomico(A.RM + col0, emax4);
+            };
+            if (__all_sync(FULL, serve)) {
+                grava(SimNao<false>());
+                return;
+            }
+            if (CPT == 1 && !__any_sync(FULL, !serve && eref < -80)) {
+                grava(SimNao<true>());
                 return;
             }
         }

@@ -70,7 +70,8 @@ def inteiros(semente):
 # ------------------------------------------------------------------------------------------------ transposition
 def em_metades(X, colunas):
     """How many (32 rows x 128 columns, columns a lane) pieces meet both conditions of the transposition in halves, of how many: exponents at most 24 apart,
-    all-zero blocks aside, and no column whose largest element lies so far down that its factor exceeds 2^15."""
+    all-zero blocks aside, and no column whose largest element lies so far down that its factor exceeds 2^15 (with one column a lane, in a block whose largest
+    exponent is below -80)."""
     m, E = (t.to(torch.int64) for t in X)
     R, C = m.shape
     falta = -C % 128
@@ -82,6 +83,8 @@ def em_metades(X, colunas):
     bits = torch.frexp(m.abs().to(torch.float64))[1].to(torch.int64)
     topo = torch.where(m != 0, bits + E[..., None], torch.full_like(m, -1000)).amax(1)
     serve = (topo == -1000) | (ref[:, 0, :, :, None] - (topo - 7) <= 15)
+    if colunas == 1:
+        serve = serve | (ref[:, 0, :, :, None] >= -80)
     serve = serve.reshape(*serve.shape[:3], 8, 4)        # 8 lanes of 4 columns in a block
     serve = serve.all(4).all(3).all(2) if colunas == 4 else serve.all(3).all(2)
     return int((perto[..., None] & serve.reshape(*perto.shape, -1)).sum()), serve.numel()
@@ -106,19 +109,52 @@ def test_transpoe_metades_todos_os_fatores(amb, R, C, colunas, afasta):
 
 
 @pytest.mark.parametrize("R,C,colunas", [(128, 192, 1), (8192, 1088, 4)])
-@pytest.mark.parametrize("fundo", [8, 9, 10])
-def test_transpoe_metades_fatores_grandes(amb, R, C, colunas, fundo):
-    """In one block of four, a column that holds nothing but ones `fundo` below the largest exponent: its factor is 2^14, 2^15 (the last that halves hold) or 2^16."""
+@pytest.mark.parametrize("e0", [-10, -80, -81])
+@pytest.mark.parametrize("fundo", [8, 9, 10, 24])
+def test_transpoe_metades_fatores_grandes(amb, R, C, colunas, e0, fundo):
+    """In one block of four, a column that holds nothing but ones `fundo` below the largest exponent: its factor is 2^14, 2^15 (the largest half), 2^16 or 2^30 (the most
+    there is), which take two multiplications, or fp32 with four columns a lane or below the exponent -80."""
     ops, oc, reg = amb
     G = casos.Gen(R + C + fundo, 32)
-    m, E = G.bloco(R, C, e0=-10, espalha=0)
-    E[1::3, 1::4] = -10 - fundo
+    m, E = G.bloco(R, C, e0=e0, espalha=0)
+    E[1::3, 1::4] = e0 - fundo
     m[:, 41::128] = 0
     m[1::3, 41::128] = 1
     tem, de = em_metades((m, E), colunas)
-    assert tem == de if fundo <= 9 else tem < de
+    assert tem == de if fundo <= 9 or (colunas == 1 and e0 >= -80) else tem < de
     X = para_gpu((m, E))
-    compara(f"transpoe {R}x{C} fundo {fundo}", list(oc.transpoe(X)), list(spec.Spec(32).transpoe(X)))
+    compara(f"transpoe {R}x{C} e0 {e0} fundo {fundo}", list(oc.transpoe(X)), list(spec.Spec(32).transpoe(X)))
+
+
+@pytest.mark.parametrize("R,C,colunas", [(128, 192, 1), (8192, 1088, 4)])
+def test_transpoe_metades_esparsa(amb, R, C, colunas):
+    """Few elements of any size at exponents 24 apart: columns with every factor in one warp, empty ones among them."""
+    ops, oc, reg = amb
+    G = casos.Gen(R + C, 32)
+    m, E = G.bloco(R, C, e0=-20, espalha=12)
+    m[torch.rand(R, C, generator=G.g) > 0.04] = 0
+    tem, de = em_metades((m, E), colunas)
+    assert tem == de if colunas == 1 else tem < de
+    X = para_gpu((m, E))
+    compara(f"transpoe {R}x{C}", list(oc.transpoe(X)), list(spec.Spec(32).transpoe(X)))
+
+
+@pytest.mark.parametrize("R,C", [(128, 192), (8192, 1088)])
+@pytest.mark.parametrize("e0", [-126, -120, -103, -102, -95, -81, -80, -10, 0])
+def test_transpoe_menor_expoente_com_mantissas(amb, R, C, e0):
+    """Blocks of exponent -127 whose mantissas are not cleared: their elements count as what they are (all but nothing), also where they are a column's only ones, or beside
+    ones 24 below the largest exponent."""
+    ops, oc, reg = amb
+    G = casos.Gen(R + C + 1000 - e0, 32)
+    m, E = G.bloco(R, C, e0=e0, espalha=0)
+    E[1::5] = max(e0 - 24, -126)
+    E[2::5] = casos.E_ZERO
+    linha = torch.arange(R) % 5
+    m[linha != 2, 7::32] = 0
+    m[(linha != 2) & (linha != 1), 9::32] = 0
+    m[linha == 1, 9::32] = 1
+    X = para_gpu((m, E))
+    compara(f"transpoe {R}x{C} e0 {e0}", list(oc.transpoe(X)), list(spec.Spec(32).transpoe(X)))
 
 
 # ------------------------------------------------------------------------------------------------ products
